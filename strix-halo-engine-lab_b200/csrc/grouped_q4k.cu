@@ -1,159 +1,96 @@
-// Routed experts, Qwen A8 family, GROUPED form for token blocks (prefill): the integer dots run on the 5th-generation
-// tensor cores (tcgen05.mma kind::i8, accumulators in tensor memory), everything after the dots is the same declared
-// FP32 arithmetic as the decode kernels, so the results are bit for bit those of gemv_q4k.cu / gemv_q4k_stream.cu
-// (contract: src/cpu/core/routed_expert.hpp:9-15, row rule routed_expert.cpp:73-108; the reference's own tensor-core
-// form is project_kernel / down_kernel over IMMA tiles, src/cuda/core/moe_a8.cuh:76-206, :225-341).
+// Routed experts, Qwen A8 family, GROUPED form for token blocks (prefill): the integer dots run on the tensor cores, everything
+// after the dots is the same declared FP32 arithmetic as the decode kernels, so the results are bit for bit those of
+// gemv_q4k.cu / gemv_q4k_stream.cu (contract: src/cpu/core/routed_expert.hpp:9-15, row rule routed_expert.cpp:73-108; the
+// reference's own tensor-core form is project_kernel / down_kernel, src/cuda/core/moe_a8.cuh:76-206, :225-341).
 //
-// Why one MMA per 32-wide group: the contract scales every group's EXACT integer dot by its own FP32 factors and adds
-// the terms in a fixed order, so the tensor core may only produce dot_g, never a sum over groups. kind::i8 has K = 32:
-// one instruction = one Q4_K group for a 128 x 64 tile (weight rows x tokens).
+// What bounds it: the FP32 pipe and the shared-memory reads that feed it. The contract scales every 32-wide group's EXACT
+// integer dot by its own factors: five FP32 operations per (row, token, group), i.e. 320 clocks per group of a 128 x 64 tile at
+// 128 lanes a clock. The dots of the same group take 136 clocks of the register-to-register integer MMA (measured: 8.5 clocks
+// per m16n8k32 and scheduler, 22.5 together with ten packed FP32 instructions), so the dots stay in REGISTERS. The form before
+// this one (tcgen05 with accumulators in tensor memory, operands unpacked to shared memory) spent 980 clocks per group, most of
+// them in its unpack -> MMA -> drain hand-overs: 1230 us for 512 tokens x 34,816 rows x 5120, @GU@ us now.
 //
-// Tile = (expert, 128 weight rows, 64 of the expert's tokens). gate/up: rows 0..63 are gate rows [64c, 64c + 64), rows
+// Tile = (expert, 128 weight rows, kGN of the expert's tokens). gate/up: rows 0..63 are gate rows [64c, 64c + 64), rows
 // 64..127 the up rows of the same outputs, so SwiGLU + the A8 rule of h finish inside the tile. down: 128 rows of H.
-// A persistent CTA per SM walks tiles round-robin; four roles:
-//   * issuer (1 warp, one thread): drives both asynchronous engines. The weight rows of a super-block arrive by two tiled
-//     TMA copies (cp.async.bulk.tensor.2d: 144 bytes x 64 rows, the tile's gate rows and up rows, or two halves of its
-//     down rows) into a raw ring, four super-blocks ahead of their use; the 4 MMAs of a stage (M 128, N 64, K 32,
-//     s8 x s8 -> s32) go into one half of tensor memory as soon as the stage's operands are published, and are
-//     committed to an mbarrier.
-//   * unpacker warps (4): per stage = half a super-block (4 groups): unpack the rows' nibbles (from the raw ring) to
-//     bytes into the MMA's canonical K-major layout (8-row x 16-byte core matrices), gather the tokens' A8 codes into
-//     the same layout (ordinary loads, one stage ahead), stage the tokens' {E_g, S_g} and the rows' 16-byte block headers.
-//   * drain warps (8): thread = (weight row = TMEM lane, 32 of the 64 tokens: the 8-token chunks alternate between the
-//     two warp groups, so a tile with few tokens still uses every warp). tcgen05.ld brings 8 dots at a time;
-//     x_g = E_g * ((d * sc_g) * float(dot_g) - (dmin * m_g) * float(S_g)), pair sums, the four chains acc_p over
-//     ascending super-blocks, (a0 + a1) + (a2 + a3) at the end - exactly the decode kernels' order.
-//   * tensor memory: 512 columns = 2 buffers x 4 groups x 64 tokens; smem stages follow the same two buffers.
-// Every wait is bounded (kWaitLimit polls); on a timeout the roles stop working, the launch sets bit 30 of the job
-// summary, frees tensor memory and returns.
-//
-// Roofline: CUDA-core FP32 issue, not the tensor pipe and not HBM - about 8 instructions per (row, token, group),
-// against 1/32 of a tensor instruction. Weights are re-read from L2 once per token tile.
+// A persistent CTA per SM walks tiles round-robin; a stage of the ring (three) is one super-block: 256 columns.
+//   * helper warps (4): the tile's weight rows arrive by two tiled TMA copies (160 bytes x 64 rows: the 144 of the super-block
+//     and 16 more, which puts rows 8 (mod 32) words apart - the fragment loads below are conflict free), the tokens' codes by
+//     16-byte asynchronous copies (288 bytes apart, for the same reason), one stage ahead. A helper thread decodes the
+//     factors of one weight row and transposes {E, S} of one token (half the groups each).
+//   * consumer warps: warp = 32 rows x every kSplit-th 8-token chunk (a tile with few tokens still uses most warps). The
+//     nibbles go from shared memory straight into A fragments (low nibbles by a mask, high nibbles left in place as 16 q), the
+//     codes into B fragments; the MMA starts at the integer 0x4b400000, so its result read as a float is M + dot with
+//     M = 1.5 * 2^23, and fma(D, M + dot, -D * M) is D * dot rounded once (D = d * scale has at most 17 significant bits, so
+//     D * M is exact): no conversion. Packed FP32 instructions work on two tokens at a time; the four chains acc_p of a lane's
+//     cells stay in registers; (a0 + a1) + (a2 + a3) at the end - exactly the decode kernels' order.
+//     A super-block with a non-finite d takes the same steps with the dot converted first (inf - inf would turn an infinity
+//     into a NaN).
+// Every wait is bounded; on a timeout the roles stop working and the launch sets B200MOE_JOB_WAIT_ABORTED in the job summary.
 #include <cuda.h>
 
-#include "declared_math.cuh"
-#include "kernels.cuh"
+#include "q4k_row.cuh"
 
 namespace b200moe {
 namespace {
+using namespace q4k;
 
-constexpr u32 kGM = 128, kGN = 64;           // tile: weight rows x tokens
-constexpr u32 kDrainWarps = 8, kLoadWarps = 4, kIssueWarps = 4;  // of the last group only warp 0 works (whole warp groups trade registers)
-constexpr u32 kGThreads = (kDrainWarps + kLoadWarps + kIssueWarps) * 32;
-constexpr u32 kStageGroups = 4;              // half a super-block per stage
-constexpr u32 kTPT = kGN / (kDrainWarps / 4);   // tokens per drain thread (32)
-constexpr u32 kDrainGroups = kDrainWarps / 4;    // warp groups sharing a tile's tokens: the 8-token chunks alternate between them
-constexpr u32 kTmemCols = 512;
-constexpr u32 kABytes = kStageGroups * kGM * 32, kBBytes = kStageGroups * kGN * 32, kEsBytes = kStageGroups * kGN * 8, kHdrBytes = kGM * 16;
-constexpr u32 kStageBytes = kABytes + kBBytes + kEsBytes + kHdrBytes;  // 28672
-constexpr u32 kOutBytes = kGN * kGM * 4;     // epilogue tile (gate/up)
+#ifndef SPLIT
+#define SPLIT 2
+#define CHUNKS 4
+#endif
+constexpr u32 kSplit = SPLIT, kChunks = CHUNKS;  // consumer warps that share a tile's tokens; 8-token chunks of each
+constexpr u32 kGM = 128, kGN = 8 * kSplit * kChunks;  // tile: weight rows x tokens
+constexpr u32 kConsumers = 4 * kSplit, kHelpers = 4;  // warps
+constexpr u32 kGThreads = (kConsumers + kHelpers) * 32;
+constexpr u32 kStages = 3;
+constexpr u32 kRowPitch = kQ4KBlock + 16, kCodePitch = 256 + 32;
+constexpr u32 kRawBytes = kGM * kRowPitch, kCodeBytes = kGN * kCodePitch, kEsBytes = 8 * kGN * 8, kFacBytes = 8 * kGM * 8, kPrivBytes = kHelpers * 32 * 32;
+constexpr u32 kStageBytes = kRawBytes + kCodeBytes + kEsBytes + kFacBytes + kPrivBytes;
+constexpr u32 kOutPitch = kGM + 4;           // floats; twice the pitch is 8 (mod 32): the fragment stores meet every bank once
+constexpr u32 kOutBytes = kGN * kOutPitch * 4;  // epilogue tile (gate/up)
 constexpr u32 kMaxUnion = 1024;
-constexpr u32 kRawDepth = 4, kRawBlock = kGM * kQ4KBlock;  // ring of raw super-blocks (128 rows x 144 B) fed by bulk copies
-constexpr u32 kBarBytes = (6 + 2 * kRawDepth) * 8 + 16;  // full[2], empty[2], ready[2], raw_full[], raw_free[]
-// above half an SM's shared memory: never two CTAs (and two TMEM allocations) per SM
-constexpr u32 kGroupedSmem = 2 * kStageBytes + kOutBytes + (kMaxUnion + 2) * 4 + kBarBytes + kRawDepth * kRawBlock + 256;
+constexpr u32 kBarBytes = 3 * kStages * 8 + 24 + kStages * 16 + 2 * 64 * 4;  // raw_full[], ready[], empty[]; abort flag; non-finite flags; token rows
+constexpr u32 kGroupedSmem = kStages * kStageBytes + kOutBytes + (kMaxUnion + 2) * 4 + kBarBytes + 64;
+static_assert(kGN <= 64 && kGN % 16 == 0, "a helper thread stages half the groups of one token");
 static_assert(kGroupedSmem > 114u * 1024u && kGroupedSmem <= 227u * 1024u, "one CTA per SM, within the shared memory of an SM");
-constexpr u32 kWaitLimit = 1u << 22;
-constexpr u32 kAbortBit = B200MOE_JOB_WAIT_ABORTED;
-// instruction descriptor: D = s32, A = B = signed 8-bit, both K-major, N = 64, M = 128
-constexpr u32 kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((kGN >> 3) << 17) | ((kGM >> 4) << 24);
+constexpr u32 kWaitLimit = 1u << 20;         // polls of up to a microsecond
+constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23 = the float with the bits 0x4b400000
+// Register split between whole warp groups, out of what the launch gives every thread (65,536 over the threads, by eights).
+constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kHelperRegs = kSplit == 2 ? 56 : 80;
+constexpr u32 kConsumerRegs = (kGThreads * kLaunchRegs - kHelpers * 32u * kHelperRegs) / (kConsumers * 32u) / 8u * 8u;
+static_assert(kConsumers * 32 * kConsumerRegs + kHelpers * 32 * kHelperRegs <= kGThreads * kLaunchRegs, "setmaxnreg split exceeds the launch's registers");
 
-__device__ __forceinline__ u32 saddr(const void* p) { return static_cast<u32>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void mbar_init(u64* bar, u32 count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(u64* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(u64* bar, u32 bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(bar)), "r"(bytes) : "memory");
-}
-// One tiled TMA copy: a box of 144 bytes x 64 rows of a [rows][row_bytes] byte tensor into shared memory (rows end up
-// contiguous, 144 bytes each). x is a multiple of 16 bytes (a super-block boundary).
-__device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, u32 x, u32 y, u64* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(saddr(dst)),
-                 "l"(reinterpret_cast<u64>(map)), "r"(x), "r"(y), "r"(saddr(bar))
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(u64* bar, u32 parity) {
-    u32 ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(saddr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(u64* bar, u32 parity, volatile u32* abort_flag) {
-    for (u32 i = 0; i < kWaitLimit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 127u) == 127u) {
-            if (*abort_flag) return false;
-            __nanosleep(64);
-        }
-    }
-    *abort_flag = 1;
-    return false;
-}
-// Shared-memory matrix descriptor, K-major, no swizzle: 8-row x 16-byte core matrices; LBO = bytes between the two
-// 16-byte K chunks of a row group, SBO = bytes between 8-row groups; bits 46-47 = 1 (Blackwell descriptor version).
-__device__ __forceinline__ u64 smem_desc(u32 addr, u32 lbo, u32 sbo) {
-    return u64((addr >> 4) & 0x3fffu) | (u64((lbo >> 4) & 0x3fffu) << 16) | (u64((sbo >> 4) & 0x3fffu) << 32) | (u64(1) << 46);
-}
-__device__ __forceinline__ void mma_i8(u32 d_tmem, u64 a_desc, u64 b_desc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdesc), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit(u64* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld8(u32 taddr, u32* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-// Ties registers to the point after tcgen05.wait::ld, so that no use of a loaded value is scheduled before the wait.
-__device__ __forceinline__ void tie8(u32* v) {
-    asm volatile("" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]));
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ float small_int_to_float(int v) { return __fsub_rn(__int_as_float(0x4b400000 + v), 12582912.0f); }
-// Two FP32 lanes per instruction (Blackwell packed FP32): each lane is one IEEE round-to-nearest multiplication, the
-// same result as two scalar instructions at half the issue slots. Only the multiplications are packed: a packed add
-// fed by a packed multiply did not reproduce the scalar bits on B200 (it behaves as contracted), so the adds stay scalar.
+// Two FP32 lanes per instruction (Blackwell packed FP32): each lane is one IEEE round-to-nearest operation, the same result
+// as two scalar instructions at half the issue slots. A packed add fed by a packed multiply did not reproduce the scalar
+// bits on B200 (it behaves as contracted), so an add is written as a * 1 + b, where the 1 is a kernel argument that no
+// compiler stage can fold away: one rounding, of a + b.
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     float2 c;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<u64&>(c)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)));
     return c;
 }
-
-struct Factors { float Dl, DMl, Dh, DMh; };
-__device__ __forceinline__ Factors q4k_factors(const uint4& hdr, u32 p) {  // routed_expert.cpp:65-71, as in gemv_q4k_stream.cu
-    const float d = half_bits_to_float(hdr.x & 0xffffu), dm = half_bits_to_float(hdr.x >> 16);
-    const u32 sc_lo = hdr.y & 0x3f3f3f3fu, mn_lo = hdr.z & 0x3f3f3f3fu;
-    const u32 sc_hi = (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
-    const u32 mn_hi = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
-    const u32 scw = p < 2u ? sc_lo : sc_hi, mnw = p < 2u ? mn_lo : mn_hi;
-    const u32 sh = 16u * (p & 1u);
-    Factors f;
-    f.Dl = __fmul_rn(d, small_int_to_float((scw >> sh) & 0xffu));
-    f.Dh = __fmul_rn(d, small_int_to_float((scw >> (sh + 8u)) & 0xffu));
-    f.DMl = __fmul_rn(dm, small_int_to_float((mnw >> sh) & 0xffu));
-    f.DMh = __fmul_rn(dm, small_int_to_float((mnw >> (sh + 8u)) & 0xffu));
-    return f;
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<u64&>(d)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)), "l"(reinterpret_cast<const u64&>(c)));
+    return d;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+// 16 weight rows x 8 tokens x one group: unsigned nibble bytes times signed codes, on top of the bits of kMagic.
+__device__ __forceinline__ void mma_magic(float2 (&d)[2], u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=r"(reinterpret_cast<u32&>(d[0].x)), "=r"(reinterpret_cast<u32&>(d[0].y)), "=r"(reinterpret_cast<u32&>(d[1].x)), "=r"(reinterpret_cast<u32&>(d[1].y))
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4b400000));
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr(dst)), "l"(src) : "memory");
 }
 
 struct GroupedArgs {
     b200moe_shape shape;
     b200moe_routes routes;
-    const u8* w0;            // gate (gate/up mode) or down tensor
-    const u8* w1;            // up
     b200moe_a8_rows in;      // x (gate/up: indexed by row) or act (down: indexed by slot)
     b200moe_a8_rows act;     // gate/up output
     float* gate_out;
@@ -163,6 +100,7 @@ struct GroupedArgs {
     u32* summary;
     u32 n_row_tiles;         // inter / 64 (gate/up) or hidden / 128 (down)
     u32 K;                   // hidden (gate/up) or inter (down)
+    float one;               // 1.0f, unknown to the compiler (mul2 / fma2)
 };
 
 struct Tile { u32 expert, eb, nt, c, tt; };
@@ -185,17 +123,95 @@ __device__ __forceinline__ Tile find_tile(const GroupedArgs& a, const u32* cum, 
     return t;
 }
 
+// One super-block of the warp's 32 rows against the tokens of its chunks. rows: the lane's first weight row of the stage (nibbles
+// of its k slice); codes: the lane's token row of chunk 0; es / fac: the lane's {E, E', S, S'} and {rows 0, 8, 16, 24} factors.
+// acc[cc][i][p]: chain p of weight row 8 i + lane / 4 and two tokens of chunk kSplit cc + w. SLOW: the dot is converted first.
+template <bool SLOW>
+__device__ __forceinline__ void superblock(const unsigned char* rows, const unsigned char* codes, const float4* es, const float4* fac, u32 n_chunks,
+                                           float2 one, float2 (&acc)[kChunks][4][4]) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        uint2 q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const uint2*>(rows + 8 * i * kRowPitch + 32 * p);
+        float Dl[4], Ml[4], Dh[4], Mh[4], Nl[4], Nh[4];
+        *reinterpret_cast<float4*>(Dl) = fac[(4 * p) * (kGM / 4)]; *reinterpret_cast<float4*>(Ml) = fac[(4 * p + 1) * (kGM / 4)];
+        *reinterpret_cast<float4*>(Dh) = fac[(4 * p + 2) * (kGM / 4)]; *reinterpret_cast<float4*>(Mh) = fac[(4 * p + 3) * (kGM / 4)];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { Nl[i] = __fmul_rn(Dl[i], -kMagic); Nh[i] = __fmul_rn(Dh[i], -kMagic); }
+#pragma unroll
+        for (int cc = 0; cc < (int)kChunks; ++cc) {
+            if (cc >= n_chunks) break;  // no valid token in these columns (warp-uniform)
+            const unsigned char* c = codes + 8 * kSplit * cc * kCodePitch + 64 * p;
+            const uint2 bl = *reinterpret_cast<const uint2*>(c), bh = *reinterpret_cast<const uint2*>(c + 32);
+            const float4 el = es[(2 * p) * (kGN / 2) + 4 * kSplit * cc], eh = es[(2 * p + 1) * (kGN / 2) + 4 * kSplit * cc];
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                float2 l[2], h[2];
+                const uint2 r0 = q[2 * mt], r1 = q[2 * mt + 1];
+                mma_magic(l, r0.x & 0x0f0f0f0fu, r1.x & 0x0f0f0f0fu, r0.y & 0x0f0f0f0fu, r1.y & 0x0f0f0f0fu, bl.x, bl.y);
+                mma_magic(h, r0.x & 0xf0f0f0f0u, r1.x & 0xf0f0f0f0u, r0.y & 0xf0f0f0f0u, r1.y & 0xf0f0f0f0u, bh.x, bh.y);
+#pragma unroll
+                for (int z = 0; z < 2; ++z) {
+                    const int i = 2 * mt + z;
+                    float2 al, ah;
+                    if (SLOW) {
+                        al = mul2(both(Dl[i]), make_float2(__fsub_rn(l[z].x, kMagic), __fsub_rn(l[z].y, kMagic)));
+                        ah = mul2(both(Dh[i]), make_float2(__fsub_rn(h[z].x, kMagic), __fsub_rn(h[z].y, kMagic)));
+                    } else {
+                        al = fma2(both(Dl[i]), l[z], both(Nl[i]));
+                        ah = fma2(both(Dh[i]), h[z], both(Nh[i]));
+                    }
+                    // x = E * ((D * float(dot)) - (DM * S)) for the pair's two groups; M holds -DM, and (-DM) * S = -(DM * S) exactly
+                    const float2 sl = fma2(al, one, mul2(both(Ml[i]), make_float2(el.z, el.w)));
+                    const float2 sh = fma2(ah, one, mul2(both(Mh[i]), make_float2(eh.z, eh.w)));
+                    const float2 x = fma2(mul2(make_float2(el.x, el.y), sl), one, mul2(make_float2(eh.x, eh.y), sh));
+                    acc[cc][i][p] = fma2(x, one, acc[cc][i][p]);
+                }
+            }
+        }
+    }
+}
+
+// SwiGLU + the A8 rule of up to four (token, 32 outputs) tasks of one warp, step by step over the four, so that their shuffle
+// and division chains overlap. g, u: the lane's gate and up values; returns per task whether a value is not finite.
+constexpr int kTasks = 4;
+__device__ __forceinline__ u32 swiglu_a8(const float (&g)[kTasks], const float (&u)[kTasks], int (&code)[kTasks], float (&delta)[kTasks], int (&sum)[kTasks]) {
+    float h[kTasks], amax[kTasks];
+    u32 bad = 0;
+#pragma unroll
+    for (int i = 0; i < kTasks; ++i) { h[i] = swiglu_qwen(g[i], u[i]); amax[i] = fabsf(h[i]); }
+#pragma unroll
+    for (int i = 0; i < kTasks; ++i) bad |= __any_sync(0xffffffffu, !finite_f(g[i]) || !finite_f(u[i]) || !finite_f(h[i])) ? 1u << i : 0u;
+#pragma unroll
+    for (int d = 16; d; d >>= 1)
+#pragma unroll
+        for (int i = 0; i < kTasks; ++i) amax[i] = fmaxf(amax[i], __shfl_xor_sync(0xffffffffu, amax[i], d));
+#pragma unroll
+    for (int i = 0; i < kTasks; ++i) {  // a8_quantize_lane (common.cuh)
+        const bool tiny = amax[i] > 0.0f && amax[i] < 0x1p-119f;
+        delta[i] = (amax[i] == 0.0f || tiny) ? 1.0f : __fdiv_rn(amax[i], 127.0f);
+        const float r = tiny ? 0.0f : rintf(__fdiv_rn(h[i], delta[i]));
+        const float lo = (-127.0f < r) ? r : -127.0f;
+        code[i] = static_cast<int>((lo < 127.0f) ? lo : 127.0f);
+        sum[i] = __reduce_add_sync(0xffffffffu, code[i]);
+    }
+    return bad;
+}
+
 template <bool kDown>
 __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
                                                                    GroupedArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char* stage0 = smem;                                       // 2 x kStageBytes
-    float* s_out = reinterpret_cast<float*>(smem + 2 * kStageBytes);    // [kGN][kGM]
-    u32* cum = reinterpret_cast<u32*>(smem + 2 * kStageBytes + kOutBytes);  // [kMaxUnion + 1]
-    u64* bars = reinterpret_cast<u64*>(cum + kMaxUnion + 2);            // full[2], empty[2], ready[2], raw_full[], raw_free[]
-    u32* s_tmem = reinterpret_cast<u32*>(bars + 6 + 2 * kRawDepth);
-    volatile u32* s_abort = s_tmem + 1;
-    unsigned char* raw = smem + ((2 * kStageBytes + kOutBytes + (kMaxUnion + 2) * 4 + kBarBytes + 127u) & ~127u);  // [kRawDepth][kRawBlock]
+    float* s_out = reinterpret_cast<float*>(smem + kStages * kStageBytes);          // [kGN][kOutPitch]
+    u64* raw_full = reinterpret_cast<u64*>(smem + kStages * kStageBytes + kOutBytes);
+    u64* ready = raw_full + kStages;
+    u64* empty = ready + kStages;
+    u32* s_abort_word = reinterpret_cast<u32*>(empty + kStages);                     // 24 bytes
+    u32* s_slow = s_abort_word + 6;                                                  // [stage][row quarter]: a non-finite d among the rows
+    u32* s_src = s_slow + kStages * 4;                                               // [tile parity][64]: A8 rows of the tile's tokens
+    u32* cum = s_src + 2 * 64;                                                       // [kMaxUnion + 1]
+    volatile u32* s_abort = s_abort_word;
 
     if (kDown && a.summary && *a.summary) return;  // a failed or aborted projection skips the stage (routed_expert.hpp:17-19)
 
@@ -204,11 +220,8 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     for (u32 j = tid; j < n_union; j += kGThreads) cum[j + 1] = (a.routes.begins[j + 1] - a.routes.begins[j] + kGN - 1) / kGN;
     if (tid == 0) {
         cum[0] = 0;
-        mbar_init(&bars[0], 1); mbar_init(&bars[1], 1);
-        mbar_init(&bars[2], kDrainWarps * 32); mbar_init(&bars[3], kDrainWarps * 32);
-        mbar_init(&bars[4], kLoadWarps * 32); mbar_init(&bars[5], kLoadWarps * 32);
-        for (u32 i = 0; i < kRawDepth; ++i) { mbar_init(&bars[6 + i], 1); mbar_init(&bars[6 + kRawDepth + i], kLoadWarps * 32); }
-        *s_abort = 0;
+        for (u32 i = 0; i < kStages; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&ready[i], kHelpers); mbar_init(&empty[i], kConsumers); }
+        *s_abort_word = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -221,264 +234,198 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
             if (j0 + lane < n_union) cum[j0 + lane + 1] = carry + v;
             carry += __shfl_sync(0xffffffffu, v, 31);
         }
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(s_tmem)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    tc_fence_before();
     __syncthreads();
-    tc_fence_after();
-    const u32 tmem = *s_tmem;
     const u32 n_tiles = cum[n_union] * a.n_row_tiles;
-    const u32 K = a.K, I = a.shape.inter, H = a.shape.hidden;
-    const u32 nblocks = K / 256;
-    const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, in_gs = in_stride / 32;
-    u64* full = bars;
-    u64* empty = bars + 2;
-    u64* ready = bars + 4;
-    u64* raw_full = bars + 6;
-    u64* raw_free = bars + 6 + kRawDepth;
+    const u32 I = a.shape.inter, H = a.shape.hidden;
+    const u32 nblocks = a.K / 256;
     bool ok = true;
-    u32 n = 0;  // stage counter of this role (all roles count alike)
     const u32 my_tiles = n_tiles > blockIdx.x ? (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
-    const u32 total_sb = my_tiles * nblocks;
-    // Register split between whole warp groups (the CTA holds 512 x 128): the drain threads - 128 accumulators each - take
-    // what the unpackers and the issuer group give up: 256 x 192 + 128 x 96 + 128 x 24 <= 512 x 128.
-    static_assert(kDrainWarps * 32 * 192 + kLoadWarps * 32 * 96 + kIssueWarps * 32 * 24 <= kGThreads * 128, "setmaxnreg split exceeds the register file share");
+    const u32 total = my_tiles * nblocks;  // stages of this CTA
 
-    if (warp >= kDrainWarps + kLoadWarps) {
-        // ============================================================================ issuer: TMA copies + MMA issue
-        // One thread drives both asynchronous engines. The weight rows of super-block m of the CTA's sequence (tiles in
-        // order, blocks in order) arrive by two tiled TMA copies (144 bytes x 64 rows each: the gate rows and the up rows
-        // of the tile, or two halves of the down rows) into ring slot m % kRawDepth, kRawDepth super-blocks ahead of
-        // their use; the four MMAs of a stage are issued as soon as the unpackers have published its operands.
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
-        if (warp == kDrainWarps + kLoadWarps) {
-            u32 ck = 0xffffffffu, cy = 0;
-            auto tma_block = [&](u32 mm) {  // lane 0 only
-                const u32 k = mm / nblocks, b = mm - k * nblocks;
-                if (k != ck) {
-                    ck = k;
-                    const Tile t = find_tile(a, cum, n_union, blockIdx.x + k * gridDim.x);
-                    cy = kDown ? t.expert * H + kGM * t.c : t.expert * I + 64u * t.c;
-                }
-                const u32 slot = mm % kRawDepth;
-                unsigned char* dst = raw + slot * kRawBlock;
-                mbar_expect_tx(&raw_full[slot], kRawBlock);
-                tma_2d(dst, &tm0, b * kQ4KBlock, cy, &raw_full[slot]);
-                tma_2d(dst + 64u * kQ4KBlock, kDown ? &tm0 : &tm1, b * kQ4KBlock, kDown ? cy + 64u : cy, &raw_full[slot]);
-            };
-            if (lane == 0) for (u32 mm = 0; mm < min(kRawDepth, total_sb); ++mm) tma_block(mm);
-            u32 m = 0;
-            for (u32 k = 0; k < my_tiles; ++k) {
-                for (u32 s = 0; s < 2 * nblocks; ++s, ++n) {
-                    const u32 buf = n & 1u, use = n >> 1, hf = s & 1u;
-                    if (ok) ok = mbar_wait(&ready[buf], use & 1u, s_abort);  // the stage's operands are in shared memory
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (ok && lane == 0) {
-                        tc_fence_after();
-                        const u32 abase = saddr(stage0 + buf * kStageBytes), bbase = abase + kABytes;
-#pragma unroll
-                        for (u32 gi = 0; gi < kStageGroups; ++gi)
-                            mma_i8(tmem + buf * (kStageGroups * kGN) + gi * kGN, smem_desc(abase + gi * (kGM * 32), 128, 256),
-                                   smem_desc(bbase + gi * (kGN * 32), 128, 256));
-                        mma_commit(&full[buf]);
-                    }
-                    if (hf == 1) {
-                        if (m + kRawDepth < total_sb) {  // the slot has been read out: the block kRawDepth ahead takes it
-                            if (ok) ok = mbar_wait(&raw_free[m % kRawDepth], (m / kRawDepth) & 1u, s_abort);
-                            ok = __all_sync(0xffffffffu, ok);
-                            if (ok && lane == 0) tma_block(m + kRawDepth);
-                        }
-                        ++m;
-                    }
-                }
-            }
-            if (!ok) for (u32 i = 0; i < 400; ++i) __nanosleep(100);  // an aborted launch: let the copies in flight land before the CTA retires
-        }
-    } else if (warp >= kDrainWarps) {
-        // ================================================================================================= unpackers
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
-        const u32 lt = tid - kDrainWarps * 32;            // 0..127 = weight row of the tile
-        // The tokens' bytes (A8 codes, deltas, sums) come by ordinary loads - L2 hits - one stage AHEAD: the registers
-        // filled here are stored in the next iteration, so their latency hides behind this stage's work.
-        const u32 tok_b = lt >> 1, half = lt & 1u, tok_e = lt & 63u, ge = lt >> 6;
-        struct Tok { uint4 cc[4]; float e0, e1; i32 s0, s1; };
-        u32 tk = 0xffffffffu;
-        const i8* t_codes = nullptr;
+    if (warp >= kConsumers) {
+        // ================================================================================================= helpers
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kHelperRegs));
+        const u32 lt = tid - kConsumers * 32;            // 0..127 = weight row of the tile
+        const u32 hw = lt >> 5, tok = lt & 63u, half = lt >> 6;  // the token whose {E, S} this thread stages, and which half of the groups
+        const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, in_gs = in_stride / 32;
+        u32 ik = 0, ib = 0, cy = 0;                      // tile and super-block of the next stage to request
         const float* t_deltas = nullptr;
         const i32* t_sums = nullptr;
-        const u32 stages_per_tile = 2 * nblocks, total_stages = my_tiles * stages_per_tile;
-        auto load_tok = [&](u32 sn, Tok& r) {  // stage sn of the CTA's sequence
-            const u32 k = sn / stages_per_tile, s = sn - k * stages_per_tile, b = s >> 1, hf = s & 1u;
-            if (k != tk) {
-                tk = k;
-                const Tile t = find_tile(a, cum, n_union, blockIdx.x + k * gridDim.x);
-                // the token this thread gathers codes for (two threads per token), and the one it stages {E, S} for
-                const u32 ent_b = t.eb + min(tok_b, t.nt - 1), ent_e = t.eb + min(tok_e, t.nt - 1);
-                const u32 src_b = kDown ? a.routes.slots[ent_b] : a.routes.rows[ent_b];
-                const u32 src_e = kDown ? a.routes.slots[ent_e] : a.routes.rows[ent_e];
-                t_codes = a.in.codes + u64(src_b) * in_stride;
-                t_deltas = a.in.deltas + u64(src_e) * in_gs;
-                t_sums = a.in.sums + u64(src_e) * in_gs;
+        // Requests stage m: rows by TMA, codes and {E, S} by asynchronous copies (one commit group per thread and stage).
+        auto request = [&](u32 m) {
+            const u32 slot = m % kStages;
+            unsigned char* st = smem + slot * kStageBytes;
+            if (ok && m >= kStages) ok = mbar_wait(&empty[slot], (m / kStages - 1u) & 1u, kWaitLimit, s_abort);
+            if (ib == 0) {  // a new tile: every helper thread publishes the A8 row of its token
+                const Tile t = find_tile(a, cum, n_union, blockIdx.x + ik * gridDim.x);
+                const u32 ent = t.eb + min(tok, t.nt - 1u);
+                const u32 src = kDown ? a.routes.slots[ent] : a.routes.rows[ent];
+                if (half == 0) s_src[(ik & 1u) * 64u + tok] = src;
+                t_deltas = a.in.deltas + u64(src) * in_gs + 4u * half;
+                t_sums = a.in.sums + u64(src) * in_gs + 4u * half;
+                cy = kDown ? t.expert * H + kGM * t.c : t.expert * I + 64u * t.c;
+                asm volatile("bar.sync 1, %0;" ::"n"(kHelpers * 32) : "memory");
             }
-            const uint4* cq = reinterpret_cast<const uint4*>(t_codes + 32u * (8u * b + 4u * hf)) + 4 * half;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) r.cc[c] = __ldg(cq + c);
-            const u32 g0 = 8u * b + 4u * hf + 2u * ge;   // this thread stages pair ge of the stage for token tok_e
-            r.e0 = __ldg(t_deltas + g0); r.e1 = __ldg(t_deltas + g0 + 1);
-            r.s0 = __ldg(t_sums + g0); r.s1 = __ldg(t_sums + g0 + 1);
-        };
-        Tok tok{};
-        if (total_stages) load_tok(0, tok);
-        u32 m = 0;  // super-block counter of the sequence
-        for (; n < total_stages; ++n) {
-            const u32 buf = n & 1u, use = n >> 1, hf = n & 1u;  // a tile has an even number of stages
-            const u32 rslot = m % kRawDepth;
-            const Tok cur = tok;
-            if (n + 1 < total_stages) load_tok(n + 1, tok);
-            if (ok && hf == 0) ok = mbar_wait(&raw_full[rslot], (m / kRawDepth) & 1u, s_abort);  // the super-block's rows have landed
-            if (ok) ok = mbar_wait(&empty[buf], (use & 1u) ^ 1u, s_abort);  // the drain is done with this buffer
-            unsigned char* st = stage0 + buf * kStageBytes;
             if (ok) {
-                const uint4* wq = reinterpret_cast<const uint4*>(raw + rslot * kRawBlock + lt * kQ4KBlock);
-                const uint4 hdr = wq[0];
-                // A: row lt, chunk c = (pair pp, 16-byte half kc): low nibbles -> group 2pp, high nibbles -> group 2pp + 1
-                const u32 core = (lt >> 3) * 256u + (lt & 7u) * 16u;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const u32 pp = c >> 1, kc = c & 1;
-                    const uint4 q = wq[1 + 4 * hf + c];
-                    uint4 lo, hi;
-                    lo.x = q.x & 0x0f0f0f0fu; lo.y = q.y & 0x0f0f0f0fu; lo.z = q.z & 0x0f0f0f0fu; lo.w = q.w & 0x0f0f0f0fu;
-                    hi.x = (q.x >> 4) & 0x0f0f0f0fu; hi.y = (q.y >> 4) & 0x0f0f0f0fu; hi.z = (q.z >> 4) & 0x0f0f0f0fu; hi.w = (q.w >> 4) & 0x0f0f0f0fu;
-                    *reinterpret_cast<uint4*>(st + (2 * pp) * (kGM * 32) + core + kc * 128u) = lo;
-                    *reinterpret_cast<uint4*>(st + (2 * pp + 1) * (kGM * 32) + core + kc * 128u) = hi;
+                if (lt == 0) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the consumers' reads precede the copies below
+                    mbar_expect_tx(&raw_full[slot], kRawBytes);
+                    tma_2d(st, &tm0, ib * kQ4KBlock, cy, &raw_full[slot]);
+                    tma_2d(st + 64u * kRowPitch, kDown ? &tm0 : &tm1, ib * kQ4KBlock, kDown ? cy + 64u : cy, &raw_full[slot]);
                 }
-                // B: token tok_b, chunks 4 * half .. + 3 of the stage's 128 code bytes: chunk = (group gi, half kc)
-                unsigned char* sb = st + kABytes + (tok_b >> 3) * 256u + (tok_b & 7u) * 16u;
+                const u32* src = s_src + (ik & 1u) * 64u;
+                unsigned char* sc = st + kRawBytes;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const u32 ch = 4 * half + c, gi = ch >> 1, kc = ch & 1u;
-                    *reinterpret_cast<uint4*>(sb + gi * (kGN * 32) + kc * 128u) = cur.cc[c];
+                for (u32 i = 0; i < kGN / 8; ++i) {  // a half warp copies the 256 codes of one token
+                    const u32 tk = (kGN / 4) * hw + 2u * i + (lane >> 4);
+                    cp_async16(sc + tk * kCodePitch + 16u * (lane & 15u), a.in.codes + u64(src[tk]) * in_stride + 256u * ib + 16u * (lane & 15u));
                 }
-                reinterpret_cast<float4*>(st + kABytes + kBBytes)[ge * kGN + tok_e] =
-                    make_float4(cur.e0, cur.e1, static_cast<float>(cur.s0), static_cast<float>(cur.s1));
-                reinterpret_cast<uint4*>(st + kABytes + kBBytes + kEsBytes)[lt] = hdr;
-                // generic-proxy accesses (the stores above, the reads of the raw slot) before the async proxy's:
-                // the tensor core reading the operands, the next TMA copy overwriting the slot
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                mbar_arrive(&ready[buf]);
-                if (hf == 1) mbar_arrive(&raw_free[rslot]);
+                unsigned char* pv = st + kRawBytes + kCodeBytes + kEsBytes + kFacBytes + 32u * lt;
+#pragma unroll
+                for (u32 i = 0; i < 4; ++i) {
+                    cp_async4(pv + 4u * i, t_deltas + 8u * ib + i);
+                    cp_async4(pv + 16u + 4u * i, t_sums + 8u * ib + i);
+                }
             }
-            if (hf == 1) ++m;
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (++ib == nblocks) { ib = 0; ++ik; }
+        };
+        if (total) request(0);
+        u32 asked = total ? 1u : 0u;
+        for (u32 m = 0; m < total; ++m) {
+            if (m + 1 < total) { request(m + 1); ++asked; }
+            else asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group keeps the count of the wait below fixed
+            const u32 slot = m % kStages;
+            unsigned char* st = smem + slot * kStageBytes;
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            if (ok) ok = mbar_wait(&raw_full[slot], (m / kStages) & 1u, kWaitLimit, s_abort);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) continue;  // no more requests or hand-overs; the tile barrier above is still met by every helper
+            const uint4 hdr = *reinterpret_cast<const uint4*>(st + lt * kRowPitch);
+            const bool slow = __any_sync(0xffffffffu, (hdr.x & 0x7c00u) == 0x7c00u);
+            if (lane == 0) s_slow[slot * 4u + hw] = slow ? 1u : 0u;
+            // the row's factors, [group][D | -DM][quarter][row % 8][row / 8 % 4]: a lane's four rows are one 128-bit load;
+            // the high nibbles' dots come as 16 * dot
+            float* fac = reinterpret_cast<float*>(st + kRawBytes + kCodeBytes + kEsBytes) + (lt & ~31u) + (lt & 7u) * 4u + ((lt >> 3) & 3u);
+#pragma unroll
+            for (u32 p = 0; p < 4; ++p) {
+                const Factors f = q4k_factors(hdr, p);
+                fac[(4 * p) * kGM] = f.Dl; fac[(4 * p + 1) * kGM] = -f.DMl;
+                fac[(4 * p + 2) * kGM] = __fmul_rn(f.Dh, 0.0625f); fac[(4 * p + 3) * kGM] = -f.DMh;
+            }
+            const unsigned char* pv = st + kRawBytes + kCodeBytes + kEsBytes + kFacBytes + 32u * lt;
+            const float4 e = *reinterpret_cast<const float4*>(pv);
+            const int4 sm = *reinterpret_cast<const int4*>(pv + 16);
+            if (tok < kGN) {
+                float* es = reinterpret_cast<float*>(st + kRawBytes + kCodeBytes) + (4u * half * (kGN / 2) + (tok >> 1)) * 4u + (tok & 1u);  // [group][token pair] {E, E', S, S'}
+                es[0] = e.x; es[2] = static_cast<float>(sm.x);
+                es[2 * kGN] = e.y; es[2 * kGN + 2] = static_cast<float>(sm.y);
+                es[4 * kGN] = e.z; es[4 * kGN + 2] = static_cast<float>(sm.z);
+                es[6 * kGN] = e.w; es[6 * kGN + 2] = static_cast<float>(sm.w);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready[slot]);
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (*s_abort && lt == 0)  // wait (bounded) for the copies still in flight before the CTA retires
+            for (u32 n = asked > kStages ? asked - kStages : 0u; n < asked; ++n)
+                for (u32 i = 0; i < (kWaitLimit >> 8); ++i)
+                    if (mbar_try_wait(&raw_full[n % kStages], (n / kStages) & 1u, kWaitHintNs)) break;
     } else {
-        // ================================================================================================ drain
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
-        const u32 quarter = warp & 3u, w = warp >> 2;   // TMEM lane quarter, token half
-        const u32 o = 32u * quarter + lane;             // weight row of the tile = TMEM lane
-        const u32 lane_addr = (32u * quarter) << 16;
+        // ================================================================================================ consumers
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
+        const u32 quarter = warp & 3u, w = warp >> 2;   // 32 rows of the tile; the 8-token chunks alternate between the kSplit warps of a quarter
+        const u32 fr = lane >> 2, ft = lane & 3u;       // fragments: rows 32 quarter + 8 i + fr (i = 0 .. 3), tokens 2 ft, 2 ft + 1 of a chunk
         const u32 act_stride = a.act.stride ? a.act.stride : a.act.width;
+        const float2 one = both(a.one);
+        u32 m = 0;
         for (u32 id = blockIdx.x; id < n_tiles; id += gridDim.x) {
             const Tile t = find_tile(a, cum, n_union, id);
-            float acc[kTPT][4];
+            const u32 n_chunks = t.nt > 8u * w ? (t.nt - 8u * w + 8u * kSplit - 1u) / (8u * kSplit) : 0u;  // chunks w, w + kSplit, ...
+            float2 acc[kChunks][4][4];
 #pragma unroll
-            for (int i = 0; i < (int)kTPT; ++i) { acc[i][0] = 0.0f; acc[i][1] = 0.0f; acc[i][2] = 0.0f; acc[i][3] = 0.0f; }
-            for (u32 b = 0; b < nblocks; ++b) {
-#pragma unroll
-                for (int hf = 0; hf < 2; ++hf, ++n) {
-                    const u32 buf = n & 1u, use = n >> 1;
-                    if (ok) ok = mbar_wait(&full[buf], use & 1u, s_abort);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) continue;
-                    tc_fence_after();
-                    const unsigned char* st = stage0 + buf * kStageBytes;
-                    const float4* es = reinterpret_cast<const float4*>(st + kABytes + kBBytes);  // [pair][token] {E_l, E_h, S_l, S_h}
-                    const uint4 hdr = reinterpret_cast<const uint4*>(st + kABytes + kBBytes + kEsBytes)[o];
-                    const u32 tbase = tmem + lane_addr + buf * (kStageGroups * kGN) + 8u * w;
-#pragma unroll
-                    for (int pp = 0; pp < 2; ++pp) {
-                        const Factors f = q4k_factors(hdr, 2 * hf + pp);
-                        const float2 D = make_float2(f.Dl, f.Dh), DMn = make_float2(-f.DMl, -f.DMh);
-#pragma unroll
-                        for (int tq = 0; tq < (int)kTPT / 8; ++tq) {  // chunk 2 * tq + w of the tile: a short tile still uses every warp
-                            if (8u * (kDrainGroups * tq + w) >= t.nt) continue;  // no valid token in these 8 columns (warp-uniform)
-                            u32 dl[8], dh[8];
-                            tmem_ld8(tbase + (2 * pp) * kGN + 8 * kDrainGroups * tq, dl);
-                            tmem_ld8(tbase + (2 * pp + 1) * kGN + 8 * kDrainGroups * tq, dh);
-                            tmem_wait_ld();
-                            tie8(dl); tie8(dh);
-                            const float4* e4 = es + pp * kGN + 8u * (kDrainGroups * tq + w);
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                const float4 e = e4[i];
-                                const float2 fd = make_float2(__int2float_rn(static_cast<int>(dl[i])), __int2float_rn(static_cast<int>(dh[i])));
-                                // x = E * ((D * float(dot)) - (DM * S)) for the pair's two groups; (-DM) * S = -(DM * S) exactly
-                                const float2 pa = mul2(D, fd), pb = mul2(DMn, make_float2(e.z, e.w));
-                                const float2 x = mul2(make_float2(e.x, e.y), make_float2(__fadd_rn(pa.x, pb.x), __fadd_rn(pa.y, pb.y)));
-                                acc[8 * tq + i][2 * hf + pp] = __fadd_rn(acc[8 * tq + i][2 * hf + pp], __fadd_rn(x.x, x.y));
-                            }
-                        }
-                    }
-                    tc_fence_before();
-                    mbar_arrive(&empty[buf]);  // every drain thread arrives: the buffer (TMEM half + stage) is free
+            for (int i = 0; i < (int)kChunks * 16; ++i) (&acc[0][0][0])[i] = make_float2(0.0f, 0.0f);
+            for (u32 b = 0; b < nblocks; ++b, ++m) {
+                const u32 slot = m % kStages, parity = (m / kStages) & 1u;
+                if (ok) ok = mbar_wait(&ready[slot], parity, kWaitLimit, s_abort);
+                if (ok) ok = mbar_wait(&raw_full[slot], parity, kWaitLimit, s_abort);  // complete by now: orders the TMA's writes before our reads
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) continue;
+                const unsigned char* st = smem + slot * kStageBytes;
+                const unsigned char* rows = st + (32u * quarter + fr) * kRowPitch + 16u + 8u * ft;
+                const unsigned char* codes = st + kRawBytes + (8u * w + fr) * kCodePitch + 8u * ft;
+                const float4* es = reinterpret_cast<const float4*>(st + kRawBytes + kCodeBytes) + 4u * w + ft;
+                const float4* fac = reinterpret_cast<const float4*>(st + kRawBytes + kCodeBytes + kEsBytes) + 8u * quarter + fr;
+                if (n_chunks) {
+                    if (s_slow[slot * 4u + quarter]) superblock<true>(rows, codes, es, fac, n_chunks, one, acc);
+                    else superblock<false>(rows, codes, es, fac, n_chunks, one, acc);
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[slot]);
             }
             // (a0 + a1) + (a2 + a3)
+            auto fold = [&](const float2* c, int second) {
+                return second ? __fadd_rn(__fadd_rn(c[0].y, c[1].y), __fadd_rn(c[2].y, c[3].y)) : __fadd_rn(__fadd_rn(c[0].x, c[1].x), __fadd_rn(c[2].x, c[3].x));
+            };
             if (kDown) {
                 if (ok) {
 #pragma unroll
-                    for (int i = 0; i < (int)kTPT; ++i) {
-                        const u32 tok = 8u * (kDrainGroups * (i >> 3) + w) + (i & 7);
-                        if (tok < t.nt) {
-                            const u32 slot = a.routes.slots[t.eb + tok];
-                            a.raw[u64(slot) * H + kGM * t.c + o] = __fadd_rn(__fadd_rn(acc[i][0], acc[i][1]), __fadd_rn(acc[i][2], acc[i][3]));
+                    for (int cz = 0; cz < 2 * (int)kChunks; ++cz) {
+                        const u32 tk = 8u * (kSplit * (cz >> 1) + w) + 2u * ft + (cz & 1);
+                        if (tk < t.nt) {
+                            float* out = a.raw + u64(a.routes.slots[t.eb + tk]) * H + kGM * t.c + 32u * quarter + fr;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) out[8 * i] = fold(acc[cz >> 1][i], cz & 1);
                         }
                     }
                 }
             } else {
-                asm volatile("bar.sync 3, %0;" ::"r"(kDrainWarps * 32) : "memory");  // the previous tile's epilogue has read s_out
+                asm volatile("bar.sync 3, %0;" ::"n"(kConsumers * 32) : "memory");  // the previous tile's epilogue has read s_out
 #pragma unroll
-                for (int i = 0; i < (int)kTPT; ++i)
-                    s_out[(8u * (kDrainGroups * (i >> 3) + w) + (i & 7)) * kGM + o] = __fadd_rn(__fadd_rn(acc[i][0], acc[i][1]), __fadd_rn(acc[i][2], acc[i][3]));
-                asm volatile("bar.sync 3, %0;" ::"r"(kDrainWarps * 32) : "memory");
-                // SwiGLU + the A8 rule: one warp per (token, 32 outputs); the tile holds 2 groups of 32 per token
-                for (u32 task = warp; ok && task < 2 * t.nt; task += kDrainWarps) {
-                    const u32 tok = task >> 1, q32 = task & 1u;
-                    const float g = s_out[tok * kGM + 32u * q32 + lane], u = s_out[tok * kGM + 64u + 32u * q32 + lane];
-                    const u32 slot = a.routes.slots[t.eb + tok], group = 2u * t.c + q32, o_col = 32u * group + lane;
-                    if (a.gate_out) { a.gate_out[u64(slot) * I + o_col] = g; a.up_out[u64(slot) * I + o_col] = u; }
-                    const float h = swiglu_qwen(g, u);
-                    const bool bad = __any_sync(0xffffffffu, !finite_f(g) || !finite_f(u) || !finite_f(h));
-                    if (bad) {  // fail closed: nothing of the group is written (routed_expert.cpp:147-156)
-                        if (lane == 0) {
-                            if (a.row_status) atomicOr(&a.row_status[a.routes.rows[t.eb + tok]], B200MOE_ROW_PROJECTION_NONFINITE);
-                            if (a.summary) atomicOr(a.summary, B200MOE_ROW_PROJECTION_NONFINITE);
-                        }
-                        continue;
+                for (int cz = 0; cz < 2 * (int)kChunks; ++cz) {
+                    float* out = s_out + (8u * (kSplit * (cz >> 1) + w) + 2u * ft + (cz & 1)) * kOutPitch + 32u * quarter + fr;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) out[8 * i] = fold(acc[cz >> 1][i], cz & 1);
+                }
+                asm volatile("bar.sync 3, %0;" ::"n"(kConsumers * 32) : "memory");
+                // SwiGLU + the A8 rule: a task is (token, 32 outputs), two per token; a warp takes the four of two tokens at a time
+                for (u32 tk0 = 2u * warp; ok && tk0 < t.nt; tk0 += 2u * kConsumers) {
+                    float g[kTasks], u[kTasks], delta[kTasks];
+                    int code[kTasks], sum[kTasks];
+#pragma unroll
+                    for (int i = 0; i < kTasks; ++i) {
+                        const float* row = s_out + min(tk0 + (i >> 1), t.nt - 1u) * kOutPitch + 32u * (i & 1) + lane;
+                        g[i] = row[0]; u[i] = row[64];
                     }
-                    float delta;
-                    int sum;
-                    const int code = a8_quantize_lane(h, &delta, &sum);
-                    a.act.codes[u64(slot) * act_stride + o_col] = static_cast<i8>(code);
-                    if (lane == 0) {
-                        a.act.deltas[u64(slot) * (act_stride / 32) + group] = delta;
-                        if (a.act.sums) a.act.sums[u64(slot) * (act_stride / 32) + group] = sum;
+                    const u32 bad = swiglu_a8(g, u, code, delta, sum);
+#pragma unroll
+                    for (int i = 0; i < kTasks; ++i) {
+                        const u32 tk = tk0 + (i >> 1);
+                        if (tk >= t.nt) break;
+                        const u32 slot = a.routes.slots[t.eb + tk], group = 2u * t.c + (i & 1), o_col = 32u * group + lane;
+                        if (a.gate_out) { a.gate_out[u64(slot) * I + o_col] = g[i]; a.up_out[u64(slot) * I + o_col] = u[i]; }
+                        if (bad >> i & 1u) {  // fail closed: nothing of the group is written (routed_expert.cpp:147-156)
+                            if (lane == 0) {
+                                if (a.row_status) atomicOr(&a.row_status[a.routes.rows[t.eb + tk]], B200MOE_ROW_PROJECTION_NONFINITE);
+                                if (a.summary) atomicOr(a.summary, B200MOE_ROW_PROJECTION_NONFINITE);
+                            }
+                            continue;
+                        }
+                        a.act.codes[u64(slot) * act_stride + o_col] = static_cast<i8>(code[i]);
+                        if (lane == 0) {
+                            a.act.deltas[u64(slot) * (act_stride / 32) + group] = delta[i];
+                            if (a.act.sums) a.act.sums[u64(slot) * (act_stride / 32) + group] = sum[i];
+                        }
                     }
                 }
             }
         }
     }
     if (!ok && lane == 0 && a.summary) atomicOr(a.summary, kAbortBit);
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-    }
 }
 
-// Tensor map of a [rows][row_bytes] byte tensor with boxes of 144 bytes x 64 rows (no swizzle, no interleave). The
+// Tensor map of a [rows][row_bytes] byte tensor with boxes of kRowPitch bytes x 64 rows (no swizzle, no interleave). The
 // encoder is the driver's cuTensorMapEncodeTiled, looked up through the runtime (no link against the driver library).
 int encode_rows_map(const u8* base, u64 row_bytes, u64 rows, CUtensorMap* out) {
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -492,7 +439,7 @@ int encode_rows_map(const u8* base, u64 row_bytes, u64 rows, CUtensorMap* out) {
     if (!fn) return fail(B200MOE_ERR_CUDA, "grouped: cuTensorMapEncodeTiled is not available from this driver");
     const cuuint64_t dims[2] = {row_bytes, rows};
     const cuuint64_t strides[1] = {row_bytes};       // bytes between rows: a multiple of 16 (144 per super-block)
-    const cuuint32_t box[2] = {kQ4KBlock, 64};
+    const cuuint32_t box[2] = {kRowPitch, 64};  // 16 bytes past the super-block: the next one's, or the fill value at the end of a row
     const cuuint32_t elem[2] = {1, 1};
     const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<u8*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -518,9 +465,9 @@ bool grouped_fits(const b200moe_shape& s, bool have_sums) { return have_sums && 
 int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     GroupedArgs a{};
-    a.shape = v.shape; a.routes = v.routes; a.w0 = v.weights.gate; a.w1 = v.weights.up; a.in = v.x; a.act = v.act;
+    a.shape = v.shape; a.routes = v.routes; a.in = v.x; a.act = v.act;
     a.gate_out = v.gate_out; a.up_out = v.up_out; a.row_status = v.row_status; a.summary = v.summary;
-    a.n_row_tiles = v.shape.inter / 64; a.K = v.shape.hidden;
+    a.n_row_tiles = v.shape.inter / 64; a.K = v.shape.hidden; a.one = 1.0f;
     CUtensorMap tm0, tm1;
     const u64 rb = u64(v.shape.hidden / 256) * kQ4KBlock, rows = u64(v.shape.experts) * v.shape.inter;
     if (int rc = encode_rows_map(v.weights.gate, rb, rows, &tm0)) return rc;
@@ -533,9 +480,9 @@ int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t strea
 int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     GroupedArgs a{};
-    a.shape = v.shape; a.routes = v.routes; a.w0 = v.weights.down; a.in = v.act; a.raw = v.raw;
+    a.shape = v.shape; a.routes = v.routes; a.in = v.act; a.raw = v.raw;
     a.summary = const_cast<u32*>(v.summary);
-    a.n_row_tiles = v.shape.hidden / kGM; a.K = v.shape.inter;
+    a.n_row_tiles = v.shape.hidden / kGM; a.K = v.shape.inter; a.one = 1.0f;
     CUtensorMap tm0;
     if (int rc = encode_rows_map(v.weights.down, u64(v.shape.inter / 256) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<true>), kGroupedSmem)) return rc;

@@ -8,14 +8,15 @@
 // 128 lanes a clock. The dots of the same group take 136 clocks of the register-to-register integer MMA (measured: 8.5 clocks
 // per m16n8k32 and scheduler, 22.5 together with ten packed FP32 instructions), so the dots stay in REGISTERS. The form before
 // this one (tcgen05 with accumulators in tensor memory, operands unpacked to shared memory) spent 980 clocks per group, most of
-// them in its unpack -> MMA -> drain hand-overs: 1230 us for 512 tokens x 34,816 rows x 5120, @GU@ us now.
+// them in its unpack -> MMA -> drain hand-overs: 1230 us for 512 tokens x 34,816 rows x 5120, 957 us now.
 //
 // Tile = (expert, 128 weight rows, kGN of the expert's tokens). gate/up: rows 0..63 are gate rows [64c, 64c + 64), rows
 // 64..127 the up rows of the same outputs, so SwiGLU + the A8 rule of h finish inside the tile. down: 128 rows of H.
 // A persistent CTA per SM walks tiles round-robin; a stage of the ring (three) is one super-block: 256 columns.
 //   * helper warps (4): the tile's weight rows arrive by two tiled TMA copies (160 bytes x 64 rows: the 144 of the super-block
-//     and 16 more, which puts rows 8 (mod 32) words apart - the fragment loads below are conflict free), the tokens' codes by
-//     16-byte asynchronous copies (288 bytes apart, for the same reason), one stage ahead. A helper thread decodes the
+//     and 16 more, which puts rows 8 (mod 32) words apart - the fragment loads below are conflict free), the tokens' codes, deltas and
+//     sums by 16-byte asynchronous copies (codes 288 bytes apart, for the same reason), one stage ahead; deltas and sums that do
+//     not lie in 16-byte units come in 4-byte copies, whose eight-way bank conflicts cost 12 % of the kernel. A helper thread decodes the
 //     factors of one weight row and transposes {E, S} of one token (half the groups each).
 //   * consumer warps: warp = 32 rows x every kSplit-th 8-token chunk (a tile with few tokens still uses most warps). The
 //     nibbles go from shared memory straight into A fragments (low nibbles by a mask, high nibbles left in place as 16 q), the
@@ -34,11 +35,10 @@ namespace b200moe {
 namespace {
 using namespace q4k;
 
-#ifndef SPLIT
-#define SPLIT 2
-#define CHUNKS 4
-#endif
-constexpr u32 kSplit = SPLIT, kChunks = CHUNKS;  // consumer warps that share a tile's tokens; 8-token chunks of each
+// Three consumer warps a scheduler with two chunks each: with two warps of four chunks (tiles of 64 tokens) the FP32 pipe sits idle
+// while both wait for their shared-memory reads and MMAs (4096 x 8 tokens over 128 experts of 2048 x 768: gate/up 1437 us against
+// 1346 us; 512 tokens x 17,408 -> 5120: down 517 against 400 us, where the narrower tiles also fill the last wave).
+constexpr u32 kSplit = 3, kChunks = 2;           // consumer warps that share a tile's tokens; 8-token chunks of each
 constexpr u32 kGM = 128, kGN = 8 * kSplit * kChunks;  // tile: weight rows x tokens
 constexpr u32 kConsumers = 4 * kSplit, kHelpers = 4;  // warps
 constexpr u32 kGThreads = (kConsumers + kHelpers) * 32;
@@ -100,6 +100,7 @@ struct GroupedArgs {
     u32* summary;
     u32 n_row_tiles;         // inter / 64 (gate/up) or hidden / 128 (down)
     u32 K;                   // hidden (gate/up) or inter (down)
+    u32 es_vec;              // the input's deltas and sums lie in whole 16-byte units
     float one;               // 1.0f, unknown to the compiler (mul2 / fma2)
 };
 
@@ -282,10 +283,15 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
                     cp_async16(sc + tk * kCodePitch + 16u * (lane & 15u), a.in.codes + u64(src[tk]) * in_stride + 256u * ib + 16u * (lane & 15u));
                 }
                 unsigned char* pv = st + kRawBytes + kCodeBytes + kEsBytes + kFacBytes + 32u * lt;
+                if (a.es_vec) {
+                    cp_async16(pv, t_deltas + 8u * ib);
+                    cp_async16(pv + 16, t_sums + 8u * ib);
+                } else {
 #pragma unroll
-                for (u32 i = 0; i < 4; ++i) {
-                    cp_async4(pv + 4u * i, t_deltas + 8u * ib + i);
-                    cp_async4(pv + 16u + 4u * i, t_sums + 8u * ib + i);
+                    for (u32 i = 0; i < 4; ++i) {
+                        cp_async4(pv + 4u * i, t_deltas + 8u * ib + i);
+                        cp_async4(pv + 16u + 4u * i, t_sums + 8u * ib + i);
+                    }
                 }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
@@ -447,6 +453,11 @@ int encode_rows_map(const u8* base, u64 row_bytes, u64 rows, CUtensorMap* out) {
     return B200MOE_OK;
 }
 
+bool es_units(const b200moe_a8_rows& x) {
+    const u32 stride = x.stride ? x.stride : x.width;
+    return stride % 128 == 0 && aligned(x.deltas, 16) && aligned(x.sums, 16);
+}
+
 bool grouped_shape_ok(const b200moe_shape& s) {
     return s.gate_type == B200MOE_TYPE_Q4_K && s.down_type == B200MOE_TYPE_Q4_K && s.hidden % 256 == 0 && s.inter % 256 == 0 &&
            s.hidden % kGM == 0 && s.inter % 64 == 0 && s.experts <= kMaxUnion;
@@ -467,7 +478,7 @@ int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t strea
     GroupedArgs a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.x; a.act = v.act;
     a.gate_out = v.gate_out; a.up_out = v.up_out; a.row_status = v.row_status; a.summary = v.summary;
-    a.n_row_tiles = v.shape.inter / 64; a.K = v.shape.hidden; a.one = 1.0f;
+    a.n_row_tiles = v.shape.inter / 64; a.K = v.shape.hidden; a.one = 1.0f; a.es_vec = es_units(v.x);
     CUtensorMap tm0, tm1;
     const u64 rb = u64(v.shape.hidden / 256) * kQ4KBlock, rows = u64(v.shape.experts) * v.shape.inter;
     if (int rc = encode_rows_map(v.weights.gate, rb, rows, &tm0)) return rc;
@@ -482,7 +493,7 @@ int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     GroupedArgs a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.act; a.raw = v.raw;
     a.summary = const_cast<u32*>(v.summary);
-    a.n_row_tiles = v.shape.hidden / kGM; a.K = v.shape.inter; a.one = 1.0f;
+    a.n_row_tiles = v.shape.hidden / kGM; a.K = v.shape.inter; a.one = 1.0f; a.es_vec = es_units(v.act);
     CUtensorMap tm0;
     if (int rc = encode_rows_map(v.weights.down, u64(v.shape.inter / 256) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<true>), kGroupedSmem)) return rc;

@@ -258,9 +258,57 @@ __global__ void __launch_bounds__(256) down_q4k_kernel(b200moe_down_view v, u32 
     }
 }
 
-// Q8_0 down in the four-chain rule (routed_expert.cpp:110-144): chain c = g % 4 adds E_g * (d * float(dot)) in
-// ascending g; value = (acc0 + acc1) + (acc2 + acc3). One warp per down row, lane = group within a run of 32.
-// grid (hidden / 32, max_union); 256 threads.
+// One 32-weight block of the four-chain down tensors: the 32 weights as bytes, the factor and (Q5_1) the minimum.
+template <bool Q51>
+struct ChainBlock { u32 q[8]; float d, mn; };
+template <bool Q51>
+__device__ __forceinline__ void load_chain_block(const u8* b, ChainBlock<Q51>& o) {
+    if (Q51) {
+        // Q5_1 (routed_expert.cpp:124-133): 24-byte blocks, 8-byte aligned. Weight k < 16 = low nibble of byte k, k >= 16 = high
+        // nibble of byte k - 16, bit k of the 32 high bits on top: unsigned 0..31. Kept raw here, spread when used.
+        const uint2* b8 = reinterpret_cast<const uint2*>(b);
+        const uint2 hd = __ldg(b8), qa = __ldg(b8 + 1), qb = __ldg(b8 + 2);
+        o.q[0] = qa.x; o.q[1] = qa.y; o.q[2] = qb.x; o.q[3] = qb.y; o.q[4] = hd.x; o.q[5] = hd.y;
+    } else {  // 34-byte blocks are 2-byte aligned: whole words where the quants lie on one, else words and a byte permute
+        const bool odd = (reinterpret_cast<uintptr_t>(b) & 2u) != 0;
+        o.d = half_bits_to_float(__ldg(reinterpret_cast<const u16*>(b)));
+        if (odd) {
+            const u32* w = reinterpret_cast<const u32*>(b + 2);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o.q[i] = __ldg(w + i);
+        } else {
+            const u32* w = reinterpret_cast<const u32*>(b);
+            u32 r[9];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[i] = __ldg(w + i);
+            r[8] = __ldg(reinterpret_cast<const u16*>(b + 32));  // nothing is read past the block
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o.q[i] = __byte_perm(r[i], r[i + 1], 0x5432u);
+        }
+    }
+}
+template <bool Q51>
+__device__ __forceinline__ void spread_chain_block(ChainBlock<Q51>& o) {
+    if (!Q51) return;
+    const u32 qs[4] = {o.q[0], o.q[1], o.q[2], o.q[3]}, hd = o.q[4], hb = o.q[5];
+    o.d = half_bits_to_float(hd & 0xffffu);
+    o.mn = half_bits_to_float(hd >> 16);
+    auto spread = [](u32 x) { return ((x & 1u) | ((x & 2u) << 7) | ((x & 4u) << 14) | ((x & 8u) << 21)) << 4; };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        o.q[i] = (qs[i] & 0x0f0f0f0fu) | spread(hb >> (4 * i));
+        o.q[4 + i] = ((qs[i] >> 4) & 0x0f0f0f0fu) | spread(hb >> (16 + 4 * i));
+    }
+}
+
+// Q8_0 / Q5_1 down in the four-chain rule (routed_expert.cpp:110-144): chain c = g % 4 adds E_g * (d * float(dot)) in
+// ascending g; value = (acc0 + acc1) + (acc2 + acc3). A lane IS one chain of one row (lane = 4 * row + chain), so the chain is a
+// plain register sum and the four lanes of a row read neighbouring blocks. (The form before this one gave a row to a warp
+// with a lane per group and handed every term round by shuffles: with 20 groups a row, 12 lanes idled and a term cost eight
+// shuffles.) What bounds it: the latency of the weight loads, so a lane asks for kChainBatch blocks at once, the first batch
+// before the entries' A8 rows are staged. 4 rows over 128 experts of 640 -> 2560, top 8, Q5_1: 43.6 -> 23.1 us.
+// grid (hidden / 64, max_union); 256 threads, 8 rows a warp.
+constexpr u32 kChainBatch = 3;
 template <bool Q51>
 __global__ void __launch_bounds__(256) down_q8_chain4_kernel(b200moe_down_view v) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -273,79 +321,59 @@ __global__ void __launch_bounds__(256) down_q8_chain4_kernel(b200moe_down_view v
     i32* s_sums = reinterpret_cast<i32*>(s_deltas + kR * groups);
     __shared__ u32 s_slots[kR];
     const u32 expert = v.routes.experts[j], eb = v.routes.begins[j], ee = v.routes.begins[j + 1];
-    const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const u64 row_bytes = u64(groups) * (Q51 ? kQ51Block : kQ8Block);
-    const u32 o0 = 32u * blockIdx.x;
-    const u8* down = v.weights.down + (u64(expert) * H + o0) * row_bytes;
-    const u32 chain = lane & 3u;
+    const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, chain = lane & 3u;
+    constexpr u32 block = Q51 ? kQ51Block : kQ8Block;
+    const u32 o = 64u * blockIdx.x + 8u * warp + (lane >> 2);
+    const u8* wrow = v.weights.down + (u64(expert) * H + o) * (u64(groups) * block);
 
     for (u32 p0 = eb; p0 < ee; p0 += kR) {
         const int nr = static_cast<int>(min(u32(kR), ee - p0));
+        ChainBlock<Q51> w[kChainBatch];
+        auto load_batch = [&](u32 g0) {
+#pragma unroll
+            for (u32 i = 0; i < kChainBatch; ++i)
+                if (g0 + 4u * i < groups) load_chain_block<Q51>(wrow + u64(g0 + 4u * i) * block, w[i]);
+        };
+        load_batch(chain);
         __syncthreads();
         if (threadIdx.x < (u32)nr) s_slots[threadIdx.x] = v.routes.slots[p0 + threadIdx.x];
         __syncthreads();
         stage_a8(v.act, s_slots, nr, I, s_codes, s_deltas, s_sums);
         __syncthreads();
-        for (u32 t = warp; t < 32; t += 8) {
-            const u8* wrow = down + u64(t) * row_bytes;
-            float acc[kR];
+        float acc[kR];
 #pragma unroll
-            for (int r = 0; r < kR; ++r) acc[r] = 0.0f;
-            for (u32 g0 = 0; g0 < groups; g0 += 32) {
-                const u32 g = g0 + lane;
-                const bool valid = g < groups;
-                u32 q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                float d = 0.0f, mn = 0.0f;
-                if (valid && Q51) {
-                    // Q5_1 (routed_expert.cpp:124-133): 24-byte blocks, 8-byte aligned. Weight k < 16 = low nibble of byte
-                    // k, k >= 16 = high nibble of byte k - 16, bit k of the 32 high bits on top: unsigned 0..31.
-                    const uint2* b8 = reinterpret_cast<const uint2*>(wrow + u64(g) * kQ51Block);
-                    const uint2 hd = __ldg(b8), qa = __ldg(b8 + 1), qb = __ldg(b8 + 2);
-                    d = half_bits_to_float(hd.x & 0xffffu);
-                    mn = half_bits_to_float(hd.x >> 16);
-                    const u32 qs[4] = {qa.x, qa.y, qb.x, qb.y};
-                    auto spread = [](u32 x) { return ((x & 1u) | ((x & 2u) << 7) | ((x & 4u) << 14) | ((x & 8u) << 21)) << 4; };
+        for (int r = 0; r < kR; ++r) acc[r] = 0.0f;
+        for (u32 g0 = chain; g0 < groups; g0 += 4u * kChainBatch) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        q[i] = (qs[i] & 0x0f0f0f0fu) | spread(hd.y >> (4 * i));
-                        q[4 + i] = ((qs[i] >> 4) & 0x0f0f0f0fu) | spread(hd.y >> (16 + 4 * i));
-                    }
-                } else if (valid) {  // 34-byte blocks are only 2-byte aligned: halfword loads
-                    const u16* b16 = reinterpret_cast<const u16*>(wrow + u64(g) * kQ8Block);
-                    d = half_bits_to_float(b16[0]);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) q[i] = u32(b16[1 + 2 * i]) | (u32(b16[2 + 2 * i]) << 16);
-                }
-                const u32 ng = min(32u, groups - g0);
+            for (u32 i = 0; i < kChainBatch; ++i) {
+                const u32 g = g0 + 4u * i;
+                if (g >= groups) break;
+                ChainBlock<Q51>& b = w[i];
+                spread_chain_block<Q51>(b);
 #pragma unroll
                 for (int r = 0; r < kR; ++r) {
                     if (r < nr) {
-                        float term = 0.0f;
-                        if (valid) {
-                            const uint4* c = reinterpret_cast<const uint4*>(s_codes + u64(r) * I + 32u * g);
-                            const uint4 c0 = c[0], c1 = c[1];
-                            int dot = 0;
-                            dot = __dp4a((int)q[0], (int)c0.x, dot); dot = __dp4a((int)q[1], (int)c0.y, dot);
-                            dot = __dp4a((int)q[2], (int)c0.z, dot); dot = __dp4a((int)q[3], (int)c0.w, dot);
-                            dot = __dp4a((int)q[4], (int)c1.x, dot); dot = __dp4a((int)q[5], (int)c1.y, dot);
-                            dot = __dp4a((int)q[6], (int)c1.z, dot); dot = __dp4a((int)q[7], (int)c1.w, dot);
-                            float combined = __fmul_rn(d, static_cast<float>(dot));
-                            if (Q51) combined = __fadd_rn(combined, __fmul_rn(mn, static_cast<float>(s_sums[r * groups + g])));
-                            term = __fmul_rn(s_deltas[r * groups + g], combined);
-                        }
-#pragma unroll
-                        for (u32 k = 0; k < 8; ++k) {  // chain c takes groups c, c + 4, ... ascending
-                            const float tv = __shfl_sync(0xffffffffu, term, chain + 4u * k);
-                            if (chain + 4u * k < ng) acc[r] = __fadd_rn(acc[r], tv);
-                        }
+                        const uint4* c = reinterpret_cast<const uint4*>(s_codes + u64(r) * I + 32u * g);
+                        const uint4 c0 = c[0], c1 = c[1];
+                        int dot = 0;
+                        dot = __dp4a((int)b.q[0], (int)c0.x, dot); dot = __dp4a((int)b.q[1], (int)c0.y, dot);
+                        dot = __dp4a((int)b.q[2], (int)c0.z, dot); dot = __dp4a((int)b.q[3], (int)c0.w, dot);
+                        dot = __dp4a((int)b.q[4], (int)c1.x, dot); dot = __dp4a((int)b.q[5], (int)c1.y, dot);
+                        dot = __dp4a((int)b.q[6], (int)c1.z, dot); dot = __dp4a((int)b.q[7], (int)c1.w, dot);
+                        float combined = __fmul_rn(b.d, static_cast<float>(dot));
+                        if (Q51) combined = __fadd_rn(combined, __fmul_rn(b.mn, static_cast<float>(s_sums[r * groups + g])));
+                        acc[r] = __fadd_rn(acc[r], __fmul_rn(s_deltas[r * groups + g], combined));
                     }
                 }
             }
+            load_batch(g0 + 4u * kChainBatch);
+        }
 #pragma unroll
-            for (int r = 0; r < kR; ++r) {
-                const float a0 = __shfl_sync(0xffffffffu, acc[r], 0), a1 = __shfl_sync(0xffffffffu, acc[r], 1);
-                const float a2 = __shfl_sync(0xffffffffu, acc[r], 2), a3 = __shfl_sync(0xffffffffu, acc[r], 3);
-                if (lane == 0 && r < nr) v.raw[u64(s_slots[r]) * H + o0 + t] = __fadd_rn(__fadd_rn(a0, a1), __fadd_rn(a2, a3));
+        for (int r = 0; r < kR; ++r) {
+            if (r < nr) {  // uniform over the block
+                const float pair = __fadd_rn(acc[r], __shfl_xor_sync(0xffffffffu, acc[r], 1));
+                const float y = __fadd_rn(pair, __shfl_xor_sync(0xffffffffu, pair, 2));
+                if (chain == 0) v.raw[u64(s_slots[r]) * H + o] = y;
             }
         }
     }
@@ -410,10 +438,10 @@ int launch_down_q8_chain4(const b200moe_down_view& v, cudaStream_t stream) {
     const u32 smem = kR * (I + I / 32 * 8);
     if (v.shape.down_type == B200MOE_TYPE_Q5_1) {
         if (int rc = set_smem(down_q8_chain4_kernel<true>, smem)) return rc;
-        down_q8_chain4_kernel<true><<<dim3(H / 32, v.max_union), 256, smem, stream>>>(v);
+        down_q8_chain4_kernel<true><<<dim3(H / 64, v.max_union), 256, smem, stream>>>(v);
     } else {
         if (int rc = set_smem(down_q8_chain4_kernel<false>, smem)) return rc;
-        down_q8_chain4_kernel<false><<<dim3(H / 32, v.max_union), 256, smem, stream>>>(v);
+        down_q8_chain4_kernel<false><<<dim3(H / 64, v.max_union), 256, smem, stream>>>(v);
     }
     return after_launch("down_q8_chain4");
 }

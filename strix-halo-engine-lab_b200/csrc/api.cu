@@ -561,11 +561,7 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
 
     // The router reads FP32 rows: bfloat16 activations are widened once (exactly) into the workspace, and both the A8
     // quantiser and the router read the widened rows (the Qwen prologue's input form, src/cuda/models/qwen/qwen_moe.cu:60-99).
-    const float* x32 = static_cast<const float*>(v->x);
-    if (v->x_is_bf16) {
-        if (int rc = launch_widen_bf16(static_cast<const u16*>(v->x), F.x_f32, u64(v->rows) * s.hidden, st)) return rc;
-        x32 = F.x_f32;
-    }
+    const float* x32 = v->x_is_bf16 ? F.x_f32 : static_cast<const float*>(v->x);
     b200moe_quantize_a8_view q{};
     q.x = x32; q.rows = v->rows; q.width = s.hidden; q.x_stride = s.hidden; q.x_is_bf16 = 0; q.out = F.x;
     b200moe_router_view r{};
@@ -577,6 +573,12 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
     const LayerScratch L = carve_layer(F.layer, s, v->capacity);
     const bool one_launch = prologue_fusable(r, s.top_k);
     const bool fused = one_launch || select_routes_fusable(r, s.top_k);
+    // Where the quantiser is a launch of its own it widens on the way (one pass over the activations instead of two).
+    b200moe_quantize_a8_view qb = q;
+    qb.x = v->x; qb.x_is_bf16 = 1;
+    const bool widen_in_quantizer = v->x_is_bf16 && !one_launch && quantize_a8_vec_ok(qb);
+    if (v->x_is_bf16 && !widen_in_quantizer)
+        if (int rc = launch_widen_bf16(static_cast<const u16*>(v->x), F.x_f32, u64(v->rows) * s.hidden, st)) return rc;
     b200moe_routes_view rv{};
     if (fused) {
         u32* row_status = v->row_status ? v->row_status : L.row_status;
@@ -590,7 +592,9 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
     if (one_launch) {
         if (int rc = launch_prologue(r, q, rv, L.summary + 1, st)) return rc;
     } else {
-        if (int rc = launch_router_logits(r, st, &q)) return rc;
+        if (widen_in_quantizer)
+            if (int rc = launch_quantize_a8(qb, st, F.x_f32, s.hidden)) return rc;
+        if (int rc = launch_router_logits(r, st, widen_in_quantizer ? nullptr : &q)) return rc;
         if (fused) { if (int rc = launch_select_routes(r, rv, st)) return rc; }
         else if (int rc = launch_router_select(r, st)) return rc;
     }

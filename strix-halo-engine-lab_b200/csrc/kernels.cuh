@@ -6,7 +6,9 @@
 namespace b200moe {
 
 // a8.cu
-int launch_quantize_a8(const b200moe_quantize_a8_view& v, cudaStream_t stream);
+// wide (optional, only with bfloat16 x and quantize_a8_vec_ok): the values as FP32 rows of wide_stride, 16-byte aligned
+bool quantize_a8_vec_ok(const b200moe_quantize_a8_view& v);
+int launch_quantize_a8(const b200moe_quantize_a8_view& v, cudaStream_t stream, float* wide = nullptr, u32 wide_stride = 0);
 int launch_rmsnorm_a8(const b200moe_rmsnorm_view& v, cudaStream_t stream);
 // out[i] = float(bfloat16 bits in[i]) (exact widening)
 int launch_widen_bf16(const u16* in, float* out, u64 count, cudaStream_t stream);

@@ -7,7 +7,7 @@
 // the CLASSES are what the warps of a CTA share out: consumer warp w owns classes 2w and 2w + 1 of all 16 rows x 8 entries
 // of a tile, i.e. blocks 2w and 2w + 1 of every run of 32 blocks, and walks the runs in ascending order - eight FP32
 // accumulators per lane, each product and each add the contract's own, in its order. When the tile's last run is done the
-// 16 x 8 x 32 class sums meet in shared memory and warp w runs the butterfly of row w (lane = class), bit for bit.
+// 16 x 8 x 32 class sums meet in shared memory and warp w runs the butterfly of row w, bit for bit.
 //
 //  * Item = (virtual expert of at most 8 entries, 32 outputs); tiles of 16 weight rows: gate rows, gate rows + 16, up rows,
 //    up rows + 16 (gate/up) or the two halves of 32 down rows. A CTA takes a contiguous range of items (items of a dense
@@ -209,7 +209,7 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
             last_jv = jv;
         }
         u32 my_slot = 0;
-        if (DOWN && lane < ne) my_slot = __ldg(a.routes.slots + vbegin + lane);
+        if (DOWN && (lane >> 2) < ne) my_slot = __ldg(a.routes.slots + vbegin + (lane >> 2));
         float* gu = s_gu + (kl & 1u) * (kGuFloats / 2);
         bool stop = false;
         for (u32 tile = 0; tile < kTiles; ++tile) {
@@ -239,25 +239,33 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
                 __syncwarp();
                 if (lane == 0) mbar_arrive(x_empty);  // the next item brings other entries
             }
-            // the class sums meet: cell (row, entry) = pair, class c at word pair * 32 + (c + pair) % 32
+            // the class sums meet: cell (row, entry) = pair, class c at word pair * 32 + (c + 4 entry + row) % 32: the 32 cells of a
+            // store and the (entry, class % 4) of a load below each meet every bank once
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const u32 pair = (gid + 8u * (i >> 1)) * kKE + 2u * t4 + (i & 1u);
-                    cls[pair * 32u + ((2u * warp + c + pair) & 31u)] = acc[c][i];
+                    const u32 row = gid + 8u * (i >> 1), entry = 2u * t4 + (i & 1u);
+                    cls[(row * kKE + entry) * 32u + ((2u * warp + c + 4u * entry + row) & 31u)] = acc[c][i];
                 }
             consumers_sync();
-            float mine = 0.0f;  // warp w folds row w of the tile: lane = class; lane i keeps the product of entry i
+            // Warp w folds row w of the tile, lane = (entry, class % 4): the butterfly's steps 16, 8 and 4 stay inside a residue
+            // class mod 4, i.e. inside the lane's eight registers; only steps 2 and 1 cross lanes. (A lane per class and five
+            // shuffles an entry kept the shuffle unit as busy as the dots of a 2048-wide row: 512 rows x 4 over 64 experts of
+            // 2048 -> 1024 took 830 us a call, 671 now.)
+            const u32 fe = lane >> 2, fq = lane & 3u;
+            float v8[8];
 #pragma unroll
-            for (u32 i = 0; i < kKE; ++i) {
-                const u32 pair = warp * kKE + i;
-                const float tot = butterfly32(cls[pair * 32u + ((lane + pair) & 31u)]);
-                if (lane == i) mine = tot;
-            }
-            if (lane < ne && ok) {
+            for (u32 i = 0; i < 8; ++i) v8[i] = cls[(warp * kKE + fe) * 32u + ((fq + 4u * i + 4u * fe + warp) & 31u)];
+#pragma unroll
+            for (u32 h = 4; h; h >>= 1)
+#pragma unroll
+                for (u32 i = 0; i < h; ++i) v8[i] = __fadd_rn(v8[i], v8[i + h]);
+            float mine = __fadd_rn(v8[0], __shfl_xor_sync(0xffffffffu, v8[0], 2));
+            mine = __fadd_rn(mine, __shfl_xor_sync(0xffffffffu, mine, 1));
+            if (fq == 0 && fe < ne && ok) {
                 if (DOWN) a.raw[u64(my_slot) * a.out_width + 32u * chunk + kTileRows * tile + warp] = mine;
-                else gu[(tile >> 1) * kKE * 32u + lane * 32u + kTileRows * (tile & 1u) + warp] = mine;
+                else gu[(tile >> 1) * kKE * 32u + fe * 32u + kTileRows * (tile & 1u) + warp] = mine;
             }
             if (tid == 0) ctl[4] = *abort_flag;  // one thread publishes the decision between the two barriers: every warp reads the same
             consumers_sync();

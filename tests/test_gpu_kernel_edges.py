@@ -1,0 +1,186 @@
+"""Edges of the kernels that large windows and small staged launches take: remainders of tiles and chunks, both sides of each
+dispatch rule, layouts that fall back to narrower copies, and values that are not finite. Bit for bit, against the CPU oracle or
+a NumPy restatement of the declared order."""
+import numpy as np
+import pytest
+
+from oracle import loader as O
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import b200moe
+    b200moe.lib()
+    return torch.device("cuda:0")
+
+
+def dv(a, dev):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+
+
+def same(a, b):
+    """Equal bits, any NaN standing for any other."""
+    a, b = np.ascontiguousarray(a, np.float32), np.ascontiguousarray(b, np.float32)
+    nan = np.isnan(a) & np.isnan(b)
+    return np.array_equal(np.where(nan, 0, a.view(np.uint32)), np.where(nan, 0, b.view(np.uint32)))
+
+
+def window(rng, E, K, rows):
+    return np.stack([rng.permutation(E)[:K] for _ in range(rows)]).astype(np.uint32)
+
+
+@pytest.mark.parametrize("tokens", [1, 8, 16, 17, 24, 25, 47, 48, 49, 97])
+def test_grouped_tile_remainders(gpu, oracle, tokens):
+    """One expert holds `tokens` rows of the window (tiles of 48 tokens in chunks of 8, three warps sharing them), another the rest."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(tokens)
+    E, H, I, rows = 3, 256, 256, 160
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+    ids = np.zeros((rows, 1), np.uint32)
+    ids[rng.permutation(rows)[:tokens]] = 2
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, 12, 12, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, 1, 12, 12)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("bits", [0x7c00, 0xfc00, 0x7e00])
+def test_grouped_factor_not_finite(gpu, oracle, bits):
+    """A down row whose super-block factor is an infinity or a NaN: the term is d * dot, not what is left of (M + dot) - M."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(bits)
+    E, H, I, rows = 2, 256, 512, 130
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+    down = down.copy()
+    blocks = down.reshape(E, H, I // 256, 144)
+    for row, b in ((5, 0), (70, 1)):
+        blocks[1, row, b, 0:2] = np.array([bits], np.uint16).view(np.uint8)
+    ids = rng.integers(0, E, (rows, 1)).astype(np.uint32)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, 12, 12, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)["raw"]
+    sh = ops.make_shape(H, I, E, 1, 12, 12)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows)
+    got = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu().numpy()
+    assert not np.isfinite(want).all() and same(got, want)
+
+
+def test_grouped_rows_of_any_stride(gpu):
+    """A8 rows 544 wide: their deltas and sums lie 68 bytes apart and take the 4-byte copies."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(5)
+    E, H, I, rows = 3, 512, 256, 150
+    gate, up, _ = (dv(t, gpu) for t in synth.expert_tensors(rng, E, H, I, 12, 12))
+    x = dv(rng.standard_normal((rows, H), dtype=np.float32), gpu)
+    r = ops.enqueue_moe_routes(dv(window(rng, E, 2, rows).view(np.int32), gpu), E, E // 2)
+    sh = ops.make_shape(H, I, E, 2, 12, 12)
+    plain = ops.enqueue_quantize_a8(x)
+    wide = ops.enqueue_quantize_a8(x, stride=H + 32)
+    out = []
+    for codes, deltas, sums in (plain, wide):
+        view = (codes, deltas, sums, rows, H, codes.shape[1])
+        out.append(ops.enqueue_routed_gate_up(sh, gate, up, r, E, view, 2 * rows, taps=True))
+    (a0, g0, u0), (a1, g1, u1) = out
+    assert torch.equal(g0, g1) and torch.equal(u0, u1) and all(torch.equal(p, q) for p, q in zip(a0, a1))
+
+
+@pytest.mark.parametrize("inter", [32, 96, 160, 672])
+@pytest.mark.parametrize("down_type", [7, 8])
+def test_four_chain_down_group_counts(gpu, oracle, inter, down_type):
+    """Fewer groups than chains, odd group counts (Q8_0 rows that start between words), a remainder of a batch of blocks."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(inter + down_type)
+    E, H, rows = 3, 256, 11  # up to 11 entries of an expert: more than one pass of eight
+    gate, up, down = synth.expert_tensors(rng, E, H, inter, 12, down_type)
+    ids = window(rng, E, 2, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, inter, E, 2, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)["raw"]
+    sh = ops.make_shape(H, inter, E, 2, 12, down_type)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), 2 * rows)
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want)
+
+
+def declared_logits(x, w):
+    """Lane class l sums products l, l + 32, ... ascending; the classes fold by the butterfly (src/ds41_moe.cpp:72-82)."""
+    acc = np.zeros((x.shape[0], w.shape[0], 32), np.float32)
+    for i in range(0, x.shape[1], 32):
+        acc = acc + w[None, :, i:i + 32] * x[:, None, i:i + 32]
+    for d in (16, 8, 4, 2, 1):
+        acc = acc[..., :d] + acc[..., d:2 * d]
+    return acc[..., 0]
+
+
+# up to 4 rows: the staged form, its runs of 2048; from 5 rows: tiles of 8 x 16 in chunks of 512 or (more tiles than SMs) 256 columns
+@pytest.mark.parametrize("rows,hidden,experts", [(1, 64, 5), (2, 2048, 61), (3, 2112, 16), (4, 4160, 33), (5, 2112, 17), (9, 576, 128), (200, 320, 128), (1201, 288, 16)])
+def test_router_logits_forms(gpu, rows, hidden, experts):
+    from b200moe import ops
+    rng = np.random.default_rng(rows)
+    x = rng.standard_normal((rows, hidden), dtype=np.float32)
+    w = (rng.standard_normal((experts, hidden)) * 0.02).astype(np.float32)
+    logits, scores, _, _ = ops.enqueue_router(ops.softmax_policy(experts, 2), x=dv(x, gpu), weight=dv(w, gpu))
+    assert logits.data_ptr() != scores.data_ptr() and same(logits.cpu(), declared_logits(x, w))
+
+
+@pytest.mark.parametrize("rows,top_k,hidden,parts", [(31, 4, 192, 4), (32, 4, 192, 4), (40, 8, 516, 8), (33, 9, 256, 3), (35, 3, 258, 2)])
+def test_combine_parts_forms(gpu, rows, top_k, hidden, parts):
+    """Both sides of the wide form's rule (rows, slots, whole 16-byte units), ranges without a slot among the parts."""
+    from b200moe import ops
+    import b200moe
+    rng = np.random.default_rng(rows)
+    E = 24
+    ids = window(rng, E, top_k, rows)
+    raw = rng.standard_normal((rows * top_k, hidden), dtype=np.float32)
+    wts = rng.uniform(0.05, 0.6, (rows, top_k)).astype(np.float32)
+    shared = rng.standard_normal((rows, hidden), dtype=np.float32)
+    order = (np.argsort(ids, axis=1) + np.arange(rows)[:, None] * top_k).astype(np.int32)
+    want = shared.copy()
+    for r in range(rows):
+        for p in range(parts):
+            s = np.zeros(hidden, np.float32)
+            for slot in order[r]:
+                if min(ids.reshape(-1)[slot] // (E // parts), parts - 1) == p:
+                    s = s + wts.reshape(-1)[slot] * raw[slot]
+            want[r] = want[r] + s
+    y, yb = ops.enqueue_moe_combine(b200moe.COMBINE_PARTS, dv(raw, gpu), dv(wts, gpu), dv(ids.view(np.int32), gpu), order=dv(order, gpu), shared=dv(shared, gpu),
+                                    parts=parts, part_experts=E // parts, bf16=True)
+    assert same(y.cpu(), want) and torch.equal(yb.cpu(), torch.from_numpy(want).bfloat16())
+
+
+@pytest.mark.parametrize("rows,width,offset", [(1, 32, 0), (7, 96, 0), (5, 224, 4), (5, 224, 1), (3, 160, 2)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_quantizer_alignments(gpu, oracle, rows, width, offset, bf16):
+    """x at an offset and a row stride that do or do not leave whole loads of four values; a NaN and an infinity are flagged."""
+    from b200moe import ops
+    rng = np.random.default_rng(width + offset)
+    x = torch.from_numpy(rng.standard_normal((rows, width + 2 * offset), dtype=np.float32)).to(gpu)
+    x[:, offset] = 0.0
+    x = (x.bfloat16() if bf16 else x)[:, offset:offset + width]
+    status = torch.zeros(rows, dtype=torch.int32, device=gpu)
+    codes, deltas, sums = ops.enqueue_quantize_a8(x, status=status)
+    wc, wd, ws = oracle.quantize_a8(x.float().cpu().numpy())
+    assert np.array_equal(codes.cpu().numpy(), wc) and same(deltas.cpu(), wd) and np.array_equal(sums.cpu().numpy(), ws) and not status.any()
+    x[rows - 1, 3] = float("nan")
+    x[0, width - 1] = float("inf")
+    ops.enqueue_quantize_a8(x, status=status)
+    assert [bool(s) for s in status.cpu()] == [r in (0, rows - 1) for r in range(rows)]
+
+
+@pytest.mark.parametrize("n", [32, 480, 512, 2592])
+def test_rmsnorm_thread_counts(gpu, n):
+    """Windows of up to two rows an SM take 32 warps a row, larger ones eight: the same bits."""
+    from b200moe import ops
+    x = torch.randn((700, n), device=gpu)
+    w = torch.rand(n, device=gpu) + 0.5
+    y, a8 = ops.enqueue_rmsnorm_a8(x, w)
+    for r in (0, 350, 699):
+        y1, b8 = ops.enqueue_rmsnorm_a8(x[r:r + 1], w)
+        assert torch.equal(y[r:r + 1], y1) and all(torch.equal(p[r:r + 1], q) for p, q in zip(a8, b8))

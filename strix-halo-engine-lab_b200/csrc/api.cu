@@ -57,15 +57,22 @@ int device_sm_count() {
 }
 
 int ensure_dynamic_smem(const void* kernel, u32 bytes) {
-    // The 48 KiB a launch gets without opting in cover static AND dynamic shared memory: kernels here declare up to a few
-    // KiB statically, so the opt-in starts below the limit.
-    if (bytes <= 40u * 1024u) return B200MOE_OK;
+    // The 48 KiB a launch gets without opting in cover static AND dynamic shared memory, so a kernel's own static arrays decide
+    // from which size on it has to opt in.
     static std::mutex m;
     static std::map<std::pair<int, const void*>, u32> granted;
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lock(m);
-    u32& have = granted[{dev, kernel}];
+    auto it = granted.find({dev, kernel});
+    if (it == granted.end()) {
+        cudaFuncAttributes a{};
+        const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+        if (e != cudaSuccess) return fail(B200MOE_ERR_CUDA, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
+        const u32 fixed = static_cast<u32>(a.sharedSizeBytes), plain = 48u * 1024u;
+        it = granted.emplace(std::make_pair(dev, kernel), fixed < plain ? plain - fixed : 0u).first;
+    }
+    u32& have = it->second;
     if (bytes <= have) return B200MOE_OK;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e != cudaSuccess) return fail(B200MOE_ERR_CUDA, "cudaFuncSetAttribute(dynamic smem %u): %s", bytes, cudaGetErrorString(e));

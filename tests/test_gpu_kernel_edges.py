@@ -1,6 +1,10 @@
 """Edges of the kernels that large windows and small staged launches take: remainders of tiles and chunks, both sides of each
 dispatch rule, layouts that fall back to narrower copies, and values that are not finite. Bit for bit, against the CPU oracle or
 a NumPy restatement of the declared order."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -202,3 +206,30 @@ def test_rmsnorm_thread_counts(gpu, n):
     for r in (0, 350, 699):
         y1, b8 = ops.enqueue_rmsnorm_a8(x[r:r + 1], w)
         assert torch.equal(y[r:r + 1], y1) and all(torch.equal(p[r:r + 1], q) for p, q in zip(a8, b8))
+
+
+SELECTION_WINDOWS = """
+import numpy as np, torch, b200moe
+from b200moe import ops, synth
+from oracle import loader as O
+H, I, K, rows, E = 256, 256, 2, {rows}, {experts}
+rng = np.random.default_rng(rows)
+gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+rw, x = synth.router_weight(rng, E, H), synth.activations(rng, rows, H)
+ffn = ops.MoeFfn(ops.make_shape(H, I, E, K, 12, 12), ops.softmax_policy(E, K), *(torch.from_numpy(a).cuda() for a in (gate, up, down, rw)), capacity=rows,
+                 combine_form=b200moe.COMBINE_FMA_SLOTS)
+y, ids, _ = ffn(torch.from_numpy(x).cuda(), want_routes=True)
+want = O.Oracle().ffn(O.Shape(H, I, E, K, 12, 12, float("inf")), O.softmax_policy(E, K), gate, up, down, rw, x, O.COMBINE_FMA_SLOTS)
+assert np.array_equal(ids.cpu().numpy().view(np.uint32), want["ids"])
+assert np.array_equal(y.cpu().numpy().view(np.uint32), want["y"].view(np.uint32))
+"""
+
+
+@pytest.mark.parametrize("rows,experts", [(30, 128), (31, 128), (32, 128), (25, 160)])
+def test_selection_scratch_beside_static_shared_memory(gpu, rows, experts):
+    """Selection and routes in one launch: the scratch (33.8 to 36 KiB) and the routes' static arrays together pass the 48 KiB that a
+    launch gets without opting in. A process of its own: an opt-in lasts as long as the process."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    path = os.pathsep.join([root, os.path.join(root, "strix-halo-engine-lab_b200")])
+    r = subprocess.run([sys.executable, "-c", SELECTION_WINDOWS.format(rows=rows, experts=experts)], capture_output=True, text=True, env=dict(os.environ, PYTHONPATH=path))
+    assert r.returncode == 0, r.stderr[-2000:]

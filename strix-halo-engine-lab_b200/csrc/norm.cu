@@ -4,12 +4,17 @@
 // s = 1 / sqrt(sum / n + eps) - IEEE division and square root. The second pass is warp-per-group: y = (x * s) * w for
 // 32 consecutive values, written out and / or quantised by the A8 rule on the spot. HBM traffic: x once (the second
 // pass hits L1 / L2), y and the A8 rows once.
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace b200moe {
 namespace {
 
-__global__ void __launch_bounds__(1024) rmsnorm_a8_kernel(b200moe_rmsnorm_view v) {
+// WARPS: warps of the CTA, 0 = as launched (8 to 32). A fixed number unrolls the second pass at 48 registers, five CTAs of 8 warps an
+// SM; as launched it takes 29, eight CTAs.
+template <u32 WARPS>
+__global__ void __launch_bounds__(WARPS ? WARPS * 32u : 1024u) rmsnorm_a8_kernel(b200moe_rmsnorm_view v) {
     __shared__ float partial[256];
     const u32 r = blockIdx.x, t = threadIdx.x, n = v.n;
     const u32 x_stride = v.x_stride ? v.x_stride : n, out_stride = v.out_stride ? v.out_stride : n;
@@ -37,7 +42,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_a8_kernel(b200moe_rmsnorm_view v
     const u32 lane = t & 31u, warp = t >> 5, groups = n / 32;
     const u32 a8_stride = v.a8.stride ? v.a8.stride : v.a8.width;
     bool bad = false;
-    for (u32 g = warp; g < groups; g += blockDim.x >> 5) {
+    for (u32 g = warp; g < groups; g += WARPS ? WARPS : blockDim.x >> 5) {
         const u32 i = 32u * g + lane;
         float y = __fmul_rn(x[i], s);
         if (v.weight) y = __fmul_rn(y, v.weight[i]);
@@ -57,13 +62,22 @@ __global__ void __launch_bounds__(1024) rmsnorm_a8_kernel(b200moe_rmsnorm_view v
     if (v.status && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&v.status[r], B200MOE_ROW_NONFINITE_ACTIVATION);
 }
 
+constexpr u32 kWideRow = 2048;
+
 }  // namespace
 
 int launch_rmsnorm_a8(const b200moe_rmsnorm_view& v, cudaStream_t stream) {
     if (v.rows == 0 || v.n == 0) return B200MOE_OK;
-    // A window that leaves SMs idle takes 32 warps a row for the second pass (the first has 256 lanes by contract): 9.2 against 13.4 us
-    // for 4 rows of 2560. From two rows an SM on, eight warps a row keep more rows in flight.
-    rmsnorm_a8_kernel<<<v.rows, v.rows <= 2u * static_cast<u32>(device_sm_count()) ? 1024 : 256, 0, stream>>>(v);
+    // Up to two rows an SM a row takes a warp per group in the second pass, up to 32 (the first pass has 256 lanes by contract): 5.8 us
+    // with 32 warps against 8.6 with eight for 1 row of 2560, 24.8 against 31.1 for 296 of 7168. Warps without a group only
+    // cost: 1 row of 256 takes 2.97 us with 32 warps, 2.73 with eight, 296 rows 3.48 and 3.02. Above two rows an SM eight warps keep
+    // more rows in flight, in the unrolled form while all rows fit on the SMs at once (740 rows of 7168: 38.6 us against 40.4
+    // as launched; 1024 rows 50.3 as launched against 64.1 with five to six CTAs an SM) and are long enough for it to matter
+    // (592 rows of 2048: 11.6 against 11.8; of 1024: 7.5 both).
+    const u32 sms = static_cast<u32>(device_sm_count());
+    const u32 warps = v.rows <= 2u * sms ? std::min(32u, (v.n / 32u + 7u) / 8u * 8u) : 8u;
+    if (v.rows > 2u * sms && v.rows <= 5u * sms && v.n >= kWideRow) rmsnorm_a8_kernel<8><<<v.rows, 256, 0, stream>>>(v);
+    else rmsnorm_a8_kernel<0><<<v.rows, 32u * warps, 0, stream>>>(v);
     return after_launch("rmsnorm_a8");
 }
 

@@ -208,6 +208,22 @@ def test_rmsnorm_thread_counts(gpu, n):
         assert torch.equal(y[r:r + 1], y1) and all(torch.equal(p[r:r + 1], q) for p, q in zip(a8, b8))
 
 
+@pytest.mark.parametrize("n", [32, 256, 288, 1024, 2016, 2048, 2592])
+@pytest.mark.parametrize("per_sm", [1, 2, 5])
+def test_rmsnorm_forms_at_their_lines(gpu, oracle, n, per_sm):
+    """Both sides of each line of the rule: a warp per group up to 32, eight warps, eight warps unrolled (2 to 5 rows an SM, 2048 wide)."""
+    from b200moe import ops
+    rng = np.random.default_rng(n)
+    w = (1.0 + 0.1 * rng.standard_normal(n)).astype(np.float32)
+    line = per_sm * torch.cuda.get_device_properties(gpu).multi_processor_count
+    for rows in (line, line + 1):
+        x = (rng.standard_normal((rows, n)) * 3.0).astype(np.float32)
+        want = oracle.rmsnorm(x, w, 1e-6)
+        wc, wd, ws = oracle.quantize_a8(want)
+        y, (codes, deltas, sums) = ops.enqueue_rmsnorm_a8(dv(x, gpu), dv(w, gpu), 1e-6)
+        assert same(y.cpu(), want) and np.array_equal(codes.cpu().numpy(), wc) and same(deltas.cpu(), wd) and np.array_equal(sums.cpu().numpy(), ws)
+
+
 SELECTION_WINDOWS = """
 import numpy as np, torch, b200moe
 from b200moe import ops, synth

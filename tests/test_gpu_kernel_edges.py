@@ -224,6 +224,26 @@ def test_rmsnorm_forms_at_their_lines(gpu, oracle, n, per_sm):
         assert same(y.cpu(), want) and np.array_equal(codes.cpu().numpy(), wc) and same(deltas.cpu(), wd) and np.array_equal(sums.cpu().numpy(), ws)
 
 
+@pytest.mark.parametrize("rows,width,offset", [(37, 1024, 0), (38, 1024, 0), (38, 1024, 4), (38, 1024, 1), (38, 1024, 2), (401, 96, 0)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_quantizer_sizes(gpu, oracle, rows, width, offset, bf16):
+    """More groups than one block of the one-value form an SM holds (8 x 148 = 1184): four values a lane where x allows whole loads,
+    the last warp partly spare; a NaN and an infinity are flagged."""
+    from b200moe import ops
+    rng = np.random.default_rng(rows + offset)
+    x = torch.from_numpy(rng.standard_normal((rows, width + 2 * offset), dtype=np.float32)).to(gpu)
+    x[:, offset] = 0.0
+    x = (x.bfloat16() if bf16 else x)[:, offset:offset + width]
+    status = torch.zeros(rows, dtype=torch.int32, device=gpu)
+    codes, deltas, sums = ops.enqueue_quantize_a8(x, status=status)
+    wc, wd, ws = oracle.quantize_a8(x.float().cpu().numpy())
+    assert np.array_equal(codes.cpu().numpy(), wc) and same(deltas.cpu(), wd) and np.array_equal(sums.cpu().numpy(), ws) and not status.any()
+    x[rows - 1, 3] = float("nan")
+    x[0, width - 1] = float("inf")
+    ops.enqueue_quantize_a8(x, status=status)
+    assert [bool(s) for s in status.cpu()] == [r in (0, rows - 1) for r in range(rows)]
+
+
 SELECTION_WINDOWS = """
 import numpy as np, torch, b200moe
 from b200moe import ops, synth

@@ -19,13 +19,16 @@ constexpr u32 kChunk = routes_detail::kChunk;
 
 using routes_detail::block_exclusive_scan;
 using routes_detail::entry_id;
+using routes_detail::kRankedTopK;
 using routes_detail::row_order;
 using routes_detail::routes_small_body;
 
-__global__ void __launch_bounds__(1024) routes_small_kernel(b200moe_routes_view v, u32 end) { routes_small_body(v, end); }
+template <bool RANKED>
+__global__ void __launch_bounds__(1024) routes_small_kernel(b200moe_routes_view v, u32 end) { routes_small_body<RANKED>(v, end); }
 
 // Decode windows: the router's selection (one warp per row) and the routes of the selected ids in ONE block, so the
 // layer prologue costs one launch less. Dynamic shared memory: rows * (2 * experts + 32) floats.
+template <bool RANKED>
 __global__ void __launch_bounds__(1024) select_routes_small_kernel(const float* logits, float* scores_out, const float* __restrict__ bias,
                                                                    b200moe_route_policy p, u32 rows, u32* ids, float* __restrict__ weights,
                                                                    b200moe_routes_view rv, u32 end) {
@@ -33,11 +36,12 @@ __global__ void __launch_bounds__(1024) select_routes_small_kernel(const float* 
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (warp < rows) select_detail::select_row(logits, scores_out, bias, p, warp, lane, sel_smem + warp * (2u * p.experts + 32u), ids, weights);
     __syncthreads();  // the ids written above are read below by the whole block
-    routes_small_body(rv, end);
+    routes_small_body<RANKED>(rv, end);
 }
 
 // ---- chunked form --------------------------------------------------------------------------------------------------
 // scratch: hist[chunks][experts], then ebegin[experts].
+template <bool RANKED>
 __global__ void __launch_bounds__(1024) routes_count_kernel(b200moe_routes_view v, u32 end, u32 chunks) {
     __shared__ u32 cnt[1024];
     const u32 t = threadIdx.x, n = v.rows * v.top_k, s = blockIdx.x * kChunk + t;
@@ -47,7 +51,7 @@ __global__ void __launch_bounds__(1024) routes_count_kernel(b200moe_routes_view 
     __syncthreads();
     if (t < v.experts) v.scratch[u64(blockIdx.x) * v.experts + t] = cnt[t];
     for (u32 r = blockIdx.x * blockDim.x + t; r < v.rows; r += gridDim.x * blockDim.x)
-        row_order(v.ids, r, v.top_k, v.experts, v.split, v.out.order, v.out.low_counts, v.row_status);
+        row_order<RANKED>(v.ids, r, v.top_k, v.experts, v.split, v.out.order, v.out.low_counts, v.row_status);
 }
 __global__ void __launch_bounds__(1024) routes_scan_kernel(b200moe_routes_view v, u32 chunks) {
     __shared__ u32 warp_tot[32], total_s, union_s, maxc;
@@ -117,8 +121,9 @@ bool select_routes_fusable(const b200moe_router_view& r, u32 top_k) {
 int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view& v, cudaStream_t stream) {
     if (r.rows == 0) return B200MOE_OK;
     const u32 smem = r.rows * (2u * r.policy.experts + 32u) * 4u;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(select_routes_small_kernel), smem)) return rc;
-    select_routes_small_kernel<<<1, 1024, smem, stream>>>(r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights, v, v.end ? v.end : v.experts);
+    const auto kernel = v.top_k <= kRankedTopK ? select_routes_small_kernel<true> : select_routes_small_kernel<false>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
+    kernel<<<1, 1024, smem, stream>>>(r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights, v, v.end ? v.end : v.experts);
     return after_launch("select_routes_small");
 }
 
@@ -132,11 +137,11 @@ int launch_routes(const b200moe_routes_view& v, cudaStream_t stream) {
     if (n == 0) return B200MOE_OK;
     const u32 end = v.end ? v.end : v.experts;
     if (n <= kChunk) {
-        routes_small_kernel<<<1, 1024, 0, stream>>>(v, end);
+        (v.top_k <= kRankedTopK ? routes_small_kernel<true> : routes_small_kernel<false>)<<<1, 1024, 0, stream>>>(v, end);
         return after_launch("routes_small");
     }
     const u32 chunks = static_cast<u32>((n + kChunk - 1) / kChunk);
-    routes_count_kernel<<<chunks, 1024, 0, stream>>>(v, end, chunks);
+    (v.top_k <= kRankedTopK ? routes_count_kernel<true> : routes_count_kernel<false>)<<<chunks, 1024, 0, stream>>>(v, end, chunks);
     if (int rc = after_launch("routes_count")) return rc;
     routes_scan_kernel<<<1, 1024, 0, stream>>>(v, chunks);
     if (int rc = after_launch("routes_scan")) return rc;

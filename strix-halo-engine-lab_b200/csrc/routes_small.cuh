@@ -8,6 +8,7 @@ namespace b200moe {
 namespace routes_detail {
 
 constexpr u32 kChunk = 1024;
+constexpr u32 kRankedTopK = 8;  // row_order: up to so many slots of a row are ranked in registers
 
 // Exclusive scan of one value per thread over the block (blockDim a multiple of 32, at most 1024); `total` gets the
 // sum. warp_tot: 32 words of shared memory.
@@ -31,21 +32,23 @@ __device__ __forceinline__ u32 block_exclusive_scan(u32 v, u32* warp_tot, u32* t
     return r;
 }
 
-// Per row: the slots sorted by expert id (stable), the low count and the route check. One thread, in the middle of a decode step's
-// chain of launches: up to eight slots are ranked in registers, all ids requested at once; more go through the insertion
-// sort, whose arrays live in local memory (37 rows x 8: 140.0 -> 137.7 us a call, 64 rows of the large layer: 983 -> 946).
+// Per row: the slots sorted by expert id (stable), the low count and the route check. One thread a row, in the middle of a call's chain
+// of launches. RANKED (top_k <= kRankedTopK): the slots are ranked in registers, all ids requested at once; more go through the
+// insertion sort, whose arrays live in local memory. The routes of 64 rows x 8 over 256 experts take 9.5 us ranked, 11.7 sorted, those
+// of 1024 x 8 over 128 24.2 and 30.2. Kernels hold one of the two: both behind a test in one kernel cost 100 rows x 10 0.3 us of 21.2.
+template <bool RANKED>
 __device__ inline void row_order(const u32* ids, u32 row, u32 top_k, u32 experts, u32 split, u32* order, u32* low_counts, u32* row_status) {
-    if (top_k <= 8u) {
-        u32 id[8], low = 0;
+    if (RANKED) {
+        u32 id[kRankedTopK], low = 0;
         bool bad = false;
 #pragma unroll
-        for (u32 k = 0; k < 8; ++k) id[k] = k < top_k ? ids[row * top_k + k] : 0xffffffffu;
+        for (u32 k = 0; k < kRankedTopK; ++k) id[k] = k < top_k ? ids[row * top_k + k] : 0xffffffffu;
 #pragma unroll
-        for (u32 k = 0; k < 8; ++k)
+        for (u32 k = 0; k < kRankedTopK; ++k)
             if (k < top_k) {
                 u32 rank = 0;
 #pragma unroll
-                for (u32 j = 0; j < 8; ++j)
+                for (u32 j = 0; j < kRankedTopK; ++j)
                     if (j != k && j < top_k) {
                         rank += (id[j] < id[k] || (id[j] == id[k] && j < k)) ? 1u : 0u;
                         bad |= id[j] == id[k];
@@ -149,6 +152,7 @@ __device__ inline void routes_tiny_body(const b200moe_routes_view& v, u32 end) {
 }
 
 // The whole build by one block. Each thread owns a contiguous run of experts for the scans.
+template <bool RANKED>
 __device__ inline void routes_small_body(const b200moe_routes_view& v, u32 end) {
     __shared__ u32 cnt[1024], ebegin[1024], sid[1024], warp_tot[32], total_s, union_s, maxc;
     const u32 t = threadIdx.x, nt = blockDim.x, n = v.rows * v.top_k;
@@ -161,7 +165,7 @@ __device__ inline void routes_small_body(const b200moe_routes_view& v, u32 end) 
         if (e != 0xffffffffu) atomicAdd(&cnt[e], 1u);
         sid[s] = e;
     }
-    for (u32 r = t; r < v.rows; r += nt) row_order(v.ids, r, v.top_k, v.experts, v.split, v.out.order, v.out.low_counts, v.row_status);
+    for (u32 r = t; r < v.rows; r += nt) row_order<RANKED>(v.ids, r, v.top_k, v.experts, v.split, v.out.order, v.out.low_counts, v.row_status);
     __syncthreads();
     const u32 per = (v.experts + nt - 1) / nt, e0 = t * per, e1 = min(e0 + per, v.experts);
     u32 c_sum = 0, c_nz = 0, c_max = 0;

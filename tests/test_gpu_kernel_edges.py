@@ -244,6 +244,24 @@ def test_quantizer_sizes(gpu, oracle, rows, width, offset, bf16):
     assert [bool(s) for s in status.cpu()] == [r in (0, rows - 1) for r in range(rows)]
 
 
+@pytest.mark.parametrize("rows,top_k", [(40, 7), (33, 8), (29, 9), (200, 8), (200, 9), (26, 10)])
+def test_routes_row_order_forms(gpu, rows, top_k):
+    """More than 256 slots (one block, then chunks of 1024): a row's slots ranked in registers up to 8, sorted above. A repeated and
+    an out-of-range id are flagged and keep a place in their row's order."""
+    import b200moe
+    from b200moe import ops
+    rng = np.random.default_rng(rows + top_k)
+    E = 24
+    ids = window(rng, E, top_k, rows)
+    ids[3, 1], ids[5, 2] = ids[3, 4], E + 7
+    status = torch.zeros(rows, dtype=torch.int32, device=gpu)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2, row_status=status)
+    want = np.argsort(ids, axis=1, kind="stable") + np.arange(rows)[:, None] * top_k
+    assert np.array_equal(r.order.cpu().numpy().reshape(rows, top_k), want)
+    assert np.array_equal(r.low_counts.cpu().numpy(), (ids < E // 2).sum(axis=1))
+    assert [int(s) for s in status.cpu()] == [b200moe.ROW_INVALID_ROUTE if i in (3, 5) else 0 for i in range(rows)]
+
+
 SELECTION_WINDOWS = """
 import numpy as np, torch, b200moe
 from b200moe import ops, synth

@@ -13,7 +13,10 @@
 //  * Each consumer warp owns whole octets (octet n goes to warp n mod W): lane = (row of the octet, pair p). A lane walks
 //    its row's super-blocks in ascending order, so the serial chain acc_p += pair_p needs no shuffle at all; the final
 //    (a0 + a1) + (a2 + a3) is two xor-shuffles. Integer -> float conversions use the exact 2^23 magic-number form.
-//  * gate/up: the last warp to finish an item's eight octets (a shared-memory counter) runs SwiGLU + the A8 rule.
+//  * gate/up: the last warp to finish an item's eight octets (a shared-memory counter) runs SwiGLU + the A8 rule. The items' results
+//    lie in a ring of item slots. The stages do not bound how far the warps drift apart - a producer waits for its own octets
+//    only, so the octets of three producers go on while a warp of the fourth is busy - hence a warp waits until the slot's previous
+//    item has been written out before it stores into it.
 //
 // Every wait on an mbarrier is bounded: after kWaitLimit polls the waiter raises an abort flag, all roles stop waiting
 // (they still walk their loops, doing no work), the producers drain the copies they have in flight (bounded), bit 30 of the
@@ -394,7 +397,8 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) gate_up_q4k_
     u64* bars = reinterpret_cast<u64*>(at);
     at += 2 * plan.stages * 8;
     u32* s_done = reinterpret_cast<u32*>(at);                         // [item_slots] octets finished
-    at += plan.item_slots * 4;
+    volatile u32* s_next = s_done + plan.item_slots;                  // [item_slots] the item that may use the slot, once one has
+    at += plan.item_slots * 8;
     u32* s_flag = reinterpret_cast<u32*>(at);
     at += 16;
     at = smem + ((at - smem + 15) & ~size_t(15));
@@ -446,6 +450,7 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) gate_up_q4k_
         float* s_g = s_gu + u64(islot) * 2 * ME * 32;
         float* s_u = s_g + ME * 32;
         if (ok) ok = stage_wait(ring, slot, cur.q, cur.phase);
+        if (ok && local_item >= plan.item_slots) ok = flag_wait(&s_next[islot], local_item, ring.abort_flag);  // the slot's previous item is written out
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) { m = nm; if (has_next) load_first(v.routes.rows, m, first); continue; }
         const unsigned char* wrow = ring.data + u64(slot) * plan.stage_bytes + rsub * plan.row_stride;
@@ -507,6 +512,11 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) gate_up_q4k_
                 v.act.deltas[u64(slot_id) * (act_stride / 32) + gx] = delta;
                 if (v.act.sums) v.act.sums[u64(slot_id) * (act_stride / 32) + gx] = sum;
             }
+        }
+        __syncwarp();
+        if (lane == 0) {  // every lane has read the slot: the next item may have it
+            __threadfence_block();
+            s_next[islot] = local_item + plan.item_slots;
         }
     }
     if (!ok && lane == 0 && v.summary) atomicOr(v.summary, kAbortBit);
@@ -649,10 +659,10 @@ u32 padded_stride(u32 row_bytes) { return ((row_bytes / 16) & 1u) ? row_bytes : 
 u32 pow2_at_least(u32 v) { u32 p = 1; while (p < v) p <<= 1; return p; }
 
 u32 plan_smem(const StreamPlan& p, u32 fixed_bytes, u32 per_item_slot_bytes) {
-    return p.stages * p.stage_bytes + p.item_slots * per_item_slot_bytes + fixed_bytes + 2 * p.stages * 8 + p.item_slots * 4 + 64;
+    return p.stages * p.stage_bytes + p.item_slots * per_item_slot_bytes + fixed_bytes + 2 * p.stages * 8 + p.item_slots * 8 + 64;
 }
-// Ring depth, consumer warps and item slots for a row length. Items in flight inside a CTA never exceed
-// (stages + warps) / 8 + 2, so item_slots covers that with room. False when fewer than 4 stages fit.
+// Ring depth, consumer warps and item slots for a row length. Warps that keep pace have at most (stages + warps) / 8 + 2 items in
+// flight, so with item_slots above that only a warp far ahead of another waits for a slot. False when fewer than 4 stages fit.
 bool make_plan(u32 row_bytes, u32 fixed_bytes, u32 per_item_slot_bytes, StreamPlan* p) {
     p->row_bytes = row_bytes;
     p->row_stride = padded_stride(row_bytes);

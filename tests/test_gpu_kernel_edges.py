@@ -262,6 +262,31 @@ def test_routes_row_order_forms(gpu, rows, top_k):
     assert [int(s) for s in status.cpu()] == [b200moe.ROW_INVALID_ROUTE if i in (3, 5) else 0 for i in range(rows)]
 
 
+@pytest.mark.parametrize("rows,top_k,experts,hidden,inter,pad,form", [(58, 4, 40, 256, 1216, 32, 0), (64, 2, 16, 512, 1024, 0, 1), (2, 32, 64, 256, 1536, 0, 0),
+                                                                     (9, 8, 32, 1024, 512, 32, 0)])
+def test_row_streaming_warps_far_apart(gpu, oracle, rows, top_k, experts, hidden, inter, pad, form):
+    """More items a CTA than item slots, and one expert with an entry for every row, whose items take far longer than the others."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows)
+    gate, up, down = synth.expert_tensors(rng, experts, hidden, inter, 12, 8)
+    ids = np.stack([np.concatenate([[0], 1 + rng.permutation(experts - 1)[:top_k - 1]]) for _ in range(rows)]).astype(np.uint32)
+    x = rng.standard_normal((rows, hidden), dtype=np.float32)
+    codes, deltas, sums = oracle.quantize_a8(x)
+    want = oracle.experts(O.Shape(hidden, inter, experts, top_k, 12, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(hidden, inter, experts, top_k, 12, 8)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), experts, experts // 2)
+    a8 = ops.enqueue_quantize_a8(dv(x, gpu), stride=hidden + pad)
+    w = dv(gate, gpu), dv(up, gpu)
+    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, form)
+    try:
+        for _ in range(20):
+            _, g, u = ops.enqueue_routed_gate_up(sh, *w, r, experts, a8 + (rows, hidden, hidden + pad), rows * top_k, taps=True)
+            assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    finally:
+        b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, 0)
+
+
 SELECTION_WINDOWS = """
 import numpy as np, torch, b200moe
 from b200moe import ops, synth

@@ -262,6 +262,69 @@ def test_routes_row_order_forms(gpu, rows, top_k):
     assert [int(s) for s in status.cpu()] == [b200moe.ROW_INVALID_ROUTE if i in (3, 5) else 0 for i in range(rows)]
 
 
+@pytest.mark.parametrize("hidden,inter,rows", [(2304, 1024, 300), (4352, 1024, 301), (6656, 1024, 311), (6912, 1024, 313), (1024, 2304, 297), (1024, 4352, 295)])
+def test_q8_items_of_16_over_several_stages(gpu, oracle, hidden, inter, rows):
+    """Rows of more than one stage of two runs (the last stage one run, whole or a part of one), the last item not full; at 6912 the
+    projection's A8 rows leave no room for 16 entries and it takes 8."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(hidden + inter)
+    gate, up, down = synth.expert_tensors(rng, 1, hidden, inter, 8, 8)
+    ids = np.zeros((rows, 1), np.uint32)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, hidden), dtype=np.float32))
+    want = oracle.experts(O.Shape(hidden, inter, 1, 1, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(hidden, inter, 1, 1, 8, 8)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), 1, 1)
+    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, 1, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, 1, act).cpu(), want["raw"])
+
+
+# rows that start between 16-byte units (x at an odd element) or have no whole number of them (hidden % 4): the register forms
+@pytest.mark.parametrize("rows,hidden,experts,offset", [(1, 2048, 61, 1), (2, 1100, 33, 1), (4, 96, 16, 2), (3, 1101, 17, 0), (9, 1024, 20, 1), (17, 1102, 35, 0), (64, 2112, 128, 1)])
+def test_router_logits_unaligned(gpu, rows, hidden, experts, offset):
+    from b200moe import ops
+    rng = np.random.default_rng(rows + offset)
+    x = rng.standard_normal((rows, hidden + offset), dtype=np.float32)
+    w = (rng.standard_normal((experts, hidden)) * 0.02).astype(np.float32)
+    pad = -hidden % 32
+    want = declared_logits(np.pad(x[:, offset:], ((0, 0), (0, pad))), np.pad(w, ((0, 0), (0, pad))))  # a product with +0 leaves a sum as it is
+    logits, _, _, _ = ops.enqueue_router(ops.softmax_policy(experts, 2), x=dv(x, gpu)[:, offset:], weight=dv(w, gpu))
+    assert same(logits.cpu(), want)
+
+
+@pytest.mark.parametrize("rows", [31, 32, 45])
+@pytest.mark.parametrize("shared", [False, True])
+def test_combine_two_parts_by_low_counts(gpu, rows, shared):
+    """The split given as a count of low slots a row (no ids), rows that fail and stay as they are, both sides of the wide form's rule."""
+    import ctypes as C
+    import b200moe
+    from b200moe import CombineView, check, lib, ptr, stream_ptr
+    rng = np.random.default_rng(rows)
+    top_k, hidden = 6, 260
+    raw = rng.standard_normal((rows * top_k, hidden), dtype=np.float32)
+    wts = rng.uniform(0.05, 0.6, (rows, top_k)).astype(np.float32)
+    sh = rng.standard_normal((rows, hidden), dtype=np.float32)
+    order = (np.stack([rng.permutation(top_k) for _ in range(rows)]) + np.arange(rows)[:, None] * top_k).astype(np.int32)
+    low = rng.integers(1, top_k, rows).astype(np.int32)
+    low[:3] = (0, top_k, 1)
+    status = (np.arange(rows) % 7 == 5).astype(np.int32)
+    want = np.full((rows, hidden), 3.0, np.float32)
+    for r in np.flatnonzero(status == 0):
+        y = sh[r].copy() if shared else np.zeros(hidden, np.float32)
+        for slots in (order[r, :low[r]], order[r, low[r]:]):
+            s = np.zeros(hidden, np.float32)
+            for slot in slots:
+                s = s + wts.reshape(-1)[slot] * raw[slot]
+            y = y + s
+        want[r] = y
+    t = {k: dv(v, gpu) for k, v in {"raw": raw, "wts": wts, "sh": sh, "order": order, "low": low, "status": status}.items()}
+    y = torch.full((rows, hidden), 3.0, device=gpu)
+    v = CombineView(ptr(t["raw"]), ptr(t["sh"]) if shared else None, ptr(t["wts"]), None, ptr(t["order"]), rows, top_k, hidden, b200moe.COMBINE_PARTS, 2, 0, -1,
+                    ptr(y), None, ptr(t["status"]), None, 0, None, 0, 0, ptr(t["low"]))
+    check(lib().b200moe_combine(C.byref(v), stream_ptr()))
+    assert same(y.cpu(), want)
+
+
 @pytest.mark.parametrize("rows,top_k,experts,hidden,inter,pad,form", [(58, 4, 40, 256, 1216, 32, 0), (64, 2, 16, 512, 1024, 0, 1), (2, 32, 64, 256, 1536, 0, 0),
                                                                      (9, 8, 32, 1024, 512, 32, 0)])
 def test_row_streaming_warps_far_apart(gpu, oracle, rows, top_k, experts, hidden, inter, pad, form):

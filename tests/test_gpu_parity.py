@@ -539,7 +539,7 @@ def test_experts_other_formats_q5_k_q5_1(gpu, oracle):
 
 
 def test_experts_q4k_grouped_tensor_core_form(gpu, oracle):
-    """Windows of 128 rows and more take the grouped form (tcgen05 integer MMAs + the same FP32 chains): stage by stage
+    """Windows of 128 rows and more take the grouped form (register-to-register integer MMAs + the same FP32 chains): stage by stage
     against the oracle like the decode forms. Cases: several token tiles per expert with a ragged last one, experts with
     few tokens, an expert range (first / end), K = 256 (two stages per tile) and a wide K."""
     import b200moe

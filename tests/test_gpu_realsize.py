@@ -41,7 +41,7 @@ def assert_exact(got, want, evaluations, what):
 
 def test_config3_prefill_real_geometry(gpu, oracle):
     """Config 3: 128 experts, top-8, 2048 x 768 Q4_K, Zipf(1.1) logit bias, bfloat16 activations, 2048 tokens through
-    b200moe_ffn (bf16 in): tiled router logits, chunked routes, grouped tcgen05 experts, slot-order merge."""
+    b200moe_ffn (bf16 in): tiled router logits, chunked routes, grouped experts, slot-order merge."""
     import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(303)
@@ -66,7 +66,7 @@ def test_config3_prefill_real_geometry(gpu, oracle):
 def test_config4_rank_share_real_geometry(gpu, oracle):
     """Config 4, one expert-parallel rank's share: hidden 7168, inter 2048, the 32 Q4_K experts of rank 3 out of 256,
     sigmoid + bias router with group-limited top-8 (8 groups, best 4) over all 256 experts; a 64-row decode window
-    (segment-streaming GEMVs at 4032-byte rows) and a 512-row window (grouped tcgen05 kernel at K = 7168); the rank's
+    (segment-streaming GEMVs at 4032-byte rows) and a 512-row window (grouped kernel at K = 7168); the rank's
     partial sum S_3 of every row; and the Q8_0 shared expert at 7168 x 2048. The oracle gets the rank's 32 experts with
     the ids renumbered (owned ids -> 0..31, all others outside the owned range)."""
     import b200moe

@@ -33,12 +33,13 @@ __device__ __forceinline__ u32 block_exclusive_scan(u32 v, u32* warp_tot, u32* t
 }
 
 // Per row: the slots sorted by expert id (stable), the low count and the route check. One thread a row, in the middle of a call's chain
-// of launches. RANKED (top_k <= kRankedTopK): the slots are ranked in registers, all ids requested at once; more go through the
-// insertion sort, whose arrays live in local memory. The routes of 64 rows x 8 over 256 experts take 9.5 us ranked, 11.7 sorted, those
-// of 1024 x 8 over 128 24.2 and 30.2. Kernels hold one of the two: both behind a test in one kernel cost 100 rows x 10 0.3 us of 21.2.
+// of launches. Up to kRankedTopK slots are ranked in registers, all ids requested at once; more go through the insertion sort, whose
+// arrays live in local memory. The routes of 64 rows x 8 over 256 experts take 9.5 us ranked, 11.7 sorted, those of 1024 x 8 over 128
+// 24.4 and 30.2. RANKED: any top_k, by a test; a kernel for more slots holds the sort alone (100 rows x 10: 21.4 us, 21.7 with the
+// test), while ranking alone gained nothing (32 rows x 8: 9.4 us, 9.2 with the test).
 template <bool RANKED>
 __device__ inline void row_order(const u32* ids, u32 row, u32 top_k, u32 experts, u32 split, u32* order, u32* low_counts, u32* row_status) {
-    if (RANKED) {
+    if (RANKED && top_k <= kRankedTopK) {
         u32 id[kRankedTopK], low = 0;
         bool bad = false;
 #pragma unroll

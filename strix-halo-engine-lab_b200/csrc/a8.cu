@@ -1,4 +1,4 @@
-// A8 activation quantiser: one warp per (row, 32-value group), one value per lane.
+// A8 activation quantiser: one warp per (row, 32-value group) and one value per lane, or eight lanes per group and four values each.
 // Contract: src/cpu/core/reference.cpp:35-55 (= src/ds41_formats.cpp:146-165).
 // HBM traffic per row: width * 4 B in (2 B for bfloat16), width * 1.25 B out: negligible beside the expert weights.
 #include <algorithm>
@@ -34,9 +34,10 @@ __global__ void __launch_bounds__(256) quantize_a8_kernel(const void* __restrict
     }
 }
 
-// The same rule with four values a lane and eight lanes a group: wide loads, three shuffles a reduction instead of five, an
-// eighth of the warps. Bound by HBM (the one-value form was bound by issue: 305 us for 8192 x 7168 FP32 after 119 us of widening, 218 us here with it). With `wide`
-// the bfloat16 values are also written out as FP32 for the router, instead of by a pass of their own before this one.
+// The same rule with four values a lane and eight lanes a group: wide loads, three shuffles a reduction instead of five, a
+// quarter of the warps. Bound by issue slots (72 % busy at 8192 x 7168 FP32) and the pipe that the divisions' reciprocals take (62 %):
+// 108 us there, 0.44 of the measured copy bandwidth; 1024 rows 15.6 us, 38.9 in the one-value form. With `wide` the bfloat16 values
+// are also written out as FP32 for the router, instead of by a pass of their own before this one (8192 x 7168: 119 + 305 -> 218 us).
 template <bool BF16>
 __global__ void __launch_bounds__(256) quantize_a8_vec_kernel(const void* __restrict__ x, u32 items, u32 groups, u32 x_stride, i8* __restrict__ codes,
                                                               float* __restrict__ deltas, i32* __restrict__ sums, u32 stride, u32* __restrict__ status,

@@ -231,7 +231,12 @@ cudaError_t clear_status(const LayerScratch& L, bool with_row_status, u32 rows, 
 
 // Plan by window size, chosen on the host from the row count (no environment reads inside numerical code): decode
 // windows of Q4_K experts take the persistent bulk-copy form, everything else the plain per-block form.
-// grouped_min_rows: 0 = the default threshold; windows of at least that many rows take the tensor-core form.
+// grouped_min_rows: 0 = the default threshold; windows of at least that many rows take the grouped form.
+// What decides is the number of entries an expert has (the grouped form's tiles hold 48, a streaming item 8), and rows only stand
+// for it: whole calls, streaming against grouped, cross between 160 and 192 rows with 8 of 128 experts of 2048 x 768 (221 and 263 us at 128
+// rows, 264 and 276 at 160, 296 and 281 at 192), between 96 and 128 rows with 6 of 60 experts of 4096 x 1536 (367 and 414, 454 and 442), above
+// 384 with 2 of 160 experts of 1024 x 512 (134 and 152), and already between 24 and 32 rows in a dense block of 5120 x 17408
+// (177 and 218, 246 and 222; 784 and 423 at 128). 128 lies in the middle of these.
 constexpr u32 kGroupedDefaultRows = 128;
 bool use_grouped(const b200moe_shape& s, u32 rows, u32 grouped_min_rows, bool have_sums) {
     const u32 least = grouped_min_rows ? grouped_min_rows : kGroupedDefaultRows;
@@ -566,8 +571,8 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
     if (!device_ready()) return B200MOE_ERR_CUDA;
     cudaStream_t st = as_stream(stream);
 
-    // The router reads FP32 rows: bfloat16 activations are widened once (exactly) into the workspace, and both the A8
-    // quantiser and the router read the widened rows (the Qwen prologue's input form, src/cuda/models/qwen/qwen_moe.cu:60-99).
+    // The router reads FP32 rows: bfloat16 activations are widened once (exactly) into the workspace (the Qwen prologue's input
+    // form, src/cuda/models/qwen/qwen_moe.cu:60-99), by the A8 quantiser where it is a launch of its own, else by a launch before.
     const float* x32 = v->x_is_bf16 ? F.x_f32 : static_cast<const float*>(v->x);
     b200moe_quantize_a8_view q{};
     q.x = x32; q.rows = v->rows; q.width = s.hidden; q.x_stride = s.hidden; q.x_is_bf16 = 0; q.out = F.x;

@@ -163,8 +163,10 @@ int launch_merge_first_error(b200moe_first_error* record, const u32* summary, u3
 }
 int launch_combine(const b200moe_combine_view& v, cudaStream_t stream) {
     if (v.rows == 0) return B200MOE_OK;
-    // Only the PARTS form, whose slot -> value chain is what the early requests hide, and from 32 rows on: the slot-order form is
-    // faster with more, lighter threads (4096 rows x 8 x 2048: 77 against 94 us), and so are a few rows (1 row: 4.4 against 4.8).
+    // Only the PARTS form, whose slot -> value chain is what the early requests hide: the slot-order form is faster with more, lighter
+    // threads (4096 rows x 8 x 2048: 77 against 94 us). 32 rows is not a crossover: at 32 x 8 x 2048, 8 parts, the forms take 4.97 and
+    // 4.24 us (x 7168: 9.5 and 6.5), at 31 4.95 and 4.23, and one row 4.5 and 4.0 (a whole call 37.2 and 35.5); fewer rows keep
+    // the first form because they have only been timed so far.
     if (v.form == B200MOE_COMBINE_PARTS && v.rows >= 32 && v.y && !v.y_blocks && v.only_part < 0 && v.top_k <= kVecTopK && v.hidden % 4 == 0 && aligned(v.raw, 16) && aligned(v.y, 16) && aligned(v.shared, 16) &&
         aligned(v.y_bf16, 8)) {
         if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_vec_kernel))) return rc;

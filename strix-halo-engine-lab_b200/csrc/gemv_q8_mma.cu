@@ -4,10 +4,10 @@
 //
 // The contract adds the terms float(dot_g) * (scale_g * delta_g) of a row into 32 lane classes (group g -> class g % 32) in
 // ascending g, then folds the classes with the butterfly v[l] += v[l ^ d], d = 16 .. 1. A class is an independent chain, so
-// the CLASSES are what the warps of a CTA share out: consumer warp w owns classes 2w and 2w + 1 of all 16 rows x 8 entries
+// the CLASSES are what the warps of a CTA share out: consumer warp w owns classes 2w and 2w + 1 of all 16 rows x 8 (or 16) entries
 // of a tile, i.e. blocks 2w and 2w + 1 of every run of 32 blocks, and walks the runs in ascending order - eight FP32
-// accumulators per lane, each product and each add the contract's own, in its order. When the tile's last run is done the
-// 16 x 8 x 32 class sums meet in shared memory and warp w runs the butterfly of row w, bit for bit.
+// accumulators per lane and 8 entries, each product and each add the contract's own, in its order. When the tile's last run is
+// done the 16 x 8 (16) x 32 class sums meet in shared memory and warp w runs the butterfly of row w, bit for bit.
 //
 //  * Item = (virtual expert of at most 8 - or, where experts have them, 16 - entries, 32 outputs); tiles of 16 weight rows: gate rows, gate rows + 16, up rows,
 //    up rows + 16 (gate/up) or the two halves of 32 down rows. A CTA takes a contiguous range of items (items of a dense
@@ -337,8 +337,10 @@ bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, bool down, MmaPlan
     p->wait_limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT) ? debug_value(B200MOE_DEBUG_WAIT_LIMIT) : kDefaultWaitLimit;
     return true;
 }
-// 16 entries an item where the experts have them on average and the items still go round the SMs twice; the A8 rows of 16 entries
-// fit up to a width of about 6000. 512 rows x 4 over 64 experts of 2048 x 1024: 671 us a call with 8, 582 with 16.
+// 16 entries an item where the experts have them on average and the items still go round the SMs twice; the A8 rows of 16 entries fit
+// up to a width of 6656 (gate/up) or 6912 (down). Whole calls over 64 experts of 2048 -> 1024, 8 against 16 entries: 387 and
+// 350 us with 16 an expert, 671 and 568 with 32. The crossover is lower, at 9 an expert: 186 and 242 us with 4, 243 and 249 with
+// 8, 283 and 258 with 10; 64 experts of 4096 -> 1536 475 and 525 with 8, 635 and 584 with 12. One expert (dense, 1024 -> 1024) gains from 33 rows on.
 bool take_16(u32 K, u32 n_chunks, u32 max_union, u64 slots, bool down, MmaPlan* p) {
     return slots >= 16ull * max_union && slots / 16u * n_chunks >= 2u * static_cast<u32>(device_sm_count()) && make_plan<2>(K, n_chunks, max_union, slots, down, p);
 }

@@ -3,7 +3,9 @@
 // gemv_q4k.cu / gemv_q4k_stream.cu (contract: src/cpu/core/routed_expert.hpp:9-15, row rule routed_expert.cpp:73-108; the
 // reference's own tensor-core form is project_kernel / down_kernel, src/cuda/core/moe_a8.cuh:76-206, :225-341).
 //
-// What bounds it: the FP32 pipe and the shared-memory reads that feed it. The contract scales every 32-wide group's EXACT
+// What bounds it: latency - no unit is full (512 tokens x 34,816 rows x 5120: issue slots 53 %, FP32 pipe 51, shared-memory wavefronts
+// 54, integer MMA 18; warps wait on fixed latencies and loads for 1.9 and 1.3 issues per issue, three to four of them a scheduler),
+// and about half the instructions are factor and code loads, masks and duplicates, a factor serving two chunks. The contract scales every 32-wide group's EXACT
 // integer dot by its own factors: five FP32 operations per (row, token, group), i.e. 320 clocks per group of a 128 x 64 tile at
 // 128 lanes a clock. The dots of the same group take 136 clocks of the register-to-register integer MMA (measured: 8.5 clocks
 // per m16n8k32 and scheduler, 22.5 together with ten packed FP32 instructions), so the dots stay in REGISTERS. The form before
@@ -56,7 +58,7 @@ static_assert(kGroupedSmem > 114u * 1024u && kGroupedSmem <= 227u * 1024u, "one 
 constexpr u32 kWaitLimit = 1u << 20;         // polls of up to a microsecond
 constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23 = the float with the bits 0x4b400000
 // Register split between whole warp groups, out of what the launch gives every thread (65,536 over the threads, by eights).
-constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kHelperRegs = kSplit == 2 ? 56 : 80;
+constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kHelperRegs = 80;
 constexpr u32 kConsumerRegs = (kGThreads * kLaunchRegs - kHelpers * 32u * kHelperRegs) / (kConsumers * 32u) / 8u * 8u;
 static_assert(kConsumers * 32 * kConsumerRegs + kHelpers * 32 * kHelperRegs <= kGThreads * kLaunchRegs, "setmaxnreg split exceeds the launch's registers");
 

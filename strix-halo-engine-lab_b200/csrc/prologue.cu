@@ -129,9 +129,8 @@ __global__ void __launch_bounds__(kWarps * 32) prologue_decode_kernel(PrologueAr
     for (u32 row = warp; row < rows; row += kWarps)
         select_detail::select_row(rv.logits, rv.scores, rv.bias, rv.policy, row, lane, xs + warp * (2u * E + 32u), rv.ids, rv.weights);
     __syncthreads();  // the ids written above are read below by the whole block
-    // At most 8 rows x 32 slots: the form for up to 256 slots, without the code and the shared arrays of the larger one
-    // (one row of 128 experts, top 8: 39.8 -> 39.0 us a call). Optional: a
-    // caller that routes elsewhere passes no outputs.
+    // At most 8 rows x 32 slots: the form for up to 256 slots, without the code, the stack and 12 KiB of shared arrays of the larger
+    // one (no difference in the time of a call beyond noise). Optional: a caller that routes elsewhere passes no outputs.
     if (a.routes.out.experts) routes_detail::routes_tiny_body(a.routes, a.routes_end);
 }
 

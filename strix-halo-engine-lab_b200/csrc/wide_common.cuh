@@ -21,7 +21,7 @@ constexpr u32 kEndItem = 0xffffffffu;
 constexpr u32 kSmemBudget = 227u * 1024u;
 constexpr u32 kDefaultWaitLimit = 1u << 22;
 
-struct VExpert {  // one word: expert index (10 bits, experts <= 1024), first entry in the routes (14 bits, slots <= 8192), entries (4 bits)
+struct VExpert {  // one word: expert index (10 bits, experts <= 1024), first entry in the routes (14 bits, slots <= 8192), entries (8 bits)
     u32 bits;
     __host__ __device__ static VExpert make(u32 expert, u32 begin, u32 ne) { return VExpert{expert | (begin << 10) | (ne << 24)}; }
     __host__ __device__ u32 expert() const { return bits & 0x3ffu; }
@@ -60,6 +60,7 @@ __device__ __forceinline__ void retire_claims(u32* claim, u32* ctl) {
 template <u32 KE = kKE>
 __device__ __forceinline__ void build_work_list(const b200moe_routes& routes, u32 n_union, u32 max_union, u32 vmax, u32 n_chunks, u32* scratch,
                                                 VExpert* table, u32* ctl) {
+    static_assert(KE >= 1 && KE <= 255, "a virtual expert holds its entry count in 8 bits");
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     u32* t_beg = scratch;
     u32* t_exp = t_beg + max_union + 1;

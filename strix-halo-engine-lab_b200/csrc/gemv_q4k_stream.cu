@@ -397,14 +397,15 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) gate_up_q4k_
     u64* bars = reinterpret_cast<u64*>(at);
     at += 2 * plan.stages * 8;
     u32* s_done = reinterpret_cast<u32*>(at);                         // [item_slots] octets finished
-    volatile u32* s_next = s_done + plan.item_slots;                  // [item_slots] the item that may use the slot, once one has
+    volatile u32* s_next = s_done + plan.item_slots;                  // [item_slots] the item that may use the slot, 0 until one has
     at += plan.item_slots * 8;
     u32* s_flag = reinterpret_cast<u32*>(at);
     at += 16;
     at = smem + ((at - smem + 15) & ~size_t(15));
     unsigned char* x_copy = at;
     const Ring ring{smem, bars, reinterpret_cast<volatile u32*>(bars + plan.stages), reinterpret_cast<volatile u32*>(bars + plan.stages) + plan.stages, s_flag};
-    for (u32 i = threadIdx.x; i < plan.item_slots; i += blockDim.x) s_done[i] = 0;
+    // s_next too: shared memory holds what the launch before left there, and a launch of the same plan leaves the very item numbers waited for.
+    for (u32 i = threadIdx.x; i < 2 * plan.item_slots; i += blockDim.x) s_done[i] = 0;
     ring_init(ring, plan.stages);
 
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;

@@ -350,6 +350,27 @@ def test_row_streaming_warps_far_apart(gpu, oracle, rows, top_k, experts, hidden
         b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, 0)
 
 
+@pytest.mark.parametrize("rows,top_k,experts,hidden,inter,pad", [(58, 4, 40, 256, 1216, 32), (9, 8, 32, 1024, 512, 32)])
+def test_row_streaming_after_a_short_launch(gpu, oracle, rows, top_k, experts, hidden, inter, pad):
+    """A launch of the same plan with an item or two a CTA, then one whose CTAs go round their item slots more than once."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows)
+    gate, up, down = synth.expert_tensors(rng, experts, hidden, inter, 12, 8)
+    ids = np.stack([np.concatenate([[0], 1 + rng.permutation(experts - 1)[:top_k - 1]]) for _ in range(rows)]).astype(np.uint32)
+    x = rng.standard_normal((rows, hidden), dtype=np.float32)
+    codes, deltas, sums = oracle.quantize_a8(x)
+    want = oracle.experts(O.Shape(hidden, inter, experts, top_k, 12, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(hidden, inter, experts, top_k, 12, 8)
+    few = np.tile(np.arange(top_k, dtype=np.int32), (rows, 1))
+    r, short = (ops.enqueue_moe_routes(dv(i, gpu), experts, experts // 2) for i in (ids.view(np.int32), few))
+    a8 = ops.enqueue_quantize_a8(dv(x, gpu), stride=hidden + pad) + (rows, hidden, hidden + pad)
+    w = dv(gate, gpu), dv(up, gpu)
+    for _ in range(20):
+        ops.enqueue_routed_gate_up(sh, *w, short, experts, a8, rows * top_k)
+        _, g, u = ops.enqueue_routed_gate_up(sh, *w, r, experts, a8, rows * top_k, taps=True)
+        assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+
+
 SELECTION_WINDOWS = """
 import numpy as np, torch, b200moe
 from b200moe import ops, synth

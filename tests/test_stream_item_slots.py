@@ -2,21 +2,23 @@
 machines under random interleavings with warps of very different speed: octet q goes to producer q mod 4 and consumer warp
 q mod W, a producer waits only for the octet that had its stage before, the warp that finishes an item's eighth octet writes the
 item out, and a warp stores into an item's slot only once the slot's previous item is written out. No slot may ever hold two
-items at once, and every item is written out."""
+items at once, and every item is written out. The words that tell whose turn a slot is start at zero, whatever an earlier launch left."""
+import os
 import random
+import re
 
 import pytest
 
 PRODUCERS, OCTETS = 4, 8
 
 
-def run(stages, warps, slots, items, rng, guarded, slow):
-    """Returns whether a store ever met another item's unwritten results, and the number of items written out."""
+def run(stages, warps, slots, items, rng, guarded, slow, words=None):
+    """Returns whether a store ever met another item's unwritten results, and the number of items written out. words: s_next at the start."""
     octets = items * OCTETS
     armed, released = set(), set()
     prod = list(range(PRODUCERS))
     cons = [{"q": w, "state": "wait"} for w in range(warps)]
-    holder, done, nxt = [None] * slots, [0] * slots, [None] * slots
+    holder, done, nxt = [None] * slots, [0] * slots, list(words or [0] * slots)
     clash, written, idle = False, 0, 0
     while written < items and not clash:
         i = rng.randrange(PRODUCERS + warps)
@@ -73,3 +75,13 @@ def test_the_stages_alone_do_not_keep_items_apart():
     rng = random.Random(3)
     assert any(run(40, 16, 16, 60, rng, False, 0)[0] for _ in range(3))
     assert any(run(31, 16, 8, 60, rng, False, 0)[0] for _ in range(3))
+
+
+def test_words_of_an_earlier_launch():
+    """Shared memory outlives a launch: one of a single lap leaves in s_next the numbers that the next launch's second lap waits for."""
+    left = [s + 16 for s in range(16)]
+    rng = random.Random(3)
+    assert any(run(40, 16, 16, 60, rng, True, 0, left)[0] for _ in range(3))
+    src = open(os.path.join(os.path.dirname(__file__), "..", "strix-halo-engine-lab_b200", "csrc", "gemv_q4k_stream.cu")).read()
+    assert re.search(r"s_next = s_done \+ plan\.item_slots;", src)
+    assert re.search(r"i < 2 \* plan\.item_slots; i \+= blockDim\.x\) s_done\[i\] = 0;\s+ring_init", src), "s_done and s_next start at zero, before the block's barrier"

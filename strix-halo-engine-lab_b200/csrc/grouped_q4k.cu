@@ -3,31 +3,33 @@
 // gemv_q4k.cu / gemv_q4k_stream.cu (contract: src/cpu/core/routed_expert.hpp:9-15, row rule routed_expert.cpp:73-108; the
 // reference's own tensor-core form is project_kernel / down_kernel, src/cuda/core/moe_a8.cuh:76-206, :225-341).
 //
-// What bounds it: latency - no unit is full (512 tokens x 34,816 rows x 5120: issue slots 53 %, FP32 pipe 51, shared-memory wavefronts
-// 54, integer MMA 18; warps wait on fixed latencies and loads for 1.9 and 1.3 issues per issue, three to four of them a scheduler),
-// and about half the instructions are factor and code loads, masks and duplicates, a factor serving two chunks. The contract scales every 32-wide group's EXACT
-// integer dot by its own factors: five FP32 operations per (row, token, group), i.e. 320 clocks per group of a 128 x 64 tile at
-// 128 lanes a clock. The dots of the same group take 136 clocks of the register-to-register integer MMA (measured: 8.5 clocks
-// per m16n8k32 and scheduler, 22.5 together with ten packed FP32 instructions), so the dots stay in REGISTERS. The form before
-// this one (tcgen05 with accumulators in tensor memory, operands unpacked to shared memory) spent 980 clocks per group, most of
-// them in its unpack -> MMA -> drain hand-overs: 1230 us for 512 tokens x 34,816 rows x 5120, 957 us now.
+// What bounds it: register reads. The contract scales every 32-wide group's EXACT integer dot by its own factors: five FP32 operations
+// per (row, token, group), ten packed instructions per MMA of 16 tokens x 8 rows x 32. On a loop of its own, in clocks of a scheduler per
+// such MMA: the ten alone 20 to 22 (a packed product or sum reads two register pairs and takes two clocks, an fma of three distinct
+// pairs takes three), with the MMA 28 (its ten operand and result registers go through the same ports; its time ADDS), 30 with the
+// conversion of the dots and the sums written as fma, 31 with a barrier per 32 MMAs. The kernel spends 36 to 40: a tenth of that is
+// SwiGLU + the A8 rule, three to five hundredths the meeting of the chains.
+// 512 tokens x 34,816 rows x 5120: 785 us (941 in the form before, a warp all four chains of 32 rows x 16 tokens, whose row factors met 16
+// tokens and cost half the instructions); 4096 x 8 tokens, skewed, over 128 experts of 2048 -> 2 x 768: 1170 us (1328).
+// The dots out of tensor memory (tcgen05.mma kind::i8) leave the ports free (24 clocks a unit on a loop of its own), but what that form
+// adds - nibbles unpacked to shared memory, MMA and commit latencies between two barriers, more code than a scheduler's instruction
+// cache holds - cost more: 1180 to 1480 us, in 16 consumer warps of one chain or 8 of two.
 //
-// Tile = (expert, 128 weight rows, kGN of the expert's tokens). gate/up: rows 0..63 are gate rows [64c, 64c + 64), rows
-// 64..127 the up rows of the same outputs, so SwiGLU + the A8 rule of h finish inside the tile. down: 128 rows of H.
-// A persistent CTA per SM walks tiles round-robin; a stage of the ring (three) is one super-block: 256 columns.
-//   * helper warps (4): the tile's weight rows arrive by two tiled TMA copies (160 bytes x 64 rows: the 144 of the super-block
-//     and 16 more, which puts rows 8 (mod 32) words apart - the fragment loads below are conflict free), the tokens' codes, deltas and
-//     sums by 16-byte asynchronous copies (codes 288 bytes apart, for the same reason), one stage ahead; deltas and sums that do
-//     not lie in 16-byte units come in 4-byte copies, whose eight-way bank conflicts cost 12 % of the kernel. A helper thread decodes the
-//     factors of one weight row and transposes {E, S} of one token (half the groups each).
-//   * consumer warps: warp = 32 rows x every kSplit-th 8-token chunk (a tile with few tokens still uses most warps). The
-//     nibbles go from shared memory straight into A fragments (low nibbles by a mask, high nibbles left in place as 16 q), the
-//     codes into B fragments; the MMA starts at the integer 0x4b400000, so its result read as a float is M + dot with
-//     M = 1.5 * 2^23, and fma(D, M + dot, -D * M) is D * dot rounded once (D = d * scale has at most 17 significant bits, so
-//     D * M is exact): no conversion. Packed FP32 instructions work on two tokens at a time; the four chains acc_p of a lane's
-//     cells stay in registers; (a0 + a1) + (a2 + a3) at the end - exactly the decode kernels' order.
-//     A super-block with a non-finite d takes the same steps with the dot converted first (inf - inf would turn an infinity
-//     into a NaN).
+// Tile = (expert, 192 weight rows, kGN of the expert's tokens). gate/up: rows 0..95 are gate rows [96c, 96c + 96), rows 96..191 the up
+// rows of the same outputs, so SwiGLU + the A8 rule of h finish inside the tile. down: 192 rows of H. The last row tile of an expert
+// ends with it and may repeat rows of the tile before (the same bits twice): a read past an expert's rows could leave the tensor, which may
+// hold fewer experts than the shape counts.
+// A persistent CTA per SM walks tiles round-robin; a stage of the ring (three) is one super-block: 256 columns, 4 pairs of groups (chains).
+//   * helper warps (4): the tile's weight rows arrive by two tiled TMA copies (144 bytes x 96 rows: consecutive rows lie 4 (mod 32) words
+//     apart, the fragment loads below are conflict free), the tokens' codes, deltas and sums by 16-byte asynchronous copies (codes 272
+//     bytes apart, for the same reason), one stage ahead. A thread of the first three warps decodes the factors of two weight rows, a lane
+//     of the fourth lays out the {E, S} of one token.
+//   * consumer warps (12): warp = 64 rows x all tokens of ONE of the four chains. The nibbles go from shared memory straight into B
+//     fragments (low nibbles by a mask, high nibbles left in place as 16 q), the codes into A fragments; a lane's two neighbouring cells
+//     are two weight rows of one token, so the rows' factors are natural register pairs and the packed instructions take a token's
+//     factors as one register for both halves. A row's factors are read once per 32 tokens, a token's once per 64 rows.
+//     The four chains of a row third meet through shared memory at the end of a tile, (a0 + a1) + (a2 + a3); gate/up then runs
+//     SwiGLU + the A8 rule, a warp four (token, 32 outputs) tasks at a time.
 // Every wait is bounded; on a timeout the roles stop working and the launch sets B200MOE_JOB_WAIT_ABORTED in the job summary.
 #include <cuda.h>
 
@@ -37,26 +39,34 @@ namespace b200moe {
 namespace {
 using namespace q4k;
 
-// Three consumer warps a scheduler with two chunks each: with two warps of four chunks (tiles of 64 tokens) the FP32 pipe sits idle
-// while both wait for their shared-memory reads and MMAs (4096 x 8 tokens over 128 experts of 2048 x 768: gate/up 1437 us against
-// 1346 us; 512 tokens x 17,408 -> 5120: down 517 against 400 us, where the narrower tiles also fill the last wave).
-constexpr u32 kSplit = 3, kChunks = 2;           // consumer warps that share a tile's tokens; 8-token chunks of each
-constexpr u32 kGM = 128, kGN = 8 * kSplit * kChunks;  // tile: weight rows x tokens
-constexpr u32 kConsumers = 4 * kSplit, kHelpers = 4;  // warps
+constexpr u32 kTokTiles = 2;                     // 16-token MMA tiles of a CTA tile
+constexpr u32 kRowTiles = 8;                     // 8-row MMA tiles of a consumer warp
+constexpr u32 kThirds = 3;                       // consumer warps of a chain
+constexpr u32 kGM = 64 * kThirds, kGN = 16 * kTokTiles;  // tile: weight rows x tokens
+constexpr u32 kOutRows = kGM / 2;                // gate/up: outputs of a tile
+constexpr u32 kConsumers = 4 * kThirds, kHelpers = 4;    // warps
 constexpr u32 kGThreads = (kConsumers + kHelpers) * 32;
 constexpr u32 kStages = 3;
-constexpr u32 kRowPitch = kQ4KBlock + 16, kCodePitch = 256 + 32;
-constexpr u32 kRawBytes = kGM * kRowPitch, kCodeBytes = kGN * kCodePitch, kEsBytes = 8 * kGN * 8, kFacBytes = 8 * kGM * 8, kPrivBytes = kHelpers * 32 * 32;
-constexpr u32 kStageBytes = kRawBytes + kCodeBytes + kEsBytes + kFacBytes + kPrivBytes;
-constexpr u32 kOutPitch = kGM + 4;           // floats; twice the pitch is 8 (mod 32): the fragment stores meet every bank once
-constexpr u32 kOutBytes = kGN * kOutPitch * 4;  // epilogue tile (gate/up)
+constexpr u32 kCodePitch = 256 + 16;
+constexpr u32 kRawBytes = kGM * kQ4KBlock, kCodeBytes = kGN * kCodePitch, kEsBytes = 4 * kGN * 16, kFacBytes = 4 * kGM * 16, kPrivBytes = kGN * 64;
+constexpr u32 kStageBytes = (kRawBytes + kCodeBytes + kEsBytes + kFacBytes + kPrivBytes + 127) / 128 * 128;
+constexpr u32 kOffCode = kRawBytes, kOffEs = kOffCode + kCodeBytes, kOffFac = kOffEs + kEsBytes, kOffPriv = kOffFac + kFacBytes;  // in a stage
+constexpr u32 kOutPitch = kGM + 8;               // floats: the 8-byte stores of a half warp (four tokens, four row pairs) meet every bank once
+constexpr u32 kOutBytes = kGN * kOutPitch * 4;   // epilogue tile (gate/up)
+constexpr u32 kFoldCells = kRowTiles / 2 * kTokTiles * 2;      // float2 cells of a lane that change hands when two chains meet
+constexpr u32 kFoldBytes = kConsumers * kFoldCells * 32 * 8;
+static_assert(kOutBytes <= kFoldBytes, "the epilogue tile takes the place of the buffers that the chains met in");
 constexpr u32 kMaxUnion = 1024;
-constexpr u32 kBarBytes = 3 * kStages * 8 + 24 + kStages * 16 + 2 * 64 * 4;  // raw_full[], ready[], empty[]; abort flag; non-finite flags; token rows
-constexpr u32 kGroupedSmem = kStages * kStageBytes + kOutBytes + (kMaxUnion + 2) * 4 + kBarBytes + 64;
-static_assert(kGN <= 64 && kGN % 16 == 0, "a helper thread stages half the groups of one token");
+// What the consumers need of a tile: {first row, tokens, first entry}, its tokens' A8 rows, its tokens' slots. The helpers run at most
+// kStages stages ahead of the consumers, a tile has at least one stage and its places are read until its end: eight places.
+constexpr u32 kTilePlaces = 8, kTileWords = 4 + 2 * kGN;
+constexpr u32 kOffFold = kStages * kStageBytes, kOffBars = kOffFold + kFoldBytes, kOffTile = kOffBars + 3 * kStages * 8 + 8,
+              kOffCum = kOffTile + kTilePlaces * kTileWords * 4;
+constexpr u32 kGroupedSmem = kOffCum + (kMaxUnion + 2) * 4;
+static_assert((kOutRows * kQ4KBlock) % 128 == 0 && kOffBars % 8 == 0, "TMA destinations, barriers");
+static_assert(kGN == 32 && kGM / 2 == (kHelpers - 1) * 32, "a helper lane stages a token, the helper threads before it two rows each");
 static_assert(kGroupedSmem > 114u * 1024u && kGroupedSmem <= 227u * 1024u, "one CTA per SM, within the shared memory of an SM");
 constexpr u32 kWaitLimit = 1u << 20;         // polls of up to a microsecond
-constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23 = the float with the bits 0x4b400000
 // Register split between whole warp groups, out of what the launch gives every thread (65,536 over the threads, by eights).
 constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kHelperRegs = 80;
 constexpr u32 kConsumerRegs = (kGThreads * kLaunchRegs - kHelpers * 32u * kHelperRegs) / (kConsumers * 32u) / 8u * 8u;
@@ -64,24 +74,25 @@ static_assert(kConsumers * 32 * kConsumerRegs + kHelpers * 32 * kHelperRegs <= k
 
 // Two FP32 lanes per instruction (Blackwell packed FP32): each lane is one IEEE round-to-nearest operation, the same result
 // as two scalar instructions at half the issue slots. A packed add fed by a packed multiply did not reproduce the scalar
-// bits on B200 (it behaves as contracted), so an add is written as a * 1 + b, where the 1 is a kernel argument that no
-// compiler stage can fold away: one rounding, of a + b.
+// bits on B200 (it behaves as contracted), so a product is written as a * b + 0: one rounding, of a * b (a product of -0 comes
+// out as +0, which no sum of the chain tells apart).
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     float2 c;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<u64&>(c)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)));
+    asm("{\n\t.reg .b64 z;\n\tmov.b64 z, 0;\n\tfma.rn.f32x2 %0, %1, %2, z;\n\t}" : "=l"(reinterpret_cast<u64&>(c)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)));
     return c;
 }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<u64&>(d)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)), "l"(reinterpret_cast<const u64&>(c)));
-    return d;
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 c;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<u64&>(c)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)));
+    return c;
 }
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
-// 16 weight rows x 8 tokens x one group: unsigned nibble bytes times signed codes, on top of the bits of kMagic.
-__device__ __forceinline__ void mma_magic(float2 (&d)[2], u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-        : "=r"(reinterpret_cast<u32&>(d[0].x)), "=r"(reinterpret_cast<u32&>(d[0].y)), "=r"(reinterpret_cast<u32&>(d[1].x)), "=r"(reinterpret_cast<u32&>(d[1].y))
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4b400000));
+__device__ __forceinline__ float2 to_float(int2 v) { return make_float2(static_cast<float>(v.x), static_cast<float>(v.y)); }
+// 16 tokens x 8 weight rows x one group: signed codes times unsigned nibble bytes. d[z]: token lane / 4 + 8 z, weight rows
+// 2 (lane % 4) and the next.
+__device__ __forceinline__ void mma_dots(int2 (&d)[2], const u32 (&a)[4], u32 b0, u32 b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=r"(d[0].x), "=r"(d[0].y), "=r"(d[1].x), "=r"(d[1].y) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
 }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(dst)), "l"(src) : "memory");
@@ -100,10 +111,10 @@ struct GroupedArgs {
     float* raw;              // down output [slots][hidden]
     u32* row_status;
     u32* summary;
-    u32 n_row_tiles;         // inter / 64 (gate/up) or hidden / 128 (down)
+    u32 n_row_tiles;         // row tiles of an expert: inter / 96 (gate/up) or hidden / 192 (down), rounded up
     u32 K;                   // hidden (gate/up) or inter (down)
     u32 es_vec;              // the input's deltas and sums lie in whole 16-byte units
-    float one;               // 1.0f, unknown to the compiler (mul2 / fma2)
+    u32 raw_vec;             // raw lies on an 8-byte boundary
 };
 
 struct Tile { u32 expert, eb, nt, c, tt; };
@@ -126,74 +137,69 @@ __device__ __forceinline__ Tile find_tile(const GroupedArgs& a, const u32* cum, 
     return t;
 }
 
-// One super-block of the warp's 32 rows against the tokens of its chunks. rows: the lane's first weight row of the stage (nibbles
-// of its k slice); codes: the lane's token row of chunk 0; es / fac: the lane's {E, E', S, S'} and {rows 0, 8, 16, 24} factors.
-// acc[cc][i][p]: chain p of weight row 8 i + lane / 4 and two tokens of chunk kSplit cc + w. SLOW: the dot is converted first.
-template <bool SLOW>
-__device__ __forceinline__ void superblock(const unsigned char* rows, const unsigned char* codes, const float4* es, const float4* fac, u32 n_chunks,
-                                           float2 one, float2 (&acc)[kChunks][4][4]) {
+// One super-block of the warp's 64 rows and chain against NMT 16-token tiles. rows: weight row lane / 4 of the stage at the pair's
+// nibbles of the lane's k slice; codes: token lane / 4 at the pair's codes; es: the pair's {E, E', S, S'} from token lane / 4 on; fac: the
+// pair's {D, D, D', D'} {-DM, -DM, -DM', -DM'} of two rows, from row pair lane % 4 on. acc[j][mt][z]: rows 8 j + 2 (lane % 4) and the
+// next of token 16 mt + 8 z + lane / 4.
+template <int NMT>
+__device__ __forceinline__ void superblock(const unsigned char* rows, const unsigned char* codes, const float4* es, const float4* fac,
+                                           float2 (&acc)[kRowTiles][kTokTiles][2]) {
+    u32 cl[NMT][4], ch[NMT][4];
+    float4 e[NMT][2];
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        uint2 q[4];
+    for (int mt = 0; mt < NMT; ++mt)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const uint2*>(rows + 8 * i * kRowPitch + 32 * p);
-        float Dl[4], Ml[4], Dh[4], Mh[4], Nl[4], Nh[4];
-        *reinterpret_cast<float4*>(Dl) = fac[(4 * p) * (kGM / 4)]; *reinterpret_cast<float4*>(Ml) = fac[(4 * p + 1) * (kGM / 4)];
-        *reinterpret_cast<float4*>(Dh) = fac[(4 * p + 2) * (kGM / 4)]; *reinterpret_cast<float4*>(Mh) = fac[(4 * p + 3) * (kGM / 4)];
+        for (int z = 0; z < 2; ++z) {
+            const unsigned char* c = codes + (16 * mt + 8 * z) * kCodePitch;
+            // word by word: an A fragment's registers alternate between its two tokens, and 64-bit loads would have to be moved apart
+            // before every MMA (four moves each: 33.2 against 30.3 clocks an MMA)
+            cl[mt][z] = *reinterpret_cast<const u32*>(c);
+            cl[mt][z + 2] = *reinterpret_cast<const u32*>(c + 16);
+            ch[mt][z] = *reinterpret_cast<const u32*>(c + 32);
+            ch[mt][z + 2] = *reinterpret_cast<const u32*>(c + 48);
+            e[mt][z] = es[16 * mt + 8 * z];
+        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { Nl[i] = __fmul_rn(Dl[i], -kMagic); Nh[i] = __fmul_rn(Dh[i], -kMagic); }
+    for (int j = 0; j < (int)kRowTiles; ++j) {
+        const u32 q0 = *reinterpret_cast<const u32*>(rows + 8 * j * kQ4KBlock), q1 = *reinterpret_cast<const u32*>(rows + 8 * j * kQ4KBlock + 16);
+        const float4 d4 = fac[8 * j], m4 = fac[8 * j + 1];
+        const float2 Dl = make_float2(d4.x, d4.y), Dh = make_float2(d4.z, d4.w), Ml = make_float2(m4.x, m4.y), Mh = make_float2(m4.z, m4.w);
 #pragma unroll
-        for (int cc = 0; cc < (int)kChunks; ++cc) {
-            if (cc >= n_chunks) break;  // no valid token in these columns (warp-uniform)
-            const unsigned char* c = codes + 8 * kSplit * cc * kCodePitch + 64 * p;
-            const uint2 bl = *reinterpret_cast<const uint2*>(c), bh = *reinterpret_cast<const uint2*>(c + 32);
-            const float4 el = es[(2 * p) * (kGN / 2) + 4 * kSplit * cc], eh = es[(2 * p + 1) * (kGN / 2) + 4 * kSplit * cc];
+        for (int mt = 0; mt < NMT; ++mt) {
+            int2 l[2], h[2];
+            mma_dots(l, cl[mt], q0 & 0x0f0f0f0fu, q1 & 0x0f0f0f0fu);
+            mma_dots(h, ch[mt], q0 & 0xf0f0f0f0u, q1 & 0xf0f0f0f0u);
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                float2 l[2], h[2];
-                const uint2 r0 = q[2 * mt], r1 = q[2 * mt + 1];
-                mma_magic(l, r0.x & 0x0f0f0f0fu, r1.x & 0x0f0f0f0fu, r0.y & 0x0f0f0f0fu, r1.y & 0x0f0f0f0fu, bl.x, bl.y);
-                mma_magic(h, r0.x & 0xf0f0f0f0u, r1.x & 0xf0f0f0f0u, r0.y & 0xf0f0f0f0u, r1.y & 0xf0f0f0f0u, bh.x, bh.y);
-#pragma unroll
-                for (int z = 0; z < 2; ++z) {
-                    const int i = 2 * mt + z;
-                    float2 al, ah;
-                    if (SLOW) {
-                        al = mul2(both(Dl[i]), make_float2(__fsub_rn(l[z].x, kMagic), __fsub_rn(l[z].y, kMagic)));
-                        ah = mul2(both(Dh[i]), make_float2(__fsub_rn(h[z].x, kMagic), __fsub_rn(h[z].y, kMagic)));
-                    } else {
-                        al = fma2(both(Dl[i]), l[z], both(Nl[i]));
-                        ah = fma2(both(Dh[i]), h[z], both(Nh[i]));
-                    }
-                    // x = E * ((D * float(dot)) - (DM * S)) for the pair's two groups; M holds -DM, and (-DM) * S = -(DM * S) exactly
-                    const float2 sl = fma2(al, one, mul2(both(Ml[i]), make_float2(el.z, el.w)));
-                    const float2 sh = fma2(ah, one, mul2(both(Mh[i]), make_float2(eh.z, eh.w)));
-                    const float2 x = fma2(mul2(make_float2(el.x, el.y), sl), one, mul2(make_float2(eh.x, eh.y), sh));
-                    acc[cc][i][p] = fma2(x, one, acc[cc][i][p]);
-                }
+            for (int z = 0; z < 2; ++z) {
+                // x = E * ((D * float(dot)) - (DM * S)) for the pair's two groups; M holds -DM, and (-DM) * S = -(DM * S) exactly
+                const float2 sl = add2(mul2(Dl, to_float(l[z])), mul2(Ml, both(e[mt][z].z)));
+                const float2 sh = add2(mul2(Dh, to_float(h[z])), mul2(Mh, both(e[mt][z].w)));
+                acc[j][mt][z] = add2(add2(mul2(both(e[mt][z].x), sl), mul2(both(e[mt][z].y), sh)), acc[j][mt][z]);
             }
         }
     }
 }
 
-// SwiGLU + the A8 rule of up to four (token, 32 outputs) tasks of one warp, step by step over the four, so that their shuffle
-// and division chains overlap. g, u: the lane's gate and up values; returns per task whether a value is not finite.
+// SwiGLU + the A8 rule of kTasks (token, 32 outputs) tasks of one warp, step by step over them, so that their chains overlap. g, u: the
+// lane's gate and up values; returns per task whether a value is not finite (code, delta and sum then mean nothing).
 constexpr int kTasks = 4;
 __device__ __forceinline__ u32 swiglu_a8(const float (&g)[kTasks], const float (&u)[kTasks], int (&code)[kTasks], float (&delta)[kTasks], int (&sum)[kTasks]) {
-    float h[kTasks], amax[kTasks];
-    u32 bad = 0;
+    float h[kTasks], x[kTasks];
+    u32 bad = 0, amax[kTasks];
 #pragma unroll
-    for (int i = 0; i < kTasks; ++i) { h[i] = swiglu_qwen(g[i], u[i]); amax[i] = fabsf(h[i]); }
+    for (int i = 0; i < kTasks; ++i) x[i] = gfx1151_expf_straight(-g[i]);
 #pragma unroll
-    for (int i = 0; i < kTasks; ++i) bad |= __any_sync(0xffffffffu, !finite_f(g[i]) || !finite_f(u[i]) || !finite_f(h[i])) ? 1u << i : 0u;
-#pragma unroll
-    for (int d = 16; d; d >>= 1)
-#pragma unroll
-        for (int i = 0; i < kTasks; ++i) amax[i] = fmaxf(amax[i], __shfl_xor_sync(0xffffffffu, amax[i], d));
+    for (int i = 0; i < kTasks; ++i) {
+        h[i] = __fmul_rn(__fdiv_rn(g[i], __fadd_rn(1.0f, x[i])), u[i]);  // swiglu_qwen (declared_math.cuh)
+        bad |= __any_sync(0xffffffffu, !finite_f(g[i]) || !finite_f(u[i]) || !finite_f(h[i])) ? 1u << i : 0u;
+        amax[i] = __reduce_max_sync(0xffffffffu, __float_as_uint(h[i]) & 0x7fffffffu);  // the bits of finite magnitudes order as they do
+    }
 #pragma unroll
     for (int i = 0; i < kTasks; ++i) {  // a8_quantize_lane (common.cuh)
-        const bool tiny = amax[i] > 0.0f && amax[i] < 0x1p-119f;
-        delta[i] = (amax[i] == 0.0f || tiny) ? 1.0f : __fdiv_rn(amax[i], 127.0f);
+        const float am = __uint_as_float(amax[i]);
+        const bool tiny = am > 0.0f && am < 0x1p-119f;
+        // am / 127 rounded once: a double product is 2^-52 from it, a quotient by 127 no closer than 2^-32 to a rounding boundary
+        delta[i] = (am == 0.0f || tiny) ? 1.0f : static_cast<float>(static_cast<double>(am) * (1.0 / 127.0));
         const float r = tiny ? 0.0f : rintf(__fdiv_rn(h[i], delta[i]));
         const float lo = (-127.0f < r) ? r : -127.0f;
         code[i] = static_cast<int>((lo < 127.0f) ? lo : 127.0f);
@@ -202,19 +208,33 @@ __device__ __forceinline__ u32 swiglu_a8(const float (&g)[kTasks], const float (
     return bad;
 }
 
+// Factors of a row whose d and dmin are finite: sc / mn hold the 6-bit scales and mins of four groups a byte each. A byte goes behind
+// the exponent of 2^23 and fma(d, 2^23 + s, -2^23 d) is d * s, exact as the product has 17 bits. f: per pair D, D' / 16 (the high nibbles'
+// dots come as 16 * dot), -DM, -DM'.
+__device__ __forceinline__ void fast_factors(u32 head, u32 sc, u32 mn, float (&f)[2][4]) {
+    const float d = half_bits_to_float(head & 0xffffu), dm = -half_bits_to_float(head >> 16), dh = __fmul_rn(d, 0.0625f);
+    const float nd = __fmul_rn(d, -8388608.0f), ndm = __fmul_rn(dm, -8388608.0f), ndh = __fmul_rn(dh, -8388608.0f);
+#pragma unroll
+    for (u32 i = 0; i < 2; ++i) {
+        f[i][0] = __fmaf_rn(d, __uint_as_float(__byte_perm(sc, 0x4b000000u, 0x7440u + 2u * i)), nd);
+        f[i][1] = __fmaf_rn(dh, __uint_as_float(__byte_perm(sc, 0x4b000000u, 0x7441u + 2u * i)), ndh);
+        f[i][2] = __fmaf_rn(dm, __uint_as_float(__byte_perm(mn, 0x4b000000u, 0x7440u + 2u * i)), ndm);
+        f[i][3] = __fmaf_rn(dm, __uint_as_float(__byte_perm(mn, 0x4b000000u, 0x7441u + 2u * i)), ndm);
+    }
+}
+
 template <bool kDown>
 __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
                                                                    GroupedArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    float* s_out = reinterpret_cast<float*>(smem + kStages * kStageBytes);          // [kGN][kOutPitch]
-    u64* raw_full = reinterpret_cast<u64*>(smem + kStages * kStageBytes + kOutBytes);
+    float2* s_fold = reinterpret_cast<float2*>(smem + kOffFold);       // [warp][kFoldCells][lane]
+    float* s_out = reinterpret_cast<float*>(smem + kOffFold);          // [kGN][kOutPitch]
+    u64* raw_full = reinterpret_cast<u64*>(smem + kOffBars);
     u64* ready = raw_full + kStages;
     u64* empty = ready + kStages;
-    u32* s_abort_word = reinterpret_cast<u32*>(empty + kStages);                     // 24 bytes
-    u32* s_slow = s_abort_word + 6;                                                  // [stage][row quarter]: a non-finite d among the rows
-    u32* s_src = s_slow + kStages * 4;                                               // [tile parity][64]: A8 rows of the tile's tokens
-    u32* cum = s_src + 2 * 64;                                                       // [kMaxUnion + 1]
-    volatile u32* s_abort = s_abort_word;
+    volatile u32* s_abort = reinterpret_cast<u32*>(empty + kStages);
+    u32* s_tile = reinterpret_cast<u32*>(smem + kOffTile);             // [kTilePlaces][kTileWords]
+    u32* cum = reinterpret_cast<u32*>(smem + kOffCum);                 // [kMaxUnion + 1]
 
     if (kDown && a.summary && *a.summary) return;  // a failed or aborted projection skips the stage (routed_expert.hpp:17-19)
 
@@ -224,7 +244,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     if (tid == 0) {
         cum[0] = 0;
         for (u32 i = 0; i < kStages; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&ready[i], kHelpers); mbar_init(&empty[i], kConsumers); }
-        *s_abort_word = 0;
+        *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -249,181 +269,246 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     if (warp >= kConsumers) {
         // ================================================================================================= helpers
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kHelperRegs));
-        const u32 lt = tid - kConsumers * 32;            // 0..127 = weight row of the tile
-        const u32 hw = lt >> 5, tok = lt & 63u, half = lt >> 6;  // the token whose {E, S} this thread stages, and which half of the groups
+        const u32 lt = tid - kConsumers * 32, hw = lt >> 5;
         const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, in_gs = in_stride / 32;
-        u32 ik = 0, ib = 0, cy = 0;                      // tile and super-block of the next stage to request
-        const float* t_deltas = nullptr;
+        u32 ik = 0, ib = 0, cy = 0;                      // tile and super-block of the next stage to request; the tile's first weight row
+        u32 slot_r = 0, lap_r = 0, asked = 0;            // its ring place and lap; stages requested
+        const float* t_deltas = nullptr;                 // the last warp: of token `lane`
         const i32* t_sums = nullptr;
-        // Requests stage m: rows by TMA, codes and {E, S} by asynchronous copies (one commit group per thread and stage).
-        auto request = [&](u32 m) {
-            const u32 slot = m % kStages;
-            unsigned char* st = smem + slot * kStageBytes;
-            if (ok && m >= kStages) ok = mbar_wait(&empty[slot], (m / kStages - 1u) & 1u, kWaitLimit, s_abort);
-            if (ib == 0) {  // a new tile: every helper thread publishes the A8 row of its token
-                const Tile t = find_tile(a, cum, n_union, blockIdx.x + ik * gridDim.x);
-                const u32 ent = t.eb + min(tok, t.nt - 1u);
-                const u32 src = kDown ? a.routes.slots[ent] : a.routes.rows[ent];
-                if (half == 0) s_src[(ik & 1u) * 64u + tok] = src;
-                t_deltas = a.in.deltas + u64(src) * in_gs + 4u * half;
-                t_sums = a.in.sums + u64(src) * in_gs + 4u * half;
-                cy = kDown ? t.expert * H + kGM * t.c : t.expert * I + 64u * t.c;
+        const i8* t_codes[kGN / 8];                      // a half warp copies the 256 codes of one token
+        // the next tile, looked up a tile ahead: what it needs is a chain of reads from memory
+        Tile nx{};
+        u32 nx_src = 0, nx_slot = 0;
+        auto look_ahead = [&](u32 k) {
+            if (k >= my_tiles) return;
+            nx = find_tile(a, cum, n_union, blockIdx.x + k * gridDim.x);
+            const u32 ent = nx.eb + min(lane, nx.nt - 1u);
+            nx_slot = a.routes.slots[ent];
+            nx_src = kDown ? nx_slot : a.routes.rows[ent];
+        };
+        // Requests the next stage: rows by TMA, codes and {E, S} by asynchronous copies.
+        auto request = [&]() {
+            unsigned char* st = smem + slot_r * kStageBytes;
+            if (ib == 0) {  // a new tile: its tokens' A8 rows and slots are published
+                u32* ti = s_tile + (ik % kTilePlaces) * kTileWords;
+                const u32 first = kDown ? min(kGM * nx.c, H - kGM) : min(kOutRows * nx.c, I - kOutRows);
+                if (hw == 0) { ti[4 + lane] = nx_src; ti[4 + kGN + lane] = nx_slot; }
+                if (lt == 0) { ti[0] = first; ti[1] = nx.nt; ti[2] = nx.eb; }
+                t_deltas = a.in.deltas + u64(nx_src) * in_gs;
+                t_sums = a.in.sums + u64(nx_src) * in_gs;
+                cy = nx.expert * (kDown ? H : I) + first;
                 asm volatile("bar.sync 1, %0;" ::"n"(kHelpers * 32) : "memory");
+#pragma unroll
+                for (u32 i = 0; i < kGN / 8; ++i) t_codes[i] = a.in.codes + u64(ti[4 + (kGN / 4) * hw + 2u * i + (lane >> 4)]) * in_stride + 16u * (lane & 15u);
+                look_ahead(ik + 1);
             }
+            if (ok && lap_r) ok = mbar_wait(&empty[slot_r], (lap_r - 1u) & 1u, kWaitLimit, s_abort);
             if (ok) {
                 if (lt == 0) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the consumers' reads precede the copies below
-                    mbar_expect_tx(&raw_full[slot], kRawBytes);
-                    tma_2d(st, &tm0, ib * kQ4KBlock, cy, &raw_full[slot]);
-                    tma_2d(st + 64u * kRowPitch, kDown ? &tm0 : &tm1, ib * kQ4KBlock, kDown ? cy + 64u : cy, &raw_full[slot]);
+                    mbar_expect_tx(&raw_full[slot_r], kRawBytes);
+                    tma_2d(st, &tm0, ib * kQ4KBlock, cy, &raw_full[slot_r]);
+                    tma_2d(st + kOutRows * kQ4KBlock, kDown ? &tm0 : &tm1, ib * kQ4KBlock, kDown ? cy + kOutRows : cy, &raw_full[slot_r]);
+                    ++asked;
                 }
-                const u32* src = s_src + (ik & 1u) * 64u;
-                unsigned char* sc = st + kRawBytes;
+                unsigned char* sc = st + kOffCode + ((kGN / 4) * hw + (lane >> 4)) * kCodePitch + 16u * (lane & 15u);
 #pragma unroll
-                for (u32 i = 0; i < kGN / 8; ++i) {  // a half warp copies the 256 codes of one token
-                    const u32 tk = (kGN / 4) * hw + 2u * i + (lane >> 4);
-                    cp_async16(sc + tk * kCodePitch + 16u * (lane & 15u), a.in.codes + u64(src[tk]) * in_stride + 256u * ib + 16u * (lane & 15u));
+                for (u32 i = 0; i < kGN / 8; ++i) { cp_async16(sc + 2u * i * kCodePitch, t_codes[i]); t_codes[i] += 256; }
+                if (hw == kHelpers - 1u) {
+                    unsigned char* pv = st + kOffPriv + 64u * lane;
+                    if (a.es_vec) {
+                        cp_async16(pv, t_deltas);
+                        cp_async16(pv + 16, t_deltas + 4);
+                        cp_async16(pv + 32, t_sums);
+                        cp_async16(pv + 48, t_sums + 4);
+                    } else {
+#pragma unroll 1
+                        for (u32 i = 0; i < 8; ++i) {
+                            cp_async4(pv + 4u * i, t_deltas + i);
+                            cp_async4(pv + 32u + 4u * i, t_sums + i);
+                        }
+                    }
+                    t_deltas += 8; t_sums += 8;
                 }
-                unsigned char* pv = st + kRawBytes + kCodeBytes + kEsBytes + kFacBytes + 32u * lt;
-                if (a.es_vec) {
-                    cp_async16(pv, t_deltas + 8u * ib);
-                    cp_async16(pv + 16, t_sums + 8u * ib);
+            }
+            if (++ib == nblocks) { ib = 0; ++ik; }
+            if (++slot_r == kStages) { slot_r = 0; ++lap_r; }
+        };
+        look_ahead(0);
+        u32 slot = 0, lap = 0;
+        for (u32 m = 0; m < total; ++m) {
+            // decoded as soon as it has landed, up to two stages before the consumers need it
+            request();
+            unsigned char* st = smem + slot * kStageBytes;
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            if (ok) ok = mbar_wait(&raw_full[slot], lap & 1u, kWaitLimit, s_abort);
+            ok = __all_sync(0xffffffffu, ok);
+            if (ok) {  // else no more requests or hand-overs; the tile barrier above is still met by every helper
+                if (hw < kHelpers - 1u) {
+                    // rows 2 lt and 2 lt + 1; which one is read first alternates, for the banks of the 128-bit reads
+                    const u32 swap = (lt >> 2) & 1u;
+                    const uint4 ha = *reinterpret_cast<const uint4*>(st + (2u * lt + swap) * kQ4KBlock), hb = *reinterpret_cast<const uint4*>(st + (2u * lt + 1u - swap) * kQ4KBlock);
+                    auto special = [](u32 w) { return (w & 0x7c00u) == 0x7c00u || (w & 0x7c000000u) == 0x7c000000u; };
+                    const bool slow = __any_sync(0xffffffffu, special(ha.x) || special(hb.x));
+                    // [pair][row pair][D, D, D', D' | -DM, -DM, -DM', -DM']
+                    float4* fac = reinterpret_cast<float4*>(st + kOffFac) + 2u * lt;
+#pragma unroll
+                    for (u32 half = 0; half < 2; ++half) {
+                        float fa[2][4], fb[2][4];
+                        auto decode = [&](const uint4& h, float (&f)[2][4]) {
+                            if (slow) {  // an infinity or a NaN: the products themselves
+#pragma unroll 1
+                                for (u32 i = 0; i < 2; ++i) {
+                                    const Factors x = q4k_factors(h, 2u * half + i);
+                                    const float v[4] = {x.Dl, __fmul_rn(x.Dh, 0.0625f), -x.DMl, -x.DMh};
+#pragma unroll
+                                    for (u32 k = 0; k < 4; ++k) { if (i == 0) f[0][k] = v[k]; else f[1][k] = v[k]; }
+                                }
+                            } else if (half == 0) {
+                                fast_factors(h.x, h.y & 0x3f3f3f3fu, h.z & 0x3f3f3f3fu, f);
+                            } else {
+                                fast_factors(h.x, (h.w & 0x0f0f0f0fu) | ((h.y >> 2) & 0x30303030u), ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u), f);
+                            }
+                        };
+                        decode(swap ? hb : ha, fa);
+                        decode(swap ? ha : hb, fb);
+#pragma unroll
+                        for (u32 i = 0; i < 2; ++i) {
+                            fac[(2u * half + i) * kGM] = make_float4(fa[i][0], fb[i][0], fa[i][1], fb[i][1]);
+                            fac[(2u * half + i) * kGM + 1] = make_float4(fa[i][2], fb[i][2], fa[i][3], fb[i][3]);
+                        }
+                    }
                 } else {
+                    const unsigned char* pv = st + kOffPriv + 64u * lane;
+                    float4* es = reinterpret_cast<float4*>(st + kOffEs) + lane;  // [pair][token] {E, E', S, S'}
 #pragma unroll
-                    for (u32 i = 0; i < 4; ++i) {
-                        cp_async4(pv + 4u * i, t_deltas + 8u * ib + i);
-                        cp_async4(pv + 16u + 4u * i, t_sums + 8u * ib + i);
+                    for (u32 i = 0; i < 2; ++i) {
+                        const float4 e = reinterpret_cast<const float4*>(pv)[i];
+                        const int4 sm = reinterpret_cast<const int4*>(pv + 32)[i];
+                        es[2 * i * kGN] = make_float4(e.x, e.y, static_cast<float>(sm.x), static_cast<float>(sm.y));
+                        es[(2 * i + 1) * kGN] = make_float4(e.z, e.w, static_cast<float>(sm.z), static_cast<float>(sm.w));
                     }
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ready[slot]);
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            if (++ib == nblocks) { ib = 0; ++ik; }
-        };
-        if (total) request(0);
-        u32 asked = total ? 1u : 0u;
-        for (u32 m = 0; m < total; ++m) {
-            if (m + 1 < total) { request(m + 1); ++asked; }
-            else asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group keeps the count of the wait below fixed
-            const u32 slot = m % kStages;
-            unsigned char* st = smem + slot * kStageBytes;
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            if (ok) ok = mbar_wait(&raw_full[slot], (m / kStages) & 1u, kWaitLimit, s_abort);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) continue;  // no more requests or hand-overs; the tile barrier above is still met by every helper
-            const uint4 hdr = *reinterpret_cast<const uint4*>(st + lt * kRowPitch);
-            const bool slow = __any_sync(0xffffffffu, (hdr.x & 0x7c00u) == 0x7c00u);
-            if (lane == 0) s_slow[slot * 4u + hw] = slow ? 1u : 0u;
-            // the row's factors, [group][D | -DM][quarter][row % 8][row / 8 % 4]: a lane's four rows are one 128-bit load;
-            // the high nibbles' dots come as 16 * dot
-            float* fac = reinterpret_cast<float*>(st + kRawBytes + kCodeBytes + kEsBytes) + (lt & ~31u) + (lt & 7u) * 4u + ((lt >> 3) & 3u);
-#pragma unroll
-            for (u32 p = 0; p < 4; ++p) {
-                const Factors f = q4k_factors(hdr, p);
-                fac[(4 * p) * kGM] = f.Dl; fac[(4 * p + 1) * kGM] = -f.DMl;
-                fac[(4 * p + 2) * kGM] = __fmul_rn(f.Dh, 0.0625f); fac[(4 * p + 3) * kGM] = -f.DMh;
-            }
-            const unsigned char* pv = st + kRawBytes + kCodeBytes + kEsBytes + kFacBytes + 32u * lt;
-            const float4 e = *reinterpret_cast<const float4*>(pv);
-            const int4 sm = *reinterpret_cast<const int4*>(pv + 16);
-            if (tok < kGN) {
-                float* es = reinterpret_cast<float*>(st + kRawBytes + kCodeBytes) + (4u * half * (kGN / 2) + (tok >> 1)) * 4u + (tok & 1u);  // [group][token pair] {E, E', S, S'}
-                es[0] = e.x; es[2] = static_cast<float>(sm.x);
-                es[2 * kGN] = e.y; es[2 * kGN + 2] = static_cast<float>(sm.y);
-                es[4 * kGN] = e.z; es[4 * kGN + 2] = static_cast<float>(sm.z);
-                es[6 * kGN] = e.w; es[6 * kGN + 2] = static_cast<float>(sm.w);
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ready[slot]);
+            if (++slot == kStages) { slot = 0; ++lap; }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        if (*s_abort && lt == 0)  // wait (bounded) for the copies still in flight before the CTA retires
-            for (u32 n = asked > kStages ? asked - kStages : 0u; n < asked; ++n)
-                for (u32 i = 0; i < (kWaitLimit >> 8); ++i)
-                    if (mbar_try_wait(&raw_full[n % kStages], (n / kStages) & 1u, kWaitHintNs)) break;
+        if (!ok && asked && lt == 0)  // wait (bounded) for the copies still in flight before the CTA retires
+            for (u32 i = 0; i < (kWaitLimit >> 8); ++i)
+                if (mbar_try_wait(&raw_full[(asked - 1u) % kStages], ((asked - 1u) / kStages) & 1u, kWaitHintNs)) break;
     } else {
         // ================================================================================================ consumers
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
-        const u32 quarter = warp & 3u, w = warp >> 2;   // 32 rows of the tile; the 8-token chunks alternate between the kSplit warps of a quarter
-        const u32 fr = lane >> 2, ft = lane & 3u;       // fragments: rows 32 quarter + 8 i + fr (i = 0 .. 3), tokens 2 ft, 2 ft + 1 of a chunk
+        const u32 p = warp & 3u, third = warp >> 2;     // chain, 64 rows of the tile
+        const u32 fr = lane >> 2, ft = lane & 3u;       // fragments: token fr (and fr + 8) of a token tile, rows 2 ft and 2 ft + 1 of a row tile
         const u32 act_stride = a.act.stride ? a.act.stride : a.act.width;
-        const float2 one = both(a.one);
-        u32 m = 0;
-        for (u32 id = blockIdx.x; id < n_tiles; id += gridDim.x) {
-            const Tile t = find_tile(a, cum, n_union, id);
-            const u32 n_chunks = t.nt > 8u * w ? (t.nt - 8u * w + 8u * kSplit - 1u) / (8u * kSplit) : 0u;  // chunks w, w + kSplit, ...
-            float2 acc[kChunks][4][4];
+        u32 slot = 0, parity = 0;
+        for (u32 ik = 0; ik < my_tiles; ++ik) {
+            const u32* ti = s_tile + (ik % kTilePlaces) * kTileWords;
+            u32 n_mt = 0;
+            float2 acc[kRowTiles][kTokTiles][2];
 #pragma unroll
-            for (int i = 0; i < (int)kChunks * 16; ++i) (&acc[0][0][0])[i] = make_float2(0.0f, 0.0f);
-            for (u32 b = 0; b < nblocks; ++b, ++m) {
-                const u32 slot = m % kStages, parity = (m / kStages) & 1u;
+            for (int i = 0; i < (int)(kRowTiles * kTokTiles * 2); ++i) (&acc[0][0][0])[i] = make_float2(0.0f, 0.0f);
+            for (u32 b = 0; b < nblocks; ++b) {
+                // asked a stage ahead, so that the answer is there (the helpers have seen the rows' copies complete before they arrive)
                 if (ok) ok = mbar_wait(&ready[slot], parity, kWaitLimit, s_abort);
-                if (ok) ok = mbar_wait(&raw_full[slot], parity, kWaitLimit, s_abort);  // complete by now: orders the TMA's writes before our reads
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) continue;
+                const u32 next = slot + 1u == kStages ? 0u : slot + 1u, next_parity = parity ^ (next == 0u ? 1u : 0u);
+                if (b == 0) n_mt = (ti[1] + 15u) / 16u;
                 const unsigned char* st = smem + slot * kStageBytes;
-                const unsigned char* rows = st + (32u * quarter + fr) * kRowPitch + 16u + 8u * ft;
-                const unsigned char* codes = st + kRawBytes + (8u * w + fr) * kCodePitch + 8u * ft;
-                const float4* es = reinterpret_cast<const float4*>(st + kRawBytes + kCodeBytes) + 4u * w + ft;
-                const float4* fac = reinterpret_cast<const float4*>(st + kRawBytes + kCodeBytes + kEsBytes) + 8u * quarter + fr;
-                if (n_chunks) {
-                    if (s_slow[slot * 4u + quarter]) superblock<true>(rows, codes, es, fac, n_chunks, one, acc);
-                    else superblock<false>(rows, codes, es, fac, n_chunks, one, acc);
-                }
+                const unsigned char* rows = st + (64u * third + fr) * kQ4KBlock + 16u + 32u * p + 4u * ft;
+                const unsigned char* codes = st + kOffCode + fr * kCodePitch + 64u * p + 4u * ft;
+                const float4* es = reinterpret_cast<const float4*>(st + kOffEs) + p * kGN + fr;
+                const float4* fac = reinterpret_cast<const float4*>(st + kOffFac) + p * kGM + 2u * (32u * third + ft);
+                if (n_mt == 2) superblock<2>(rows, codes, es, fac, acc);
+                else superblock<1>(rows, codes, es, fac, acc);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[slot]);
+                slot = next; parity = next_parity;
             }
-            // (a0 + a1) + (a2 + a3)
-            auto fold = [&](const float2* c, int second) {
-                return second ? __fadd_rn(__fadd_rn(c[0].y, c[1].y), __fadd_rn(c[2].y, c[3].y)) : __fadd_rn(__fadd_rn(c[0].x, c[1].x), __fadd_rn(c[2].x, c[3].x));
-            };
+            // (a0 + a1) + (a2 + a3). Warp p hands half of its row tiles to warp p ^ 1 of its third and adds what that hands over, then does the
+            // same with half of what is left and warp p ^ 2. Buffer p is written by warp p, then by warp p ^ 1 (which alone has read it), then
+            // read by warp p ^ 3. The barriers are met on every path.
+            if (kDown) asm volatile("bar.sync %0, 128;" ::"r"(4u + third) : "memory");  // the previous tile's last reads of the buffers
+            else asm volatile("bar.sync 2, %0;" ::"n"(kConsumers * 32) : "memory");     // ... and of s_out
+            float2* bufs = s_fold + 4u * third * (kFoldCells * 32) + lane;
+            float2* mine = bufs + p * (kFoldCells * 32);
+            float2* theirs = bufs + (p ^ 1u) * (kFoldCells * 32);
+            const float2* last = bufs + (p ^ 3u) * (kFoldCells * 32);
+            const bool odd = p & 1u, high = p >> 1;
+            auto pick = [](bool c, float2 x, float2 y) { return make_float2(c ? x.x : y.x, c ? x.y : y.y); };
+            auto add = [](float2 x, float2 y) { return make_float2(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y)); };
+            constexpr int n = 2 * kTokTiles;  // cells of a row tile
+            float2* cells = &acc[0][0][0];
+#pragma unroll
+            for (int i = 0; i < 4 * n; ++i) mine[32 * i] = pick(odd, cells[i], cells[4 * n + i]);
+            asm volatile("bar.sync %0, 128;" ::"r"(4u + third) : "memory");
+            float2 out[2][kTokTiles][2];
+#pragma unroll
+            for (int i = 0; i < 2 * n; ++i) {
+                const float2 s0 = add(pick(odd, cells[4 * n + i], cells[i]), theirs[32 * i]), s1 = add(pick(odd, cells[6 * n + i], cells[2 * n + i]), theirs[32 * (2 * n + i)]);
+                theirs[32 * i] = pick(high, s0, s1);
+                (&out[0][0][0])[i] = pick(high, s1, s0);
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(4u + third) : "memory");
+#pragma unroll
+            for (int i = 0; i < 2 * n; ++i) (&out[0][0][0])[i] = add((&out[0][0][0])[i], last[32 * i]);
+            const u32 row0 = 64u * third + 32u * (p & 1u) + 16u * (p >> 1) + 2u * ft;  // the lane's first row of the two row tiles that are left to it
+            const u32 nt = ok ? ti[1] : 0u, first = ti[0], eb = ti[2];
             if (kDown) {
-                if (ok) {
 #pragma unroll
-                    for (int cz = 0; cz < 2 * (int)kChunks; ++cz) {
-                        const u32 tk = 8u * (kSplit * (cz >> 1) + w) + 2u * ft + (cz & 1);
-                        if (tk < t.nt) {
-                            float* out = a.raw + u64(a.routes.slots[t.eb + tk]) * H + kGM * t.c + 32u * quarter + fr;
+                for (int cz = 0; cz < n; ++cz) {
+                    const u32 tk = 8u * cz + fr;
+                    if (tk < nt) {
+                        float* to = a.raw + u64(ti[4 + kGN + tk]) * H + first + row0;
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) out[8 * i] = fold(acc[cz >> 1][i], cz & 1);
+                        for (int i = 0; i < 2; ++i) {
+                            const float2 v = out[i][cz >> 1][cz & 1];
+                            if (a.raw_vec) *reinterpret_cast<float2*>(to + 8 * i) = v;
+                            else { to[8 * i] = v.x; to[8 * i + 1] = v.y; }
                         }
                     }
                 }
             } else {
-                asm volatile("bar.sync 3, %0;" ::"n"(kConsumers * 32) : "memory");  // the previous tile's epilogue has read s_out
+                asm volatile("bar.sync 2, %0;" ::"n"(kConsumers * 32) : "memory");  // the buffers have been read
 #pragma unroll
-                for (int cz = 0; cz < 2 * (int)kChunks; ++cz) {
-                    float* out = s_out + (8u * (kSplit * (cz >> 1) + w) + 2u * ft + (cz & 1)) * kOutPitch + 32u * quarter + fr;
+                for (int cz = 0; cz < n; ++cz) {
+                    float* to = s_out + (8u * cz + fr) * kOutPitch + row0;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) out[8 * i] = fold(acc[cz >> 1][i], cz & 1);
+                    for (int i = 0; i < 2; ++i) *reinterpret_cast<float2*>(to + 8 * i) = out[i][cz >> 1][cz & 1];
                 }
-                asm volatile("bar.sync 3, %0;" ::"n"(kConsumers * 32) : "memory");
-                // SwiGLU + the A8 rule: a task is (token, 32 outputs), two per token; a warp takes the four of two tokens at a time
-                for (u32 tk0 = 2u * warp; ok && tk0 < t.nt; tk0 += 2u * kConsumers) {
+                asm volatile("bar.sync 2, %0;" ::"n"(kConsumers * 32) : "memory");
+                // SwiGLU + the A8 rule: a task is (token, one of its three groups of 32 outputs)
+                constexpr u32 per = kOutRows / 32;
+                for (u32 k0 = kTasks * warp; k0 < per * nt; k0 += kTasks * kConsumers) {
                     float g[kTasks], u[kTasks], delta[kTasks];
                     int code[kTasks], sum[kTasks];
 #pragma unroll
                     for (int i = 0; i < kTasks; ++i) {
-                        const float* row = s_out + min(tk0 + (i >> 1), t.nt - 1u) * kOutPitch + 32u * (i & 1) + lane;
-                        g[i] = row[0]; u[i] = row[64];
+                        const u32 k = min(k0 + i, per * nt - 1u), tk = k / per;
+                        const float* src = s_out + tk * kOutPitch + 32u * (k - per * tk) + lane;
+                        g[i] = src[0]; u[i] = src[kOutRows];
                     }
                     const u32 bad = swiglu_a8(g, u, code, delta, sum);
 #pragma unroll
                     for (int i = 0; i < kTasks; ++i) {
-                        const u32 tk = tk0 + (i >> 1);
-                        if (tk >= t.nt) break;
-                        const u32 slot = a.routes.slots[t.eb + tk], group = 2u * t.c + (i & 1), o_col = 32u * group + lane;
-                        if (a.gate_out) { a.gate_out[u64(slot) * I + o_col] = g[i]; a.up_out[u64(slot) * I + o_col] = u[i]; }
+                        const u32 k = k0 + i, tk = k / per;
+                        if (k >= per * nt) break;
+                        const u32 slot_id = ti[4 + kGN + tk], group = first / 32u + (k - per * tk), o_col = 32u * group + lane;
+                        if (a.gate_out) { a.gate_out[u64(slot_id) * I + o_col] = g[i]; a.up_out[u64(slot_id) * I + o_col] = u[i]; }
                         if (bad >> i & 1u) {  // fail closed: nothing of the group is written (routed_expert.cpp:147-156)
                             if (lane == 0) {
-                                if (a.row_status) atomicOr(&a.row_status[a.routes.rows[t.eb + tk]], B200MOE_ROW_PROJECTION_NONFINITE);
+                                if (a.row_status) atomicOr(&a.row_status[a.routes.rows[eb + tk]], B200MOE_ROW_PROJECTION_NONFINITE);
                                 if (a.summary) atomicOr(a.summary, B200MOE_ROW_PROJECTION_NONFINITE);
                             }
                             continue;
                         }
-                        a.act.codes[u64(slot) * act_stride + o_col] = static_cast<i8>(code[i]);
+                        a.act.codes[u64(slot_id) * act_stride + o_col] = static_cast<i8>(code[i]);
                         if (lane == 0) {
-                            a.act.deltas[u64(slot) * (act_stride / 32) + group] = delta[i];
-                            if (a.act.sums) a.act.sums[u64(slot) * (act_stride / 32) + group] = sum[i];
+                            a.act.deltas[u64(slot_id) * (act_stride / 32) + group] = delta[i];
+                            if (a.act.sums) a.act.sums[u64(slot_id) * (act_stride / 32) + group] = sum[i];
                         }
                     }
                 }
@@ -433,7 +518,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     if (!ok && lane == 0 && a.summary) atomicOr(a.summary, kAbortBit);
 }
 
-// Tensor map of a [rows][row_bytes] byte tensor with boxes of kRowPitch bytes x 64 rows (no swizzle, no interleave). The
+// Tensor map of a [rows][row_bytes] byte tensor with boxes of a super-block x 96 rows (no swizzle, no interleave). The
 // encoder is the driver's cuTensorMapEncodeTiled, looked up through the runtime (no link against the driver library).
 int encode_rows_map(const u8* base, u64 row_bytes, u64 rows, CUtensorMap* out) {
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -447,7 +532,7 @@ int encode_rows_map(const u8* base, u64 row_bytes, u64 rows, CUtensorMap* out) {
     if (!fn) return fail(B200MOE_ERR_CUDA, "grouped: cuTensorMapEncodeTiled is not available from this driver");
     const cuuint64_t dims[2] = {row_bytes, rows};
     const cuuint64_t strides[1] = {row_bytes};       // bytes between rows: a multiple of 16 (144 per super-block)
-    const cuuint32_t box[2] = {kRowPitch, 64};  // 16 bytes past the super-block: the next one's, or the fill value at the end of a row
+    const cuuint32_t box[2] = {kQ4KBlock, kOutRows};
     const cuuint32_t elem[2] = {1, 1};
     const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<u8*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -462,7 +547,7 @@ bool es_units(const b200moe_a8_rows& x) {
 
 bool grouped_shape_ok(const b200moe_shape& s) {
     return s.gate_type == B200MOE_TYPE_Q4_K && s.down_type == B200MOE_TYPE_Q4_K && s.hidden % 256 == 0 && s.inter % 256 == 0 &&
-           s.hidden % kGM == 0 && s.inter % 64 == 0 && s.experts <= kMaxUnion;
+           s.experts <= kMaxUnion;
 }
 
 int grid_size() {
@@ -480,7 +565,7 @@ int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t strea
     GroupedArgs a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.x; a.act = v.act;
     a.gate_out = v.gate_out; a.up_out = v.up_out; a.row_status = v.row_status; a.summary = v.summary;
-    a.n_row_tiles = v.shape.inter / 64; a.K = v.shape.hidden; a.one = 1.0f; a.es_vec = es_units(v.x);
+    a.n_row_tiles = (v.shape.inter + kOutRows - 1) / kOutRows; a.K = v.shape.hidden; a.es_vec = es_units(v.x);
     CUtensorMap tm0, tm1;
     const u64 rb = u64(v.shape.hidden / 256) * kQ4KBlock, rows = u64(v.shape.experts) * v.shape.inter;
     if (int rc = encode_rows_map(v.weights.gate, rb, rows, &tm0)) return rc;
@@ -495,7 +580,7 @@ int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     GroupedArgs a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.act; a.raw = v.raw;
     a.summary = const_cast<u32*>(v.summary);
-    a.n_row_tiles = v.shape.hidden / kGM; a.K = v.shape.inter; a.one = 1.0f; a.es_vec = es_units(v.act);
+    a.n_row_tiles = (v.shape.hidden + kGM - 1) / kGM; a.K = v.shape.inter; a.es_vec = es_units(v.act); a.raw_vec = aligned(v.raw, 8);
     CUtensorMap tm0;
     if (int rc = encode_rows_map(v.weights.down, u64(v.shape.inter / 256) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<true>), kGroupedSmem)) return rc;

@@ -56,6 +56,35 @@ def test_grouped_tile_remainders(gpu, oracle, tokens):
     assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
 
 
+@pytest.mark.parametrize("tokens,H,I,scale,special", [(31, 512, 512, 1, 0), (33, 256, 768, 1, 0), (63, 768, 256, 1, 0x7c00), (64, 1024, 1024, 400, 0),
+                                                      (65, 256, 2048, 400, 0xfe00)])
+def test_grouped_row_tiles_of_a_share(gpu, oracle, tokens, H, I, scale, special):
+    """Row tiles (96 outputs, 192 down rows) that end inside an expert, token tiles of 32 and their halves, tensors that hold fewer
+    experts than the shape counts, gates beyond both limits of exp, a dmin that is not finite."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(tokens)
+    E, rows = 2, 130
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+    blocks = gate.copy().reshape(-1, 144)
+    if scale != 1:
+        blocks[:, 0:4] = (blocks[:, 0:4].copy().view(np.float16).astype(np.float32) * scale).astype(np.float16).view(np.uint8)
+    gate = blocks.reshape(-1)
+    down = down.copy()
+    if special:
+        down.reshape(E, H, I // 256, 144)[1, 7, 0, 2:4] = np.array([special], np.uint16).view(np.uint8)
+    ids = np.zeros((rows, 1), np.uint32)
+    ids[rng.permutation(rows)[:tokens]] = 1
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, 12, 12, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    if scale != 1:
+        assert np.abs(want["gate"]).max() > 110
+    sh = ops.make_shape(H, I, 4, 1, 12, 12)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), 4, 2)
+    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, 4, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, 4, act).cpu(), want["raw"])
+
+
 @pytest.mark.parametrize("bits", [0x7c00, 0xfc00, 0x7e00])
 def test_grouped_factor_not_finite(gpu, oracle, bits):
     """A down row whose super-block factor is an infinity or a NaN: the term is d * dot, not what is left of (M + dot) - M."""

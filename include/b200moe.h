@@ -79,7 +79,7 @@ uint64_t b200moe_launch_count(void);
                                       * before its n-th stage (no copy of that stage is issued, none is left in flight); 0 = never */
 #define B200MOE_DEBUG_DECODE_FORM 2u /* decode windows: 0 = chosen by the plan, 1 = row streaming (Q4_K), 2 = segment streaming (Q4_K;
                                       * Q8_0: the dp4a token-block form), 3 = per-block (Q8_0: one row per warp), 4 = the Q8_0
-                                      * tensor-core form (each only where it applies) */
+                                      * tensor-core form, 5 = the grouped Q8_0 form (each only where it applies) */
 int b200moe_debug_set(uint32_t key, uint32_t value);
 
 /* ------------------------------------------------------------------------------------------------ A8 activations

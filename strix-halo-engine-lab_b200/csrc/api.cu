@@ -262,10 +262,20 @@ DecodeForm pick_decode_form(bool row_stream_fits, bool wide_fits, u32 rows, u32 
 // gemv_q8_mma.cu (rows of 1024 to 7168 weights), else the dp4a token-block form of gemv_q8_wide.cu. Measured on B200: a
 // 7168 x 2048 dense block over 8 rows takes 49 + 18 us in the dp4a token-block form against 55 + 30 us with one row per
 // warp; one row over four experts of 2048 x 1024 is 2 us faster with one row per warp.
-enum class Q8Form { row_per_warp, wide, mma };
-Q8Form pick_q8_form(bool wide_fits, bool mma_fits, u32 rows) {
+// The grouped form (grouped_q8.cu, tiles of 32 entries) takes over from the tensor-core form at 10 entries an expert and 20 rows: whole calls, the
+// two in this order, 64 experts of 2048 x 1024: 199 and 236 us with 6 entries, 249 and 239 with 8, 328 and 240 with 12; 16 experts of
+// 4096 x 1536: 167 and 188 with 8, 241 and 196 with 16; one expert of 7168 x 2048: 49 and 64 us with 16 rows, 63 and 61 with 24, 101
+// and 66 with 64. Where the tensor-core form does not apply (rows below 1024 or above 7168 weights) it takes over from the dp4a form at 2
+// entries and 12 rows: 48 experts of 1024 x 512 109 and 93 us with 2 entries, one expert of 2048 x 8192 66 and 79 us with 8 rows,
+// 76 and 70 with 16, of 768 x 4096 49 and 51 with 8, 50 and 49 with 16.
+enum class Q8Form { row_per_warp, wide, mma, grouped };
+bool q8_grouped_pays(bool mma_fits, u32 rows, const b200moe_shape& s) {
+    return rows >= (mma_fits ? 20u : 12u) && u64(rows) * s.top_k >= u64(mma_fits ? 10u : 2u) * s.experts;
+}
+Q8Form pick_q8_form(bool wide_fits, bool mma_fits, bool grouped_fits, u32 rows, const b200moe_shape& s) {
     const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
     if (forced == 3) return Q8Form::row_per_warp;
+    if (grouped_fits && (forced == 5 || (forced == 0 && q8_grouped_pays(mma_fits, rows, s)))) return Q8Form::grouped;
     if (forced == 4 && mma_fits) return Q8Form::mma;
     if (forced == 2 && wide_fits) return Q8Form::wide;
     if (forced == 0 && rows >= kRowStreamRows) {
@@ -277,7 +287,8 @@ Q8Form pick_q8_form(bool wide_fits, bool mma_fits, u32 rows) {
 int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0) {
     if (v.shape.gate_type == B200MOE_TYPE_Q2_K) return launch_gate_up_ds41_any(v, st);  // the generic form of the family reads every block type
     if (!is_kquant(v.shape.gate_type)) {
-        switch (pick_q8_form(q8_wide_gate_up_fits(v, rows), q8_mma_gate_up_fits(v, rows), rows)) {
+        switch (pick_q8_form(q8_wide_gate_up_fits(v, rows), q8_mma_gate_up_fits(v, rows), grouped_q8_gate_up_fits(v), rows, v.shape)) {
+            case Q8Form::grouped: return launch_gate_up_q8_grouped(v, st);
             case Q8Form::mma: return launch_gate_up_q8_mma(v, rows, st);
             case Q8Form::wide: return launch_gate_up_q8_wide(v, rows, st);
             default: return launch_gate_up_q8(v, st);
@@ -302,7 +313,8 @@ int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grou
     }
     if (is_kquant(v.shape.gate_type)) return launch_down_q8_chain4(v, st);  // chain4: Q8_0 and Q5_1 blocks
     if (v.shape.down_type == B200MOE_TYPE_Q2_K) return launch_down_ds41_any(v, st);
-    switch (pick_q8_form(q8_wide_down_fits(v, rows), q8_mma_down_fits(v, rows), rows)) {
+    switch (pick_q8_form(q8_wide_down_fits(v, rows), q8_mma_down_fits(v, rows), grouped_q8_down_fits(v), rows, v.shape)) {
+        case Q8Form::grouped: return launch_down_q8_grouped(v, st);
         case Q8Form::mma: return launch_down_q8_mma(v, rows, st);
         case Q8Form::wide: return launch_down_q8_wide(v, rows, st);
         default: return launch_down_q8(v, st);

@@ -76,9 +76,7 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 __device__ __forceinline__ int warp_sum_i(int v) {
-#pragma unroll
-    for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-    return v;
+    return __reduce_add_sync(0xffffffffu, v);
 }
 // The declared butterfly: v[l] = v[l] + v[l ^ d], d = 16 .. 1 (src/core/integer_math.hpp:43-47). Addition is
 // commutative bit for bit, so every lane ends with the tree's value.

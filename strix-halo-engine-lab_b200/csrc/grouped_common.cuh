@@ -1,0 +1,78 @@
+// Pieces shared by the grouped forms (grouped_q4k.cu, grouped_q8.cu): packed FP32, asynchronous copies, and the tiles of a window - an
+// expert, up to GN of its entries, one of its row tiles - that a persistent grid walks round-robin.
+#pragma once
+#include "q4k_row.cuh"
+
+namespace b200moe {
+namespace grouped {
+
+constexpr u32 kMaxUnion = 1024;
+
+// Two FP32 lanes per instruction (Blackwell packed FP32): each lane is one IEEE round-to-nearest operation, the same result
+// as two scalar instructions at half the issue slots. A packed add fed by a packed multiply did not reproduce the scalar
+// bits on B200 (it behaves as contracted), so a product is written as a * b + 0: one rounding, of a * b (a product of -0 comes
+// out as +0, which no sum of a chain that starts at +0 tells apart).
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 c;
+    asm("{\n\t.reg .b64 z;\n\tmov.b64 z, 0;\n\tfma.rn.f32x2 %0, %1, %2, z;\n\t}" : "=l"(reinterpret_cast<u64&>(c)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)));
+    return c;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 c;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<u64&>(c)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)));
+    return c;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 to_float(int2 v) { return make_float2(static_cast<float>(v.x), static_cast<float>(v.y)); }
+__device__ __forceinline__ float2 pick(bool c, float2 x, float2 y) { return make_float2(c ? x.x : y.x, c ? x.y : y.y); }
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(q4k::saddr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(q4k::saddr(dst)), "l"(src) : "memory");
+}
+
+struct Tile { u32 expert, eb, nt, c, tt; };
+
+// cum[j]: token tiles of the first j experts of the union (n_union + 1 words of shared memory). Every thread of the block calls it.
+template <u32 GN>
+__device__ __forceinline__ void count_tiles(const b200moe_routes& routes, u32 n_union, u32* cum) {
+    const u32 tid = threadIdx.x, lane = tid & 31u;
+    for (u32 j = tid; j < n_union; j += blockDim.x) cum[j + 1] = (routes.begins[j + 1] - routes.begins[j] + GN - 1) / GN;
+    if (tid == 0) cum[0] = 0;
+    __syncthreads();
+    if (tid < 32) {  // inclusive scan, 32 at a time
+        u32 carry = 0;
+        for (u32 j0 = 0; j0 < n_union; j0 += 32) {
+            u32 v = j0 + lane < n_union ? cum[j0 + lane + 1] : 0u;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) { const u32 o = __shfl_up_sync(0xffffffffu, v, d); if (lane >= (u32)d) v += o; }
+            if (j0 + lane < n_union) cum[j0 + lane + 1] = carry + v;
+            carry += __shfl_sync(0xffffffffu, v, 31);
+        }
+    }
+    __syncthreads();
+}
+
+// Tile id -> (union expert, token tile, row tile): row tiles fastest, then the expert's token tiles, experts ascending.
+template <u32 GN>
+__device__ __forceinline__ Tile find_tile(const b200moe_routes& routes, u32 n_row_tiles, const u32* cum, u32 n_union, u32 id) {
+    const u32 q = id / n_row_tiles;
+    Tile t;
+    t.c = id - q * n_row_tiles;
+    u32 lo = 0, hi = n_union;  // largest j with cum[j] <= q
+    while (hi - lo > 1) {
+        const u32 mid = (lo + hi) >> 1;
+        if (cum[mid] <= q) lo = mid; else hi = mid;
+    }
+    t.tt = q - cum[lo];
+    t.expert = routes.experts[lo];
+    const u32 b0 = routes.begins[lo], b1 = routes.begins[lo + 1];
+    t.eb = b0 + GN * t.tt;
+    t.nt = min(GN, b1 - t.eb);
+    return t;
+}
+
+}  // namespace grouped
+}  // namespace b200moe

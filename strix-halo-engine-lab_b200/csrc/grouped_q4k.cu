@@ -33,11 +33,12 @@
 // Every wait is bounded; on a timeout the roles stop working and the launch sets B200MOE_JOB_WAIT_ABORTED in the job summary.
 #include <cuda.h>
 
-#include "q4k_row.cuh"
+#include "grouped_common.cuh"
 
 namespace b200moe {
 namespace {
 using namespace q4k;
+using namespace grouped;
 
 constexpr u32 kTokTiles = 2;                     // 16-token MMA tiles of a CTA tile
 constexpr u32 kRowTiles = 8;                     // 8-row MMA tiles of a consumer warp
@@ -56,7 +57,6 @@ constexpr u32 kOutBytes = kGN * kOutPitch * 4;   // epilogue tile (gate/up)
 constexpr u32 kFoldCells = kRowTiles / 2 * kTokTiles * 2;      // float2 cells of a lane that change hands when two chains meet
 constexpr u32 kFoldBytes = kConsumers * kFoldCells * 32 * 8;
 static_assert(kOutBytes <= kFoldBytes, "the epilogue tile takes the place of the buffers that the chains met in");
-constexpr u32 kMaxUnion = 1024;
 // What the consumers need of a tile: {first row, tokens, first entry}, its tokens' A8 rows, its tokens' slots. The helpers run at most
 // kStages stages ahead of the consumers, a tile has at least one stage and its places are read until its end: eight places.
 constexpr u32 kTilePlaces = 8, kTileWords = 4 + 2 * kGN;
@@ -72,35 +72,12 @@ constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kHelperRegs = 80;
 constexpr u32 kConsumerRegs = (kGThreads * kLaunchRegs - kHelpers * 32u * kHelperRegs) / (kConsumers * 32u) / 8u * 8u;
 static_assert(kConsumers * 32 * kConsumerRegs + kHelpers * 32 * kHelperRegs <= kGThreads * kLaunchRegs, "setmaxnreg split exceeds the launch's registers");
 
-// Two FP32 lanes per instruction (Blackwell packed FP32): each lane is one IEEE round-to-nearest operation, the same result
-// as two scalar instructions at half the issue slots. A packed add fed by a packed multiply did not reproduce the scalar
-// bits on B200 (it behaves as contracted), so a product is written as a * b + 0: one rounding, of a * b (a product of -0 comes
-// out as +0, which no sum of the chain tells apart).
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 c;
-    asm("{\n\t.reg .b64 z;\n\tmov.b64 z, 0;\n\tfma.rn.f32x2 %0, %1, %2, z;\n\t}" : "=l"(reinterpret_cast<u64&>(c)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)));
-    return c;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 c;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<u64&>(c)) : "l"(reinterpret_cast<const u64&>(a)), "l"(reinterpret_cast<const u64&>(b)));
-    return c;
-}
-__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 to_float(int2 v) { return make_float2(static_cast<float>(v.x), static_cast<float>(v.y)); }
 // 16 tokens x 8 weight rows x one group: signed codes times unsigned nibble bytes. d[z]: token lane / 4 + 8 z, weight rows
 // 2 (lane % 4) and the next.
 __device__ __forceinline__ void mma_dots(int2 (&d)[2], const u32 (&a)[4], u32 b0, u32 b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
         : "=r"(d[0].x), "=r"(d[0].y), "=r"(d[1].x), "=r"(d[1].y) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
 }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr(dst)), "l"(src) : "memory");
-}
-
 struct GroupedArgs {
     b200moe_shape shape;
     b200moe_routes routes;
@@ -116,26 +93,6 @@ struct GroupedArgs {
     u32 es_vec;              // the input's deltas and sums lie in whole 16-byte units
     u32 raw_vec;             // raw lies on an 8-byte boundary
 };
-
-struct Tile { u32 expert, eb, nt, c, tt; };
-
-// Tile id -> (union expert, token tile, row tile): row tiles fastest, then the expert's token tiles, experts ascending.
-__device__ __forceinline__ Tile find_tile(const GroupedArgs& a, const u32* cum, u32 n_union, u32 id) {
-    const u32 q = id / a.n_row_tiles;
-    Tile t;
-    t.c = id - q * a.n_row_tiles;
-    u32 lo = 0, hi = n_union;  // largest j with cum[j] <= q
-    while (hi - lo > 1) {
-        const u32 mid = (lo + hi) >> 1;
-        if (cum[mid] <= q) lo = mid; else hi = mid;
-    }
-    t.tt = q - cum[lo];
-    t.expert = a.routes.experts[lo];
-    const u32 b0 = a.routes.begins[lo], b1 = a.routes.begins[lo + 1];
-    t.eb = b0 + kGN * t.tt;
-    t.nt = min(kGN, b1 - t.eb);
-    return t;
-}
 
 // One super-block of the warp's 64 rows and chain against NMT 16-token tiles. rows: weight row lane / 4 of the stage at the pair's
 // nibbles of the lane's k slice; codes: token lane / 4 at the pair's codes; es: the pair's {E, E', S, S'} from token lane / 4 on; fac: the
@@ -240,25 +197,12 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
 
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const u32 n_union = min(a.routes.counts[0], kMaxUnion);
-    for (u32 j = tid; j < n_union; j += kGThreads) cum[j + 1] = (a.routes.begins[j + 1] - a.routes.begins[j] + kGN - 1) / kGN;
     if (tid == 0) {
-        cum[0] = 0;
         for (u32 i = 0; i < kStages; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&ready[i], kHelpers); mbar_init(&empty[i], kConsumers); }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();
-    if (warp == 0) {  // inclusive scan of the token-tile counts, 32 at a time
-        u32 carry = 0;
-        for (u32 j0 = 0; j0 < n_union; j0 += 32) {
-            u32 v = j0 + lane < n_union ? cum[j0 + lane + 1] : 0u;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) { const u32 o = __shfl_up_sync(0xffffffffu, v, d); if (lane >= (u32)d) v += o; }
-            if (j0 + lane < n_union) cum[j0 + lane + 1] = carry + v;
-            carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-    }
-    __syncthreads();
+    count_tiles<kGN>(a.routes, n_union, cum);
     const u32 n_tiles = cum[n_union] * a.n_row_tiles;
     const u32 I = a.shape.inter, H = a.shape.hidden;
     const u32 nblocks = a.K / 256;
@@ -281,7 +225,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
         u32 nx_src = 0, nx_slot = 0;
         auto look_ahead = [&](u32 k) {
             if (k >= my_tiles) return;
-            nx = find_tile(a, cum, n_union, blockIdx.x + k * gridDim.x);
+            nx = find_tile<kGN>(a.routes, a.n_row_tiles, cum, n_union, blockIdx.x + k * gridDim.x);
             const u32 ent = nx.eb + min(lane, nx.nt - 1u);
             nx_slot = a.routes.slots[ent];
             nx_src = kDown ? nx_slot : a.routes.rows[ent];
@@ -438,7 +382,6 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
             float2* theirs = bufs + (p ^ 1u) * (kFoldCells * 32);
             const float2* last = bufs + (p ^ 3u) * (kFoldCells * 32);
             const bool odd = p & 1u, high = p >> 1;
-            auto pick = [](bool c, float2 x, float2 y) { return make_float2(c ? x.x : y.x, c ? x.y : y.y); };
             auto add = [](float2 x, float2 y) { return make_float2(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y)); };
             constexpr int n = 2 * kTokTiles;  // cells of a row tile
             float2* cells = &acc[0][0][0];

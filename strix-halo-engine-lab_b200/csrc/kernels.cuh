@@ -65,6 +65,11 @@ bool q8_mma_gate_up_fits(const b200moe_gate_up_view& v, u32 rows);
 bool q8_mma_down_fits(const b200moe_down_view& v, u32 rows);
 int launch_gate_up_q8_mma(const b200moe_gate_up_view& v, u32 rows, cudaStream_t stream);
 int launch_down_q8_mma(const b200moe_down_view& v, u32 rows, cudaStream_t stream);
+// grouped_q8.cu: the same contract for experts with many entries, class sums in registers.
+bool grouped_q8_gate_up_fits(const b200moe_gate_up_view& v);
+bool grouped_q8_down_fits(const b200moe_down_view& v);
+int launch_gate_up_q8_grouped(const b200moe_gate_up_view& v, cudaStream_t stream);
+int launch_down_q8_grouped(const b200moe_down_view& v, cudaStream_t stream);
 // value of a B200MOE_DEBUG_* hook (api.cu)
 u32 debug_value(u32 key);
 

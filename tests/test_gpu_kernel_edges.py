@@ -160,6 +160,30 @@ def test_q8_entry_blocks(gpu, oracle, tokens):
     assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
 
 
+@pytest.mark.parametrize("tokens,H,I", [(1, 256, 512), (15, 512, 768), (16, 768, 256), (17, 1024, 1280), (32, 1280, 1024), (33, 2304, 256), (64, 7424, 256)])
+def test_q8_grouped_units(gpu, oracle, tokens, H, I):
+    """The grouped Q8_0 form: rows of 1 to 29 units (empty sets, sets of unequal length), token tiles with one and with two halves."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(tokens + H)
+    E, rows = 2, 50 + tokens
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 8, 8)
+    ids = np.zeros((rows, 1), np.uint32)
+    ids[rng.permutation(rows)[:tokens]] = 1
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, 1, 8, 8)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    import b200moe
+    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, 5)
+    try:
+        act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
+        raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+    finally:
+        b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_AUTO)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    assert same(raw.cpu(), want["raw"])
+
+
 def declared_logits(x, w):
     """Lane class l sums products l, l + 32, ... ascending; the classes fold by the butterfly (src/ds41_moe.cpp:72-82)."""
     acc = np.zeros((x.shape[0], w.shape[0], 32), np.float32)

@@ -25,8 +25,10 @@
 //    bytes, high nibbles left in place as 16 q; the k order inside a group is permuted the same way on both sides, which
 //    an exact integer sum does not see). The accumulator fragment gives lane (entry, t) the dots of rows 2t and 2t + 1,
 //    and the lane runs the same FP32 operation sequence on them with the rows' factors fetched from a per-warp scratch:
-//    the kernel is bound by issue slots (ncu: three quarters of them busy at config 4), and this form needs about half
-//    the instructions of the dp4a form at 8 entries; from 3 or 4 entries on it was measured slower than dp4a. Both forms produce the contract's bits.
+//    the kernel is bound by issue slots, and at 8 entries this form needs a third of the dp4a form's instructions. It takes over at
+//    5 entries: 64 rows of the large layer (256 experts of 7168 -> 2048, 4.4 entries each) took 876 us a call with that line, 888 with 4, 909
+//    with 3, 967 with 2. Both forms run two cells a packed FP32 instruction (two rows, or two entries) and produce the contract's bits;
+//    with scalar operations and dots converted by addition the call took 930 us.
 //
 // Every wait is bounded (plan.wait_limit polls): a waiter that runs out raises the CTA's abort flag, every role leaves
 // its loops, the producers wait (bounded) for the copies they still have in flight, B200MOE_JOB_WAIT_ABORTED is set in the
@@ -36,6 +38,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "grouped_common.cuh"
 #include "wide_common.cuh"
 
 namespace b200moe {
@@ -43,10 +46,11 @@ namespace b200moe {
 namespace {
 using namespace q4k;
 using namespace wide;
+using namespace grouped;  // packed FP32
 
 constexpr u32 kItemRows = 64;
 constexpr u32 kMmaMinEntries = 5;                       // items with at least this many entries take the mma form
-constexpr u32 kFacFloats = 128;                         // per-warp scratch of the mma form: [D, DM, D', DM'][pair][row]
+constexpr u32 kFacPitch = 36, kFacFloats = 4 * kFacPitch;  // per-warp scratch of the mma form: floats of a pair (a lane's store: 2 ways a bank)
 
 struct WidePlan {
     u32 S;              // super-blocks per stage
@@ -98,6 +102,17 @@ __device__ __forceinline__ float tree4(float a) {
     return __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 16));
 }
 
+// Decoded factors of one super-block for pair p as the chains use them: D of the even group, D / 16 of the odd one (the high nibbles stay in
+// place: their dots come as 16 * dot), and -DM of both. A scale's byte goes behind the exponent of 2^23, less 2^23.
+__device__ __forceinline__ float4 pair_factors(const uint4& hdr, u32 p) {
+    const float d = half_bits_to_float(hdr.x & 0xffffu), dm = -half_bits_to_float(hdr.x >> 16);
+    const u32 sc = p < 2u ? hdr.y & 0x3f3f3f3fu : (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
+    const u32 mn = p < 2u ? hdr.z & 0x3f3f3f3fu : ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
+    const u32 sel = 0x7440u + 2u * (p & 1u);
+    auto byte = [](u32 w, u32 s) { return __fsub_rn(__uint_as_float(__byte_perm(w, 0x4b000000u, s)), 8388608.0f); };
+    return make_float4(__fmul_rn(d, byte(sc, sel)), __fmul_rn(__fmul_rn(d, 0.0625f), byte(sc, sel + 1u)), __fmul_rn(dm, byte(mn, sel)), __fmul_rn(dm, byte(mn, sel + 1u)));
+}
+
 // One stage of one weight row (this lane's pair p of nbk super-blocks, ascending) against NR staged A8 rows. blk: the
 // row's first super-block of the stage; xs: entry 0's area of the stage ({codes[S * 256], deltas[S * 8], sums[S * 8]},
 // the next entry x_entry_bytes further). acc[r] is the lane's chain acc_p of entry r.
@@ -108,52 +123,67 @@ __device__ __forceinline__ void stage_rows(const uint4* blk, u32 nbk, u32 p, con
     for (u32 b = 0; b < S; ++b, blk += kQ4KBlock / 16) {
         if (b >= nbk) break;
         const uint4 hdr = blk[0], q0 = blk[1 + 2 * p], q1 = blk[2 + 2 * p];
-        const Factors f = q4k_factors(hdr, p);
+        const float4 f = pair_factors(hdr, p);
         const Nibbles n = split_nibbles(q0, q1);
+        float lo[NR], hi[NR];
+        float2 e[NR], sm[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             const unsigned char* xe = xs + r * x_entry_bytes;
             const uint4* c = reinterpret_cast<const uint4*>(xe + 256u * b + 64u * p);
             const uint4 c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
-            const float2 e = *reinterpret_cast<const float2*>(xe + 256u * S + 32u * b + 8u * p);
-            const int2 sm = *reinterpret_cast<const int2*>(xe + 288u * S + 32u * b + 8u * p);
-            int lo, hi;
-            dots(n, c0, c1, c2, c3, &lo, &hi);
-            acc[r] = __fadd_rn(acc[r], pair_value(f, lo, hi, e.x, e.y, small_int_to_float(sm.x), small_int_to_float(sm.y)));
+            e[r] = *reinterpret_cast<const float2*>(xe + 256u * S + 32u * b + 8u * p);
+            sm[r] = to_float(*reinterpret_cast<const int2*>(xe + 288u * S + 32u * b + 8u * p));
+            int l, h;
+            dots(n, c0, c1, c2, c3, &l, &h);
+            lo[r] = static_cast<float>(l); hi[r] = static_cast<float>(h);
+        }
+        // x = E * ((D * float(dot)) - (DM * S)) for the pair's two groups; f holds -DM, and (-DM) * S = -(DM * S) exactly
+#pragma unroll
+        for (int r = 0; r + 1 < NR; r += 2) {  // two entries an instruction
+            const float2 sl = add2(mul2(both(f.x), make_float2(lo[r], lo[r + 1])), mul2(both(f.z), make_float2(sm[r].x, sm[r + 1].x)));
+            const float2 sh = add2(mul2(both(f.y), make_float2(hi[r], hi[r + 1])), mul2(both(f.w), make_float2(sm[r].y, sm[r + 1].y)));
+            const float2 x = add2(mul2(make_float2(e[r].x, e[r + 1].x), sl), mul2(make_float2(e[r].y, e[r + 1].y), sh));
+            acc[r] = __fadd_rn(acc[r], x.x);
+            acc[r + 1] = __fadd_rn(acc[r + 1], x.y);
+        }
+        if (NR & 1) {
+            constexpr int r = NR - 1;
+            const float sl = __fadd_rn(__fmul_rn(f.x, lo[r]), __fmul_rn(f.z, sm[r].x)), sh = __fadd_rn(__fmul_rn(f.y, hi[r]), __fmul_rn(f.w, sm[r].y));
+            acc[r] = __fadd_rn(acc[r], __fadd_rn(__fmul_rn(e[r].x, sl), __fmul_rn(e[r].y, sh)));
         }
     }
 }
 // ---- the mma form of one stage ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void mma_s8u8(int& c0, int& c1, u32 a0, u32 a2, u32 b0, u32 b1) {
+__device__ __forceinline__ int2 mma_s8u8(u32 a0, u32 a2, u32 b0, u32 b1) {
     // D (16 x 8, s32) = A (16 x 32, s8, row) * B (32 x 8, u8, col); rows 8 .. 15 of A are zero (at most 8 entries).
+    int2 c;
     int c2, c3;
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-                 : "=r"(c0), "=r"(c1), "=r"(c2), "=r"(c3)
+                 : "=r"(c.x), "=r"(c.y), "=r"(c2), "=r"(c3)
                  : "r"(a0), "r"(0), "r"(a2), "r"(0), "r"(b0), "r"(b1), "r"(0));
-}
-// x_2p + x_2p+1 of one (row, entry, super-block, pair) from the two exact group dots; hi16 = 16 * dot of the odd group.
-__device__ __forceinline__ float pair_from_dots(float Dl, float DMl, float Dh, float DMh, int lo, int hi16, float El, float Eh, float Sl, float Sh) {
-    const float xl = __fmul_rn(El, __fsub_rn(__fmul_rn(Dl, static_cast<float>(lo)), __fmul_rn(DMl, Sl)));
-    const float xh = __fmul_rn(Eh, __fsub_rn(__fmul_rn(Dh, static_cast<float>(hi16 >> 4)), __fmul_rn(DMh, Sh)));
-    return __fadd_rn(xl, xh);
+    return c;
 }
 // One stage of the warp's 8 weight rows against up to 8 staged A8 rows with tensor-core dots. w8: the warp's first row of
-// the stage (rows row_seg_bytes apart); fac: the warp's scratch. Lane = (e = lane >> 2, t = lane & 3): acc[4 * i + p] is the
-// chain acc_p of (row 2t + i, entry e). Lanes of absent entries compute on stale shared memory and are never stored.
+// the stage (rows row_seg_bytes apart); fac: the warp's scratch. Lane = (e = lane >> 2, t = lane & 3): acc[p] holds the
+// chains acc_p of rows 2t and 2t + 1 with entry e. Lanes of absent entries compute on stale shared memory and are never stored.
+// The two rows share every instruction: 27 a (pair, two rows) where scalar operations, conversions by addition and shifts took 43.
 template <class G>
-__device__ __forceinline__ void stage_rows_mma(const unsigned char* w8, u32 nbk, u32 lane, const unsigned char* xs, float* fac, float* acc) {
+__device__ __forceinline__ void stage_rows_mma(const unsigned char* w8, u32 nbk, u32 lane, const unsigned char* xs, float* fac, float2 (&acc)[4]) {
     constexpr u32 row_seg_bytes = G::row_seg_bytes, x_entry_bytes = G::x_entry_bytes, S = G::S;
     const u32 p = lane >> 3, rr = lane & 7u;   // factor decode: lane = (pair, row), as in the dp4a form
     const u32 e = lane >> 2, t = lane & 3u;    // mma fragments: lane = (entry or weight row, k slice)
     const unsigned char* xe = xs + e * x_entry_bytes;
     const unsigned char* wdec = w8 + rr * row_seg_bytes;
     const unsigned char* wfrag = w8 + e * row_seg_bytes + 16u + 8u * t;   // B fragment: weight row n = lane >> 2
+    float* put = fac + kFacPitch * p + 8u * (rr >> 1) + (rr & 1u);        // [pair][row pair][D, D, D', D' | -DM, -DM, -DM', -DM']
+    const float4* get = reinterpret_cast<const float4*>(fac + 8u * t);
 #pragma unroll 1
     for (u32 b = 0; b < nbk; ++b) {  // rolled: the body is long, and the form runs where the instruction cache matters
         const uint4 hdr = *reinterpret_cast<const uint4*>(wdec + kQ4KBlock * b);
-        const Factors f = q4k_factors(hdr, p);
+        const float4 f = pair_factors(hdr, p);
         __syncwarp();   // the previous block's readers are done with the scratch
-        fac[(0 * 4 + p) * 8 + rr] = f.Dl; fac[(1 * 4 + p) * 8 + rr] = f.DMl; fac[(2 * 4 + p) * 8 + rr] = f.Dh; fac[(3 * 4 + p) * 8 + rr] = f.DMh;  // bank = lane
+        put[0] = f.x; put[2] = f.y; put[4] = f.z; put[6] = f.w;
         __syncwarp();
         const float4 e0 = *reinterpret_cast<const float4*>(xe + 256u * S + 32u * b), e1 = *reinterpret_cast<const float4*>(xe + 256u * S + 32u * b + 16u);
         const int4 s0 = *reinterpret_cast<const int4*>(xe + 288u * S + 32u * b), s1 = *reinterpret_cast<const int4*>(xe + 288u * S + 32u * b + 16u);
@@ -164,15 +194,13 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* w8, u32 nbk,
             const uint2 w = *reinterpret_cast<const uint2*>(wfrag + kQ4KBlock * b + 32u * pp);   // 8 bytes = 16 nibbles: k slice t of groups 2pp, 2pp + 1
             const uint2 al = *reinterpret_cast<const uint2*>(xe + 256u * b + 64u * pp + 8u * t);          // the entry's codes, group 2pp, same k slice
             const uint2 ah = *reinterpret_cast<const uint2*>(xe + 256u * b + 64u * pp + 32u + 8u * t);    // group 2pp + 1
-            int l0, l1, h0, h1;
-            mma_s8u8(l0, l1, al.x, al.y, w.x & 0x0f0f0f0fu, w.y & 0x0f0f0f0fu);
-            mma_s8u8(h0, h1, ah.x, ah.y, w.x & 0xf0f0f0f0u, w.y & 0xf0f0f0f0u);
-            const float El = E[2 * pp], Eh = E[2 * pp + 1];
-            const float Sl = small_int_to_float(Sg[2 * pp]), Sh = small_int_to_float(Sg[2 * pp + 1]);
-            const float2 Dl = *reinterpret_cast<const float2*>(fac + (0 * 4 + pp) * 8 + 2 * t), DMl = *reinterpret_cast<const float2*>(fac + (1 * 4 + pp) * 8 + 2 * t);
-            const float2 Dh = *reinterpret_cast<const float2*>(fac + (2 * 4 + pp) * 8 + 2 * t), DMh = *reinterpret_cast<const float2*>(fac + (3 * 4 + pp) * 8 + 2 * t);
-            acc[pp] = __fadd_rn(acc[pp], pair_from_dots(Dl.x, DMl.x, Dh.x, DMh.x, l0, h0, El, Eh, Sl, Sh));
-            acc[4 + pp] = __fadd_rn(acc[4 + pp], pair_from_dots(Dl.y, DMl.y, Dh.y, DMh.y, l1, h1, El, Eh, Sl, Sh));
+            const float4 d4 = get[kFacPitch / 4 * pp], m4 = get[kFacPitch / 4 * pp + 1];
+            const float2 l = to_float(mma_s8u8(al.x, al.y, w.x & 0x0f0f0f0fu, w.y & 0x0f0f0f0fu));
+            const float2 h = to_float(mma_s8u8(ah.x, ah.y, w.x & 0xf0f0f0f0u, w.y & 0xf0f0f0f0u));
+            const float Sl = static_cast<float>(Sg[2 * pp]), Sh = static_cast<float>(Sg[2 * pp + 1]);
+            const float2 sl = add2(mul2(make_float2(d4.x, d4.y), l), mul2(make_float2(m4.x, m4.y), both(Sl)));
+            const float2 sh = add2(mul2(make_float2(d4.z, d4.w), h), mul2(make_float2(m4.z, m4.w), both(Sh)));
+            acc[pp] = add2(add2(mul2(both(E[2 * pp]), sl), mul2(both(E[2 * pp + 1]), sh)), acc[pp]);
         }
     }
 }
@@ -317,9 +345,12 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         const VExpert ve = table[jv];
         const u32 ne = ve.ne(), vbegin = ve.begin();
         const bool mma = ne >= kMmaMinEntries;
-        float acc[kKE];
+        float acc[kMmaMinEntries - 1];
+        float2 acc2[4];  // mma form
 #pragma unroll
-        for (int r = 0; r < (int)kKE; ++r) acc[r] = 0.0f;
+        for (int r = 0; r < (int)kMmaMinEntries - 1; ++r) acc[r] = 0.0f;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc2[r] = make_float2(0.0f, 0.0f);
         // the item's stages, with the form and the entry count fixed at compile time inside the loop (NR = 0: the mma form)
         auto run = [&](auto tag) {
             constexpr int NR = decltype(tag)::value;
@@ -331,7 +362,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 }
                 const unsigned char* st = g_stage + slot * plan.stage_bytes;
                 const u32 nbk = min(G::S, plan.nb - s * G::S);
-                if constexpr (NR == 0) stage_rows_mma<G>(st + 8u * w * G::row_seg_bytes, nbk, lane, st + G::w_bytes, fac, acc);
+                if constexpr (NR == 0) stage_rows_mma<G>(st + 8u * w * G::row_seg_bytes, nbk, lane, st + G::w_bytes, fac, acc2);
                 else stage_rows<NR, G>(reinterpret_cast<const uint4*>(st + (8u * w + rr) * G::row_seg_bytes), nbk, p, st + G::w_bytes, acc);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&g_empty[slot]);  // the stage is free for the producer
@@ -347,8 +378,8 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         }
         if (!ok) break;
         // mma form: lane (e = lane >> 2, t = lane & 3) holds the four chains of rows 2t and 2t + 1 of entry e
-        const float m0 = __fadd_rn(__fadd_rn(acc[0], acc[1]), __fadd_rn(acc[2], acc[3]));
-        const float m1 = __fadd_rn(__fadd_rn(acc[4], acc[5]), __fadd_rn(acc[6], acc[7]));
+        const float m0 = __fadd_rn(__fadd_rn(acc2[0].x, acc2[1].x), __fadd_rn(acc2[2].x, acc2[3].x));
+        const float m1 = __fadd_rn(__fadd_rn(acc2[0].y, acc2[1].y), __fadd_rn(acc2[2].y, acc2[3].y));
         const u32 me = lane >> 2, mt = lane & 3u;
         if (DOWN) {
             if (mma) {

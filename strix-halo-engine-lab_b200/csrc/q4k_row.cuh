@@ -98,26 +98,19 @@ __device__ __forceinline__ Nibbles split_nibbles(const uint4& q0, const uint4& q
     return n;
 }
 // Exact group dots: two interleaved chains of four for each group (integer sums are order free). c0, c1: the 32 codes of
-// group 2p; c2, c3: those of group 2p + 1.
+// group 2p; c2, c3: those of group 2p + 1, whose dot comes as 16 * dot.
 __device__ __forceinline__ void dots(const Nibbles& n, const uint4& c0, const uint4& c1, const uint4& c2, const uint4& c3, int* lo, int* hi) {
     int la = __dp4a(static_cast<int>(n.lo[0]), static_cast<int>(c0.x), 0), lb = __dp4a(static_cast<int>(n.lo[1]), static_cast<int>(c0.y), 0);
     la = __dp4a(static_cast<int>(n.lo[2]), static_cast<int>(c0.z), la); lb = __dp4a(static_cast<int>(n.lo[3]), static_cast<int>(c0.w), lb);
     la = __dp4a(static_cast<int>(n.lo[4]), static_cast<int>(c1.x), la); lb = __dp4a(static_cast<int>(n.lo[5]), static_cast<int>(c1.y), lb);
     la = __dp4a(static_cast<int>(n.lo[6]), static_cast<int>(c1.z), la); lb = __dp4a(static_cast<int>(n.lo[7]), static_cast<int>(c1.w), lb);
-    // bytes 16 * q (unsigned) times signed codes = 16 * dot, an exact shift away
+    // bytes 16 * q (unsigned) times signed codes = 16 * dot
     int ha = dp4a_us(n.hi[0], c2.x, 0), hb = dp4a_us(n.hi[1], c2.y, 0);
     ha = dp4a_us(n.hi[2], c2.z, ha); hb = dp4a_us(n.hi[3], c2.w, hb);
     ha = dp4a_us(n.hi[4], c3.x, ha); hb = dp4a_us(n.hi[5], c3.y, hb);
     ha = dp4a_us(n.hi[6], c3.z, ha); hb = dp4a_us(n.hi[7], c3.w, hb);
     *lo = la + lb;
-    *hi = (ha + hb) >> 4;
+    *hi = ha + hb;
 }
-// x_2p + x_2p+1 with x_j = E_g * (D_j * float(dot_j) - DM_j * float(S_g)).
-__device__ __forceinline__ float pair_value(const Factors& f, int lo, int hi, float El, float Eh, float Sl, float Sh) {
-    const float xl = __fmul_rn(El, __fsub_rn(__fmul_rn(f.Dl, small_int_to_float(lo)), __fmul_rn(f.DMl, Sl)));
-    const float xh = __fmul_rn(Eh, __fsub_rn(__fmul_rn(f.Dh, small_int_to_float(hi)), __fmul_rn(f.DMh, Sh)));
-    return __fadd_rn(xl, xh);
-}
-
 }  // namespace q4k
 }  // namespace b200moe

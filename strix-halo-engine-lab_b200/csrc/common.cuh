@@ -70,10 +70,12 @@ __device__ __forceinline__ float half_bits_to_float(u32 h) {  // exact for every
     return __half2float(__ushort_as_half(static_cast<unsigned short>(h)));
 }
 __device__ __forceinline__ bool finite_f(float x) { return (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u; }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int d = 16; d; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
-    return v;
+// The largest of a warp's magnitudes; a NaN is left out, as std::max(amax, |x|) leaves it out, unless there is nothing else. The bits of
+// magnitudes order as they do, so one reduction instruction does it.
+__device__ __forceinline__ float warp_max_abs(float x) {
+    const bool nan = x != x;
+    const u32 m = __reduce_max_sync(0xffffffffu, nan ? 0u : __float_as_uint(x) & 0x7fffffffu);
+    return __all_sync(0xffffffffu, nan) ? __uint_as_float(0x7fffffffu) : __uint_as_float(m);
 }
 __device__ __forceinline__ int warp_sum_i(int v) {
     return __reduce_add_sync(0xffffffffu, v);
@@ -88,7 +90,7 @@ __device__ __forceinline__ float butterfly32(float v) {
 // One A8 group of 32 values held one per lane (src/cpu/core/reference.cpp:35-55). Returns the code; delta and sum
 // are the same in every lane.
 __device__ __forceinline__ int a8_quantize_lane(float x, float* delta_out, int* sum_out) {
-    const float amax = warp_max(fabsf(x));  // NaN operands are ignored, as std::max(amax, |x|) ignores them
+    const float amax = warp_max_abs(x);
     const bool tiny = amax > 0.0f && amax < 0x1p-119f;
     const float delta = (amax == 0.0f || tiny) ? 1.0f : __fdiv_rn(amax, 127.0f);
     const float r = tiny ? 0.0f : rintf(__fdiv_rn(x, delta));

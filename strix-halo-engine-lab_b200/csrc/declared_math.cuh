@@ -10,11 +10,9 @@ __device__ __forceinline__ float pow2i(int k) { return __uint_as_float(static_ca
 // exp(x) from basic IEEE operations (include/strix/ds41_moe.hpp:38-54): Cody-Waite reduction by ln 2, degree-7 Taylor
 // polynomial in Horner form with separate multiply and add, two-step power-of-two scaling.
 __device__ __forceinline__ float declared_exp(float x) {
-    if (!(x == x)) return x;
-    if (x > 88.0f) return __uint_as_float(0x7f800000u);
-    if (x < -103.0f) return 0.0f;
-    const float n = rintf(__fmul_rn(x, 1.44269504f));
-    const float r = __fsub_rn(__fsub_rn(x, __fmul_rn(n, 0.693359375f)), __fmul_rn(n, -2.12194440e-4f));
+    const float c = fminf(fmaxf(x, -104.0f), 89.0f);  // selects at the end replace the cases, so that several evaluations overlap
+    const float n = rintf(__fmul_rn(c, 1.44269504f));
+    const float r = __fsub_rn(__fsub_rn(c, __fmul_rn(n, 0.693359375f)), __fmul_rn(n, -2.12194440e-4f));
     float p = 1.98412698e-4f;
     p = __fadd_rn(__fmul_rn(p, r), 1.38888889e-3f);
     p = __fadd_rn(__fmul_rn(p, r), 8.33333333e-3f);
@@ -24,7 +22,10 @@ __device__ __forceinline__ float declared_exp(float x) {
     p = __fadd_rn(__fmul_rn(p, r), 1.0f);
     p = __fadd_rn(__fmul_rn(p, r), 1.0f);
     const int k = static_cast<int>(n), k1 = k / 2, k2 = k - k1;
-    return __fmul_rn(__fmul_rn(p, pow2i(k1)), pow2i(k2));
+    float f = __fmul_rn(__fmul_rn(p, pow2i(k1)), pow2i(k2));
+    if (x > 88.0f) f = __uint_as_float(0x7f800000u);
+    if (x < -103.0f) f = 0.0f;
+    return x == x ? f : x;
 }
 // ln of a positive normal float (include/strix/ds41_moe.hpp:65-79).
 __device__ __forceinline__ float declared_log(float y) {
@@ -61,26 +62,12 @@ __device__ __forceinline__ float swiglu_ds41(float gate, float up, float limit) 
 
 // gfx1151 expf twin at zero correction tables (src/cpu/core/routed_expert.cpp:208-261): Cody-Waite split of
 // x * log2(e) with two fused steps, v_exp(a) = float(exp2(double(a))) for |a| < 1, scaled by 2^e.
-// The host evaluates exp2 in double with the C library; the device's double exp2 differs from it by at most one
-// double ulp, which changes the rounded float only when the double lands within 2^-29 of a float rounding boundary.
+// The host evaluates exp2 in double with the C library; a double within an ulp or two of it changes the rounded float only when it lands
+// within 2^-29 of a float rounding boundary. 2^a is its series in a ln 2 (degree 13: the remainder for |a| <= 0.51 is 2^-57), 2^e comes in
+// two steps, as a subnormal result is then rounded once. Selects replace the cases: outside the two limits e and a are not meaningful and
+// not used, a NaN passes through. Equal to the form with CUDA's exp2(double), scalbnf and branches for every one of the 2^32 floats; that
+// form's calls kept several evaluations of a warp from overlapping: 551 clocks each where this one takes a third of the instructions.
 __device__ __forceinline__ float gfx1151_expf(float x) {
-    const float kLog2e = __uint_as_float(0x3fb8aa3bu), kLog2eLo = __uint_as_float(0x32a5705fu);
-    const float ph = __fmul_rn(x, kLog2e);
-    const float e = rintf(ph);
-    float pl = __fmaf_rn(x, kLog2e, -ph);
-    pl = __fmaf_rn(x, kLog2eLo, pl);
-    const float a = __fadd_rn(__fsub_rn(ph, e), pl);
-    float y;
-    if (fabsf(a) < 1.0f) y = scalbnf(static_cast<float>(exp2(static_cast<double>(a))), static_cast<int>(e));
-    else y = a != a ? a : 0.0f;
-    if (__uint_as_float(0xc2ce8ed0u) > x) y = 0.0f;
-    if (__uint_as_float(0x42b17218u) < x) y = __uint_as_float(0x7f800000u);
-    return y;
-}
-// The same function without a branch, for callers that run several at once: the same reduction; 2^a by its series in a ln 2 (degree 13:
-// the remainder for |a| <= 0.51 is 2^-57); 2^e in two steps, as a subnormal result
-// is then rounded once. Selects replace the cases: outside the two limits e and a are not meaningful and not used, a NaN passes through.
-__device__ __forceinline__ float gfx1151_expf_straight(float x) {
     const float kLog2e = __uint_as_float(0x3fb8aa3bu), kLog2eLo = __uint_as_float(0x32a5705fu);
     const float ph = __fmul_rn(x, kLog2e);
     const float big = __fadd_rn(ph, 12582912.0f), e = __fsub_rn(big, 12582912.0f);  // rint for |ph| < 2^22, its integer in big's low bits

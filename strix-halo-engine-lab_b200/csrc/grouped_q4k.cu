@@ -144,7 +144,7 @@ __device__ __forceinline__ u32 swiglu_a8(const float (&g)[kTasks], const float (
     float h[kTasks], x[kTasks];
     u32 bad = 0, amax[kTasks];
 #pragma unroll
-    for (int i = 0; i < kTasks; ++i) x[i] = gfx1151_expf_straight(-g[i]);
+    for (int i = 0; i < kTasks; ++i) x[i] = gfx1151_expf(-g[i]);
 #pragma unroll
     for (int i = 0; i < kTasks; ++i) {
         h[i] = __fmul_rn(__fdiv_rn(g[i], __fadd_rn(1.0f, x[i])), u[i]);  // swiglu_qwen (declared_math.cuh)

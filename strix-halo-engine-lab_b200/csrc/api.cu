@@ -231,16 +231,21 @@ cudaError_t clear_status(const LayerScratch& L, bool with_row_status, u32 rows, 
 
 // Plan by window size, chosen on the host from the row count (no environment reads inside numerical code): decode
 // windows of Q4_K experts take the persistent bulk-copy form, everything else the plain per-block form.
-// grouped_min_rows: 0 = the default threshold; windows of at least that many rows take the grouped form.
-// What decides is the number of entries an expert has (the grouped form's tiles hold 48, a streaming item 8), and rows only stand
-// for it: whole calls, streaming against grouped, cross between 160 and 192 rows with 8 of 128 experts of 2048 x 768 (221 and 263 us at 128
-// rows, 264 and 276 at 160, 296 and 281 at 192), between 96 and 128 rows with 6 of 60 experts of 4096 x 1536 (367 and 414, 454 and 442), above
-// 384 with 2 of 160 experts of 1024 x 512 (134 and 152), and already between 24 and 32 rows in a dense block of 5120 x 17408
-// (177 and 218, 246 and 222; 784 and 423 at 128). 128 lies in the middle of these.
-constexpr u32 kGroupedDefaultRows = 128;
-bool use_grouped(const b200moe_shape& s, u32 rows, u32 grouped_min_rows, bool have_sums) {
-    const u32 least = grouped_min_rows ? grouped_min_rows : kGroupedDefaultRows;
-    return rows >= least && grouped_fits(s, have_sums);
+// grouped_min_rows: 0 = chosen here; windows of at least that many rows take the grouped form.
+// What decides is the number of entries an expert has (the grouped form's tiles hold 32, a streaming item 8), and that there is work for
+// its latency. Whole calls, streaming against grouped: 128 experts of 2048 x 768 215 and 231 us with 8 entries, 256 and 242 with 10, 342 and
+// 268 with 16; 60 of 4096 x 1536 350 and 363 with 9.6, 432 and 378 with 12.8; 160 of 1024 x 512 150 and 161 with 6.4, 192 and 176 with 9.6;
+// 64 of 7168 x 2048 675 and 750 with 8, 909 and 832 with 12; 32 of 1536 x 1024 98 and 101 us with 32 rows (8 entries), 127 and 114 with 64.
+// One expert (a dense block): 5120 x 17408 179 and 227 us with 24 rows, 242 and 226 with 32, 427 and 268 with 64; 7168 x 18432 273 and 266,
+// 319 and 264, 580 and 321; 3584 x 14336 152 and 182 with 32 rows, 264 and 212 with 64; 2048 x 8192 104 and 119 with 64, 163 and 135 with 100.
+// Where the segment-streaming form does not apply (more than 8192 slots, rows that bulk copies cannot take) the alternative is the
+// per-block form, and 128 rows are the line.
+constexpr u32 kGroupedEntries = 9, kGroupedRows = 64, kGroupedRowsWide = 32, kGroupedWideInter = 16384, kGroupedRowsElse = 128;
+bool use_grouped(const b200moe_shape& s, u32 rows, u32 grouped_min_rows, bool have_sums, bool streams) {
+    if (!grouped_fits(s, have_sums)) return false;
+    if (grouped_min_rows) return rows >= grouped_min_rows;
+    if (!streams) return rows >= kGroupedRowsElse;
+    return u64(rows) * s.top_k >= u64(kGroupedEntries) * s.experts && rows >= (s.inter >= kGroupedWideInter ? kGroupedRowsWide : kGroupedRows);
 }
 // Decode forms of the Q4_K GEMVs: windows of one or two rows over rows of up to kRowStreamK weights take the row-streaming
 // form (a ring of whole rows, its work split fixed per CTA), everything else the segment-streaming form (any row length;
@@ -295,17 +300,19 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
         }
     }
     if (v.shape.gate_type == B200MOE_TYPE_Q5_K) return launch_gate_up_q4k(v, st);  // the per-block form reads both K-quant layouts
-    if (use_grouped(v.shape, rows, grouped_min_rows, v.x.sums != nullptr)) return launch_gate_up_q4k_grouped(v, st);
-    switch (pick_decode_form(stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, v.shape.hidden)) {
+    const bool wide_fits = wide_gate_up_fits(v, rows);
+    if (use_grouped(v.shape, rows, grouped_min_rows, v.x.sums != nullptr, wide_fits)) return launch_gate_up_q4k_grouped(v, st);
+    switch (pick_decode_form(stream_gate_up_fits(v, rows), wide_fits, rows, v.shape.hidden)) {
         case DecodeForm::row_stream: return launch_gate_up_q4k_stream(v, rows, st);
         case DecodeForm::wide: return launch_gate_up_q4k_wide(v, rows, st);
         default: return launch_gate_up_q4k(v, st);
     }
 }
 int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0) {
-    if (v.shape.down_type == B200MOE_TYPE_Q4_K && use_grouped(v.shape, rows, grouped_min_rows, v.act.sums != nullptr)) return launch_down_q4k_grouped(v, st);
     if (v.shape.down_type == B200MOE_TYPE_Q4_K) {
-        switch (pick_decode_form(stream_down_fits(v, rows), wide_down_fits(v, rows), rows, v.shape.inter)) {
+        const bool wide_fits = wide_down_fits(v, rows);
+        if (use_grouped(v.shape, rows, grouped_min_rows, v.act.sums != nullptr, wide_fits)) return launch_down_q4k_grouped(v, st);
+        switch (pick_decode_form(stream_down_fits(v, rows), wide_fits, rows, v.shape.inter)) {
             case DecodeForm::row_stream: return launch_down_q4k_stream(v, rows, st);
             case DecodeForm::wide: return launch_down_q4k_wide(v, rows, st);
             default: return launch_down_q4k(v, st);

@@ -85,6 +85,23 @@ def test_grouped_row_tiles_of_a_share(gpu, oracle, tokens, H, I, scale, special)
     assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, 4, act).cpu(), want["raw"])
 
 
+@pytest.mark.parametrize("rows,top_k,E,I", [(63, 1, 1, 512), (64, 1, 1, 512), (71, 2, 16, 256), (72, 2, 16, 256), (31, 1, 1, 16384), (32, 1, 1, 16384), (140, 1, 20, 256)])
+def test_grouped_form_lines(gpu, oracle, rows, top_k, E, I):
+    """Both sides of the lines between the streaming and the grouped Q4_K form: 64 rows (32 of a wide block), nine entries an expert."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows)
+    H = 256
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, 12, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, top_k, 12, 12)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
+
+
 @pytest.mark.parametrize("bits", [0x7c00, 0xfc00, 0x7e00])
 def test_grouped_factor_not_finite(gpu, oracle, bits):
     """A down row whose super-block factor is an infinity or a NaN: the term is d * dot, not what is left of (M + dot) - M."""

@@ -121,6 +121,36 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
     }
 }
 
+// The slot-order form over whole rows with up to kVecTopK slots and even rows: two outputs a thread, and every word that the thread reads - the
+// row's status, the job's summary, weights, values - is asked for before any of them is looked at: a small window is a chain of
+// memory latencies (three in the general form, with two block barriers between them), a large one wants bytes in flight.
+// 4096 rows x 8 x 2048: 79 us in the general form, 60 here (5.0 TB/s); 8 rows 3.1 and 2.2; 37 rows 4.0 and 2.8.
+__global__ void __launch_bounds__(128) combine_slots_kernel(b200moe_combine_view v) {
+    const u32 o = 2u * (blockIdx.x * 128u + threadIdx.x);
+    if (o >= v.hidden) return;
+    const u32 job = v.summary ? __ldg(v.summary) : 0u;
+    for (u32 row = blockIdx.y; row < v.rows; row += gridDim.y) {
+        const u32 status = v.row_status ? __ldg(v.row_status + row) : 0u;
+        float2 x[kVecTopK];
+        float w[kVecTopK];
+#pragma unroll
+        for (u32 k = 0; k < kVecTopK; ++k)
+            if (k < v.top_k) {
+                x[k] = __ldg(reinterpret_cast<const float2*>(v.raw + (u64(row) * v.top_k + k) * v.hidden + o));
+                w[k] = __ldg(v.weights + row * v.top_k + k);
+            }
+        const float2 sh = v.shared ? __ldg(reinterpret_cast<const float2*>(v.shared + u64(row) * v.hidden + o)) : make_float2(0.0f, 0.0f);
+        float2 y = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (u32 k = 0; k < kVecTopK; ++k)
+            if (k < v.top_k) y = make_float2(__fmaf_rn(w[k], x[k].x, y.x), __fmaf_rn(w[k], x[k].y, y.y));
+        if (v.shared) y = make_float2(__fadd_rn(y.x, sh.x), __fadd_rn(y.y, sh.y));
+        if (job & B200MOE_JOB_WAIT_ABORTED) return;  // an aborted stage left raw partly unwritten
+        if (status) continue;                        // fail closed (qwen_moe.cu:291)
+        *reinterpret_cast<float2*>(v.y + u64(row) * v.hidden + o) = y;
+        if (v.y_bf16) *reinterpret_cast<u32*>(v.y_bf16 + u64(row) * v.hidden + o) = bf16_rne_bits(y.x) | (u32(bf16_rne_bits(y.y)) << 16);
+    }
+}
 __global__ void __launch_bounds__(256) canonical_sum_kernel(const float* a, const float* b, const float* c, u64 count, float* y) {
     const u64 i = u64(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= count) return;
@@ -163,14 +193,16 @@ int launch_merge_first_error(b200moe_first_error* record, const u32* summary, u3
 }
 int launch_combine(const b200moe_combine_view& v, cudaStream_t stream) {
     if (v.rows == 0) return B200MOE_OK;
-    // Only the PARTS form, whose slot -> value chain is what the early requests hide: the slot-order form is faster with more, lighter
-    // threads (4096 rows x 8 x 2048: 77 against 94 us). 32 rows is not a crossover: at 32 x 8 x 2048, 8 parts, the forms take 4.97 and
-    // 4.24 us (x 7168: 9.5 and 6.5), at 31 4.95 and 4.23, and one row 4.5 and 4.0 (a whole call 37.2 and 35.5); fewer rows keep
-    // the first form because they have only been timed so far.
-    if (v.form == B200MOE_COMBINE_PARTS && v.rows >= 32 && v.y && !v.y_blocks && v.only_part < 0 && v.top_k <= kVecTopK && v.hidden % 4 == 0 && aligned(v.raw, 16) && aligned(v.y, 16) && aligned(v.shared, 16) &&
-        aligned(v.y_bf16, 8)) {
+    // PARTS in one row: a whole call 37.2 us in the general form, 35.5 in the wide one; 32 rows x 8 x 2048 of 8 parts 5.0 and 4.2 us.
+    const bool whole = v.y && !v.y_blocks && v.top_k <= kVecTopK;
+    if (v.form == B200MOE_COMBINE_PARTS && whole && v.only_part < 0 && v.hidden % 4 == 0 && aligned(v.raw, 16) && aligned(v.y, 16) && aligned(v.shared, 16) && aligned(v.y_bf16, 8)) {
         if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_vec_kernel))) return rc;
         combine_vec_kernel<<<dim3((v.hidden + 511) / 512, std::min<u32>(v.rows, 65535u)), 128, 0, stream>>>(v);
+        return after_launch("combine");
+    }
+    if (v.form == B200MOE_COMBINE_FMA_SLOTS && whole && v.hidden % 2 == 0 && aligned(v.raw, 8) && aligned(v.y, 8) && aligned(v.shared, 8) && aligned(v.y_bf16, 4)) {
+        if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_slots_kernel))) return rc;
+        combine_slots_kernel<<<dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 128, 0, stream>>>(v);
         return after_launch("combine");
     }
     if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_kernel))) return rc;

@@ -8,6 +8,7 @@
 // HBM: the logits kernel streams the FP32 router matrix once per RT-row tile ([experts][hidden] * 4 B); the select
 // kernel touches rows * experts * 4 B. Both are small beside the expert weights.
 #include "declared_math.cuh"
+#include "grouped_common.cuh"
 #include "kernels.cuh"
 
 namespace b200moe {
@@ -135,11 +136,11 @@ __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float* __
         }
         asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group keeps the count of the wait below fixed
     };
-    float acc[kTileRows][ET];
+    float2 acc[kTileRows / 2][ET];  // pairs of rows
 #pragma unroll
-    for (int r = 0; r < (int)kTileRows; ++r)
+    for (int r = 0; r < (int)kTileRows / 2; ++r)
 #pragma unroll
-        for (int e = 0; e < (int)ET; ++e) acc[r][e] = 0.0f;
+        for (int e = 0; e < (int)ET; ++e) acc[r][e] = make_float2(0.0f, 0.0f);
     issue(0);
     issue(1);
     for (u32 c = 0; c < n_chunks; ++c) {
@@ -150,15 +151,19 @@ __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float* __
         const u32 ncol = min(kTileCols, hidden - c * kTileCols);
 #pragma unroll 4
         for (u32 col = lane; col < ncol; col += 32) {
-            float xv[kTileRows], wv[ET];
+            float2 xv[kTileRows / 2];
+            float wv[ET];
 #pragma unroll
-            for (int r = 0; r < (int)kTileRows; ++r) xv[r] = st[r * kTileCols + col];
+            for (int r = 0; r < (int)kTileRows / 2; ++r) xv[r] = make_float2(st[2 * r * kTileCols + col], st[(2 * r + 1) * kTileCols + col]);
 #pragma unroll
             for (int e = 0; e < (int)ET; ++e) wv[e] = st[(kTileRows + ET * warp + e) * kTileCols + col];
 #pragma unroll
-            for (int r = 0; r < (int)kTileRows; ++r)
+            for (int r = 0; r < (int)kTileRows / 2; ++r)
 #pragma unroll
-                for (int e = 0; e < (int)ET; ++e) acc[r][e] = __fadd_rn(acc[r][e], __fmul_rn(wv[e], xv[r]));
+                for (int e = 0; e < (int)ET; ++e) {
+                    if (kTileCols == 256) acc[r][e] = grouped::add2(grouped::mul2(grouped::both(wv[e]), xv[r]), acc[r][e]);
+                    else acc[r][e] = make_float2(__fadd_rn(acc[r][e].x, __fmul_rn(wv[e], xv[r].x)), __fadd_rn(acc[r][e].y, __fmul_rn(wv[e], xv[r].y)));
+                }
         }
         __syncthreads();  // the stage is refilled by the copies issued two iterations on
     }
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float* __
     for (int r = 0; r < (int)kTileRows; ++r)
 #pragma unroll
         for (int e = 0; e < (int)ET; ++e) {
-            float z = butterfly32(acc[r][e]);
+            float z = butterfly32(r & 1 ? acc[r / 2][e].y : acc[r / 2][e].x);
             const u32 row = r0 + r, ex = e0 + ET * warp + e;
             if (lane == 0 && row < rows && ex < experts) {
                 if (logit_bias) z = __fadd_rn(z, logit_bias[ex]);

@@ -222,7 +222,7 @@ def test_router_logits_forms(gpu, rows, hidden, experts):
     assert logits.data_ptr() != scores.data_ptr() and same(logits.cpu(), declared_logits(x, w))
 
 
-@pytest.mark.parametrize("rows,top_k,hidden,parts", [(31, 4, 192, 4), (32, 4, 192, 4), (40, 8, 516, 8), (33, 9, 256, 3), (35, 3, 258, 2)])
+@pytest.mark.parametrize("rows,top_k,hidden,parts", [(1, 8, 512, 8), (7, 4, 260, 2), (31, 4, 192, 4), (32, 4, 192, 4), (40, 8, 516, 8), (33, 9, 256, 3), (35, 3, 258, 2)])
 def test_combine_parts_forms(gpu, rows, top_k, hidden, parts):
     """Both sides of the wide form's rule (rows, slots, whole 16-byte units), ranges without a slot among the parts."""
     from b200moe import ops
@@ -244,6 +244,28 @@ def test_combine_parts_forms(gpu, rows, top_k, hidden, parts):
             want[r] = want[r] + s
     y, yb = ops.enqueue_moe_combine(b200moe.COMBINE_PARTS, dv(raw, gpu), dv(wts, gpu), dv(ids.view(np.int32), gpu), order=dv(order, gpu), shared=dv(shared, gpu),
                                     parts=parts, part_experts=E // parts, bf16=True)
+    assert same(y.cpu(), want) and torch.equal(yb.cpu(), torch.from_numpy(want).bfloat16())
+
+
+@pytest.mark.parametrize("rows,top_k,hidden,offset", [(1, 8, 2048, 0), (3, 1, 258, 0), (2, 5, 64, 0), (5, 8, 322, 1), (4, 9, 256, 0), (700, 2, 66, 0)])
+@pytest.mark.parametrize("shared", [False, True])
+def test_combine_slot_order_forms(gpu, oracle, rows, top_k, hidden, offset, shared):
+    """Both sides of the pair form's rule (slots, 8-byte rows); a row whose status is set is left as it was."""
+    from b200moe import ops
+    import b200moe
+    rng = np.random.default_rng(rows + hidden)
+    ids = window(rng, 16, top_k, rows)
+    flat = rng.standard_normal(rows * top_k * hidden + offset, dtype=np.float32)
+    raw = flat[offset:].reshape(rows * top_k, hidden)
+    wts = rng.uniform(0.05, 0.6, (rows, top_k)).astype(np.float32)
+    sh = rng.standard_normal((rows, hidden), dtype=np.float32) if shared else None
+    want = oracle.combine(O.COMBINE_FMA_SLOTS, raw, wts, ids)
+    want = want + sh if shared else want
+    status = np.zeros(rows, np.int32)
+    status[rows // 2] = 1 if rows > 1 else 0
+    want[status != 0] = 0.0
+    y, yb = ops.enqueue_moe_combine(b200moe.COMBINE_FMA_SLOTS, dv(flat, gpu)[offset:].view(rows * top_k, hidden), dv(wts, gpu), dv(ids.view(np.int32), gpu),
+                                    shared=dv(sh, gpu) if shared else None, row_status=dv(status, gpu), bf16=True)
     assert same(y.cpu(), want) and torch.equal(yb.cpu(), torch.from_numpy(want).bfloat16())
 
 

@@ -4,15 +4,15 @@
 //
 // The contract adds the terms float(dot_g) * (scale_g * delta_g) of a row into 32 lane classes (group g -> class g % 32) in
 // ascending g, then folds the classes with the butterfly v[l] += v[l ^ d], d = 16 .. 1. A class is an independent chain, so
-// the CLASSES are what the warps of a CTA share out: consumer warp w owns classes 2w and 2w + 1 of all 16 rows x 8 (or 16) entries
+// the CLASSES are what the warps of a CTA share out: consumer warp w owns classes 2w and 2w + 1 of all 16 rows x 8 entries
 // of a tile, i.e. blocks 2w and 2w + 1 of every run of 32 blocks, and walks the runs in ascending order - eight FP32
-// accumulators per lane and 8 entries, each product and each add the contract's own, in its order. When the tile's last run is
-// done the 16 x 8 (16) x 32 class sums meet in shared memory and warp w runs the butterfly of row w, bit for bit.
+// accumulators per lane, each product and each add the contract's own, in its order. When the tile's last run is
+// done the 16 x 8 x 32 class sums meet in shared memory and warp w runs the butterfly of row w, bit for bit.
 //
-//  * Item = (virtual expert of at most 8 - or, where experts have them, 16 - entries, 32 outputs); tiles of 16 weight rows: gate rows, gate rows + 16, up rows,
+//  * Item = (virtual expert of at most 8 entries, 32 outputs); tiles of 16 weight rows: gate rows, gate rows + 16, up rows,
 //    up rows + 16 (gate/up) or the two halves of 32 down rows. A CTA takes a contiguous range of items (items of a dense
 //    block cost the same), so consecutive items mostly share their entries, whose A8 rows stay in shared memory.
-//  * A stage = 16 rows x up to 4 (2) runs, one tiled TMA copy per run (box 138 x 64-bit = 1104 bytes per row: the run's 1088
+//  * A stage = 16 rows x up to 4 runs, one tiled TMA copy per run (box 138 x 64-bit = 1104 bytes per row: the run's 1088
 //    bytes and 16 more, which puts consecutive rows 20 words apart - the eight rows and four k slices of an A fragment load
 //    then fall into 32 different banks). Two stages in flight. The entries' codes lie 4 (mod 32) words apart for the same reason.
 //  * Q8_0 blocks are 34 bytes: the quants of an even block of a run start 2 (mod 4) bytes in (two words and a byte permute
@@ -37,15 +37,10 @@ constexpr u32 kRunBox = kTileRows * kRowPitch;                     // 17,664
 constexpr u32 kStages = 2;
 constexpr u32 kMmaWarps = 16;                                      // consumer warps; one producer warp after them
 constexpr u32 kMmaThreads = (kMmaWarps + 1) * 32;
-// Entries of an item: NT blocks of 8. With NT = 2 a weight fragment meets 16 entries, the weight rows are streamed out of L2 half as
-// often and a tile's barriers serve twice the cells; a stage is then two runs instead of four, which leaves room for the A8 rows.
-template <u32 NT>
-struct Items {
-    static constexpr u32 KE = 8 * NT;
-    static constexpr u32 stage_runs = NT == 1 ? 4 : 2, stage_bytes = stage_runs * kRunBox;
-    static constexpr u32 cls_floats = kTileRows * KE * 32;         // class sums of a tile
-    static constexpr u32 gu_floats = 2 * 2 * KE * 32;              // [item parity][gate | up][entry][32]
-};
+constexpr u32 KE = kKE;                                            // entries of an item
+constexpr u32 kStageRuns = 4, kStageBytes = kStageRuns * kRunBox;
+constexpr u32 kClsFloats = kTileRows * KE * 32;                    // class sums of a tile
+constexpr u32 kGuFloats = 2 * 2 * KE * 32;                         // [item parity][gate | up][entry][32]
 constexpr u32 kMaxK = 7168;                                        // the entries' A8 rows of a whole item stay in shared memory
 
 struct MmaPlan {
@@ -76,9 +71,9 @@ __device__ __forceinline__ void mma_s8s8(int (&c)[4], u32 a0, u32 a1, u32 a2, u3
 // One block of one run: rows gid and gid + 8 of the tile (A), the item's entries in blocks of 8 (B), this lane's four (row, entry)
 // cells of each. ODD: the block's position in its run is odd (quants on a word). blk: byte offset of the block in a row;
 // codes / deltas: the first entries' A8 rows at this block, for this lane's fragment cells. nb: blocks of entries that hold any.
-template <bool ODD, u32 NT>
+template <bool ODD>
 __device__ __forceinline__ void block_step(const unsigned char* rowA, const unsigned char* rowB, u32 blk, u32 t4, const unsigned char* codes,
-                                           const unsigned char* d0p, u32 xc_pitch, u32 xd_pitch, u32 nb, float (&acc)[NT][4]) {
+                                           const unsigned char* d0p, u32 xd_pitch, float (&acc)[4]) {
     u32 a0, a1, a2, a3;
     float sA, sB;
     if (ODD) {  // block at 2 (mod 4): the scale is the high half of the word before the quants
@@ -95,26 +90,20 @@ __device__ __forceinline__ void block_step(const unsigned char* rowA, const unsi
         sA = half_bits_to_float(*reinterpret_cast<const unsigned short*>(rowA + blk));
         sB = half_bits_to_float(*reinterpret_cast<const unsigned short*>(rowB + blk));
     }
-#pragma unroll
-    for (u32 nt = 0; nt < NT; ++nt) {
-        if (nt && nt >= nb) break;  // warp-uniform
-        const u32* pc = reinterpret_cast<const u32*>(codes + 8u * nt * xc_pitch);
-        const float d0 = *reinterpret_cast<const float*>(d0p + 8u * nt * xd_pitch), d1 = *reinterpret_cast<const float*>(d0p + (8u * nt + 1u) * xd_pitch);
-        int c[4];
-        mma_s8s8(c, a0, a1, a2, a3, pc[0], pc[4]);
-        // c[0]: (row gid, entry 2 t4), c[1]: (gid, 2 t4 + 1), c[2]: (gid + 8, 2 t4), c[3]: (gid + 8, 2 t4 + 1)
-        acc[nt][0] = __fadd_rn(acc[nt][0], __fmul_rn(static_cast<float>(c[0]), __fmul_rn(sA, d0)));
-        acc[nt][1] = __fadd_rn(acc[nt][1], __fmul_rn(static_cast<float>(c[1]), __fmul_rn(sA, d1)));
-        acc[nt][2] = __fadd_rn(acc[nt][2], __fmul_rn(static_cast<float>(c[2]), __fmul_rn(sB, d0)));
-        acc[nt][3] = __fadd_rn(acc[nt][3], __fmul_rn(static_cast<float>(c[3]), __fmul_rn(sB, d1)));
-    }
+    const u32* pc = reinterpret_cast<const u32*>(codes);
+    const float d0 = *reinterpret_cast<const float*>(d0p), d1 = *reinterpret_cast<const float*>(d0p + xd_pitch);
+    int c[4];
+    mma_s8s8(c, a0, a1, a2, a3, pc[0], pc[4]);
+    // c[0]: (row gid, entry 2 t4), c[1]: (gid, 2 t4 + 1), c[2]: (gid + 8, 2 t4), c[3]: (gid + 8, 2 t4 + 1)
+    acc[0] = __fadd_rn(acc[0], __fmul_rn(static_cast<float>(c[0]), __fmul_rn(sA, d0)));
+    acc[1] = __fadd_rn(acc[1], __fmul_rn(static_cast<float>(c[1]), __fmul_rn(sA, d1)));
+    acc[2] = __fadd_rn(acc[2], __fmul_rn(static_cast<float>(c[2]), __fmul_rn(sB, d0)));
+    acc[3] = __fadd_rn(acc[3], __fmul_rn(static_cast<float>(c[3]), __fmul_rn(sB, d1)));
 }
 
-template <bool DOWN, u32 NT>
+template <bool DOWN>
 __global__ void __launch_bounds__(kMmaThreads, 1)
 q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, MmaArgs a, MmaPlan plan) {
-    using It = Items<NT>;
-    constexpr u32 KE = It::KE;
     extern __shared__ __align__(128) unsigned char smem[];
     if (DOWN && a.summary && *a.summary) return;
     u32 n_union = a.routes.counts[0];
@@ -122,11 +111,11 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
     if (n_union > plan.max_union) n_union = plan.max_union;
 
     unsigned char* ring = smem;
-    unsigned char* xc = ring + kStages * It::stage_bytes;
+    unsigned char* xc = ring + kStages * kStageBytes;
     unsigned char* xd = xc + KE * plan.xc_pitch;
     float* cls = reinterpret_cast<float*>(xd + KE * plan.xd_pitch);
-    float* s_gu = cls + It::cls_floats;
-    unsigned char* at = reinterpret_cast<unsigned char*>(s_gu + (DOWN ? 0u : It::gu_floats));
+    float* s_gu = cls + kClsFloats;
+    unsigned char* at = reinterpret_cast<unsigned char*>(s_gu + (DOWN ? 0u : kGuFloats));
     VExpert* table = reinterpret_cast<VExpert*>(at);
     at += (u64(plan.vmax) * sizeof(VExpert) + 15) & ~u64(15);
     u64* full = reinterpret_cast<u64*>(at);
@@ -142,7 +131,7 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
     if (tid == kStages) { mbar_init(x_full, 1); mbar_init(x_empty, kMmaWarps); }
     if (tid < 8) ctl[tid] = 0;
     if (tid <= kStages) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    build_work_list<KE>(a.routes, n_union, plan.max_union, plan.vmax, plan.n_chunks, reinterpret_cast<u32*>(smem), table, ctl);
+    build_work_list(a.routes, n_union, plan.max_union, plan.vmax, plan.n_chunks, reinterpret_cast<u32*>(smem), table, ctl);
     const u32 n_items = ctl[3];
     const u32 k0 = static_cast<u32>(u64(n_items) * blockIdx.x / gridDim.x), k1 = static_cast<u32>(u64(n_items) * (blockIdx.x + 1) / gridDim.x);
     if (k0 == k1) return;
@@ -169,12 +158,12 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the consumers' reads precede the copies below
-                const u32 run0 = s * It::stage_runs, nr = min(It::stage_runs, plan.nruns - run0);
+                const u32 run0 = s * kStageRuns, nr = min(kStageRuns, plan.nruns - run0);
                 if (lane == 0) mbar_expect_tx(&full[slot], nr * kRunBox);
                 __syncwarp();
                 if (lane < nr) {
                     const u32 y = ve.expert() * a.rows_per_expert + 32u * chunk + kTileRows * (DOWN ? tile : (tile & 1u));
-                    tma_2d(ring + slot * It::stage_bytes + lane * kRunBox, (DOWN || tile < 2u) ? &tm0 : &tm1, (run0 + lane) * (kRunBytes / 8), y, &full[slot]);
+                    tma_2d(ring + slot * kStageBytes + lane * kRunBox, (DOWN || tile < 2u) ? &tm0 : &tm1, (run0 + lane) * (kRunBytes / 8), y, &full[slot]);
                 }
                 if (si == 0 && new_x) {  // the entries' A8 rows, requested right after the item's first stage
                     if (xl) ok = mbar_wait(x_empty, (xl - 1u) & 1u, plan.wait_limit, abort_flag);
@@ -220,29 +209,26 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
             ++xl;
             last_jv = jv;
         }
-        const u32 nb = (ne + 7u) / 8u;
-        u32 my_slot[NT];
-#pragma unroll
-        for (u32 nt = 0; nt < NT; ++nt) my_slot[nt] = DOWN && 8u * nt + (lane >> 2) < ne ? __ldg(a.routes.slots + vbegin + 8u * nt + (lane >> 2)) : 0u;
-        float* gu = s_gu + (kl & 1u) * (It::gu_floats / 2);
+        const u32 my_slot = DOWN && (lane >> 2) < ne ? __ldg(a.routes.slots + vbegin + (lane >> 2)) : 0u;
+        float* gu = s_gu + (kl & 1u) * (kGuFloats / 2);
         bool stop = false;
         for (u32 tile = 0; tile < kTiles; ++tile) {
-            float acc[2][NT][4];
+            float acc[2][4];
 #pragma unroll
-            for (u32 i = 0; i < 2 * NT * 4; ++i) (&acc[0][0][0])[i] = 0.0f;
+            for (u32 i = 0; i < 8; ++i) (&acc[0][0])[i] = 0.0f;
             for (u32 s = 0; s < plan.nst; ++s, ++t) {
                 const u32 slot = t & 1u;
                 if (ok) ok = mbar_wait(&full[slot], (t >> 1) & 1u, plan.wait_limit, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) continue;  // a wait ran out somewhere: no more work, but every warp still meets the barriers below
-                const u32 run0 = s * It::stage_runs, nr = min(It::stage_runs, plan.nruns - run0);
-                const unsigned char* box = ring + slot * It::stage_bytes;
+                const u32 run0 = s * kStageRuns, nr = min(kStageRuns, plan.nruns - run0);
+                const unsigned char* box = ring + slot * kStageBytes;
                 for (u32 r = 0; r < nr; ++r, box += kRunBox) {
                     const u32 b = (run0 + r) * kRunBlocks + 2u * warp;  // even block of this warp in the run
                     const unsigned char* rowA = box + gid * kRowPitch;
                     const unsigned char* rowB = rowA + 8u * kRowPitch;
-                    if (b < plan.groups) block_step<false, NT>(rowA, rowB, blk_even, t4, my_codes + 32u * b, my_d0 + 4u * b, plan.xc_pitch, plan.xd_pitch, nb, acc[0]);
-                    if (b + 1u < plan.groups) block_step<true, NT>(rowA, rowB, blk_odd, t4, my_codes + 32u * (b + 1u), my_d0 + 4u * (b + 1u), plan.xc_pitch, plan.xd_pitch, nb, acc[1]);
+                    if (b < plan.groups) block_step<false>(rowA, rowB, blk_even, t4, my_codes + 32u * b, my_d0 + 4u * b, plan.xd_pitch, acc[0]);
+                    if (b + 1u < plan.groups) block_step<true>(rowA, rowB, blk_odd, t4, my_codes + 32u * (b + 1u), my_d0 + 4u * (b + 1u), plan.xd_pitch, acc[1]);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[slot]);  // the stage is free for the producer
@@ -256,35 +242,28 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (u32 nt = 0; nt < NT; ++nt)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const u32 row = gid + 8u * (i >> 1), entry = 8u * nt + 2u * t4 + (i & 1u);
-                        cls[(row * KE + entry) * 32u + ((2u * warp + c + 4u * entry + row) & 31u)] = acc[c][nt][i];
-                    }
+                for (int i = 0; i < 4; ++i) {
+                    const u32 row = gid + 8u * (i >> 1), entry = 2u * t4 + (i & 1u);
+                    cls[(row * KE + entry) * 32u + ((2u * warp + c + 4u * entry + row) & 31u)] = acc[c][i];
+                }
             consumers_sync();
             // Warp w folds row w of the tile, lane = (entry, class % 4): the butterfly's steps 16, 8 and 4 stay inside a residue
             // class mod 4, i.e. inside the lane's eight registers; only steps 2 and 1 cross lanes. (A lane per class and five
             // shuffles an entry kept the shuffle unit as busy as the dots of a 2048-wide row: 512 rows x 4 over 64 experts of
             // 2048 -> 1024 took 830 us a call, 671 now.)
-            const u32 fq = lane & 3u;
+            const u32 fq = lane & 3u, fe = lane >> 2;
+            float v8[8];
 #pragma unroll
-            for (u32 nt = 0; nt < NT; ++nt) {
-                if (nt && nt >= nb) break;
-                const u32 fe = 8u * nt + (lane >> 2);
-                float v8[8];
+            for (u32 i = 0; i < 8; ++i) v8[i] = cls[(warp * KE + fe) * 32u + ((fq + 4u * i + 4u * fe + warp) & 31u)];
 #pragma unroll
-                for (u32 i = 0; i < 8; ++i) v8[i] = cls[(warp * KE + fe) * 32u + ((fq + 4u * i + 4u * fe + warp) & 31u)];
+            for (u32 h = 4; h; h >>= 1)
 #pragma unroll
-                for (u32 h = 4; h; h >>= 1)
-#pragma unroll
-                    for (u32 i = 0; i < h; ++i) v8[i] = __fadd_rn(v8[i], v8[i + h]);
-                float mine = __fadd_rn(v8[0], __shfl_xor_sync(0xffffffffu, v8[0], 2));
-                mine = __fadd_rn(mine, __shfl_xor_sync(0xffffffffu, mine, 1));
-                if (fq == 0 && fe < ne && ok) {
-                    if (DOWN) a.raw[u64(my_slot[nt]) * a.out_width + 32u * chunk + kTileRows * tile + warp] = mine;
-                    else gu[(tile >> 1) * KE * 32u + fe * 32u + kTileRows * (tile & 1u) + warp] = mine;
-                }
+                for (u32 i = 0; i < h; ++i) v8[i] = __fadd_rn(v8[i], v8[i + h]);
+            float mine = __fadd_rn(v8[0], __shfl_xor_sync(0xffffffffu, v8[0], 2));
+            mine = __fadd_rn(mine, __shfl_xor_sync(0xffffffffu, mine, 1));
+            if (fq == 0 && fe < ne && ok) {
+                if (DOWN) a.raw[u64(my_slot) * a.out_width + 32u * chunk + kTileRows * tile + warp] = mine;
+                else gu[(tile >> 1) * KE * 32u + fe * 32u + kTileRows * (tile & 1u) + warp] = mine;
             }
             if (tid == 0) ctl[4] = *abort_flag;  // one thread publishes the decision between the two barriers: every warp reads the same
             consumers_sync();
@@ -310,39 +289,28 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
 }
 
 u32 round_up(u32 v, u32 a) { return (v + a - 1) / a * a; }
-template <u32 NT>
 u32 plan_smem(const MmaPlan& p, bool down) {
-    using It = Items<NT>;
-    return kStages * It::stage_bytes + It::KE * (p.xc_pitch + p.xd_pitch) + It::cls_floats * 4 + (down ? 0u : It::gu_floats * 4) +
+    return kStages * kStageBytes + KE * (p.xc_pitch + p.xd_pitch) + kClsFloats * 4 + (down ? 0u : kGuFloats * 4) +
            round_up(p.vmax * static_cast<u32>(sizeof(VExpert)), 16) + (2 * kStages + 2) * 8 + 64;
 }
 
-template <u32 NT>
 bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, bool down, MmaPlan* p) {
-    using It = Items<NT>;
     // whole runs of 32 blocks exist, rows of K / 32 * 34 bytes are multiples of 16, the staged A8 rows fit beside the ring
     if (K < 1024 || K > kMaxK || K % 256 || max_union == 0 || slots == 0 || slots > 8192) return false;
     p->K = K;
     p->groups = K / 32;
     p->nruns = (p->groups + kRunBlocks - 1) / kRunBlocks;
-    p->nst = (p->nruns + It::stage_runs - 1) / It::stage_runs;
+    p->nst = (p->nruns + kStageRuns - 1) / kStageRuns;
     p->xc_pitch = K + 16;      // K is a multiple of 128 bytes: entries lie 4 (mod 32) words apart
     p->xd_pitch = K / 8 + 16;
     p->n_chunks = n_chunks;
     p->max_union = max_union;
-    p->vmax = max_union + static_cast<u32>(slots / It::KE) + 1;
+    p->vmax = max_union + static_cast<u32>(slots / KE) + 1;
     if (u64(p->vmax) * n_chunks >= (1ull << 31)) return false;
-    if (plan_smem<NT>(*p, down) > kSmemBudget) return false;
-    if (work_list_scratch_words<It::KE>(max_union, p->vmax) * 4 > kStages * It::stage_bytes) return false;  // the work list is built in the ring
+    if (plan_smem(*p, down) > kSmemBudget) return false;
+    if (work_list_scratch_words(max_union, p->vmax) * 4 > kStages * kStageBytes) return false;  // the work list is built in the ring
     p->wait_limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT) ? debug_value(B200MOE_DEBUG_WAIT_LIMIT) : kDefaultWaitLimit;
     return true;
-}
-// 16 entries an item where the experts have them on average and the items still go round the SMs twice; the A8 rows of 16 entries fit
-// up to a width of 6656 (gate/up) or 6912 (down). Whole calls over 64 experts of 2048 -> 1024, 8 against 16 entries: 387 and
-// 350 us with 16 an expert, 671 and 568 with 32. The crossover is lower, at 9 an expert: 186 and 242 us with 4, 243 and 249 with
-// 8, 283 and 258 with 10; 64 experts of 4096 -> 1536 475 and 525 with 8, 635 and 584 with 12. One expert (dense, 1024 -> 1024) gains from 33 rows on.
-bool take_16(u32 K, u32 n_chunks, u32 max_union, u64 slots, bool down, MmaPlan* p) {
-    return slots >= 16ull * max_union && slots / 16u * n_chunks >= 2u * static_cast<u32>(device_sm_count()) && make_plan<2>(K, n_chunks, max_union, slots, down, p);
 }
 bool a8_ok(const b200moe_a8_rows& x) {
     const u32 stride = x.stride ? x.stride : x.width;
@@ -354,19 +322,18 @@ bool a8_ok(const b200moe_a8_rows& x) {
 bool q8_mma_gate_up_fits(const b200moe_gate_up_view& v, u32 rows) {
     MmaPlan p{};
     return v.shape.gate_type == B200MOE_TYPE_Q8_0 && v.shape.down_type == B200MOE_TYPE_Q8_0 && rows && a8_ok(v.x) && v.shape.inter % 32 == 0 &&
-           aligned(v.weights.gate, 16) && aligned(v.weights.up, 16) && make_plan<1>(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, false, &p);
+           aligned(v.weights.gate, 16) && aligned(v.weights.up, 16) && make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, false, &p);
 }
 bool q8_mma_down_fits(const b200moe_down_view& v, u32 rows) {
     MmaPlan p{};
     return v.shape.gate_type == B200MOE_TYPE_Q8_0 && v.shape.down_type == B200MOE_TYPE_Q8_0 && rows && a8_ok(v.act) && v.shape.hidden % 32 == 0 &&
-           aligned(v.weights.down, 16) && make_plan<1>(v.shape.inter, v.shape.hidden / 32, v.max_union, u64(rows) * v.shape.top_k, true, &p);
+           aligned(v.weights.down, 16) && make_plan(v.shape.inter, v.shape.hidden / 32, v.max_union, u64(rows) * v.shape.top_k, true, &p);
 }
 
 int launch_gate_up_q8_mma(const b200moe_gate_up_view& v, u32 rows, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     MmaPlan p{};
-    const bool wide16 = take_16(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, false, &p);
-    if (!wide16 && !make_plan<1>(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, false, &p))
+    if (!make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, false, &p))
         return fail(B200MOE_ERR_UNSUPPORTED, "gate_up: the Q8_0 tensor-core form does not apply to this shape");
     MmaArgs a{};
     a.routes = v.routes; a.in = v.x; a.act = v.act; a.gate_out = v.gate_out; a.up_out = v.up_out; a.summary = v.summary;
@@ -375,8 +342,8 @@ int launch_gate_up_q8_mma(const b200moe_gate_up_view& v, u32 rows, cudaStream_t 
     const u64 rb = u64(p.groups) * kQ8Block, total_rows = u64(v.shape.experts) * v.shape.inter;
     if (int rc = rows_map(v.weights.gate, rb, total_rows, kRowPitch, kTileRows, &tm0)) return rc;
     if (int rc = rows_map(v.weights.up, rb, total_rows, kRowPitch, kTileRows, &tm1)) return rc;
-    const u32 smem = wide16 ? plan_smem<2>(p, false) : plan_smem<1>(p, false);
-    const auto kernel = wide16 ? q8_mma_kernel<false, 2> : q8_mma_kernel<false, 1>;
+    const u32 smem = plan_smem(p, false);
+    const auto kernel = q8_mma_kernel<false>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
     kernel<<<sm_count(), kMmaThreads, smem, stream>>>(tm0, tm1, a, p);
     return after_launch("gate_up_q8_mma");
@@ -385,16 +352,15 @@ int launch_gate_up_q8_mma(const b200moe_gate_up_view& v, u32 rows, cudaStream_t 
 int launch_down_q8_mma(const b200moe_down_view& v, u32 rows, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     MmaPlan p{};
-    const bool wide16 = take_16(v.shape.inter, v.shape.hidden / 32, v.max_union, u64(rows) * v.shape.top_k, true, &p);
-    if (!wide16 && !make_plan<1>(v.shape.inter, v.shape.hidden / 32, v.max_union, u64(rows) * v.shape.top_k, true, &p))
+    if (!make_plan(v.shape.inter, v.shape.hidden / 32, v.max_union, u64(rows) * v.shape.top_k, true, &p))
         return fail(B200MOE_ERR_UNSUPPORTED, "down: the Q8_0 tensor-core form does not apply to this shape");
     MmaArgs a{};
     a.routes = v.routes; a.in = v.act; a.raw = v.raw; a.summary = const_cast<u32*>(v.summary);
     a.rows_per_expert = v.shape.hidden; a.out_width = v.shape.hidden; a.limit = v.shape.limit;
     CUtensorMap tm0;
     if (int rc = rows_map(v.weights.down, u64(p.groups) * kQ8Block, u64(v.shape.experts) * v.shape.hidden, kRowPitch, kTileRows, &tm0)) return rc;
-    const u32 smem = wide16 ? plan_smem<2>(p, true) : plan_smem<1>(p, true);
-    const auto kernel = wide16 ? q8_mma_kernel<true, 2> : q8_mma_kernel<true, 1>;
+    const u32 smem = plan_smem(p, true);
+    const auto kernel = q8_mma_kernel<true>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
     kernel<<<sm_count(), kMmaThreads, smem, stream>>>(tm0, tm0, a, p);
     return after_launch("down_q8_mma");

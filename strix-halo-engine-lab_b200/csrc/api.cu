@@ -270,12 +270,13 @@ DecodeForm pick_decode_form(bool row_stream_fits, bool wide_fits, u32 rows, u32 
 // The grouped form (grouped_q8.cu, tiles of 32 entries) takes over from the tensor-core form at 10 entries an expert and 20 rows: whole calls, the
 // two in this order, 64 experts of 2048 x 1024: 199 and 236 us with 6 entries, 249 and 239 with 8, 328 and 240 with 12; 16 experts of
 // 4096 x 1536: 167 and 188 with 8, 241 and 196 with 16; one expert of 7168 x 2048: 49 and 64 us with 16 rows, 63 and 61 with 24, 101
-// and 66 with 64. Where the tensor-core form does not apply (rows below 1024 or above 7168 weights) it takes over from the dp4a form at 2
-// entries and 12 rows: 48 experts of 1024 x 512 109 and 93 us with 2 entries, one expert of 2048 x 8192 66 and 79 us with 8 rows,
-// 76 and 70 with 16, of 768 x 4096 49 and 51 with 8, 50 and 49 with 16.
+// and 66 with 64. Where the tensor-core form does not apply (rows below 1024 or above 7168 weights) it takes over from the dp4a form at 5
+// entries and 12 rows: down of 32 experts of 1536 x 768 94 and 107 us a call with 2.6 entries, 108 and 109 with 5.2, 124 and 116 with 7.5; of
+// 48 of 2048 x 512 120 and 120 with 4, 136 and 124 with 6; one expert of 4096 x 12288 78 and 84 us with 8 rows, 107 and 104 with 12, 152
+// and 110 with 24.
 enum class Q8Form { row_per_warp, wide, mma, grouped };
 bool q8_grouped_pays(bool mma_fits, u32 rows, const b200moe_shape& s) {
-    return rows >= (mma_fits ? 20u : 12u) && u64(rows) * s.top_k >= u64(mma_fits ? 10u : 2u) * s.experts;
+    return rows >= (mma_fits ? 20u : 12u) && u64(rows) * s.top_k >= u64(mma_fits ? 10u : 5u) * s.experts;
 }
 Q8Form pick_q8_form(bool wide_fits, bool mma_fits, bool grouped_fits, u32 rows, const b200moe_shape& s) {
     const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);

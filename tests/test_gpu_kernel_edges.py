@@ -201,6 +201,23 @@ def test_q8_grouped_units(gpu, oracle, tokens, H, I):
     assert same(raw.cpu(), want["raw"])
 
 
+@pytest.mark.parametrize("rows,top_k,E,H,I", [(19, 1, 1, 1024, 1024), (20, 1, 1, 1024, 1024), (24, 4, 10, 1024, 1024), (25, 4, 10, 1024, 1024),
+                                             (11, 1, 1, 512, 512), (12, 1, 1, 512, 512), (12, 4, 10, 512, 768), (13, 4, 10, 512, 768)])
+def test_q8_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I):
+    """Both sides of the lines between the streaming and the grouped Q8_0 form, where the tensor-core form applies and where it does not."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 8, 8)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, top_k, 8, 8)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
+
+
 def declared_logits(x, w):
     """Lane class l sums products l, l + 32, ... ascending; the classes fold by the butterfly (src/ds41_moe.cpp:72-82)."""
     acc = np.zeros((x.shape[0], w.shape[0], 32), np.float32)

@@ -79,6 +79,7 @@ struct WideArgs {
     u32* summary;
     u32 rows_per_expert;   // weight rows of one expert: inter (gate/up) or hidden (down)
     u32 out_width;         // inter (gate/up) or hidden (down)
+    u32 raw_vec;           // raw lies on an 8-byte boundary
 };
 
 // Stage geometry for S super-blocks per stage, as compile-time constants: the kernels are bound by issue slots, and
@@ -385,7 +386,8 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             if (mma) {
                 if (me < ne) {
                     float* dst = a.raw + u64(__ldg(a.routes.slots + vbegin + me)) * a.out_width + kItemRows * chunk + 8u * w + 2u * mt;
-                    *reinterpret_cast<float2*>(dst) = make_float2(m0, m1);
+                    if (a.raw_vec) *reinterpret_cast<float2*>(dst) = make_float2(m0, m1);
+                    else { dst[0] = m0; dst[1] = m1; }
                 }
             } else {
 #pragma unroll
@@ -534,7 +536,7 @@ int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, cudaStream_t stre
     apply_hooks(&p);
     WideArgs a{};
     a.routes = v.routes; a.in = v.act; a.raw = v.raw; a.summary = const_cast<u32*>(v.summary);
-    a.rows_per_expert = v.shape.hidden; a.out_width = v.shape.hidden;
+    a.rows_per_expert = v.shape.hidden; a.out_width = v.shape.hidden; a.raw_vec = aligned(v.raw, 8);
     CUtensorMap tm0;
     if (int rc = rows_map(v.weights.down, u64(p.nb) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, p.S * kQ4KBlock, 64, &tm0)) return rc;
     const u32 smem = plan_smem(p, true);

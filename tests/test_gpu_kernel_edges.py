@@ -505,3 +505,51 @@ def test_selection_scratch_beside_static_shared_memory(gpu, rows, experts):
     path = os.pathsep.join([root, os.path.join(root, "strix-halo-engine-lab_b200")])
     r = subprocess.run([sys.executable, "-c", SELECTION_WINDOWS.format(rows=rows, experts=experts)], capture_output=True, text=True, env=dict(os.environ, PYTHONPATH=path))
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("rows,top_k,E,types", [(9, 1, 1, (12, 12)), (40, 2, 10, (12, 12)), (160, 2, 64, (12, 12)), (70, 1, 1, (12, 12)), (24, 1, 1, (8, 8)),
+                                                (9, 1, 1, (8, 8))])
+def test_down_into_a_slice_on_a_4_byte_boundary(gpu, oracle, rows, top_k, E, types):
+    """raw one float past an 8-byte boundary: streaming windows below and above 128 rows with experts of five entries and more, the grouped and
+    the Q8_0 forms; a dense block's y is such a raw too. The word before and the words after it are left alone."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows)
+    H, I = 256, 256
+    gate, up, down = synth.expert_tensors(rng, E, H, I, *types)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, *types, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, top_k, *types)
+    x = (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu))
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, x, rows * top_k)
+    flat = torch.full((rows * top_k * H + 3,), -7.0, device=gpu)
+    raw = flat[1:1 + rows * top_k * H].view(rows * top_k, H)
+    assert raw.data_ptr() % 8 == 4
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act, raw=raw).cpu(), want["raw"])
+    assert flat[0].item() == -7.0 and bool((flat[1 + rows * top_k * H:] == -7.0).all())
+
+
+@pytest.mark.parametrize("rows,types", [(70, (12, 12)), (33, (8, 8))])
+def test_grouped_forms_with_deltas_off_16_bytes(gpu, oracle, rows, types):
+    """Deltas and sums 8 bytes past a 16-byte boundary: the grouped forms copy them a word at a time."""
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows)
+    E, H, I = 2, 256, 512
+    gate, up, down = synth.expert_tensors(rng, E, H, I, *types)
+    ids = window(rng, E, 1, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, *types, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+
+    def off(t):  # the same values two words into a larger array
+        flat = torch.zeros(t.numel() + 2, dtype=t.dtype, device=gpu)
+        flat[2:] = t.reshape(-1)
+        out = flat[2:].view(t.shape)
+        assert out.data_ptr() % 16 == 8
+        return out
+
+    sh = ops.make_shape(H, I, E, 1, *types)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), off(dv(deltas, gpu)), off(dv(sums, gpu))), rows, taps=True)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, (act[0], off(act[1]), off(act[2]))).cpu(), want["raw"])

@@ -332,6 +332,10 @@ float orc_declared_exp(float x) { return declared_exp(x); }
 float orc_declared_log1p(float x) { return declared_log1p(x); }
 float orc_sqrt_softplus(float z) { return sqrt_softplus(z); }
 float orc_gfx1151_expf(float x) { return gfx1151_expf(x); }
+// out[i] = exp of the float with the bits x[i]: the gfx1151 twin (gfx1151 != 0) or the declared one
+void orc_exp_bits(const u32* x, u32 n, int gfx1151, float* out) {
+    for (u32 i = 0; i < n; ++i) out[i] = gfx1151 ? gfx1151_expf(bits_f(x[i])) : declared_exp(bits_f(x[i]));
+}
 float orc_swiglu_ds41(float g, float u, float limit) { return swiglu_ds41(g, u, limit); }
 float orc_swiglu_qwen(float g, float u) { return swiglu_qwen(g, u); }
 

@@ -63,10 +63,12 @@ __device__ __forceinline__ float swiglu_ds41(float gate, float up, float limit) 
 // gfx1151 expf twin at zero correction tables (src/cpu/core/routed_expert.cpp:208-261): Cody-Waite split of
 // x * log2(e) with two fused steps, v_exp(a) = float(exp2(double(a))) for |a| < 1, scaled by 2^e.
 // The host evaluates exp2 in double with the C library; a double within an ulp or two of it changes the rounded float only when it lands
-// within 2^-29 of a float rounding boundary. 2^a is its series in a ln 2 (degree 13: the remainder for |a| <= 0.51 is 2^-57), 2^e comes in
-// two steps, as a subnormal result is then rounded once. Selects replace the cases: outside the two limits e and a are not meaningful and
-// not used, a NaN passes through. Equal to the form with CUDA's exp2(double), scalbnf and branches for every one of the 2^32 floats; that
-// form's calls kept several evaluations of a warp from overlapping: 551 clocks each where this one takes a third of the instructions.
+// within 2^-29 of a float rounding boundary. 2^a = 1 + a P(a), P the series of (2^a - 1) / a (degree 12: the remainder for |a| <= 0.51 is
+// 2^-57): the one addition of 1 comes last, so that the sum is off by little more than its own rounding. (With the 1 inside the first pair of
+// terms one float came out wrong, 0x1.0dcadep-9, whose double lies 0.44 ulp from the middle of two floats.) 2^e comes in two steps, as a
+// subnormal result is then rounded once. Selects replace the cases: outside the two limits e and a are not meaningful and not used, a NaN
+// passes through. The result is the host form's for every float, and that of CUDA's exp2(double), scalbnf and branches, whose calls kept
+// several evaluations of a warp from overlapping: 551 clocks each where this one takes a third of the instructions.
 __device__ __forceinline__ float gfx1151_expf(float x) {
     const float kLog2e = __uint_as_float(0x3fb8aa3bu), kLog2eLo = __uint_as_float(0x32a5705fu);
     const float ph = __fmul_rn(x, kLog2e);
@@ -74,14 +76,13 @@ __device__ __forceinline__ float gfx1151_expf(float x) {
     float pl = __fmaf_rn(x, kLog2e, -ph);
     pl = __fmaf_rn(x, kLog2eLo, pl);
     const double a = static_cast<double>(__fadd_rn(__fsub_rn(ph, e), pl));
-    // sum of ln(2)^k / k! a^k, pairwise (Estrin): five dependent steps instead of thirteen
+    // P = sum of ln(2)^k / k! a^(k - 1), pairwise (Estrin): six dependent steps with the last one instead of thirteen
     const double a2 = __dmul_rn(a, a), a4 = __dmul_rn(a2, a2), a8 = __dmul_rn(a4, a4);
-    const double c2 = __fma_rn(0x1.c6b08d704a0cp-5, a, 0x1.ebfbdff82c58fp-3), c4 = __fma_rn(0x1.5d87fe78a6731p-10, a, 0x1.3b2ab6fba4e77p-7), c6 = __fma_rn(0x1.ffcbfc588b0c7p-17, a, 0x1.430912f86c787p-13);
-    const double c8 = __fma_rn(0x1.b5253d395e7c4p-24, a, 0x1.62c0223a5c824p-20), c10 = __fma_rn(0x1.e8cac7351bb25p-32, a, 0x1.e4cf5158b8ecap-28), c12 = __fma_rn(0x1.816193166d0f9p-40, a, 0x1.c3bd650fc2986p-36);
-    const double c0 = __fma_rn(0x1.62e42fefa39efp-1, a, 1.0), low = __fma_rn(c2, a2, c0);
-    const double mid = __fma_rn(c6, a2, c4), high = __fma_rn(c12, a4, __fma_rn(c10, a2, c8));
-    const double y = __fma_rn(high, a8, __fma_rn(mid, a4, low));
-    const int k = min(max(static_cast<int>(__float_as_uint(big)) - 0x4b400000, -160), 160), k1 = k >> 1, k2 = k - k1;
+    const double c1 = __fma_rn(0x1.ebfbdff82c58fp-3, a, 0x1.62e42fefa39efp-1), c3 = __fma_rn(0x1.3b2ab6fba4e77p-7, a, 0x1.c6b08d704a0cp-5), c5 = __fma_rn(0x1.430912f86c787p-13, a, 0x1.5d87fe78a6731p-10);
+    const double c7 = __fma_rn(0x1.62c0223a5c824p-20, a, 0x1.ffcbfc588b0c7p-17), c9 = __fma_rn(0x1.e4cf5158b8ecap-28, a, 0x1.b5253d395e7c4p-24), c11 = __fma_rn(0x1.c3bd650fc2986p-36, a, 0x1.e8cac7351bb25p-32);
+    const double low = __fma_rn(c3, a2, c1), mid = __fma_rn(c7, a2, c5), high = __fma_rn(0x1.816193166d0f9p-40, a4, __fma_rn(c11, a2, c9));
+    const double y = __fma_rn(__fma_rn(high, a8, __fma_rn(mid, a4, low)), a, 1.0);
+    const int k = min(max(static_cast<int>(__float_as_uint(big) - 0x4b400000u), -160), 160), k1 = k >> 1, k2 = k - k1;
     float f = __fmul_rn(__fmul_rn(static_cast<float>(y), pow2i(k1)), pow2i(k2));
     if (__uint_as_float(0xc2ce8ed0u) > x) f = 0.0f;
     if (__uint_as_float(0x42b17218u) < x) f = __uint_as_float(0x7f800000u);

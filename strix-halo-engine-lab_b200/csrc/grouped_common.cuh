@@ -33,6 +33,19 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(q4k::saddr(dst)), "l"(src) : "memory");
 }
 
+// Bounds of a launch's waits: polls of up to a microsecond, and the stage before which a CTA's producers stop asking for copies (test hook).
+struct Waits { u32 limit, stall_stage; };
+inline Waits debug_waits() {
+    const u32 limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT), stall = debug_value(B200MOE_DEBUG_STALL_STAGE);
+    return Waits{limit ? limit : 1u << 20, stall ? stall - 1u : 0xffffffffu};
+}
+// Waits (bounded) until the copies of the last `asked` stages have landed: a CTA must not retire before them. One thread calls it.
+__device__ __forceinline__ void drain(u64* full, u32 stages, u32 asked, u32 limit) {
+    for (u32 n = asked > stages ? asked - stages : 0u; n < asked; ++n)
+        for (u32 i = 0; i < (limit >> 4) + 64u; ++i)
+            if (q4k::mbar_try_wait(&full[n % stages], (n / stages) & 1u, q4k::kWaitHintNs)) break;
+}
+
 struct Tile { u32 expert, eb, nt, c, tt; };
 
 // cum[j]: token tiles of the first j experts of the union (n_union + 1 words of shared memory). Every thread of the block calls it.

@@ -21,7 +21,8 @@
 // the stage's mbarrier. Consumer warps (16): mma.sync m16n8k32 (tokens x weight rows, s8 x s8) straight from shared memory; a lane's two
 // neighbouring cells are two weight rows of one token (packed FP32). Q8_0 blocks are 34 bytes: the quants of an even block start 2 (mod 4)
 // bytes in (two words and a byte permute per register), those of an odd block on a word.
-// Every wait is bounded; on a timeout the roles stop working and the launch sets B200MOE_JOB_WAIT_ABORTED in the job summary.
+// Every wait is bounded; on a timeout the roles stop working, the producers wait (bounded) for the copies in flight and the launch sets
+// B200MOE_JOB_WAIT_ABORTED in the job summary.
 #include <type_traits>
 
 #include "grouped_common.cuh"
@@ -51,7 +52,6 @@ constexpr u32 kOffSum = kStages * kStageBytes, kOffOut = kOffSum + kSumBytes, kO
               kOffCum = kOffTile + kTilePlaces * kTileWords * 4, kSmem = kOffCum + (kMaxUnion + 2) * 4;
 static_assert(kStageBytes % 128 == 0 && (32 * kUnitBytes) % 128 == 0 && kOffBars % 8 == 0, "TMA destinations, barriers");
 static_assert(kSmem > 114u * 1024u && kSmem <= 227u * 1024u, "one CTA per SM, within the shared memory of an SM");
-constexpr u32 kWaitLimit = 1u << 20;             // polls of up to a microsecond
 constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kProducerRegs = 64;
 constexpr u32 kConsumerRegs = (kGThreads * kLaunchRegs - kProducers * 32u * kProducerRegs) / (kConsumers * 32u) / 8u * 8u;
 static_assert(kConsumers * 32 * kConsumerRegs + kProducers * 32 * kProducerRegs <= kGThreads * kLaunchRegs, "setmaxnreg split exceeds the launch's registers");
@@ -69,6 +69,7 @@ struct Q8Args {
     u32 K;                   // hidden (gate/up) or inter (down)
     u32 delta_vec;           // the input's deltas lie in whole 16-byte units
     u32 raw_vec;             // raw lies on an 8-byte boundary
+    Waits waits;
 };
 
 // 16 tokens x 8 weight rows x one block. d[z]: token lane / 4 + 8 z, weight rows 2 (lane % 4) and the next.
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
     float* s_out = reinterpret_cast<float*>(smem + kOffOut);           // [kTokens][kOutPitch]
     u64* full = reinterpret_cast<u64*>(smem + kOffBars);
     u64* empty = full + kStages;
-    volatile u32* s_abort = reinterpret_cast<u32*>(empty + kStages);
+    volatile u32* s_abort = reinterpret_cast<u32*>(empty + kStages);   // and the stages that the first producer has asked for
     u32* s_tile = reinterpret_cast<u32*>(smem + kOffTile);             // [kTilePlaces][kTileWords]
     u32* cum = reinterpret_cast<u32*>(smem + kOffCum);                 // [kMaxUnion + 1]
 
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
         const u32 lt = tid - kConsumers * 32, hw = lt >> 5;
         const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, in_gs = in_stride / 32;
         u32 ring = 0, lap = 0, ik = 0, u = 0, cy = 0;    // u: unit of the next stage; cy: the tile's first weight row
+        u32 fed = 0;                                     // stages that this warp has asked for
         bool fresh = true;                               // the next stage begins a tile
         const i8* t_codes[kTokens / 8];                  // a half warp copies the 256 codes of one token
         const float* t_deltas = nullptr;                 // two threads copy the 8 deltas of one token
@@ -171,9 +173,11 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
                 look_ahead(ik + 1);
                 fresh = false;
             }
-            if (ok && lap) ok = mbar_wait(&empty[ring], (lap - 1u) & 1u, kWaitLimit, s_abort);
+            const bool feed = m < a.waits.stall_stage;
+            if (ok && feed && lap) ok = mbar_wait(&empty[ring], (lap - 1u) & 1u, a.waits.limit, s_abort);
             ok = __all_sync(0xffffffffu, ok);
-            if (ok) {
+            if (ok && feed) {
+                ++fed;
                 unsigned char* st = smem + ring * kStageBytes;
                 if (lt == 0) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the consumers' reads precede the copies below
@@ -202,9 +206,14 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
                 u = set == 0u ? 2u : set == 2u ? 1u : 3u;
             }
         }
+        // The last producer to leave has seen every copy land, on every path: a consumer's wait may run out after the last stage was asked for.
+        // A warp that gave up earlier than the first one makes up for its arrivals, so that the stages' phases complete.
         asm volatile("cp.async.wait_all;" ::: "memory");
-        if (!ok && lt == 0)  // wait (bounded) for the copies still in flight before the CTA retires
-            for (u32 i = 0; i < 400; ++i) __nanosleep(100);
+        if (lt == 0) s_abort[1] = fed;
+        asm volatile("bar.sync 1, %0;" ::"n"(kProducers * 32) : "memory");
+        const u32 asked = s_abort[1];
+        for (; fed < asked; ++fed) mbar_arrive(&full[fed % kStages]);
+        if (lt == 0) drain(full, kStages, asked, a.waits.limit);
     } else {
         // =============================================================================================== consumers
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
@@ -231,8 +240,8 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
                 while (left) {
                     const bool two = left > 1u;
                     const u32 next = ring + 1u == kStages ? 0u : ring + 1u, next_parity = parity ^ (next == 0u ? 1u : 0u);
-                    if (ok) ok = mbar_wait(&full[ring], parity, kWaitLimit, s_abort);
-                    if (ok && two) ok = mbar_wait(&full[next], next_parity, kWaitLimit, s_abort);
+                    if (ok) ok = mbar_wait(&full[ring], parity, a.waits.limit, s_abort);
+                    if (ok && two) ok = mbar_wait(&full[next], next_parity, a.waits.limit, s_abort);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     if (nt == 0) nt = ti[1];
@@ -360,7 +369,7 @@ int launch_gate_up_q8_grouped(const b200moe_gate_up_view& v, cudaStream_t stream
     if (v.max_union == 0) return B200MOE_OK;
     Q8Args a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.x; a.act = v.act; a.gate_out = v.gate_out; a.up_out = v.up_out; a.summary = v.summary;
-    a.n_row_tiles = v.shape.inter / 32; a.K = v.shape.hidden; a.delta_vec = delta_units(v.x);
+    a.n_row_tiles = v.shape.inter / 32; a.K = v.shape.hidden; a.delta_vec = delta_units(v.x); a.waits = debug_waits();
     CUtensorMap tm0, tm1;
     const u64 rb = u64(v.shape.hidden / 32) * kQ8Block, rows = u64(v.shape.experts) * v.shape.inter;
     if (int rc = wide::rows_map(v.weights.gate, rb, rows, kUnitBytes, 32, &tm0)) return rc;
@@ -374,7 +383,7 @@ int launch_down_q8_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     Q8Args a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.act; a.raw = v.raw; a.summary = const_cast<u32*>(v.summary);
-    a.n_row_tiles = v.shape.hidden / kRows; a.K = v.shape.inter; a.delta_vec = delta_units(v.act); a.raw_vec = aligned(v.raw, 8);
+    a.n_row_tiles = v.shape.hidden / kRows; a.K = v.shape.inter; a.delta_vec = delta_units(v.act); a.raw_vec = aligned(v.raw, 8); a.waits = debug_waits();
     CUtensorMap tm0;
     if (int rc = wide::rows_map(v.weights.down, u64(v.shape.inter / 32) * kQ8Block, u64(v.shape.experts) * v.shape.hidden, kUnitBytes, 32, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q8_kernel<true>), kSmem)) return rc;

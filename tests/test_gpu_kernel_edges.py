@@ -553,3 +553,41 @@ def test_grouped_forms_with_deltas_off_16_bytes(gpu, oracle, rows, types):
     act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), off(dv(deltas, gpu)), off(dv(sums, gpu))), rows, taps=True)
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
     assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, (act[0], off(act[1]), off(act[2]))).cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("types,H,I,stall", [((8, 8), 1024, 512, 1), ((8, 8), 1024, 1024, 3), ((8, 8), 256, 2560, 2)])
+def test_grouped_waits_run_out(gpu, oracle, types, H, I, stall):
+    """Producers that stop asking for copies before a stage (test hook): the consumers' waits run out, both launches return and set
+    B200MOE_JOB_WAIT_ABORTED, a down that sees the bit writes nothing; the same calls without the hooks give the oracle's bits."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(stall)
+    E, rows = 2, 70
+    gate, up, down = synth.expert_tensors(rng, E, H, I, *types)
+    ids = window(rng, E, 1, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, *types, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, 1, *types)
+    g, u, d = dv(gate, gpu), dv(up, gpu), dv(down, gpu)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    x = (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu))
+    good = ops.enqueue_routed_gate_up(sh, g, u, r, E, x, rows)
+    flags = torch.zeros(8, dtype=torch.int32, device=gpu)
+    b200moe.debug_set(b200moe.DEBUG_WAIT_LIMIT, 2048)
+    b200moe.debug_set(b200moe.DEBUG_STALL_STAGE, stall)
+    try:
+        ops.enqueue_routed_gate_up(sh, g, u, r, E, x, rows, summary=flags[:1])
+        torch.cuda.synchronize()
+        assert flags[0].item() & b200moe.JOB_WAIT_ABORTED
+        raw = torch.full((rows, H), 7.0, device=gpu)
+        ops.enqueue_routed_down(sh, d, r, E, good, raw=raw, summary=flags[:1])
+        assert bool((raw == 7.0).all())
+        ops.enqueue_routed_down(sh, d, r, E, good, summary=flags[4:5])
+        torch.cuda.synchronize()
+        assert flags[4].item() & b200moe.JOB_WAIT_ABORTED
+    finally:
+        b200moe.debug_set(b200moe.DEBUG_WAIT_LIMIT, 0)
+        b200moe.debug_set(b200moe.DEBUG_STALL_STAGE, 0)
+    act, gt, ut = ops.enqueue_routed_gate_up(sh, g, u, r, E, x, rows, taps=True)
+    assert same(gt.cpu(), want["gate"]) and same(ut.cpu(), want["up"])
+    assert same(ops.enqueue_routed_down(sh, d, r, E, act).cpu(), want["raw"])

@@ -30,7 +30,8 @@
 //     factors as one register for both halves. A row's factors are read once per 32 tokens, a token's once per 64 rows.
 //     The four chains of a row third meet through shared memory at the end of a tile, (a0 + a1) + (a2 + a3); gate/up then runs
 //     SwiGLU + the A8 rule, a warp four (token, 32 outputs) tasks at a time.
-// Every wait is bounded; on a timeout the roles stop working and the launch sets B200MOE_JOB_WAIT_ABORTED in the job summary.
+// Every wait is bounded; on a timeout the roles stop working, the first helper waits (bounded) for the copies in flight and the launch sets
+// B200MOE_JOB_WAIT_ABORTED in the job summary.
 #include <cuda.h>
 
 #include "grouped_common.cuh"
@@ -66,7 +67,8 @@ constexpr u32 kGroupedSmem = kOffCum + (kMaxUnion + 2) * 4;
 static_assert((kOutRows * kQ4KBlock) % 128 == 0 && kOffBars % 8 == 0, "TMA destinations, barriers");
 static_assert(kGN == 32 && kGM / 2 == (kHelpers - 1) * 32, "a helper lane stages a token, the helper threads before it two rows each");
 static_assert(kGroupedSmem > 114u * 1024u && kGroupedSmem <= 227u * 1024u, "one CTA per SM, within the shared memory of an SM");
-constexpr u32 kWaitLimit = 1u << 20;         // polls of up to a microsecond
+// Polls of up to a microsecond. Fixed here: a limit out of the arguments cost the consumers' loop 2 % (512 rows of the dense block 1170 -> 1194 us a call).
+constexpr u32 kWaitLimit = 1u << 20;
 // Register split between whole warp groups, out of what the launch gives every thread (65,536 over the threads, by eights).
 constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kHelperRegs = 80;
 constexpr u32 kConsumerRegs = (kGThreads * kLaunchRegs - kHelpers * 32u * kHelperRegs) / (kConsumers * 32u) / 8u * 8u;
@@ -92,6 +94,7 @@ struct GroupedArgs {
     u32 K;                   // hidden (gate/up) or inter (down)
     u32 es_vec;              // the input's deltas and sums lie in whole 16-byte units
     u32 raw_vec;             // raw lies on an 8-byte boundary
+    u32 stall_stage;         // test hook: the helpers stop asking for stages before this one
 };
 
 // One super-block of the warp's 64 rows and chain against NMT 16-token tiles. rows: weight row lane / 4 of the stage at the pair's
@@ -282,6 +285,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
         u32 slot = 0, lap = 0;
         for (u32 m = 0; m < total; ++m) {
             // decoded as soon as it has landed, up to two stages before the consumers need it
+            if (m == a.stall_stage) break;
             request();
             unsigned char* st = smem + slot * kStageBytes;
             asm volatile("cp.async.wait_all;" ::: "memory");
@@ -338,9 +342,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
             }
             if (++slot == kStages) { slot = 0; ++lap; }
         }
-        if (!ok && asked && lt == 0)  // wait (bounded) for the copies still in flight before the CTA retires
-            for (u32 i = 0; i < (kWaitLimit >> 8); ++i)
-                if (mbar_try_wait(&raw_full[(asked - 1u) % kStages], ((asked - 1u) / kStages) & 1u, kWaitHintNs)) break;
+        if (!ok && lt == 0) drain(raw_full, kStages, asked, kWaitLimit);  // else it has seen every stage land
     } else {
         // ================================================================================================ consumers
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
@@ -508,7 +510,7 @@ int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t strea
     GroupedArgs a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.x; a.act = v.act;
     a.gate_out = v.gate_out; a.up_out = v.up_out; a.row_status = v.row_status; a.summary = v.summary;
-    a.n_row_tiles = (v.shape.inter + kOutRows - 1) / kOutRows; a.K = v.shape.hidden; a.es_vec = es_units(v.x);
+    a.n_row_tiles = (v.shape.inter + kOutRows - 1) / kOutRows; a.K = v.shape.hidden; a.es_vec = es_units(v.x); a.stall_stage = debug_waits().stall_stage;
     CUtensorMap tm0, tm1;
     const u64 rb = u64(v.shape.hidden / 256) * kQ4KBlock, rows = u64(v.shape.experts) * v.shape.inter;
     if (int rc = encode_rows_map(v.weights.gate, rb, rows, &tm0)) return rc;
@@ -523,7 +525,7 @@ int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     GroupedArgs a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.act; a.raw = v.raw;
     a.summary = const_cast<u32*>(v.summary);
-    a.n_row_tiles = (v.shape.hidden + kGM - 1) / kGM; a.K = v.shape.inter; a.es_vec = es_units(v.act); a.raw_vec = aligned(v.raw, 8);
+    a.n_row_tiles = (v.shape.hidden + kGM - 1) / kGM; a.K = v.shape.inter; a.es_vec = es_units(v.act); a.raw_vec = aligned(v.raw, 8); a.stall_stage = debug_waits().stall_stage;
     CUtensorMap tm0;
     if (int rc = encode_rows_map(v.weights.down, u64(v.shape.inter / 256) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<true>), kGroupedSmem)) return rc;

@@ -555,10 +555,12 @@ def test_grouped_forms_with_deltas_off_16_bytes(gpu, oracle, rows, types):
     assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, (act[0], off(act[1]), off(act[2]))).cpu(), want["raw"])
 
 
-@pytest.mark.parametrize("types,H,I,stall", [((8, 8), 1024, 512, 1), ((8, 8), 1024, 1024, 3), ((8, 8), 256, 2560, 2)])
+@pytest.mark.parametrize("types,H,I,stall", [((8, 8), 1024, 512, 1), ((8, 8), 1024, 1024, 3), ((8, 8), 256, 2560, 2),
+                                              ((12, 12), 1024, 512, 1), ((12, 12), 1024, 1024, 3), ((12, 12), 256, 8192, 2)])
 def test_grouped_waits_run_out(gpu, oracle, types, H, I, stall):
-    """Producers that stop asking for copies before a stage (test hook): the consumers' waits run out, both launches return and set
-    B200MOE_JOB_WAIT_ABORTED, a down that sees the bit writes nothing; the same calls without the hooks give the oracle's bits."""
+    """Producers that stop asking for copies before a stage (test hook): the consumers' waits run out (the Q4_K kernel's after its fixed limit of
+    about a second), both launches return and set B200MOE_JOB_WAIT_ABORTED, a down that sees the bit writes nothing; the same calls without the
+    hooks give the oracle's bits."""
     import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(stall)

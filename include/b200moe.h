@@ -69,6 +69,8 @@ int b200moe_abi_version(void);
 const char* b200moe_last_error(void);
 /* Number of kernels this library has launched in the calling process (all threads); a plain counter for reports. */
 uint64_t b200moe_launch_count(void);
+/* Name of the kernel that this library launched last on the calling thread ("" when none): which form a call took. */
+const char* b200moe_last_launch(void);
 
 /* Test and measurement hooks: process-wide values read when a kernel is launched. They exist so that the tests can make a
  * bounded wait run out WITHOUT a device fault and so that the forms of the decode GEMVs can be compared on one input; a
@@ -78,9 +80,9 @@ uint64_t b200moe_launch_count(void);
                                       * (2^22; grouped Q8_0 2^20). The grouped Q4_K kernel's limit is fixed (2^20) */
 #define B200MOE_DEBUG_STALL_STAGE 1u /* n > 0: in every CTA of the Q4_K segment-streaming kernel the first producer, in every CTA of a grouped
                                       * kernel all producers stop feeding before their n-th stage (no copy of that stage is issued, none is left in flight); 0 = never */
-#define B200MOE_DEBUG_DECODE_FORM 2u /* decode windows: 0 = chosen by the plan, 1 = row streaming (Q4_K), 2 = segment streaming (Q4_K;
+#define B200MOE_DEBUG_DECODE_FORM 2u /* gate/up and down: 0 = chosen by the plan, 1 = row streaming (Q4_K), 2 = segment streaming (Q4_K;
                                       * Q8_0: the dp4a token-block form), 3 = per-block (Q8_0: one row per warp), 4 = the Q8_0
-                                      * tensor-core form, 5 = the grouped Q8_0 form (each only where it applies) */
+                                      * tensor-core form, 5 = the grouped form (each only where it applies; grouped_min_rows is not looked at then) */
 int b200moe_debug_set(uint32_t key, uint32_t value);
 
 /* ------------------------------------------------------------------------------------------------ A8 activations

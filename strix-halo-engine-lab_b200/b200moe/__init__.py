@@ -16,7 +16,7 @@ TYPE_Q8_0, TYPE_Q4_K = 8, 12
 ROW_INVALID_ROUTE, ROW_NONFINITE_ACTIVATION, ROW_INVALID_DELTA, ROW_PROJECTION_NONFINITE = 1, 2, 4, 8
 JOB_WAIT_ABORTED = 0x40000000
 DEBUG_WAIT_LIMIT, DEBUG_STALL_STAGE, DEBUG_DECODE_FORM = 0, 1, 2
-FORM_AUTO, FORM_ROW_STREAM, FORM_SEGMENT_STREAM, FORM_PER_BLOCK, FORM_TENSOR = 0, 1, 2, 3, 4
+FORM_AUTO, FORM_ROW_STREAM, FORM_SEGMENT_STREAM, FORM_PER_BLOCK, FORM_TENSOR, FORM_GROUPED = 0, 1, 2, 3, 4, 5
 SCORE_SOFTMAX, SCORE_SIGMOID, SCORE_SQRT_SOFTPLUS = 0, 1, 2
 KEY_FLOAT_SERIAL, KEY_ORDERED_BITS = 0, 1
 ORDER_SELECTION, ORDER_ASCENDING_ID = 0, 1
@@ -211,7 +211,7 @@ def enqueue(schema, view, stream=None, abi_revision=None, nbytes=None):
     return lib().b200moe_enqueue(C.byref(a), stream)
 
 
-EXPORTS = ["b200moe_abi_version", "b200moe_last_error", "b200moe_launch_count", "b200moe_debug_set", "b200moe_quantize_a8", "b200moe_rmsnorm_a8", "b200moe_q8_0_a8",
+EXPORTS = ["b200moe_abi_version", "b200moe_last_error", "b200moe_launch_count", "b200moe_last_launch", "b200moe_debug_set", "b200moe_quantize_a8", "b200moe_rmsnorm_a8", "b200moe_q8_0_a8",
            "b200moe_router", "b200moe_routes_scratch_words", "b200moe_build_routes", "b200moe_routes_static_max_words",
            "b200moe_build_routes_static", "b200moe_gate_row_bytes",
            "b200moe_down_row_bytes", "b200moe_expert_bytes", "b200moe_gate_up", "b200moe_down", "b200moe_combine",
@@ -240,6 +240,7 @@ def lib():
         L = C.CDLL(LIB_PATH)
         L.b200moe_last_error.restype = C.c_char_p
         L.b200moe_launch_count.restype = u64
+        L.b200moe_last_launch.restype = C.c_char_p
         L.b200moe_debug_set.restype = C.c_int
         L.b200moe_debug_set.argtypes = [u32, u32]
         for n in ("b200moe_gate_row_bytes", "b200moe_down_row_bytes", "b200moe_expert_bytes"):
@@ -353,6 +354,7 @@ def lib():
         L.b200moe_abi_version.restype = C.c_int
         L.b200moe_abi_version.argtypes = []
         L.b200moe_last_error.argtypes = []
+        L.b200moe_last_launch.argtypes = []
         L.b200moe_launch_count.argtypes = []
         _lib = L
     return _lib
@@ -365,6 +367,11 @@ def check(rc):
     if rc == ERR_INVALID_ARGUMENT:
         raise InvalidArgument(rc, text)
     raise B200MoeError(rc, text)
+
+
+def last_launch():
+    """Name of the kernel launched last on the calling thread: which form a call took."""
+    return lib().b200moe_last_launch().decode()
 
 
 def debug_set(key, value):

@@ -26,7 +26,12 @@ std::atomic<u64>& launch_counter() {
     static std::atomic<u64> n{0};
     return n;
 }
+const char*& last_launch_slot() {
+    thread_local const char* name = "";
+    return name;
+}
 int after_launch(const char* what) {
+    last_launch_slot() = what;
     launch_counter().fetch_add(1, std::memory_order_relaxed);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(B200MOE_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
@@ -241,27 +246,28 @@ cudaError_t clear_status(const LayerScratch& L, bool with_row_status, u32 rows, 
 // Where the segment-streaming form does not apply (more than 8192 slots, rows that bulk copies cannot take) the alternative is the
 // per-block form, and 128 rows are the line.
 constexpr u32 kGroupedEntries = 9, kGroupedRows = 64, kGroupedRowsWide = 32, kGroupedWideInter = 16384, kGroupedRowsElse = 128;
-bool use_grouped(const b200moe_shape& s, u32 rows, u32 grouped_min_rows, bool have_sums, bool streams) {
-    if (!grouped_fits(s, have_sums)) return false;
+bool grouped_pays(const b200moe_shape& s, u32 rows, u32 grouped_min_rows, bool streams) {
     if (grouped_min_rows) return rows >= grouped_min_rows;
     if (!streams) return rows >= kGroupedRowsElse;
     return u64(rows) * s.top_k >= u64(kGroupedEntries) * s.experts && rows >= (s.inter >= kGroupedWideInter ? kGroupedRowsWide : kGroupedRows);
 }
-// Decode forms of the Q4_K GEMVs: windows of one or two rows over rows of up to kRowStreamK weights take the row-streaming
+// The other forms of the Q4_K GEMVs: windows of one or two rows over rows of up to kRowStreamK weights take the row-streaming
 // form (a ring of whole rows, its work split fixed per CTA), everything else the segment-streaming form (any row length;
 // its items are dealt out dynamically), the per-block form being what is left. Measured on B200 at hidden 2048, 128
 // experts, top-8: one row 36.0 against 37.1 us per step, eight rows 76.5 against 70.4 us. B200MOE_DEBUG_DECODE_FORM forces
-// one of them where it applies.
+// one of the four where it applies, whatever grouped_min_rows says.
 constexpr u32 kRowStreamRows = 8, kRowStreamMaxRows = 2, kRowStreamK = 2048;
-enum class DecodeForm { row_stream, wide, block };
-DecodeForm pick_decode_form(bool row_stream_fits, bool wide_fits, u32 rows, u32 K) {
+enum class Q4Form { grouped, row_stream, wide, block };
+Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_fits, bool wide_fits, u32 rows, u32 grouped_min_rows, u32 K) {
     const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
-    if (forced == 1 && row_stream_fits) return DecodeForm::row_stream;
-    if (forced == 2 && wide_fits) return DecodeForm::wide;
-    if (forced == 3) return DecodeForm::block;
-    if (row_stream_fits && ((rows <= kRowStreamMaxRows && K <= kRowStreamK) || (rows <= kRowStreamRows && !wide_fits))) return DecodeForm::row_stream;
-    if (wide_fits) return DecodeForm::wide;
-    return row_stream_fits ? DecodeForm::row_stream : DecodeForm::block;
+    if (forced == 1 && row_stream_fits) return Q4Form::row_stream;
+    if (forced == 2 && wide_fits) return Q4Form::wide;
+    if (forced == 3) return Q4Form::block;
+    if (forced == 5 && grouped_fits) return Q4Form::grouped;
+    if (grouped_fits && grouped_pays(s, rows, grouped_min_rows, wide_fits)) return Q4Form::grouped;
+    if (row_stream_fits && ((rows <= kRowStreamMaxRows && K <= kRowStreamK) || (rows <= kRowStreamRows && !wide_fits))) return Q4Form::row_stream;
+    if (wide_fits) return Q4Form::wide;
+    return row_stream_fits ? Q4Form::row_stream : Q4Form::block;
 }
 // The DS41 family (Q8_0 x A8): one weight row per warp below kRowStreamRows rows; from there on the tensor-core form of
 // gemv_q8_mma.cu (rows of 1024 to 7168 weights), else the dp4a token-block form of gemv_q8_wide.cu. Measured on B200: a
@@ -301,21 +307,19 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
         }
     }
     if (v.shape.gate_type == B200MOE_TYPE_Q5_K) return launch_gate_up_q4k(v, st);  // the per-block form reads both K-quant layouts
-    const bool wide_fits = wide_gate_up_fits(v, rows);
-    if (use_grouped(v.shape, rows, grouped_min_rows, v.x.sums != nullptr, wide_fits)) return launch_gate_up_q4k_grouped(v, st);
-    switch (pick_decode_form(stream_gate_up_fits(v, rows), wide_fits, rows, v.shape.hidden)) {
-        case DecodeForm::row_stream: return launch_gate_up_q4k_stream(v, rows, st);
-        case DecodeForm::wide: return launch_gate_up_q4k_wide(v, rows, st);
+    switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.x.sums != nullptr), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, grouped_min_rows, v.shape.hidden)) {
+        case Q4Form::grouped: return launch_gate_up_q4k_grouped(v, st);
+        case Q4Form::row_stream: return launch_gate_up_q4k_stream(v, rows, st);
+        case Q4Form::wide: return launch_gate_up_q4k_wide(v, rows, st);
         default: return launch_gate_up_q4k(v, st);
     }
 }
 int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0) {
     if (v.shape.down_type == B200MOE_TYPE_Q4_K) {
-        const bool wide_fits = wide_down_fits(v, rows);
-        if (use_grouped(v.shape, rows, grouped_min_rows, v.act.sums != nullptr, wide_fits)) return launch_down_q4k_grouped(v, st);
-        switch (pick_decode_form(stream_down_fits(v, rows), wide_fits, rows, v.shape.inter)) {
-            case DecodeForm::row_stream: return launch_down_q4k_stream(v, rows, st);
-            case DecodeForm::wide: return launch_down_q4k_wide(v, rows, st);
+        switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.act.sums != nullptr), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, grouped_min_rows, v.shape.inter)) {
+            case Q4Form::grouped: return launch_down_q4k_grouped(v, st);
+            case Q4Form::row_stream: return launch_down_q4k_stream(v, rows, st);
+            case Q4Form::wide: return launch_down_q4k_wide(v, rows, st);
             default: return launch_down_q4k(v, st);
         }
     }
@@ -338,6 +342,7 @@ extern "C" {
 
 int b200moe_abi_version(void) { return B200MOE_ABI_VERSION; }
 const char* b200moe_last_error(void) { return last_error_slot().c_str(); }
+const char* b200moe_last_launch(void) { return last_launch_slot(); }
 uint64_t b200moe_launch_count(void) { return launch_counter().load(std::memory_order_relaxed); }
 int b200moe_debug_set(uint32_t key, uint32_t value) {
     B200_REQUIRE(key < 3, "debug_set: unknown key %u", key);

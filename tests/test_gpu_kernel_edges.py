@@ -85,9 +85,11 @@ def test_grouped_row_tiles_of_a_share(gpu, oracle, tokens, H, I, scale, special)
     assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, 4, act).cpu(), want["raw"])
 
 
-@pytest.mark.parametrize("rows,top_k,E,I", [(63, 1, 1, 512), (64, 1, 1, 512), (71, 2, 16, 256), (72, 2, 16, 256), (31, 1, 1, 16384), (32, 1, 1, 16384), (140, 1, 20, 256)])
-def test_grouped_form_lines(gpu, oracle, rows, top_k, E, I):
+@pytest.mark.parametrize("rows,top_k,E,I,form", [(63, 1, 1, 512, "wide"), (64, 1, 1, 512, "grouped"), (71, 2, 16, 256, "wide"), (72, 2, 16, 256, "grouped"),
+                                                 (31, 1, 1, 16384, "wide"), (32, 1, 1, 16384, "grouped"), (140, 1, 20, 256, "wide")])
+def test_grouped_form_lines(gpu, oracle, rows, top_k, E, I, form):
     """Both sides of the lines between the streaming and the grouped Q4_K form: 64 rows (32 of a wide block), nine entries an expert."""
+    import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(rows)
     H = 256
@@ -98,8 +100,10 @@ def test_grouped_form_lines(gpu, oracle, rows, top_k, E, I):
     sh = ops.make_shape(H, I, E, top_k, 12, 12)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
     act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
+    assert b200moe.last_launch() == "gate_up_q4k_" + form
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
-    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
+    raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+    assert b200moe.last_launch() == "down_q4k_" + form and same(raw.cpu(), want["raw"])
 
 
 @pytest.mark.parametrize("bits", [0x7c00, 0xfc00, 0x7e00])
@@ -191,7 +195,7 @@ def test_q8_grouped_units(gpu, oracle, tokens, H, I):
     sh = ops.make_shape(H, I, E, 1, 8, 8)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
     import b200moe
-    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, 5)
+    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_GROUPED)
     try:
         act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
         raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
@@ -201,10 +205,11 @@ def test_q8_grouped_units(gpu, oracle, tokens, H, I):
     assert same(raw.cpu(), want["raw"])
 
 
-@pytest.mark.parametrize("rows,top_k,E,H,I", [(19, 1, 1, 1024, 1024), (20, 1, 1, 1024, 1024), (24, 4, 10, 1024, 1024), (25, 4, 10, 1024, 1024),
-                                             (11, 1, 1, 512, 512), (12, 1, 1, 512, 512), (12, 4, 10, 512, 768), (13, 4, 10, 512, 768)])
-def test_q8_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I):
+@pytest.mark.parametrize("rows,top_k,E,H,I,form", [(19, 1, 1, 1024, 1024, "mma"), (20, 1, 1, 1024, 1024, "grouped"), (24, 4, 10, 1024, 1024, "mma"), (25, 4, 10, 1024, 1024, "grouped"),
+                                                   (11, 1, 1, 512, 512, "wide"), (12, 1, 1, 512, 512, "grouped"), (12, 4, 10, 512, 768, "wide"), (13, 4, 10, 512, 768, "grouped")])
+def test_q8_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I, form):
     """Both sides of the lines between the streaming and the grouped Q8_0 form, where the tensor-core form applies and where it does not."""
+    import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(rows)
     gate, up, down = synth.expert_tensors(rng, E, H, I, 8, 8)
@@ -214,8 +219,10 @@ def test_q8_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I):
     sh = ops.make_shape(H, I, E, top_k, 8, 8)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
     act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
+    assert b200moe.last_launch() == "gate_up_q8_" + form
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
-    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
+    raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+    assert b200moe.last_launch() == "down_q8_" + form and same(raw.cpu(), want["raw"])
 
 
 def declared_logits(x, w):
@@ -593,3 +600,30 @@ def test_grouped_waits_run_out(gpu, oracle, types, H, I, stall):
     act, gt, ut = ops.enqueue_routed_gate_up(sh, g, u, r, E, x, rows, taps=True)
     assert same(gt.cpu(), want["gate"]) and same(ut.cpu(), want["up"])
     assert same(ops.enqueue_routed_down(sh, d, r, E, act).cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("types,form,stem", [((12, 12), "FORM_SEGMENT_STREAM", "q4k_wide"), ((12, 12), "FORM_PER_BLOCK", "q4k"), ((12, 12), "FORM_GROUPED", "q4k_grouped"),
+                                             ((8, 8), "FORM_SEGMENT_STREAM", "q8_wide"), ((8, 8), "FORM_PER_BLOCK", "q8"), ((8, 8), "FORM_TENSOR", "q8_mma"),
+                                             ((8, 8), "FORM_GROUPED", "q8_grouped")])
+@pytest.mark.parametrize("rows,top_k", [(9, 1), (70, 2)])
+def test_forced_form_is_the_one_that_runs(gpu, oracle, types, form, stem, rows, top_k):
+    """A forced form beats the choice by rows and entries (70 entries an expert, where the plan takes the grouped forms, and about 4)."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows)
+    E, H, I = 2, 1024, 1024
+    gate, up, down = synth.expert_tensors(rng, E, H, I, *types)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, *types, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, top_k, *types)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, getattr(b200moe, form))
+    try:
+        act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
+        assert b200moe.last_launch() == "gate_up_" + stem
+        raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+        assert b200moe.last_launch() == "down_" + stem
+    finally:
+        b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_AUTO)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])

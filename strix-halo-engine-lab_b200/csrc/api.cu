@@ -1,5 +1,6 @@
 // The C ABI (include/b200moe.h): host-side validation and composition. Argument errors are reported before anything
 // is enqueued; nothing here allocates, synchronises (except b200moe_ffn_host, which says so) or starts threads.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -269,25 +270,44 @@ Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_f
     if (wide_fits) return Q4Form::wide;
     return row_stream_fits ? Q4Form::row_stream : Q4Form::block;
 }
+// What a window is for the kernels that walk it item by item, known from its sizes alone: the items of eight entries and the tiles of 32 that
+// its experts make when the entries are spread evenly (the last item of an expert is half full on average, and an expert has one tile until it has
+// about 20 entries), and whether a tile has 16 entries at most.
+struct Window { u64 items8, tiles32; bool few; };
+Window window_of(const b200moe_shape& s, u32 rows, u32 max_union) {
+    if (s.experts == 1) return Window{(u64(rows) + 7) / 8, (u64(rows) + 31) / 32, rows <= 16};
+    const u64 e16 = 16 * u64(rows) * s.top_k / s.experts;  // entries an expert, in sixteenths
+    return Window{(max_union * std::max<u64>(16, e16 / 8 + 7) + 15) / 16, (max_union * std::max<u64>(16, (e16 + 192) / 32) + 15) / 16, e16 <= 12 * 16};
+}
+u64 waves(u64 items, u64 at_once) { return (items + at_once - 1) / at_once; }
 // The DS41 family (Q8_0 x A8): one weight row per warp below kRowStreamRows rows; from there on the tensor-core form of
 // gemv_q8_mma.cu (rows of 1024 to 7168 weights), else the dp4a token-block form of gemv_q8_wide.cu. Measured on B200: a
 // 7168 x 2048 dense block over 8 rows takes 49 + 18 us in the dp4a token-block form against 55 + 30 us with one row per
 // warp; one row over four experts of 2048 x 1024 is 2 us faster with one row per warp.
-// The grouped form (grouped_q8.cu, tiles of 32 entries) takes over from the tensor-core form at 10 entries an expert and 20 rows: whole calls, the
-// two in this order, 64 experts of 2048 x 1024: 199 and 236 us with 6 entries, 249 and 239 with 8, 328 and 240 with 12; 16 experts of
-// 4096 x 1536: 167 and 188 with 8, 241 and 196 with 16; one expert of 7168 x 2048: 49 and 64 us with 16 rows, 63 and 61 with 24, 101
-// and 66 with 64. Where the tensor-core form does not apply (rows below 1024 or above 7168 weights) it takes over from the dp4a form at 5
-// entries and 12 rows: down of 32 experts of 1536 x 768 94 and 107 us a call with 2.6 entries, 108 and 109 with 5.2, 124 and 116 with 7.5; of
-// 48 of 2048 x 512 120 and 120 with 4, 136 and 124 with 6; one expert of 4096 x 12288 78 and 84 us with 8 rows, 107 and 104 with 12, 152
-// and 110 with 24.
+// The grouped form (grouped_q8.cu, tiles of 32 entries) takes over from the tensor-core form where its waves of tiles take less time than the
+// other's waves of items, both by their sizes: a tile 1.9 us + 0.605 a unit of 256 columns with up to 16 entries, 2.6 + 0.77 with more, an item of
+// 32 gate and up rows 3 us + 0.33 a unit, one of 32 down rows half of that. Tensor-core and grouped form, gate/up and down: one expert of
+// 2048 x 17408 28.8 and 32.3 us with 8 rows, 51.4 and 32.9 with 16, 72 and 39 with 20; of 7168 x 2048 18.6 and 22.8, 16.5 and 12.4 with 16 rows; of
+// 1024 x 1024 8.4 and 10.3 (down) with 20; four of 2048 x 4096, top-2, 45 and 33, 22 and 16.6 with 20 rows; 64 of 2048 x 1024, top-4, 94.5 and
+// 94.8, 71 and 68 with 96 rows, 117 and 95.5, 84 and 68 with 128; 16 of 4096 x 1536, top-2, 69 and 74, 53 and 43 with 64. The rule takes the better
+// form in all but four of 336 such launches (8 to 192 rows, 1 to 64 experts), within 1 % of it there. Where the tensor-core form does not apply (rows below
+// 1024 or above 7168 weights) the grouped one takes over from the dp4a form at 4 entries an expert: down of 48 experts of 2048 x 512 36.8 and 39 us with 3,
+// 41 and 38.5 with 4, 49 and 39 with 5; of 32 of 1536 x 768 29 and 28 with 4.5; one expert of 2048 x 17408 45 and 43 us with 8 rows, 53.4 and 53.5 with
+// 17, of 4096 x 12288 35 and 33 with 8, 84 and 40 with 24.
 enum class Q8Form { row_per_warp, wide, mma, grouped };
-bool q8_grouped_pays(bool mma_fits, u32 rows, const b200moe_shape& s) {
-    return rows >= (mma_fits ? 20u : 12u) && u64(rows) * s.top_k >= u64(mma_fits ? 10u : 5u) * s.experts;
+bool q8_grouped_pays(const b200moe_shape& s, bool mma_fits, u32 rows, u32 max_union, bool down) {
+    if (rows < kRowStreamRows) return false;
+    if (!mma_fits) return u64(rows) * s.top_k >= u64(4) * s.experts;
+    const Window w = window_of(s, rows, max_union);
+    const u64 units = (down ? s.inter : s.hidden) / 256, sms = static_cast<u64>(device_sm_count());
+    const u64 tile = w.few ? 1900 + 605 * units : 2600 + 770 * units, item = (3000 + 330 * units) / (down ? 2 : 1);  // ns
+    const u64 grouped = waves(w.tiles32 * (down ? s.hidden / 64 : s.inter / 32), sms) * tile, tensor = waves(w.items8 * ((down ? s.hidden : s.inter) / 32), sms) * item;
+    return grouped < tensor;
 }
-Q8Form pick_q8_form(bool wide_fits, bool mma_fits, bool grouped_fits, u32 rows, const b200moe_shape& s) {
+Q8Form pick_q8_form(const b200moe_shape& s, bool wide_fits, bool mma_fits, bool grouped_fits, u32 rows, u32 max_union, bool down) {
     const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
     if (forced == 3) return Q8Form::row_per_warp;
-    if (grouped_fits && (forced == 5 || (forced == 0 && q8_grouped_pays(mma_fits, rows, s)))) return Q8Form::grouped;
+    if (grouped_fits && (forced == 5 || (forced == 0 && q8_grouped_pays(s, mma_fits, rows, max_union, down)))) return Q8Form::grouped;
     if (forced == 4 && mma_fits) return Q8Form::mma;
     if (forced == 2 && wide_fits) return Q8Form::wide;
     if (forced == 0 && rows >= kRowStreamRows) {
@@ -299,7 +319,7 @@ Q8Form pick_q8_form(bool wide_fits, bool mma_fits, bool grouped_fits, u32 rows, 
 int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0) {
     if (v.shape.gate_type == B200MOE_TYPE_Q2_K) return launch_gate_up_ds41_any(v, st);  // the generic form of the family reads every block type
     if (!is_kquant(v.shape.gate_type)) {
-        switch (pick_q8_form(q8_wide_gate_up_fits(v, rows), q8_mma_gate_up_fits(v, rows), grouped_q8_gate_up_fits(v), rows, v.shape)) {
+        switch (pick_q8_form(v.shape, q8_wide_gate_up_fits(v, rows), q8_mma_gate_up_fits(v, rows), grouped_q8_gate_up_fits(v), rows, v.max_union, false)) {
             case Q8Form::grouped: return launch_gate_up_q8_grouped(v, st);
             case Q8Form::mma: return launch_gate_up_q8_mma(v, rows, st);
             case Q8Form::wide: return launch_gate_up_q8_wide(v, rows, st);
@@ -325,7 +345,7 @@ int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grou
     }
     if (is_kquant(v.shape.gate_type)) return launch_down_q8_chain4(v, st);  // chain4: Q8_0 and Q5_1 blocks
     if (v.shape.down_type == B200MOE_TYPE_Q2_K) return launch_down_ds41_any(v, st);
-    switch (pick_q8_form(q8_wide_down_fits(v, rows), q8_mma_down_fits(v, rows), grouped_q8_down_fits(v), rows, v.shape)) {
+    switch (pick_q8_form(v.shape, q8_wide_down_fits(v, rows), q8_mma_down_fits(v, rows), grouped_q8_down_fits(v), rows, v.max_union, true)) {
         case Q8Form::grouped: return launch_down_q8_grouped(v, st);
         case Q8Form::mma: return launch_down_q8_mma(v, rows, st);
         case Q8Form::wide: return launch_down_q8_wide(v, rows, st);

@@ -1,6 +1,7 @@
 """Edges of the kernels that large windows and small staged launches take: remainders of tiles and chunks, both sides of each
 dispatch rule, layouts that fall back to narrower copies, and values that are not finite. Bit for bit, against the CPU oracle or
 a NumPy restatement of the declared order."""
+import contextlib
 import os
 import subprocess
 import sys
@@ -32,6 +33,16 @@ def same(a, b):
     a, b = np.ascontiguousarray(a, np.float32), np.ascontiguousarray(b, np.float32)
     nan = np.isnan(a) & np.isnan(b)
     return np.array_equal(np.where(nan, 0, a.view(np.uint32)), np.where(nan, 0, b.view(np.uint32)))
+
+
+@contextlib.contextmanager
+def forced(form):
+    import b200moe
+    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, form)
+    try:
+        yield
+    finally:
+        b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_AUTO)
 
 
 def window(rng, E, K, rows):
@@ -205,10 +216,14 @@ def test_q8_grouped_units(gpu, oracle, tokens, H, I):
     assert same(raw.cpu(), want["raw"])
 
 
-@pytest.mark.parametrize("rows,top_k,E,H,I,form", [(19, 1, 1, 1024, 1024, "mma"), (20, 1, 1, 1024, 1024, "grouped"), (24, 4, 10, 1024, 1024, "mma"), (25, 4, 10, 1024, 1024, "grouped"),
-                                                   (11, 1, 1, 512, 512, "wide"), (12, 1, 1, 512, 512, "grouped"), (12, 4, 10, 512, 768, "wide"), (13, 4, 10, 512, 768, "grouped")])
-def test_q8_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I, form):
-    """Both sides of the lines between the streaming and the grouped Q8_0 form, where the tensor-core form applies and where it does not."""
+@pytest.mark.parametrize("rows,top_k,E,H,I,gate_form,down_form", [
+    (8, 1, 1, 1024, 7168, "q8_mma", "q8_mma"), (9, 1, 1, 1024, 7168, "q8_grouped", "q8_mma"), (16, 1, 1, 1024, 7168, "q8_grouped", "q8_mma"),
+    (17, 4, 10, 1024, 1024, "q8_mma", "q8_mma"), (18, 4, 10, 1024, 1024, "q8_grouped", "q8_mma"), (40, 4, 10, 1024, 1024, "q8_grouped", "q8_grouped"),
+    (20, 2, 2, 1024, 9728, "q8_grouped", "q8_grouped"), (7, 1, 1, 512, 512, "q8", "q8"), (8, 1, 1, 512, 512, "q8_grouped", "q8_grouped"),
+    (9, 4, 10, 512, 768, "q8_wide", "q8_wide"), (10, 4, 10, 512, 768, "q8_grouped", "q8_grouped")])
+def test_q8_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I, gate_form, down_form):
+    """Both sides of the lines between the streaming and the grouped Q8_0 form, where the tensor-core form applies and where it does not: gate/up and
+    down choose each for itself."""
     import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(rows)
@@ -219,10 +234,10 @@ def test_q8_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I, form):
     sh = ops.make_shape(H, I, E, top_k, 8, 8)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
     act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
-    assert b200moe.last_launch() == "gate_up_q8_" + form
+    assert b200moe.last_launch() == "gate_up_" + gate_form
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
     raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
-    assert b200moe.last_launch() == "down_q8_" + form and same(raw.cpu(), want["raw"])
+    assert b200moe.last_launch() == "down_" + down_form and same(raw.cpu(), want["raw"])
 
 
 def declared_logits(x, w):
@@ -514,12 +529,14 @@ def test_selection_scratch_beside_static_shared_memory(gpu, rows, experts):
     assert r.returncode == 0, r.stderr[-2000:]
 
 
-@pytest.mark.parametrize("rows,top_k,E,types", [(9, 1, 1, (12, 12)), (40, 2, 10, (12, 12)), (160, 2, 64, (12, 12)), (70, 1, 1, (12, 12)), (24, 1, 1, (8, 8)),
-                                                (9, 1, 1, (8, 8))])
-def test_down_into_a_slice_on_a_4_byte_boundary(gpu, oracle, rows, top_k, E, types):
+@pytest.mark.parametrize("rows,top_k,E,types,form", [(9, 1, 1, (12, 12), 2), (40, 2, 10, (12, 12), 2), (160, 2, 64, (12, 12), 0), (70, 1, 1, (12, 12), 5), (24, 1, 1, (8, 8), 5),
+                                                     (9, 1, 1, (8, 8), 2)])
+def test_down_into_a_slice_on_a_4_byte_boundary(gpu, oracle, rows, top_k, E, types, form):
     """raw one float past an 8-byte boundary: streaming windows below and above 128 rows with experts of five entries and more, the grouped and
     the Q8_0 forms; a dense block's y is such a raw too. The word before and the words after it are left alone."""
+    import b200moe
     from b200moe import ops, synth
+    forms = {0: "q4k_wide", b200moe.FORM_SEGMENT_STREAM: {12: "q4k_wide", 8: "q8_wide"}[types[0]], b200moe.FORM_GROUPED: {12: "q4k_grouped", 8: "q8_grouped"}[types[0]]}
     rng = np.random.default_rng(rows)
     H, I = 256, 256
     gate, up, down = synth.expert_tensors(rng, E, H, I, *types)
@@ -533,13 +550,17 @@ def test_down_into_a_slice_on_a_4_byte_boundary(gpu, oracle, rows, top_k, E, typ
     flat = torch.full((rows * top_k * H + 3,), -7.0, device=gpu)
     raw = flat[1:1 + rows * top_k * H].view(rows * top_k, H)
     assert raw.data_ptr() % 8 == 4
-    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act, raw=raw).cpu(), want["raw"])
+    with forced(form):
+        ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act, raw=raw)
+        assert b200moe.last_launch() == "down_" + forms[form]
+    assert same(raw.cpu(), want["raw"])
     assert flat[0].item() == -7.0 and bool((flat[1 + rows * top_k * H:] == -7.0).all())
 
 
 @pytest.mark.parametrize("rows,types", [(70, (12, 12)), (33, (8, 8))])
 def test_grouped_forms_with_deltas_off_16_bytes(gpu, oracle, rows, types):
     """Deltas and sums 8 bytes past a 16-byte boundary: the grouped forms copy them a word at a time."""
+    import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(rows)
     E, H, I = 2, 256, 512
@@ -557,9 +578,10 @@ def test_grouped_forms_with_deltas_off_16_bytes(gpu, oracle, rows, types):
 
     sh = ops.make_shape(H, I, E, 1, *types)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
-    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), off(dv(deltas, gpu)), off(dv(sums, gpu))), rows, taps=True)
-    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
-    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, (act[0], off(act[1]), off(act[2]))).cpu(), want["raw"])
+    with forced(b200moe.FORM_GROUPED):
+        act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), off(dv(deltas, gpu)), off(dv(sums, gpu))), rows, taps=True)
+        raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, (act[0], off(act[1]), off(act[2])))
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
 
 
 @pytest.mark.parametrize("types,H,I,stall", [((8, 8), 1024, 512, 1), ((8, 8), 1024, 1024, 3), ((8, 8), 256, 2560, 2),
@@ -582,6 +604,7 @@ def test_grouped_waits_run_out(gpu, oracle, types, H, I, stall):
     x = (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu))
     good = ops.enqueue_routed_gate_up(sh, g, u, r, E, x, rows)
     flags = torch.zeros(8, dtype=torch.int32, device=gpu)
+    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_GROUPED)
     b200moe.debug_set(b200moe.DEBUG_WAIT_LIMIT, 2048)
     b200moe.debug_set(b200moe.DEBUG_STALL_STAGE, stall)
     try:
@@ -595,11 +618,12 @@ def test_grouped_waits_run_out(gpu, oracle, types, H, I, stall):
         torch.cuda.synchronize()
         assert flags[4].item() & b200moe.JOB_WAIT_ABORTED
     finally:
-        b200moe.debug_set(b200moe.DEBUG_WAIT_LIMIT, 0)
-        b200moe.debug_set(b200moe.DEBUG_STALL_STAGE, 0)
-    act, gt, ut = ops.enqueue_routed_gate_up(sh, g, u, r, E, x, rows, taps=True)
-    assert same(gt.cpu(), want["gate"]) and same(ut.cpu(), want["up"])
-    assert same(ops.enqueue_routed_down(sh, d, r, E, act).cpu(), want["raw"])
+        for key in (b200moe.DEBUG_DECODE_FORM, b200moe.DEBUG_WAIT_LIMIT, b200moe.DEBUG_STALL_STAGE):
+            b200moe.debug_set(key, 0)
+    with forced(b200moe.FORM_GROUPED):
+        act, gt, ut = ops.enqueue_routed_gate_up(sh, g, u, r, E, x, rows, taps=True)
+        raw = ops.enqueue_routed_down(sh, d, r, E, act)
+    assert same(gt.cpu(), want["gate"]) and same(ut.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
 
 
 @pytest.mark.parametrize("types,form,stem", [((12, 12), "FORM_SEGMENT_STREAM", "q4k_wide"), ((12, 12), "FORM_PER_BLOCK", "q4k"), ((12, 12), "FORM_GROUPED", "q4k_grouped"),

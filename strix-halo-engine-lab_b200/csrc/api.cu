@@ -235,41 +235,6 @@ cudaError_t clear_status(const LayerScratch& L, bool with_row_status, u32 rows, 
     return cudaMemsetAsync(L.summary, 0, static_cast<size_t>(e - b), st);
 }
 
-// Plan by window size, chosen on the host from the row count (no environment reads inside numerical code): decode
-// windows of Q4_K experts take the persistent bulk-copy form, everything else the plain per-block form.
-// grouped_min_rows: 0 = chosen here; windows of at least that many rows take the grouped form.
-// What decides is the number of entries an expert has (the grouped form's tiles hold 32, a streaming item 8), and that there is work for
-// its latency. Whole calls, streaming against grouped: 128 experts of 2048 x 768 215 and 231 us with 8 entries, 256 and 242 with 10, 342 and
-// 268 with 16; 60 of 4096 x 1536 350 and 363 with 9.6, 432 and 378 with 12.8; 160 of 1024 x 512 150 and 161 with 6.4, 192 and 176 with 9.6;
-// 64 of 7168 x 2048 675 and 750 with 8, 909 and 832 with 12; 32 of 1536 x 1024 98 and 101 us with 32 rows (8 entries), 127 and 114 with 64.
-// One expert (a dense block): 5120 x 17408 179 and 227 us with 24 rows, 242 and 226 with 32, 427 and 268 with 64; 7168 x 18432 273 and 266,
-// 319 and 264, 580 and 321; 3584 x 14336 152 and 182 with 32 rows, 264 and 212 with 64; 2048 x 8192 104 and 119 with 64, 163 and 135 with 100.
-// Where the segment-streaming form does not apply (more than 8192 slots, rows that bulk copies cannot take) the alternative is the
-// per-block form, and 128 rows are the line.
-constexpr u32 kGroupedEntries = 9, kGroupedRows = 64, kGroupedRowsWide = 32, kGroupedWideInter = 16384, kGroupedRowsElse = 128;
-bool grouped_pays(const b200moe_shape& s, u32 rows, u32 grouped_min_rows, bool streams) {
-    if (grouped_min_rows) return rows >= grouped_min_rows;
-    if (!streams) return rows >= kGroupedRowsElse;
-    return u64(rows) * s.top_k >= u64(kGroupedEntries) * s.experts && rows >= (s.inter >= kGroupedWideInter ? kGroupedRowsWide : kGroupedRows);
-}
-// The other forms of the Q4_K GEMVs: windows of one or two rows over rows of up to kRowStreamK weights take the row-streaming
-// form (a ring of whole rows, its work split fixed per CTA), everything else the segment-streaming form (any row length;
-// its items are dealt out dynamically), the per-block form being what is left. Measured on B200 at hidden 2048, 128
-// experts, top-8: one row 36.0 against 37.1 us per step, eight rows 76.5 against 70.4 us. B200MOE_DEBUG_DECODE_FORM forces
-// one of the four where it applies, whatever grouped_min_rows says.
-constexpr u32 kRowStreamRows = 8, kRowStreamMaxRows = 2, kRowStreamK = 2048;
-enum class Q4Form { grouped, row_stream, wide, block };
-Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_fits, bool wide_fits, u32 rows, u32 grouped_min_rows, u32 K) {
-    const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
-    if (forced == 1 && row_stream_fits) return Q4Form::row_stream;
-    if (forced == 2 && wide_fits) return Q4Form::wide;
-    if (forced == 3) return Q4Form::block;
-    if (forced == 5 && grouped_fits) return Q4Form::grouped;
-    if (grouped_fits && grouped_pays(s, rows, grouped_min_rows, wide_fits)) return Q4Form::grouped;
-    if (row_stream_fits && ((rows <= kRowStreamMaxRows && K <= kRowStreamK) || (rows <= kRowStreamRows && !wide_fits))) return Q4Form::row_stream;
-    if (wide_fits) return Q4Form::wide;
-    return row_stream_fits ? Q4Form::row_stream : Q4Form::block;
-}
 // What a window is for the kernels that walk it item by item, known from its sizes alone: the items of eight entries and the tiles of 32 that
 // its experts make when the entries are spread evenly (the last item of an expert is half full on average, and an expert has one tile until it has
 // about 20 entries), and whether a tile has 16 entries at most.
@@ -280,6 +245,51 @@ Window window_of(const b200moe_shape& s, u32 rows, u32 max_union) {
     return Window{(max_union * std::max<u64>(16, e16 / 8 + 7) + 15) / 16, (max_union * std::max<u64>(16, (e16 + 192) / 32) + 15) / 16, e16 <= 12 * 16};
 }
 u64 waves(u64 items, u64 at_once) { return (items + at_once - 1) / at_once; }
+// Plan by window size, chosen on the host from the sizes (no environment reads inside numerical code): decode
+// windows of Q4_K experts take the persistent bulk-copy forms, prompts the grouped form.
+// grouped_min_rows: windows of at least that many rows take the grouped form; 0 = chosen here, for gate/up and down each.
+// Where the segment-streaming form applies, the grouped one (tiles of 32 entries) takes over from it (items of 8) where its waves take less time,
+// both by their sizes: a tile 2 us + 1.75 a super-block of its rows; an item 1.2 us + 0.7 a super-block (2 + 0.7 where rows have less than three and a
+// stage holds one), two an SM, or 0.5 a super-block where there are no more items than SMs. Streaming and grouped form, gate/up and down: one expert of
+// 5120 x 17408 139 and 90 us, 103 and 126 with 32 rows, 254 and 129, 160 and 126 with 64; of 2048 x 17408 68 and 45, 39 and 126 with 32, 119 and 64, 60
+// and 125 with 64 (11 down tiles); of 2048 x 8192 60 and 45, 33 and 62 with 64; of 256 x 512 8.4 and 12.4, 9 and 10.4 with 64; 128 of 2048 x 768, top-8,
+// 105 and 116, 58 and 71 with 128 rows, 146 and 118, 77 and 73 with 192; 64 of 7168 x 2048, top-8, 466 and 488, 239 and 256 with 80, 545 and 491,
+// 279 and 253 with 96; 96 of 2560 x 1280, top-2, 170 and 186, 88 and 101 with 432; 16 of 2048 x 1024, top-2, 33 and 36, 21 and 21 with 96. Over 199
+// windows (16 to 1000 rows, 1 to 160 experts) the two launches together take at most 2.5 % longer than in the streaming form. The estimate is good
+// to a few percent; below 32 rows it has not been followed, below 48 only where it sees a quarter of the time gained.
+// Where the segment-streaming form does not apply (more than 8192 slots, rows that bulk copies cannot take) the alternative is the
+// per-block form, and 128 rows are the line.
+constexpr u32 kGroupedLeastRows = 32, kGroupedSureRows = 48, kGroupedRowsElse = 128;
+bool grouped_pays(const b200moe_shape& s, u32 rows, u32 max_union, u32 grouped_min_rows, bool streams, bool down) {
+    if (grouped_min_rows) return rows >= grouped_min_rows;
+    if (!streams) return rows >= kGroupedRowsElse;
+    if (rows < kGroupedLeastRows) return false;
+    const Window w = window_of(s, rows, max_union);
+    const u64 blocks = (down ? s.inter : s.hidden) / 256, sms = static_cast<u64>(device_sm_count());
+    const u64 items = w.items8 * (down ? s.hidden / 64 : s.inter / 32), start = blocks < 3 ? 2000 : 1200;  // ns
+    const u64 streaming = items <= sms ? start + 500 * blocks : waves(items, 2 * sms) * (start + 700 * blocks);
+    const u64 grouped = waves(w.tiles32 * grouped_row_tiles(down ? s.hidden : s.inter, down), sms) * (2000 + 1750 * blocks);
+    return grouped * (rows < kGroupedSureRows ? 13 : 10) < streaming * 10;
+}
+// The other forms of the Q4_K GEMVs: windows of one or two rows over rows of up to kRowStreamK weights take the row-streaming
+// form (a ring of whole rows, its work split fixed per CTA), everything else the segment-streaming form (any row length;
+// its items are dealt out dynamically), the per-block form being what is left. Measured on B200 at hidden 2048, 128
+// experts, top-8: one row 36.0 against 37.1 us per step, eight rows 76.5 against 70.4 us. B200MOE_DEBUG_DECODE_FORM forces
+// one of the four where it applies, whatever grouped_min_rows says.
+constexpr u32 kRowStreamRows = 8, kRowStreamMaxRows = 2, kRowStreamK = 2048;
+enum class Q4Form { grouped, row_stream, wide, block };
+Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_fits, bool wide_fits, u32 rows, u32 max_union, u32 grouped_min_rows, bool down) {
+    const u32 K = down ? s.inter : s.hidden;
+    const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
+    if (forced == 1 && row_stream_fits) return Q4Form::row_stream;
+    if (forced == 2 && wide_fits) return Q4Form::wide;
+    if (forced == 3) return Q4Form::block;
+    if (forced == 5 && grouped_fits) return Q4Form::grouped;
+    if (grouped_fits && grouped_pays(s, rows, max_union, grouped_min_rows, wide_fits, down)) return Q4Form::grouped;
+    if (row_stream_fits && ((rows <= kRowStreamMaxRows && K <= kRowStreamK) || (rows <= kRowStreamRows && !wide_fits))) return Q4Form::row_stream;
+    if (wide_fits) return Q4Form::wide;
+    return row_stream_fits ? Q4Form::row_stream : Q4Form::block;
+}
 // The DS41 family (Q8_0 x A8): one weight row per warp below kRowStreamRows rows; from there on the tensor-core form of
 // gemv_q8_mma.cu (rows of 1024 to 7168 weights), else the dp4a token-block form of gemv_q8_wide.cu. Measured on B200: a
 // 7168 x 2048 dense block over 8 rows takes 49 + 18 us in the dp4a token-block form against 55 + 30 us with one row per
@@ -289,8 +299,8 @@ u64 waves(u64 items, u64 at_once) { return (items + at_once - 1) / at_once; }
 // 32 gate and up rows 3 us + 0.33 a unit, one of 32 down rows half of that. Tensor-core and grouped form, gate/up and down: one expert of
 // 2048 x 17408 28.8 and 32.3 us with 8 rows, 51.4 and 32.9 with 16, 72 and 39 with 20; of 7168 x 2048 18.6 and 22.8, 16.5 and 12.4 with 16 rows; of
 // 1024 x 1024 8.4 and 10.3 (down) with 20; four of 2048 x 4096, top-2, 45 and 33, 22 and 16.6 with 20 rows; 64 of 2048 x 1024, top-4, 94.5 and
-// 94.8, 71 and 68 with 96 rows, 117 and 95.5, 84 and 68 with 128; 16 of 4096 x 1536, top-2, 69 and 74, 53 and 43 with 64. The rule takes the better
-// form in all but four of 336 such launches (8 to 192 rows, 1 to 64 experts), within 1 % of it there. Where the tensor-core form does not apply (rows below
+// 94.8, 71 and 68 with 96 rows, 117 and 95.5, 84 and 68 with 128; 16 of 4096 x 1536, top-2, 69 and 74, 53 and 43 with 64. Over 336 such
+// launches (8 to 192 rows, 1 to 64 experts) the rule takes the better form, or one within 3.5 % of it. Where the tensor-core form does not apply (rows below
 // 1024 or above 7168 weights) the grouped one takes over from the dp4a form at 4 entries an expert: down of 48 experts of 2048 x 512 36.8 and 39 us with 3,
 // 41 and 38.5 with 4, 49 and 39 with 5; of 32 of 1536 x 768 29 and 28 with 4.5; one expert of 2048 x 17408 45 and 43 us with 8 rows, 53.4 and 53.5 with
 // 17, of 4096 x 12288 35 and 33 with 8, 84 and 40 with 24.
@@ -327,7 +337,7 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
         }
     }
     if (v.shape.gate_type == B200MOE_TYPE_Q5_K) return launch_gate_up_q4k(v, st);  // the per-block form reads both K-quant layouts
-    switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.x.sums != nullptr), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, grouped_min_rows, v.shape.hidden)) {
+    switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.x.sums != nullptr), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, v.max_union, grouped_min_rows, false)) {
         case Q4Form::grouped: return launch_gate_up_q4k_grouped(v, st);
         case Q4Form::row_stream: return launch_gate_up_q4k_stream(v, rows, st);
         case Q4Form::wide: return launch_gate_up_q4k_wide(v, rows, st);
@@ -336,7 +346,7 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
 }
 int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0) {
     if (v.shape.down_type == B200MOE_TYPE_Q4_K) {
-        switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.act.sums != nullptr), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, grouped_min_rows, v.shape.inter)) {
+        switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.act.sums != nullptr), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, v.max_union, grouped_min_rows, true)) {
             case Q4Form::grouped: return launch_down_q4k_grouped(v, st);
             case Q4Form::row_stream: return launch_down_q4k_stream(v, rows, st);
             case Q4Form::wide: return launch_down_q4k_wide(v, rows, st);

@@ -504,13 +504,14 @@ int grid_size() {
 }  // namespace
 
 bool grouped_fits(const b200moe_shape& s, bool have_sums) { return have_sums && grouped_shape_ok(s); }
+u32 grouped_row_tiles(u32 outputs, bool down) { return (outputs + (down ? kGM : kOutRows) - 1) / (down ? kGM : kOutRows); }
 
 int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     GroupedArgs a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.x; a.act = v.act;
     a.gate_out = v.gate_out; a.up_out = v.up_out; a.row_status = v.row_status; a.summary = v.summary;
-    a.n_row_tiles = (v.shape.inter + kOutRows - 1) / kOutRows; a.K = v.shape.hidden; a.es_vec = es_units(v.x); a.stall_stage = debug_waits().stall_stage;
+    a.n_row_tiles = grouped_row_tiles(v.shape.inter, false); a.K = v.shape.hidden; a.es_vec = es_units(v.x); a.stall_stage = debug_waits().stall_stage;
     CUtensorMap tm0, tm1;
     const u64 rb = u64(v.shape.hidden / 256) * kQ4KBlock, rows = u64(v.shape.experts) * v.shape.inter;
     if (int rc = encode_rows_map(v.weights.gate, rb, rows, &tm0)) return rc;
@@ -525,7 +526,7 @@ int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     GroupedArgs a{};
     a.shape = v.shape; a.routes = v.routes; a.in = v.act; a.raw = v.raw;
     a.summary = const_cast<u32*>(v.summary);
-    a.n_row_tiles = (v.shape.hidden + kGM - 1) / kGM; a.K = v.shape.inter; a.es_vec = es_units(v.act); a.raw_vec = aligned(v.raw, 8); a.stall_stage = debug_waits().stall_stage;
+    a.n_row_tiles = grouped_row_tiles(v.shape.hidden, true); a.K = v.shape.inter; a.es_vec = es_units(v.act); a.raw_vec = aligned(v.raw, 8); a.stall_stage = debug_waits().stall_stage;
     CUtensorMap tm0;
     if (int rc = encode_rows_map(v.weights.down, u64(v.shape.inter / 256) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<true>), kGroupedSmem)) return rc;

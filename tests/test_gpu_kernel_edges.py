@@ -45,12 +45,19 @@ def forced(form):
         b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_AUTO)
 
 
+@pytest.fixture
+def grouped_form(gpu):
+    import b200moe
+    with forced(b200moe.FORM_GROUPED):
+        yield
+
+
 def window(rng, E, K, rows):
     return np.stack([rng.permutation(E)[:K] for _ in range(rows)]).astype(np.uint32)
 
 
 @pytest.mark.parametrize("tokens", [1, 8, 16, 17, 24, 25, 47, 48, 49, 97])
-def test_grouped_tile_remainders(gpu, oracle, tokens):
+def test_grouped_tile_remainders(gpu, oracle, tokens, grouped_form):
     """One expert holds `tokens` rows of the window (tiles of 48 tokens in chunks of 8, three warps sharing them), another the rest."""
     from b200moe import ops, synth
     rng = np.random.default_rng(tokens)
@@ -69,7 +76,7 @@ def test_grouped_tile_remainders(gpu, oracle, tokens):
 
 @pytest.mark.parametrize("tokens,H,I,scale,special", [(31, 512, 512, 1, 0), (33, 256, 768, 1, 0), (63, 768, 256, 1, 0x7c00), (64, 1024, 1024, 400, 0),
                                                       (65, 256, 2048, 400, 0xfe00)])
-def test_grouped_row_tiles_of_a_share(gpu, oracle, tokens, H, I, scale, special):
+def test_grouped_row_tiles_of_a_share(gpu, oracle, tokens, H, I, scale, special, grouped_form):
     """Row tiles (96 outputs, 192 down rows) that end inside an expert, token tiles of 32 and their halves, tensors that hold fewer
     experts than the shape counts, gates beyond both limits of exp, a dmin that is not finite."""
     from b200moe import ops, synth
@@ -96,14 +103,16 @@ def test_grouped_row_tiles_of_a_share(gpu, oracle, tokens, H, I, scale, special)
     assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, 4, act).cpu(), want["raw"])
 
 
-@pytest.mark.parametrize("rows,top_k,E,I,form", [(63, 1, 1, 512, "wide"), (64, 1, 1, 512, "grouped"), (71, 2, 16, 256, "wide"), (72, 2, 16, 256, "grouped"),
-                                                 (31, 1, 1, 16384, "wide"), (32, 1, 1, 16384, "grouped"), (140, 1, 20, 256, "wide")])
-def test_grouped_form_lines(gpu, oracle, rows, top_k, E, I, form):
-    """Both sides of the lines between the streaming and the grouped Q4_K form: 64 rows (32 of a wide block), nine entries an expert."""
+@pytest.mark.parametrize("rows,top_k,E,H,I,gate_form,down_form", [
+    (144, 1, 1, 512, 512, "wide", "wide"), (145, 1, 1, 512, 512, "grouped", "wide"), (32, 1, 1, 512, 4096, "wide", "wide"), (33, 1, 1, 512, 4096, "grouped", "wide"),
+    (31, 1, 1, 768, 6144, "wide", "wide"), (32, 1, 1, 768, 6144, "grouped", "wide"), (40, 1, 1, 1024, 8192, "wide", "wide"), (41, 1, 1, 1024, 8192, "grouped", "wide"),
+    (47, 4, 16, 512, 512, "wide", "wide"), (48, 4, 16, 512, 512, "grouped", "wide"), (62, 4, 16, 512, 512, "grouped", "grouped"), (140, 1, 20, 256, 256, "wide", "wide")])
+def test_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I, gate_form, down_form):
+    """Both sides of the lines between the streaming and the grouped Q4_K form (gate/up and down choose each for itself): fewer items than SMs, an
+    estimate that has to be a quarter better below 48 rows, never below 32."""
     import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(rows)
-    H = 256
     gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
     ids = window(rng, E, top_k, rows)
     codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
@@ -111,14 +120,14 @@ def test_grouped_form_lines(gpu, oracle, rows, top_k, E, I, form):
     sh = ops.make_shape(H, I, E, top_k, 12, 12)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
     act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
-    assert b200moe.last_launch() == "gate_up_q4k_" + form
+    assert b200moe.last_launch() == "gate_up_q4k_" + gate_form
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
     raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
-    assert b200moe.last_launch() == "down_q4k_" + form and same(raw.cpu(), want["raw"])
+    assert b200moe.last_launch() == "down_q4k_" + down_form and same(raw.cpu(), want["raw"])
 
 
 @pytest.mark.parametrize("bits", [0x7c00, 0xfc00, 0x7e00])
-def test_grouped_factor_not_finite(gpu, oracle, bits):
+def test_grouped_factor_not_finite(gpu, oracle, bits, grouped_form):
     """A down row whose super-block factor is an infinity or a NaN: the term is d * dot, not what is left of (M + dot) - M."""
     from b200moe import ops, synth
     rng = np.random.default_rng(bits)
@@ -138,7 +147,7 @@ def test_grouped_factor_not_finite(gpu, oracle, bits):
     assert not np.isfinite(want).all() and same(got, want)
 
 
-def test_grouped_rows_of_any_stride(gpu):
+def test_grouped_rows_of_any_stride(gpu, grouped_form):
     """A8 rows 544 wide: their deltas and sums lie 68 bytes apart and take the 4-byte copies."""
     from b200moe import ops, synth
     rng = np.random.default_rng(5)

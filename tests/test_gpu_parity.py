@@ -539,8 +539,8 @@ def test_experts_other_formats_q5_k_q5_1(gpu, oracle):
 
 
 def test_experts_q4k_grouped_tensor_core_form(gpu, oracle):
-    """Windows of 128 rows and more take the grouped form (register-to-register integer MMAs + the same FP32 chains): stage by stage
-    against the oracle like the decode forms. Cases: several token tiles per expert with a ragged last one, experts with
+    """Windows of 128 rows and more, in the form that their sizes choose and in the grouped one (register-to-register integer MMAs + the same FP32
+    chains): stage by stage against the oracle like the decode forms. Cases: several token tiles per expert with a ragged last one, experts with
     few tokens, an expert range (first / end), K = 256 (two stages per tile) and a wide K."""
     import b200moe
     from b200moe import synth
@@ -551,8 +551,15 @@ def test_experts_q4k_grouped_tensor_core_form(gpu, oracle):
         ids = np.stack([rng.permutation(E)[:K] for _ in range(rows)]).astype(np.uint32)
         wts = rng.uniform(0.05, 0.6, size=(rows, K)).astype(np.float32)
         sh, osh = shape_pair(H, I, E, K, 12, 12)
-        run_stages(gpu, oracle, sh, osh, gate, up, down, x, ids, wts, b200moe.COMBINE_FMA_SLOTS, exact=False)
-        run_stages(gpu, oracle, sh, osh, gate, up, down, x, ids, wts, b200moe.COMBINE_FMA_SLOTS, first=1, end=E - 1, exact=False)
+        want = want_part = None
+        for form in (b200moe.FORM_AUTO, b200moe.FORM_GROUPED):
+            b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, form)
+            try:
+                _, want = run_stages(gpu, oracle, sh, osh, gate, up, down, x, ids, wts, b200moe.COMBINE_FMA_SLOTS, exact=False, want=want)
+                _, want_part = run_stages(gpu, oracle, sh, osh, gate, up, down, x, ids, wts, b200moe.COMBINE_FMA_SLOTS, first=1, end=E - 1, exact=False,
+                                          want=want_part)
+            finally:
+                b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_AUTO)
 
 
 def test_experts_q4k_collisions_and_empty_experts(gpu, oracle):
@@ -569,7 +576,7 @@ def test_experts_q4k_collisions_and_empty_experts(gpu, oracle):
         ids = np.tile(np.array([[7, 2]], np.uint32), (rows, 1))
         wts = rng.uniform(0.05, 0.6, size=(rows, K)).astype(np.float32)
         want = None
-        for form in (b200moe.FORM_AUTO, b200moe.FORM_ROW_STREAM, b200moe.FORM_SEGMENT_STREAM):  # 64 entries: 8 virtual experts of 8
+        for form in (b200moe.FORM_AUTO, b200moe.FORM_ROW_STREAM, b200moe.FORM_SEGMENT_STREAM, b200moe.FORM_GROUPED):  # 64 entries: 8 virtual experts of 8
             b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, form)
             try:
                 _, want = run_stages(gpu, oracle, sh, osh, gate, up, down, x, ids, wts, b200moe.COMBINE_FMA_SLOTS, exact=False, want=want)

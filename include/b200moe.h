@@ -77,7 +77,7 @@ const char* b200moe_last_launch(void);
  * production caller never sets them. The reference has the same kind of seam (TierDev::timeout_ns,
  * src/cuda/tiered_experts.cu:107-127). Returns B200MOE_ERR_INVALID_ARGUMENT for an unknown key. */
 #define B200MOE_DEBUG_WAIT_LIMIT 0u  /* polls of every bounded wait in the streaming and the grouped Q8_0 kernels; 0 = the default
-                                      * (2^22; grouped Q8_0 2^20). The grouped Q4_K kernel's limit is fixed (2^20) */
+                                      * (2^22; grouped Q8_0 2^20). The grouped Q4_K kernel's limit is fixed (2^18, about a second) */
 #define B200MOE_DEBUG_STALL_STAGE 1u /* n > 0: in every CTA of the Q4_K segment-streaming kernel the first producer, in every CTA of a grouped
                                       * kernel all producers stop feeding before their n-th stage (no copy of that stage is issued, none is left in flight); 0 = never */
 #define B200MOE_DEBUG_DECODE_FORM 2u /* gate/up and down: 0 = chosen by the plan, 1 = row streaming (Q4_K), 2 = segment streaming (Q4_K;

@@ -33,7 +33,7 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(q4k::saddr(dst)), "l"(src) : "memory");
 }
 
-// Bounds of a launch's waits: polls of up to a microsecond, and the stage before which a CTA's producers stop asking for copies (test hook).
+// Bounds of a launch's waits: polls (a microsecond's hint each, about four in fact), and the stage before which a CTA's producers stop asking for copies (test hook).
 struct Waits { u32 limit, stall_stage; };
 inline Waits debug_waits() {
     const u32 limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT), stall = debug_value(B200MOE_DEBUG_STALL_STAGE);

@@ -67,8 +67,8 @@ constexpr u32 kGroupedSmem = kOffCum + (kMaxUnion + 2) * 4;
 static_assert((kOutRows * kQ4KBlock) % 128 == 0 && kOffBars % 8 == 0, "TMA destinations, barriers");
 static_assert(kGN == 32 && kGM / 2 == (kHelpers - 1) * 32, "a helper lane stages a token, the helper threads before it two rows each");
 static_assert(kGroupedSmem > 114u * 1024u && kGroupedSmem <= 227u * 1024u, "one CTA per SM, within the shared memory of an SM");
-// Polls of up to a microsecond. Fixed here: a limit out of the arguments cost the consumers' loop 2 % (512 rows of the dense block 1170 -> 1194 us a call).
-constexpr u32 kWaitLimit = 1u << 20;
+// Polls of up to four microseconds: about a second. Fixed here: a limit out of the arguments cost the consumers' loop 2 % (512 rows of the dense block 1170 -> 1194 us a call).
+constexpr u32 kWaitLimit = 1u << 18;
 // Register split between whole warp groups, out of what the launch gives every thread (65,536 over the threads, by eights).
 constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kHelperRegs = 80;
 constexpr u32 kConsumerRegs = (kGThreads * kLaunchRegs - kHelpers * 32u * kHelperRegs) / (kConsumers * 32u) / 8u * 8u;

@@ -87,8 +87,11 @@ __device__ __forceinline__ float butterfly32(float v) {
     for (int d = 16; d; d >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, d));
     return v;
 }
+// amax / 127 rounded once, by a product in double: that is 2^-52 from the quotient, which lies no closer than 2^-32 to a rounding boundary
+// (magnitudes from 2^-119 on, whose quotients are normal).
+__device__ __forceinline__ float over_127(float amax) { return static_cast<float>(static_cast<double>(amax) * (1.0 / 127.0)); }
 // One A8 group of 32 values held one per lane (src/cpu/core/reference.cpp:35-55). Returns the code; delta and sum
-// are the same in every lane.
+// are the same in every lane. A group of NaNs alone gets a NaN for its delta, where the host rule gives 1 (codes of -127 in both).
 __device__ __forceinline__ int a8_quantize_lane(float x, float* delta_out, int* sum_out) {
     const float amax = warp_max_abs(x);
     const bool tiny = amax > 0.0f && amax < 0x1p-119f;

@@ -158,8 +158,7 @@ __device__ __forceinline__ u32 swiglu_a8(const float (&g)[kTasks], const float (
     for (int i = 0; i < kTasks; ++i) {  // a8_quantize_lane (common.cuh)
         const float am = __uint_as_float(amax[i]);
         const bool tiny = am > 0.0f && am < 0x1p-119f;
-        // am / 127 rounded once: a double product is 2^-52 from it, a quotient by 127 no closer than 2^-32 to a rounding boundary
-        delta[i] = (am == 0.0f || tiny) ? 1.0f : static_cast<float>(static_cast<double>(am) * (1.0 / 127.0));
+        delta[i] = (am == 0.0f || tiny) ? 1.0f : over_127(am);
         const float r = tiny ? 0.0f : rintf(__fdiv_rn(h[i], delta[i]));
         const float lo = (-127.0f < r) ? r : -127.0f;
         code[i] = static_cast<int>((lo < 127.0f) ? lo : 127.0f);

@@ -21,6 +21,15 @@ __global__ void exp_kernel(const u32* x, u32 n, int gfx1151, float* out) {
     const u32 i = blockIdx.x * 256u + threadIdx.x;
     if (i < n) out[i] = gfx1151 ? gfx1151_expf(__uint_as_float(x[i])) : declared_exp(__uint_as_float(x[i]));
 }
+// over_127 against the division for every float from 2^-119 on
+__global__ void over_127_kernel(u32* wrong) {
+    for (u32 i = 0x04000000u + blockIdx.x * 256u + threadIdx.x; i < 0x7f800000u; i += gridDim.x * 256u)
+        if (__float_as_uint(over_127(__uint_as_float(i))) != __float_as_uint(__fdiv_rn(__uint_as_float(i), 127.0f))) atomicAdd(wrong, 1u);
+}
+extern "C" int over_127_wrong(u32* wrong) {
+    over_127_kernel<<<1480, 256>>>(wrong);
+    return cudaGetLastError();
+}
 extern "C" int exp_bits(const u32* x, u32 n, int gfx1151, float* out) {
     exp_kernel<<<(n + 255) / 256, 256>>>(x, n, gfx1151, out);
     return cudaGetLastError();
@@ -69,3 +78,28 @@ def test_exp_for_every_float(device, oracle, gfx1151):
             got = got.cpu().numpy()
             wrong = (got.view(np.uint32) != want.view(np.uint32)) & ~(np.isnan(got) & np.isnan(want))
             assert not wrong.any(), (hex(int(c[wrong][0])), float(got[wrong][0]), float(want[wrong][0]), int(wrong.sum()))
+
+
+def test_over_127_is_the_quotient(device):
+    assert bits_of(2.0 ** -119) == 0x04000000
+    wrong = torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert device.over_127_wrong(C.c_void_p(wrong.data_ptr())) == 0
+    assert wrong.item() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 300])
+def test_a8_groups_with_nan(oracle, rows):
+    """Both forms of the quantiser on groups with 0, 1, 31 and 32 NaNs of either sign: a NaN does not count for the maximum and its code is -127;
+    a group of NaNs alone keeps a NaN as its delta."""
+    from b200moe import ops
+    rng = np.random.default_rng(rows)
+    x = rng.standard_normal((rows, 32 * 32), dtype=np.float32)
+    groups = x.reshape(-1, 32)
+    for i, g in enumerate(groups):
+        n = (0, 1, 31, 32)[i % 4]
+        g[rng.permutation(32)[:n]] = np.array([0x7fc00000, 0xffc00001], np.uint32).view(np.float32)[i // 4 % 2]
+    codes, deltas, sums = oracle.quantize_a8(x)
+    got = [t.cpu().numpy() for t in ops.enqueue_quantize_a8(torch.from_numpy(x).cuda())]
+    alone = np.isnan(groups).all(axis=1).reshape(rows, -1)
+    assert np.array_equal(got[0], codes) and np.array_equal(got[2], sums)
+    assert np.isnan(got[1][alone]).all() and np.array_equal(got[1][~alone].view(np.uint32), deltas[~alone].view(np.uint32))

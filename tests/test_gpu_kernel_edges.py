@@ -58,7 +58,7 @@ def window(rng, E, K, rows):
 
 @pytest.mark.parametrize("tokens", [1, 8, 16, 17, 24, 25, 47, 48, 49, 97])
 def test_grouped_tile_remainders(gpu, oracle, tokens, grouped_form):
-    """One expert holds `tokens` rows of the window (tiles of 48 tokens in chunks of 8, three warps sharing them), another the rest."""
+    """One expert holds `tokens` rows of the window (tiles of 32 tokens in halves of 16), another the rest."""
     from b200moe import ops, synth
     rng = np.random.default_rng(tokens)
     E, H, I, rows = 3, 256, 256, 160
@@ -185,7 +185,8 @@ def test_four_chain_down_group_counts(gpu, oracle, inter, down_type):
 
 @pytest.mark.parametrize("tokens", [0, 1, 8, 9, 16, 17, 25, 40])
 def test_q8_entry_blocks(gpu, oracle, tokens):
-    """Items of 16 entries (two blocks of 8): an expert whose last item holds one block, one entry or none of the second block."""
+    """Items of 8 entries of the tensor-core form: an expert with none, with one whole item, or with a last item of one entry."""
+    import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(tokens)
     E, H, I, rows = 3, 1024, 1280, 300
@@ -196,14 +197,16 @@ def test_q8_entry_blocks(gpu, oracle, tokens):
     want = oracle.experts(O.Shape(H, I, E, 1, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
     sh = ops.make_shape(H, I, E, 1, 8, 8)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
-    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
-    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
-    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act).cpu(), want["raw"])
+    with forced(b200moe.FORM_TENSOR):
+        act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
+        raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
 
 
 @pytest.mark.parametrize("tokens,H,I", [(1, 256, 512), (15, 512, 768), (16, 768, 256), (17, 1024, 1280), (32, 1280, 1024), (33, 2304, 256), (64, 7424, 256)])
 def test_q8_grouped_units(gpu, oracle, tokens, H, I):
     """The grouped Q8_0 form: rows of 1 to 29 units (empty sets, sets of unequal length), token tiles with one and with two halves."""
+    import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(tokens + H)
     E, rows = 2, 50 + tokens
@@ -214,13 +217,9 @@ def test_q8_grouped_units(gpu, oracle, tokens, H, I):
     want = oracle.experts(O.Shape(H, I, E, 1, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
     sh = ops.make_shape(H, I, E, 1, 8, 8)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
-    import b200moe
-    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_GROUPED)
-    try:
+    with forced(b200moe.FORM_GROUPED):
         act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
         raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
-    finally:
-        b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_AUTO)
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
     assert same(raw.cpu(), want["raw"])
 
@@ -651,12 +650,9 @@ def test_forced_form_is_the_one_that_runs(gpu, oracle, types, form, stem, rows, 
     want = oracle.experts(O.Shape(H, I, E, top_k, *types, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
     sh = ops.make_shape(H, I, E, top_k, *types)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
-    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, getattr(b200moe, form))
-    try:
+    with forced(getattr(b200moe, form)):
         act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
         assert b200moe.last_launch() == "gate_up_" + stem
         raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
         assert b200moe.last_launch() == "down_" + stem
-    finally:
-        b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, b200moe.FORM_AUTO)
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])

@@ -434,19 +434,29 @@ C4_PARTS = 8          # the fold always has 8 expert ranges: 1 GPU and 8 GPUs gi
 C4_GLOBAL_BATCH = 64
 
 
-def gate_up_kernel_name(cfg, rows, form):
-    """The routed gate/up kernel the library picks for a decode window of `rows` rows (csrc/api.cu: pick_decode_form,
-    use_q8_wide), or the one --form forces."""
-    if cfg["gate_type"] != 12:
-        return "q8_wide_kernel<gate/up>" if (form == 2 or (form == 0 and rows >= 8)) else "gate_up_q8_kernel"
-    if form == 3:
-        return "gate_up_q4k_kernel (per-block form)"
-    stream = form == 1 or (form == 0 and rows <= 2 and cfg["hidden"] <= 2048)
-    return "gate_up_q4k_stream_kernel" if stream else "q4k_wide_kernel<gate/up>"
+GATE_UP_KERNELS = {
+    "gate_up_q4k_wide": "q4k_wide_kernel<gate/up> (routed experts, segment-streaming GEMV)",
+    "gate_up_q4k_grouped": "grouped_q4k_kernel<gate/up> (routed experts over a token block, tensor-core dots)",
+    "gate_up_q4k_stream": "gate_up_q4k_stream_kernel", "gate_up_q4k": "gate_up_q4k_kernel (per-block form)",
+    "gate_up_q8": "gate_up_q8_kernel", "gate_up_q8_wide": "q8_wide_kernel<gate/up>", "gate_up_q8_mma": "q8_mma_kernel<gate/up>",
+    "gate_up_q8_grouped": "grouped_q8_kernel<gate/up>"}
+
+
+def gate_up_kernel_name(shape, gate, up, x, ids, first=0, end=0):
+    """The routed gate/up kernel that the library launches for this window (x: its rows, ids: their experts; [first, end): the experts held here),
+    from one launch of that stage alone, outside the timed regions."""
+    import b200moe
+    from b200moe import ops
+    rows, top_k = ids.shape
+    routes = ops.enqueue_moe_routes(ids, shape.experts, shape.experts // 2, first, end, first)
+    span = (end or shape.experts) - first
+    ops.enqueue_routed_gate_up(shape, gate, up, routes, min(rows * top_k, span), ops.enqueue_quantize_a8(x), rows * top_k)
+    name = b200moe.last_launch()
+    return GATE_UP_KERNELS.get(name, name)
 
 
 def c4_phase(batch):
-    """Windows of 128 rows and more are token blocks (the routed experts then take the grouped tensor-core form)."""
+    """Windows of 128 rows and more are token blocks."""
     return "prefill" if batch >= 128 else "decode"
 
 
@@ -673,6 +683,8 @@ def large_arm(args, cfg, rank, world, dev):
         mine = ids[(ids >= rank * per) & (ids < (rank + 1) * per)]
         uniq.append(len(np.unique(mine)))
         entries.append(mine.size)
+    gate_up_kernel = gate_up_kernel_name(shape, gate, up, torch.from_numpy(batches[-1]).to(dev), torch.from_numpy(ids).to(dev), rank * per if world > 1 else 0,
+                                         (rank + 1) * per if world > 1 else 0)
     uniq, entries = np.array(uniq, np.float64), np.array(entries, np.float64)
 
     # ---- timed region 1: the K-step block, replayed from a CUDA graph, repeated until the region is >= 0.25 s ------
@@ -786,9 +798,7 @@ def large_arm(args, cfg, rank, world, dev):
         "e2e": {"value": B * K / (host_ms / 1000.0), "unit": UNIT, "h2d_bytes_per_step": B * H * 4, "d2h_bytes_per_step": B * H * 4,
                 "ms_per_step": host_ms / K},
         "gpu_launches": int(round(launches_per_step * K)),
-        "roofline": {"kernel": "q4k_wide_kernel<gate/up> (routed experts, segment-streaming GEMV)" if B < 128 else
-                               "grouped_q4k_kernel<gate/up> (routed experts over a token block, tensor-core dots; quoted against HBM on its distinct-expert bytes)",
-                     "bound": "hbm", "achieved": achieved, "peak": peak,
+        "roofline": {"kernel": gate_up_kernel, "bound": "hbm", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "peak_kind": f"{peak_kind} HBM copy", "frac_of_nominal_8tbs": achieved / 8000.0,
                      "traffic": float(allr[slow, 4]) * C4_TRAFFIC_RATIO,
                      "traffic_note": "scaled by distinct experts from the ncu capture of a reduced layer (x 1.03 algorithmic): profiles/wide_kernels_c4_decode.md",
@@ -1056,7 +1066,7 @@ def decode_arm(args, cfg, rank, world, dev):
         "e2e": {"value": tokens / (host_ms / 1000.0), "unit": UNIT, "h2d_bytes_per_step": B * H * 4, "d2h_bytes_per_step": B * H * 4,
                 "ms_per_step": host_ms / K},
         "gpu_launches": int(round(launches_per_step * K)),
-        "roofline": {"kernel": gate_up_kernel_name(cfg, B, args.form), "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"kernel": gate_up_kernel_name(shape, layers[0].gate, layers[0].up, xs[0], ids), "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": f"{peak_kind} HBM copy",
                      # dram read + write per launch from an ncu capture of this kernel on this workload: 1.00 of the algorithmic bytes
                      "traffic": algo_bytes * NCU_TRAFFIC_RATIO if cfg["gate_type"] == 12 else None,

@@ -412,7 +412,7 @@ int b200moe_ep_ffn(void* ep, const b200moe_ep_step_view* view, void* stream);
 
 /* ------------------------------------------------------------------------------------------------ whole layer
  * Routes from the router's ids, gate/up, down and the combine. Decode GEMVs below grouped_min_rows rows, the grouped
- * tensor-core GEMM from there (0 = never). Replaces enqueue_moe_layer(MoeLayerView)
+ * tensor-core GEMM of the Q4_K experts from there (0 = chosen by the window's sizes). Replaces enqueue_moe_layer(MoeLayerView)
  * (include/strix/cuda/ds41_moe.hpp:139-156) and qwen_moe::enqueue_routed + enqueue_combine (qwen_moe.hpp:105-107). */
 typedef struct b200moe_layer_view {
     b200moe_shape shape;

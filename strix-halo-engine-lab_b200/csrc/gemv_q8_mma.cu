@@ -1,6 +1,6 @@
-// Q8_0 x A8 experts over windows of 8 rows and more, integer dots on the tensor cores: the lane-class contract of
-// src/ds41_formats.cpp:188-197 (product_q8_0) with one mma.sync.m16n8k32 (s8 x s8 -> s32) per (16 weight rows, 8 entries,
-// block) instead of 16 x 8 dp4a chains of eight.
+// Q8_0 x A8 experts over windows of 8 rows and more with few entries an expert (grouped_q8.cu takes the others), integer dots on the
+// tensor cores: the lane-class contract of src/ds41_formats.cpp:188-197 (product_q8_0) with one mma.sync.m16n8k32 (s8 x s8 -> s32) per
+// (16 weight rows, 8 entries, block) instead of 16 x 8 dp4a chains of eight.
 //
 // The contract adds the terms float(dot_g) * (scale_g * delta_g) of a row into 32 lane classes (group g -> class g % 32) in
 // ascending g, then folds the classes with the butterfly v[l] += v[l ^ d], d = 16 .. 1. A class is an independent chain, so
@@ -68,9 +68,9 @@ __device__ __forceinline__ void mma_s8s8(int (&c)[4], u32 a0, u32 a1, u32 a2, u3
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
-// One block of one run: rows gid and gid + 8 of the tile (A), the item's entries in blocks of 8 (B), this lane's four (row, entry)
-// cells of each. ODD: the block's position in its run is odd (quants on a word). blk: byte offset of the block in a row;
-// codes / deltas: the first entries' A8 rows at this block, for this lane's fragment cells. nb: blocks of entries that hold any.
+// One block of one run: rows gid and gid + 8 of the tile (A), the item's entries (B), this lane's four (row, entry)
+// cells. ODD: the block's position in its run is odd (quants on a word). blk: byte offset of the block in a row;
+// codes / d0p: the entries' A8 rows at this block, for this lane's fragment cells.
 template <bool ODD>
 __device__ __forceinline__ void block_step(const unsigned char* rowA, const unsigned char* rowB, u32 blk, u32 t4, const unsigned char* codes,
                                            const unsigned char* d0p, u32 xd_pitch, float (&acc)[4]) {
@@ -250,7 +250,7 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
             // Warp w folds row w of the tile, lane = (entry, class % 4): the butterfly's steps 16, 8 and 4 stay inside a residue
             // class mod 4, i.e. inside the lane's eight registers; only steps 2 and 1 cross lanes. (A lane per class and five
             // shuffles an entry kept the shuffle unit as busy as the dots of a 2048-wide row: 512 rows x 4 over 64 experts of
-            // 2048 -> 1024 took 830 us a call, 671 now.)
+            // 2048 -> 1024, in this form, took 830 us a call with them and 671 without.)
             const u32 fq = lane & 3u, fe = lane >> 2;
             float v8[8];
 #pragma unroll

@@ -22,7 +22,7 @@
 // A persistent CTA per SM walks tiles round-robin; a stage of the ring (three) is one super-block: 256 columns, 4 pairs of groups (chains).
 //   * helper warps (4): the tile's weight rows arrive by two tiled TMA copies (144 bytes x 96 rows: consecutive rows lie 4 (mod 32) words
 //     apart, the fragment loads below are conflict free), the tokens' codes, deltas and sums by 16-byte asynchronous copies (codes 272
-//     bytes apart, for the same reason), one stage ahead. A thread of the first three warps decodes the factors of two weight rows, a lane
+//     bytes apart, for the same reason), up to three stages ahead of the consumers. A thread of the first three warps decodes the factors of two weight rows, a lane
 //     of the fourth lays out the {E, S} of one token.
 //   * consumer warps (12): warp = 64 rows x all tokens of ONE of the four chains. The nibbles go from shared memory straight into B
 //     fragments (low nibbles by a mask, high nibbles left in place as 16 q), the codes into A fragments; a lane's two neighbouring cells
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
 #pragma unroll
             for (int i = 0; i < (int)(kRowTiles * kTokTiles * 2); ++i) (&acc[0][0][0])[i] = make_float2(0.0f, 0.0f);
             for (u32 b = 0; b < nblocks; ++b) {
-                // asked a stage ahead, so that the answer is there (the helpers have seen the rows' copies complete before they arrive)
+                // the helpers have seen the rows' copies complete before they arrive
                 if (ok) ok = mbar_wait(&ready[slot], parity, kWaitLimit, s_abort);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) continue;

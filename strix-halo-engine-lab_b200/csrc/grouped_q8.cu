@@ -13,14 +13,15 @@
 // and 27 for an even block; in the kernel 33 instructions and 49 clocks, the rest being waits and addresses of every second unit, the
 // meeting of the sets and warps once per tile, and SwiGLU. Eight warps of all 64 rows had fewer instructions (27 an MMA) and were slower
 // (399 against 353 us a call, 512 rows below): two warps a scheduler do not cover each other's latencies.
-// 512 rows x 4 over 64 experts of 2048 -> 1024: gate/up 182, down 110 us (282 and 221 in gemv_q8_mma.cu); 8192 rows of a dense
-// 7168 -> 2048 block 2630 and 1450 us (5110 and 3110).
+// Both instantiations spill a little at their 96 registers (52 bytes stored and 100 loaded in gate/up, 48 and 80 in down).
+// 512 rows x 4 over 64 experts of 2048 -> 1024: gate/up 173, down 112 us (344 and 253 in gemv_q8_mma.cu); 8192 rows of a dense
+// 7168 -> 2048 block 2530 and 1430 us (4960 and 3810).
 //
 // A persistent CTA per SM walks tiles round-robin. Producer warps (4): the unit's weight rows by tiled TMA (272 bytes x 32 rows: rows lie
 // 4 (mod 32) words apart, the fragment loads are conflict free), the tokens' codes and deltas by 16-byte asynchronous copies, all counted on
 // the stage's mbarrier. The places of absent tokens keep what an earlier tile left there (their cells are never stored): copies of the tile's last token
-// in them had every CTA ask for the same lines again and again (gate/up of one expert of 2048 x 17408, 16 rows: 56.6 us, 32.9 without). Consumer warps (16): mma.sync m16n8k32 (tokens x weight rows, s8 x s8) straight from shared memory; a lane's two
-// neighbouring cells are two weight rows of one token (packed FP32). Q8_0 blocks are 34 bytes: the quants of an even block start 2 (mod 4)
+// in them had every CTA ask for the same lines again and again (gate/up of one expert of 2048 x 17408, 16 rows: 56.6 us, 32.9 without).
+// Consumer warps (16): mma.sync m16n8k32 (tokens x weight rows, s8 x s8) straight from shared memory; a lane's two neighbouring cells are two weight rows of one token (packed FP32). Q8_0 blocks are 34 bytes: the quants of an even block start 2 (mod 4)
 // bytes in (two words and a byte permute per register), those of an odd block on a word.
 // Every wait is bounded; on a timeout the roles stop working, the producers wait (bounded) for the copies in flight and the launch sets
 // B200MOE_JOB_WAIT_ABORTED in the job summary.

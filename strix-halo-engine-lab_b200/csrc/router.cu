@@ -104,8 +104,8 @@ __global__ void __launch_bounds__(kFewWarps * 32) router_logits_few_kernel(const
 // Windows of more than 4 rows: a CTA owns 8 rows x 16 experts and walks the hidden width in chunks of COLS columns that
 // all 128 threads stage into shared memory with 16-byte asynchronous copies, three chunks in flight; a warp keeps an
 // 8 x 4 tile of lane-class sums. Chunks of 256 columns leave room for three CTAs an SM, of 512 for one: with more tiles than SMs the
-// former hide each other's latency (8192 x 256 x 7168: 2309 us with 512, 1442 with 256; two FP32 operations a product bound it
-// at 835), a window with fewer tiles is a chain of chunks and wants the longer ones (64 x 256 x 7168: 23 against 33 us). The x tile
+// former hide each other's latency (8192 x 256 x 7168: 2309 us with 512, 1442 with 256, 1271 with two rows a packed instruction too; two FP32
+// operations a product bound it at 835), a window with fewer tiles is a chain of chunks and wants the longer ones (64 x 256 x 7168: 23 against 33 us). The x tile
 // is then read from HBM / L2 once per 16 experts instead of once per expert (a
 // 64-row window over 256 experts of width 7168 pulled 470 MB through L2 in the form above), and the copies of two chunks
 // cover the arithmetic of one. Same products, same order: lane l of a warp meets columns l, l + 32, ... ascending.

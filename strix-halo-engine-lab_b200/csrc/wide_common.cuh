@@ -41,8 +41,7 @@ __device__ __forceinline__ u32 warp_inclusive_scan(u32 v, u32 lane) {
 // needs no memset. Why not a fixed share per CTA: the time of an item depends on its entries in a way a cost estimate only
 // approximates, and with a dozen items per group a mis-estimate leaves SMs idle for the last tenth of the kernel.
 constexpr u32 kClaimBits = 22, kClaimMask = (1u << kClaimBits) - 1u;
-template <u32 KE = kKE>
-__host__ __device__ constexpr u32 work_list_scratch_words(u32 max_union, u32 vmax) { return 2 * max_union + 2 + vmax + KE; }
+__host__ __device__ constexpr u32 work_list_scratch_words(u32 max_union, u32 vmax) { return 2 * max_union + 2 + vmax + kKE; }
 __device__ __forceinline__ u32 claim_item(u32* claim) { return atomicAdd(claim, 1u) & kClaimMask; }
 // Called once per producer warp (lane 0) when it will claim no more; ctl[1] counts the CTA's producers that have finished.
 __device__ __forceinline__ void retire_claims(u32* claim, u32* ctl) {
@@ -51,16 +50,14 @@ __device__ __forceinline__ void retire_claims(u32* claim, u32* ctl) {
     if ((before >> kClaimBits) == gridDim.x - 1u) atomicExch(claim, 0u);
 }
 
-// Builds the work list: `table` gets the virtual experts (an expert of the union with at most KE of its entries; an expert
+// Builds the work list: `table` gets the virtual experts (an expert of the union with at most kKE of its entries; an expert
 // with more entries appears several times) ORDERED BY ENTRIES, most first (stable within a count): items are claimed in
 // table order, so the long items start first and the kernel's tail is made of short ones. ctl[3] = items (virtual expert
 // major x n_chunks chunks). Every CTA builds the same list. `scratch` is shared memory that is free until the first copy is
 // issued (work_list_scratch_words(max_union, vmax) words). Every thread of the block calls it; it holds four block barriers.
-// n_union <= max_union; the block has at least KE warps.
-template <u32 KE = kKE>
+// n_union <= max_union; the block has at least kKE warps.
 __device__ __forceinline__ void build_work_list(const b200moe_routes& routes, u32 n_union, u32 max_union, u32 vmax, u32 n_chunks, u32* scratch,
                                                 VExpert* table, u32* ctl) {
-    static_assert(KE >= 1 && KE <= 255, "a virtual expert holds its entry count in 8 bits");
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     u32* t_beg = scratch;
     u32* t_exp = t_beg + max_union + 1;
@@ -76,26 +73,26 @@ __device__ __forceinline__ void build_work_list(const b200moe_routes& routes, u3
         for (u32 j0 = 0; j0 < n_union; j0 += 32) {
             const u32 j = j0 + lane;
             const u32 eb = j < n_union ? t_beg[j] : 0u, ne = j < n_union ? t_beg[j + 1] - eb : 0u;
-            const u32 nv = (ne + KE - 1) / KE;
+            const u32 nv = (ne + kKE - 1) / kKE;
             const u32 iv = warp_inclusive_scan(nv, lane);
             u32 pos = n_virtual + iv - nv;
-            for (u32 k = 0; k < nv && pos < vmax; ++k, ++pos) unsorted[pos] = VExpert::make(t_exp[j], eb + k * KE, min(KE, ne - k * KE));
+            for (u32 k = 0; k < nv && pos < vmax; ++k, ++pos) unsorted[pos] = VExpert::make(t_exp[j], eb + k * kKE, min(kKE, ne - k * kKE));
             n_virtual += __shfl_sync(0xffffffffu, iv, 31);
         }
         if (n_virtual > vmax) n_virtual = vmax;
         if (lane == 0) { ctl[2] = n_virtual; ctl[3] = n_virtual * n_chunks; }
     }
     __syncthreads();
-    // counting sort by entries, descending: warp b places the virtual experts of KE - b entries
+    // counting sort by entries, descending: warp b places the virtual experts of kKE - b entries
     const u32 n_virtual = ctl[2];
-    const u32 want = KE - warp;
-    if (warp < KE) {
+    const u32 want = kKE - warp;
+    if (warp < kKE) {
         u32 n = 0;
         for (u32 i0 = 0; i0 < n_virtual; i0 += 32) n += __popc(__ballot_sync(0xffffffffu, i0 + lane < n_virtual && unsorted[i0 + lane].ne() == want));
         if (lane == 0) s_hist[warp] = n;
     }
     __syncthreads();
-    if (warp < KE) {
+    if (warp < kKE) {
         u32 pos = 0;
         for (u32 b = 0; b < warp; ++b) pos += s_hist[b];
         for (u32 i0 = 0; i0 < n_virtual; i0 += 32) {

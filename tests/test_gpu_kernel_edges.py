@@ -402,9 +402,9 @@ def test_routes_row_order_forms(gpu, rows, top_k):
 
 
 @pytest.mark.parametrize("hidden,inter,rows", [(2304, 1024, 300), (4352, 1024, 301), (6656, 1024, 311), (6912, 1024, 313), (1024, 2304, 297), (1024, 4352, 295)])
-def test_q8_items_of_16_over_several_stages(gpu, oracle, hidden, inter, rows):
-    """Rows of more than one stage of two runs (the last stage one run, whole or a part of one), the last item not full; at 6912 the
-    projection's A8 rows leave no room for 16 entries and it takes 8."""
+def test_q8_items_over_several_stages(gpu, oracle, hidden, inter, rows):
+    """The tensor-core form over rows of one and of two stages of four runs (the last run a part of one), the last item not full."""
+    import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(hidden + inter)
     gate, up, down = synth.expert_tensors(rng, 1, hidden, inter, 8, 8)
@@ -413,9 +413,12 @@ def test_q8_items_of_16_over_several_stages(gpu, oracle, hidden, inter, rows):
     want = oracle.experts(O.Shape(hidden, inter, 1, 1, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
     sh = ops.make_shape(hidden, inter, 1, 1, 8, 8)
     r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), 1, 1)
-    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, 1, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
-    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
-    assert same(ops.enqueue_routed_down(sh, dv(down, gpu), r, 1, act).cpu(), want["raw"])
+    with forced(b200moe.FORM_TENSOR):
+        act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, 1, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows, taps=True)
+        assert b200moe.last_launch() == "gate_up_q8_mma"
+        raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, 1, act)
+        assert b200moe.last_launch() == "down_q8_mma"
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
 
 
 # rows that start between 16-byte units (x at an odd element) or have no whole number of them (hidden % 4): the register forms

@@ -9,9 +9,10 @@ namespace b200moe {
 namespace {
 
 template <bool BF16>
-__global__ void __launch_bounds__(256) quantize_a8_kernel(const void* __restrict__ x, u32 rows, u32 groups, u32 x_stride,
-                                                          i8* __restrict__ codes, float* __restrict__ deltas,
-                                                          i32* __restrict__ sums, u32 stride, u32* __restrict__ status) {
+__global__ void __launch_bounds__(256) quantize_a8_kernel(const void* x, u32 rows, u32 groups, u32 x_stride,
+                                                          i8* codes, float* deltas,
+                                                          i32* sums, u32 stride, u32* status) {
+    chain_begin();
     const u32 lane = threadIdx.x & 31u;
     const u64 item = u64(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= u64(rows) * groups) return;
@@ -39,9 +40,10 @@ __global__ void __launch_bounds__(256) quantize_a8_kernel(const void* __restrict
 // 108 us there, 0.44 of the measured copy bandwidth; 1024 rows 15.6 us, 38.9 in the one-value form. With `wide` the bfloat16 values
 // are also written out as FP32 for the router, instead of by a pass of their own before this one (8192 x 7168: 119 + 305 -> 218 us).
 template <bool BF16>
-__global__ void __launch_bounds__(256) quantize_a8_vec_kernel(const void* __restrict__ x, u32 items, u32 groups, u32 x_stride, i8* __restrict__ codes,
-                                                              float* __restrict__ deltas, i32* __restrict__ sums, u32 stride, u32* __restrict__ status,
-                                                              float* __restrict__ wide, u32 wide_stride) {
+__global__ void __launch_bounds__(256) quantize_a8_vec_kernel(const void* x, u32 items, u32 groups, u32 x_stride, i8* codes,
+                                                              float* deltas, i32* sums, u32 stride, u32* status,
+                                                              float* wide, u32 wide_stride) {
+    chain_begin();
     const u32 t = blockIdx.x * 256u + threadIdx.x, sub = t & 7u;
     const bool valid = (t >> 3) < items;
     const u32 item = valid ? t >> 3 : items - 1u;  // spare lanes of the last warp repeat its last group and store nothing
@@ -49,11 +51,11 @@ __global__ void __launch_bounds__(256) quantize_a8_vec_kernel(const void* __rest
     const u64 at = u64(r) * x_stride + 32u * g + 4u * sub;
     float v[4];
     if (BF16) {
-        const uint2 b = __ldg(reinterpret_cast<const uint2*>(static_cast<const u16*>(x) + at));
+        const uint2 b = load(reinterpret_cast<const uint2*>(static_cast<const u16*>(x) + at));
         v[0] = __uint_as_float(b.x << 16); v[1] = __uint_as_float(b.x & 0xffff0000u); v[2] = __uint_as_float(b.y << 16); v[3] = __uint_as_float(b.y & 0xffff0000u);
         if (wide && valid) *reinterpret_cast<float4*>(wide + u64(r) * wide_stride + 32u * g + 4u * sub) = make_float4(v[0], v[1], v[2], v[3]);
     } else {
-        const float4 f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(x) + at));
+        const float4 f = load(reinterpret_cast<const float4*>(static_cast<const float*>(x) + at));
         v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
     }
     float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));  // NaN operands are ignored (a8_quantize_lane)
@@ -83,7 +85,8 @@ __global__ void __launch_bounds__(256) quantize_a8_vec_kernel(const void* __rest
 }
 
 // bfloat16 bit patterns widened to FP32 (exact): the router reads FP32 rows.
-__global__ void __launch_bounds__(256) widen_bf16_kernel(const u16* __restrict__ in, float* __restrict__ out, u64 count) {
+__global__ void __launch_bounds__(256) widen_bf16_kernel(const u16* in, float* out, u64 count) {
+    chain_begin();
     for (u64 i = u64(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += u64(gridDim.x) * blockDim.x)
         out[i] = __uint_as_float(static_cast<u32>(in[i]) << 16);
 }
@@ -93,7 +96,7 @@ __global__ void __launch_bounds__(256) widen_bf16_kernel(const u16* __restrict__
 int launch_widen_bf16(const u16* in, float* out, u64 count, cudaStream_t stream) {
     if (count == 0) return B200MOE_OK;
     const u32 blocks = static_cast<u32>(std::min<u64>((count + 255) / 256, 148u * 16u));
-    widen_bf16_kernel<<<blocks, 256, 0, stream>>>(in, out, count);
+    chain_launch(widen_bf16_kernel, blocks, 256, 0, stream, in, out, count);
     return after_launch("widen_bf16");
 }
 
@@ -113,16 +116,16 @@ int launch_quantize_a8(const b200moe_quantize_a8_view& v, cudaStream_t stream, f
     if (quantize_a8_vec_ok(v) && (wide || items > 8u * static_cast<u32>(device_sm_count()))) {
         const u32 vec_blocks = static_cast<u32>((items + 31) / 32);
         if (v.x_is_bf16)
-            quantize_a8_vec_kernel<true><<<vec_blocks, 256, 0, stream>>>(v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, wide, wide_stride);
+            chain_launch(quantize_a8_vec_kernel<true>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, wide, wide_stride);
         else
-            quantize_a8_vec_kernel<false><<<vec_blocks, 256, 0, stream>>>(v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, nullptr, 0);
+            chain_launch(quantize_a8_vec_kernel<false>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, nullptr, 0);
         return after_launch("quantize_a8");
     }
     const u32 blocks = static_cast<u32>((items + 7) / 8);
     if (v.x_is_bf16)
-        quantize_a8_kernel<true><<<blocks, 256, 0, stream>>>(v.x, v.rows, groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status);
+        chain_launch(quantize_a8_kernel<true>, blocks, 256, 0, stream, v.x, v.rows, groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status);
     else
-        quantize_a8_kernel<false><<<blocks, 256, 0, stream>>>(v.x, v.rows, groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status);
+        chain_launch(quantize_a8_kernel<false>, blocks, 256, 0, stream, v.x, v.rows, groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status);
     return after_launch("quantize_a8");
 }
 

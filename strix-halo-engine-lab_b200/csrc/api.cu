@@ -227,12 +227,10 @@ FfnScratch carve_ffn(void* ws, const b200moe_shape& s, u32 capacity) {
     return F;
 }
 
-// Zeroes the job summary (4 words) and, when it lives in the workspace, the per-row status behind it. The two sections
-// are neighbours in the workspace (carve_layer), so one memset node covers both and the padding between them.
-cudaError_t clear_status(const LayerScratch& L, bool with_row_status, u32 rows, cudaStream_t st) {
-    const unsigned char* b = reinterpret_cast<const unsigned char*>(L.summary);
-    const unsigned char* e = with_row_status ? reinterpret_cast<const unsigned char*>(L.row_status + rows) : b + 16;
-    return cudaMemsetAsync(L.summary, 0, static_cast<size_t>(e - b), st);
+// The status words that a call owns: the job summary and, where the caller gives none of his own, the rows' status. They are cleared by the launch that
+// builds the routes (a caller's summary word too): a memset node in front of it cost 3 us of a short call.
+RoutesClear clear_of(const LayerScratch& L, u32* caller_row_status, u32* caller_summary) {
+    return RoutesClear{caller_row_status ? nullptr : L.row_status, L.summary, caller_summary};
 }
 
 // What a window is for the kernels that walk it item by item, known from its sizes alone: the items of eight entries and the tiles of 32 that
@@ -466,7 +464,7 @@ extern "C" {
 int b200moe_build_routes(const b200moe_routes_view* v, void* stream) {
     if (int rc = b200moe_check_routes_view(v)) return rc;
     if (!device_ready()) return B200MOE_ERR_CUDA;
-    return launch_routes(*v, as_stream(stream));
+    return launch_routes(*v, RoutesClear{}, as_stream(stream));
 }
 
 int b200moe_gate_up(const b200moe_gate_up_view* v, void* stream) {
@@ -552,11 +550,6 @@ static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_rea
 
     u32* row_status = v->row_status ? v->row_status : L.row_status;
     u32* summary = v->summary ? v->summary : L.summary;
-    if (!routes_ready) {
-        cudaError_t ce = clear_status(L, !v->row_status, v->rows, st);
-        if (ce == cudaSuccess && v->summary) ce = cudaMemsetAsync(v->summary, 0, sizeof(u32), st);
-        if (ce != cudaSuccess) return fail(B200MOE_ERR_CUDA, "layer: cudaMemsetAsync: %s", cudaGetErrorString(ce));
-    }
 
     b200moe_routes_view rv{};
     rv.ids = v->ids; rv.rows = v->rows; rv.top_k = s.top_k; rv.experts = s.experts;
@@ -567,7 +560,7 @@ static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_rea
         if (v->stage_events && v->stage_events[i]) cudaEventRecord(static_cast<cudaEvent_t>(v->stage_events[i]), st);
     };
     tap(0);
-    if (!routes_ready) if (int rc = launch_routes(rv, st)) return rc;
+    if (!routes_ready) if (int rc = launch_routes(rv, clear_of(L, v->row_status, v->summary), st)) return rc;
     tap(1);
 
     const u32 span = (v->end ? v->end : s.experts) - v->first;
@@ -634,37 +627,33 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
     b200moe_router_view r{};
     r.x = x32; r.x_stride = s.hidden; r.rows = v->rows; r.hidden = s.hidden;
     r.weight = v->router_weight; r.logit_bias = v->logit_bias; r.bias = v->select_bias; r.policy = v->policy;
-    r.logits = F.logits; r.scores = F.logits;
+    r.logits = F.logits;  // the scores are not asked for
     r.ids = v->ids ? v->ids : F.ids; r.weights = v->route_weights ? v->route_weights : F.weights;
-    // Decode windows: one launch for A8 + logits + selection + routes; 9..32 rows: selection and routes share a launch.
+    // Up to 8 rows: one launch for A8 and logits. Up to 32: selection and routes share a launch.
     const LayerScratch L = carve_layer(F.layer, s, v->capacity);
-    const bool one_launch = prologue_fusable(r, s.top_k);
-    const bool fused = one_launch || select_routes_fusable(r, s.top_k);
+    const bool fused = select_routes_fusable(r, s.top_k), one_launch = fused && prologue_fusable(r, s.top_k);
     // Where the quantiser is a launch of its own it widens on the way (one pass over the activations instead of two).
     b200moe_quantize_a8_view qb = q;
     qb.x = v->x; qb.x_is_bf16 = 1;
     const bool widen_in_quantizer = v->x_is_bf16 && !one_launch && quantize_a8_vec_ok(qb);
-    if (v->x_is_bf16 && !widen_in_quantizer)
+    if (v->x_is_bf16 && !widen_in_quantizer && !one_launch)
         if (int rc = launch_widen_bf16(static_cast<const u16*>(v->x), F.x_f32, u64(v->rows) * s.hidden, st)) return rc;
     b200moe_routes_view rv{};
     if (fused) {
         u32* row_status = v->row_status ? v->row_status : L.row_status;
-        cudaError_t ce = clear_status(L, !v->row_status, v->rows, st);  // summary word, prologue ticket, row status
-        if (ce == cudaSuccess && v->summary) ce = cudaMemsetAsync(v->summary, 0, sizeof(u32), st);
-        if (ce != cudaSuccess) return fail(B200MOE_ERR_CUDA, "ffn: cudaMemsetAsync: %s", cudaGetErrorString(ce));
         rv.ids = r.ids; rv.rows = v->rows; rv.top_k = s.top_k; rv.experts = s.experts;
         rv.split = v->part_experts ? v->part_experts : s.experts / 2;
         rv.scratch = L.routes_scratch; rv.row_status = row_status; rv.out = L.routes;
     }
     if (one_launch) {
-        if (int rc = launch_prologue(r, q, rv, L.summary + 1, st)) return rc;
+        if (int rc = launch_prologue(r, v->x_is_bf16 ? qb : q, st)) return rc;  // widens on the way
     } else {
         if (widen_in_quantizer)
             if (int rc = launch_quantize_a8(qb, st, F.x_f32, s.hidden)) return rc;
         if (int rc = launch_router_logits(r, st, widen_in_quantizer ? nullptr : &q)) return rc;
-        if (fused) { if (int rc = launch_select_routes(r, rv, st)) return rc; }
-        else if (int rc = launch_router_select(r, st)) return rc;
+        if (!fused) if (int rc = launch_router_select(r, st)) return rc;
     }
+    if (fused) if (int rc = launch_select_routes(r, rv, clear_of(L, v->row_status, v->summary), st)) return rc;
 
     b200moe_layer_view lv{};
     lv.shape = s; lv.weights = v->weights; lv.rows = v->rows; lv.x = F.x; lv.ids = r.ids; lv.route_weights = r.weights;

@@ -18,6 +18,7 @@ constexpr u32 kMaxTopK = 32;
 
 // grid (ceil(hidden / 256), min(rows, 65535)); 256 threads; a block walks rows blockIdx.y, blockIdx.y + gridDim.y, ...
 __global__ void __launch_bounds__(256) combine_kernel(b200moe_combine_view v) {
+    chain_begin();
     const u32 o = blockIdx.x * blockDim.x + threadIdx.x;
     if (v.summary && (*v.summary & B200MOE_JOB_WAIT_ABORTED)) return;  // an aborted stage left raw partly unwritten
     __shared__ float s_w[kMaxTopK];
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(256) combine_kernel(b200moe_combine_view v) {
 // and their order are those of combine_kernel.
 constexpr u32 kVecTopK = 8;
 __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v) {
+    chain_begin();
     const u32 o = 4u * (blockIdx.x * 128u + threadIdx.x);
     if (o >= v.hidden || (v.summary && (*v.summary & B200MOE_JOB_WAIT_ABORTED))) return;
     for (u32 row = blockIdx.y; row < v.rows; row += gridDim.y) {
@@ -90,11 +92,11 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
             if (k < v.top_k) {
-                slot[k] = __ldg(v.order + row * v.top_k + k);
-                x[k] = __ldg(reinterpret_cast<const float4*>(v.raw + u64(slot[k]) * v.hidden + o));
-                w[k] = __ldg(v.weights + slot[k]);
+                slot[k] = load(v.order + row * v.top_k + k);
+                x[k] = load(reinterpret_cast<const float4*>(v.raw + u64(slot[k]) * v.hidden + o));
+                w[k] = load(v.weights + slot[k]);
             }
-        const float4 sh = v.shared ? __ldg(reinterpret_cast<const float4*>(v.shared + u64(row) * v.hidden + o)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 sh = v.shared ? load(reinterpret_cast<const float4*>(v.shared + u64(row) * v.hidden + o)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         float4 y = sh, sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         u32 p = 0;
         bool run = true;  // a slot out of order ends the walk, as it does in combine_kernel
@@ -105,7 +107,7 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
             if (run && k < v.top_k) {
-                const u32 part = v.low_counts ? (k < v.low_counts[row] ? 0u : 1u) : min(__ldg(v.ids + slot[k]) / v.part_experts, v.parts - 1);
+                const u32 part = v.low_counts ? (k < v.low_counts[row] ? 0u : 1u) : min(load(v.ids + slot[k]) / v.part_experts, v.parts - 1);
                 for (; p < part; ++p) flush();
                 run = part == p;
                 if (run) {
@@ -126,20 +128,21 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
 // memory latencies (three in the general form, with two block barriers between them), a large one wants bytes in flight.
 // 4096 rows x 8 x 2048: 79 us in the general form, 60 here (5.0 TB/s); 8 rows 3.1 and 2.2; 37 rows 4.0 and 2.8.
 __global__ void __launch_bounds__(128) combine_slots_kernel(b200moe_combine_view v) {
+    chain_begin();
     const u32 o = 2u * (blockIdx.x * 128u + threadIdx.x);
     if (o >= v.hidden) return;
-    const u32 job = v.summary ? __ldg(v.summary) : 0u;
+    const u32 job = v.summary ? load(v.summary) : 0u;
     for (u32 row = blockIdx.y; row < v.rows; row += gridDim.y) {
-        const u32 status = v.row_status ? __ldg(v.row_status + row) : 0u;
+        const u32 status = v.row_status ? load(v.row_status + row) : 0u;
         float2 x[kVecTopK];
         float w[kVecTopK];
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
             if (k < v.top_k) {
-                x[k] = __ldg(reinterpret_cast<const float2*>(v.raw + (u64(row) * v.top_k + k) * v.hidden + o));
-                w[k] = __ldg(v.weights + row * v.top_k + k);
+                x[k] = load(reinterpret_cast<const float2*>(v.raw + (u64(row) * v.top_k + k) * v.hidden + o));
+                w[k] = load(v.weights + row * v.top_k + k);
             }
-        const float2 sh = v.shared ? __ldg(reinterpret_cast<const float2*>(v.shared + u64(row) * v.hidden + o)) : make_float2(0.0f, 0.0f);
+        const float2 sh = v.shared ? load(reinterpret_cast<const float2*>(v.shared + u64(row) * v.hidden + o)) : make_float2(0.0f, 0.0f);
         float2 y = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
@@ -159,11 +162,13 @@ __global__ void __launch_bounds__(256) canonical_sum_kernel(const float* a, cons
 }
 
 __global__ void __launch_bounds__(256) fill_u32_kernel(u32* p, u32 value, u64 count) {
+    chain_begin();
     const u64 i = u64(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < count) p[i] = value;
 }
 
 __global__ void __launch_bounds__(256) row_order_kernel(const u32* ids, u32 rows, u32 top_k, u32* order) {
+    chain_begin();
     const u32 row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= rows) return;
     u32 key[kMaxTopK], slot[kMaxTopK];
@@ -197,16 +202,16 @@ int launch_combine(const b200moe_combine_view& v, cudaStream_t stream) {
     const bool whole = v.y && !v.y_blocks && v.top_k <= kVecTopK;
     if (v.form == B200MOE_COMBINE_PARTS && whole && v.only_part < 0 && v.hidden % 4 == 0 && aligned(v.raw, 16) && aligned(v.y, 16) && aligned(v.shared, 16) && aligned(v.y_bf16, 8)) {
         if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_vec_kernel))) return rc;
-        combine_vec_kernel<<<dim3((v.hidden + 511) / 512, std::min<u32>(v.rows, 65535u)), 128, 0, stream>>>(v);
+        chain_launch(combine_vec_kernel, dim3((v.hidden + 511) / 512, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v);
         return after_launch("combine");
     }
     if (v.form == B200MOE_COMBINE_FMA_SLOTS && whole && v.hidden % 2 == 0 && aligned(v.raw, 8) && aligned(v.y, 8) && aligned(v.shared, 8) && aligned(v.y_bf16, 4)) {
         if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_slots_kernel))) return rc;
-        combine_slots_kernel<<<dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 128, 0, stream>>>(v);
+        chain_launch(combine_slots_kernel, dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v);
         return after_launch("combine");
     }
     if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_kernel))) return rc;
-    combine_kernel<<<dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 256, 0, stream>>>(v);
+    chain_launch(combine_kernel, dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 256, 0, stream, v);
     return after_launch("combine");
 }
 int launch_canonical_sum(const float* a, const float* b, const float* c, u64 count, float* y, cudaStream_t stream) {
@@ -216,12 +221,12 @@ int launch_canonical_sum(const float* a, const float* b, const float* c, u64 cou
 }
 int launch_fill_u32(u32* p, u32 value, u64 count, cudaStream_t stream) {
     if (count == 0) return B200MOE_OK;
-    fill_u32_kernel<<<static_cast<u32>((count + 255) / 256), 256, 0, stream>>>(p, value, count);
+    chain_launch(fill_u32_kernel, static_cast<u32>((count + 255) / 256), 256, 0, stream, p, value, count);
     return after_launch("fill_u32");
 }
 int launch_row_order(const u32* ids, u32 rows, u32 top_k, u32* order, cudaStream_t stream) {
     if (rows == 0) return B200MOE_OK;
-    row_order_kernel<<<(rows + 255) / 256, 256, 0, stream>>>(ids, rows, top_k, order);
+    chain_launch(row_order_kernel, (rows + 255) / 256, 256, 0, stream, ids, rows, top_k, order);
     return after_launch("row_order");
 }
 

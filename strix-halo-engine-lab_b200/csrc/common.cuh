@@ -66,6 +66,31 @@ inline bool down_reads_sums(u32 type) { return type == B200MOE_TYPE_Q4_K || type
 
 // ---- device helpers ------------------------------------------------------------------------------------------------
 #if defined(__CUDACC__)
+// ---- the chain of a call's launches ----------------------------------------------------------------------------------
+// A call is a chain of dependent launches, most of them a few microseconds long. Each is enqueued with programmatic stream
+// serialisation: it is brought onto the SMs while the launch before it still runs and waits there, in chain_begin, until
+// that one has completed and its writes are visible. Every kernel launched so calls chain_begin before it touches global
+// memory, on every path: a launch that has passed it knows that everything enqueued before it is complete, which is also what lets it
+// admit its successor at once. Written data is read by plain loads (load below), never through the read-only path: the kernel
+// runs already while its predecessor writes, and such a load may be moved in front of the wait.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_admit() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_begin() {
+    chain_wait();
+    chain_admit();
+}
+template <class T>
+__device__ __forceinline__ T load(const T* p) { return *p; }
+// Enqueues a kernel of the chain; its status is read by after_launch.
+template <class... P, class... A>
+inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = attr; c.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
 __device__ __forceinline__ float half_bits_to_float(u32 h) {  // exact for every fp16 value, subnormals included
     return __half2float(__ushort_as_half(static_cast<unsigned short>(h)));
 }

@@ -66,7 +66,7 @@ struct Ep {
     unsigned char* win[kMaxWorld];
     EpLayout lay;
     float** yblocks[2];  // device arrays [world]: block `rank` of every home rank's parts, per parity
-    u32* counters;       // device: [0] completed steps, [1] dispatch ticket, [2] the dispatch wait gave up, [3] fold ticket, [4] prologue ticket
+    u32* counters;       // device: [0] completed steps, [1] dispatch ticket, [2] the dispatch wait gave up, [3] fold ticket
     u32 calls;
     u32 wait_polls;
 };
@@ -313,14 +313,12 @@ int b200moe_ep_ffn(void* handle, const b200moe_ep_step_view* v, void* stream) {
     r.x = x32; r.x_stride = s.hidden; r.rows = v->rows; r.hidden = s.hidden;
     r.weight = v->router_weight; r.logit_bias = v->logit_bias; r.bias = v->select_bias; r.policy = ep->policy;
     r.logits = W.logits; r.scores = W.logits; r.ids = W.ids; r.weights = W.wts;
-    if (prologue_fusable(r, s.top_k)) {  // decode windows: A8 + logits + selection in one launch (no local routes: null outputs)
-        b200moe_routes_view none{};
-        none.rows = v->rows; none.top_k = s.top_k; none.experts = s.experts;
-        if (int rc = launch_prologue(r, q, none, ep->counters + 4, st)) return rc;
+    if (prologue_fusable(r, s.top_k)) {  // decode windows: A8 and logits in one launch
+        if (int rc = launch_prologue(r, q, st)) return rc;
     } else {
         if (int rc = launch_router_logits(r, st, &q)) return rc;
-        if (int rc = launch_router_select(r, st)) return rc;
     }
+    if (int rc = launch_router_select(r, st)) return rc;
 
     // 2. dispatch, then wait for every rank's rows
     EpDev d{};

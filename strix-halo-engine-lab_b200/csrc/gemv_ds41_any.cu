@@ -30,7 +30,7 @@ __device__ __forceinline__ float term_q2_k(const u8* __restrict__ wrow, u32 g, c
     int qx[2] = {0, 0}, sx[2] = {0, 0};
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const u32 qw = (__ldg(q + i) >> shift) & 0x03030303u, xw = x[i];
+        const u32 qw = (load(q + i) >> shift) & 0x03030303u, xw = x[i];
         qx[i >> 2] = __dp4a(static_cast<int>(qw), static_cast<int>(xw), qx[i >> 2]);
         sx[i >> 2] = __dp4a(0x01010101, static_cast<int>(xw), sx[i >> 2]);
     }
@@ -45,11 +45,11 @@ __device__ __forceinline__ float term_q2_k(const u8* __restrict__ wrow, u32 g, c
 __device__ __forceinline__ float term_q8_0(const u8* __restrict__ wrow, u32 g, const i8* __restrict__ codes, float delta) {
     const unsigned short* blk = reinterpret_cast<const unsigned short*>(wrow + u64(g) * kQ8Block);
     const unsigned short* x = reinterpret_cast<const unsigned short*>(codes);
-    const float scale = half_bits_to_float(__ldg(blk));
+    const float scale = half_bits_to_float(load(blk));
     int dot = 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        const u32 w = __ldg(blk + 1 + i), c = x[i];
+        const u32 w = load(blk + 1 + i), c = x[i];
         dot += static_cast<int>(static_cast<signed char>(w & 0xffu)) * static_cast<int>(static_cast<signed char>(c & 0xffu));
         dot += static_cast<int>(static_cast<signed char>(w >> 8)) * static_cast<int>(static_cast<signed char>(c >> 8));
     }
@@ -79,6 +79,7 @@ __device__ __forceinline__ void ds41_row(const u8* __restrict__ wrow, u32 groups
 // grid (inter / 32, max_union): one CTA = one expert x one 32-output group; 8 warps walk the 64 rows (32 gate, 32 up).
 template <u32 TYPE>
 __global__ void __launch_bounds__(kWarps * 32) gate_up_ds41_any_kernel(b200moe_gate_up_view v) {
+    chain_begin();
     __shared__ float s_g[kR * 32], s_u[kR * 32];
     __shared__ u32 s_slots[kR];
     __shared__ const i8* s_codes[kR];
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kWarps * 32) gate_up_ds41_any_kernel(b200moe_g
 // grid (hidden / 32, max_union): 8 warps walk 32 down rows.
 template <u32 TYPE>
 __global__ void __launch_bounds__(kWarps * 32) down_ds41_any_kernel(b200moe_down_view v) {
+    chain_begin();
     __shared__ u32 s_slots[kR];
     __shared__ const i8* s_codes[kR];
     __shared__ const float* s_deltas[kR];
@@ -171,16 +173,16 @@ __global__ void __launch_bounds__(kWarps * 32) down_ds41_any_kernel(b200moe_down
 int launch_gate_up_ds41_any(const b200moe_gate_up_view& v, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     const dim3 grid(v.shape.inter / 32, v.max_union);
-    if (v.shape.gate_type == B200MOE_TYPE_Q2_K) gate_up_ds41_any_kernel<B200MOE_TYPE_Q2_K><<<grid, kWarps * 32, 0, stream>>>(v);
-    else gate_up_ds41_any_kernel<B200MOE_TYPE_Q8_0><<<grid, kWarps * 32, 0, stream>>>(v);
+    if (v.shape.gate_type == B200MOE_TYPE_Q2_K) chain_launch(gate_up_ds41_any_kernel<B200MOE_TYPE_Q2_K>, grid, kWarps * 32, 0, stream, v);
+    else chain_launch(gate_up_ds41_any_kernel<B200MOE_TYPE_Q8_0>, grid, kWarps * 32, 0, stream, v);
     return after_launch("gate_up_ds41_any");
 }
 
 int launch_down_ds41_any(const b200moe_down_view& v, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     const dim3 grid(v.shape.hidden / 32, v.max_union);
-    if (v.shape.down_type == B200MOE_TYPE_Q2_K) down_ds41_any_kernel<B200MOE_TYPE_Q2_K><<<grid, kWarps * 32, 0, stream>>>(v);
-    else down_ds41_any_kernel<B200MOE_TYPE_Q8_0><<<grid, kWarps * 32, 0, stream>>>(v);
+    if (v.shape.down_type == B200MOE_TYPE_Q2_K) chain_launch(down_ds41_any_kernel<B200MOE_TYPE_Q2_K>, grid, kWarps * 32, 0, stream, v);
+    else chain_launch(down_ds41_any_kernel<B200MOE_TYPE_Q8_0>, grid, kWarps * 32, 0, stream, v);
     return after_launch("down_ds41_any");
 }
 

@@ -80,10 +80,10 @@ __device__ __forceinline__ void q4k_row(const u8* __restrict__ wrow, u32 nblocks
         k.hdr = make_uint4(0, 0, 0, 0); k.q0 = k.hdr; k.q1 = k.hdr; k.h0 = k.hdr; k.h1 = k.hdr;
         if (b < nblocks) {
             const uint4* blk = reinterpret_cast<const uint4*>(wrow + u64(b) * (Q5K ? kQ5KBlock : kQ4KBlock));
-            k.hdr = __ldg(blk);
-            if (Q5K) { k.h0 = __ldg(blk + 1); k.h1 = __ldg(blk + 2); }  // Q5_K: 32 bytes of high bits between header and nibbles
-            k.q0 = __ldg(blk + (Q5K ? 3 : 1) + 2 * p);
-            k.q1 = __ldg(blk + (Q5K ? 4 : 2) + 2 * p);
+            k.hdr = load(blk);
+            if (Q5K) { k.h0 = load(blk + 1); k.h1 = load(blk + 2); }  // Q5_K: 32 bytes of high bits between header and nibbles
+            k.q0 = load(blk + (Q5K ? 3 : 1) + 2 * p);
+            k.q1 = load(blk + (Q5K ? 4 : 2) + 2 * p);
         }
         return k;
     };
@@ -149,6 +149,7 @@ __device__ __forceinline__ void stage_a8(const b200moe_a8_rows& src, const u32* 
 // grid (inter / 32, max_union); 256 threads. One CTA = one expert x one 32-output group (= one A8 group of h).
 template <int LPR, bool Q5K>
 __global__ void __launch_bounds__(256) gate_up_q4k_kernel(b200moe_gate_up_view v) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const u32 j = blockIdx.y;
     if (j >= v.routes.counts[0]) return;
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(256) gate_up_q4k_kernel(b200moe_gate_up_view v
 // the dense block has one "expert") down rows per CTA, Q4_K rows over K = inter.
 template <int LPR>
 __global__ void __launch_bounds__(256) down_q4k_kernel(b200moe_down_view v, u32 rows_per_cta) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (v.summary && *v.summary) return;  // a failed projection skips the whole down stage (routed_expert.hpp:17-19)
     const u32 j = blockIdx.y;
@@ -267,21 +269,21 @@ __device__ __forceinline__ void load_chain_block(const u8* b, ChainBlock<Q51>& o
         // Q5_1 (routed_expert.cpp:124-133): 24-byte blocks, 8-byte aligned. Weight k < 16 = low nibble of byte k, k >= 16 = high
         // nibble of byte k - 16, bit k of the 32 high bits on top: unsigned 0..31. Kept raw here, spread when used.
         const uint2* b8 = reinterpret_cast<const uint2*>(b);
-        const uint2 hd = __ldg(b8), qa = __ldg(b8 + 1), qb = __ldg(b8 + 2);
+        const uint2 hd = load(b8), qa = load(b8 + 1), qb = load(b8 + 2);
         o.q[0] = qa.x; o.q[1] = qa.y; o.q[2] = qb.x; o.q[3] = qb.y; o.q[4] = hd.x; o.q[5] = hd.y;
     } else {  // 34-byte blocks are 2-byte aligned: whole words where the quants lie on one, else words and a byte permute
         const bool odd = (reinterpret_cast<uintptr_t>(b) & 2u) != 0;
-        o.d = half_bits_to_float(__ldg(reinterpret_cast<const u16*>(b)));
+        o.d = half_bits_to_float(load(reinterpret_cast<const u16*>(b)));
         if (odd) {
             const u32* w = reinterpret_cast<const u32*>(b + 2);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o.q[i] = __ldg(w + i);
+            for (int i = 0; i < 8; ++i) o.q[i] = load(w + i);
         } else {
             const u32* w = reinterpret_cast<const u32*>(b);
             u32 r[9];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) r[i] = __ldg(w + i);
-            r[8] = __ldg(reinterpret_cast<const u16*>(b + 32));  // nothing is read past the block
+            for (int i = 0; i < 8; ++i) r[i] = load(w + i);
+            r[8] = load(reinterpret_cast<const u16*>(b + 32));  // nothing is read past the block
 #pragma unroll
             for (int i = 0; i < 8; ++i) o.q[i] = __byte_perm(r[i], r[i + 1], 0x5432u);
         }
@@ -311,6 +313,7 @@ __device__ __forceinline__ void spread_chain_block(ChainBlock<Q51>& o) {
 constexpr u32 kChainBatch = 3;
 template <bool Q51>
 __global__ void __launch_bounds__(256) down_q8_chain4_kernel(b200moe_down_view v) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (v.summary && *v.summary) return;
     const u32 j = blockIdx.y;
@@ -396,10 +399,10 @@ int launch_gate_up_q4k(const b200moe_gate_up_view& v, cudaStream_t stream) {
     {                                                                                \
         if (v.shape.gate_type == B200MOE_TYPE_Q5_K) {                                \
             if (int rc = set_smem(gate_up_q4k_kernel<L, true>, smem)) return rc;     \
-            gate_up_q4k_kernel<L, true><<<grid, 256, smem, stream>>>(v);             \
+            chain_launch(gate_up_q4k_kernel<L, true>, grid, 256, smem, stream, v);             \
         } else {                                                                     \
             if (int rc = set_smem(gate_up_q4k_kernel<L, false>, smem)) return rc;    \
-            gate_up_q4k_kernel<L, false><<<grid, 256, smem, stream>>>(v);            \
+            chain_launch(gate_up_q4k_kernel<L, false>, grid, 256, smem, stream, v);            \
         }                                                                            \
     }
     switch (lanes_per_row(H / 256)) {
@@ -421,7 +424,7 @@ int launch_down_q4k(const b200moe_down_view& v, cudaStream_t stream) {
 #define B200_DN(L)                                                     \
     {                                                                  \
         if (int rc = set_smem(down_q4k_kernel<L>, smem)) return rc;    \
-        down_q4k_kernel<L><<<grid, 256, smem, stream>>>(v, rpc);       \
+        chain_launch(down_q4k_kernel<L>, grid, 256, smem, stream, v, rpc);       \
     }
     switch (lanes_per_row(I / 256)) {
         case 32: B200_DN(32) break;
@@ -438,10 +441,10 @@ int launch_down_q8_chain4(const b200moe_down_view& v, cudaStream_t stream) {
     const u32 smem = kR * (I + I / 32 * 8);
     if (v.shape.down_type == B200MOE_TYPE_Q5_1) {
         if (int rc = set_smem(down_q8_chain4_kernel<true>, smem)) return rc;
-        down_q8_chain4_kernel<true><<<dim3(H / 64, v.max_union), 256, smem, stream>>>(v);
+        chain_launch(down_q8_chain4_kernel<true>, dim3(H / 64, v.max_union), 256, smem, stream, v);
     } else {
         if (int rc = set_smem(down_q8_chain4_kernel<false>, smem)) return rc;
-        down_q8_chain4_kernel<false><<<dim3(H / 64, v.max_union), 256, smem, stream>>>(v);
+        chain_launch(down_q8_chain4_kernel<false>, dim3(H / 64, v.max_union), 256, smem, stream, v);
     }
     return after_launch("down_q8_chain4");
 }

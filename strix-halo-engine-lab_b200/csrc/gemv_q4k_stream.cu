@@ -197,7 +197,7 @@ __device__ __forceinline__ void item_range(const StreamPlan& plan, const b200moe
     u32 total = 0;
     for (u32 j0 = 0; j0 < n_union; j0 += 32) {
         const u32 j = j0 + lane;
-        const u32 c = j < n_union ? item_cost(__ldg(routes.begins + j + 1) - __ldg(routes.begins + j)) * nc : 0u;
+        const u32 c = j < n_union ? item_cost(load(routes.begins + j + 1) - load(routes.begins + j)) * nc : 0u;
         total += __shfl_sync(0xffffffffu, warp_inclusive_scan(c, lane), 31);
     }
     const u32 n_items = n_union * nc;
@@ -205,7 +205,7 @@ __device__ __forceinline__ void item_range(const StreamPlan& plan, const b200moe
     u32 lo = n_items, hi = n_items, cum = 0;  // a boundary at `total` means "past the last item"
     for (u32 j0 = 0; j0 < n_union; j0 += 32) {
         const u32 j = j0 + lane;
-        const u32 ci = j < n_union ? item_cost(__ldg(routes.begins + j + 1) - __ldg(routes.begins + j)) : 0u;
+        const u32 ci = j < n_union ? item_cost(load(routes.begins + j + 1) - load(routes.begins + j)) : 0u;
         const u32 c = ci * nc, incl = warp_inclusive_scan(c, lane), excl = cum + incl - c;
         const bool h0 = c && B0 >= excl && B0 < excl + c, h1 = c && B1 >= excl && B1 < excl + c;
         const u32 c0 = h0 ? j * nc + (B0 - excl + ci - 1) / ci : 0u, c1 = h1 ? j * nc + (B1 - excl + ci - 1) / ci : 0u;
@@ -240,13 +240,13 @@ __device__ __forceinline__ Meta load_meta(const StreamPlan& plan, const b200moe_
     u32 j;
     Meta m;
     split_item(plan, item, &j, &m.chunk);
-    m.eb = __ldg(routes.begins + j);
-    m.ne = __ldg(routes.begins + j + 1) - m.eb;
+    m.eb = load(routes.begins + j);
+    m.ne = load(routes.begins + j + 1) - m.eb;
     return m;
 }
-__device__ __forceinline__ void load_first(const u32* __restrict__ ids, const Meta& m, u32* first) {
+__device__ __forceinline__ void load_first(const u32* ids, const Meta& m, u32* first) {
 #pragma unroll
-    for (int r = 0; r < kR; ++r) first[r] = __ldg(ids + m.eb + min(u32(r), m.ne - 1u));
+    for (int r = 0; r < kR; ++r) first[r] = load(ids + m.eb + min(u32(r), m.ne - 1u));
 }
 
 // ---- the row rule over one octet -----------------------------------------------------------------------------------
@@ -388,6 +388,7 @@ __device__ __forceinline__ void finish_x_rows(u32 rows, u32 H, unsigned char* ds
 }
 
 __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) gate_up_q4k_stream_kernel(b200moe_gate_up_view v, StreamPlan plan) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
     const u32 H = v.shape.hidden, I = v.shape.inter, nblocks = H / 256;
     const u32 ME = plan.max_entries;
@@ -527,6 +528,7 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) gate_up_q4k_
 // Item = (expert, 64 hidden outputs) = 8 octets. Activations (the A8 of h) are read from global memory: every lane of a
 // row group reads the same addresses, so the loads are broadcasts served by L1 / L2.
 __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) down_q4k_stream_kernel(b200moe_down_view v, StreamPlan plan) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
     const u32 H = v.shape.hidden, I = v.shape.inter, nblocks = I / 256;
     u64* bars = reinterpret_cast<u64*>(smem + u64(plan.stages) * plan.stage_bytes);
@@ -566,12 +568,12 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) down_q4k_str
         u32 j_lo, j_hi, unused;
         split_item(plan, first_item, &j_lo, &unused);
         split_item(plan, first_item + n_local - 1u, &j_hi, &unused);
-        eb_lo = __ldg(v.routes.begins + j_lo);
-        n_stage = min(__ldg(v.routes.begins + j_hi + 1) - eb_lo, plan.stage_entries);
+        eb_lo = load(v.routes.begins + j_lo);
+        n_stage = min(load(v.routes.begins + j_hi + 1) - eb_lo, plan.stage_entries);
         const u32 gs = act_stride / 32, nthreads = plan.warps * 32;
         const bool al16 = (reinterpret_cast<uintptr_t>(v.act.deltas) % 16 == 0) && (reinterpret_cast<uintptr_t>(v.act.sums) % 16 == 0) && gs % 4 == 0 && I % 128 == 0;
         for (u32 e = 0; e < n_stage; ++e) {
-            const u32 sl = __ldg(v.routes.slots + eb_lo + e);
+            const u32 sl = load(v.routes.slots + eb_lo + e);
             const u32 d = saddr(a_copy + u64(e) * a_row);
             const i8* src = v.act.codes + u64(sl) * act_stride;
             for (u32 c = threadIdx.x; c < I / 16; c += nthreads) cp_async(d + 16u * c, src + 16u * c, 16);
@@ -712,7 +714,7 @@ int launch_gate_up_q4k_stream(const b200moe_gate_up_view& v, u32 rows, cudaStrea
     p.x_rows = rows;
     const u32 smem = plan_smem(p, x_bytes, slot_bytes);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(gate_up_q4k_stream_kernel), smem)) return rc;
-    gate_up_q4k_stream_kernel<<<sm_count(), (p.warps + kProducers) * 32, smem, stream>>>(v, p);
+    chain_launch(gate_up_q4k_stream_kernel, sm_count(), (p.warps + kProducers) * 32, smem, stream, v, p);
     return after_launch("gate_up_q4k_stream");
 }
 
@@ -726,7 +728,7 @@ int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, cudaStream_t st
     p.stage_entries = down_stage_entries(v);
     const u32 smem = plan_smem(p, down_fixed_bytes(v), 0);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(down_q4k_stream_kernel), smem)) return rc;
-    down_q4k_stream_kernel<<<sm_count(), (p.warps + kProducers) * 32, smem, stream>>>(v, p);
+    chain_launch(down_q4k_stream_kernel, sm_count(), (p.warps + kProducers) * 32, smem, stream, v, p);
     return after_launch("down_q4k_stream");
 }
 

@@ -211,6 +211,7 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* w8, u32 nbk,
 template <bool DOWN, u32 S_>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, WideArgs a, WidePlan plan) {
+    chain_begin();
     using G = Geo<S_>;
     extern __shared__ __align__(128) unsigned char smem[];
     if (DOWN && a.summary && *a.summary) return;  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
@@ -277,7 +278,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             }
             const u32 ve_ne = ve.ne();
             u32 r = 0;
-            if (e < ve_ne) r = __ldg((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
+            if (e < ve_ne) r = load((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
             const u32 nsegs = end ? 1u : plan.nseg;
             for (u32 s = 0; s < nsegs; ++s, ++t, ++slot) {
                 if (slot == plan.stages) { slot = 0; ++use; }
@@ -346,6 +347,13 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         const VExpert ve = table[jv];
         const u32 ne = ve.ne(), vbegin = ve.begin();
         const bool mma = ne >= kMmaMinEntries;
+        u32 slots[kMmaMinEntries - 1] = {}, slot_id = 0;  // asked for before the stages, used behind them
+        if (DOWN && mma) slot_id = (lane >> 2) < ne ? load(a.routes.slots + vbegin + (lane >> 2)) : 0u;
+        if (!DOWN) slot_id = w < ne ? load(a.routes.slots + vbegin + w) : 0u;
+        if (DOWN && !mma) {
+#pragma unroll
+            for (int r = 0; r < (int)kMmaMinEntries - 1; ++r) slots[r] = load(a.routes.slots + vbegin + min(u32(r), ne - 1u));
+        }
         float acc[kMmaMinEntries - 1];
         float2 acc2[4];  // mma form
 #pragma unroll
@@ -385,7 +393,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         if (DOWN) {
             if (mma) {
                 if (me < ne) {
-                    float* dst = a.raw + u64(__ldg(a.routes.slots + vbegin + me)) * a.out_width + kItemRows * chunk + 8u * w + 2u * mt;
+                    float* dst = a.raw + u64(slot_id) * a.out_width + kItemRows * chunk + 8u * w + 2u * mt;
                     if (a.raw_vec) *reinterpret_cast<float2*>(dst) = make_float2(m0, m1);
                     else { dst[0] = m0; dst[1] = m1; }
                 }
@@ -394,7 +402,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 for (int r = 0; r < (int)kMmaMinEntries - 1; ++r) {
                     if (r < (int)ne) {
                         const float val = tree4(acc[r]);
-                        if (p == 0) a.raw[u64(__ldg(a.routes.slots + vbegin + r)) * a.out_width + kItemRows * chunk + 8u * w + rr] = val;
+                        if (p == 0) a.raw[u64(slots[r]) * a.out_width + kItemRows * chunk + 8u * w + rr] = val;
                     }
                 }
             }
@@ -420,13 +428,13 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             if (!ok) break;
             if (w < ne) {  // SwiGLU + the A8 rule over the 32 outputs of entry w
                 const float gv = gu[w * 32 + lane], uv = gu[kKE * 32 + w * 32 + lane];
-                const u32 slot_id = __ldg(a.routes.slots + vbegin + w), o_col = 32u * chunk + lane;
+                const u32 o_col = 32u * chunk + lane;
                 if (a.gate_out) { a.gate_out[u64(slot_id) * a.out_width + o_col] = gv; a.up_out[u64(slot_id) * a.out_width + o_col] = uv; }
                 const float h = swiglu_qwen(gv, uv);
                 const bool bad = __any_sync(0xffffffffu, !finite_f(gv) || !finite_f(uv) || !finite_f(h));
                 if (bad) {  // fail closed: nothing of the group is written (routed_expert.cpp:147-156)
                     if (lane == 0) {
-                        if (a.row_status) atomicOr(&a.row_status[__ldg(a.routes.rows + vbegin + w)], B200MOE_ROW_PROJECTION_NONFINITE);
+                        if (a.row_status) atomicOr(&a.row_status[load(a.routes.rows + vbegin + w)], B200MOE_ROW_PROJECTION_NONFINITE);
                         if (a.summary) atomicOr(a.summary, B200MOE_ROW_PROJECTION_NONFINITE);
                     }
                 } else {
@@ -520,10 +528,10 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_
     const u32 smem = plan_smem(p, false);
     if (p.S == 3) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<false, 3>), smem)) return rc;
-        q4k_wide_kernel<false, 3><<<sm_count(), kThreads, smem, stream>>>(tm0, tm1, a, p);
+        chain_launch(q4k_wide_kernel<false, 3>, sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
     } else {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<false, 1>), smem)) return rc;
-        q4k_wide_kernel<false, 1><<<sm_count(), kThreads, smem, stream>>>(tm0, tm1, a, p);
+        chain_launch(q4k_wide_kernel<false, 1>, sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
     }
     return after_launch("gate_up_q4k_wide");
 }
@@ -542,10 +550,10 @@ int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, cudaStream_t stre
     const u32 smem = plan_smem(p, true);
     if (p.S == 3) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<true, 3>), smem)) return rc;
-        q4k_wide_kernel<true, 3><<<sm_count(), kThreads, smem, stream>>>(tm0, tm0, a, p);
+        chain_launch(q4k_wide_kernel<true, 3>, sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
     } else {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<true, 1>), smem)) return rc;
-        q4k_wide_kernel<true, 1><<<sm_count(), kThreads, smem, stream>>>(tm0, tm0, a, p);
+        chain_launch(q4k_wide_kernel<true, 1>, sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
     }
     return after_launch("down_q4k_wide");
 }

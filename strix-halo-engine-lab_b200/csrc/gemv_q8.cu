@@ -38,7 +38,7 @@ __device__ __forceinline__ void run_load(const u8* src, u32 nb, u32 lane, RunReg
     const uint4* s4 = reinterpret_cast<const uint4*>(src);
     const u32 n16 = nb * kQ8Block / 16;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) if (lane + 32u * k < n16) r.v[k] = __ldg(s4 + lane + 32u * k);
+    for (int k = 0; k < 3; ++k) if (lane + 32u * k < n16) r.v[k] = load(s4 + lane + 32u * k);
 }
 __device__ __forceinline__ void run_store(u32* stage, u32 nb, u32 lane, const RunRegs& r) {
     uint4* d4 = reinterpret_cast<uint4*>(stage);
@@ -135,6 +135,7 @@ __device__ __forceinline__ void stage_rows(const b200moe_a8_rows& src, const u32
 
 // Dense site: out[r][o] for o in [first, first + count). grid (ceil(count / 32)); 256 threads; rows in passes of 8.
 __global__ void __launch_bounds__(1024) q8_0_a8_kernel(b200moe_q8a8_view v, u32 align) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const u32 K = v.width, groups = K / 32, nw = blockDim.x >> 5;
     i8* s_codes = reinterpret_cast<i8*>(smem_raw);
@@ -172,6 +173,7 @@ __global__ void __launch_bounds__(1024) q8_0_a8_kernel(b200moe_q8a8_view v, u32 
 
 // Routed gate/up: grid (inter / 32, max_union); 256 threads; one CTA = one expert x one 32-output group.
 __global__ void __launch_bounds__(1024) gate_up_q8_kernel(b200moe_gate_up_view v, u32 align) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const u32 j = blockIdx.y, nw = blockDim.x >> 5;
     if (j >= v.routes.counts[0]) return;
@@ -236,6 +238,7 @@ __global__ void __launch_bounds__(1024) gate_up_q8_kernel(b200moe_gate_up_view v
 
 // Routed down: grid (hidden / 32, max_union); 256 threads.
 __global__ void __launch_bounds__(1024) down_q8_kernel(b200moe_down_view v, u32 align) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (v.summary && *v.summary) return;
     const u32 j = blockIdx.y, nw = blockDim.x >> 5;
@@ -291,7 +294,7 @@ int launch_q8_0_a8(const b200moe_q8a8_view& v, cudaStream_t stream) {
     const u32 nw = kDenseWarps;
     const u32 smem = kR * (K + K / 32 * 4) + nw * kStageBytes;
     if (int rc = set_smem(q8_0_a8_kernel, smem)) return rc;
-    q8_0_a8_kernel<<<(v.count + 31) / 32, nw * 32, smem, stream>>>(v, align);
+    chain_launch(q8_0_a8_kernel, (v.count + 31) / 32, nw * 32, smem, stream, v, align);
     return after_launch("q8_0_a8");
 }
 
@@ -310,7 +313,7 @@ int launch_gate_up_q8(const b200moe_gate_up_view& v, cudaStream_t stream) {
     const u32 nw = kRoutedWarps;   // 64 weight rows per CTA: two per warp, the second one prefetched
     const u32 smem = kR * (H + H / 32 * 4) + 2 * kR * 32 * 4 + nw * kStageBytes;
     if (int rc = set_smem(gate_up_q8_kernel, smem)) return rc;
-    gate_up_q8_kernel<<<dim3(I / 32, v.max_union, pass_split(I / 32 * v.max_union, v.x.rows)), nw * 32, smem, stream>>>(v, align);
+    chain_launch(gate_up_q8_kernel, dim3(I / 32, v.max_union, pass_split(I / 32 * v.max_union, v.x.rows)), nw * 32, smem, stream, v, align);
     return after_launch("gate_up_q8");
 }
 
@@ -321,7 +324,7 @@ int launch_down_q8(const b200moe_down_view& v, cudaStream_t stream) {
     const u32 nw = kRoutedWarps;   // 32 weight rows per CTA: one per warp, every row of the expert in flight at once
     const u32 smem = kR * (I + I / 32 * 4) + nw * kStageBytes;
     if (int rc = set_smem(down_q8_kernel, smem)) return rc;
-    down_q8_kernel<<<dim3(H / 32, v.max_union, pass_split(H / 32 * v.max_union, v.act.rows)), nw * 32, smem, stream>>>(v, align);
+    chain_launch(down_q8_kernel, dim3(H / 32, v.max_union, pass_split(H / 32 * v.max_union, v.act.rows)), nw * 32, smem, stream, v, align);
     return after_launch("down_q8");
 }
 

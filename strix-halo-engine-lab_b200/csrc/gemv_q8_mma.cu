@@ -104,6 +104,7 @@ __device__ __forceinline__ void block_step(const unsigned char* rowA, const unsi
 template <bool DOWN>
 __global__ void __launch_bounds__(kMmaThreads, 1)
 q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, MmaArgs a, MmaPlan plan) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
     if (DOWN && a.summary && *a.summary) return;
     u32 n_union = a.routes.counts[0];
@@ -150,7 +151,7 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
             const bool new_x = jv != last_jv;
             last_jv = jv;
             u32 r = 0;
-            if (new_x && e < ne) r = __ldg((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
+            if (new_x && e < ne) r = load((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
             for (u32 si = 0; si < kTiles * plan.nst && ok; ++si, ++t) {
                 const u32 tile = si / plan.nst, s = si - tile * plan.nst;
                 const u32 slot = t & 1u, use = t >> 1;
@@ -209,7 +210,7 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
             ++xl;
             last_jv = jv;
         }
-        const u32 my_slot = DOWN && (lane >> 2) < ne ? __ldg(a.routes.slots + vbegin + (lane >> 2)) : 0u;
+        const u32 mine = DOWN ? lane >> 2 : warp, my_slot = mine < ne ? load(a.routes.slots + vbegin + mine) : 0u;  // asked for before the tiles, used behind them
         float* gu = s_gu + (kl & 1u) * (kGuFloats / 2);
         bool stop = false;
         for (u32 tile = 0; tile < kTiles; ++tile) {
@@ -272,7 +273,7 @@ q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ C
         if (stop) break;
         if (!DOWN && warp < ne) {  // swiglu_clamped + the A8 rule over the 32 outputs of entry `warp` (src/ds41_moe.cpp:134-146)
             const float gv = gu[warp * 32u + lane], uv = gu[KE * 32u + warp * 32u + lane];
-            const u32 slot_id = __ldg(a.routes.slots + vbegin + warp), o_col = 32u * chunk + lane;
+            const u32 slot_id = my_slot, o_col = 32u * chunk + lane;
             if (a.gate_out) { a.gate_out[u64(slot_id) * a.out_width + o_col] = gv; a.up_out[u64(slot_id) * a.out_width + o_col] = uv; }
             const float h = swiglu_ds41(gv, uv, a.limit);  // NaN propagates: this family has no status rule
             float delta;
@@ -345,7 +346,7 @@ int launch_gate_up_q8_mma(const b200moe_gate_up_view& v, u32 rows, cudaStream_t 
     const u32 smem = plan_smem(p, false);
     const auto kernel = q8_mma_kernel<false>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-    kernel<<<sm_count(), kMmaThreads, smem, stream>>>(tm0, tm1, a, p);
+    chain_launch(kernel, sm_count(), kMmaThreads, smem, stream, tm0, tm1, a, p);
     return after_launch("gate_up_q8_mma");
 }
 
@@ -362,7 +363,7 @@ int launch_down_q8_mma(const b200moe_down_view& v, u32 rows, cudaStream_t stream
     const u32 smem = plan_smem(p, true);
     const auto kernel = q8_mma_kernel<true>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-    kernel<<<sm_count(), kMmaThreads, smem, stream>>>(tm0, tm0, a, p);
+    chain_launch(kernel, sm_count(), kMmaThreads, smem, stream, tm0, tm0, a, p);
     return after_launch("down_q8_mma");
 }
 

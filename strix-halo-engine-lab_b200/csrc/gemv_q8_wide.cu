@@ -103,6 +103,7 @@ __device__ __forceinline__ void q8_stage(const unsigned char* w4, u32 nb, u32 ne
 template <bool DOWN>
 __global__ void __launch_bounds__(kThreads, 1)
 q8_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, Q8Args a, Q8Plan plan) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
     if (DOWN && a.summary && *a.summary) return;
     u32 n_union = a.routes.counts[0];
@@ -165,7 +166,7 @@ q8_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
             }
             const u32 ve_ne = ve.ne();
             u32 r = 0;
-            if (e < ve_ne) r = __ldg((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
+            if (e < ve_ne) r = load((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
             const u32 n = end ? 1u : item_stages;
             for (u32 s = 0; s < n; ++s, ++t, ++slot) {
                 if (slot == plan.stages) { slot = 0; ++use; }
@@ -222,6 +223,7 @@ q8_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
         const u32 jv = item / plan.n_chunks, chunk = item - jv * plan.n_chunks;
         const VExpert ve = table[jv];
         const u32 ne = ve.ne(), vbegin = ve.begin();
+        const u32 mine = DOWN ? lane : w, my_slot = mine < ne ? load(a.routes.slots + vbegin + mine) : 0u;  // asked for before the stages, used behind them
         float* gu = s_gu + u64((g * 2 + (kl & 1u)) * 2) * kKE * 32;
         for (u32 mat = 0; mat < (DOWN ? 1u : 2u); ++mat) {
             float cls[4][kKE];
@@ -249,8 +251,9 @@ q8_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
                         const float val = butterfly32(cls[r][t]);
+                        const u32 slot_id = __shfl_sync(0xffffffffu, my_slot, t);
                         if (lane == 0) {
-                            if (DOWN) a.raw[u64(__ldg(a.routes.slots + vbegin + t)) * a.out_width + kRows * chunk + 4u * w + r] = val;
+                            if (DOWN) a.raw[u64(slot_id) * a.out_width + kRows * chunk + 4u * w + r] = val;
                             else gu[mat * kKE * 32 + t * 32 + 4u * w + r] = val;
                         }
                     }
@@ -266,7 +269,7 @@ q8_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
             if (!ok) break;
             if (w < ne) {  // swiglu_clamped + the A8 rule over the 32 outputs of entry w (src/ds41_moe.cpp:134-146)
                 const float gv = gu[w * 32 + lane], uv = gu[kKE * 32 + w * 32 + lane];
-                const u32 slot_id = __ldg(a.routes.slots + vbegin + w), o_col = 32u * chunk + lane;
+                const u32 slot_id = my_slot, o_col = 32u * chunk + lane;
                 if (a.gate_out) { a.gate_out[u64(slot_id) * a.out_width + o_col] = gv; a.up_out[u64(slot_id) * a.out_width + o_col] = uv; }
                 const float h = swiglu_ds41(gv, uv, a.limit);  // NaN propagates: this family has no status rule
                 float delta;
@@ -339,7 +342,7 @@ int launch_gate_up_q8_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_t
     if (int rc = rows_map(v.weights.up, rb, total_rows, kRunBytes, kRows, &tm1)) return rc;
     const u32 smem = plan_smem(p, false);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q8_wide_kernel<false>), smem)) return rc;
-    q8_wide_kernel<false><<<sm_count(), kThreads, smem, stream>>>(tm0, tm1, a, p);
+    chain_launch(q8_wide_kernel<false>, sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
     return after_launch("gate_up_q8_wide");
 }
 
@@ -355,7 +358,7 @@ int launch_down_q8_wide(const b200moe_down_view& v, u32 rows, cudaStream_t strea
     if (int rc = rows_map(v.weights.down, u64(p.groups) * kQ8Block, u64(v.shape.experts) * v.shape.hidden, kRunBytes, kRows, &tm0)) return rc;
     const u32 smem = plan_smem(p, true);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q8_wide_kernel<true>), smem)) return rc;
-    q8_wide_kernel<true><<<sm_count(), kThreads, smem, stream>>>(tm0, tm0, a, p);
+    chain_launch(q8_wide_kernel<true>, sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
     return after_launch("down_q8_wide");
 }
 

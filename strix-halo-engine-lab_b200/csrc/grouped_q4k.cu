@@ -185,6 +185,7 @@ __device__ __forceinline__ void fast_factors(u32 head, u32 sc, u32 mn, float (&f
 template <bool kDown>
 __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
                                                                    GroupedArgs a) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
     float2* s_fold = reinterpret_cast<float2*>(smem + kOffFold);       // [warp][kFoldCells][lane]
     float* s_out = reinterpret_cast<float*>(smem + kOffFold);          // [kGN][kOutPitch]
@@ -516,7 +517,7 @@ int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t strea
     if (int rc = encode_rows_map(v.weights.gate, rb, rows, &tm0)) return rc;
     if (int rc = encode_rows_map(v.weights.up, rb, rows, &tm1)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<false>), kGroupedSmem)) return rc;
-    grouped_q4k_kernel<false><<<grid_size(), kGThreads, kGroupedSmem, stream>>>(tm0, tm1, a);
+    chain_launch(grouped_q4k_kernel<false>, grid_size(), kGThreads, kGroupedSmem, stream, tm0, tm1, a);
     return after_launch("gate_up_q4k_grouped");
 }
 
@@ -529,7 +530,7 @@ int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     CUtensorMap tm0;
     if (int rc = encode_rows_map(v.weights.down, u64(v.shape.inter / 256) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<true>), kGroupedSmem)) return rc;
-    grouped_q4k_kernel<true><<<grid_size(), kGThreads, kGroupedSmem, stream>>>(tm0, tm0, a);
+    chain_launch(grouped_q4k_kernel<true>, grid_size(), kGThreads, kGroupedSmem, stream, tm0, tm0, a);
     return after_launch("down_q4k_grouped");
 }
 

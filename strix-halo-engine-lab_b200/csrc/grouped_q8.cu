@@ -115,6 +115,7 @@ __device__ __forceinline__ void unit_step(const unsigned char* rows, const unsig
 
 template <bool kDown>
 __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, Q8Args a) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
     float2* s_sum = reinterpret_cast<float2*>(smem + kOffSum);         // [row half][block][cell][lane]
     float* s_out = reinterpret_cast<float*>(smem + kOffOut);           // [kTokens][kOutPitch]
@@ -379,7 +380,7 @@ int launch_gate_up_q8_grouped(const b200moe_gate_up_view& v, cudaStream_t stream
     if (int rc = wide::rows_map(v.weights.gate, rb, rows, kUnitBytes, 32, &tm0)) return rc;
     if (int rc = wide::rows_map(v.weights.up, rb, rows, kUnitBytes, 32, &tm1)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q8_kernel<false>), kSmem)) return rc;
-    grouped_q8_kernel<false><<<device_sm_count(), kGThreads, kSmem, stream>>>(tm0, tm1, a);
+    chain_launch(grouped_q8_kernel<false>, device_sm_count(), kGThreads, kSmem, stream, tm0, tm1, a);
     return after_launch("gate_up_q8_grouped");
 }
 
@@ -391,7 +392,7 @@ int launch_down_q8_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     CUtensorMap tm0;
     if (int rc = wide::rows_map(v.weights.down, u64(v.shape.inter / 32) * kQ8Block, u64(v.shape.experts) * v.shape.hidden, kUnitBytes, 32, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q8_kernel<true>), kSmem)) return rc;
-    grouped_q8_kernel<true><<<device_sm_count(), kGThreads, kSmem, stream>>>(tm0, tm0, a);
+    chain_launch(grouped_q8_kernel<true>, device_sm_count(), kGThreads, kSmem, stream, tm0, tm0, a);
     return after_launch("down_q8_grouped");
 }
 

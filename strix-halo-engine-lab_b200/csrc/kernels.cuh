@@ -20,7 +20,9 @@ int launch_router_select(const b200moe_router_view& v, cudaStream_t stream);
 
 // routes.cu
 u64 routes_scratch_words(u32 rows, u32 top_k, u32 experts);
-int launch_routes(const b200moe_routes_view& v, cudaStream_t stream);
+// what the first launch of a call that owns its status words clears on the way (each may be null): rows, 4 and 1 words
+struct RoutesClear { u32* row_status; u32* summary4; u32* summary; };
+int launch_routes(const b200moe_routes_view& v, const RoutesClear& clear, cudaStream_t stream);
 int launch_dense_routes(const b200moe_routes& out, u32 rows, u32* row_status, u32* summary4, cudaStream_t stream);
 // grouped (token-block) form of the Q4_K experts on the tensor cores (grouped_q4k.cu)
 bool grouped_fits(const b200moe_shape& s, bool have_sums);
@@ -29,7 +31,7 @@ int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t strea
 int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream);
 // decode windows: selection of r (logits already present) and the routes of the selected ids in one launch
 bool select_routes_fusable(const b200moe_router_view& r, u32 top_k);
-int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view& v, cudaStream_t stream);
+int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view& v, const RoutesClear& clear, cudaStream_t stream);
 
 // gemv_q8.cu: Q8_0 x A8 products in the 32-lane-class contract (dense rows and the routed DS41-family experts)
 int launch_q8_0_a8(const b200moe_q8a8_view& v, cudaStream_t stream);
@@ -74,10 +76,9 @@ int launch_down_q8_grouped(const b200moe_down_view& v, cudaStream_t stream);
 // value of a B200MOE_DEBUG_* hook (api.cu)
 u32 debug_value(u32 key);
 
-// prologue.cu: A8 + router + routes of a decode window (rows <= 8) in one launch; ticket: a zeroed workspace word
+// prologue.cu: A8 + router logits of a decode window (rows <= 8) in one launch; q.x / q.x_is_bf16 say where the activations are (r.x is not read)
 bool prologue_fusable(const b200moe_router_view& r, u32 top_k);
-int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view& q, const b200moe_routes_view& routes, u32* ticket,
-                    cudaStream_t stream);
+int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view& q, cudaStream_t stream);
 
 // combine.cu
 int launch_merge_first_error(b200moe_first_error* record, const u32* summary, u32 domain, cudaStream_t stream);

@@ -15,10 +15,11 @@ namespace {
 // SM; as launched it takes 29, eight CTAs.
 template <u32 WARPS>
 __global__ void __launch_bounds__(WARPS ? WARPS * 32u : 1024u) rmsnorm_a8_kernel(b200moe_rmsnorm_view v) {
+    chain_begin();
     __shared__ float partial[256];
     const u32 r = blockIdx.x, t = threadIdx.x, n = v.n;
     const u32 x_stride = v.x_stride ? v.x_stride : n, out_stride = v.out_stride ? v.out_stride : n;
-    const float* __restrict__ x = v.x + u64(r) * x_stride;
+    const float* x = v.x + u64(r) * x_stride;
     const u32 lanes = n >= 512u ? 256u : 128u;
     float a = 0.0f;
     if (t < lanes) {
@@ -76,8 +77,8 @@ int launch_rmsnorm_a8(const b200moe_rmsnorm_view& v, cudaStream_t stream) {
     // (592 rows of 2048: 11.6 against 11.8; of 1024: 7.5 both).
     const u32 sms = static_cast<u32>(device_sm_count());
     const u32 warps = v.rows <= 2u * sms ? std::min(32u, (v.n / 32u + 7u) / 8u * 8u) : 8u;
-    if (v.rows > 2u * sms && v.rows <= 5u * sms && v.n >= kWideRow) rmsnorm_a8_kernel<8><<<v.rows, 256, 0, stream>>>(v);
-    else rmsnorm_a8_kernel<0><<<v.rows, 32u * warps, 0, stream>>>(v);
+    if (v.rows > 2u * sms && v.rows <= 5u * sms && v.n >= kWideRow) chain_launch(rmsnorm_a8_kernel<8>, v.rows, 256, 0, stream, v);
+    else chain_launch(rmsnorm_a8_kernel<0>, v.rows, 32u * warps, 0, stream, v);
     return after_launch("rmsnorm_a8");
 }
 

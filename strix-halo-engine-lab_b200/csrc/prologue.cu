@@ -1,52 +1,57 @@
-// Layer prologue of decode windows (up to 8 rows) in ONE launch: A8 of the activations, router logits, score
-// transform + top-k selection + weights, and the window routes.
+// Front of a layer call over a decode window (up to 8 rows) in ONE launch: A8 of the activations and the router logits. Selection and routes follow in
+// a launch of one block (routes.cu).
 //
-// Contracts are those of the stand-alone kernels (a8.cu, router.cu, routes.cu): logits in the declared lane-strided
-// order without fused multiply-add (src/ds41_moe.cpp:72-82), the route policy's transforms and k-pass selection
-// (include/strix/moe/route_policy.hpp:99-156), build_window_routes (src/ds41_moe.cpp:11-61). Bits do not change.
+// Contracts are those of the stand-alone kernels (a8.cu, router.cu): logits in the declared lane-strided order without fused multiply-add
+// (src/ds41_moe.cpp:72-82). Bits do not change; bfloat16 activations are widened (exactly) on the way.
 //
-// Shape: blocks [0, logit_blocks) take eight experts each, one warp per expert. A warp copies its expert's current
-// 2048-wide run to shared memory asynchronously, the block does the same with that run of every activation row, then
-// each lane walks its lane class in ascending order. The
-// block that finishes last (a ticket counter in the workspace) runs selection (one warp per row) and the routes.
-// Blocks past logit_blocks quantise the activations. Everything the expert kernels need is ready after this launch.
+// Shape: blocks [0, logit_blocks) take four experts each. The block copies its experts' current 2048 columns and those of every activation row to
+// shared memory asynchronously, in four groups of columns, and works on a group while the next ones arrive; a warp walks the lane classes of its
+// experts and rows in ascending order. Blocks past logit_blocks quantise the activations, a warp a group of 32.
+// What bounds it: latency, of one trip to memory and of the serial chains. With selection and routes in the block that finishes last (a ticket in the
+// workspace), which had to find their code and read the logits back, the front took 10 / 12.3 / 20 us (1 row over 64 and 128 experts, 8 rows over
+// 128, hidden 2048), of it 6 to 12 us in that block.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "router_select.cuh"
-#include "routes_small.cuh"
 
 namespace b200moe {
 namespace {
 
-// Eight experts (= warps) per logits block. Fewer experts per block spread the logits over more CTAs but every CTA stages the
-// window's activation rows itself: measured on B200 at config 2, batch 8, 4 and 2 experts per block cost 80.6 and 92.5 us per
-// step against 76.2 us with 8 (no difference at batch 1).
-constexpr u32 kRunElems = 2048, kWarps = 8;
+constexpr u32 kRunElems = 2048, kGroupElems = 512, kBlockExperts = 4;
 
 __device__ __forceinline__ u32 smem_addr(const void* p) { return static_cast<u32>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ float4 widen4(uint2 b) {
+    return make_float4(__uint_as_float(b.x << 16), __uint_as_float(b.x & 0xffff0000u), __uint_as_float(b.y << 16), __uint_as_float(b.y & 0xffff0000u));
+}
 
 struct PrologueArgs {
     b200moe_router_view r;
     b200moe_quantize_a8_view q;
-    b200moe_routes_view routes;
-    u32 routes_end;
     u32 logit_blocks;
-    u32* ticket;  // zero before the first launch; the block that finishes last puts it back to zero
+    u32 x_vec, w_vec;  // rows in whole units of four values on their boundary
 };
 
-template <int RT>
-__global__ void __launch_bounds__(kWarps * 32) prologue_decode_kernel(PrologueArgs a) {
-    extern __shared__ __align__(16) float xs[];  // [rows + kWarps][kRunElems] while the logits run, select scratch afterwards
-    __shared__ u32 s_last;
+// A warp takes EW experts x RW rows of the block's 4 x RT.
+template <int RT, int EW, int RW>
+__global__ void __launch_bounds__(32 * (int(kBlockExperts) / EW) * (RT / RW)) prologue_decode_kernel(PrologueArgs a) {
+    constexpr u32 kWarps = (kBlockExperts / EW) * (RT / RW), kThreads = 32 * kWarps;
+    extern __shared__ __align__(16) float xs[];  // [RT rows | experts][kRunElems]
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const b200moe_quantize_a8_view& qv = a.q;
+    const u32 x_stride = qv.x_stride ? qv.x_stride : qv.width;
+    const bool bf16 = qv.x_is_bf16;
+    const u16* x16 = static_cast<const u16*>(qv.x);
+    const float* x32 = static_cast<const float*>(qv.x);
+    chain_begin();
 
     if (blockIdx.x >= a.logit_blocks) {  // ---- A8 quantiser: one warp per (row, 32-value group)
-        const b200moe_quantize_a8_view& qv = a.q;
         const u32 groups = qv.width / 32;
         const u64 item = u64(blockIdx.x - a.logit_blocks) * kWarps + warp;
         if (item >= u64(qv.rows) * groups) return;
-        const u32 r = static_cast<u32>(item / groups), g = static_cast<u32>(item % groups);
-        const u32 xst = qv.x_stride ? qv.x_stride : qv.width, st = qv.out.stride ? qv.out.stride : qv.width;
-        const float v = static_cast<const float*>(qv.x)[u64(r) * xst + 32u * g + lane];
+        const u32 r = static_cast<u32>(item / groups), g = static_cast<u32>(item % groups), st = qv.out.stride ? qv.out.stride : qv.width;
+        const u64 at = u64(r) * x_stride + 32u * g + lane;
+        const float v = bf16 ? __uint_as_float(static_cast<u32>(x16[at]) << 16) : x32[at];
         float delta;
         int sum;
         const int code = a8_quantize_lane(v, &delta, &sum);
@@ -59,104 +64,116 @@ __global__ void __launch_bounds__(kWarps * 32) prologue_decode_kernel(PrologueAr
         return;
     }
 
-    // ---- router logits: warp = expert
+    // ---- router logits
     const b200moe_router_view& rv = a.r;
     const u32 E = rv.policy.experts, H = rv.hidden, rows = rv.rows;
-    const u32 x_stride = rv.x_stride ? rv.x_stride : H;
-    const u32 e = blockIdx.x * kWarps + warp;
-    const float* wr = rv.weight + u64(min(e, E - 1)) * H;
-    const bool vec4 = (reinterpret_cast<uintptr_t>(rv.x) % 16 == 0) && x_stride % 4 == 0 && H % 4 == 0;
-    const bool wvec4 = (reinterpret_cast<uintptr_t>(rv.weight) % 16 == 0) && H % 4 == 0;
-    float* ws = xs + rows * kRunElems + warp * kRunElems;  // this warp's expert row run
-    float acc[RT];
+    const u32 e_base = blockIdx.x * kBlockExperts, e0 = EW * (warp % (kBlockExperts / EW)), r0 = RW * (warp / (kBlockExperts / EW));
+    float acc[EW][RW];
 #pragma unroll
-    for (int r = 0; r < RT; ++r) acc[r] = 0.0f;
-    // Both operands are staged with asynchronous copies from short rolled loops: every request of the run is in flight
-    // at once, and the code stays small (this kernel runs once per step on cold instruction caches, so straight-line
-    // unrolled code would pay a fetch miss per line).
+    for (int e = 0; e < EW; ++e)
+#pragma unroll
+        for (int r = 0; r < RW; ++r) acc[e][r] = 0.0f;
+    // The copies come from short rolled loops: every request of the run is in flight at once, and the code stays small (the kernel runs once a call on
+    // cold instruction caches, where straight-line code pays a fetch a line).
+    auto copy_row = [&](u32 row, const float* src, u32 n, bool vec) {  // n values to row `row`, all threads
+        const u32 dst = smem_addr(xs + row);
+        if (vec) {
+            for (u32 i = threadIdx.x; i < n / 4; i += kThreads) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(src + 4u * i) : "memory");
+        } else {
+            for (u32 i = threadIdx.x; i < n; i += kThreads) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * i), "l"(src + i) : "memory");
+        }
+    };
     for (u32 c0 = 0; c0 < H; c0 += kRunElems) {
         const u32 n_el = min(kRunElems, H - c0);
-        __syncthreads();  // the previous run has been consumed
-        {
-            const float* src = wr + c0;
-            const u32 dst = smem_addr(ws);
-            if (wvec4) {
-                for (u32 i = lane; i < n_el / 4; i += 32)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(src + 4u * i) : "memory");
-            } else {
-                for (u32 i = lane; i < n_el; i += 32)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * i), "l"(src + i) : "memory");
+        if (c0) __syncthreads();  // the previous run has been consumed
+#pragma unroll 1
+        for (u32 g0 = 0; g0 < kRunElems; g0 += kGroupElems) {
+            const u32 n = g0 < n_el ? min(kGroupElems, n_el - g0) : 0u;
+#pragma unroll 1
+            for (u32 e = 0; e < kBlockExperts; ++e) copy_row((RT + e) * kRunElems + g0, rv.weight + u64(min(e_base + e, E - 1)) * H + c0 + g0, n, a.w_vec);
+            if (!bf16) {
+#pragma unroll 1
+                for (u32 r = 0; r < rows; ++r) copy_row(r * kRunElems + g0, x32 + u64(r) * x_stride + c0 + g0, n, a.x_vec);
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        for (u32 r = 0; r < rows; ++r) {
-            const float* src = rv.x + u64(r) * x_stride + c0;
-            const u32 dst = smem_addr(xs + r * kRunElems);
-            if (vec4) {  // rows, strides and run starts are all multiples of four floats
-                for (u32 i = threadIdx.x; i < n_el / 4; i += kWarps * 32)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(src + 4u * i) : "memory");
-            } else {
-                for (u32 i = threadIdx.x; i < n_el; i += kWarps * 32)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * i), "l"(src + i) : "memory");
-            }
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
+        if (bf16) {
+#pragma unroll 1
+            for (u32 r = 0; r < rows; ++r) {
+                const u16* src = x16 + u64(r) * x_stride + c0;
+                float* dst = xs + r * kRunElems;
+                if (a.x_vec) {
 #pragma unroll 4
-        for (u32 i = lane; i < n_el; i += 32) {  // the lane class in ascending order (src/ds41_moe.cpp:72-82)
-            const float w = ws[i];
+                    for (u32 i = threadIdx.x; i < n_el / 4; i += kThreads) reinterpret_cast<float4*>(dst)[i] = widen4(reinterpret_cast<const uint2*>(src)[i]);
+                } else {
+                    for (u32 i = threadIdx.x; i < n_el; i += kThreads) dst[i] = __uint_as_float(static_cast<u32>(src[i]) << 16);
+                }
+            }
+        }
+#pragma unroll 1
+        for (u32 g0 = 0; g0 < n_el; g0 += kGroupElems) {
+            switch (g0 / kGroupElems) {
+                case 0: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+                case 1: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+                case 2: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+                default: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+            }
+            __syncthreads();
+            const u32 g1 = min(g0 + kGroupElems, n_el);
+            const float *ws = xs + (RT + e0) * kRunElems, *xr = xs + r0 * kRunElems;
+#pragma unroll 8
+            for (u32 i = g0 + lane; i < g1; i += 32) {  // the lane class in ascending order (src/ds41_moe.cpp:72-82)
+                float w[EW], x[RW];
 #pragma unroll
-            for (int r = 0; r < RT; ++r)
-                if (r < (int)rows) acc[r] = __fadd_rn(acc[r], __fmul_rn(w, xs[r * kRunElems + i]));
+                for (int e = 0; e < EW; ++e) w[e] = ws[e * kRunElems + i];
+#pragma unroll
+                for (int r = 0; r < RW; ++r) x[r] = xr[r * kRunElems + i];
+#pragma unroll
+                for (int e = 0; e < EW; ++e)
+#pragma unroll
+                    for (int r = 0; r < RW; ++r) acc[e][r] = __fadd_rn(acc[e][r], __fmul_rn(w[e], x[r]));
+            }
         }
     }
 #pragma unroll
-    for (int r = 0; r < RT; ++r) {
-        float z = butterfly32(acc[r]);
-        if (lane == 0 && r < (int)rows && e < E) {
-            if (rv.logit_bias) z = __fadd_rn(z, rv.logit_bias[e]);
-            rv.logits[u64(r) * E + e] = z;
+    for (int e = 0; e < EW; ++e)
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            float z = butterfly32(acc[e][r]);
+            const u32 ex = e_base + e0 + e, row = r0 + r;
+            if (lane == 0 && row < rows && ex < E) {
+                if (rv.logit_bias) z = __fadd_rn(z, rv.logit_bias[ex]);
+                rv.logits[u64(row) * E + ex] = z;
+            }
         }
-    }
-
-    // ---- the last block to finish selects and builds the routes
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(a.ticket, 1u) == a.logit_blocks - 1) ? 1u : 0u;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x == 0) *a.ticket = 0;  // every block has taken its ticket: ready for the next launch without a memset
-    for (u32 row = warp; row < rows; row += kWarps)
-        select_detail::select_row(rv.logits, rv.scores, rv.bias, rv.policy, row, lane, xs + warp * (2u * E + 32u), rv.ids, rv.weights);
-    __syncthreads();  // the ids written above are read below by the whole block
-    // At most 8 rows x 32 slots: the form for up to 256 slots, without the code, the stack and 12 KiB of shared arrays of the larger
-    // one (no difference in the time of a call beyond noise). Optional: a caller that routes elsewhere passes no outputs.
-    if (a.routes.out.experts) routes_detail::routes_tiny_body(a.routes, a.routes_end);
 }
 
 }  // namespace
 
 bool prologue_fusable(const b200moe_router_view& r, u32 top_k) {
-    return r.rows >= 1 && r.rows <= 8 && u64(r.rows) * top_k <= 256u && kWarps * (2u * r.policy.experts + 32u) * 4u <= 64u * 1024u;
+    return r.rows >= 1 && r.rows <= 8 && u64(r.rows) * top_k <= 256u && r.rows * select_detail::scratch_floats(r.policy.experts) * 4u <= 64u * 1024u;
 }
 
-int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view& q, const b200moe_routes_view& routes, u32* ticket,
-                    cudaStream_t stream) {
+int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view& q, cudaStream_t stream) {
     PrologueArgs a{};
-    a.r = r; a.q = q; a.routes = routes; a.routes_end = routes.end ? routes.end : routes.experts; a.ticket = ticket;
-    a.logit_blocks = (r.policy.experts + kWarps - 1) / kWarps;
-    const u32 quant_blocks = static_cast<u32>((u64(q.rows) * (q.width / 32) + kWarps - 1) / kWarps);
-    const u32 smem = std::max<u32>((r.rows + kWarps) * kRunElems * 4u, kWarps * (2u * r.policy.experts + 32u) * 4u);
-    const dim3 grid(a.logit_blocks + quant_blocks);
-#define B200_PRO(RT)                                                                                            \
-    {                                                                                                           \
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(prologue_decode_kernel<RT>), smem)) return rc; \
-        if (int rc = prefer_max_shared(reinterpret_cast<const void*>(prologue_decode_kernel<RT>))) return rc;       \
-        prologue_decode_kernel<RT><<<grid, kWarps * 32, smem, stream>>>(a);                                     \
+    a.r = r; a.q = q;
+    a.logit_blocks = (r.policy.experts + kBlockExperts - 1) / kBlockExperts;
+    const u32 xs = q.x_stride ? q.x_stride : q.width;
+    a.x_vec = aligned(q.x, q.x_is_bf16 ? 8 : 16) && xs % 4 == 0 && r.hidden % 4 == 0;
+    a.w_vec = aligned(r.weight, 16) && r.hidden % 4 == 0;
+    const u64 items = u64(q.rows) * (q.width / 32);
+#define B200_PRO(RT, EW, RW)                                                                                         \
+    {                                                                                                                \
+        constexpr u32 warps = (kBlockExperts / EW) * (RT / RW), smem = (RT + kBlockExperts) * kRunElems * 4u;        \
+        const auto kernel = prologue_decode_kernel<RT, EW, RW>;                                                      \
+        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;                    \
+        if (int rc = prefer_max_shared(reinterpret_cast<const void*>(kernel))) return rc;                            \
+        chain_launch(kernel, a.logit_blocks + static_cast<u32>((items + warps - 1) / warps), 32 * warps, smem, stream, a); \
     }
-    if (r.rows <= 2) B200_PRO(2)
-    else if (r.rows <= 4) B200_PRO(4)
-    else B200_PRO(8)
+    if (r.rows == 1) B200_PRO(1, 1, 1)
+    else if (r.rows == 2) B200_PRO(2, 1, 2)
+    else if (r.rows <= 4) B200_PRO(4, 1, 2)
+    else B200_PRO(8, 2, 2)
 #undef B200_PRO
     return after_launch("prologue_decode");
 }

@@ -16,9 +16,10 @@ namespace {
 
 // One warp computes an RT x ET tile of logits over the whole hidden width; lane = lane class.
 template <int RT, int ET>
-__global__ void __launch_bounds__(128) router_logits_kernel(const float* __restrict__ x, u32 x_stride, u32 rows, u32 hidden,
-                                                            const float* __restrict__ w, u32 experts,
-                                                            const float* __restrict__ logit_bias, float* __restrict__ logits) {
+__global__ void __launch_bounds__(128) router_logits_kernel(const float* x, u32 x_stride, u32 rows, u32 hidden,
+                                                            const float* w, u32 experts,
+                                                            const float* logit_bias, float* logits) {
+    chain_begin();
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const u32 e0 = (blockIdx.x * 4u + warp) * ET, r0 = blockIdx.y * RT;
     if (e0 >= experts) return;
@@ -39,7 +40,7 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const float* __restr
 #pragma unroll
         for (int r = 0; r < RT; ++r) xv[r] = xr[r][i];
 #pragma unroll
-        for (int e = 0; e < ET; ++e) wv[e] = __ldg(wr[e] + i);
+        for (int e = 0; e < ET; ++e) wv[e] = load(wr[e] + i);
 #pragma unroll
         for (int r = 0; r < RT; ++r)
 #pragma unroll
@@ -67,8 +68,9 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // Two experts a CTA spread a window over as many SMs as it has.
 constexpr u32 kFewRun = 2048, kFewWarps = 2;
 template <int RT>
-__global__ void __launch_bounds__(kFewWarps * 32) router_logits_few_kernel(const float* __restrict__ x, u32 x_stride, u32 rows, u32 hidden, const float* __restrict__ w,
-                                                                          u32 experts, const float* __restrict__ logit_bias, float* __restrict__ logits) {
+__global__ void __launch_bounds__(kFewWarps * 32) router_logits_few_kernel(const float* x, u32 x_stride, u32 rows, u32 hidden, const float* w,
+                                                                          u32 experts, const float* logit_bias, float* logits) {
+    chain_begin();
     extern __shared__ __align__(16) float few_smem[];  // [RT rows | kFewWarps experts][kFewRun]
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, e0 = blockIdx.x * kFewWarps, e = e0 + warp;
     float acc[RT];
@@ -113,9 +115,10 @@ constexpr u32 kTileRows = 8, kTileExperts = 16, kTileStages = 3;
 constexpr u32 tile_smem_bytes(u32 cols) { return kTileStages * (kTileRows + kTileExperts) * cols * 4u; }
 
 template <u32 kTileCols>
-__global__ void __launch_bounds__(128) router_logits_tile_kernel(const float* __restrict__ x, u32 x_stride, u32 rows, u32 hidden,
-                                                                 const float* __restrict__ w, u32 experts,
-                                                                 const float* __restrict__ logit_bias, float* __restrict__ logits) {
+__global__ void __launch_bounds__(128) router_logits_tile_kernel(const float* x, u32 x_stride, u32 rows, u32 hidden,
+                                                                 const float* w, u32 experts,
+                                                                 const float* logit_bias, float* logits) {
+    chain_begin();
     extern __shared__ __align__(16) float tile_smem[];
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     constexpr u32 ET = kTileExperts / 4, kTileStageFloats = (kTileRows + kTileExperts) * kTileCols;
@@ -189,14 +192,15 @@ namespace b200moe {
 namespace {
 
 // One warp per row; shared memory per warp: scores[experts] + choice[experts] + 32 group scores.
-__global__ void __launch_bounds__(128) router_select_kernel(const float* logits, float* scores_out, const float* __restrict__ bias,
-                                                            b200moe_route_policy p, u32 rows, u32* __restrict__ ids,
-                                                            float* __restrict__ weights) {
-    extern __shared__ float smem[];
+__global__ void __launch_bounds__(128) router_select_kernel(const float* logits, float* scores_out, const float* bias,
+                                                            b200moe_route_policy p, u32 rows, u32* ids,
+                                                            float* weights) {
+    chain_begin();
+    extern __shared__ __align__(16) float smem[];
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const u32 row = blockIdx.x * 4u + warp;
     if (row >= rows) return;
-    select_detail::select_row(logits, scores_out, bias, p, row, lane, smem + warp * (2u * p.experts + 32u), ids, weights);
+    select_detail::select_row(logits, scores_out, bias, p, row, lane, smem + warp * select_detail::scratch_floats(p.experts), ids, weights);
 }
 
 }  // namespace
@@ -206,19 +210,18 @@ int launch_router_logits(const b200moe_router_view& v, cudaStream_t stream, cons
     if (v.rows == 0) return B200MOE_OK;
     if (fused_quantize) if (int rc = launch_quantize_a8(*fused_quantize, stream)) return rc;
 #define B200_LOGITS(RT, ET)                                                                                   \
-    router_logits_kernel<RT, ET><<<dim3((E + 4 * ET - 1) / (4 * ET), (v.rows + RT - 1) / RT), 128, 0, stream>>>( \
-        v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits)
+    chain_launch(router_logits_kernel<RT, ET>, dim3((E + 4 * ET - 1) / (4 * ET), (v.rows + RT - 1) / RT), 128, 0, stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits)
     const bool vec = aligned(v.x, 16) && aligned(v.weight, 16) && xs % 4 == 0 && v.hidden % 4 == 0;  // whole 16-byte units for the staged forms
 #define B200_FEW(RT)                                                                                                                  \
     {                                                                                                                                 \
         constexpr u32 smem = (RT + kFewWarps) * kFewRun * sizeof(float);                                                              \
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(router_logits_few_kernel<RT>), smem)) return rc;               \
-        router_logits_few_kernel<RT><<<(E + kFewWarps - 1) / kFewWarps, kFewWarps * 32, smem, stream>>>(v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
+        chain_launch(router_logits_few_kernel<RT>, (E + kFewWarps - 1) / kFewWarps, kFewWarps * 32, smem, stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
     }
 #define B200_TILE(COLS)                                                                                                               \
     {                                                                                                                                 \
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(router_logits_tile_kernel<COLS>), tile_smem_bytes(COLS))) return rc; \
-        router_logits_tile_kernel<COLS><<<grid, 128, tile_smem_bytes(COLS), stream>>>(v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
+        chain_launch(router_logits_tile_kernel<COLS>, grid, 128, tile_smem_bytes(COLS), stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
     }
     if (v.rows <= 4 && vec) {
         if (v.rows == 1) B200_FEW(1)
@@ -241,8 +244,8 @@ int launch_router_logits(const b200moe_router_view& v, cudaStream_t stream, cons
 
 int launch_router_select(const b200moe_router_view& v, cudaStream_t stream) {
     if (v.rows == 0) return B200MOE_OK;
-    const u32 smem = 4u * (2u * v.policy.experts + 32u) * sizeof(float);
-    router_select_kernel<<<(v.rows + 3) / 4, 128, smem, stream>>>(v.logits, v.scores, v.bias, v.policy, v.rows, v.ids, v.weights);
+    const u32 smem = 4u * select_detail::scratch_floats(v.policy.experts) * sizeof(float);
+    chain_launch(router_select_kernel, (v.rows + 3) / 4, 128, smem, stream, v.logits, v.scores, v.bias, v.policy, v.rows, v.ids, v.weights);
     return after_launch("router_select");
 }
 

@@ -66,106 +66,151 @@ __device__ __forceinline__ u32 k_pass(u32 key, const float* c, u32 n, u32 lane, 
     return pick;
 }
 
-// Warp arg-max of (value, id) pairs under the order of beats(); kNone = no candidate. Rolled: these selections run once
-// per step in one warp per row on cold instruction caches, where a fetched line costs more than the instructions in it.
-__device__ __forceinline__ void warp_best(u32 key, u32& pick, float& best) {
-#pragma unroll 1
-    for (int d = 16; d; d >>= 1) {
-        const u32 op = __shfl_xor_sync(0xffffffffu, pick, d);
-        const float ob = __shfl_xor_sync(0xffffffffu, best, d);
-        if (op != kNone && (pick == kNone || beats(key, ob, op, best, pick))) { pick = op; best = ob; }
-    }
-}
+// The value whose key it is (a zero's sign is gone).
+__device__ __forceinline__ float key_value(u32 k) { return __uint_as_float((k & 0x80000000u) ? k & 0x7fffffffu : ~k); }
 
-// Fast path of one row, one warp: the row's choices live in registers (EPL per lane), no group limit, and no NaN among
-// the choices (then the serial scan of the contract is plain "largest choice, lowest id on ties", so a warp arg-max
-// per pass gives the same picks). Returns false - having written nothing - when the row needs the general path.
-// `s` = this warp's scratch of at least `experts` floats (shared memory).
+// Fast path of one row, one warp: the row's choices live in registers (EPL per lane, expert lane + 32 j) as ordered keys, none of them a NaN:
+// the contract's serial scans are then "largest choice, lowest id on ties" under either key rule, which two warp reductions a pass give (the
+// largest key, then the lowest id that has it; 0 is no candidate's key). Groups are runs of 2^i lanes or whole runs of 32 experts: a group's two
+// best are merged by shuffles or reductions. Returns false - with nothing stored - when the row needs the general path. `s` = this warp's
+// scratch of at least `experts` floats on a 16-byte boundary (shared memory); holds the scores afterwards.
+// The work is a chain of latencies in one warp, mostly run once a call on cold instruction caches, so the long steps (exp, quotient) are
+// rolled loops of four values a lane: 8 rows of 128 took 12,800 clocks with a shuffle tree a pass and everything unrolled.
 template <int EPL>
-__device__ __forceinline__ bool select_row_fast(const float* logits, float* scores_out, const float* __restrict__ bias,
-                                                const b200moe_route_policy& p, u32 row, u32 lane, float* s,
-                                                u32* __restrict__ ids, float* __restrict__ weights) {
-    const u32 E = p.experts;
+__device__ __forceinline__ bool select_row_fast(const float* logits, float* scores_out, const float* bias, const b200moe_route_policy& p, u32 row, u32 lane, float* s, u32* picked) {
+    const u32 E = p.experts, per = E / p.n_group;
     const float* z = logits + u64(row) * E;
-    float sc[EPL], c[EPL];
     const float ninf = -__uint_as_float(0x7f800000u);
-    if (p.score == B200MOE_SCORE_SOFTMAX) {  // route_policy.hpp:135-144
-        float zz[EPL];
-        float m = ninf;
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) { const u32 e = lane + 32u * j; zz[j] = e < E ? z[e] : ninf; m = zz[j] > m ? zz[j] : m; }
-#pragma unroll
-        for (int d = 16; d; d >>= 1) { const float o = __shfl_xor_sync(0xffffffffu, m, d); m = o > m ? o : m; }
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) { const u32 e = lane + 32u * j; sc[j] = declared_exp(__fsub_rn(zz[j], m)); if (e < E) s[e] = sc[j]; }
-        __syncwarp();
-        float sum = 0.0f;
-#pragma unroll 8
-        for (u32 e = 0; e < E; ++e) sum = __fadd_rn(sum, s[e]);  // ascending serial sum (the declared order), every lane alike
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) sc[j] = __fdiv_rn(sc[j], sum);
-        __syncwarp();
-    } else {
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) {
-            const u32 e = lane + 32u * j;
-            const float zj = e < E ? z[e] : 0.0f;
-            sc[j] = p.score == B200MOE_SCORE_SIGMOID ? sigmoid_score(zj) : sqrt_softplus_score(zj);
-        }
-    }
-    bool has_nan = false;
+    float m = ninf;
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {
         const u32 e = lane + 32u * j;
-        c[j] = (p.selection_bias && e < E) ? __fadd_rn(sc[j], bias[e]) : sc[j];
-        has_nan |= e < E && c[j] != c[j];
+        if (e < E) { const float v = z[e]; s[e] = v; m = v > m ? v : m; }
     }
-    if (__any_sync(0xffffffffu, has_nan)) return false;
+    if (p.score == B200MOE_SCORE_SOFTMAX) {  // route_policy.hpp:135-144
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) { const u32 e = lane + 32u * j; if (e < E) s[e] = sc[j]; }  // scores for the weight step
-    if (scores_out) {
+        for (int d = 16; d; d >>= 1) { const float o = __shfl_xor_sync(0xffffffffu, m, d); m = o > m ? o : m; }
+#pragma unroll 1
+        for (u32 e0 = lane; e0 < E; e0 += 128) {
+            float v[4];
 #pragma unroll
-        for (int j = 0; j < EPL; ++j) { const u32 e = lane + 32u * j; if (e < E) scores_out[u64(row) * E + e] = sc[j]; }
+            for (u32 i = 0; i < 4; ++i) v[i] = e0 + 32u * i < E ? s[e0 + 32u * i] : ninf;
+#pragma unroll
+            for (u32 i = 0; i < 4; ++i) v[i] = declared_exp(__fsub_rn(v[i], m));
+#pragma unroll
+            for (u32 i = 0; i < 4; ++i) if (e0 + 32u * i < E) s[e0 + 32u * i] = v[i];
+        }
+        __syncwarp();
+        float sum = 0.0f;  // ascending serial sum (the declared order), every lane alike
+#pragma unroll 4
+        for (u32 e = 0; e + 4 <= E; e += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(s + e);
+            sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
+        }
+        for (u32 e = E & ~3u; e < E; ++e) sum = __fadd_rn(sum, s[e]);
+        __syncwarp();
+#pragma unroll 1
+        for (u32 e0 = lane; e0 < E; e0 += 128)
+#pragma unroll
+            for (u32 i = 0; i < 4; ++i) if (e0 + 32u * i < E) s[e0 + 32u * i] = __fdiv_rn(s[e0 + 32u * i], sum);
+    } else {
+#pragma unroll 1
+        for (u32 e0 = lane; e0 < E; e0 += 128) {
+            float v[4];
+#pragma unroll
+            for (u32 i = 0; i < 4; ++i) v[i] = e0 + 32u * i < E ? s[e0 + 32u * i] : 0.0f;
+            if (p.score == B200MOE_SCORE_SIGMOID) {
+#pragma unroll
+                for (u32 i = 0; i < 4; ++i) v[i] = sigmoid_score(v[i]);
+            } else {
+#pragma unroll
+                for (u32 i = 0; i < 4; ++i) v[i] = sqrt_softplus_score(v[i]);
+            }
+#pragma unroll
+            for (u32 i = 0; i < 4; ++i) if (e0 + 32u * i < E) s[e0 + 32u * i] = v[i];
+        }
     }
-    __syncwarp();
-    u32 taken = 0, my_id = kNone;
-    for (u32 k = 0; k < p.top_k; ++k) {
-        u32 pick = kNone;
-        float best = 0.0f;
+    u32 key[EPL];  // a lane reads the scores that it wrote itself
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) {
+        const u32 e = lane + 32u * j;
+        float c = 0.0f;
+        if (e < E) c = p.selection_bias ? __fadd_rn(s[e], bias[e]) : s[e];
+        bad |= c != c;
+        key[j] = e < E ? ordered_key(c) : 0u;
+    }
+    if (__any_sync(0xffffffffu, bad)) return false;
+    if (p.n_group > 1) {
+        u32 b0 = 0, b1 = 0;  // lane g: the two best of group g
+        const u32 runs = per >> 5, shift = 31u - __clz(per);
+        if (runs) {
+            u32 g = 0, i = 0;
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) {
+                const u32 m0 = __reduce_max_sync(0xffffffffu, key[j]);
+                const u32 first = __ffs(__ballot_sync(0xffffffffu, key[j] == m0)) - 1u;
+                const u32 m1 = __reduce_max_sync(0xffffffffu, lane == first ? 0u : key[j]);
+                if (lane == g) { b1 = max(min(b0, m0), max(b1, m1)); b0 = max(b0, m0); }
+                if (++i == runs) { i = 0; ++g; }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) {
+                u32 t0 = key[j], t1 = 0;
+#pragma unroll 1
+                for (u32 d = per >> 1; d; d >>= 1) {
+                    const u32 o0 = __shfl_xor_sync(0xffffffffu, t0, d), o1 = __shfl_xor_sync(0xffffffffu, t1, d);
+                    t1 = max(min(t0, o0), max(t1, o1));
+                    t0 = max(t0, o0);
+                }
+                const u32 at = lane << shift, g0 = __shfl_sync(0xffffffffu, t0, at & 31u), g1 = __shfl_sync(0xffffffffu, t1, at & 31u);
+                if ((at >> 5) == (u32)j) { b0 = g0; b1 = g1; }
+            }
+        }
+        const bool mine = lane < p.n_group;
+        const float score = mine ? __fadd_rn(key_value(b0), key_value(b1)) : 0.0f;
+        if (__any_sync(0xffffffffu, score != score)) return false;
+        u32 gkey = mine ? ordered_key(score) : 0u, gmask = 0;
+#pragma unroll 1
+        for (u32 k = 0; k < p.topk_group; ++k) {
+            const u32 best = __reduce_max_sync(0xffffffffu, gkey), at = __ffs(__ballot_sync(0xffffffffu, gkey == best)) - 1u;
+            gmask |= 1u << at;
+            if (lane == at) gkey = 0u;
+        }
+        u32 g = 0, i = 0;
 #pragma unroll
         for (int j = 0; j < EPL; ++j) {
-            const u32 e = lane + 32u * j;
-            if (e < E && !((taken >> j) & 1u) && (pick == kNone || beats(p.key, c[j], e, best, pick))) { pick = e; best = c[j]; }
+            const u32 group = runs ? g : (lane + 32u * j) >> shift;
+            if (!((gmask >> (group & 31u)) & 1u)) key[j] = 0u;
+            if (++i == runs) { i = 0; ++g; }
         }
-        warp_best(p.key, pick, best);
-        if (pick != kNone && (pick & 31u) == lane) taken |= 1u << (pick >> 5);
-        if (lane == k) my_id = pick;
     }
-    if (p.order == B200MOE_ORDER_ASCENDING_ID) {
-        u32 rank = 0;
-        for (u32 k = 0; k < p.top_k; ++k) { const u32 o = __shfl_sync(0xffffffffu, my_id, k); rank += (o < my_id) ? 1u : 0u; }
-        u32 sorted = kNone;
-        for (u32 k = 0; k < p.top_k; ++k) {
-            const u32 o = __shfl_sync(0xffffffffu, my_id, k), orank = __shfl_sync(0xffffffffu, rank, k);
-            if (orank == lane) sorted = o;
-        }
-        my_id = sorted;
+    if (scores_out) for (u32 e = lane; e < E; e += 32) scores_out[u64(row) * E + e] = s[e];
+    __syncwarp();
+    u32 my_id = kNone;
+#pragma unroll 1
+    for (u32 k = 0; k < p.top_k; ++k) {
+        u32 top = 0;
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) top = max(top, key[j]);
+        const u32 best = __reduce_max_sync(0xffffffffu, top);
+        u32 id = kNone;
+#pragma unroll
+        for (int j = EPL - 1; j >= 0; --j) if (key[j] == best) id = lane + 32u * j;
+        id = best ? __reduce_min_sync(0xffffffffu, id) : kNone;
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) if (lane + 32u * j == id) key[j] = 0u;
+        if (lane == k) my_id = id;
     }
-    const float my_s = (lane < p.top_k && my_id != kNone) ? s[my_id] : 0.0f;
-    float sum = 0.0f;  // ((0 + s0) + s1) + ... in output order (route_policy.hpp:121-123)
-    for (u32 k = 0; k < p.top_k; ++k) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, my_s, k));
-    const bool renorm = p.renormalize && (p.top_k > 1 || p.renorm_single);
-    const float den = __fadd_rn(sum, p.renorm_eps);
-    if (lane < p.top_k) {
-        ids[u64(row) * p.top_k + lane] = my_id;
-        weights[u64(row) * p.top_k + lane] = __fmul_rn(renorm ? __fdiv_rn(my_s, den) : my_s, p.scale);
-    }
+    *picked = my_id;
     return true;
 }
 
 // Output order, weights and the stores of one row; lane k holds pick k in `my_id`, s[] the scores.
+// ids_copy: the row's ids once more (shared memory), for a block that goes on with them.
 __device__ __forceinline__ void finish_row(const b200moe_route_policy& p, u32 row, u32 lane, const float* s, u32 my_id,
-                                        u32* __restrict__ ids, float* __restrict__ weights) {
+                                        u32* ids, float* weights, u32* ids_copy) {
     if (p.order == B200MOE_ORDER_ASCENDING_ID) {  // rank sort of the (distinct) ids held one per lane
         u32 rank = 0;
         for (u32 k = 0; k < p.top_k; ++k) { const u32 o = __shfl_sync(0xffffffffu, my_id, k); rank += (o < my_id) ? 1u : 0u; }
@@ -183,19 +228,27 @@ __device__ __forceinline__ void finish_row(const b200moe_route_policy& p, u32 ro
     const float den = __fadd_rn(sum, p.renorm_eps);
     if (lane < p.top_k) {
         ids[u64(row) * p.top_k + lane] = my_id;
+        if (ids_copy) ids_copy[row * p.top_k + lane] = my_id;
         weights[u64(row) * p.top_k + lane] = __fmul_rn(renorm ? __fdiv_rn(my_s, den) : my_s, p.scale);
     }
 }
 
-// One warp selects one row. `s` points to this warp's scratch of 2 * experts + 32 floats (shared memory).
-__device__ __forceinline__ void select_row(const float* logits, float* scores_out, const float* __restrict__ bias,
+// One warp selects one row. `s` points to this warp's scratch of 2 * experts + 32 floats on a 16-byte boundary (shared memory).
+__host__ __device__ constexpr u32 scratch_floats(u32 experts) { return (2u * experts + 32u + 3u) & ~3u; }
+__device__ __forceinline__ void select_row(const float* logits, float* scores_out, const float* bias,
                                            const b200moe_route_policy& p, u32 row, u32 lane, float* s,
-                                           u32* __restrict__ ids, float* __restrict__ weights) {
-    const u32 E = p.experts;
-    if (p.n_group == 1 && E <= 256) {  // registers hold the row: the fast path unless a NaN choice needs the serial rule
-        const bool done = E <= 128 ? select_row_fast<4>(logits, scores_out, bias, p, row, lane, s, ids, weights)
-                                   : select_row_fast<8>(logits, scores_out, bias, p, row, lane, s, ids, weights);
-        if (done) return;
+                                           u32* ids, float* weights, u32* ids_copy = nullptr) {
+    const u32 E = p.experts, run = E / p.n_group;
+    if (p.n_group == 1 || run % 32 == 0 || (run < 32 && (run & (run - 1u)) == 0)) {  // the fast path unless a NaN needs the serial rule
+        u32 my_id = kNone;
+        const bool done = E <= 128 ? select_row_fast<4>(logits, scores_out, bias, p, row, lane, s, &my_id)
+                        : E <= 256 ? select_row_fast<8>(logits, scores_out, bias, p, row, lane, s, &my_id)
+                                   : select_row_fast<32>(logits, scores_out, bias, p, row, lane, s, &my_id);
+        if (done) {
+            finish_row(p, row, lane, s, my_id, ids, weights, ids_copy);
+            return;
+        }
+        __syncwarp();
     }
     float* c = s + E;
     float* gs = c + E;
@@ -222,65 +275,6 @@ __device__ __forceinline__ void select_row(const float* logits, float* scores_ou
     if (scores_out) for (u32 e = lane; e < E; e += 32) scores_out[u64(row) * E + e] = s[e];
 
     u32 allowed = 0xffffffffu, per = E;
-    if (p.n_group > 1 && (E / p.n_group) % 32 == 0 && p.n_group <= 32) {
-        // Groups of whole 32-expert runs and no NaN among the choices: every serial scan of the contract is then "largest
-        // choice, lowest id on ties", which a warp arg-max reproduces; bit j of `live` = this lane's candidate lane + 32 j
-        // is still to be had. Short rolled loops over shared memory keep the code small (see warp_best).
-        per = E / p.n_group;
-        bool bad = false;
-        for (u32 e = lane; e < E; e += 32) bad |= c[e] != c[e];
-        float my_gs = 0.0f;
-        if (!__any_sync(0xffffffffu, bad)) {
-#pragma unroll 1
-            for (u32 g = 0; g < p.n_group; ++g) {
-                u32 i0 = kNone, i1 = kNone;
-                float b0 = 0.0f, b1 = 0.0f;
-#pragma unroll 1
-                for (u32 e = g * per + lane; e < (g + 1) * per; e += 32) { const float v = c[e]; if (i0 == kNone || beats(p.key, v, e, b0, i0)) { i0 = e; b0 = v; } }
-                warp_best(p.key, i0, b0);
-#pragma unroll 1
-                for (u32 e = g * per + lane; e < (g + 1) * per; e += 32) { const float v = c[e]; if (e != i0 && (i1 == kNone || beats(p.key, v, e, b1, i1))) { i1 = e; b1 = v; } }
-                warp_best(p.key, i1, b1);
-                const float v = __fadd_rn(b0, b1);
-                bad |= v != v;
-                if (lane == g) my_gs = v;
-            }
-        }
-        if (!__any_sync(0xffffffffu, bad)) {
-            u32 gmask = 0;
-#pragma unroll 1
-            for (u32 k = 0; k < p.topk_group; ++k) {
-                u32 pick = (lane < p.n_group && !((gmask >> lane) & 1u)) ? lane : kNone;
-                float best = my_gs;
-                warp_best(p.key, pick, best);
-                if (pick != kNone) gmask |= 1u << pick;
-            }
-            const u32 m = per >> 5;
-            u32 live = 0;
-            for (u32 j = 0, g = 0, i = 0; lane + 32u * j < E; ++j) {  // register j belongs to group j / m
-                if ((gmask >> g) & 1u) live |= 1u << j;
-                if (++i == m) { i = 0; ++g; }
-            }
-            u32 my_id = kNone;
-#pragma unroll 1
-            for (u32 k = 0; k < p.top_k; ++k) {
-                u32 pick = kNone;
-                float best = 0.0f;
-#pragma unroll 1
-                for (u32 rest = live; rest; rest &= rest - 1u) {
-                    const u32 e = lane + 32u * (__ffs(rest) - 1u);
-                    const float v = c[e];
-                    if (pick == kNone || beats(p.key, v, e, best, pick)) { pick = e; best = v; }
-                }
-                warp_best(p.key, pick, best);
-                if (pick != kNone && (pick & 31u) == lane) live &= ~(1u << (pick >> 5));
-                if (lane == k) my_id = pick;
-            }
-            finish_row(p, row, lane, s, my_id, ids, weights);
-            return;
-        }
-        per = E;  // a NaN: the serial rules below decide
-    }
     if (p.n_group > 1) {  // group-limited extension (include/b200moe.h): group score = its two best choices summed
         per = E / p.n_group;
         if (lane < p.n_group) {
@@ -304,7 +298,7 @@ __device__ __forceinline__ void select_row(const float* logits, float* scores_ou
         const u32 pick = k_pass(p.key, c, E, lane, taken, allowed, per);
         if (lane == k) my_id = pick;
     }
-    finish_row(p, row, lane, s, my_id, ids, weights);
+    finish_row(p, row, lane, s, my_id, ids, weights, ids_copy);
 }
 
 

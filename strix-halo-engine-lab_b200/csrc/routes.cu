@@ -8,6 +8,8 @@
 //
 // Two forms: up to 1024 slots (decode windows) one block does everything; above that three launches over chunks of
 // 1024 slots (per-chunk histograms, a scan over chunks and experts, then the stable fill).
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "router_select.cuh"
 #include "routes_small.cuh"
@@ -23,26 +25,36 @@ using routes_detail::kRankedTopK;
 using routes_detail::row_order;
 using routes_detail::routes_small_body;
 
-template <bool RANKED>
-__global__ void __launch_bounds__(1024) routes_small_kernel(b200moe_routes_view v, u32 end) { routes_small_body<RANKED>(v, end); }
+using routes_detail::Clear;
+using routes_detail::counts_bytes;
+
+__global__ void __launch_bounds__(1024) routes_small_kernel(b200moe_routes_view v, u32 end, Clear clear) {
+    extern __shared__ __align__(16) u16 counts[];
+    chain_begin();
+    routes_detail::clear_words(clear, v.rows);  // in front of the body's first barrier
+    routes_small_body(v, end, v.ids, counts);
+}
 
 // Decode windows: the router's selection (one warp per row) and the routes of the selected ids in ONE block, so the
-// layer prologue costs one launch less. Dynamic shared memory: rows * (2 * experts + 32) floats.
-template <bool RANKED>
-__global__ void __launch_bounds__(1024) select_routes_small_kernel(const float* logits, float* scores_out, const float* __restrict__ bias,
-                                                                   b200moe_route_policy p, u32 rows, u32* ids, float* __restrict__ weights,
-                                                                   b200moe_routes_view rv, u32 end) {
-    extern __shared__ float sel_smem[];
+// layer prologue costs one launch less. Dynamic shared memory: the rows' selection scratch, then the routes' counts in its place.
+__global__ void __launch_bounds__(1024) select_routes_small_kernel(const float* logits, float* scores_out, const float* bias,
+                                                                   b200moe_route_policy p, u32 rows, u32* ids, float* weights,
+                                                                   b200moe_routes_view rv, u32 end, Clear clear) {
+    extern __shared__ __align__(16) float sel_smem[];
+    __shared__ u32 s_ids[kChunk];
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    if (warp < rows) select_detail::select_row(logits, scores_out, bias, p, warp, lane, sel_smem + warp * (2u * p.experts + 32u), ids, weights);
-    __syncthreads();  // the ids written above are read below by the whole block
-    routes_small_body<RANKED>(rv, end);
+    chain_begin();
+    routes_detail::clear_words(clear, rows);
+    if (warp < rows) select_detail::select_row(logits, scores_out, bias, p, warp, lane, sel_smem + warp * select_detail::scratch_floats(p.experts), ids, weights, s_ids);
+    __syncthreads();  // the ids are read by the whole block
+    routes_small_body(rv, end, s_ids, reinterpret_cast<u16*>(sel_smem));
 }
 
 // ---- chunked form --------------------------------------------------------------------------------------------------
 // scratch: hist[chunks][experts], then ebegin[experts].
 template <bool RANKED>
-__global__ void __launch_bounds__(1024) routes_count_kernel(b200moe_routes_view v, u32 end, u32 chunks) {
+__global__ void __launch_bounds__(1024) routes_count_kernel(b200moe_routes_view v, u32 end, u32 chunks, Clear clear) {
+    chain_begin();
     __shared__ u32 cnt[1024];
     const u32 t = threadIdx.x, n = v.rows * v.top_k, s = blockIdx.x * kChunk + t;
     cnt[t] = 0;
@@ -50,16 +62,32 @@ __global__ void __launch_bounds__(1024) routes_count_kernel(b200moe_routes_view 
     if (s < n) { const u32 e = entry_id(v.ids, s, v.top_k, v.experts, v.first, end); if (e != 0xffffffffu) atomicAdd(&cnt[e], 1u); }
     __syncthreads();
     if (t < v.experts) v.scratch[u64(blockIdx.x) * v.experts + t] = cnt[t];
-    for (u32 r = blockIdx.x * blockDim.x + t; r < v.rows; r += gridDim.x * blockDim.x)
+    if (blockIdx.x == 0) {
+        if (clear.summary4 && t < 4) clear.summary4[t] = 0u;
+        if (clear.summary && t == 0) *clear.summary = 0u;
+    }
+    for (u32 r = blockIdx.x * blockDim.x + t; r < v.rows; r += gridDim.x * blockDim.x) {
+        if (clear.row_status) clear.row_status[r] = 0u;  // the row's status is this thread's alone in this launch
         row_order<RANKED>(v.ids, r, v.top_k, v.experts, v.split, v.out.order, v.out.low_counts, v.row_status);
+    }
 }
 __global__ void __launch_bounds__(1024) routes_scan_kernel(b200moe_routes_view v, u32 chunks) {
+    chain_begin();
     __shared__ u32 warp_tot[32], total_s, union_s, maxc;
     const u32 t = threadIdx.x;
     if (t == 0) maxc = 0;
     u32 c = 0;
     if (t < v.experts)
-        for (u32 k = 0; k < chunks; ++k) { u32* h = &v.scratch[u64(k) * v.experts + t]; const u32 x = *h; *h = c; c += x; }
+        for (u32 k0 = 0; k0 < chunks; k0 += 8) {  // eight chunks' counts asked for at once
+            u32 x[8];
+#pragma unroll
+            for (u32 k = 0; k < 8; ++k) x[k] = k0 + k < chunks ? v.scratch[u64(k0 + k) * v.experts + t] : 0u;
+#pragma unroll
+            for (u32 k = 0; k < 8; ++k) {
+                if (k0 + k < chunks) v.scratch[u64(k0 + k) * v.experts + t] = c;
+                c += x[k];
+            }
+        }
     __syncthreads();
     const u32 begin = block_exclusive_scan(c, warp_tot, &total_s);
     const u32 uidx = block_exclusive_scan(c ? 1u : 0u, warp_tot, &union_s);
@@ -72,16 +100,20 @@ __global__ void __launch_bounds__(1024) routes_scan_kernel(b200moe_routes_view v
     }
 }
 __global__ void __launch_bounds__(1024) routes_fill_kernel(b200moe_routes_view v, u32 end, u32 chunks) {
-    __shared__ u32 sid[1024];
+    extern __shared__ __align__(16) u16 counts[];  // [32][experts]
     const u32 t = threadIdx.x, n = v.rows * v.top_k, s = blockIdx.x * kChunk + t;
+    routes_detail::clear_counts(counts, 32, v.experts);
+    chain_begin();
     u32 e = 0xffffffffu;
     if (s < n) e = entry_id(v.ids, s, v.top_k, v.experts, v.first, end);
-    sid[t] = e;
+    const u32 base = e == 0xffffffffu ? 0u : v.scratch[u64(chunks) * v.experts + e] + v.scratch[u64(blockIdx.x) * v.experts + e];
+    __syncthreads();
+    const u32 peers = routes_detail::count_run(counts, t / 32u, v.experts, e);
+    __syncthreads();
+    if (t < v.experts) routes_detail::sum_runs(counts, 32, v.experts, t);
     __syncthreads();
     if (e == 0xffffffffu) return;
-    u32 rank = 0;
-    for (u32 i = 0; i < t; ++i) rank += sid[i] == e ? 1u : 0u;
-    const u32 pos = v.scratch[u64(chunks) * v.experts + e] + v.scratch[u64(blockIdx.x) * v.experts + e] + rank;
+    const u32 pos = base + routes_detail::rank_of(counts, t / 32u, v.experts, e, peers);
     v.out.rows[pos] = s / v.top_k;
     v.out.slots[pos] = s;
 }
@@ -91,6 +123,7 @@ __global__ void __launch_bounds__(1024) routes_fill_kernel(b200moe_routes_view v
 // the job's status words cleared in the same launch: what build_window_routes (src/ds41_moe.cpp:11-43) gives for ids = 0,
 // without the sort and without the memsets in front of it.
 __global__ void __launch_bounds__(256) dense_routes_kernel(b200moe_routes out, u32 rows, u32* row_status, u32* summary4) {
+    chain_begin();
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < rows) {
         out.rows[i] = i;
@@ -115,37 +148,43 @@ u64 routes_scratch_words(u32 rows, u32 top_k, u32 experts) {
     return (chunks + 1) * experts + 4;
 }
 
+u32 small_threads(u32 slots, u32 experts) { return std::min(1024u, std::max(256u, (std::max(slots, experts) + 31u) / 32u * 32u)); }
+
 bool select_routes_fusable(const b200moe_router_view& r, u32 top_k) {
-    return r.rows <= 32 && u64(r.rows) * top_k <= kChunk && u64(r.rows) * (2u * r.policy.experts + 32u) * 4u <= 96u * 1024u;
+    return r.rows <= 32 && u64(r.rows) * top_k <= kChunk && u64(r.rows) * select_detail::scratch_floats(r.policy.experts) * 4u <= 96u * 1024u;
 }
-int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view& v, cudaStream_t stream) {
+int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view& v, const RoutesClear& clear, cudaStream_t stream) {
     if (r.rows == 0) return B200MOE_OK;
-    const u32 smem = r.rows * (2u * r.policy.experts + 32u) * 4u;
-    const auto kernel = v.top_k <= kRankedTopK ? select_routes_small_kernel<true> : select_routes_small_kernel<false>;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-    kernel<<<1, 1024, smem, stream>>>(r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights, v, v.end ? v.end : v.experts);
+    const u32 n = v.rows * v.top_k, smem = std::max(r.rows * select_detail::scratch_floats(r.policy.experts) * 4u, counts_bytes(n, v.experts));
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(select_routes_small_kernel), smem)) return rc;
+    chain_launch(select_routes_small_kernel, 1, std::max(32u * r.rows, small_threads(n, v.experts)), smem, stream, r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights,
+                 v, v.end ? v.end : v.experts, Clear{clear.row_status, clear.summary4, clear.summary});
     return after_launch("select_routes_small");
 }
 
 int launch_dense_routes(const b200moe_routes& out, u32 rows, u32* row_status, u32* summary4, cudaStream_t stream) {
-    dense_routes_kernel<<<(rows + 255) / 256, 256, 0, stream>>>(out, rows, row_status, summary4);
+    chain_launch(dense_routes_kernel, (rows + 255) / 256, 256, 0, stream, out, rows, row_status, summary4);
     return after_launch("dense_routes");
 }
 
-int launch_routes(const b200moe_routes_view& v, cudaStream_t stream) {
+int launch_routes(const b200moe_routes_view& v, const RoutesClear& clear, cudaStream_t stream) {
     const u64 n = u64(v.rows) * v.top_k;
     if (n == 0) return B200MOE_OK;
     const u32 end = v.end ? v.end : v.experts;
+    const Clear c{clear.row_status, clear.summary4, clear.summary};
+    const u32 smem = counts_bytes(static_cast<u32>(std::min<u64>(n, kChunk)), v.experts);
     if (n <= kChunk) {
-        (v.top_k <= kRankedTopK ? routes_small_kernel<true> : routes_small_kernel<false>)<<<1, 1024, 0, stream>>>(v, end);
+        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(routes_small_kernel), smem)) return rc;
+        chain_launch(routes_small_kernel, 1, small_threads(static_cast<u32>(n), v.experts), smem, stream, v, end, c);
         return after_launch("routes_small");
     }
     const u32 chunks = static_cast<u32>((n + kChunk - 1) / kChunk);
-    (v.top_k <= kRankedTopK ? routes_count_kernel<true> : routes_count_kernel<false>)<<<chunks, 1024, 0, stream>>>(v, end, chunks);
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(routes_fill_kernel), smem)) return rc;
+    chain_launch((v.top_k <= kRankedTopK ? routes_count_kernel<true> : routes_count_kernel<false>), chunks, 1024, 0, stream, v, end, chunks, c);
     if (int rc = after_launch("routes_count")) return rc;
-    routes_scan_kernel<<<1, 1024, 0, stream>>>(v, chunks);
+    chain_launch(routes_scan_kernel, 1, 1024, 0, stream, v, chunks);
     if (int rc = after_launch("routes_scan")) return rc;
-    routes_fill_kernel<<<chunks, 1024, 0, stream>>>(v, end, chunks);
+    chain_launch(routes_fill_kernel, chunks, 1024, smem, stream, v, end, chunks);
     return after_launch("routes_fill");
 }
 

@@ -87,95 +87,91 @@ __device__ __forceinline__ bool owned(u32 e, u32 experts, u32 first, u32 end) { 
 __device__ __forceinline__ u32 entry_id(const u32* ids, u32 s, u32 top_k, u32 experts, u32 first, u32 end) {
     const u32 e = ids[s];
     if (!owned(e, experts, first, end)) return 0xffffffffu;
-    for (u32 i = s - s % top_k; i < s; ++i)
-        if (ids[i] == e) return 0xffffffffu;
-    return e;
+    bool repeats = false;
+    for (u32 i = s - s % top_k; i < s; ++i) repeats |= ids[i] == e;  // no early way out: the loads overlap
+    return repeats ? 0xffffffffu : e;
 }
 
-// Windows of up to 256 slots (decode): every slot's thread counts what it needs directly from the ids in shared memory
-// - O(slots) work per thread, three block barriers, no scans. Same outputs as the general body below.
-__device__ inline void routes_tiny_body(const b200moe_routes_view& v, u32 end) {
-    __shared__ u32 sid[256], srank[256], red[4];
-    const u32 t = threadIdx.x, nt = blockDim.x, n = v.rows * v.top_k, K = v.top_k;
-    if (t < 4) red[t] = 0;
-    for (u32 s = t; s < n; s += nt) {
-        sid[s] = entry_id(v.ids, s, K, v.experts, v.first, end);
-    }
-    __syncthreads();
-    for (u32 s = t; s < n; s += nt) {  // rank among the slots of the same expert (ascending slot = ascending row)
-        const u32 e = sid[s];
-        u32 rank = 0;
-        for (u32 i = 0; i < s; ++i) rank += sid[i] == e ? 1u : 0u;
-        srank[s] = rank;
-    }
-    __syncthreads();
-    for (u32 s = t; s < n; s += nt) {
-        const u32 e = sid[s];
-        // the row's order, low count and route check (every slot places itself)
-        {
-            const u32 row = s / K, raw = v.ids[s];
-            u32 pos = 0, low = 0;
-            bool bad = raw >= v.experts;
-            for (u32 k = 0; k < K; ++k) {
-                const u32 o = v.ids[row * K + k], so = row * K + k;
-                pos += (o < raw || (o == raw && so < s)) ? 1u : 0u;
-                bad |= (o == raw && so != s);
-                low += o < v.split ? 1u : 0u;
-            }
-            v.out.order[row * K + pos] = s;
-            if (s == row * K) v.out.low_counts[row] = low;
-            if (bad && v.row_status) atomicOr(&v.row_status[row], B200MOE_ROW_INVALID_ROUTE);
-        }
-        if (e == 0xffffffffu) continue;
-        u32 before = 0, uidx = 0, cnt = 0;
-        for (u32 i = 0; i < n; ++i) {
-            const u32 o = sid[i];
-            before += o < e ? 1u : 0u;                          // 0xffffffff (not owned) is never below e
-            uidx += (o < e && srank[i] == 0) ? 1u : 0u;
-            cnt += o == e ? 1u : 0u;
-        }
-        const u32 rank = srank[s], pos = before + rank;
-        v.out.rows[pos] = s / K;
-        v.out.slots[pos] = s;
-        if (rank == 0) {
-            v.out.experts[uidx] = e - v.base;
-            v.out.begins[uidx + 1] = before + cnt;
-            atomicAdd(&red[0], 1u);
-            atomicMax(&red[1], cnt);
-            atomicAdd(&red[2], cnt);
-        }
-    }
-    __syncthreads();
-    if (t == 0) {
-        v.out.begins[0] = 0;
-        v.out.counts[0] = red[0]; v.out.counts[1] = red[1]; v.out.counts[2] = red[2]; v.out.counts[3] = 0;
-    }
+// What the first launch of a call that owns its status words clears on the way (all optional).
+struct Clear {
+    u32* row_status;  // rows words
+    u32* summary4;    // 4 words
+    u32* summary;     // 1 word
+};
+__device__ __forceinline__ void clear_words(const Clear& c, u32 rows) {
+    if (c.row_status) for (u32 r = threadIdx.x; r < rows; r += blockDim.x) c.row_status[r] = 0u;
+    if (c.summary4 && threadIdx.x < 4) c.summary4[threadIdx.x] = 0u;
+    if (c.summary && threadIdx.x == 0) *c.summary = 0u;
 }
 
-// The whole build by one block. Each thread owns a contiguous run of experts for the scans.
-template <bool RANKED>
-__device__ inline void routes_small_body(const b200moe_routes_view& v, u32 end) {
-    __shared__ u32 cnt[1024], ebegin[1024], sid[1024], warp_tot[32], total_s, union_s, maxc;
-    const u32 t = threadIdx.x, nt = blockDim.x, n = v.rows * v.top_k;
-    if (n <= 256) { routes_tiny_body(v, end); return; }
-    for (u32 i = t; i < 1024; i += nt) cnt[i] = 0;
+// The rank of a slot among the slots of its expert: within the slot's warp by a match, over the warps before by counts that each run of 32 slots
+// leaves in shared memory, [runs][experts] 16-bit words. A thread's own walk over the slots before took 14 us for 1024 slots, 6 for 64.
+__device__ __forceinline__ void clear_counts(u16* counts, u32 runs, u32 experts) {
+    for (u32 i = threadIdx.x; i < (runs * experts + 1u) / 2u; i += blockDim.x) reinterpret_cast<u32*>(counts)[i] = 0u;
+}
+__device__ __forceinline__ u32 count_run(u16* counts, u32 run, u32 experts, u32 e) {  // a whole warp; e: 0xffffffff for none. The lanes with the same expert
+    const u32 peers = __match_any_sync(0xffffffffu, e);
+    if (e != 0xffffffffu && (threadIdx.x & 31u) == __ffs(peers) - 1u) counts[run * experts + e] = static_cast<u16>(__popc(peers));
+    return peers;
+}
+__device__ __forceinline__ u32 sum_runs(u16* counts, u32 runs, u32 experts, u32 e) {  // exclusive sums in place; the total
+    u32 n = 0;
+#pragma unroll 4
+    for (u32 w = 0; w < runs; ++w) { const u32 c = counts[w * experts + e]; counts[w * experts + e] = static_cast<u16>(n); n += c; }
+    return n;
+}
+__device__ __forceinline__ u32 rank_of(const u16* counts, u32 run, u32 experts, u32 e, u32 peers) {
+    return counts[run * experts + e] + __popc(peers & ((1u << (threadIdx.x & 31u)) - 1u));
+}
+__host__ __device__ constexpr u32 counts_bytes(u32 slots, u32 experts) { return (((slots + 31u) / 32u * experts * 2u) + 15u) / 16u * 16u; }
+
+// The whole build of a window of up to kChunk slots by one block. ids: the slots' experts, global or shared memory (written before a barrier);
+// counts: counts_bytes(slots, experts) of shared memory. A slot's place in its row, the row's low count and check come from the row's ids in
+// shared memory, its place among its expert's entries from the ranks above and one scan over the experts: five block barriers.
+__device__ inline void routes_small_body(const b200moe_routes_view& v, u32 end, const u32* ids, u16* counts) {
+    __shared__ u32 sid[kChunk], ent[kChunk], ebegin[1024], warp_tot[32], total_s, maxc;
+    const u32 t = threadIdx.x, nt = blockDim.x, lane = t & 31u, n = v.rows * v.top_k, K = v.top_k, E = v.experts, runs = (n + 31u) / 32u;
+    clear_counts(counts, runs, E);
+    for (u32 s = t; s < n; s += nt) sid[s] = ids[s];
     if (t == 0) maxc = 0;
     __syncthreads();
-    for (u32 s = t; s < n; s += nt) {
-        const u32 e = entry_id(v.ids, s, v.top_k, v.experts, v.first, end);
-        if (e != 0xffffffffu) atomicAdd(&cnt[e], 1u);
-        sid[s] = e;
+    for (u32 s = t; s - lane < n; s += nt) {
+        u32 e = 0xffffffffu;
+        if (s < n) {
+            const u32 row = s / K, first = row * K, id = sid[s];
+            u32 pos = 0, low = 0;
+            bool bad = id >= E, repeats = false;  // an earlier slot of the row has the id: no entry (entry_id)
+            for (u32 i = first; i < first + K; ++i) {
+                const u32 o = sid[i];
+                const bool same = o == id && i != s, before = i < s;
+                pos += (o < id || (same && before)) ? 1u : 0u;
+                low += o < v.split ? 1u : 0u;
+                bad |= same;
+                repeats |= same && before;
+            }
+            v.out.order[first + pos] = s;
+            if (s == first) v.out.low_counts[row] = low;
+            if (bad && v.row_status) atomicOr(&v.row_status[row], B200MOE_ROW_INVALID_ROUTE);
+            if (!repeats && owned(id, E, v.first, end)) e = id;
+            ent[s] = e;
+        }
+        count_run(counts, s / 32u, E, e);
     }
-    for (u32 r = t; r < v.rows; r += nt) row_order<RANKED>(v.ids, r, v.top_k, v.experts, v.split, v.out.order, v.out.low_counts, v.row_status);
     __syncthreads();
-    const u32 per = (v.experts + nt - 1) / nt, e0 = t * per, e1 = min(e0 + per, v.experts);
-    u32 c_sum = 0, c_nz = 0, c_max = 0;
-    for (u32 e = e0; e < e1; ++e) { const u32 c = cnt[e]; c_sum += c; c_nz += c ? 1u : 0u; c_max = max(c_max, c); }
-    u32 begin = block_exclusive_scan(c_sum, warp_tot, &total_s);
-    u32 uidx = block_exclusive_scan(c_nz, warp_tot, &union_s);
-    if (c_max) atomicMax(&maxc, c_max);
+    const u32 per = (E + nt - 1) / nt, e0 = min(t * per, E), e1 = min(e0 + per, E);  // a thread's experts
+    u32 sum = 0, most = 0;  // entries, and experts that have some in the upper half (up to 1024 each)
     for (u32 e = e0; e < e1; ++e) {
-        const u32 c = cnt[e];
+        const u32 c = sum_runs(counts, runs, E, e);
+        ebegin[e] = c;
+        sum += c + (c ? 0x10000u : 0u);
+        most = max(most, c);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0 && most) atomicMax(&maxc, most);
+    const u32 at = block_exclusive_scan(sum, warp_tot, &total_s);
+    u32 begin = at & 0xffffu, uidx = at >> 16;
+    for (u32 e = e0; e < e1; ++e) {
+        const u32 c = ebegin[e];
         ebegin[e] = begin;
         if (c) { v.out.experts[uidx] = e - v.base; v.out.begins[uidx + 1] = begin + c; ++uidx; }
         begin += c;
@@ -183,15 +179,13 @@ __device__ inline void routes_small_body(const b200moe_routes_view& v, u32 end) 
     __syncthreads();
     if (t == 0) {
         v.out.begins[0] = 0;
-        v.out.counts[0] = union_s; v.out.counts[1] = maxc; v.out.counts[2] = total_s; v.out.counts[3] = 0;
+        v.out.counts[0] = total_s >> 16; v.out.counts[1] = maxc; v.out.counts[2] = total_s & 0xffffu; v.out.counts[3] = 0;
     }
-    for (u32 s = t; s < n; s += nt) {
-        const u32 e = sid[s];
+    for (u32 s = t; s - lane < n; s += nt) {
+        const u32 e = s < n ? ent[s] : 0xffffffffu, peers = __match_any_sync(0xffffffffu, e);
         if (e == 0xffffffffu) continue;
-        u32 rank = 0;
-        for (u32 i = 0; i < s; ++i) rank += sid[i] == e ? 1u : 0u;
-        const u32 pos = ebegin[e] + rank;
-        v.out.rows[pos] = s / v.top_k;
+        const u32 pos = ebegin[e] + rank_of(counts, s / 32u, E, e, peers);
+        v.out.rows[pos] = s / K;
         v.out.slots[pos] = s;
     }
 }

@@ -64,8 +64,8 @@ __device__ __forceinline__ void build_work_list(const b200moe_routes& routes, u3
     VExpert* unsorted = reinterpret_cast<VExpert*>(t_exp + max_union);
     u32* s_hist = reinterpret_cast<u32*>(unsorted + vmax);
     for (u32 j = tid; j <= n_union; j += blockDim.x) {
-        t_beg[j] = __ldg(routes.begins + j);
-        if (j < n_union) t_exp[j] = __ldg(routes.experts + j);
+        t_beg[j] = load(routes.begins + j);
+        if (j < n_union) t_exp[j] = load(routes.experts + j);
     }
     __syncthreads();
     if (warp == 0) {

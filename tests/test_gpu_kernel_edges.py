@@ -659,3 +659,68 @@ def test_forced_form_is_the_one_that_runs(gpu, oracle, types, form, stem, rows, 
         raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
         assert b200moe.last_launch() == "down_" + stem
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+
+
+# choices in registers: up to 128, 256 and 1024 experts; groups of whole runs of 32 (one, two, three a group), of 2 to 16 lanes, and of 12 (general path)
+@pytest.mark.parametrize("experts,top_k,groups,kept", [(1, 1, 1, 1), (60, 6, 1, 1), (127, 32, 1, 1), (129, 8, 1, 1), (256, 8, 1, 1), (1000, 8, 1, 1), (1024, 32, 1, 1), (256, 8, 8, 4),
+                                                       (256, 8, 4, 2), (192, 6, 2, 1), (512, 8, 8, 3), (64, 8, 32, 5), (64, 8, 8, 4), (128, 8, 8, 4), (96, 8, 8, 4)])
+@pytest.mark.parametrize("score", [O.SOFTMAX, O.SIGMOID])
+def test_selection_by_reductions(gpu, oracle, experts, top_k, groups, kept, score):
+    """Random rows, rows full of ties (four values, zeros of both signs), rows with infinities and a row with a NaN, under both key rules."""
+    import b200moe
+    from b200moe import ops
+    rng = np.random.default_rng(experts + groups)
+    rows = 9
+    z = rng.standard_normal((rows, experts)).astype(np.float32)
+    z[1:4] = rng.integers(-1, 3, (3, experts)).astype(np.float32)
+    z[2, rng.random(experts) < 0.5] *= np.float32(-0.0)
+    z[4:6, rng.integers(0, experts, 4)] = -np.inf
+    z[6, rng.integers(0, experts)] = np.inf
+    z[7, rng.integers(0, experts)] = np.nan
+    bias = rng.integers(-2, 2, experts).astype(np.float32)
+    for key in (O.FLOAT_SERIAL, O.ORDERED_BITS):
+        for order in (O.SELECTION, O.ASCENDING_ID):
+            for with_bias in (0, 1):
+                pol = O.RoutePolicy(score, with_bias, key, order, experts, top_k, groups, kept, 1, 1, 1e-20, 1.5)
+                b = bias if with_bias else None
+                ws, wi, ww = oracle.router(pol, logits=z, bias=b)[1:]
+                view = b200moe.RoutePolicy(*(getattr(pol, f) for f, _ in pol._fields_))
+                gs, gi, gw = ops.enqueue_router(view, logits=dv(z, gpu), bias=None if b is None else dv(b, gpu))[1:]
+                assert same(gs.cpu(), ws) and np.array_equal(gi.cpu().numpy().view(np.uint32), wi) and same(gw.cpu(), ww)
+
+
+@pytest.mark.parametrize("rows,top_k,experts", [(1, 1, 1), (31, 1, 40), (4, 8, 16), (33, 1, 1024), (8, 32, 1000), (1024, 1, 2), (1024, 1, 1024), (341, 3, 7), (1025, 1, 3), (412, 5, 300), (9000, 2, 5)])
+def test_routes_ranks(gpu, oracle, rows, top_k, experts):
+    """Runs of 32 slots with a remainder, more than 255 entries an expert, one block and chunks of 1024 slots that cut rows."""
+    from b200moe import ops
+    ids = window(np.random.default_rng(rows), experts, top_k, rows)
+    want = oracle.routes(ids, experts, experts // 2, 0, 0, 0)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), experts, experts // 2)
+    n, m = int(want["counts"][0]), int(want["counts"][2])
+    assert np.array_equal(r.counts.cpu().numpy()[:3], want["counts"][:3].astype(np.int32)) and int(r.counts[3]) == 0
+    for name, size in (("experts", n), ("begins", n + 1), ("rows", m), ("slots", m), ("order", rows * top_k), ("low_counts", rows)):
+        assert np.array_equal(getattr(r, name).cpu().numpy().view(np.uint32)[:size], want[name][:size]), name
+
+
+@pytest.mark.parametrize("rows,hidden,experts,offset,bf16", [(1, 256, 5, 0, False), (2, 2304, 9, 0, True), (3, 768, 33, 1, False), (4, 512, 16, 0, True), (5, 2304, 6, 1, True), (8, 4352, 10, 0, False), (9, 512, 12, 0, True)])
+def test_decode_front(gpu, oracle, rows, hidden, experts, offset, bf16):
+    """A8 and logits of up to eight rows in one launch, whole columns and several runs, rows off their boundary, bfloat16 widened on the way."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + hidden)
+    I, K = 256, 2
+    gate, up, down = synth.expert_tensors(rng, experts, hidden, I, 12, 12)
+    rw = synth.router_weight(rng, experts, hidden)
+    flat = torch.from_numpy(rng.standard_normal(rows * hidden + offset, dtype=np.float32)).to(gpu)
+    flat = flat.bfloat16() if bf16 else flat
+    x = flat[offset:].view(rows, hidden)
+    status = torch.zeros(rows, dtype=torch.int32, device=gpu)
+    summary = torch.full((1,), 12, dtype=torch.int32, device=gpu)
+    ffn = ops.MoeFfn(ops.make_shape(hidden, I, experts, K, 12, 12), ops.softmax_policy(experts, K), *(dv(a, gpu) for a in (gate, up, down, rw)), capacity=rows,
+                     combine_form=b200moe.COMBINE_FMA_SLOTS)
+    want = oracle.ffn(O.Shape(hidden, I, experts, K, 12, 12, float("inf")), O.softmax_policy(experts, K), gate, up, down, rw, x.float().cpu().numpy(), O.COMBINE_FMA_SLOTS)
+    ffn.ws.fill_(0xff)  # what the workspace held before does not matter
+    for _ in range(2):
+        y, ids, wts = ffn(x, want_routes=True, row_status=status, summary=summary)
+        assert np.array_equal(ids.cpu().numpy().view(np.uint32), want["ids"]) and same(y.cpu(), want["y"])
+        assert int(summary[0]) == 0 and not status.any()

@@ -15,20 +15,19 @@
 //    conflict free) PLUS the same K range of the A8 rows of the item's entries (codes, deltas, sums: three bulk copies per
 //    entry), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
 //  * Two groups of eight consumer warps share a CTA, each with its own ring of stages and its own producer warp; a group's
-//    producer claims the next item of the grid while its consumers still work on the stages in the ring. Lane =
-//    (pair p, row): a lane walks its row's super-blocks in ascending order across the item's stages, the serial chains
-//    acc_p += pair_p never leave their lane, and (a0 + a1) + (a2 + a3) is two xor-shuffles at the end of the item.
-//  * gate/up: the group meets on an mbarrier once per item and eight warps run SwiGLU + the A8 rule of one entry each.
-//  * Two forms of the integer dots, chosen per item by its entry count. Up to kMmaMinEntries - 1 entries: dp4a, lane =
-//    (pair, row), 16 dp4a per (super-block, pair, entry). From kMmaMinEntries entries: the warp's 8 rows x up to 8 entries
-//    x 32 weights of a group are ONE mma.sync.m16n8k32 (A = the entries' codes, signed; B = the rows' nibbles as unsigned
-//    bytes, high nibbles left in place as 16 q; the k order inside a group is permuted the same way on both sides, which
-//    an exact integer sum does not see). The accumulator fragment gives lane (entry, t) the dots of rows 2t and 2t + 1,
-//    and the lane runs the same FP32 operation sequence on them with the rows' factors fetched from a per-warp scratch:
-//    the kernel is bound by issue slots, and at 8 entries this form needs a third of the dp4a form's instructions. It takes over at
-//    5 entries: 64 rows of the large layer (256 experts of 7168 -> 2048, 4.4 entries each) took 876 us a call with that line, 888 with 4, 909
-//    with 3, 967 with 2. Both forms run two cells a packed FP32 instruction (two rows, or two entries) and produce the contract's bits;
-//    with scalar operations and dots converted by addition the call took 930 us.
+//    producer claims the next item of the grid while its consumers still work on the stages in the ring. The serial chains
+//    acc_p += pair_p never leave their lane.
+//  * Two forms of the integer dots, chosen per item by its entry count. One entry: dp4a, lane = (pair p, one of the warp's 8 rows); (a0 + a1) +
+//    (a2 + a3) is two xor-shuffles at the end of the item. From two entries: mma.sync.m16n8k32 (A = nibbles of 16 rows as unsigned bytes, the high ones
+//    left in place as 16 q; B = the codes of up to 8 entries, signed), a warp 32 rows of ONE chain; the four chains meet in shared memory at the end of
+//    the item. With up to 4 entries the eight columns hold them twice, and a lane works for one of the two row tiles only. The row pair of a lane's
+//    cells shares every packed FP32 instruction; both forms produce the contract's bits.
+//  * gate/up: the group meets on an mbarrier once per item and a warp an entry runs SwiGLU + the A8 rule; down: a warp an entry stores the sums.
+// What bounds it: the latency of dependent instructions with four consumer warps a scheduler (64 rows over 64 experts of 7168 -> 2048: 62 % of the issue
+// slots, 67 % of the shared memory's cycles, 49 % of the DRAM's). A warp with 8 rows of four chains, whose factors met 8 rows and which took the tensor cores from
+// 5 entries and dp4a of up to 4 entries below, read shared memory twice as much: 64 rows of the large layer (256 experts) 880 to 917 us a call, 804 to 855
+// now; dense 5120 x 17408, 8 rows, 84.5 and 77.9; 37 rows over 128 experts of 2048 -> 768 112.0 and 109.3. Copies of 144-byte rows (a super-block
+// each) into a ring of 4 stages of two super-blocks instead of 2 of three: dense 1 row 49.8 -> 57.5, 8 rows 84.4 -> 98.3.
 //
 // Every wait is bounded (plan.wait_limit polls): a waiter that runs out raises the CTA's abort flag, every role leaves
 // its loops, the producers wait (bounded) for the copies they still have in flight, B200MOE_JOB_WAIT_ABORTED is set in the
@@ -48,17 +47,19 @@ using namespace q4k;
 using namespace wide;
 using namespace grouped;  // packed FP32
 
-constexpr u32 kItemRows = 64;
-constexpr u32 kMmaMinEntries = 5;                       // items with at least this many entries take the mma form
-constexpr u32 kFacPitch = 36, kFacFloats = 4 * kFacPitch;  // per-warp scratch of the mma form: floats of a pair (a lane's store: 2 ways a bank)
+constexpr u32 kItemRows = 64, kHalfRows = 32;           // an item's two halves: gate and up rows (gate/up), or the first and second 32 of 64 down rows
+constexpr u32 kDpEntries = 1;                           // items of one entry take dp4a, items with more the tensor cores
+constexpr u32 kFewEntries = 4;                          // up to so many a lane of the mma form works for one of the two row tiles only
+constexpr u32 kFacFloats = kHalfRows * 4;               // per-warp scratch of the mma form, a super-block: a pair's four factors of 32 rows
+constexpr u32 kMeetPitch = 36, kMeetFloats = 4 * 2 * kKE * kMeetPitch;  // [pair][half][entry][32 + 4]: a half warp's stores (8 rows, 4 entry pairs) meet every bank once
 
+constexpr u32 kMaxStages = 8;
 struct WidePlan {
     u32 S;              // super-blocks per stage
     u32 nb;             // super-blocks per row
     u32 nseg;           // stages per item
     u32 stages;         // ring depth per group
-    u32 row_seg_bytes;  // S * 144
-    u32 w_bytes;        // 64 * row_seg_bytes
+    u32 w_bytes;        // 64 * S * 144
     u32 x_entry_bytes;  // >= S * 320: codes, deltas, sums of one entry over the stage's K range (+ padding)
     u32 stage_bytes;
     u32 n_chunks;       // items per (virtual) expert
@@ -82,18 +83,19 @@ struct WideArgs {
     u32 raw_vec;           // raw lies on an 8-byte boundary
 };
 
-// Stage geometry for S super-blocks per stage, as compile-time constants: the kernels are bound by issue slots, and
-// address arithmetic on run-time strides was a measurable part of them.
-constexpr u32 x_entry_bytes_of(u32 S) {  // codes, deltas, sums of one entry over a stage, padded so that entries lie 8 or 24
-    u32 b = S * 320u;                     // (mod 32) words apart: the mma form reads 8 bytes per lane at (entry, k slice) and
-    while ((b / 4) % 32 != 8 && (b / 4) % 32 != 24) b += 16;  // four entries then cover all banks once
+// Stage geometry for S super-blocks per stage, as compile-time constants: address
+// arithmetic on run-time strides was a measurable part of the instructions. Weight rows lie S * 144 bytes apart, S odd: an odd multiple of 4 (mod 32) words, so a
+// warp's 128-bit reads of 8 rows and its fragments' word reads are conflict free.
+constexpr u32 x_entry_bytes_of(u32 S) {  // codes, deltas, sums of one entry over a stage, padded so that entries lie an odd multiple of
+    u32 b = S * 320u;                     // 4 (mod 32) words apart: the fragments' word reads of eight entries meet every bank once
+    while ((b / 4) % 8 != 4) b += 16;
     return b;
 }
 template <u32 S_>
 struct Geo {
     static constexpr u32 S = S_;
-    static constexpr u32 row_seg_bytes = S * kQ4KBlock;
-    static constexpr u32 w_bytes = kItemRows * row_seg_bytes;
+    static constexpr u32 row_bytes = S * kQ4KBlock, half_bytes = kHalfRows * row_bytes;
+    static constexpr u32 w_bytes = 2 * half_bytes;
     static constexpr u32 x_entry_bytes = x_entry_bytes_of(S);
 };
 
@@ -114,95 +116,106 @@ __device__ __forceinline__ float4 pair_factors(const uint4& hdr, u32 p) {
     return make_float4(__fmul_rn(d, byte(sc, sel)), __fmul_rn(__fmul_rn(d, 0.0625f), byte(sc, sel + 1u)), __fmul_rn(dm, byte(mn, sel)), __fmul_rn(dm, byte(mn, sel + 1u)));
 }
 
-// One stage of one weight row (this lane's pair p of nbk super-blocks, ascending) against NR staged A8 rows. blk: the
-// row's first super-block of the stage; xs: entry 0's area of the stage ({codes[S * 256], deltas[S * 8], sums[S * 8]},
-// the next entry x_entry_bytes further). acc[r] is the lane's chain acc_p of entry r.
-template <int NR, class G>
-__device__ __forceinline__ void stage_rows(const uint4* blk, u32 nbk, u32 p, const unsigned char* xs, float* acc) {
-    constexpr u32 x_entry_bytes = G::x_entry_bytes, S = G::S;
+// One stage of one weight row (this lane's pair p of nbk super-blocks, ascending) against one staged A8 row. blk: the row's first
+// super-block of the stage; xs: the entry's area of the stage {codes[S * 256], deltas[S * 8], sums[S * 8]}.
+template <class G>
+__device__ __forceinline__ void stage_row(const unsigned char* blk, u32 nbk, u32 p, const unsigned char* xs, float& acc) {
+    constexpr u32 S = G::S;
 #pragma unroll
-    for (u32 b = 0; b < S; ++b, blk += kQ4KBlock / 16) {
+    for (u32 b = 0; b < S; ++b, blk += kQ4KBlock) {
         if (b >= nbk) break;
-        const uint4 hdr = blk[0], q0 = blk[1 + 2 * p], q1 = blk[2 + 2 * p];
+        const uint4* w = reinterpret_cast<const uint4*>(blk);
+        const uint4 hdr = w[0], q0 = w[1 + 2 * p], q1 = w[2 + 2 * p];
         const float4 f = pair_factors(hdr, p);
         const Nibbles n = split_nibbles(q0, q1);
-        float lo[NR], hi[NR];
-        float2 e[NR], sm[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const unsigned char* xe = xs + r * x_entry_bytes;
-            const uint4* c = reinterpret_cast<const uint4*>(xe + 256u * b + 64u * p);
-            const uint4 c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
-            e[r] = *reinterpret_cast<const float2*>(xe + 256u * S + 32u * b + 8u * p);
-            sm[r] = to_float(*reinterpret_cast<const int2*>(xe + 288u * S + 32u * b + 8u * p));
-            int l, h;
-            dots(n, c0, c1, c2, c3, &l, &h);
-            lo[r] = static_cast<float>(l); hi[r] = static_cast<float>(h);
-        }
+        const uint4* c = reinterpret_cast<const uint4*>(xs + 256u * b + 64u * p);
+        const uint4 c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
+        const float2 e = *reinterpret_cast<const float2*>(xs + 256u * S + 32u * b + 8u * p);
+        const float2 sm = to_float(*reinterpret_cast<const int2*>(xs + 288u * S + 32u * b + 8u * p));
+        int l, h;
+        dots(n, c0, c1, c2, c3, &l, &h);
         // x = E * ((D * float(dot)) - (DM * S)) for the pair's two groups; f holds -DM, and (-DM) * S = -(DM * S) exactly
-#pragma unroll
-        for (int r = 0; r + 1 < NR; r += 2) {  // two entries an instruction
-            const float2 sl = add2(mul2(both(f.x), make_float2(lo[r], lo[r + 1])), mul2(both(f.z), make_float2(sm[r].x, sm[r + 1].x)));
-            const float2 sh = add2(mul2(both(f.y), make_float2(hi[r], hi[r + 1])), mul2(both(f.w), make_float2(sm[r].y, sm[r + 1].y)));
-            const float2 x = add2(mul2(make_float2(e[r].x, e[r + 1].x), sl), mul2(make_float2(e[r].y, e[r + 1].y), sh));
-            acc[r] = __fadd_rn(acc[r], x.x);
-            acc[r + 1] = __fadd_rn(acc[r + 1], x.y);
-        }
-        if (NR & 1) {
-            constexpr int r = NR - 1;
-            const float sl = __fadd_rn(__fmul_rn(f.x, lo[r]), __fmul_rn(f.z, sm[r].x)), sh = __fadd_rn(__fmul_rn(f.y, hi[r]), __fmul_rn(f.w, sm[r].y));
-            acc[r] = __fadd_rn(acc[r], __fadd_rn(__fmul_rn(e[r].x, sl), __fmul_rn(e[r].y, sh)));
-        }
+        const float sl = __fadd_rn(__fmul_rn(f.x, static_cast<float>(l)), __fmul_rn(f.z, sm.x));
+        const float sh = __fadd_rn(__fmul_rn(f.y, static_cast<float>(h)), __fmul_rn(f.w, sm.y));
+        acc = __fadd_rn(acc, __fadd_rn(__fmul_rn(e.x, sl), __fmul_rn(e.y, sh)));
     }
 }
 // ---- the mma form of one stage ---------------------------------------------------------------------------------------
-__device__ __forceinline__ int2 mma_s8u8(u32 a0, u32 a2, u32 b0, u32 b1) {
-    // D (16 x 8, s32) = A (16 x 32, s8, row) * B (32 x 8, u8, col); rows 8 .. 15 of A are zero (at most 8 entries).
-    int2 c;
-    int c2, c3;
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-                 : "=r"(c.x), "=r"(c.y), "=r"(c2), "=r"(c3)
-                 : "r"(a0), "r"(0), "r"(a2), "r"(0), "r"(b0), "r"(b1), "r"(0));
-    return c;
+// 16 weight rows x 8 entries x one group: unsigned nibble bytes times signed codes. d[0], d[1]: row lane / 4, entries 2 (lane % 4) and the next; d[2],
+// d[3]: row lane / 4 + 8.
+__device__ __forceinline__ void mma_u8s8(int (&d)[4], const u32 (&a)[4], u32 mask, u32 b0, u32 b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a[0] & mask), "r"(a[1] & mask), "r"(a[2] & mask), "r"(a[3] & mask), "r"(b0), "r"(b1), "r"(0));
 }
-// One stage of the warp's 8 weight rows against up to 8 staged A8 rows with tensor-core dots. w8: the warp's first row of
-// the stage (rows row_seg_bytes apart); fac: the warp's scratch. Lane = (e = lane >> 2, t = lane & 3): acc[p] holds the
-// chains acc_p of rows 2t and 2t + 1 with entry e. Lanes of absent entries compute on stale shared memory and are never stored.
-// The two rows share every instruction: 27 a (pair, two rows) where scalar operations, conversions by addition and shifts took 43.
-template <class G>
-__device__ __forceinline__ void stage_rows_mma(const unsigned char* w8, u32 nbk, u32 lane, const unsigned char* xs, float* fac, float2 (&acc)[4]) {
-    constexpr u32 row_seg_bytes = G::row_seg_bytes, x_entry_bytes = G::x_entry_bytes, S = G::S;
-    const u32 p = lane >> 3, rr = lane & 7u;   // factor decode: lane = (pair, row), as in the dp4a form
-    const u32 e = lane >> 2, t = lane & 3u;    // mma fragments: lane = (entry or weight row, k slice)
-    const unsigned char* xe = xs + e * x_entry_bytes;
-    const unsigned char* wdec = w8 + rr * row_seg_bytes;
-    const unsigned char* wfrag = w8 + e * row_seg_bytes + 16u + 8u * t;   // B fragment: weight row n = lane >> 2
-    float* put = fac + kFacPitch * p + 8u * (rr >> 1) + (rr & 1u);        // [pair][row pair][D, D, D', D' | -DM, -DM, -DM', -DM']
-    const float4* get = reinterpret_cast<const float4*>(fac + 8u * t);
-#pragma unroll 1
-    for (u32 b = 0; b < nbk; ++b) {  // rolled: the body is long, and the form runs where the instruction cache matters
-        const uint4 hdr = *reinterpret_cast<const uint4*>(wdec + kQ4KBlock * b);
-        const float4 f = pair_factors(hdr, p);
-        __syncwarp();   // the previous block's readers are done with the scratch
-        put[0] = f.x; put[2] = f.y; put[4] = f.z; put[6] = f.w;
-        __syncwarp();
-        const float4 e0 = *reinterpret_cast<const float4*>(xe + 256u * S + 32u * b), e1 = *reinterpret_cast<const float4*>(xe + 256u * S + 32u * b + 16u);
-        const int4 s0 = *reinterpret_cast<const int4*>(xe + 288u * S + 32u * b), s1 = *reinterpret_cast<const int4*>(xe + 288u * S + 32u * b + 16u);
-        const float E[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
-        const int Sg[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+// One stage of the warp's 32 weight rows and chain (pair p) against up to 8 staged A8 rows with tensor-core dots. blk: the half's first row and super-block
+// of the stage; fac: the warp's scratch, S x kFacFloats. acc[j][e]: the chain of rows 16 j + lane / 4 and the row 8 further with entry 2 (lane % 4) + e; these two rows
+// share every packed instruction. MANY: items of five entries or more. Else the eight columns hold the entries twice, and of a lane's cells the first
+// tile's count in lanes with lane % 4 < 2, the second tile's in the others: acc[0] alone is used, and half of the work after the dots falls away.
+// Absent entries compute on stale shared memory and are never stored.
+// Why 32 rows of one chain, and not 8 rows of four chains as before: what bounds the loop is what it reads from shared memory (128 bytes a clock). A token's
+// codes, deltas and sums are read once per 32 rows and a row's factors once per two entries and row pair: 44 (MANY) or 36 wavefronts a warp and super-block
+// where the form before took 88; dp4a takes 32 for one entry and 20 more for every further one.
+template <bool MANY, class G>
+__device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk, u32 p, u32 lane, const unsigned char* xs, float* fac, float2 (&acc)[MANY ? 2 : 1][2]) {
+    constexpr u32 x_entry_bytes = G::x_entry_bytes, S = G::S;
+    const u32 g = lane >> 2, t = lane & 3u;
+    {   // the factors, lane = row: rows i and i + 8 of a tile meet by a shuffle, so that a row pair lies in natural register pairs
+        const bool high = lane & 8u;
+        float4* put = reinterpret_cast<float4*>(fac) + 2u * (8u * (lane >> 4) + (lane & 7u)) + (high ? 1u : 0u);  // [tile][row pair]{D, D, D', D'} {-DM, -DM, -DM', -DM'}
+        __syncwarp();   // the previous stage's readers are done with the scratch
 #pragma unroll
-        for (int pp = 0; pp < 4; ++pp) {
-            const uint2 w = *reinterpret_cast<const uint2*>(wfrag + kQ4KBlock * b + 32u * pp);   // 8 bytes = 16 nibbles: k slice t of groups 2pp, 2pp + 1
-            const uint2 al = *reinterpret_cast<const uint2*>(xe + 256u * b + 64u * pp + 8u * t);          // the entry's codes, group 2pp, same k slice
-            const uint2 ah = *reinterpret_cast<const uint2*>(xe + 256u * b + 64u * pp + 32u + 8u * t);    // group 2pp + 1
-            const float4 d4 = get[kFacPitch / 4 * pp], m4 = get[kFacPitch / 4 * pp + 1];
-            const float2 l = to_float(mma_s8u8(al.x, al.y, w.x & 0x0f0f0f0fu, w.y & 0x0f0f0f0fu));
-            const float2 h = to_float(mma_s8u8(ah.x, ah.y, w.x & 0xf0f0f0f0u, w.y & 0xf0f0f0f0u));
-            const float Sl = static_cast<float>(Sg[2 * pp]), Sh = static_cast<float>(Sg[2 * pp + 1]);
-            const float2 sl = add2(mul2(make_float2(d4.x, d4.y), l), mul2(make_float2(m4.x, m4.y), both(Sl)));
-            const float2 sh = add2(mul2(make_float2(d4.z, d4.w), h), mul2(make_float2(m4.z, m4.w), both(Sh)));
-            acc[pp] = add2(add2(mul2(both(E[2 * pp]), sl), mul2(both(E[2 * pp + 1]), sh)), acc[pp]);
+        for (u32 b = 0; b < S; ++b) {
+            if (b >= nbk) break;
+            const float4 f = pair_factors(*reinterpret_cast<const uint4*>(blk + b * kQ4KBlock + lane * G::row_bytes), p);
+            const float u = __shfl_xor_sync(0xffffffffu, high ? f.x : f.z, 8), v = __shfl_xor_sync(0xffffffffu, high ? f.y : f.w, 8);
+            put[b * (kFacFloats / 4)] = high ? make_float4(u, f.z, v, f.w) : make_float4(f.x, u, f.y, v);
         }
+        __syncwarp();
+    }
+    const unsigned char* rows = blk + g * G::row_bytes + 16u + 32u * p + 4u * t;
+    const unsigned char* codes = xs + (MANY ? g : g & 3u) * x_entry_bytes + 64u * p + 4u * t;
+    const unsigned char* es = xs + 2u * (MANY ? t : t & 1u) * x_entry_bytes + 256u * S + 8u * p;
+    const float4* get = reinterpret_cast<const float4*>(fac) + 2u * g;
+    const bool second = t >= 2u;  // of the few form
+#pragma unroll
+    for (u32 b = 0; b < nbk; ++b) {
+        u32 a[2][4], bl[2], bh[2];
+#pragma unroll
+        for (u32 j = 0; j < 2; ++j)
+#pragma unroll
+            for (u32 i = 0; i < 4; ++i) a[j][i] = *reinterpret_cast<const u32*>(rows + (16u * j + 8u * (i & 1u)) * G::row_bytes + 16u * (i >> 1));
+#pragma unroll
+        for (u32 i = 0; i < 2; ++i) { bl[i] = *reinterpret_cast<const u32*>(codes + 16u * i); bh[i] = *reinterpret_cast<const u32*>(codes + 32u + 16u * i); }
+        float2 E[2], Sg[2];
+#pragma unroll
+        for (u32 e = 0; e < 2; ++e) {
+            E[e] = *reinterpret_cast<const float2*>(es + e * x_entry_bytes);
+            Sg[e] = to_float(*reinterpret_cast<const int2*>(es + e * x_entry_bytes + 32u * S));
+        }
+        int l[2][4], h[2][4];
+#pragma unroll
+        for (u32 j = 0; j < 2; ++j) {
+            mma_u8s8(l[j], a[j], 0x0f0f0f0fu, bl[0], bl[1]);
+            mma_u8s8(h[j], a[j], 0xf0f0f0f0u, bh[0], bh[1]);
+        }
+        if (!MANY) {
+#pragma unroll
+            for (u32 i = 0; i < 4; ++i) { l[0][i] = second ? l[1][i] : l[0][i]; h[0][i] = second ? h[1][i] : h[0][i]; }
+        }
+#pragma unroll
+        for (u32 j = 0; j < (MANY ? 2u : 1u); ++j) {
+            const u32 tile = MANY ? j : (second ? 1u : 0u);
+            const float4 d4 = get[16u * tile], m4 = get[16u * tile + 1u];
+            const float2 Dl = make_float2(d4.x, d4.y), Dh = make_float2(d4.z, d4.w), Ml = make_float2(m4.x, m4.y), Mh = make_float2(m4.z, m4.w);
+#pragma unroll
+            for (u32 e = 0; e < 2; ++e) {
+                const float2 sl = add2(mul2(Dl, to_float(make_int2(l[j][e], l[j][e + 2]))), mul2(Ml, both(Sg[e].x)));
+                const float2 sh = add2(mul2(Dh, to_float(make_int2(h[j][e], h[j][e + 2]))), mul2(Mh, both(Sg[e].y)));
+                acc[j][e] = add2(add2(mul2(both(E[e].x), sl), mul2(both(E[e].y), sh)), acc[j][e]);
+            }
+        }
+        rows += kQ4KBlock; codes += 256; es += 32; get += kFacFloats / 4;
     }
 }
 
@@ -221,16 +234,17 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     u32* claim = a.routes.counts + 3;  // the grid's claim word (wide_common.cuh)
 
     unsigned char* at = smem + kGroups * plan.stages * plan.stage_bytes;
-    float* s_gu = reinterpret_cast<float*>(at);  // [group][buffer][gate | up][entry][32]
-    if (!DOWN) at += kGroups * 2 * 2 * kKE * 32 * 4;
+    float* s_meet = reinterpret_cast<float*>(at);  // [group][kMeetFloats]: an item's chains
+    at += kGroups * kMeetFloats * 4;
     VExpert* table = reinterpret_cast<VExpert*>(at);
     at += (u64(plan.vmax) * sizeof(VExpert) + 15) & ~u64(15);  // what follows holds 8- and 16-byte objects
-    float* s_fac = reinterpret_cast<float*>(at);  // [consumer warp][kFacFloats]
-    at += kConsumerWarps * kFacFloats * 4;
+    float* s_fac = reinterpret_cast<float*>(at);  // [consumer warp][S][kFacFloats]
+    at += kConsumerWarps * S_ * kFacFloats * 4;
     u64* full = reinterpret_cast<u64*>(at);
     u64* empty = full + kGroups * plan.stages;
-    u64* gu_bar = empty + kGroups * plan.stages;
-    at += (2 * kGroups * plan.stages + kGroups) * 8;
+    u64* met = empty + kGroups * plan.stages;  // a group's item: its chains are there
+    u64* left = met + kGroups;                 // ... and have been read
+    at += (2 * kGroups * plan.stages + 2 * kGroups) * 8;
     u32* slot_item = reinterpret_cast<u32*>(at);
     at += kGroups * plan.stages * 4;
     u32* ctl = reinterpret_cast<u32*>(at);  // [0] abort flag, [1] producers that have retired, [2] virtual experts, [3] items
@@ -238,9 +252,9 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     if (tid < kGroups * plan.stages) { mbar_init(&full[tid], 1); mbar_init(&empty[tid], kGroupWarps); }
-    if (tid < kGroups) mbar_init(&gu_bar[tid], kGroupWarps);
+    if (tid < 2 * kGroups) mbar_init(&met[tid], kGroupWarps);
     if (tid < 4) ctl[tid] = 0;
-    if (tid < kGroups * plan.stages + kGroups) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (tid < kGroups * plan.stages + 2 * kGroups) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 
     // ---- the virtual expert list (the stage area is free until the first copy is issued: it holds the copied routes)
     build_work_list(a.routes, n_union, plan.max_union, plan.vmax, plan.n_chunks, reinterpret_cast<u32*>(smem), table, ctl);
@@ -295,18 +309,14 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 unsigned char* dst = g_stage + slot * plan.stage_bytes;
                 if (lane == 0) {
                     g_item[slot] = item;
-                    mbar_expect_tx(&g_full[slot], G::w_bytes + ve_ne * nbk * 320u);
+                    mbar_expect_tx(&g_full[slot], G::w_bytes + ve_ne * nbk * 320u);  // whole boxes: what lies past the row is filled
                 }
                 __syncwarp();
                 if (lane == 0) {
                     const u32 x = s * G::S * (kQ4KBlock / 8);  // 64-bit elements: a multiple of 18, i.e. of 144 bytes
-                    if (DOWN) {
-                        tma_2d(dst, &tm0, x, ve.expert() * a.rows_per_expert + kItemRows * chunk, &g_full[slot]);
-                    } else {
-                        const u32 y = ve.expert() * a.rows_per_expert + 32u * chunk;
-                        tma_2d(dst, &tm0, x, y, &g_full[slot]);
-                        tma_2d(dst + 32u * G::row_seg_bytes, &tm1, x, y, &g_full[slot]);
-                    }
+                    const u32 y = ve.expert() * a.rows_per_expert + (DOWN ? kItemRows : kHalfRows) * chunk;
+                    tma_2d(dst, &tm0, x, y, &g_full[slot]);
+                    tma_2d(dst + G::half_bytes, &tm1, x, DOWN ? y + kHalfRows : y, &g_full[slot]);
                 }
                 if (e < ve_ne) {
                     unsigned char* xd = dst + G::w_bytes + e * G::x_entry_bytes;
@@ -328,14 +338,17 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 
     // ------------------------------------------------------------------------------------------ consumer warps
     const u32 g = warp / kGroupWarps, w = warp % kGroupWarps;
-    const u32 p = lane >> 3, rr = lane & 7u;
-    float* fac = s_fac + warp * kFacFloats;
+    const u32 p = lane >> 3, rr = lane & 7u;     // dp4a form: lane = (pair, one of the warp's 8 rows)
+    const u32 mp = w & 3u, half = w >> 2;        // mma form: the warp's chain and half of the item
+    const u32 me = lane >> 2, mt = lane & 3u;
+    float* fac = s_fac + warp * (S_ * kFacFloats);
+    float* meet = s_meet + g * kMeetFloats;
     u64* g_full = full + g * plan.stages;
     u64* g_empty = empty + g * plan.stages;
     const u32* g_item = slot_item + g * plan.stages;
     const unsigned char* g_stage = smem + g * plan.stages * plan.stage_bytes;
     const u32 act_stride = DOWN ? 0u : (a.act.stride ? a.act.stride : a.act.width);
-    u32 slot = 0, phase = 0, kl = 0;  // ring position of the group's next stage, kept incrementally (no divisions in the loop)
+    u32 slot = 0, phase = 0, kl = 0;  // ring position of the group's next stage, kept incrementally (no divisions in the loop); meetings so far
     bool ok = true;
     for (;;) {
         ok = mbar_wait(&g_full[slot], phase, plan.wait_limit, abort_flag);
@@ -346,23 +359,10 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         const u32 jv = item / plan.n_chunks, chunk = item - jv * plan.n_chunks;
         const VExpert ve = table[jv];
         const u32 ne = ve.ne(), vbegin = ve.begin();
-        const bool mma = ne >= kMmaMinEntries;
-        u32 slots[kMmaMinEntries - 1] = {}, slot_id = 0;  // asked for before the stages, used behind them
-        if (DOWN && mma) slot_id = (lane >> 2) < ne ? load(a.routes.slots + vbegin + (lane >> 2)) : 0u;
-        if (!DOWN) slot_id = w < ne ? load(a.routes.slots + vbegin + w) : 0u;
-        if (DOWN && !mma) {
-#pragma unroll
-            for (int r = 0; r < (int)kMmaMinEntries - 1; ++r) slots[r] = load(a.routes.slots + vbegin + min(u32(r), ne - 1u));
-        }
-        float acc[kMmaMinEntries - 1];
-        float2 acc2[4];  // mma form
-#pragma unroll
-        for (int r = 0; r < (int)kMmaMinEntries - 1; ++r) acc[r] = 0.0f;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc2[r] = make_float2(0.0f, 0.0f);
-        // the item's stages, with the form and the entry count fixed at compile time inside the loop (NR = 0: the mma form)
-        auto run = [&](auto tag) {
-            constexpr int NR = decltype(tag)::value;
+        const bool mma = ne > kDpEntries;
+        const u32 slot_id = w < ne ? load(a.routes.slots + vbegin + w) : 0u;  // asked for before the stages, used behind them
+        // the item's stages, with the form fixed at compile time inside the loop
+        auto stages = [&](auto step) {
             for (u32 s = 0; s < plan.nseg; ++s) {
                 if (s) {
                     ok = mbar_wait(&g_full[slot], phase, plan.wait_limit, abort_flag);
@@ -370,64 +370,76 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                     if (!ok) return;
                 }
                 const unsigned char* st = g_stage + slot * plan.stage_bytes;
-                const u32 nbk = min(G::S, plan.nb - s * G::S);
-                if constexpr (NR == 0) stage_rows_mma<G>(st + 8u * w * G::row_seg_bytes, nbk, lane, st + G::w_bytes, fac, acc2);
-                else stage_rows<NR, G>(reinterpret_cast<const uint4*>(st + (8u * w + rr) * G::row_seg_bytes), nbk, p, st + G::w_bytes, acc);
+                step(st, min(G::S, plan.nb - s * G::S));
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&g_empty[slot]);  // the stage is free for the producer
                 if (++slot == plan.stages) { slot = 0; phase ^= 1u; }
             }
         };
-        switch (mma ? 0u : ne) {
-            case 0: run(std::integral_constant<int, 0>{}); break;
-            case 1: run(std::integral_constant<int, 1>{}); break;
-            case 2: run(std::integral_constant<int, 2>{}); break;
-            case 3: run(std::integral_constant<int, 3>{}); break;
-            default: run(std::integral_constant<int, 4>{}); break;
+        // the chains meet in shared memory, once the previous item's have been read
+        auto hand_over = [&](auto store) {
+            if (kl) ok = mbar_wait(&left[g], (kl - 1u) & 1u, plan.wait_limit, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) return;
+            store();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&met[g]);
+            ok = mbar_wait(&met[g], kl & 1u, plan.wait_limit, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+        };
+        auto run_mma = [&](auto many) {
+            constexpr bool MANY = decltype(many)::value;
+            float2 acc[MANY ? 2 : 1][2];
+#pragma unroll
+            for (u32 j = 0; j < (MANY ? 2u : 1u); ++j) { acc[j][0] = make_float2(0.0f, 0.0f); acc[j][1] = make_float2(0.0f, 0.0f); }
+            stages([&](const unsigned char* st, u32 nbk) { stage_rows_mma<MANY, G>(st + half * G::half_bytes, nbk, mp, lane, st + G::w_bytes, fac, acc); });
+            if (!ok) return;
+            hand_over([&]() {
+#pragma unroll
+                for (u32 j = 0; j < (MANY ? 2u : 1u); ++j)
+#pragma unroll
+                    for (u32 e = 0; e < 2; ++e) {
+                        const u32 tile = MANY ? j : mt >> 1, entry = 2u * (MANY ? mt : mt & 1u) + e;
+                        float* to = meet + ((2u * mp + half) * kKE + entry) * kMeetPitch + 16u * tile + me;
+                        to[0] = acc[j][e].x;
+                        to[8] = acc[j][e].y;
+                    }
+            });
+        };
+        if (!mma) {
+            const u32 only_slot = DOWN ? load(a.routes.slots + vbegin) : 0u;
+            float acc = 0.0f;
+            stages([&](const unsigned char* st, u32 nbk) { stage_row<G>(st + half * G::half_bytes + (8u * mp + rr) * G::row_bytes, nbk, p, st + G::w_bytes, acc); });
+            if (!ok) break;
+            const float val = tree4(acc);
+            if (DOWN) {
+                if (p == 0) a.raw[u64(only_slot) * a.out_width + kItemRows * chunk + 8u * w + rr] = val;
+                continue;
+            }
+            hand_over([&]() { if (p == 0) meet[half * kKE * kMeetPitch + 8u * mp + rr] = val; });
+        } else if (ne > kFewEntries) {
+            run_mma(std::true_type{});
+        } else {
+            run_mma(std::false_type{});
         }
         if (!ok) break;
-        // mma form: lane (e = lane >> 2, t = lane & 3) holds the four chains of rows 2t and 2t + 1 of entry e
-        const float m0 = __fadd_rn(__fadd_rn(acc2[0].x, acc2[1].x), __fadd_rn(acc2[2].x, acc2[3].x));
-        const float m1 = __fadd_rn(__fadd_rn(acc2[0].y, acc2[1].y), __fadd_rn(acc2[2].y, acc2[3].y));
-        const u32 me = lane >> 2, mt = lane & 3u;
-        if (DOWN) {
-            if (mma) {
-                if (me < ne) {
-                    float* dst = a.raw + u64(slot_id) * a.out_width + kItemRows * chunk + 8u * w + 2u * mt;
-                    if (a.raw_vec) *reinterpret_cast<float2*>(dst) = make_float2(m0, m1);
-                    else { dst[0] = m0; dst[1] = m1; }
-                }
-            } else {
+        if (w < ne) {
+            const float* mine = meet + w * kMeetPitch;
+            constexpr u32 kHalf = kKE * kMeetPitch, kPair = 2 * kHalf;
+            if (DOWN) {  // two neighbouring outputs of entry w a lane
+                float2 c[4];
 #pragma unroll
-                for (int r = 0; r < (int)kMmaMinEntries - 1; ++r) {
-                    if (r < (int)ne) {
-                        const float val = tree4(acc[r]);
-                        if (p == 0) a.raw[u64(slots[r]) * a.out_width + kItemRows * chunk + 8u * w + rr] = val;
-                    }
+                for (u32 i = 0; i < 4; ++i) c[i] = *reinterpret_cast<const float2*>(mine + i * kPair + (lane >> 4) * kHalf + 2u * (lane & 15u));
+                const float v0 = __fadd_rn(__fadd_rn(c[0].x, c[1].x), __fadd_rn(c[2].x, c[3].x)), v1 = __fadd_rn(__fadd_rn(c[0].y, c[1].y), __fadd_rn(c[2].y, c[3].y));
+                float* dst = a.raw + u64(slot_id) * a.out_width + kItemRows * chunk + 2u * lane;
+                if (a.raw_vec) *reinterpret_cast<float2*>(dst) = make_float2(v0, v1);
+                else { dst[0] = v0; dst[1] = v1; }
+            } else {  // SwiGLU + the A8 rule over the 32 outputs of entry w
+                float gv = mine[lane], uv = mine[kHalf + lane];
+                if (mma) {
+                    gv = __fadd_rn(__fadd_rn(gv, mine[kPair + lane]), __fadd_rn(mine[2 * kPair + lane], mine[3 * kPair + lane]));
+                    uv = __fadd_rn(__fadd_rn(uv, mine[kPair + kHalf + lane]), __fadd_rn(mine[2 * kPair + kHalf + lane], mine[3 * kPair + kHalf + lane]));
                 }
-            }
-        } else {
-            // the item's 2 x 32 outputs of every entry meet in shared memory; then one warp per entry runs the epilogue
-            float* gu = s_gu + u64((g * 2 + (kl & 1u)) * 2) * kKE * 32;
-            if (mma) {
-                if (me < ne) *reinterpret_cast<float2*>(gu + (w >> 2) * kKE * 32 + me * 32 + 8u * (w & 3u) + 2u * mt) = make_float2(m0, m1);
-            } else {
-                float* mine = gu + (w >> 2) * kKE * 32 + 8u * (w & 3u) + rr;
-#pragma unroll
-                for (int r = 0; r < (int)kMmaMinEntries - 1; ++r) {
-                    if (r < (int)ne) {
-                        const float val = tree4(acc[r]);
-                        if (p == 0) mine[r * 32] = val;
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&gu_bar[g]);
-            ok = mbar_wait(&gu_bar[g], kl & 1u, plan.wait_limit, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            if (w < ne) {  // SwiGLU + the A8 rule over the 32 outputs of entry w
-                const float gv = gu[w * 32 + lane], uv = gu[kKE * 32 + w * 32 + lane];
                 const u32 o_col = 32u * chunk + lane;
                 if (a.gate_out) { a.gate_out[u64(slot_id) * a.out_width + o_col] = gv; a.up_out[u64(slot_id) * a.out_width + o_col] = uv; }
                 const float h = swiglu_qwen(gv, uv);
@@ -449,6 +461,8 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 }
             }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&left[g]);
         ++kl;
     }
     if (!ok && lane == 0 && a.summary) atomicOr(a.summary, kAbortBit);
@@ -456,20 +470,19 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 
 u32 round_up(u32 v, u32 a) { return (v + a - 1) / a * a; }
 
-u32 fixed_smem(const WidePlan& p, bool down) {
-    return (down ? 0u : kGroups * 2 * 2 * kKE * 32 * 4) + round_up(p.vmax * static_cast<u32>(sizeof(VExpert)), 16) + kConsumerWarps * kFacFloats * 4 +
-           (2 * kGroups * p.stages + kGroups) * 8 + kGroups * p.stages * 4 + 64;
+u32 fixed_smem(const WidePlan& p) {
+    return kGroups * kMeetFloats * 4 + round_up(p.vmax * static_cast<u32>(sizeof(VExpert)), 16) + kConsumerWarps * p.S * kFacFloats * 4 +
+           (2 * kGroups * p.stages + 2 * kGroups) * 8 + kGroups * p.stages * 4 + 64;
 }
-u32 plan_smem(const WidePlan& p, bool down) { return kGroups * p.stages * p.stage_bytes + fixed_smem(p, down); }
+u32 plan_smem(const WidePlan& p) { return kGroups * p.stages * p.stage_bytes + fixed_smem(p); }
 
 // K: the row length; n_chunks: items per expert; slots: rows * top_k of the window. False when the form does not apply.
-bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, bool down, WidePlan* p) {
+bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, WidePlan* p) {
     if (K == 0 || K % 256 || max_union == 0 || slots == 0 || slots > 8192) return false;
     p->nb = K / 256;
-    p->S = p->nb >= 3 ? 3u : 1u;  // odd: rows S * 144 bytes apart stay conflict free
+    p->S = p->nb >= 3 ? 3u : 1u;  // odd: see Geo
     p->nseg = (p->nb + p->S - 1) / p->S;
-    p->row_seg_bytes = p->S * kQ4KBlock;
-    p->w_bytes = kItemRows * p->row_seg_bytes;
+    p->w_bytes = kItemRows * p->S * kQ4KBlock;
     p->x_entry_bytes = x_entry_bytes_of(p->S);
     // a stage holds the A8 segments of as many entries as a virtual expert of this window can have: windows of fewer than
     // kKE slots get smaller stages and with them a deeper ring
@@ -478,8 +491,8 @@ bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, bool down, WidePla
     p->max_union = max_union;
     p->vmax = max_union + static_cast<u32>(slots / kKE) + 1;
     if (u64(p->vmax) * n_chunks + 4096 >= kClaimMask) return false;  // items and the groups' closing claims fit the claim word's count
-    for (p->stages = 5; p->stages >= 2; --p->stages)
-        if (plan_smem(*p, down) <= kSmemBudget) break;
+    for (p->stages = kMaxStages; p->stages >= 2; --p->stages)
+        if (plan_smem(*p) <= kSmemBudget) break;
     if (p->stages < 2) return false;
     if (work_list_scratch_words(max_union, p->vmax) * 4 > kGroups * p->stages * p->stage_bytes) return false;  // the work list is built in the stage area
     p->wait_limit = kDefaultWaitLimit;
@@ -504,18 +517,18 @@ void apply_hooks(WidePlan* p) {
 bool wide_gate_up_fits(const b200moe_gate_up_view& v, u32 rows) {
     WidePlan p{};
     return v.shape.gate_type == B200MOE_TYPE_Q4_K && rows && a8_bulk_ok(v.x) && v.shape.inter % 32 == 0 &&
-           make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, false, &p);
+           make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, &p);
 }
 bool wide_down_fits(const b200moe_down_view& v, u32 rows) {
     WidePlan p{};
     return v.shape.down_type == B200MOE_TYPE_Q4_K && rows && a8_bulk_ok(v.act) && v.shape.hidden % 64 == 0 &&
-           make_plan(v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, true, &p);
+           make_plan(v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, &p);
 }
 
 int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     WidePlan p{};
-    if (!make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, false, &p))
+    if (!make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, &p))
         return fail(B200MOE_ERR_UNSUPPORTED, "gate_up: the segment-streaming form does not apply to this shape");
     apply_hooks(&p);
     WideArgs a{};
@@ -523,9 +536,9 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_
     a.row_status = v.row_status; a.summary = v.summary; a.rows_per_expert = v.shape.inter; a.out_width = v.shape.inter;
     CUtensorMap tm0, tm1;
     const u64 rb = u64(p.nb) * kQ4KBlock, total_rows = u64(v.shape.experts) * v.shape.inter;
-    if (int rc = rows_map(v.weights.gate, rb, total_rows, p.S * kQ4KBlock, 32, &tm0)) return rc;
-    if (int rc = rows_map(v.weights.up, rb, total_rows, p.S * kQ4KBlock, 32, &tm1)) return rc;
-    const u32 smem = plan_smem(p, false);
+    if (int rc = rows_map(v.weights.gate, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &tm0)) return rc;
+    if (int rc = rows_map(v.weights.up, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &tm1)) return rc;
+    const u32 smem = plan_smem(p);
     if (p.S == 3) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<false, 3>), smem)) return rc;
         chain_launch(q4k_wide_kernel<false, 3>, sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
@@ -539,15 +552,15 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_
 int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     WidePlan p{};
-    if (!make_plan(v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, true, &p))
+    if (!make_plan(v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, &p))
         return fail(B200MOE_ERR_UNSUPPORTED, "down: the segment-streaming form does not apply to this shape");
     apply_hooks(&p);
     WideArgs a{};
     a.routes = v.routes; a.in = v.act; a.raw = v.raw; a.summary = const_cast<u32*>(v.summary);
     a.rows_per_expert = v.shape.hidden; a.out_width = v.shape.hidden; a.raw_vec = aligned(v.raw, 8);
     CUtensorMap tm0;
-    if (int rc = rows_map(v.weights.down, u64(p.nb) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, p.S * kQ4KBlock, 64, &tm0)) return rc;
-    const u32 smem = plan_smem(p, true);
+    if (int rc = rows_map(v.weights.down, u64(p.nb) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, p.S * kQ4KBlock, kHalfRows, &tm0)) return rc;
+    const u32 smem = plan_smem(p);
     if (p.S == 3) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<true, 3>), smem)) return rc;
         chain_launch(q4k_wide_kernel<true, 3>, sm_count(), kThreads, smem, stream, tm0, tm0, a, p);

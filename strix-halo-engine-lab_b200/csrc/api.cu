@@ -324,7 +324,7 @@ Q8Form pick_q8_form(const b200moe_shape& s, bool wide_fits, bool mma_fits, bool 
     }
     return Q8Form::row_per_warp;
 }
-int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0) {
+int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0, const ChainHints& hints = {}) {
     if (v.shape.gate_type == B200MOE_TYPE_Q2_K) return launch_gate_up_ds41_any(v, st);  // the generic form of the family reads every block type
     if (!is_kquant(v.shape.gate_type)) {
         switch (pick_q8_form(v.shape, q8_wide_gate_up_fits(v, rows), q8_mma_gate_up_fits(v, rows), grouped_q8_gate_up_fits(v), rows, v.max_union, false)) {
@@ -338,16 +338,16 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
     switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.x.sums != nullptr), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, v.max_union, grouped_min_rows, false)) {
         case Q4Form::grouped: return launch_gate_up_q4k_grouped(v, st);
         case Q4Form::row_stream: return launch_gate_up_q4k_stream(v, rows, st);
-        case Q4Form::wide: return launch_gate_up_q4k_wide(v, rows, st);
+        case Q4Form::wide: return launch_gate_up_q4k_wide(v, rows, hints, st);
         default: return launch_gate_up_q4k(v, st);
     }
 }
-int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0) {
+int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0, const ChainHints& hints = {}) {
     if (v.shape.down_type == B200MOE_TYPE_Q4_K) {
         switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.act.sums != nullptr), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, v.max_union, grouped_min_rows, true)) {
             case Q4Form::grouped: return launch_down_q4k_grouped(v, st);
-            case Q4Form::row_stream: return launch_down_q4k_stream(v, rows, st);
-            case Q4Form::wide: return launch_down_q4k_wide(v, rows, st);
+            case Q4Form::row_stream: return launch_down_q4k_stream(v, rows, hints, st);
+            case Q4Form::wide: return launch_down_q4k_wide(v, rows, hints, st);
             default: return launch_down_q4k(v, st);
         }
     }
@@ -357,7 +357,7 @@ int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grou
         case Q8Form::grouped: return launch_down_q8_grouped(v, st);
         case Q8Form::mma: return launch_down_q8_mma(v, rows, st);
         case Q8Form::wide: return launch_down_q8_wide(v, rows, st);
-        default: return launch_down_q8(v, st);
+        default: return launch_down_q8(v, hints, st);
     }
 }
 
@@ -571,14 +571,15 @@ static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_rea
     gu.shape = s; gu.weights = v->weights; gu.routes = L.routes; gu.max_union = max_union;
     gu.x = v->x; gu.act = L.act; gu.row_status = row_status; gu.summary = summary;
     tap(2);
-    if (int rc = enqueue_gate_up(gu, v->rows, st, v->grouped_min_rows)) return rc;
+    const u64 slots = u64(v->rows) * s.top_k;
+    if (int rc = enqueue_gate_up(gu, v->rows, st, v->grouped_min_rows, ChainHints{false, 0, slots})) return rc;
     tap(3);
 
     b200moe_down_view dn{};
     dn.shape = s; dn.weights = v->weights; dn.routes = L.routes; dn.max_union = max_union;
     dn.act = L.act; dn.raw = raw; dn.summary = summary;
     tap(4);
-    if (int rc = enqueue_down(dn, v->rows, st, v->grouped_min_rows)) return rc;
+    if (int rc = enqueue_down(dn, v->rows, st, v->grouped_min_rows, ChainHints{true, 0, slots})) return rc;  // gate/up was admitted after the routes
     tap(5);
 
     if (!v->y && !v->y_blocks) return B200MOE_OK;
@@ -710,10 +711,10 @@ int b200moe_dense_ffn(const b200moe_dense_view* v, void* stream) {
     b200moe_gate_up_view gu{};
     gu.shape = s; gu.weights = v->weights; gu.routes = L.routes; gu.max_union = 1; gu.x = v->x; gu.act = L.act;
     gu.row_status = L.row_status; gu.summary = L.summary;
-    if (int rc = enqueue_gate_up(gu, v->rows, st)) return rc;
+    if (int rc = enqueue_gate_up(gu, v->rows, st, 0, ChainHints{false, v->rows, v->rows})) return rc;
     b200moe_down_view dn{};
     dn.shape = s; dn.weights = v->weights; dn.routes = L.routes; dn.max_union = 1; dn.act = L.act; dn.raw = v->y; dn.summary = L.summary;
-    if (int rc = enqueue_down(dn, v->rows, st)) return rc;
+    if (int rc = enqueue_down(dn, v->rows, st, 0, ChainHints{true, v->rows, v->rows})) return rc;
     if (v->y_bf16) {
         // bfloat16 RNE copy of y through the FMA_SLOTS combine with unit weights: fma(1, y, +0) = y exactly
         float* ones = reinterpret_cast<float*>(L.aux);  // the ids are no longer read once the routes exist

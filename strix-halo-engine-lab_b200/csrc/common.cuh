@@ -81,6 +81,8 @@ __device__ __forceinline__ void chain_begin() {
 }
 template <class T>
 __device__ __forceinline__ T load(const T* p) { return *p; }
+// The same past the L1 cache, for what is known to be complete before the wait (ChainHints): the multiprocessor's L1 may hold lines of an earlier call.
+__device__ __forceinline__ u32 load_l2(const u32* p) { return __ldcg(p); }
 // Enqueues a kernel of the chain; its status is read by after_launch.
 template <class... P, class... A>
 inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, cudaStream_t stream, A&&... args) {

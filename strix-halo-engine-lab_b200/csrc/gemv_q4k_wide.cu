@@ -64,9 +64,12 @@ struct WidePlan {
     u32 stage_bytes;
     u32 n_chunks;       // items per (virtual) expert
     u32 max_union;      // bound of the union
+    u32 n_bound;        // ... that the routes' arrays are known to hold too, or 0
     u32 vmax;           // capacity of the virtual expert list
     u32 wait_limit;
     u32 stall_stage;    // test hook: group 0's producer stops before this stage (0xffffffff: never)
+    u32 early;          // routes and weights are complete before the launch in front was admitted (ChainHints)
+    u32 dense_rows;     // rows of a dense block: its entries need no routes; 0 otherwise
 };
 
 struct WideArgs {
@@ -162,7 +165,7 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk
     const u32 g = lane >> 2, t = lane & 3u;
     {   // the factors, lane = row: rows i and i + 8 of a tile meet by a shuffle, so that a row pair lies in natural register pairs
         const bool high = lane & 8u;
-        float4* put = reinterpret_cast<float4*>(fac) + 2u * (8u * (lane >> 4) + (lane & 7u)) + (high ? 1u : 0u);  // [tile][row pair]{D, D, D', D'} {-DM, -DM, -DM', -DM'}
+        float4* put = reinterpret_cast<float4*>(fac) + 8u * (lane >> 4) + (lane & 7u) + (high ? 16u : 0u);  // [tile][row pair]{D, D, D', D'}, then {-DM, -DM, -DM', -DM'}
         __syncwarp();   // the previous stage's readers are done with the scratch
 #pragma unroll
         for (u32 b = 0; b < S; ++b) {
@@ -176,7 +179,7 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk
     const unsigned char* rows = blk + g * G::row_bytes + 16u + 32u * p + 4u * t;
     const unsigned char* codes = xs + (MANY ? g : g & 3u) * x_entry_bytes + 64u * p + 4u * t;
     const unsigned char* es = xs + 2u * (MANY ? t : t & 1u) * x_entry_bytes + 256u * S + 8u * p;
-    const float4* get = reinterpret_cast<const float4*>(fac) + 2u * g;
+    const float4* get = reinterpret_cast<const float4*>(fac) + g;
     const bool second = t >= 2u;  // of the few form
 #pragma unroll
     for (u32 b = 0; b < nbk; ++b) {
@@ -206,7 +209,7 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk
 #pragma unroll
         for (u32 j = 0; j < (MANY ? 2u : 1u); ++j) {
             const u32 tile = MANY ? j : (second ? 1u : 0u);
-            const float4 d4 = get[16u * tile], m4 = get[16u * tile + 1u];
+            const float4 d4 = get[8u * tile], m4 = get[8u * tile + 16u];
             const float2 Dl = make_float2(d4.x, d4.y), Dh = make_float2(d4.z, d4.w), Ml = make_float2(m4.x, m4.y), Mh = make_float2(m4.z, m4.w);
 #pragma unroll
             for (u32 e = 0; e < 2; ++e) {
@@ -224,13 +227,10 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk
 template <bool DOWN, u32 S_>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, WideArgs a, WidePlan plan) {
-    chain_begin();
     using G = Geo<S_>;
     extern __shared__ __align__(128) unsigned char smem[];
-    if (DOWN && a.summary && *a.summary) return;  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
-    u32 n_union = a.routes.counts[0];
-    if (n_union == 0) return;
-    if (n_union > plan.max_union) n_union = plan.max_union;
+    // An early launch makes its list and asks for the weights of its groups' first items before it waits for the launch in front. Every path waits.
+    const bool early = plan.early;
     u32* claim = a.routes.counts + 3;  // the grid's claim word (wide_common.cuh)
 
     unsigned char* at = smem + kGroups * plan.stages * plan.stage_bytes;
@@ -256,10 +256,17 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     if (tid < 4) ctl[tid] = 0;
     if (tid < kGroups * plan.stages + 2 * kGroups) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 
+    if (!early) chain_begin();
+    if (DOWN && !early && a.summary && *a.summary) return;  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
+
     // ---- the virtual expert list (the stage area is free until the first copy is issued: it holds the copied routes)
-    build_work_list(a.routes, n_union, plan.max_union, plan.vmax, plan.n_chunks, reinterpret_cast<u32*>(smem), table, ctl);
+    if (plan.dense_rows) build_dense_list(plan.dense_rows, plan.n_chunks, table, ctl);
+    else build_work_list(a.routes, plan.n_bound ? plan.n_bound : min(load_l2(a.routes.counts), plan.max_union), plan.max_union, plan.vmax, plan.n_chunks, reinterpret_cast<u32*>(smem), table, ctl);
     const u32 n_items = ctl[3];
-    if (n_items == 0) return;  // every CTA alike: nobody claims, the claim word stays zero
+    if (n_items == 0) {  // every CTA alike: nobody claims, the claim word stays zero
+        if (early) chain_begin();
+        return;
+    }
 
     // ------------------------------------------------------------------------------------------ producer warps
     if (warp >= kConsumerWarps) {
@@ -272,6 +279,38 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, in_gs = in_stride / 32;
         u32 t = 0, slot = 0, use = 0;  // stage count, ring position, lap
         bool ok = true, first = true;
+        auto ask_weights = [&](u32 s, const VExpert& ve, u32 chunk, unsigned char* dst, u64* bar) {  // one lane
+            const u32 x = s * G::S * (kQ4KBlock / 8);  // 64-bit elements: a multiple of 18, i.e. of 144 bytes
+            const u32 y = ve.expert() * a.rows_per_expert + (DOWN ? kItemRows : kHalfRows) * chunk;
+            tma_2d(dst, &tm0, x, y, bar);
+            tma_2d(dst + G::half_bytes, &tm1, x, DOWN ? y + kHalfRows : y, bar);
+        };
+        u32 ahead = 0;  // stages of the first item whose weights were asked for before the wait
+        if (early) {
+            const u32 k = g * gridDim.x + blockIdx.x;
+            if (k < n_items) {
+                ahead = min(plan.nseg, plan.stages);
+                if (g == 0) ahead = min(ahead, plan.stall_stage);
+                if (lane == 0) {
+                    const u32 jv = k / plan.n_chunks;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the list was made in the stages' memory
+                    for (u32 s = 0; s < ahead; ++s) {
+                        mbar_expect_more(&g_full[s], G::w_bytes);
+                        ask_weights(s, table[jv], k - jv * plan.n_chunks, g_stage + s * plan.stage_bytes, &g_full[s]);
+                    }
+                }
+            }
+            chain_begin();
+            if (DOWN && a.summary && *a.summary) {  // the stage is skipped: the weights land (the wait is bounded) before the CTA retires
+                if (lane == 0) {
+                    for (u32 s = 0; s < ahead; ++s) mbar_arrive(&g_full[s]);
+                    for (u32 s = 0; s < ahead; ++s)
+                        for (u32 i = 0; i < (plan.wait_limit >> 4) + 64u; ++i)
+                            if (mbar_try_wait(&g_full[s], 0)) break;
+                }
+                return;
+            }
+        }
         for (;;) {
             // A group's first item needs no round trip: group 0 of CTA b takes item b, group 1 item gridDim.x + b - so a
             // launch with fewer items than groups runs one group per SM, which has the SM's issue slots to itself.
@@ -292,7 +331,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             }
             const u32 ve_ne = ve.ne();
             u32 r = 0;
-            if (e < ve_ne) r = load((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
+            if (e < ve_ne) r = plan.dense_rows ? ve.begin() + e : load((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
             const u32 nsegs = end ? 1u : plan.nseg;
             for (u32 s = 0; s < nsegs; ++s, ++t, ++slot) {
                 if (slot == plan.stages) { slot = 0; ++use; }
@@ -309,15 +348,10 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 unsigned char* dst = g_stage + slot * plan.stage_bytes;
                 if (lane == 0) {
                     g_item[slot] = item;
-                    mbar_expect_tx(&g_full[slot], G::w_bytes + ve_ne * nbk * 320u);  // whole boxes: what lies past the row is filled
+                    mbar_expect_tx(&g_full[slot], (t < ahead ? 0u : G::w_bytes) + ve_ne * nbk * 320u);  // whole boxes: what lies past the row is filled
                 }
                 __syncwarp();
-                if (lane == 0) {
-                    const u32 x = s * G::S * (kQ4KBlock / 8);  // 64-bit elements: a multiple of 18, i.e. of 144 bytes
-                    const u32 y = ve.expert() * a.rows_per_expert + (DOWN ? kItemRows : kHalfRows) * chunk;
-                    tma_2d(dst, &tm0, x, y, &g_full[slot]);
-                    tma_2d(dst + G::half_bytes, &tm1, x, DOWN ? y + kHalfRows : y, &g_full[slot]);
-                }
+                if (lane == 0 && t >= ahead) ask_weights(s, ve, chunk, dst, &g_full[slot]);
                 if (e < ve_ne) {
                     unsigned char* xd = dst + G::w_bytes + e * G::x_entry_bytes;
                     if (part == 0) bulk_g2s(xd, a.in.codes + u64(r) * in_stride + u64(s) * G::S * 256u, nbk * 256u, &g_full[slot]);
@@ -337,6 +371,10 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     }
 
     // ------------------------------------------------------------------------------------------ consumer warps
+    if (early) {
+        chain_begin();
+        if (DOWN && a.summary && *a.summary) return;
+    }
     const u32 g = warp / kGroupWarps, w = warp % kGroupWarps;
     const u32 p = lane >> 3, rr = lane & 7u;     // dp4a form: lane = (pair, one of the warp's 8 rows)
     const u32 mp = w & 3u, half = w >> 2;        // mma form: the warp's chain and half of the item
@@ -360,7 +398,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         const VExpert ve = table[jv];
         const u32 ne = ve.ne(), vbegin = ve.begin();
         const bool mma = ne > kDpEntries;
-        const u32 slot_id = w < ne ? load(a.routes.slots + vbegin + w) : 0u;  // asked for before the stages, used behind them
+        const u32 slot_id = w >= ne ? 0u : plan.dense_rows ? vbegin + w : load(a.routes.slots + vbegin + w);  // asked for before the stages, used behind them
         // the item's stages, with the form fixed at compile time inside the loop
         auto stages = [&](auto step) {
             for (u32 s = 0; s < plan.nseg; ++s) {
@@ -407,7 +445,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             });
         };
         if (!mma) {
-            const u32 only_slot = DOWN ? load(a.routes.slots + vbegin) : 0u;
+            const u32 only_slot = !DOWN ? 0u : plan.dense_rows ? vbegin : load(a.routes.slots + vbegin);
             float acc = 0.0f;
             stages([&](const unsigned char* st, u32 nbk) { stage_row<G>(st + half * G::half_bytes + (8u * mp + rr) * G::row_bytes, nbk, p, st + G::w_bytes, acc); });
             if (!ok) break;
@@ -446,7 +484,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 const bool bad = __any_sync(0xffffffffu, !finite_f(gv) || !finite_f(uv) || !finite_f(h));
                 if (bad) {  // fail closed: nothing of the group is written (routed_expert.cpp:147-156)
                     if (lane == 0) {
-                        if (a.row_status) atomicOr(&a.row_status[load(a.routes.rows + vbegin + w)], B200MOE_ROW_PROJECTION_NONFINITE);
+                        if (a.row_status) atomicOr(&a.row_status[plan.dense_rows ? vbegin + w : load(a.routes.rows + vbegin + w)], B200MOE_ROW_PROJECTION_NONFINITE);
                         if (a.summary) atomicOr(a.summary, B200MOE_ROW_PROJECTION_NONFINITE);
                     }
                 } else {
@@ -525,12 +563,13 @@ bool wide_down_fits(const b200moe_down_view& v, u32 rows) {
            make_plan(v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, &p);
 }
 
-int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_t stream) {
+int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     WidePlan p{};
     if (!make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, &p))
         return fail(B200MOE_ERR_UNSUPPORTED, "gate_up: the segment-streaming form does not apply to this shape");
     apply_hooks(&p);
+    p.early = hints.routes_done || hints.dense_rows; p.dense_rows = hints.dense_rows; p.n_bound = static_cast<u32>(std::min<u64>(v.max_union, hints.slots));
     WideArgs a{};
     a.routes = v.routes; a.in = v.x; a.act = v.act; a.gate_out = v.gate_out; a.up_out = v.up_out;
     a.row_status = v.row_status; a.summary = v.summary; a.rows_per_expert = v.shape.inter; a.out_width = v.shape.inter;
@@ -549,12 +588,13 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_
     return after_launch("gate_up_q4k_wide");
 }
 
-int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, cudaStream_t stream) {
+int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     WidePlan p{};
     if (!make_plan(v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, &p))
         return fail(B200MOE_ERR_UNSUPPORTED, "down: the segment-streaming form does not apply to this shape");
     apply_hooks(&p);
+    p.early = hints.routes_done || hints.dense_rows; p.dense_rows = hints.dense_rows; p.n_bound = static_cast<u32>(std::min<u64>(v.max_union, hints.slots));
     WideArgs a{};
     a.routes = v.routes; a.in = v.act; a.raw = v.raw; a.summary = const_cast<u32*>(v.summary);
     a.rows_per_expert = v.shape.hidden; a.out_width = v.shape.hidden; a.raw_vec = aligned(v.raw, 8);

@@ -38,7 +38,7 @@ __device__ __forceinline__ void run_load(const u8* src, u32 nb, u32 lane, RunReg
     const uint4* s4 = reinterpret_cast<const uint4*>(src);
     const u32 n16 = nb * kQ8Block / 16;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) if (lane + 32u * k < n16) r.v[k] = load(s4 + lane + 32u * k);
+    for (int k = 0; k < 3; ++k) if (lane + 32u * k < n16) r.v[k] = __ldcg(s4 + lane + 32u * k);  // past the L1 cache: read once, and by an early launch before its wait
 }
 __device__ __forceinline__ void run_store(u32* stage, u32 nb, u32 lane, const RunRegs& r) {
     uint4* d4 = reinterpret_cast<uint4*>(stage);
@@ -237,18 +237,21 @@ __global__ void __launch_bounds__(1024) gate_up_q8_kernel(b200moe_gate_up_view v
 }
 
 // Routed down: grid (hidden / 32, max_union); 256 threads.
-__global__ void __launch_bounds__(1024) down_q8_kernel(b200moe_down_view v, u32 align) {
-    chain_begin();
+__global__ void __launch_bounds__(1024) down_q8_kernel(b200moe_down_view v, u32 align, u32 early) {
+    // An early launch (ChainHints) asks for its warps' first weight rows before it waits for the launch in front. Every path waits.
+    if (!early) chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (v.summary && *v.summary) return;
     const u32 j = blockIdx.y, nw = blockDim.x >> 5;
-    if (j >= v.routes.counts[0]) return;
+    if (j >= load_l2(v.routes.counts)) {
+        if (early) chain_begin();
+        return;
+    }
     const u32 H = v.shape.hidden, I = v.shape.inter, groups = I / 32;
     i8* s_codes = reinterpret_cast<i8*>(smem_raw);
     float* s_deltas = reinterpret_cast<float*>(smem_raw + u64(kR) * I);
     u32* s_stage = reinterpret_cast<u32*>(s_deltas + kR * groups);
     __shared__ u32 s_slots[kR];
-    const u32 expert = v.routes.experts[j], eb = v.routes.begins[j], ee = v.routes.begins[j + 1];
+    const u32 expert = load_l2(v.routes.experts + j), eb = load_l2(v.routes.begins + j), ee = load_l2(v.routes.begins + j + 1);
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     u32* stage = s_stage + warp * (kStageBytes / 4);
     const u64 row_bytes = u64(groups) * kQ8Block;
@@ -261,6 +264,8 @@ __global__ void __launch_bounds__(1024) down_q8_kernel(b200moe_down_view v, u32 
         run_load(down + u64(warp) * row_bytes, min(32u, groups), lane, pre);
         have_pre = true;
     }
+    if (early) chain_begin();
+    if (v.summary && *v.summary) return;
     for (u32 p0 = eb + kR * blockIdx.z; p0 < ee; p0 += kR * gridDim.z) {  // grid.z shares an expert's passes of kR entries
         const int nr = static_cast<int>(min(u32(kR), ee - p0));
         __syncthreads();
@@ -317,14 +322,14 @@ int launch_gate_up_q8(const b200moe_gate_up_view& v, cudaStream_t stream) {
     return after_launch("gate_up_q8");
 }
 
-int launch_down_q8(const b200moe_down_view& v, cudaStream_t stream) {
+int launch_down_q8(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     const u32 H = v.shape.hidden, I = v.shape.inter;
     const u32 align = (aligned(v.weights.down, 16) && (I / 32 * kQ8Block) % 16 == 0) ? 16u : 2u;
     const u32 nw = kRoutedWarps;   // 32 weight rows per CTA: one per warp, every row of the expert in flight at once
     const u32 smem = kR * (I + I / 32 * 4) + nw * kStageBytes;
     if (int rc = set_smem(down_q8_kernel, smem)) return rc;
-    chain_launch(down_q8_kernel, dim3(H / 32, v.max_union, pass_split(H / 32 * v.max_union, v.act.rows)), nw * 32, smem, stream, v, align);
+    chain_launch(down_q8_kernel, dim3(H / 32, v.max_union, pass_split(H / 32 * v.max_union, v.act.rows)), nw * 32, smem, stream, v, align, u32(hints.routes_done));
     return after_launch("down_q8");
 }
 

@@ -5,6 +5,12 @@
 
 namespace b200moe {
 
+// What a caller that composes the launches of a layer knows about those in front of one. routes_done: the routes were complete before the launch in
+// front was admitted (chain_begin), so they and the weights may be read before the wait. dense_rows: the launch belongs to a dense block of so many
+// rows (entry i is row i and slot i of the only expert), whose weights were complete before the launch in front was admitted. slots: the routes'
+// arrays hold so many entries, whatever the union is (0: not known).
+struct ChainHints { bool routes_done; u32 dense_rows; u64 slots; };
+
 // a8.cu
 // wide (optional, only with bfloat16 x and quantize_a8_vec_ok): the values as FP32 rows of wide_stride, 16-byte aligned
 bool quantize_a8_vec_ok(const b200moe_quantize_a8_view& v);
@@ -36,7 +42,7 @@ int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view
 // gemv_q8.cu: Q8_0 x A8 products in the 32-lane-class contract (dense rows and the routed DS41-family experts)
 int launch_q8_0_a8(const b200moe_q8a8_view& v, cudaStream_t stream);
 int launch_gate_up_q8(const b200moe_gate_up_view& v, cudaStream_t stream);
-int launch_down_q8(const b200moe_down_view& v, cudaStream_t stream);
+int launch_down_q8(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream);
 
 // gemv_q4k.cu: Q4_K x A8 rows in the four-chain contract (routed Qwen-family experts; Q8_0 four-chain down)
 int launch_gate_up_q4k(const b200moe_gate_up_view& v, cudaStream_t stream);
@@ -50,14 +56,14 @@ int launch_down_q8_chain4(const b200moe_down_view& v, cudaStream_t stream);
 bool stream_gate_up_fits(const b200moe_gate_up_view& v, u32 rows);
 bool stream_down_fits(const b200moe_down_view& v, u32 rows);
 int launch_gate_up_q4k_stream(const b200moe_gate_up_view& v, u32 rows, cudaStream_t stream);
-int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, cudaStream_t stream);
+int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
 
 // gemv_q4k_wide.cu: the same contracts with SEGMENTS of the rows (and of the entries' A8 rows) streamed by TMA: any row
 // length, windows of any size whose routes fit shared memory
 bool wide_gate_up_fits(const b200moe_gate_up_view& v, u32 rows);
 bool wide_down_fits(const b200moe_down_view& v, u32 rows);
-int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_t stream);
-int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, cudaStream_t stream);
+int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
+int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
 // gemv_q8_wide.cu: the Q8_0 x A8 lane-class contract in the same streaming skeleton, for windows of many rows.
 bool q8_wide_gate_up_fits(const b200moe_gate_up_view& v, u32 rows);
 bool q8_wide_down_fits(const b200moe_down_view& v, u32 rows);

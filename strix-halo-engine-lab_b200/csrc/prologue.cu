@@ -73,14 +73,15 @@ __global__ void __launch_bounds__(32 * (int(kBlockExperts) / EW) * (RT / RW)) pr
     for (int e = 0; e < EW; ++e)
 #pragma unroll
         for (int r = 0; r < RW; ++r) acc[e][r] = 0.0f;
-    // The copies come from short rolled loops: every request of the run is in flight at once, and the code stays small (the kernel runs once a call on
-    // cold instruction caches, where straight-line code pays a fetch a line).
-    auto copy_row = [&](u32 row, const float* src, u32 n, bool vec) {  // n values to row `row`, all threads
-        const u32 dst = smem_addr(xs + row);
+    // A warp copies the group's columns of one row at a time; every request of the run is in flight at once.
+    auto copy_row = [&](u32 to, const float* src, u32 n, bool vec) {  // n values to xs[to ..]
+        const u32 dst = smem_addr(xs + to);
         if (vec) {
-            for (u32 i = threadIdx.x; i < n / 4; i += kThreads) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(src + 4u * i) : "memory");
+#pragma unroll
+            for (u32 i = 0; i < kGroupElems / 128; ++i)
+                if (lane + 32u * i < n / 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (lane + 32u * i)), "l"(src + 4u * (lane + 32u * i)) : "memory");
         } else {
-            for (u32 i = threadIdx.x; i < n; i += kThreads) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * i), "l"(src + i) : "memory");
+            for (u32 i = lane; i < n; i += 32) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * i), "l"(src + i) : "memory");
         }
     };
     for (u32 c0 = 0; c0 < H; c0 += kRunElems) {
@@ -90,10 +91,10 @@ __global__ void __launch_bounds__(32 * (int(kBlockExperts) / EW) * (RT / RW)) pr
         for (u32 g0 = 0; g0 < kRunElems; g0 += kGroupElems) {
             const u32 n = g0 < n_el ? min(kGroupElems, n_el - g0) : 0u;
 #pragma unroll 1
-            for (u32 e = 0; e < kBlockExperts; ++e) copy_row((RT + e) * kRunElems + g0, rv.weight + u64(min(e_base + e, E - 1)) * H + c0 + g0, n, a.w_vec);
-            if (!bf16) {
-#pragma unroll 1
-                for (u32 r = 0; r < rows; ++r) copy_row(r * kRunElems + g0, x32 + u64(r) * x_stride + c0 + g0, n, a.x_vec);
+            for (u32 j = warp; j < kBlockExperts + (bf16 ? 0u : rows); j += kWarps) {
+                const bool is_w = j < kBlockExperts;
+                const float* src = is_w ? rv.weight + u64(min(e_base + j, E - 1)) * H : x32 + u64(j - kBlockExperts) * x_stride;
+                copy_row((is_w ? RT + j : j - kBlockExperts) * kRunElems + g0, src + c0 + g0, n, is_w ? a.w_vec : a.x_vec);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         }

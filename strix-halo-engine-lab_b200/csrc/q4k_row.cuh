@@ -24,6 +24,10 @@ __device__ __forceinline__ void mbar_arrive(u64* bar) {
 __device__ __forceinline__ void mbar_expect_tx(u64* bar, u32 bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(bar)), "r"(bytes) : "memory");
 }
+// Bytes to come, without an arrival: the phase completes with them and the arrivals.
+__device__ __forceinline__ void mbar_expect_more(u64* bar, u32 bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(bytes) : "memory");
+}
 // One poll. The instruction may suspend the warp until the phase completes or `hint_ns` nanoseconds have passed: a waiting
 // warp then issues nothing, instead of spinning in the issue slots that the working warps of its scheduler need.
 __device__ __forceinline__ bool mbar_try_wait(u64* bar, u32 parity, u32 hint_ns = 0) {

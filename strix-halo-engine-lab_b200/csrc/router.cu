@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(128) router_select_kernel(const float* logits,
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const u32 row = blockIdx.x * 4u + warp;
     if (row >= rows) return;
-    select_detail::select_row(logits, scores_out, bias, p, row, lane, smem + warp * select_detail::scratch_floats(p.experts), ids, weights);
+    select_detail::select_row<1024>(logits, scores_out, bias, p, row, lane, smem + warp * select_detail::scratch_floats(p.experts), ids, weights);
 }
 
 }  // namespace

@@ -238,6 +238,8 @@ __device__ __forceinline__ void finish_row(const b200moe_route_policy& p, u32 ro
 
 // One warp selects one row. `s` points to this warp's scratch of 2 * experts + 32 floats on a 16-byte boundary (shared memory).
 __host__ __device__ constexpr u32 scratch_floats(u32 experts) { return (2u * experts + 32u + 3u) & ~3u; }
+// MAXE: the most experts that the calling kernel sees.
+template <u32 MAXE>
 __device__ __forceinline__ void select_row(const float* logits, float* scores_out, const float* bias,
                                            const b200moe_route_policy& p, u32 row, u32 lane, float* s,
                                            u32* ids, float* weights, u32* ids_copy = nullptr) {
@@ -245,8 +247,8 @@ __device__ __forceinline__ void select_row(const float* logits, float* scores_ou
     if (p.n_group == 1 || run % 32 == 0 || (run < 32 && (run & (run - 1u)) == 0)) {  // the fast path unless a NaN needs the serial rule
         u32 my_id = kNone;
         const bool done = E <= 128 ? select_row_fast<4>(logits, scores_out, bias, p, row, lane, s, &my_id)
-                        : E <= 256 ? select_row_fast<8>(logits, scores_out, bias, p, row, lane, s, &my_id)
-                                   : select_row_fast<32>(logits, scores_out, bias, p, row, lane, s, &my_id);
+                        : MAXE <= 256 || E <= 256 ? select_row_fast<8>(logits, scores_out, bias, p, row, lane, s, &my_id)
+                                   : select_row_fast<MAXE <= 256 ? 8 : 32>(logits, scores_out, bias, p, row, lane, s, &my_id);
         if (done) {
             finish_row(p, row, lane, s, my_id, ids, weights, ids_copy);
             return;

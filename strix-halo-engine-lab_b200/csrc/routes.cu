@@ -36,16 +36,18 @@ __global__ void __launch_bounds__(1024) routes_small_kernel(b200moe_routes_view 
 }
 
 // Decode windows: the router's selection (one warp per row) and the routes of the selected ids in ONE block, so the
-// layer prologue costs one launch less. Dynamic shared memory: the rows' selection scratch, then the routes' counts in its place.
-__global__ void __launch_bounds__(1024) select_routes_small_kernel(const float* logits, float* scores_out, const float* bias,
-                                                                   b200moe_route_policy p, u32 rows, u32* ids, float* weights,
-                                                                   b200moe_routes_view rv, u32 end, Clear clear) {
+// layer prologue costs one launch less. Dynamic shared memory: the rows' selection scratch, then the routes' counts in its place. Up to 256 experts
+// (their keys fit the 64 registers that a block of 1024 threads has) and 8 rows in the form of 256 threads.
+template <u32 THREADS>
+__global__ void __launch_bounds__(THREADS) select_routes_small_kernel(const float* logits, float* scores_out, const float* bias,
+                                                                      b200moe_route_policy p, u32 rows, u32* ids, float* weights,
+                                                                      b200moe_routes_view rv, u32 end, Clear clear) {
     extern __shared__ __align__(16) float sel_smem[];
     __shared__ u32 s_ids[kChunk];
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     chain_begin();
     routes_detail::clear_words(clear, rows);
-    if (warp < rows) select_detail::select_row(logits, scores_out, bias, p, warp, lane, sel_smem + warp * select_detail::scratch_floats(p.experts), ids, weights, s_ids);
+    if (warp < rows) select_detail::select_row<256>(logits, scores_out, bias, p, warp, lane, sel_smem + warp * select_detail::scratch_floats(p.experts), ids, weights, s_ids);
     __syncthreads();  // the ids are read by the whole block
     routes_small_body(rv, end, s_ids, reinterpret_cast<u16*>(sel_smem));
 }
@@ -151,14 +153,16 @@ u64 routes_scratch_words(u32 rows, u32 top_k, u32 experts) {
 u32 small_threads(u32 slots, u32 experts) { return std::min(1024u, std::max(256u, (std::max(slots, experts) + 31u) / 32u * 32u)); }
 
 bool select_routes_fusable(const b200moe_router_view& r, u32 top_k) {
-    return r.rows <= 32 && u64(r.rows) * top_k <= kChunk && u64(r.rows) * select_detail::scratch_floats(r.policy.experts) * 4u <= 96u * 1024u;
+    return r.rows <= 32 && u64(r.rows) * top_k <= kChunk && r.policy.experts <= 256 && u64(r.rows) * select_detail::scratch_floats(r.policy.experts) * 4u <= 96u * 1024u;
 }
 int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view& v, const RoutesClear& clear, cudaStream_t stream) {
     if (r.rows == 0) return B200MOE_OK;
     const u32 n = v.rows * v.top_k, smem = std::max(r.rows * select_detail::scratch_floats(r.policy.experts) * 4u, counts_bytes(n, v.experts));
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(select_routes_small_kernel), smem)) return rc;
-    chain_launch(select_routes_small_kernel, 1, std::max(32u * r.rows, small_threads(n, v.experts)), smem, stream, r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights,
-                 v, v.end ? v.end : v.experts, Clear{clear.row_status, clear.summary4, clear.summary});
+    const u32 threads = std::max(32u * r.rows, small_threads(n, v.experts));
+    const auto kernel = threads <= 256u ? select_routes_small_kernel<256> : select_routes_small_kernel<1024>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
+    chain_launch(kernel, 1, threads, smem, stream, r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights, v, v.end ? v.end : v.experts,
+                 Clear{clear.row_status, clear.summary4, clear.summary});
     return after_launch("select_routes_small");
 }
 

@@ -55,18 +55,19 @@ __device__ __forceinline__ void retire_claims(u32* claim, u32* ctl) {
 // table order, so the long items start first and the kernel's tail is made of short ones. ctl[3] = items (virtual expert
 // major x n_chunks chunks). Every CTA builds the same list. `scratch` is shared memory that is free until the first copy is
 // issued (work_list_scratch_words(max_union, vmax) words). Every thread of the block calls it; it holds four block barriers.
-// n_union <= max_union; the block has at least kKE warps.
-__device__ __forceinline__ void build_work_list(const b200moe_routes& routes, u32 n_union, u32 max_union, u32 vmax, u32 n_chunks, u32* scratch,
+// n_bound <= max_union bounds the union (and the routes' arrays: slots of the window); the block has at least kKE warps.
+__device__ __forceinline__ void build_work_list(const b200moe_routes& routes, u32 n_bound, u32 max_union, u32 vmax, u32 n_chunks, u32* scratch,
                                                 VExpert* table, u32* ctl) {
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     u32* t_beg = scratch;
     u32* t_exp = t_beg + max_union + 1;
     VExpert* unsorted = reinterpret_cast<VExpert*>(t_exp + max_union);
     u32* s_hist = reinterpret_cast<u32*>(unsorted + vmax);
-    for (u32 j = tid; j <= n_union; j += blockDim.x) {
-        t_beg[j] = load(routes.begins + j);
-        if (j < n_union) t_exp[j] = load(routes.experts + j);
+    for (u32 j = tid; j <= n_bound; j += blockDim.x) {  // together with the count: one trip to memory instead of two
+        t_beg[j] = load_l2(routes.begins + j);
+        if (j < n_bound) t_exp[j] = load_l2(routes.experts + j);
     }
+    const u32 n_union = min(load_l2(routes.counts), n_bound);
     __syncthreads();
     if (warp == 0) {
         u32 n_virtual = 0;
@@ -102,6 +103,14 @@ __device__ __forceinline__ void build_work_list(const b200moe_routes& routes, u3
             pos += __popc(m);
         }
     }
+    __syncthreads();
+}
+
+// The list of a dense block: its rows are the entries of expert 0, in order.
+__device__ __forceinline__ void build_dense_list(u32 rows, u32 n_chunks, VExpert* table, u32* ctl) {
+    const u32 n_virtual = (rows + kKE - 1) / kKE;
+    for (u32 j = threadIdx.x; j < n_virtual; j += blockDim.x) table[j] = VExpert::make(0, j * kKE, min(kKE, rows - j * kKE));
+    if (threadIdx.x == 0) { ctl[2] = n_virtual; ctl[3] = n_virtual * n_chunks; }
     __syncthreads();
 }
 

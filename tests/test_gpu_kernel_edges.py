@@ -724,3 +724,53 @@ def test_decode_front(gpu, oracle, rows, hidden, experts, offset, bf16):
         y, ids, wts = ffn(x, want_routes=True, row_status=status, summary=summary)
         assert np.array_equal(ids.cpu().numpy().view(np.uint32), want["ids"]) and same(y.cpu(), want["y"])
         assert int(summary[0]) == 0 and not status.any()
+
+
+@pytest.mark.parametrize("H,I", [(256, 512), (512, 256), (768, 1024), (1024, 768), (1280, 1536)])
+def test_segment_streaming_entry_counts(gpu, oracle, H, I):
+    """Experts of 1 to 9 and 17 entries (one, a few, many a tile; several items an expert), rows of 1 to 6 super-blocks (whole stages and remainders)."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(H + I)
+    counts = [1, 2, 3, 4, 5, 6, 7, 8, 9, 17]
+    E, rows = len(counts), max(counts)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+    ids = np.concatenate([np.full(n, e) for e, n in enumerate(counts)]).astype(np.uint32)[:, None]
+    rng.shuffle(ids)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((len(ids), H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, 12, 12, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, 1, 12, 12)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    with forced(b200moe.FORM_SEGMENT_STREAM):
+        act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), len(ids), taps=True)
+        assert b200moe.last_launch() == "gate_up_q4k_wide"
+        raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+        assert b200moe.last_launch() == "down_q4k_wide"
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("rows,H,I,form", [(1, 512, 512, "FORM_ROW_STREAM"), (2, 512, 2048, "FORM_ROW_STREAM"), (1, 512, 5120, "FORM_SEGMENT_STREAM"), (9, 2560, 512, "FORM_SEGMENT_STREAM")])
+def test_down_skipped_after_its_weights_were_asked_for(gpu, oracle, rows, H, I, form):
+    """A dense block, whose down asks for weights before gate/up has finished: a projection that is not finite skips it (y stays as it was), the next
+    call gives the oracle's bits; the same for the routed layer, whose rows all fail."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, 1, H, I, 12, 12)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    bad = deltas.copy()
+    bad[rows - 1, 0] = np.inf
+    want = oracle.experts(O.Shape(H, I, 1, 1, 12, 12, float("inf")), gate, up, down, np.zeros((rows, 1), np.uint32), codes, deltas, sums)
+    sh = ops.make_shape(H, I, 1, 1, 12, 12)
+    w = dv(gate, gpu), dv(up, gpu), dv(down, gpu)
+    layer = ops.MoeLayer(sh, *w, capacity=rows, combine_form=b200moe.COMBINE_FMA_SLOTS)
+    ids, one = torch.zeros((rows, 1), dtype=torch.int32, device=gpu), torch.ones((rows, 1), device=gpu)
+    with forced(getattr(b200moe, form)):
+        for _ in range(3):
+            fail, good = ((dv(codes, gpu), dv(d, gpu), dv(sums, gpu)) for d in (bad, deltas))
+            assert not ops.enqueue_dense_ffn(sh, *w, fail).any()
+            assert same(ops.enqueue_dense_ffn(sh, *w, good).cpu(), want["raw"])
+            status = torch.zeros(rows, dtype=torch.int32, device=gpu)
+            y = layer(fail, ids, one, row_status=status)
+            assert int(status[rows - 1]) == b200moe.ROW_PROJECTION_NONFINITE and not y[rows - 1].any()
+            assert same(layer(good, ids, one).cpu(), want["raw"])

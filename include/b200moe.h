@@ -446,6 +446,9 @@ typedef struct b200moe_layer_view {
 } b200moe_layer_view;
 uint64_t b200moe_layer_workspace_bytes(const b200moe_shape* shape, uint32_t capacity);
 int b200moe_layer(const b200moe_layer_view* view, void* stream);
+/* The same over outputs that were not initialised: rows of y and y_bf16 that b200moe_layer leaves as they were - those of a
+ * failed row, all of an aborted job - are set to zero (without y_blocks). */
+int b200moe_layer_fresh(const b200moe_layer_view* view, void* stream);
 
 /* Router + A8 + layer from FP32 (or bfloat16) activations: one token block through the whole FFN. */
 typedef struct b200moe_ffn_view {
@@ -495,6 +498,8 @@ typedef struct b200moe_dense_view {
     uint64_t workspace_bytes;     /* b200moe_layer_workspace_bytes(shape, rows) */
 } b200moe_dense_view;
 int b200moe_dense_ffn(const b200moe_dense_view* view, void* stream);
+/* The same over a y that was not initialised: what b200moe_dense_ffn leaves as it was is set to zero. */
+int b200moe_dense_ffn_fresh(const b200moe_dense_view* view, void* stream);
 
 /* ------------------------------------------------------------------------------------------ tensor parallelism, one call
  * The dense block under tensor parallelism behind one enqueue-only call: the rank's share of b200moe_dense_ffn (gate / up

@@ -22,8 +22,8 @@ def enqueue_quantize_a8(x, status=None, stride=0):
     """x [rows][width] float32 or bfloat16 -> (codes int8, deltas float32, sums int32)."""
     rows, width = x.shape
     st = stride or width
-    codes = torch.empty((rows, st), dtype=torch.int8, device=x.device)
-    deltas = torch.empty((rows, st // 32 if st % 32 == 0 else 1), dtype=torch.float32, device=x.device)
+    codes = x.new_empty((rows, st), dtype=torch.int8)
+    deltas = x.new_empty((rows, st // 32 if st % 32 == 0 else 1), dtype=torch.float32)
     sums = torch.empty_like(deltas, dtype=torch.int32)
     v = QuantizeA8View(ptr(x), rows, width, x.stride(0), int(x.dtype == torch.bfloat16),
                        A8Rows(ptr(codes), ptr(deltas), ptr(sums), rows, width, st), ptr(status))
@@ -35,11 +35,11 @@ def enqueue_rmsnorm_a8(x, weight=None, eps=1e-6, want_out=True, want_a8=True, st
     """x [rows][n] float32 -> (y float32 or None, (codes, deltas, sums) or None): RMSNorm and the A8 of its output in one launch."""
     from . import RmsnormView
     rows, n = x.shape
-    y = torch.empty((rows, n), dtype=torch.float32, device=x.device) if want_out else None
+    y = x.new_empty((rows, n), dtype=torch.float32) if want_out else None
     a8, rows_view = None, A8Rows()
     if want_a8:
-        codes = torch.empty((rows, n), dtype=torch.int8, device=x.device)
-        deltas = torch.empty((rows, max(n // 32, 1)), dtype=torch.float32, device=x.device)
+        codes = x.new_empty((rows, n), dtype=torch.int8)
+        deltas = x.new_empty((rows, max(n // 32, 1)), dtype=torch.float32)
         sums = torch.empty_like(deltas, dtype=torch.int32)
         a8, rows_view = (codes, deltas, sums), A8Rows(ptr(codes), ptr(deltas), ptr(sums), rows, n, n)
     v = RmsnormView(ptr(x), rows, n, x.stride(0), ptr(weight), eps, ptr(y), 0, rows_view, ptr(status))
@@ -64,13 +64,12 @@ def enqueue_router(policy, x=None, weight=None, logits=None, logit_bias=None, bi
     """Returns (logits, scores, ids, weights). Either x and weight, or logits."""
     if x is not None:
         rows, hidden = x.shape
-        logits = torch.empty((rows, policy.experts), dtype=torch.float32, device=x.device)
+        logits = x.new_empty((rows, policy.experts), dtype=torch.float32)
     else:
         rows, hidden = logits.shape[0], 0
-    dev = logits.device
     scores = torch.empty_like(logits)
-    ids = torch.empty((rows, policy.top_k), dtype=torch.int32, device=dev)
-    wts = torch.empty((rows, policy.top_k), dtype=torch.float32, device=dev)
+    ids = logits.new_empty((rows, policy.top_k), dtype=torch.int32)
+    wts = torch.empty_like(ids, dtype=torch.float32)
     v = RouterView(ptr(x), x.stride(0) if x is not None else 0, rows, hidden, ptr(weight), ptr(logit_bias), ptr(bias), policy,
                    ptr(logits), ptr(scores), ptr(ids), ptr(wts))
     check(lib().b200moe_router(C.byref(v), stream_ptr()))
@@ -165,14 +164,15 @@ class MoeLayer:
         there (peer buffers under expert parallelism) and no y is returned."""
         rows = ids.shape[0]
         dev = self.gate.device
-        y = torch.zeros((rows, self.shape.hidden), dtype=torch.float32, device=dev) if combine and y_blocks is None else None
-        yb = torch.zeros((rows, self.shape.hidden), dtype=torch.bfloat16, device=dev) if bf16 else None
+        fresh = combine and y_blocks is None  # the call itself leaves zeros where it writes nothing
+        y = self.gate.new_empty((rows, self.shape.hidden), dtype=torch.float32) if fresh else None
+        yb = (self.gate.new_empty if fresh else self.gate.new_zeros)((rows, self.shape.hidden), dtype=torch.bfloat16) if bf16 else None
         raw = torch.zeros((rows * self.shape.top_k, self.shape.hidden), dtype=torch.float32, device=dev) if want_raw else None
         v = LayerView(self.shape, ExpertWeights(ptr(self.gate), ptr(self.up), ptr(self.down)), rows, a8_rows(*x_a8), ptr(ids),
                       ptr(route_weights), ptr(shared), first, end, base, self.combine_form, self.parts, self.part_experts, only_part,
                       ptr(raw), ptr(y), ptr(yb), ptr(row_status), ptr(self.ws), self.ws_bytes, self.capacity, self.grouped_min_rows, None,
                       ptr(y_blocks), y_block_rows)
-        check(lib().b200moe_layer(C.byref(v), stream_ptr()))
+        check((lib().b200moe_layer_fresh if fresh else lib().b200moe_layer)(C.byref(v), stream_ptr()))
         out = [y]
         if want_raw:
             out.append(raw)
@@ -215,7 +215,7 @@ class MoeFfn:
         """x: [rows][hidden] float32 or bfloat16 (widened exactly before the router and the A8 quantiser)."""
         rows = x.shape[0]
         if y is None:
-            y = torch.empty((rows, self.shape.hidden), dtype=torch.float32, device=x.device)
+            y = x.new_empty((rows, self.shape.hidden), dtype=torch.float32)
         ids = torch.empty((rows, self.shape.top_k), dtype=torch.int32, device=x.device) if want_routes else None
         wts = torch.empty((rows, self.shape.top_k), dtype=torch.float32, device=x.device) if want_routes else None
         v = self._view(rows, x, y, ids, wts, shared, row_status, summary=summary)
@@ -231,13 +231,12 @@ class MoeFfn:
 
 def enqueue_dense_ffn(shape, gate, up, down, x_a8, bf16=False):
     rows = x_a8[0].shape[0]
-    dev = gate.device
     ws_bytes = int(lib().b200moe_layer_workspace_bytes(C.byref(shape), rows))
-    ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=dev)
-    y = torch.zeros((rows, shape.hidden), dtype=torch.float32, device=dev)
-    yb = torch.zeros((rows, shape.hidden), dtype=torch.bfloat16, device=dev) if bf16 else None
+    ws = gate.new_empty(max(ws_bytes, 256), dtype=torch.uint8)
+    y = gate.new_empty((rows, shape.hidden), dtype=torch.float32)  # the call itself leaves zeros where it writes nothing
+    yb = gate.new_empty((rows, shape.hidden), dtype=torch.bfloat16) if bf16 else None
     v = DenseView(shape, ExpertWeights(ptr(gate), ptr(up), ptr(down)), rows, a8_rows(*x_a8), ptr(y), ptr(yb), ptr(ws), ws_bytes)
-    check(lib().b200moe_dense_ffn(C.byref(v), stream_ptr()))
+    check(lib().b200moe_dense_ffn_fresh(C.byref(v), stream_ptr()))
     return (y, yb) if bf16 else y
 
 

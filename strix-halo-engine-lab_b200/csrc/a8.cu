@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256) widen_bf16_kernel(const u16* in, float* o
 int launch_widen_bf16(const u16* in, float* out, u64 count, cudaStream_t stream) {
     if (count == 0) return B200MOE_OK;
     const u32 blocks = static_cast<u32>(std::min<u64>((count + 255) / 256, 148u * 16u));
-    chain_launch(widen_bf16_kernel, blocks, 256, 0, stream, in, out, count);
+    small_launch(widen_bf16_kernel, blocks, 256, 0, stream, in, out, count);
     return after_launch("widen_bf16");
 }
 
@@ -116,16 +116,16 @@ int launch_quantize_a8(const b200moe_quantize_a8_view& v, cudaStream_t stream, f
     if (quantize_a8_vec_ok(v) && (wide || items > 8u * static_cast<u32>(device_sm_count()))) {
         const u32 vec_blocks = static_cast<u32>((items + 31) / 32);
         if (v.x_is_bf16)
-            chain_launch(quantize_a8_vec_kernel<true>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, wide, wide_stride);
+            small_launch(quantize_a8_vec_kernel<true>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, wide, wide_stride);
         else
-            chain_launch(quantize_a8_vec_kernel<false>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, nullptr, 0);
+            small_launch(quantize_a8_vec_kernel<false>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, nullptr, 0);
         return after_launch("quantize_a8");
     }
     const u32 blocks = static_cast<u32>((items + 7) / 8);
     if (v.x_is_bf16)
-        chain_launch(quantize_a8_kernel<true>, blocks, 256, 0, stream, v.x, v.rows, groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status);
+        small_launch(quantize_a8_kernel<true>, blocks, 256, 0, stream, v.x, v.rows, groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status);
     else
-        chain_launch(quantize_a8_kernel<false>, blocks, 256, 0, stream, v.x, v.rows, groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status);
+        small_launch(quantize_a8_kernel<false>, blocks, 256, 0, stream, v.x, v.rows, groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status);
     return after_launch("quantize_a8");
 }
 

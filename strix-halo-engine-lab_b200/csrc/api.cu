@@ -56,9 +56,14 @@ bool device_ready() {
     return ok;
 }
 
-int device_sm_count() {
+int device_sm_count() {  // asked of the runtime once a device
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];
     int dev = 0, n = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return n;
+    if (dev < kDevices && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+    n = 148;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && dev < kDevices) known[dev].store(n, std::memory_order_relaxed);
     return n;
 }
 
@@ -519,12 +524,13 @@ uint64_t b200moe_layer_workspace_bytes(const b200moe_shape* s, uint32_t capacity
     return carve_layer(nullptr, *s, capacity).bytes;
 }
 
-static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_ready);
-int b200moe_layer(const b200moe_layer_view* v, void* stream) { return layer_impl(v, stream, false); }
+static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_ready, bool fresh);
+int b200moe_layer(const b200moe_layer_view* v, void* stream) { return layer_impl(v, stream, false, false); }
+int b200moe_layer_fresh(const b200moe_layer_view* v, void* stream) { return layer_impl(v, stream, false, true); }
 
 // routes_ready: the caller (b200moe_ffn) has already built the routes of v->ids into this workspace and cleared the
-// status words (the fused select + routes launch of decode windows).
-static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_ready) {
+// status words (the fused select + routes launch of decode windows). fresh: rows that the call fails to write become zeros.
+static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_ready, bool fresh) {
     B200_REQUIRE(v, "null view");
     if (int rc = check_shape(v->shape)) return rc;
     const b200moe_shape& s = v->shape;
@@ -593,7 +599,7 @@ static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_rea
     cv.row_status = is_kquant(s.gate_type) ? row_status : nullptr;
     cv.summary = summary;
     tap(6);
-    const int rc = launch_combine(cv, st);
+    const int rc = launch_combine(cv, st, fresh);
     tap(7);
     return rc;
 }
@@ -663,7 +669,7 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
     lv.workspace = F.layer; lv.workspace_bytes = v->workspace_bytes - (static_cast<unsigned char*>(F.layer) - static_cast<unsigned char*>(v->workspace));
     lv.capacity = v->capacity; lv.grouped_min_rows = v->grouped_min_rows; lv.stage_events = v->stage_events;
     lv.summary = v->summary;
-    return layer_impl(&lv, stream, fused);
+    return layer_impl(&lv, stream, fused, false);
 }
 
 int b200moe_ffn_host(const b200moe_ffn_view* v, const void* x_host, float* y_host, void* stream) {
@@ -691,7 +697,10 @@ int b200moe_ffn_host(const b200moe_ffn_view* v, const void* x_host, float* y_hos
     return B200MOE_OK;
 }
 
-int b200moe_dense_ffn(const b200moe_dense_view* v, void* stream) {
+static int dense_impl(const b200moe_dense_view* v, void* stream, bool fresh);
+int b200moe_dense_ffn(const b200moe_dense_view* v, void* stream) { return dense_impl(v, stream, false); }
+int b200moe_dense_ffn_fresh(const b200moe_dense_view* v, void* stream) { return dense_impl(v, stream, true); }
+static int dense_impl(const b200moe_dense_view* v, void* stream, bool fresh) {
     B200_REQUIRE(v, "null view");
     B200_REQUIRE(v->shape.experts == 1 && v->shape.top_k == 1, "dense_ffn: shape.experts and shape.top_k must be 1");
     if (int rc = check_shape(v->shape)) return rc;
@@ -706,8 +715,8 @@ int b200moe_dense_ffn(const b200moe_dense_view* v, void* stream) {
         return fail(B200MOE_ERR_WORKSPACE, "dense_ffn: workspace of %llu bytes needed, %llu given", (unsigned long long)L.bytes, (unsigned long long)v->workspace_bytes);
     if (!device_ready()) return B200MOE_ERR_CUDA;
     cudaStream_t st = as_stream(stream);
-    // every row is one entry of the single expert (slot = row): the routes are written directly, the status words with them
-    if (int rc = launch_dense_routes(L.routes, v->rows, L.row_status, L.summary, st)) return rc;
+    // every row is one entry of the single expert (slot = row): the routes are written directly, the status words with them; y is zero until down writes it
+    if (int rc = launch_dense_routes(L.routes, v->rows, L.row_status, L.summary, fresh ? v->y : nullptr, u64(v->rows) * s.hidden, st)) return rc;
     b200moe_gate_up_view gu{};
     gu.shape = s; gu.weights = v->weights; gu.routes = L.routes; gu.max_union = 1; gu.x = v->x; gu.act = L.act;
     gu.row_status = L.row_status; gu.summary = L.summary;

@@ -13,6 +13,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <utility>
 
 #include "../../include/b200moe.h"
 
@@ -92,6 +93,12 @@ inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, 
     cudaLaunchConfig_t c{};
     c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = attr; c.numAttrs = 1;
     (void)cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+// A launch that needs little shared memory: see prefer_max_shared (a preference that cannot be set is no error).
+template <class... P, class... A>
+inline void small_launch(void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, cudaStream_t stream, A&&... args) {
+    (void)prefer_max_shared(reinterpret_cast<const void*>(kernel));
+    chain_launch(kernel, grid, block, smem, stream, std::forward<A>(args)...);
 }
 __device__ __forceinline__ float half_bits_to_float(u32 h) {  // exact for every fp16 value, subnormals included
     return __half2float(__ushort_as_half(static_cast<unsigned short>(h)));

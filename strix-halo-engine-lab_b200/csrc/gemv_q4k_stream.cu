@@ -663,15 +663,6 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) down_q4k_str
     if (!ok && lane == 0 && v.summary) atomicOr(const_cast<u32*>(v.summary), kAbortBit);
 }
 
-int sm_count() {
-    static int n = [] {
-        int dev = 0, v = 148;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        return v;
-    }();
-    return n;
-}
-
 constexpr u32 kSmemBudget = 224u * 1024u;
 
 u32 padded_stride(u32 row_bytes) { return ((row_bytes / 16) & 1u) ? row_bytes : row_bytes + 16; }
@@ -730,7 +721,7 @@ int launch_gate_up_q4k_stream(const b200moe_gate_up_view& v, u32 rows, cudaStrea
     p.x_rows = rows;
     const u32 smem = plan_smem(p, x_bytes, slot_bytes);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(gate_up_q4k_stream_kernel), smem)) return rc;
-    chain_launch(gate_up_q4k_stream_kernel, sm_count(), (p.warps + kProducers) * 32, smem, stream, v, p);
+    chain_launch(gate_up_q4k_stream_kernel, device_sm_count(), (p.warps + kProducers) * 32, smem, stream, v, p);
     return after_launch("gate_up_q4k_stream");
 }
 
@@ -745,7 +736,7 @@ int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, const ChainHint
     p.early = hints.routes_done;
     const u32 smem = plan_smem(p, down_fixed_bytes(v), 0);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(down_q4k_stream_kernel), smem)) return rc;
-    chain_launch(down_q4k_stream_kernel, sm_count(), (p.warps + kProducers) * 32, smem, stream, v, p);
+    chain_launch(down_q4k_stream_kernel, device_sm_count(), (p.warps + kProducers) * 32, smem, stream, v, p);
     return after_launch("down_q4k_stream");
 }
 

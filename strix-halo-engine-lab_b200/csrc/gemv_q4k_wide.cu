@@ -580,10 +580,10 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const Chain
     const u32 smem = plan_smem(p);
     if (p.S == 3) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<false, 3>), smem)) return rc;
-        chain_launch(q4k_wide_kernel<false, 3>, sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
+        chain_launch(q4k_wide_kernel<false, 3>, device_sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
     } else {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<false, 1>), smem)) return rc;
-        chain_launch(q4k_wide_kernel<false, 1>, sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
+        chain_launch(q4k_wide_kernel<false, 1>, device_sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
     }
     return after_launch("gate_up_q4k_wide");
 }
@@ -603,10 +603,10 @@ int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints&
     const u32 smem = plan_smem(p);
     if (p.S == 3) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<true, 3>), smem)) return rc;
-        chain_launch(q4k_wide_kernel<true, 3>, sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
+        chain_launch(q4k_wide_kernel<true, 3>, device_sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
     } else {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<true, 1>), smem)) return rc;
-        chain_launch(q4k_wide_kernel<true, 1>, sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
+        chain_launch(q4k_wide_kernel<true, 1>, device_sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
     }
     return after_launch("down_q4k_wide");
 }

@@ -346,7 +346,7 @@ int launch_gate_up_q8_mma(const b200moe_gate_up_view& v, u32 rows, cudaStream_t 
     const u32 smem = plan_smem(p, false);
     const auto kernel = q8_mma_kernel<false>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-    chain_launch(kernel, sm_count(), kMmaThreads, smem, stream, tm0, tm1, a, p);
+    chain_launch(kernel, device_sm_count(), kMmaThreads, smem, stream, tm0, tm1, a, p);
     return after_launch("gate_up_q8_mma");
 }
 
@@ -363,7 +363,7 @@ int launch_down_q8_mma(const b200moe_down_view& v, u32 rows, cudaStream_t stream
     const u32 smem = plan_smem(p, true);
     const auto kernel = q8_mma_kernel<true>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-    chain_launch(kernel, sm_count(), kMmaThreads, smem, stream, tm0, tm0, a, p);
+    chain_launch(kernel, device_sm_count(), kMmaThreads, smem, stream, tm0, tm0, a, p);
     return after_launch("down_q8_mma");
 }
 

@@ -342,7 +342,7 @@ int launch_gate_up_q8_wide(const b200moe_gate_up_view& v, u32 rows, cudaStream_t
     if (int rc = rows_map(v.weights.up, rb, total_rows, kRunBytes, kRows, &tm1)) return rc;
     const u32 smem = plan_smem(p, false);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q8_wide_kernel<false>), smem)) return rc;
-    chain_launch(q8_wide_kernel<false>, sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
+    chain_launch(q8_wide_kernel<false>, device_sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
     return after_launch("gate_up_q8_wide");
 }
 
@@ -358,7 +358,7 @@ int launch_down_q8_wide(const b200moe_down_view& v, u32 rows, cudaStream_t strea
     if (int rc = rows_map(v.weights.down, u64(p.groups) * kQ8Block, u64(v.shape.experts) * v.shape.hidden, kRunBytes, kRows, &tm0)) return rc;
     const u32 smem = plan_smem(p, true);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q8_wide_kernel<true>), smem)) return rc;
-    chain_launch(q8_wide_kernel<true>, sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
+    chain_launch(q8_wide_kernel<true>, device_sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
     return after_launch("down_q8_wide");
 }
 

@@ -35,6 +35,7 @@
 #include <cuda.h>
 
 #include "grouped_common.cuh"
+#include "wide_common.cuh"
 
 namespace b200moe {
 namespace {
@@ -254,8 +255,8 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
                 if (lt == 0) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the consumers' reads precede the copies below
                     mbar_expect_tx(&raw_full[slot_r], kRawBytes);
-                    tma_2d(st, &tm0, ib * kQ4KBlock, cy, &raw_full[slot_r]);
-                    tma_2d(st + kOutRows * kQ4KBlock, kDown ? &tm0 : &tm1, ib * kQ4KBlock, kDown ? cy + kOutRows : cy, &raw_full[slot_r]);
+                    tma_2d(st, &tm0, ib * (kQ4KBlock / 8), cy, &raw_full[slot_r]);
+                    tma_2d(st + kOutRows * kQ4KBlock, kDown ? &tm0 : &tm1, ib * (kQ4KBlock / 8), kDown ? cy + kOutRows : cy, &raw_full[slot_r]);
                     ++asked;
                 }
                 unsigned char* sc = st + kOffCode + ((kGN / 4) * hw + (lane >> 4)) * kCodePitch + 16u * (lane & 15u);
@@ -463,28 +464,6 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     if (!ok && lane == 0 && a.summary) atomicOr(a.summary, kAbortBit);
 }
 
-// Tensor map of a [rows][row_bytes] byte tensor with boxes of a super-block x 96 rows (no swizzle, no interleave). The
-// encoder is the driver's cuTensorMapEncodeTiled, looked up through the runtime (no link against the driver library).
-int encode_rows_map(const u8* base, u64 row_bytes, u64 rows, CUtensorMap* out) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
-        return reinterpret_cast<EncodeFn>(p);
-    }();
-    if (!fn) return fail(B200MOE_ERR_CUDA, "grouped: cuTensorMapEncodeTiled is not available from this driver");
-    const cuuint64_t dims[2] = {row_bytes, rows};
-    const cuuint64_t strides[1] = {row_bytes};       // bytes between rows: a multiple of 16 (144 per super-block)
-    const cuuint32_t box[2] = {kQ4KBlock, kOutRows};
-    const cuuint32_t elem[2] = {1, 1};
-    const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<u8*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(B200MOE_ERR_CUDA, "grouped: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
-    return B200MOE_OK;
-}
-
 bool es_units(const b200moe_a8_rows& x) {
     const u32 stride = x.stride ? x.stride : x.width;
     return stride % 128 == 0 && aligned(x.deltas, 16) && aligned(x.sums, 16);
@@ -493,12 +472,6 @@ bool es_units(const b200moe_a8_rows& x) {
 bool grouped_shape_ok(const b200moe_shape& s) {
     return s.gate_type == B200MOE_TYPE_Q4_K && s.down_type == B200MOE_TYPE_Q4_K && s.hidden % 256 == 0 && s.inter % 256 == 0 &&
            s.experts <= kMaxUnion;
-}
-
-int grid_size() {
-    int dev = 0, n = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
 }
 
 }  // namespace
@@ -514,10 +487,10 @@ int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t strea
     a.n_row_tiles = grouped_row_tiles(v.shape.inter, false); a.K = v.shape.hidden; a.es_vec = es_units(v.x); a.stall_stage = debug_waits().stall_stage;
     CUtensorMap tm0, tm1;
     const u64 rb = u64(v.shape.hidden / 256) * kQ4KBlock, rows = u64(v.shape.experts) * v.shape.inter;
-    if (int rc = encode_rows_map(v.weights.gate, rb, rows, &tm0)) return rc;
-    if (int rc = encode_rows_map(v.weights.up, rb, rows, &tm1)) return rc;
+    if (int rc = wide::rows_map(v.weights.gate, rb, rows, kQ4KBlock, kOutRows, &tm0)) return rc;
+    if (int rc = wide::rows_map(v.weights.up, rb, rows, kQ4KBlock, kOutRows, &tm1)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<false>), kGroupedSmem)) return rc;
-    chain_launch(grouped_q4k_kernel<false>, grid_size(), kGThreads, kGroupedSmem, stream, tm0, tm1, a);
+    chain_launch(grouped_q4k_kernel<false>, device_sm_count(), kGThreads, kGroupedSmem, stream, tm0, tm1, a);
     return after_launch("gate_up_q4k_grouped");
 }
 
@@ -528,9 +501,9 @@ int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream) {
     a.summary = const_cast<u32*>(v.summary);
     a.n_row_tiles = grouped_row_tiles(v.shape.hidden, true); a.K = v.shape.inter; a.es_vec = es_units(v.act); a.raw_vec = aligned(v.raw, 8); a.stall_stage = debug_waits().stall_stage;
     CUtensorMap tm0;
-    if (int rc = encode_rows_map(v.weights.down, u64(v.shape.inter / 256) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, &tm0)) return rc;
+    if (int rc = wide::rows_map(v.weights.down, u64(v.shape.inter / 256) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, kQ4KBlock, kOutRows, &tm0)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_q4k_kernel<true>), kGroupedSmem)) return rc;
-    chain_launch(grouped_q4k_kernel<true>, grid_size(), kGThreads, kGroupedSmem, stream, tm0, tm0, a);
+    chain_launch(grouped_q4k_kernel<true>, device_sm_count(), kGThreads, kGroupedSmem, stream, tm0, tm0, a);
     return after_launch("down_q4k_grouped");
 }
 

@@ -29,7 +29,8 @@ u64 routes_scratch_words(u32 rows, u32 top_k, u32 experts);
 // what the first launch of a call that owns its status words clears on the way (each may be null): rows, 4 and 1 words
 struct RoutesClear { u32* row_status; u32* summary4; u32* summary; };
 int launch_routes(const b200moe_routes_view& v, const RoutesClear& clear, cudaStream_t stream);
-int launch_dense_routes(const b200moe_routes& out, u32 rows, u32* row_status, u32* summary4, cudaStream_t stream);
+// zero (optional): count floats cleared on the way
+int launch_dense_routes(const b200moe_routes& out, u32 rows, u32* row_status, u32* summary4, float* zero, u64 count, cudaStream_t stream);
 // grouped (token-block) form of the Q4_K experts on the tensor cores (grouped_q4k.cu)
 bool grouped_fits(const b200moe_shape& s, bool have_sums);
 u32 grouped_row_tiles(u32 outputs, bool down);  // of an expert
@@ -88,7 +89,8 @@ int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view
 
 // combine.cu
 int launch_merge_first_error(b200moe_first_error* record, const u32* summary, u32 domain, cudaStream_t stream);
-int launch_combine(const b200moe_combine_view& v, cudaStream_t stream);
+// zero_skipped: rows of y and y_bf16 that a failed row or an aborted job leaves out become zeros
+int launch_combine(const b200moe_combine_view& v, cudaStream_t stream, bool zero_skipped = false);
 int launch_canonical_sum(const float* a, const float* b, const float* c, u64 count, float* y, cudaStream_t stream);
 int launch_fill_u32(u32* p, u32 value, u64 count, cudaStream_t stream);
 // order[row][k] (slots in ascending expert id) for the PARTS combine when no routes were built

@@ -77,8 +77,8 @@ int launch_rmsnorm_a8(const b200moe_rmsnorm_view& v, cudaStream_t stream) {
     // (592 rows of 2048: 11.6 against 11.8; of 1024: 7.5 both).
     const u32 sms = static_cast<u32>(device_sm_count());
     const u32 warps = v.rows <= 2u * sms ? std::min(32u, (v.n / 32u + 7u) / 8u * 8u) : 8u;
-    if (v.rows > 2u * sms && v.rows <= 5u * sms && v.n >= kWideRow) chain_launch(rmsnorm_a8_kernel<8>, v.rows, 256, 0, stream, v);
-    else chain_launch(rmsnorm_a8_kernel<0>, v.rows, 32u * warps, 0, stream, v);
+    if (v.rows > 2u * sms && v.rows <= 5u * sms && v.n >= kWideRow) small_launch(rmsnorm_a8_kernel<8>, v.rows, 256, 0, stream, v);
+    else small_launch(rmsnorm_a8_kernel<0>, v.rows, 32u * warps, 0, stream, v);
     return after_launch("rmsnorm_a8");
 }
 

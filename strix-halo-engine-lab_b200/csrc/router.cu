@@ -210,18 +210,18 @@ int launch_router_logits(const b200moe_router_view& v, cudaStream_t stream, cons
     if (v.rows == 0) return B200MOE_OK;
     if (fused_quantize) if (int rc = launch_quantize_a8(*fused_quantize, stream)) return rc;
 #define B200_LOGITS(RT, ET)                                                                                   \
-    chain_launch(router_logits_kernel<RT, ET>, dim3((E + 4 * ET - 1) / (4 * ET), (v.rows + RT - 1) / RT), 128, 0, stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits)
+    small_launch(router_logits_kernel<RT, ET>, dim3((E + 4 * ET - 1) / (4 * ET), (v.rows + RT - 1) / RT), 128, 0, stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits)
     const bool vec = aligned(v.x, 16) && aligned(v.weight, 16) && xs % 4 == 0 && v.hidden % 4 == 0;  // whole 16-byte units for the staged forms
 #define B200_FEW(RT)                                                                                                                  \
     {                                                                                                                                 \
         constexpr u32 smem = (RT + kFewWarps) * kFewRun * sizeof(float);                                                              \
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(router_logits_few_kernel<RT>), smem)) return rc;               \
-        chain_launch(router_logits_few_kernel<RT>, (E + kFewWarps - 1) / kFewWarps, kFewWarps * 32, smem, stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
+        small_launch(router_logits_few_kernel<RT>, (E + kFewWarps - 1) / kFewWarps, kFewWarps * 32, smem, stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
     }
 #define B200_TILE(COLS)                                                                                                               \
     {                                                                                                                                 \
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(router_logits_tile_kernel<COLS>), tile_smem_bytes(COLS))) return rc; \
-        chain_launch(router_logits_tile_kernel<COLS>, grid, 128, tile_smem_bytes(COLS), stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
+        small_launch(router_logits_tile_kernel<COLS>, grid, 128, tile_smem_bytes(COLS), stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
     }
     if (v.rows <= 4 && vec) {
         if (v.rows == 1) B200_FEW(1)
@@ -245,7 +245,7 @@ int launch_router_logits(const b200moe_router_view& v, cudaStream_t stream, cons
 int launch_router_select(const b200moe_router_view& v, cudaStream_t stream) {
     if (v.rows == 0) return B200MOE_OK;
     const u32 smem = 4u * select_detail::scratch_floats(v.policy.experts) * sizeof(float);
-    chain_launch(router_select_kernel, (v.rows + 3) / 4, 128, smem, stream, v.logits, v.scores, v.bias, v.policy, v.rows, v.ids, v.weights);
+    small_launch(router_select_kernel, (v.rows + 3) / 4, 128, smem, stream, v.logits, v.scores, v.bias, v.policy, v.rows, v.ids, v.weights);
     return after_launch("router_select");
 }
 

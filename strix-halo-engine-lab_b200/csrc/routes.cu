@@ -124,9 +124,14 @@ __global__ void __launch_bounds__(1024) routes_fill_kernel(b200moe_routes_view v
 // The routes of a dense block (one expert, top-1: every row is one entry of expert 0, slot = row) written directly, with
 // the job's status words cleared in the same launch: what build_window_routes (src/ds41_moe.cpp:11-43) gives for ids = 0,
 // without the sort and without the memsets in front of it.
-__global__ void __launch_bounds__(256) dense_routes_kernel(b200moe_routes out, u32 rows, u32* row_status, u32* summary4) {
+__global__ void __launch_bounds__(256) dense_routes_kernel(b200moe_routes out, u32 rows, u32* row_status, u32* summary4, float* zero, u64 count) {
     chain_begin();
-    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+    if (zero) {
+        const u64 whole = reinterpret_cast<uintptr_t>(zero) % 16 == 0 ? count / 4 : 0;
+        for (u64 k = i; k < whole; k += threads) reinterpret_cast<float4*>(zero)[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (u64 k = 4 * whole + i; k < count; k += threads) zero[k] = 0.0f;
+    }
     if (i < rows) {
         out.rows[i] = i;
         out.slots[i] = i;
@@ -161,13 +166,14 @@ int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view
     const u32 threads = std::max(32u * r.rows, small_threads(n, v.experts));
     const auto kernel = threads <= 256u ? select_routes_small_kernel<256> : select_routes_small_kernel<1024>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-    chain_launch(kernel, 1, threads, smem, stream, r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights, v, v.end ? v.end : v.experts,
+    small_launch(kernel, 1, threads, smem, stream, r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights, v, v.end ? v.end : v.experts,
                  Clear{clear.row_status, clear.summary4, clear.summary});
     return after_launch("select_routes_small");
 }
 
-int launch_dense_routes(const b200moe_routes& out, u32 rows, u32* row_status, u32* summary4, cudaStream_t stream) {
-    chain_launch(dense_routes_kernel, (rows + 255) / 256, 256, 0, stream, out, rows, row_status, summary4);
+int launch_dense_routes(const b200moe_routes& out, u32 rows, u32* row_status, u32* summary4, float* zero, u64 count, cudaStream_t stream) {
+    const u64 most = std::max<u64>(rows, zero ? std::min<u64>((count + 3) / 4, 256ull * 8ull * static_cast<u32>(device_sm_count())) : 0);
+    small_launch(dense_routes_kernel, static_cast<u32>((most + 255) / 256), 256, 0, stream, out, rows, row_status, summary4, zero, count);
     return after_launch("dense_routes");
 }
 
@@ -179,16 +185,16 @@ int launch_routes(const b200moe_routes_view& v, const RoutesClear& clear, cudaSt
     const u32 smem = counts_bytes(static_cast<u32>(std::min<u64>(n, kChunk)), v.experts);
     if (n <= kChunk) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(routes_small_kernel), smem)) return rc;
-        chain_launch(routes_small_kernel, 1, small_threads(static_cast<u32>(n), v.experts), smem, stream, v, end, c);
+        small_launch(routes_small_kernel, 1, small_threads(static_cast<u32>(n), v.experts), smem, stream, v, end, c);
         return after_launch("routes_small");
     }
     const u32 chunks = static_cast<u32>((n + kChunk - 1) / kChunk);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(routes_fill_kernel), smem)) return rc;
-    chain_launch((v.top_k <= kRankedTopK ? routes_count_kernel<true> : routes_count_kernel<false>), chunks, 1024, 0, stream, v, end, chunks, c);
+    small_launch((v.top_k <= kRankedTopK ? routes_count_kernel<true> : routes_count_kernel<false>), chunks, 1024, 0, stream, v, end, chunks, c);
     if (int rc = after_launch("routes_count")) return rc;
-    chain_launch(routes_scan_kernel, 1, 1024, 0, stream, v, chunks);
+    small_launch(routes_scan_kernel, 1, 1024, 0, stream, v, chunks);
     if (int rc = after_launch("routes_scan")) return rc;
-    chain_launch(routes_fill_kernel, chunks, 1024, smem, stream, v, end, chunks);
+    small_launch(routes_fill_kernel, chunks, 1024, smem, stream, v, end, chunks);
     return after_launch("routes_fill");
 }
 

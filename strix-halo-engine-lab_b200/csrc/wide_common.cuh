@@ -114,12 +114,6 @@ __device__ __forceinline__ void build_dense_list(u32 rows, u32 n_chunks, VExpert
     __syncthreads();
 }
 
-inline int sm_count() {
-    int dev = 0, v = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v;
-}
-
 // Tensor map of a [rows][row_bytes] tensor seen as 64-bit elements, boxes of box_bytes (a multiple of 16) x box_rows rows,
 // no swizzle. The encoder is the driver's cuTensorMapEncodeTiled, looked up through the runtime (no link against
 // the driver library). Encoded maps are kept per (device, tensor, geometry): encoding is host work of a few microseconds

@@ -7,16 +7,16 @@
 // per (row, token, group), ten packed instructions per MMA of 16 tokens x 8 rows x 32. On a loop of its own, in clocks of a scheduler per
 // such MMA: the ten alone 20 to 22 (a packed product or sum reads two register pairs and takes two clocks, an fma of three distinct
 // pairs takes three), with the MMA 28 (its ten operand and result registers go through the same ports; its time ADDS), 30 with the
-// conversion of the dots and the sums written as fma, 31 with a barrier per 32 MMAs. The kernel spends 36 to 40: a tenth of that is
-// SwiGLU + the A8 rule, three to five hundredths the meeting of the chains.
-// 512 tokens x 34,816 rows x 5120: 785 us (941 in the form before, a warp all four chains of 32 rows x 16 tokens, whose row factors met 16
-// tokens and cost half the instructions); 4096 x 8 tokens, skewed, over 128 experts of 2048 -> 2 x 768: 1170 us (1328).
+// conversion of the dots and the sums written as fma, 31 with a barrier per 32 MMAs. The kernel spends 36 to 38; the end of a tile (the
+// chains' meeting, SwiGLU + the A8 rule) is paid where the other two thirds' warps leave the schedulers free.
+// gate/up of 4096 x 8 tokens, skewed, over 128 experts of 2048 -> 2 x 768: 1070 us (1124 while all twelve consumer warps met at a tile's end, with gate rows in
+// one half of the tile's rows and their up rows in the other); of 512 tokens x 34,816 rows x 5120, whose tiles are longer: 805 us (810).
 // The dots out of tensor memory (tcgen05.mma kind::i8) leave the ports free (24 clocks a unit on a loop of its own), but what that form
 // adds - nibbles unpacked to shared memory, MMA and commit latencies between two barriers, more code than a scheduler's instruction
 // cache holds - cost more: 1180 to 1480 us, in 16 consumer warps of one chain or 8 of two.
 //
 // Tile = (expert, 192 weight rows, kGN of the expert's tokens). gate/up: rows 0..95 are gate rows [96c, 96c + 96), rows 96..191 the up
-// rows of the same outputs, so SwiGLU + the A8 rule of h finish inside the tile. down: 192 rows of H. The last row tile of an expert
+// rows of the same outputs; a third of the consumers takes 32 of the gate rows and their up rows, so SwiGLU + the A8 rule of h finish inside the third. down: 192 rows of H. The last row tile of an expert
 // ends with it and may repeat rows of the tile before (the same bits twice): a read past an expert's rows could leave the tensor, which may
 // hold fewer experts than the shape counts.
 // A persistent CTA per SM walks tiles round-robin; a stage of the ring (three) is one super-block: 256 columns, 4 pairs of groups (chains).
@@ -29,7 +29,7 @@
 //     are two weight rows of one token, so the rows' factors are natural register pairs and the packed instructions take a token's
 //     factors as one register for both halves. A row's factors are read once per 32 tokens, a token's once per 64 rows.
 //     The four chains of a row third meet through shared memory at the end of a tile, (a0 + a1) + (a2 + a3); gate/up then runs
-//     SwiGLU + the A8 rule, a warp four (token, 32 outputs) tasks at a time.
+//     SwiGLU + the A8 rule, a warp two tokens at a time. A third's barriers are its own: the thirds drift apart and end their tiles at different times.
 // Every wait is bounded; on a timeout the roles stop working, the first helper waits (bounded) for the copies in flight and the launch sets
 // B200MOE_JOB_WAIT_ABORTED in the job summary.
 #include <cuda.h>
@@ -54,11 +54,11 @@ constexpr u32 kCodePitch = 256 + 16;
 constexpr u32 kRawBytes = kGM * kQ4KBlock, kCodeBytes = kGN * kCodePitch, kEsBytes = 4 * kGN * 16, kFacBytes = 4 * kGM * 16, kPrivBytes = kGN * 64;
 constexpr u32 kStageBytes = (kRawBytes + kCodeBytes + kEsBytes + kFacBytes + kPrivBytes + 127) / 128 * 128;
 constexpr u32 kOffCode = kRawBytes, kOffEs = kOffCode + kCodeBytes, kOffFac = kOffEs + kEsBytes, kOffPriv = kOffFac + kFacBytes;  // in a stage
-constexpr u32 kOutPitch = kGM + 8;               // floats: the 8-byte stores of a half warp (four tokens, four row pairs) meet every bank once
-constexpr u32 kOutBytes = kGN * kOutPitch * 4;   // epilogue tile (gate/up)
+constexpr u32 kOutPitch = 64 + 8;                // floats: the 8-byte stores of a half warp (four tokens, four row pairs) meet every bank once
+constexpr u32 kOutBytes = kGN * kOutPitch * 4;   // a third's epilogue tile (gate/up): 32 gate and 32 up values a token
 constexpr u32 kFoldCells = kRowTiles / 2 * kTokTiles * 2;      // float2 cells of a lane that change hands when two chains meet
 constexpr u32 kFoldBytes = kConsumers * kFoldCells * 32 * 8;
-static_assert(kOutBytes <= kFoldBytes, "the epilogue tile takes the place of the buffers that the chains met in");
+static_assert(kOutBytes <= kFoldBytes / kThirds, "a third's epilogue tile takes the place of the buffers that its chains met in");
 // What the consumers need of a tile: {first row, tokens, first entry}, its tokens' A8 rows, its tokens' slots. The helpers run at most
 // kStages stages ahead of the consumers, a tile has at least one stage and its places are read until its end: eight places.
 constexpr u32 kTilePlaces = 8, kTileWords = 4 + 2 * kGN;
@@ -102,7 +102,8 @@ struct GroupedArgs {
 // nibbles of the lane's k slice; codes: token lane / 4 at the pair's codes; es: the pair's {E, E', S, S'} from token lane / 4 on; fac: the
 // pair's {D, D, D', D'} {-DM, -DM, -DM', -DM'} of two rows, from row pair lane % 4 on. acc[j][mt][z]: rows 8 j + 2 (lane % 4) and the
 // next of token 16 mt + 8 z + lane / 4.
-template <int NMT>
+// SPLIT (gate/up): the warp's row tiles 4 to 7 are up rows, kOutRows behind the gate rows of the same outputs in tiles 0 to 3.
+template <int NMT, bool SPLIT>
 __device__ __forceinline__ void superblock(const unsigned char* rows, const unsigned char* codes, const float4* es, const float4* fac,
                                            float2 (&acc)[kRowTiles][kTokTiles][2]) {
     u32 cl[NMT][4], ch[NMT][4];
@@ -122,8 +123,9 @@ __device__ __forceinline__ void superblock(const unsigned char* rows, const unsi
         }
 #pragma unroll
     for (int j = 0; j < (int)kRowTiles; ++j) {
-        const u32 q0 = *reinterpret_cast<const u32*>(rows + 8 * j * kQ4KBlock), q1 = *reinterpret_cast<const u32*>(rows + 8 * j * kQ4KBlock + 16);
-        const float4 d4 = fac[8 * j], m4 = fac[8 * j + 1];
+        const int row = 8 * j + (SPLIT && j >= (int)kRowTiles / 2 ? (int)kOutRows - 32 : 0);
+        const u32 q0 = *reinterpret_cast<const u32*>(rows + row * kQ4KBlock), q1 = *reinterpret_cast<const u32*>(rows + row * kQ4KBlock + 16);
+        const float4 d4 = fac[row], m4 = fac[row + 1];
         const float2 Dl = make_float2(d4.x, d4.y), Dh = make_float2(d4.z, d4.w), Ml = make_float2(m4.x, m4.y), Mh = make_float2(m4.z, m4.w);
 #pragma unroll
         for (int mt = 0; mt < NMT; ++mt) {
@@ -143,7 +145,7 @@ __device__ __forceinline__ void superblock(const unsigned char* rows, const unsi
 
 // SwiGLU + the A8 rule of kTasks (token, 32 outputs) tasks of one warp, step by step over them, so that their chains overlap. g, u: the
 // lane's gate and up values; returns per task whether a value is not finite (code, delta and sum then mean nothing).
-constexpr int kTasks = 4;
+constexpr int kTasks = 2;
 __device__ __forceinline__ u32 swiglu_a8(const float (&g)[kTasks], const float (&u)[kTasks], int (&code)[kTasks], float (&delta)[kTasks], int (&sum)[kTasks]) {
     float h[kTasks], x[kTasks];
     u32 bad = 0, amax[kTasks];
@@ -189,7 +191,6 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
     float2* s_fold = reinterpret_cast<float2*>(smem + kOffFold);       // [warp][kFoldCells][lane]
-    float* s_out = reinterpret_cast<float*>(smem + kOffFold);          // [kGN][kOutPitch]
     u64* raw_full = reinterpret_cast<u64*>(smem + kOffBars);
     u64* ready = raw_full + kStages;
     u64* empty = ready + kStages;
@@ -347,7 +348,9 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     } else {
         // ================================================================================================ consumers
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
-        const u32 p = warp & 3u, third = warp >> 2;     // chain, 64 rows of the tile
+        const u32 p = warp & 3u, third = warp >> 2;     // chain, 64 rows of the tile: gate/up 32 gate rows and the up rows of the same outputs
+        const u32 row_base = (kDown ? 64u : 32u) * third;
+        float* s_out = reinterpret_cast<float*>(smem + kOffFold + third * (kFoldBytes / kThirds));  // [kGN][kOutPitch], the third's
         const u32 fr = lane >> 2, ft = lane & 3u;       // fragments: token fr (and fr + 8) of a token tile, rows 2 ft and 2 ft + 1 of a row tile
         const u32 act_stride = a.act.stride ? a.act.stride : a.act.width;
         u32 slot = 0, parity = 0;
@@ -365,12 +368,12 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
                 const u32 next = slot + 1u == kStages ? 0u : slot + 1u, next_parity = parity ^ (next == 0u ? 1u : 0u);
                 if (b == 0) n_mt = (ti[1] + 15u) / 16u;
                 const unsigned char* st = smem + slot * kStageBytes;
-                const unsigned char* rows = st + (64u * third + fr) * kQ4KBlock + 16u + 32u * p + 4u * ft;
+                const unsigned char* rows = st + (row_base + fr) * kQ4KBlock + 16u + 32u * p + 4u * ft;
                 const unsigned char* codes = st + kOffCode + fr * kCodePitch + 64u * p + 4u * ft;
                 const float4* es = reinterpret_cast<const float4*>(st + kOffEs) + p * kGN + fr;
-                const float4* fac = reinterpret_cast<const float4*>(st + kOffFac) + p * kGM + 2u * (32u * third + ft);
-                if (n_mt == 2) superblock<2>(rows, codes, es, fac, acc);
-                else superblock<1>(rows, codes, es, fac, acc);
+                const float4* fac = reinterpret_cast<const float4*>(st + kOffFac) + p * kGM + row_base + 2u * ft;
+                if (n_mt == 2) superblock<2, !kDown>(rows, codes, es, fac, acc);
+                else superblock<1, !kDown>(rows, codes, es, fac, acc);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[slot]);
                 slot = next; parity = next_parity;
@@ -378,8 +381,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
             // (a0 + a1) + (a2 + a3). Warp p hands half of its row tiles to warp p ^ 1 of its third and adds what that hands over, then does the
             // same with half of what is left and warp p ^ 2. Buffer p is written by warp p, then by warp p ^ 1 (which alone has read it), then
             // read by warp p ^ 3. The barriers are met on every path.
-            if (kDown) asm volatile("bar.sync %0, 128;" ::"r"(4u + third) : "memory");  // the previous tile's last reads of the buffers
-            else asm volatile("bar.sync 2, %0;" ::"n"(kConsumers * 32) : "memory");     // ... and of s_out
+            asm volatile("bar.sync %0, 128;" ::"r"(4u + third) : "memory");  // the previous tile's last reads of the buffers and of s_out
             float2* bufs = s_fold + 4u * third * (kFoldCells * 32) + lane;
             float2* mine = bufs + p * (kFoldCells * 32);
             float2* theirs = bufs + (p ^ 1u) * (kFoldCells * 32);
@@ -401,14 +403,14 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
             asm volatile("bar.sync %0, 128;" ::"r"(4u + third) : "memory");
 #pragma unroll
             for (int i = 0; i < 2 * n; ++i) (&out[0][0][0])[i] = add((&out[0][0][0])[i], last[32 * i]);
-            const u32 row0 = 64u * third + 32u * (p & 1u) + 16u * (p >> 1) + 2u * ft;  // the lane's first row of the two row tiles that are left to it
+            const u32 row0 = 32u * (p & 1u) + 16u * (p >> 1) + 2u * ft;  // the lane's first of the third's 64 rows in the two row tiles that are left to it
             const u32 nt = ok ? ti[1] : 0u, first = ti[0], eb = ti[2];
             if (kDown) {
 #pragma unroll
                 for (int cz = 0; cz < n; ++cz) {
                     const u32 tk = 8u * cz + fr;
                     if (tk < nt) {
-                        float* to = a.raw + u64(ti[4 + kGN + tk]) * H + first + row0;
+                        float* to = a.raw + u64(ti[4 + kGN + tk]) * H + first + row_base + row0;
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
                             const float2 v = out[i][cz >> 1][cz & 1];
@@ -418,31 +420,31 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
                     }
                 }
             } else {
-                asm volatile("bar.sync 2, %0;" ::"n"(kConsumers * 32) : "memory");  // the buffers have been read
+                asm volatile("bar.sync %0, 128;" ::"r"(4u + third) : "memory");  // the buffers have been read
 #pragma unroll
                 for (int cz = 0; cz < n; ++cz) {
                     float* to = s_out + (8u * cz + fr) * kOutPitch + row0;
 #pragma unroll
                     for (int i = 0; i < 2; ++i) *reinterpret_cast<float2*>(to + 8 * i) = out[i][cz >> 1][cz & 1];
                 }
-                asm volatile("bar.sync 2, %0;" ::"n"(kConsumers * 32) : "memory");
-                // SwiGLU + the A8 rule: a task is (token, one of its three groups of 32 outputs)
-                constexpr u32 per = kOutRows / 32;
-                for (u32 k0 = kTasks * warp; k0 < per * nt; k0 += kTasks * kConsumers) {
+                asm volatile("bar.sync %0, 128;" ::"r"(4u + third) : "memory");
+                // SwiGLU + the A8 rule over the third's 32 outputs of every token. No barrier here is met by more than the third's four warps, which lie on four
+                // schedulers: while one third is at its tile's end, the others keep the schedulers busy.
+                const u32 group = first / 32u + third, o_col = 32u * group + lane;
+                for (u32 k0 = kTasks * p; k0 < nt; k0 += kTasks * 4u) {
                     float g[kTasks], u[kTasks], delta[kTasks];
                     int code[kTasks], sum[kTasks];
 #pragma unroll
                     for (int i = 0; i < kTasks; ++i) {
-                        const u32 k = min(k0 + i, per * nt - 1u), tk = k / per;
-                        const float* src = s_out + tk * kOutPitch + 32u * (k - per * tk) + lane;
-                        g[i] = src[0]; u[i] = src[kOutRows];
+                        const float* src = s_out + min(k0 + i, nt - 1u) * kOutPitch + lane;
+                        g[i] = src[0]; u[i] = src[32];
                     }
                     const u32 bad = swiglu_a8(g, u, code, delta, sum);
 #pragma unroll
                     for (int i = 0; i < kTasks; ++i) {
-                        const u32 k = k0 + i, tk = k / per;
-                        if (k >= per * nt) break;
-                        const u32 slot_id = ti[4 + kGN + tk], group = first / 32u + (k - per * tk), o_col = 32u * group + lane;
+                        const u32 tk = k0 + i;
+                        if (tk >= nt) break;
+                        const u32 slot_id = ti[4 + kGN + tk];
                         if (a.gate_out) { a.gate_out[u64(slot_id) * I + o_col] = g[i]; a.up_out[u64(slot_id) * I + o_col] = u[i]; }
                         if (bad >> i & 1u) {  // fail closed: nothing of the group is written (routed_expert.cpp:147-156)
                             if (lane == 0) {

@@ -356,7 +356,7 @@ int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grou
             default: return launch_down_q4k(v, st);
         }
     }
-    if (is_kquant(v.shape.gate_type)) return launch_down_q8_chain4(v, st);  // chain4: Q8_0 and Q5_1 blocks
+    if (is_kquant(v.shape.gate_type)) return launch_down_q8_chain4(v, hints, st);  // chain4: Q8_0 and Q5_1 blocks
     if (v.shape.down_type == B200MOE_TYPE_Q2_K) return launch_down_ds41_any(v, st);
     switch (pick_q8_form(v.shape, q8_wide_down_fits(v, rows), q8_mma_down_fits(v, rows), grouped_q8_down_fits(v), rows, v.max_union, true)) {
         case Q8Form::grouped: return launch_down_q8_grouped(v, st);

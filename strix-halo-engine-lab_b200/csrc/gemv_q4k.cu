@@ -18,6 +18,7 @@
 // Roofline: HBM. Algorithmic bytes per (expert, call) = 2 * inter * hidden / 256 * 144 (gate, up) and
 // hidden * inter / 256 * 144 (down), read once however many of the <= 8 staged rows use the expert.
 #include "declared_math.cuh"
+#include "grouped_common.cuh"
 #include "kernels.cuh"
 
 namespace b200moe {
@@ -382,6 +383,178 @@ __global__ void __launch_bounds__(256) down_q8_chain4_kernel(b200moe_down_view v
     }
 }
 
+// The same rule with the weight rows brought in by bulk copies: rows_per_item rows of an expert lie one behind the other in memory, so an item = (expert, that
+// many rows) is ONE copy. A CTA of 4 threads a row walks its items round-robin over two stages: an item's weights are asked for two items ahead,
+// its entries' A8 rows (up to `cap` of them, the rest in further passes) one item ahead by asynchronous copies. An early launch (ChainHints) asks for its
+// first two items' weights before it waits for the launch in front.
+// What bounds it: the trip to HBM and the start, for the few items a CTA has in a decode window. The form above, whose 1280 CTAs (4 rows over 128 experts of
+// 640 -> 2560, top 8, Q5_1) each made that trip twice from registers, eight a multiprocessor and a second wave of 96, took 20 us.
+struct ChainPlan {
+    u32 rows_per_item, n_chunks, cap, stage_bytes, a8_bytes;  // a8_bytes: of `cap` entries
+    u32 early, wait_limit;
+};
+template <bool Q51>
+__global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_view v, ChainPlan plan) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const u32 H = v.shape.hidden, I = v.shape.inter, groups = I / 32, R = plan.rows_per_item;
+    constexpr u32 block = Q51 ? kQ51Block : kQ8Block;
+    const u64 row_bytes = u64(groups) * block;
+    __shared__ u64 full[2];
+    __shared__ u32 s_abort, s_slots[2][kR];
+    const u32 tid = threadIdx.x, chain = tid & 3u, my_row = tid >> 2;
+    if (tid == 0) {
+        q4k::mbar_init(&full[0], 1); q4k::mbar_init(&full[1], 1);
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (!plan.early) chain_begin();
+    const u32 n_items = load_l2(v.routes.counts) * plan.n_chunks;
+    auto ask = [&](u32 n, u32 item) {  // one thread
+        const u32 j = item / plan.n_chunks, chunk = item - j * plan.n_chunks;
+        unsigned char* st = smem_raw + (n & 1u) * plan.stage_bytes;
+        const u32 bytes = R * static_cast<u32>(row_bytes);
+        q4k::mbar_expect_tx(&full[n & 1u], bytes);
+        q4k::bulk_g2s(st, v.weights.down + (u64(load_l2(v.routes.experts + j)) * H + R * chunk) * row_bytes, bytes, &full[n & 1u]);
+    };
+    u32 asked = 0;
+    if (tid == 0)
+        for (; asked < 2 && blockIdx.x + asked * gridDim.x < n_items; ++asked) ask(asked, blockIdx.x + asked * gridDim.x);
+    if (plan.early) chain_begin();
+    auto drain = [&](u32 from) {  // one thread: the copies asked for land (the wait is bounded) before the CTA retires
+        for (u32 n = from; n < asked; ++n)
+            for (u32 i = 0; i < (plan.wait_limit >> 4) + 64u; ++i)
+                if (q4k::mbar_try_wait(&full[n & 1u], (n >> 1) & 1u, q4k::kWaitHintNs)) break;
+    };
+    if (v.summary && *v.summary) {  // a failed projection skips the whole down stage (routed_expert.hpp:17-19)
+        if (tid == 0) drain(0);
+        return;
+    }
+    unsigned char* a8 = smem_raw + 2 * plan.stage_bytes;
+    const u32 stride = v.act.stride ? v.act.stride : v.act.width;
+    const bool vec = reinterpret_cast<uintptr_t>(v.act.codes) % 16 == 0 && stride % 16 == 0;
+    // entries [first, first + nr) into buffer b: codes[nr][I], deltas[cap][groups], sums[cap][groups]
+    auto stage = [&](u32 b, u32 first, u32 nr) {
+        unsigned char* to = a8 + b * plan.a8_bytes;
+        float* deltas = reinterpret_cast<float*>(to + plan.cap * I);
+        i32* sums = reinterpret_cast<i32*>(deltas + plan.cap * groups);
+        for (u32 r = 0; r < nr; ++r) {
+            const u32 slot = load(v.routes.slots + first + r);
+            if (tid == 0) s_slots[b][r] = slot;
+            const i8* c = v.act.codes + u64(slot) * stride;
+            if (vec) for (u32 i = tid; i < I / 16; i += blockDim.x) grouped::cp_async16(to + r * I + 16u * i, c + 16u * i);
+            else for (u32 i = tid; i < I / 4; i += blockDim.x) *reinterpret_cast<u32*>(to + r * I + 4u * i) = *reinterpret_cast<const u32*>(c + 4u * i);
+            const float* d = v.act.deltas + u64(slot) * (stride / 32);
+            const i32* sm = v.act.sums ? v.act.sums + u64(slot) * (stride / 32) : nullptr;
+            for (u32 i = tid; i < groups; i += blockDim.x) {
+                grouped::cp_async4(deltas + r * groups + i, d + i);
+                if (Q51) grouped::cp_async4(sums + r * groups + i, sm + i);
+            }
+        }
+    };
+    auto entries = [&](u32 item, u32& first, u32& count) {
+        const u32 j = item / plan.n_chunks;
+        first = load(v.routes.begins + j);
+        count = load(v.routes.begins + j + 1) - first;
+    };
+    u32 first = 0, count = 0;
+    if (blockIdx.x < n_items) {
+        entries(blockIdx.x, first, count);
+        stage(0, first, min(plan.cap, count));
+    }
+    bool ok = true;
+    u32 n = 0;
+    for (u32 item = blockIdx.x; item < n_items; item += gridDim.x, ++n) {
+        const u32 b = n & 1u, o = R * (item % plan.n_chunks) + my_row;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        u32 next_first = 0, next_count = 0;
+        if (item + gridDim.x < n_items) {
+            entries(item + gridDim.x, next_first, next_count);
+            stage(b ^ 1u, next_first, min(plan.cap, next_count));
+        }
+        ok = q4k::mbar_wait(&full[b], (n >> 1) & 1u, plan.wait_limit, &s_abort);
+        if (__syncthreads_or(!ok)) { ok = false; break; }
+        const unsigned char* wrow = smem_raw + b * plan.stage_bytes + u64(my_row) * row_bytes;
+        const unsigned char* from = a8 + b * plan.a8_bytes;
+        const float* deltas = reinterpret_cast<const float*>(from + plan.cap * I);
+        const i32* sums = reinterpret_cast<const i32*>(deltas + plan.cap * groups);
+        for (u32 p0 = 0; p0 < count; p0 += plan.cap) {
+            const u32 nr = min(plan.cap, count - p0);
+            if (p0) {  // an expert of more entries: the passes after the first
+                __syncthreads();
+                stage(b, first + p0, nr);
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncthreads();
+            }
+            float acc[kR];
+#pragma unroll
+            for (int r = 0; r < kR; ++r) acc[r] = 0.0f;
+#pragma unroll 2
+            for (u32 g = chain; g < groups; g += 4) {
+                ChainBlock<Q51> w;
+                load_chain_block<Q51>(wrow + g * block, w);
+                spread_chain_block<Q51>(w);
+#pragma unroll
+                for (int r = 0; r < kR; ++r) {
+                    if (r < (int)nr) {
+                        const uint4* c = reinterpret_cast<const uint4*>(from + r * I + 32u * g);
+                        const uint4 c0 = c[0], c1 = c[1];
+                        int da = __dp4a((int)w.q[0], (int)c0.x, 0), db = __dp4a((int)w.q[4], (int)c1.x, 0);
+                        da = __dp4a((int)w.q[1], (int)c0.y, da); db = __dp4a((int)w.q[5], (int)c1.y, db);
+                        da = __dp4a((int)w.q[2], (int)c0.z, da); db = __dp4a((int)w.q[6], (int)c1.z, db);
+                        da = __dp4a((int)w.q[3], (int)c0.w, da); db = __dp4a((int)w.q[7], (int)c1.w, db);
+                        float combined = __fmul_rn(w.d, static_cast<float>(da + db));
+                        if (Q51) combined = __fadd_rn(combined, __fmul_rn(w.mn, static_cast<float>(sums[r * groups + g])));
+                        acc[r] = __fadd_rn(acc[r], __fmul_rn(deltas[r * groups + g], combined));
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < kR; ++r) {
+                if (r < (int)nr) {  // uniform over the block
+                    const float pair = __fadd_rn(acc[r], __shfl_xor_sync(0xffffffffu, acc[r], 1));
+                    const float y = __fadd_rn(pair, __shfl_xor_sync(0xffffffffu, pair, 2));
+                    if (chain == 0) v.raw[u64(s_slots[b][r]) * H + o] = y;
+                }
+            }
+        }
+        __syncthreads();  // the stage and the buffer have been read
+        if (tid == 0 && item + 2 * gridDim.x < n_items) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            ask(n + 2, item + 2 * gridDim.x);
+            ++asked;
+        }
+        first = next_first; count = next_count;
+    }
+    if (!ok) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (tid == 0) {
+            drain(n);
+            if (v.summary) atomicOr(const_cast<u32*>(v.summary), q4k::kAbortBit);
+        }
+    }
+}
+
+// Rows of an item and entries of a pass: as many rows (64, 32 or 16) as let three CTAs share a multiprocessor, fewer CTAs for rows so long that not even 16
+// do. False: the rows are too long for two stages.
+bool chain_plan(const b200moe_down_view& v, ChainPlan* p, u32* smem, u32* per_sm) {
+    const u32 I = v.shape.inter, H = v.shape.hidden, block = v.shape.down_type == B200MOE_TYPE_Q5_1 ? kQ51Block : kQ8Block;
+    const u64 row_bytes = u64(I / 32) * block;
+    p->cap = std::min<u32>(kR, std::max(1u, v.act.rows / v.shape.top_k));
+    p->a8_bytes = (p->cap * (I + I / 32 * 8) + 15u) / 16u * 16u;
+    p->wait_limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT) ? debug_value(B200MOE_DEBUG_WAIT_LIMIT) : 1u << 18;
+    for (u32 R = 64; R >= 16; R /= 2) {
+        const u64 stage = (R * row_bytes + 127) / 128 * 128, total = 2 * (stage + p->a8_bytes);
+        if (total > 75u * 1024u && !(R == 16 && total <= 226u * 1024u)) continue;
+        p->rows_per_item = R; p->n_chunks = H / R; p->stage_bytes = static_cast<u32>(stage);
+        *smem = static_cast<u32>(total);
+        *per_sm = std::max(1u, std::min(2048u / (4u * R), 227u * 1024u / (*smem + 1024u)));
+        return u64(p->n_chunks) * v.max_union < (1u << 30);
+    }
+    return false;
+}
+
 template <class K>
 int set_smem(K kernel, u32 bytes) {
     return ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), bytes);
@@ -435,17 +608,24 @@ int launch_down_q4k(const b200moe_down_view& v, cudaStream_t stream) {
     return after_launch("down_q4k");
 }
 
-int launch_down_q8_chain4(const b200moe_down_view& v, cudaStream_t stream) {
+int launch_down_q8_chain4(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream) {
     const u32 H = v.shape.hidden, I = v.shape.inter;
     if (v.max_union == 0) return B200MOE_OK;
-    const u32 smem = kR * (I + I / 32 * 8);
-    if (v.shape.down_type == B200MOE_TYPE_Q5_1) {
-        if (int rc = set_smem(down_q8_chain4_kernel<true>, smem)) return rc;
-        chain_launch(down_q8_chain4_kernel<true>, dim3(H / 64, v.max_union), 256, smem, stream, v);
-    } else {
-        if (int rc = set_smem(down_q8_chain4_kernel<false>, smem)) return rc;
-        chain_launch(down_q8_chain4_kernel<false>, dim3(H / 64, v.max_union), 256, smem, stream, v);
+    const bool q51 = v.shape.down_type == B200MOE_TYPE_Q5_1;
+    ChainPlan p{};
+    u32 smem = 0, per_sm = 0;
+    if (debug_value(B200MOE_DEBUG_DECODE_FORM) != 3 && aligned(v.weights.down, 16) && chain_plan(v, &p, &smem, &per_sm)) {
+        p.early = hints.routes_done;
+        const u32 grid = static_cast<u32>(std::min<u64>(u64(per_sm) * static_cast<u32>(device_sm_count()), u64(p.n_chunks) * v.max_union));
+        const auto kernel = q51 ? down_chain4_stream_kernel<true> : down_chain4_stream_kernel<false>;
+        if (int rc = set_smem(kernel, smem)) return rc;
+        chain_launch(kernel, grid, 4 * p.rows_per_item, smem, stream, v, p);
+        return after_launch("down_chain4_stream");
     }
+    const u32 bytes = kR * (I + I / 32 * 8);
+    const auto kernel = q51 ? down_q8_chain4_kernel<true> : down_q8_chain4_kernel<false>;
+    if (int rc = set_smem(kernel, bytes)) return rc;
+    chain_launch(kernel, dim3(H / 64, v.max_union), 256, bytes, stream, v);
     return after_launch("down_q8_chain4");
 }
 

@@ -774,3 +774,21 @@ def test_down_skipped_after_its_weights_were_asked_for(gpu, oracle, rows, H, I, 
             y = layer(fail, ids, one, row_status=status)
             assert int(status[rows - 1]) == b200moe.ROW_PROJECTION_NONFINITE and not y[rows - 1].any()
             assert same(layer(good, ids, one).cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("down_type", [7, 8])
+@pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 256, 32), (4, 8, 16, 512, 640), (9, 2, 3, 256, 544), (20, 1, 1, 512, 1536), (3, 2, 4, 256, 3104), (2, 1, 2, 256, 8192)])
+def test_four_chain_down_by_bulk_copies(gpu, oracle, rows, top_k, E, H, I, down_type):
+    """Items of 64, 32 and 16 rows, rows too long for them, 1 to 20 entries an expert (several passes), more items than CTAs and fewer."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)
+    sh = ops.make_shape(H, I, E, top_k, 12, down_type)
+    layer = ops.MoeLayer(sh, dv(gate, gpu), dv(up, gpu), dv(down, gpu), capacity=rows, combine_form=b200moe.COMBINE_FMA_SLOTS)
+    x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
+    for _ in range(2):
+        assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])

@@ -307,7 +307,7 @@ Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_f
 // 1024 or above 7168 weights) the grouped one takes over from the dp4a form at 4 entries an expert: down of 48 experts of 2048 x 512 36.8 and 39 us with 3,
 // 41 and 38.5 with 4, 49 and 39 with 5; of 32 of 1536 x 768 29 and 28 with 4.5; one expert of 2048 x 17408 45 and 43 us with 8 rows, 53.4 and 53.5 with
 // 17, of 4096 x 12288 35 and 33 with 8, 84 and 40 with 24.
-enum class Q8Form { row_per_warp, wide, mma, grouped };
+enum class Q8Form { row_per_warp, shot, wide, mma, grouped };
 bool q8_grouped_pays(const b200moe_shape& s, bool mma_fits, u32 rows, u32 max_union, bool down) {
     if (rows < kRowStreamRows) return false;
     if (!mma_fits) return u64(rows) * s.top_k >= u64(4) * s.experts;
@@ -317,7 +317,7 @@ bool q8_grouped_pays(const b200moe_shape& s, bool mma_fits, u32 rows, u32 max_un
     const u64 grouped = waves(w.tiles32 * (down ? s.hidden / 64 : s.inter / 32), sms) * tile, tensor = waves(w.items8 * ((down ? s.hidden : s.inter) / 32), sms) * item;
     return grouped < tensor;
 }
-Q8Form pick_q8_form(const b200moe_shape& s, bool wide_fits, bool mma_fits, bool grouped_fits, u32 rows, u32 max_union, bool down) {
+Q8Form pick_q8_form(const b200moe_shape& s, bool shot_fits, bool wide_fits, bool mma_fits, bool grouped_fits, u32 rows, u32 max_union, bool down) {
     const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
     if (forced == 3) return Q8Form::row_per_warp;
     if (grouped_fits && (forced == 5 || (forced == 0 && q8_grouped_pays(s, mma_fits, rows, max_union, down)))) return Q8Form::grouped;
@@ -327,12 +327,14 @@ Q8Form pick_q8_form(const b200moe_shape& s, bool wide_fits, bool mma_fits, bool 
         if (mma_fits) return Q8Form::mma;
         if (wide_fits) return Q8Form::wide;
     }
+    if (forced == 0 && rows < kRowStreamRows && shot_fits) return Q8Form::shot;
     return Q8Form::row_per_warp;
 }
 int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0, const ChainHints& hints = {}) {
     if (v.shape.gate_type == B200MOE_TYPE_Q2_K) return launch_gate_up_ds41_any(v, st);  // the generic form of the family reads every block type
     if (!is_kquant(v.shape.gate_type)) {
-        switch (pick_q8_form(v.shape, q8_wide_gate_up_fits(v, rows), q8_mma_gate_up_fits(v, rows), grouped_q8_gate_up_fits(v), rows, v.max_union, false)) {
+        switch (pick_q8_form(v.shape, q8_shot_gate_up_fits(v, rows), q8_wide_gate_up_fits(v, rows), q8_mma_gate_up_fits(v, rows), grouped_q8_gate_up_fits(v), rows, v.max_union, false)) {
+            case Q8Form::shot: return launch_gate_up_q8_shot(v, rows, hints, st);
             case Q8Form::grouped: return launch_gate_up_q8_grouped(v, st);
             case Q8Form::mma: return launch_gate_up_q8_mma(v, rows, st);
             case Q8Form::wide: return launch_gate_up_q8_wide(v, rows, st);
@@ -358,7 +360,8 @@ int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grou
     }
     if (is_kquant(v.shape.gate_type)) return launch_down_q8_chain4(v, hints, st);  // chain4: Q8_0 and Q5_1 blocks
     if (v.shape.down_type == B200MOE_TYPE_Q2_K) return launch_down_ds41_any(v, st);
-    switch (pick_q8_form(v.shape, q8_wide_down_fits(v, rows), q8_mma_down_fits(v, rows), grouped_q8_down_fits(v), rows, v.max_union, true)) {
+    switch (pick_q8_form(v.shape, q8_shot_down_fits(v, rows), q8_wide_down_fits(v, rows), q8_mma_down_fits(v, rows), grouped_q8_down_fits(v), rows, v.max_union, true)) {
+        case Q8Form::shot: return launch_down_q8_shot(v, rows, hints, st);
         case Q8Form::grouped: return launch_down_q8_grouped(v, st);
         case Q8Form::mma: return launch_down_q8_mma(v, rows, st);
         case Q8Form::wide: return launch_down_q8_wide(v, rows, st);

@@ -65,6 +65,11 @@ bool wide_gate_up_fits(const b200moe_gate_up_view& v, u32 rows);
 bool wide_down_fits(const b200moe_down_view& v, u32 rows);
 int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
 int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
+// gemv_q8_shot.cu: the same contract, a CTA one item with all of its weights asked for at once (windows of a few rows)
+bool q8_shot_gate_up_fits(const b200moe_gate_up_view& v, u32 rows);
+bool q8_shot_down_fits(const b200moe_down_view& v, u32 rows);
+int launch_gate_up_q8_shot(const b200moe_gate_up_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
+int launch_down_q8_shot(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
 // gemv_q8_wide.cu: the Q8_0 x A8 lane-class contract in the same streaming skeleton, for windows of many rows.
 bool q8_wide_gate_up_fits(const b200moe_gate_up_view& v, u32 rows);
 bool q8_wide_down_fits(const b200moe_down_view& v, u32 rows);

@@ -792,3 +792,27 @@ def test_four_chain_down_by_bulk_copies(gpu, oracle, rows, top_k, E, H, I, down_
     x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
     for _ in range(2):
         assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 256, 256), (1, 4, 8, 2048, 1024), (2, 2, 3, 1280, 2304), (3, 2, 4, 3328, 512), (7, 1, 1, 7168, 4352), (7, 3, 3, 4096, 1024), (5, 2, 40, 512, 768)])
+def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I):
+    """Windows below 8 rows: rows of one run, of whole and broken runs, of more runs than places; 1 to 7 entries an expert, in one pass and in several."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + H)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 8, 8)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 8, 8, 7.0), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, top_k, 8, 8, 7.0)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    w = dv(gate, gpu), dv(up, gpu), dv(down, gpu)
+    x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
+    act, g, u = ops.enqueue_routed_gate_up(sh, *w[:2], r, E, x, rows * top_k, taps=True)
+    assert b200moe.last_launch() == "gate_up_q8"
+    raw = ops.enqueue_routed_down(sh, w[2], r, E, act)
+    assert b200moe.last_launch() == "down_q8"
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+    layer = ops.MoeLayer(sh, *w, capacity=rows, combine_form=b200moe.COMBINE_PARTS, parts=1)
+    for _ in range(2):  # down asks for its weights before its wait
+        assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])

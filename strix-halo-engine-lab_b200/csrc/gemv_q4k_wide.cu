@@ -13,7 +13,7 @@
 //  * A stage = S = 3 super-blocks of the item's 64 rows (one or two tiled TMA copies of 432 bytes x 32 / 64 rows: the rows
 //    lie 432 bytes apart in shared memory, an odd count of 16-byte units, which keeps the 128-bit reads of eight rows
 //    conflict free) PLUS the same K range of the A8 rows of the item's entries (codes, deltas, sums: three bulk copies per
-//    entry), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
+//    entry, or 16-byte asynchronous copies), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
 //  * Two groups of eight consumer warps share a CTA, each with its own ring of stages and its own producer warp; a group's
 //    producer claims the next item of the grid while its consumers still work on the stages in the ring. The serial chains
 //    acc_p += pair_p never leave their lane.
@@ -224,7 +224,10 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk
 
 // 18 warps: two of the SM's four register partitions (16 K registers each) hold five warps, which caps a thread at
 // 16384 / (5 x 32) = 102 registers, 96 after rounding - what this launch bound gives (112 was tried: the launch is refused).
-template <bool DOWN, u32 S_>
+// ASYNC: how the entries' A8 rows come in. A bulk copy holds the producer for about 180 clocks, 24 of them a stage for eight entries; asynchronous copies cost
+// instructions that a stage of few entries does not repay. Bulk and asynchronous, us a call: dense 5120 x 17408, 8 rows 77.8 and 74.8, 16 rows 112.5 and
+// 109.7, 5 rows 70.8 and 72.7, 1 row 43.9 and 50. A choice per item inside one kernel costs the items of one entry 1.5 us of these 43.9.
+template <bool DOWN, u32 S_, bool ASYNC>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, WideArgs a, WidePlan plan) {
     using G = Geo<S_>;
@@ -275,10 +278,27 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         u64* g_empty = empty + g * plan.stages;
         u32* g_item = slot_item + g * plan.stages;
         unsigned char* g_stage = smem + g * plan.stages * plan.stage_bytes;
-        const u32 e = lane / 3u, part = lane - 3u * e;  // lanes 0 .. 3 * ne - 1 copy one piece of one entry each
+        const u32 e = lane / 3u, part = lane - 3u * e;  // bulk copies: lanes 0 .. 3 * ne - 1 copy one piece of one entry each
         const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, in_gs = in_stride / 32;
         u32 t = 0, slot = 0, use = 0;  // stage count, ring position, lap
         bool ok = true, first = true;
+        // ASYNC: 16-byte asynchronous copies, 20 units a super-block and entry {16 of codes, 2 of deltas, 2 of sums}; a lane takes units `lane` and `lane` + 32 of every entry.
+        auto copy_entries = [&](u32 s, u32 nbk, u32 ne, u32 my_row, unsigned char* xd) {
+#pragma unroll
+            for (u32 half = 0; half < (20u * G::S + 31u) / 32u; ++half) {
+                const u32 u = lane + 32u * half;
+                const bool is_codes = u < 16u * nbk, is_deltas = u < 18u * nbk;
+                const unsigned char* base = is_codes ? reinterpret_cast<const unsigned char*>(a.in.codes) + s * G::S * 256u + 16u * u
+                                          : is_deltas ? reinterpret_cast<const unsigned char*>(a.in.deltas) + s * G::S * 32u + 16u * (u - 16u * nbk)
+                                                      : reinterpret_cast<const unsigned char*>(a.in.sums) + s * G::S * 32u + 16u * (u - 18u * nbk);
+                const u32 pitch = is_codes ? in_stride : in_stride / 8u;  // bytes between rows
+                unsigned char* to = xd + (is_codes ? 16u * u : is_deltas ? 256u * G::S + 16u * (u - 16u * nbk) : 288u * G::S + 16u * (u - 18u * nbk));
+                for (u32 e = 0; e < ne; ++e) {
+                    const u32 row = __shfl_sync(0xffffffffu, my_row, e);
+                    if (u < 20u * nbk) cp_async16(to + e * G::x_entry_bytes, base + u64(row) * pitch);
+                }
+            }
+        };
         auto ask_weights = [&](u32 s, const VExpert& ve, u32 chunk, unsigned char* dst, u64* bar) {  // one lane
             const u32 x = s * G::S * (kQ4KBlock / 8);  // 64-bit elements: a multiple of 18, i.e. of 144 bytes
             const u32 y = ve.expert() * a.rows_per_expert + (DOWN ? kItemRows : kHalfRows) * chunk;
@@ -330,8 +350,9 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 ve = table[jv];
             }
             const u32 ve_ne = ve.ne();
+            const u32 mine = ASYNC ? lane : e;  // the entry whose row the lane reads
             u32 r = 0;
-            if (e < ve_ne) r = plan.dense_rows ? ve.begin() + e : load((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + e);
+            if (mine < ve_ne) r = plan.dense_rows ? ve.begin() + mine : load((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + mine);
             const u32 nsegs = end ? 1u : plan.nseg;
             for (u32 s = 0; s < nsegs; ++s, ++t, ++slot) {
                 if (slot == plan.stages) { slot = 0; ++use; }
@@ -348,11 +369,18 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 unsigned char* dst = g_stage + slot * plan.stage_bytes;
                 if (lane == 0) {
                     g_item[slot] = item;
-                    mbar_expect_tx(&g_full[slot], (t < ahead ? 0u : G::w_bytes) + ve_ne * nbk * 320u);  // whole boxes: what lies past the row is filled
+                    const u32 w_bytes = t < ahead ? 0u : G::w_bytes;  // whole boxes: what lies past the row is filled
+                    if (ASYNC) mbar_expect_more(&g_full[slot], w_bytes);
+                    else mbar_expect_tx(&g_full[slot], w_bytes + ve_ne * nbk * 320u);
                 }
                 __syncwarp();
                 if (lane == 0 && t >= ahead) ask_weights(s, ve, chunk, dst, &g_full[slot]);
-                if (e < ve_ne) {
+                if (ASYNC) {  // the arrival that lets the stage complete comes behind the lanes' copies, each of which adds one of its own while it is under way
+                    copy_entries(s, nbk, ve_ne, r, dst + G::w_bytes);
+                    asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(saddr(&g_full[slot])) : "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&g_full[slot]);
+                } else if (e < ve_ne) {
                     unsigned char* xd = dst + G::w_bytes + e * G::x_entry_bytes;
                     if (part == 0) bulk_g2s(xd, a.in.codes + u64(r) * in_stride + u64(s) * G::S * 256u, nbk * 256u, &g_full[slot]);
                     else if (part == 1) bulk_g2s(xd + 256u * G::S, a.in.deltas + u64(r) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
@@ -361,6 +389,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             }
             if (!ok || end) break;
         }
+        if (ASYNC) asm volatile("cp.async.wait_all;" ::: "memory");
         if (!ok && lane == 0) {  // wait (bounded) for the copies still in flight before the CTA retires
             for (u32 n = t > plan.stages ? t - plan.stages : 0u; n < t; ++n)
                 for (u32 i = 0; i < (plan.wait_limit >> 4) + 64u; ++i)
@@ -544,6 +573,9 @@ bool a8_bulk_ok(const b200moe_a8_rows& x) {
     return x.sums && aligned(x.codes, 16) && aligned(x.deltas, 16) && aligned(x.sums, 16) && stride % 128 == 0;
 }
 
+// Windows whose experts have kKE entries or more on average: their A8 rows come in by asynchronous copies (the figures are with the kernel).
+bool whole_items(u32 max_union, u64 slots) { return slots >= u64(kKE) * max_union; }
+
 void apply_hooks(WidePlan* p) {
     const u32 limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT), stall = debug_value(B200MOE_DEBUG_STALL_STAGE);
     if (limit) p->wait_limit = limit;
@@ -578,13 +610,9 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const Chain
     if (int rc = rows_map(v.weights.gate, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &tm0)) return rc;
     if (int rc = rows_map(v.weights.up, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &tm1)) return rc;
     const u32 smem = plan_smem(p);
-    if (p.S == 3) {
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<false, 3>), smem)) return rc;
-        chain_launch(q4k_wide_kernel<false, 3>, device_sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
-    } else {
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<false, 1>), smem)) return rc;
-        chain_launch(q4k_wide_kernel<false, 1>, device_sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
-    }
+    const auto kernel = p.S != 3 ? q4k_wide_kernel<false, 1, false> : whole_items(v.max_union, u64(rows) * v.shape.top_k) ? q4k_wide_kernel<false, 3, true> : q4k_wide_kernel<false, 3, false>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
+    chain_launch(kernel, device_sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
     return after_launch("gate_up_q4k_wide");
 }
 
@@ -601,13 +629,9 @@ int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints&
     CUtensorMap tm0;
     if (int rc = rows_map(v.weights.down, u64(p.nb) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, p.S * kQ4KBlock, kHalfRows, &tm0)) return rc;
     const u32 smem = plan_smem(p);
-    if (p.S == 3) {
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<true, 3>), smem)) return rc;
-        chain_launch(q4k_wide_kernel<true, 3>, device_sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
-    } else {
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(q4k_wide_kernel<true, 1>), smem)) return rc;
-        chain_launch(q4k_wide_kernel<true, 1>, device_sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
-    }
+    const auto kernel = p.S != 3 ? q4k_wide_kernel<true, 1, false> : whole_items(v.max_union, u64(rows) * v.shape.top_k) ? q4k_wide_kernel<true, 3, true> : q4k_wide_kernel<true, 3, false>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
+    chain_launch(kernel, device_sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
     return after_launch("down_q4k_wide");
 }
 

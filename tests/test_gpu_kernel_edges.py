@@ -776,24 +776,6 @@ def test_down_skipped_after_its_weights_were_asked_for(gpu, oracle, rows, H, I, 
             assert same(layer(good, ids, one).cpu(), want["raw"])
 
 
-@pytest.mark.parametrize("down_type", [7, 8])
-@pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 256, 32), (4, 8, 16, 512, 640), (9, 2, 3, 256, 544), (20, 1, 1, 512, 1536), (3, 2, 4, 256, 3104), (2, 1, 2, 256, 8192)])
-def test_four_chain_down_by_bulk_copies(gpu, oracle, rows, top_k, E, H, I, down_type):
-    """Items of 64, 32 and 16 rows, rows too long for them, 1 to 20 entries an expert (several passes), more items than CTAs and fewer."""
-    import b200moe
-    from b200moe import ops, synth
-    rng = np.random.default_rng(rows + I)
-    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
-    ids = window(rng, E, top_k, rows)
-    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
-    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)
-    sh = ops.make_shape(H, I, E, top_k, 12, down_type)
-    layer = ops.MoeLayer(sh, dv(gate, gpu), dv(up, gpu), dv(down, gpu), capacity=rows, combine_form=b200moe.COMBINE_FMA_SLOTS)
-    x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
-    for _ in range(2):
-        assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])
-
-
 @pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 256, 256), (1, 4, 8, 2048, 1024), (2, 2, 3, 1280, 2304), (3, 2, 4, 3328, 512), (7, 1, 1, 7168, 4352), (7, 3, 3, 4096, 1024), (5, 2, 40, 512, 768)])
 def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I):
     """Windows below 8 rows: rows of one run, of whole and broken runs, of more runs than places; 1 to 7 entries an expert, in one pass and in several."""
@@ -815,4 +797,39 @@ def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I):
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
     layer = ops.MoeLayer(sh, *w, capacity=rows, combine_form=b200moe.COMBINE_PARTS, parts=1)
     for _ in range(2):  # down asks for its weights before its wait
+        assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("rows,H,I", [(1, 512, 256), (1, 2560, 1280), (2, 64 * 148, 768), (4, 512, 1024), (5, 1024, 2048), (8, 2048, 1536), (8, 64 * 148 + 256, 512), (9, 512, 768), (7, 512, 768), (17, 1280, 2560)])
+def test_dense_rows_of_few_and_whole_items(gpu, oracle, rows, H, I):
+    """Dense blocks next to the line between bulk and asynchronous copies of the A8 rows (8 rows), with whole and broken last items, more and fewer items than
+    CTAs; rows of 1 to 10 super-blocks."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + H)
+    H = H // 256 * 256
+    gate, up, down = synth.expert_tensors(rng, 1, H, I, 12, 12)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, 1, 1, 12, 12, float("inf")), gate, up, down, np.zeros((rows, 1), np.uint32), codes, deltas, sums)
+    with forced(b200moe.FORM_SEGMENT_STREAM):
+        for _ in range(2):
+            y = ops.enqueue_dense_ffn(ops.make_shape(H, I, 1, 1, 12, 12), dv(gate, gpu), dv(up, gpu), dv(down, gpu), (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)))
+            assert b200moe.last_launch() == "down_q4k_wide" and same(y.cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("down_type", [7, 8])
+@pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 256, 32), (4, 8, 16, 512, 640), (9, 2, 3, 256, 544), (20, 1, 1, 512, 1536), (3, 2, 4, 256, 3104), (2, 1, 2, 256, 8192)])
+def test_four_chain_down_by_bulk_copies(gpu, oracle, rows, top_k, E, H, I, down_type):
+    """Items of 64, 32 and 16 rows, rows too long for them, 1 to 20 entries an expert (several passes), more items than CTAs and fewer."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)
+    sh = ops.make_shape(H, I, E, top_k, 12, down_type)
+    layer = ops.MoeLayer(sh, dv(gate, gpu), dv(up, gpu), dv(down, gpu), capacity=rows, combine_form=b200moe.COMBINE_FMA_SLOTS)
+    x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
+    for _ in range(2):
         assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])

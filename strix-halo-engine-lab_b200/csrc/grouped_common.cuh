@@ -48,40 +48,59 @@ __device__ __forceinline__ void drain(u64* full, u32 stages, u32 asked, u32 limi
 
 struct Tile { u32 expert, eb, nt, c, tt; };
 
-// cum[j]: token tiles of the first j experts of the union (n_union + 1 words of shared memory). Every thread of the block calls it.
-template <u32 GN>
-__device__ __forceinline__ void count_tiles(const b200moe_routes& routes, u32 n_union, u32* cum) {
+// Token tiles of an expert with n entries, GN entries each. SHORT_LAST: but for a last one of at most GN / 2, which is cheaper (half of the MMAs).
+template <u32 GN, bool SHORT_LAST>
+__device__ __forceinline__ u32 whole_tiles(u32 n) { return (n + (SHORT_LAST ? GN / 2 : GN) - 1) / GN; }
+
+// cum[j]: whole token tiles of the first j experts of the union; cum[kTileCounts + j]: their short last ones (n_union + 1 words each). Every thread of the
+// block calls it. Returns the token tiles of the window.
+constexpr u32 kTileCounts = kMaxUnion + 1;
+template <u32 GN, bool SHORT_LAST>
+__device__ __forceinline__ u32 count_tiles(const b200moe_routes& routes, u32 n_union, u32* cum) {
     const u32 tid = threadIdx.x, lane = tid & 31u;
-    for (u32 j = tid; j < n_union; j += blockDim.x) cum[j + 1] = (routes.begins[j + 1] - routes.begins[j] + GN - 1) / GN;
-    if (tid == 0) cum[0] = 0;
+    for (u32 j = tid; j < n_union; j += blockDim.x) {
+        const u32 n = routes.begins[j + 1] - routes.begins[j], whole = whole_tiles<GN, SHORT_LAST>(n);
+        cum[j + 1] = whole;
+        cum[kTileCounts + j + 1] = n > GN * whole ? 1u : 0u;
+    }
+    if (tid < 2) cum[kTileCounts * tid] = 0;
     __syncthreads();
-    if (tid < 32) {  // inclusive scan, 32 at a time
+    if (tid < 64) {  // inclusive scans, 32 at a time
+        u32* c = cum + kTileCounts * (tid >> 5);
         u32 carry = 0;
         for (u32 j0 = 0; j0 < n_union; j0 += 32) {
-            u32 v = j0 + lane < n_union ? cum[j0 + lane + 1] : 0u;
+            u32 v = j0 + lane < n_union ? c[j0 + lane + 1] : 0u;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) { const u32 o = __shfl_up_sync(0xffffffffu, v, d); if (lane >= (u32)d) v += o; }
-            if (j0 + lane < n_union) cum[j0 + lane + 1] = carry + v;
+            if (j0 + lane < n_union) c[j0 + lane + 1] = carry + v;
             carry += __shfl_sync(0xffffffffu, v, 31);
         }
     }
     __syncthreads();
+    return cum[n_union] + cum[kTileCounts + n_union];
 }
 
-// Tile id -> (union expert, token tile, row tile): row tiles fastest, then the expert's token tiles, experts ascending.
-template <u32 GN>
+// Tile id -> (union expert, token tile, row tile): row tiles fastest, then the expert's token tiles, experts ascending. SHORT_LAST: the whole token tiles of all
+// experts first, then the short ones. The CTAs walk the ids round-robin, so each then gets as many of either sort as any other, or one more; in one row of
+// experts their shares of the short ones are a matter of chance. Q8_0, 64 experts of 2048 -> 1024, 512 and 2048 rows of top 4: 327 -> 320 and 939 -> 932 us a
+// call. Not for Q4_K, whose short tiles cost nearly what whole ones do and find the weights in L2 behind these: 128 experts of 2048 -> 768, 512 and 4096
+// rows of top 8: 332 -> 337 and 1807 -> 1817.
+template <u32 GN, bool SHORT_LAST>
 __device__ __forceinline__ Tile find_tile(const b200moe_routes& routes, u32 n_row_tiles, const u32* cum, u32 n_union, u32 id) {
-    const u32 q = id / n_row_tiles;
+    u32 q = id / n_row_tiles;
     Tile t;
     t.c = id - q * n_row_tiles;
+    const u32 n_whole = cum[n_union];
+    const bool whole = !SHORT_LAST || q < n_whole;
+    if (!whole) { q -= n_whole; cum += kTileCounts; }
     u32 lo = 0, hi = n_union;  // largest j with cum[j] <= q
     while (hi - lo > 1) {
         const u32 mid = (lo + hi) >> 1;
         if (cum[mid] <= q) lo = mid; else hi = mid;
     }
-    t.tt = q - cum[lo];
     t.expert = routes.experts[lo];
     const u32 b0 = routes.begins[lo], b1 = routes.begins[lo + 1];
+    t.tt = whole ? q - cum[lo] : whole_tiles<GN, SHORT_LAST>(b1 - b0);
     t.eb = b0 + GN * t.tt;
     t.nt = min(GN, b1 - t.eb);
     return t;

@@ -64,7 +64,7 @@ static_assert(kOutBytes <= kFoldBytes / kThirds, "a third's epilogue tile takes 
 constexpr u32 kTilePlaces = 8, kTileWords = 4 + 2 * kGN;
 constexpr u32 kOffFold = kStages * kStageBytes, kOffBars = kOffFold + kFoldBytes, kOffTile = kOffBars + 3 * kStages * 8 + 8,
               kOffCum = kOffTile + kTilePlaces * kTileWords * 4;
-constexpr u32 kGroupedSmem = kOffCum + (kMaxUnion + 2) * 4;
+constexpr u32 kGroupedSmem = kOffCum + 2 * kTileCounts * 4;
 static_assert((kOutRows * kQ4KBlock) % 128 == 0 && kOffBars % 8 == 0, "TMA destinations, barriers");
 static_assert(kGN == 32 && kGM / 2 == (kHelpers - 1) * 32, "a helper lane stages a token, the helper threads before it two rows each");
 static_assert(kGroupedSmem > 114u * 1024u && kGroupedSmem <= 227u * 1024u, "one CTA per SM, within the shared memory of an SM");
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     u64* empty = ready + kStages;
     volatile u32* s_abort = reinterpret_cast<u32*>(empty + kStages);
     u32* s_tile = reinterpret_cast<u32*>(smem + kOffTile);             // [kTilePlaces][kTileWords]
-    u32* cum = reinterpret_cast<u32*>(smem + kOffCum);                 // [kMaxUnion + 1]
+    u32* cum = reinterpret_cast<u32*>(smem + kOffCum);                 // [2][kTileCounts]
 
     if (kDown && a.summary && *a.summary) return;  // a failed or aborted projection skips the stage (routed_expert.hpp:17-19)
 
@@ -207,8 +207,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    count_tiles<kGN>(a.routes, n_union, cum);
-    const u32 n_tiles = cum[n_union] * a.n_row_tiles;
+    const u32 n_tiles = count_tiles<kGN, false>(a.routes, n_union, cum) * a.n_row_tiles;
     const u32 I = a.shape.inter, H = a.shape.hidden;
     const u32 nblocks = a.K / 256;
     bool ok = true;
@@ -230,7 +229,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
         u32 nx_src = 0, nx_slot = 0;
         auto look_ahead = [&](u32 k) {
             if (k >= my_tiles) return;
-            nx = find_tile<kGN>(a.routes, a.n_row_tiles, cum, n_union, blockIdx.x + k * gridDim.x);
+            nx = find_tile<kGN, false>(a.routes, a.n_row_tiles, cum, n_union, blockIdx.x + k * gridDim.x);
             const u32 ent = nx.eb + min(lane, nx.nt - 1u);
             nx_slot = a.routes.slots[ent];
             nx_src = kDown ? nx_slot : a.routes.rows[ent];

@@ -51,7 +51,7 @@ constexpr u32 kOutBytes = kTokens * kOutPitch * 4;
 // kStages stages ahead, a tile has at least one: eight places.
 constexpr u32 kTilePlaces = 8, kTileWords = 4 + 2 * kTokens;
 constexpr u32 kOffSum = kStages * kStageBytes, kOffOut = kOffSum + kSumBytes, kOffBars = kOffOut + kOutBytes, kOffTile = kOffBars + 2 * kStages * 8 + 8,
-              kOffCum = kOffTile + kTilePlaces * kTileWords * 4, kSmem = kOffCum + (kMaxUnion + 2) * 4;
+              kOffCum = kOffTile + kTilePlaces * kTileWords * 4, kSmem = kOffCum + 2 * kTileCounts * 4;
 static_assert(kStageBytes % 128 == 0 && (32 * kUnitBytes) % 128 == 0 && kOffBars % 8 == 0, "TMA destinations, barriers");
 static_assert(kSmem > 114u * 1024u && kSmem <= 227u * 1024u, "one CTA per SM, within the shared memory of an SM");
 constexpr u32 kLaunchRegs = 65536u / kGThreads / 8u * 8u, kProducerRegs = 64;
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
     u64* empty = full + kStages;
     volatile u32* s_abort = reinterpret_cast<u32*>(empty + kStages);   // and the stages that the first producer has asked for
     u32* s_tile = reinterpret_cast<u32*>(smem + kOffTile);             // [kTilePlaces][kTileWords]
-    u32* cum = reinterpret_cast<u32*>(smem + kOffCum);                 // [kMaxUnion + 1]
+    u32* cum = reinterpret_cast<u32*>(smem + kOffCum);                 // [2][kTileCounts]
 
     if (kDown && a.summary && *a.summary) return;  // an aborted projection skips the stage
 
@@ -134,8 +134,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    count_tiles<kTokens>(a.routes, n_union, cum);
-    const u32 n_tiles = cum[n_union] * a.n_row_tiles;
+    const u32 n_tiles = count_tiles<kTokens, true>(a.routes, n_union, cum) * a.n_row_tiles;
     const u32 I = a.shape.inter, H = a.shape.hidden;
     const u32 units = a.K / 256;
     bool ok = true;
@@ -157,7 +156,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
         u32 nx_src = 0, nx_slot = 0;
         auto look_ahead = [&](u32 k) {
             if (k >= my_tiles) return;
-            nx = find_tile<kTokens>(a.routes, a.n_row_tiles, cum, n_union, blockIdx.x + k * gridDim.x);
+            nx = find_tile<kTokens, true>(a.routes, a.n_row_tiles, cum, n_union, blockIdx.x + k * gridDim.x);
             const u32 ent = nx.eb + min(lane, nx.nt - 1u);
             nx_slot = a.routes.slots[ent];
             nx_src = kDown ? nx_slot : a.routes.rows[ent];

@@ -103,25 +103,46 @@ __global__ void __launch_bounds__(kFewWarps * 32) router_logits_few_kernel(const
     }
 }
 
-// Windows of more than 4 rows: a CTA owns 8 rows x 16 experts and walks the hidden width in chunks of COLS columns that
-// all 128 threads stage into shared memory with 16-byte asynchronous copies, three chunks in flight; a warp keeps an
-// 8 x 4 tile of lane-class sums. Chunks of 256 columns leave room for three CTAs an SM, of 512 for one: with more tiles than SMs the
-// former hide each other's latency (8192 x 256 x 7168: 2309 us with 512, 1442 with 256, 1271 with two rows a packed instruction too; two FP32
-// operations a product bound it at 835), a window with fewer tiles is a chain of chunks and wants the longer ones (64 x 256 x 7168: 23 against 33 us). The x tile
-// is then read from HBM / L2 once per 16 experts instead of once per expert (a
-// 64-row window over 256 experts of width 7168 pulled 470 MB through L2 in the form above), and the copies of two chunks
-// cover the arithmetic of one. Same products, same order: lane l of a warp meets columns l, l + 32, ... ascending.
-constexpr u32 kTileRows = 8, kTileExperts = 16, kTileStages = 3;
-constexpr u32 tile_smem_bytes(u32 cols) { return kTileStages * (kTileRows + kTileExperts) * cols * 4u; }
+// Windows of more than 4 rows: a CTA owns 8 WR rows x 4 ET experts and walks the hidden width in chunks of COLS columns that
+// all its threads stage into shared memory with 16-byte asynchronous copies, three chunks in flight; a warp keeps an
+// 8 x ET tile of lane-class sums. Same products, same order: lane l of a warp meets columns l, l + 32, ... ascending. Three sizes of it:
+//  * 512 columns, 8 x 16: windows with no more tiles than multiprocessors, a chain of chunks (64 x 256 x 7168: 21 us, 33 with 256 columns).
+//  * 256 columns, 8 x 16: room for three CTAs a multiprocessor, which hide each other's latency, and two rows a packed instruction.
+//  * 128 columns, 16 x 32: two CTAs of eight warps, a warp 8 x 8. A column costs a warp 16 reads of shared memory for 64 products where the form above reads
+//    12 for 32, and a row of x comes out of L2 half as often. 8192 x 256 x 7168 1243 -> 1108 us, 4096 x 128 x 2048 101 -> 89; two FP32 operations a
+//    product bound them at 835 and 60. With few waves of its larger tiles it is no better: 1500 x 128 x 2560 50.9 and 50.0, 2048 x 128 x 2048 52.5
+//    and 52.6, 1024 x 256 x 7168 169.7 and 171.9.
+// A tile's end: the sums of 32 cells meet at once (butterfly32_all); cell by cell they took 160 exchanges instead of 31 (8 x 128 x 2048 8.2 -> 7.0 us,
+// 4096 x 128 x 2048 109 -> 101).
+constexpr u32 kTileStages = 3;
+template <u32 WR, u32 ET>
+struct LogitsTile {
+    static constexpr u32 rows = 8 * WR, experts = 4 * ET, threads = 128 * WR;
+    static constexpr u32 smem_bytes(u32 cols) { return kTileStages * (rows + experts) * cols * 4u; }
+};
 
-template <u32 kTileCols>
-__global__ void __launch_bounds__(128) router_logits_tile_kernel(const float* x, u32 x_stride, u32 rows, u32 hidden,
+// butterfly32 of 32 values at once: each step hands half of what is left to the lane's partner, so that 31 exchanges do for 160. Lane l ends with value l.
+__device__ __forceinline__ float butterfly32_all(float (&v)[32], u32 lane) {
+#pragma unroll
+    for (u32 d = 16; d; d >>= 1)
+#pragma unroll
+        for (u32 i = 0; i < d; ++i) {
+            const bool up = lane & d;
+            const float theirs = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + d], d);
+            v[i] = __fadd_rn(up ? v[i + d] : v[i], theirs);
+        }
+    return v[0];
+}
+
+template <u32 kTileCols, u32 WR, u32 ET>
+__global__ void __launch_bounds__(128 * WR) router_logits_tile_kernel(const float* x, u32 x_stride, u32 rows, u32 hidden,
                                                                  const float* w, u32 experts,
                                                                  const float* logit_bias, float* logits) {
     chain_begin();
     extern __shared__ __align__(16) float tile_smem[];
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    constexpr u32 ET = kTileExperts / 4, kTileStageFloats = (kTileRows + kTileExperts) * kTileCols;
+    constexpr u32 kTileRows = LogitsTile<WR, ET>::rows, kTileExperts = LogitsTile<WR, ET>::experts, kTileStageFloats = (kTileRows + kTileExperts) * kTileCols;
+    const u32 wr = 8u * (warp >> 2), we = ET * (warp & 3u);  // the warp's first row and expert of the tile
     const u32 r0 = blockIdx.y * kTileRows, e0 = blockIdx.x * kTileExperts;
     const u32 n_chunks = (hidden + kTileCols - 1) / kTileCols;
     auto issue = [&](u32 c) {
@@ -131,7 +152,7 @@ __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float* x,
             const u32 at = tid % (kTileCols / 4), j0 = tid / (kTileCols / 4);
             if (at < nvec) {
 #pragma unroll
-                for (u32 j = j0; j < kTileRows + kTileExperts; j += 512 / kTileCols) {
+                for (u32 j = j0; j < kTileRows + kTileExperts; j += 512 * WR / kTileCols) {
                     const float* src = j < kTileRows ? x + u64(min(r0 + j, rows - 1)) * x_stride : w + u64(min(e0 + j - kTileRows, experts - 1)) * hidden;
                     cp_async16(st + j * kTileCols + 4 * at, src + col0 + 4 * at);
                 }
@@ -139,48 +160,59 @@ __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float* x,
         }
         asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group keeps the count of the wait below fixed
     };
-    float2 acc[kTileRows / 2][ET];  // pairs of rows
+    float2 acc[4][ET];  // pairs of rows
 #pragma unroll
-    for (int r = 0; r < (int)kTileRows / 2; ++r)
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int e = 0; e < (int)ET; ++e) acc[r][e] = make_float2(0.0f, 0.0f);
     issue(0);
     issue(1);
     for (u32 c = 0; c < n_chunks; ++c) {
-        issue(c + 2);
-        asm volatile("cp.async.wait_group 2;" ::: "memory");
-        __syncthreads();
+        if (kTileCols == 512) {
+            issue(c + 2);
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            __syncthreads();
+        } else {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+            issue(c + 2);
+        }
         const float* st = tile_smem + (c % kTileStages) * kTileStageFloats;
         const u32 ncol = min(kTileCols, hidden - c * kTileCols);
 #pragma unroll 4
         for (u32 col = lane; col < ncol; col += 32) {
-            float2 xv[kTileRows / 2];
+            float2 xv[4];
             float wv[ET];
 #pragma unroll
-            for (int r = 0; r < (int)kTileRows / 2; ++r) xv[r] = make_float2(st[2 * r * kTileCols + col], st[(2 * r + 1) * kTileCols + col]);
+            for (int r = 0; r < 4; ++r) xv[r] = make_float2(st[(wr + 2 * r) * kTileCols + col], st[(wr + 2 * r + 1) * kTileCols + col]);
 #pragma unroll
-            for (int e = 0; e < (int)ET; ++e) wv[e] = st[(kTileRows + ET * warp + e) * kTileCols + col];
+            for (int e = 0; e < (int)ET; ++e) wv[e] = st[(kTileRows + we + e) * kTileCols + col];
 #pragma unroll
-            for (int r = 0; r < (int)kTileRows / 2; ++r)
+            for (int r = 0; r < 4; ++r)
 #pragma unroll
                 for (int e = 0; e < (int)ET; ++e) {
-                    if (kTileCols == 256) acc[r][e] = grouped::add2(grouped::mul2(grouped::both(wv[e]), xv[r]), acc[r][e]);
+                    if (kTileCols <= 256) acc[r][e] = grouped::add2(grouped::mul2(grouped::both(wv[e]), xv[r]), acc[r][e]);
                     else acc[r][e] = make_float2(__fadd_rn(acc[r][e].x, __fmul_rn(wv[e], xv[r].x)), __fadd_rn(acc[r][e].y, __fmul_rn(wv[e], xv[r].y)));
                 }
         }
-        __syncthreads();  // the stage is refilled by the copies issued two iterations on
+        if (kTileCols == 512) __syncthreads();  // the stage is refilled by the copies issued two iterations on
     }
+    constexpr u32 kSetRows = 32 / ET;  // 32 cells at a time
 #pragma unroll
-    for (int r = 0; r < (int)kTileRows; ++r)
+    for (u32 s = 0; s < 8 / kSetRows; ++s) {
+        float v[32];
 #pragma unroll
-        for (int e = 0; e < (int)ET; ++e) {
-            float z = butterfly32(r & 1 ? acc[r / 2][e].y : acc[r / 2][e].x);
-            const u32 row = r0 + r, ex = e0 + ET * warp + e;
-            if (lane == 0 && row < rows && ex < experts) {
-                if (logit_bias) z = __fadd_rn(z, logit_bias[ex]);
-                logits[u64(row) * experts + ex] = z;
-            }
+        for (u32 i = 0; i < 32; ++i) {
+            const u32 r = kSetRows * s + i / ET;
+            v[i] = r & 1u ? acc[r / 2][i % ET].y : acc[r / 2][i % ET].x;
         }
+        float z = butterfly32_all(v, lane);
+        const u32 row = r0 + wr + kSetRows * s + lane / ET, ex = e0 + we + lane % ET;
+        if (row < rows && ex < experts) {
+            if (logit_bias) z = __fadd_rn(z, logit_bias[ex]);
+            logits[u64(row) * experts + ex] = z;
+        }
+    }
 }
 
 }  // namespace
@@ -218,10 +250,12 @@ int launch_router_logits(const b200moe_router_view& v, cudaStream_t stream, cons
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(router_logits_few_kernel<RT>), smem)) return rc;               \
         small_launch(router_logits_few_kernel<RT>, (E + kFewWarps - 1) / kFewWarps, kFewWarps * 32, smem, stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
     }
-#define B200_TILE(COLS)                                                                                                               \
+#define B200_TILE(COLS, WR, ET)                                                                                                       \
     {                                                                                                                                 \
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(router_logits_tile_kernel<COLS>), tile_smem_bytes(COLS))) return rc; \
-        small_launch(router_logits_tile_kernel<COLS>, grid, 128, tile_smem_bytes(COLS), stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
+        using T = LogitsTile<WR, ET>;                                                                                                 \
+        const auto kernel = router_logits_tile_kernel<COLS, WR, ET>;                                                                  \
+        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), T::smem_bytes(COLS))) return rc;                      \
+        small_launch(kernel, dim3((E + T::experts - 1) / T::experts, (v.rows + T::rows - 1) / T::rows), T::threads, T::smem_bytes(COLS), stream, v.x, xs, v.rows, v.hidden, v.weight, E, v.logit_bias, v.logits); \
     }
     if (v.rows <= 4 && vec) {
         if (v.rows == 1) B200_FEW(1)
@@ -231,9 +265,12 @@ int launch_router_logits(const b200moe_router_view& v, cudaStream_t stream, cons
     else if (v.rows == 2) B200_LOGITS(2, 1);
     else if (v.rows <= 4) B200_LOGITS(4, 1);
     else if (vec) {
-        const dim3 grid((E + kTileExperts - 1) / kTileExperts, (v.rows + kTileRows - 1) / kTileRows);
-        if (u64(grid.x) * grid.y > static_cast<u32>(device_sm_count())) B200_TILE(256)
-        else B200_TILE(512)
+        // the figures are with the kernel
+        auto tiles = [&](u32 rows, u32 experts) { return u64((v.rows + rows - 1) / rows) * ((E + experts - 1) / experts); };
+        const u64 sms = static_cast<u32>(device_sm_count());
+        if (tiles(LogitsTile<2, 8>::rows, LogitsTile<2, 8>::experts) >= 6 * sms) B200_TILE(128, 2, 8)
+        else if (tiles(LogitsTile<1, 4>::rows, LogitsTile<1, 4>::experts) > sms) B200_TILE(256, 1, 4)
+        else B200_TILE(512, 1, 4)
     } else if (v.rows <= 16) B200_LOGITS(8, 1);
     else B200_LOGITS(8, 4);
 #undef B200_FEW

@@ -833,3 +833,15 @@ def test_four_chain_down_by_bulk_copies(gpu, oracle, rows, top_k, E, H, I, down_
     x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
     for _ in range(2):
         assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("rows,hidden,experts", [(1, 132, 1), (5, 100, 33), (9, 516, 15), (600, 260, 40), (1201, 388, 17), (7120, 132, 33), (14207, 4, 1), (3560, 260, 130)])
+def test_router_logits_tiles(gpu, rows, hidden, experts):
+    """The three tile sizes, with rows, experts and columns that end inside a tile, a run of 32 columns and a chunk."""
+    from b200moe import ops
+    rng = np.random.default_rng(rows)
+    x, w, b = (rng.standard_normal(s, dtype=np.float32) for s in ((rows, hidden), (experts, hidden), experts))
+    z = ops.enqueue_router(ops.softmax_policy(experts, 1), x=dv(x, gpu), weight=dv(w, gpu), logit_bias=dv(b, gpu))[0]
+    at = np.unique(np.concatenate([np.arange(min(rows, 33)), np.arange(max(0, rows - 33), rows)]))
+    whole = [(0, 0), (0, -hidden % 32)]  # zero products leave a sum that starts at +0 as it is
+    assert same(z.cpu().numpy()[at], declared_logits(np.pad(x[at], whole), np.pad(w, whole)) + b)

@@ -252,14 +252,12 @@ u64 waves(u64 items, u64 at_once) { return (items + at_once - 1) / at_once; }
 // windows of Q4_K experts take the persistent bulk-copy forms, prompts the grouped form.
 // grouped_min_rows: windows of at least that many rows take the grouped form; 0 = chosen here, for gate/up and down each.
 // Where the segment-streaming form applies, the grouped one (tiles of 32 entries) takes over from it (items of 8) where its waves take less time,
-// both by their sizes: a tile 2 us + 1.75 a super-block of its rows; an item 1.2 us + 0.7 a super-block (2 + 0.7 where rows have less than three and a
-// stage holds one), two an SM, or 0.5 a super-block where there are no more items than SMs. Streaming and grouped form, gate/up and down: one expert of
-// 5120 x 17408 139 and 90 us, 103 and 126 with 32 rows, 254 and 129, 160 and 126 with 64; of 2048 x 17408 68 and 45, 39 and 126 with 32, 119 and 64, 60
-// and 125 with 64 (11 down tiles); of 2048 x 8192 60 and 45, 33 and 62 with 64; of 256 x 512 8.4 and 12.4, 9 and 10.4 with 64; 128 of 2048 x 768, top-8,
-// 105 and 116, 58 and 71 with 128 rows, 146 and 118, 77 and 73 with 192; 64 of 7168 x 2048, top-8, 466 and 488, 239 and 256 with 80, 545 and 491,
-// 279 and 253 with 96; 96 of 2560 x 1280, top-2, 170 and 186, 88 and 101 with 432; 16 of 2048 x 1024, top-2, 33 and 36, 21 and 21 with 96. Over 199
-// windows (16 to 1000 rows, 1 to 160 experts) the two launches together take at most 2.5 % longer than in the streaming form. The estimate is good
-// to a few percent; below 32 rows it has not been followed, below 48 only where it sees a quarter of the time gained.
+// both by their sizes: a tile 2 us + 1.75 a super-block of its rows; an item 1 us + 0.56 a super-block (1.7 + 0.56 where rows have less than three and a
+// stage holds one), two an SM, or 0.5 a super-block where there are no more items than SMs. Whole calls with both launches in the streaming and in the
+// grouped form, us: 128 experts of 2048 x 768, top-8, 167 and 216 with 128 rows, 200 and 220 with 160, 223 and 226 with 192; 64 of 7168 x 2048, top-8,
+// 548 and 778 with 64 rows, 639 and 778 with 80, 741 and 793 with 96, 896 and 813 with 128; one expert of 5120 x 17408 134 and 224 with 24 rows, 185
+// to 195 and 226 with 32, 241 and 259 with 48, 322 and 268 with 64; of 2048 x 8192 78 and 114 with 64. The estimates lie within 5 % of these. Below 32 rows
+// they have not been followed, below 48 only where they see more than a few percent gained.
 // Where the segment-streaming form does not apply (more than 8192 slots, rows that bulk copies cannot take) the alternative is the
 // per-block form, and 128 rows are the line.
 constexpr u32 kGroupedLeastRows = 32, kGroupedSureRows = 48, kGroupedRowsElse = 128;
@@ -269,51 +267,52 @@ bool grouped_pays(const b200moe_shape& s, u32 rows, u32 max_union, u32 grouped_m
     if (rows < kGroupedLeastRows) return false;
     const Window w = window_of(s, rows, max_union);
     const u64 blocks = (down ? s.inter : s.hidden) / 256, sms = static_cast<u64>(device_sm_count());
-    const u64 items = w.items8 * (down ? s.hidden / 64 : s.inter / 32), start = blocks < 3 ? 2000 : 1200;  // ns
-    const u64 streaming = items <= sms ? start + 500 * blocks : waves(items, 2 * sms) * (start + 700 * blocks);
+    const u64 items = w.items8 * (down ? s.hidden / 64 : s.inter / 32), start = blocks < 3 ? 1700 : 1000;  // ns
+    const u64 streaming = items <= sms ? start + 500 * blocks : waves(items, 2 * sms) * (start + 560 * blocks);
     const u64 grouped = waves(w.tiles32 * grouped_row_tiles(down ? s.hidden : s.inter, down), sms) * (2000 + 1750 * blocks);
-    return grouped * (rows < kGroupedSureRows ? 13 : 10) < streaming * 10;
+    return grouped * (rows < kGroupedSureRows ? 107 : 100) < streaming * 100;
 }
-// The other forms of the Q4_K GEMVs: windows of one or two rows over rows of up to kRowStreamK weights take the row-streaming
-// form (a ring of whole rows, its work split fixed per CTA), everything else the segment-streaming form (any row length;
-// its items are dealt out dynamically), the per-block form being what is left. Measured on B200 at hidden 2048, 128
-// experts, top-8: one row 36.0 against 37.1 us per step, eight rows 76.5 against 70.4 us. B200MOE_DEBUG_DECODE_FORM forces
+// The other forms of the Q4_K GEMVs: the segment-streaming form (any row length; its items are dealt out dynamically) wherever it applies, else the
+// row-streaming form (a ring of whole rows, its work split fixed per CTA) and the per-block form. The row-streaming form had windows of one and two
+// rows over rows of up to 2048 weights, until the other began its launches with the weights of its first items. Whole calls, row and segment streaming, us: 128
+// experts of 2048 x 768, one row, top 1 to 16, 30.8 and 28.7, 32.9 and 30.8, 36.9 and 34.7 (top 8), 45.1 and 41.2; two rows, top 8, 43.0 and 39.2; 16
+// experts of 512 x 256 28.7 and 26.6; dense 2048 x 2048 23.7 and 17.5, 512 x 512 21.5 and 15.4. B200MOE_DEBUG_DECODE_FORM forces
 // one of the four where it applies, whatever grouped_min_rows says.
-constexpr u32 kRowStreamRows = 8, kRowStreamMaxRows = 2, kRowStreamK = 2048;
 enum class Q4Form { grouped, row_stream, wide, block };
 Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_fits, bool wide_fits, u32 rows, u32 max_union, u32 grouped_min_rows, bool down) {
-    const u32 K = down ? s.inter : s.hidden;
     const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
     if (forced == 1 && row_stream_fits) return Q4Form::row_stream;
     if (forced == 2 && wide_fits) return Q4Form::wide;
     if (forced == 3) return Q4Form::block;
     if (forced == 5 && grouped_fits) return Q4Form::grouped;
     if (grouped_fits && grouped_pays(s, rows, max_union, grouped_min_rows, wide_fits, down)) return Q4Form::grouped;
-    if (row_stream_fits && ((rows <= kRowStreamMaxRows && K <= kRowStreamK) || (rows <= kRowStreamRows && !wide_fits))) return Q4Form::row_stream;
     if (wide_fits) return Q4Form::wide;
     return row_stream_fits ? Q4Form::row_stream : Q4Form::block;
 }
-// The DS41 family (Q8_0 x A8): one weight row per warp below kRowStreamRows rows; from there on the tensor-core form of
-// gemv_q8_mma.cu (rows of 1024 to 7168 weights), else the dp4a token-block form of gemv_q8_wide.cu. Measured on B200: a
-// 7168 x 2048 dense block over 8 rows takes 49 + 18 us in the dp4a token-block form against 55 + 30 us with one row per
-// warp; one row over four experts of 2048 x 1024 is 2 us faster with one row per warp.
+// The DS41 family (Q8_0 x A8). Below kFewRows rows: a CTA one item with all its weights asked for at once (gemv_q8_shot.cu, rows of whole units of 256
+// weights), else one weight row per warp. From there on the tensor-core form of gemv_q8_mma.cu (rows of 1024 to 7168 weights), else the dp4a token-block form of
+// gemv_q8_wide.cu. The one-item form pays by the entry and keeps a multiprocessor for one item, so it gives way to the tensor-core form early where an expert has
+// more than four entries of long rows, and late where a window is sparse over short ones. Whole calls, one-item and tensor-core form, us: one expert of
+// 7168 x 2048 45 and 53 with 1 row, 55 and 56 with 4, 59 and 57 with 5, 64 and 59 with 7; of 2048 x 1024 31 and 37, 35 and 37 with 4, 37 and 39 with 6,
+// 39 and 38 with 7; 64 of 2048 x 1024, top-4, 80 and 81 with 7 rows, 86 and 90 with 8, 115 and 121 with 12, 125 and 123 with 14; 128 of these 90
+// and 98 with 8 rows, 119 and 123 with 12, 143 and 147 with 16; 16 of 4096 x 1536, top-2, 61 and 64 with 4, 82 and 80 with 6, 86 and 82 with 8.
 // The grouped form (grouped_q8.cu, tiles of 32 entries) takes over from the tensor-core form where its waves of tiles take less time than the
-// other's waves of items, both by their sizes: a tile 1.9 us + 0.605 a unit of 256 columns with up to 16 entries, 2.6 + 0.77 with more, an item of
+// other's waves of items, both by their sizes: a tile 2.3 us + 0.7 a unit of 256 columns with up to 16 entries, 2.6 + 0.77 with more, an item of
 // 32 gate and up rows 3 us + 0.33 a unit, one of 32 down rows half of that. Tensor-core and grouped form, gate/up and down: one expert of
 // 2048 x 17408 28.8 and 32.3 us with 8 rows, 51.4 and 32.9 with 16, 72 and 39 with 20; of 7168 x 2048 18.6 and 22.8, 16.5 and 12.4 with 16 rows; of
-// 1024 x 1024 8.4 and 10.3 (down) with 20; four of 2048 x 4096, top-2, 45 and 33, 22 and 16.6 with 20 rows; 64 of 2048 x 1024, top-4, 94.5 and
-// 94.8, 71 and 68 with 96 rows, 117 and 95.5, 84 and 68 with 128; 16 of 4096 x 1536, top-2, 69 and 74, 53 and 43 with 64. Over 336 such
-// launches (8 to 192 rows, 1 to 64 experts) the rule takes the better form, or one within 3.5 % of it. Where the tensor-core form does not apply (rows below
+// 1024 x 1024 8.4 and 10.3 (down) with 20; four of 2048 x 4096, top-2, 45 and 33, 22 and 16.6 with 20 rows; 64 of 2048 x 1024, top-4, whole
+// calls, 180 and 196 with 80 rows, 183 and 197 with 96, 207 and 198 with 112, 230 and 200 with 128; 16 of 4096 x 1536, top-2, 69 and 74, 53 and 43 with 64. Where the tensor-core form does not apply (rows below
 // 1024 or above 7168 weights) the grouped one takes over from the dp4a form at 4 entries an expert: down of 48 experts of 2048 x 512 36.8 and 39 us with 3,
 // 41 and 38.5 with 4, 49 and 39 with 5; of 32 of 1536 x 768 29 and 28 with 4.5; one expert of 2048 x 17408 45 and 43 us with 8 rows, 53.4 and 53.5 with
 // 17, of 4096 x 12288 35 and 33 with 8, 84 and 40 with 24.
+constexpr u32 kFewRows = 8;
 enum class Q8Form { row_per_warp, shot, wide, mma, grouped };
 bool q8_grouped_pays(const b200moe_shape& s, bool mma_fits, u32 rows, u32 max_union, bool down) {
-    if (rows < kRowStreamRows) return false;
+    if (rows < kFewRows) return false;
     if (!mma_fits) return u64(rows) * s.top_k >= u64(4) * s.experts;
     const Window w = window_of(s, rows, max_union);
     const u64 units = (down ? s.inter : s.hidden) / 256, sms = static_cast<u64>(device_sm_count());
-    const u64 tile = w.few ? 1900 + 605 * units : 2600 + 770 * units, item = (3000 + 330 * units) / (down ? 2 : 1);  // ns
+    const u64 tile = w.few ? 2300 + 700 * units : 2600 + 770 * units, item = (3000 + 330 * units) / (down ? 2 : 1);  // ns
     const u64 grouped = waves(w.tiles32 * (down ? s.hidden / 64 : s.inter / 32), sms) * tile, tensor = waves(w.items8 * ((down ? s.hidden : s.inter) / 32), sms) * item;
     return grouped < tensor;
 }
@@ -323,11 +322,14 @@ Q8Form pick_q8_form(const b200moe_shape& s, bool shot_fits, bool wide_fits, bool
     if (grouped_fits && (forced == 5 || (forced == 0 && q8_grouped_pays(s, mma_fits, rows, max_union, down)))) return Q8Form::grouped;
     if (forced == 4 && mma_fits) return Q8Form::mma;
     if (forced == 2 && wide_fits) return Q8Form::wide;
-    if (forced == 0 && rows >= kRowStreamRows) {
-        if (mma_fits) return Q8Form::mma;
-        if (wide_fits) return Q8Form::wide;
+    if (forced == 0) {
+        const u64 slots = u64(rows) * s.top_k;
+        const u32 longest = std::max(s.hidden, s.inter);
+        const bool shot = rows < kFewRows ? longest <= 2048 || slots <= u64(4) * s.experts || !mma_fits : longest <= 2048 && 4 * slots <= u64(3) * s.experts;
+        if (shot_fits && shot) return Q8Form::shot;
+        if (mma_fits && (rows >= kFewRows || shot_fits)) return Q8Form::mma;
+        if (wide_fits && rows >= kFewRows) return Q8Form::wide;
     }
-    if (forced == 0 && rows < kRowStreamRows && shot_fits) return Q8Form::shot;
     return Q8Form::row_per_warp;
 }
 int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0, const ChainHints& hints = {}) {

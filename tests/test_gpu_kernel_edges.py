@@ -776,9 +776,11 @@ def test_down_skipped_after_its_weights_were_asked_for(gpu, oracle, rows, H, I, 
             assert same(layer(good, ids, one).cpu(), want["raw"])
 
 
-@pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 256, 256), (1, 4, 8, 2048, 1024), (2, 2, 3, 1280, 2304), (3, 2, 4, 3328, 512), (7, 1, 1, 7168, 4352), (7, 3, 3, 4096, 1024), (5, 2, 40, 512, 768)])
+@pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 256, 256), (1, 4, 8, 2048, 1024), (2, 2, 3, 1280, 2304), (3, 2, 4, 3328, 512), (4, 1, 1, 7168, 4352),
+                                                    (4, 3, 3, 4096, 1024), (7, 1, 1, 2048, 1024), (5, 2, 40, 512, 768), (9, 1, 12, 2048, 512), (30, 3, 120, 1024, 1280)])
 def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I):
-    """Windows below 8 rows: rows of one run, of whole and broken runs, of more runs than places; 1 to 7 entries an expert, in one pass and in several."""
+    """Windows below 8 rows and sparse ones above: rows of one run, of whole and broken runs, of more runs than places; 1 to 9 entries an expert, in one pass
+    and in several."""
     import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(rows + H)

@@ -85,31 +85,36 @@ __global__ void __launch_bounds__(256) combine_kernel(b200moe_combine_view v, bo
 // The PARTS form over whole rows with up to kVecTopK slots and 16-byte rows: four outputs a thread, every slot's values requested before the
 // first is used and no block-wide step, so that a block's loads overlap. Bound by HBM (raw read once, y written once): the
 // one-output form above, with one load in flight a thread, took 1441 us for 8192 rows x 8 x 7168, this one 613 us. The additions
-// and their order are those of combine_kernel.
+// and their order are those of combine_kernel. A small window is a chain of memory latencies: the job's summary, the row's status and its order are asked for
+// together, then all that the order leads to
+// (one row over 64 Q8_0 experts of 2048 -> 1024, top 4, 24.7 -> 23.0 us a call, 512 rows 316 -> 312).
+// early: weights, ids, order and low_counts were complete before the launch in front was admitted (ChainHints), so that what the order leads to is known
+// before the wait.
 constexpr u32 kVecTopK = 8;
-__global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v, bool zero_skipped) {
-    chain_begin();
+__global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v, bool zero_skipped, bool early) {
+    if (!early) chain_begin();
     const u32 o = 4u * (blockIdx.x * 128u + threadIdx.x);
-    const bool aborted = v.summary && (*v.summary & B200MOE_JOB_WAIT_ABORTED);
-    if (o >= v.hidden || (aborted && !zero_skipped)) return;
     for (u32 row = blockIdx.y; row < v.rows; row += gridDim.y) {
-        if (aborted || (v.row_status && v.row_status[row])) {
-            if (zero_skipped) {
-                *reinterpret_cast<float4*>(v.y + u64(row) * v.hidden + o) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (v.y_bf16) *reinterpret_cast<uint2*>(v.y_bf16 + u64(row) * v.hidden + o) = make_uint2(0u, 0u);
-            }
-            continue;
-        }
-        u32 slot[kVecTopK];
+        u32 slot[kVecTopK], part[kVecTopK];
         float w[kVecTopK];
         float4 x[kVecTopK];
+        const u32 low = v.low_counts ? load_l2(v.low_counts + row) : 0u;
+#pragma unroll
+        for (u32 k = 0; k < kVecTopK; ++k)
+            if (k < v.top_k) slot[k] = min(load_l2(v.order + row * v.top_k + k), v.rows * v.top_k - 1u);  // the order of a row whose status is not zero may mean nothing
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
             if (k < v.top_k) {
-                slot[k] = load(v.order + row * v.top_k + k);
-                x[k] = load(reinterpret_cast<const float4*>(v.raw + u64(slot[k]) * v.hidden + o));
-                w[k] = load(v.weights + slot[k]);
+                w[k] = __uint_as_float(load_l2(reinterpret_cast<const u32*>(v.weights) + slot[k]));
+                part[k] = v.low_counts ? (k < low ? 0u : 1u) : min(load_l2(v.ids + slot[k]) / v.part_experts, v.parts - 1);
             }
+        if (early && row == blockIdx.y) chain_begin();
+        if (o >= v.hidden) return;
+        const bool aborted = v.summary && (load(v.summary) & B200MOE_JOB_WAIT_ABORTED);
+        const u32 status = v.row_status ? load(v.row_status + row) : 0u;
+#pragma unroll
+        for (u32 k = 0; k < kVecTopK; ++k)
+            if (k < v.top_k) x[k] = load(reinterpret_cast<const float4*>(v.raw + u64(slot[k]) * v.hidden + o));
         const float4 sh = v.shared ? load(reinterpret_cast<const float4*>(v.shared + u64(row) * v.hidden + o)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         float4 y = sh, sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         u32 p = 0;
@@ -121,15 +126,18 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
             if (run && k < v.top_k) {
-                const u32 part = v.low_counts ? (k < v.low_counts[row] ? 0u : 1u) : min(load(v.ids + slot[k]) / v.part_experts, v.parts - 1);
-                for (; p < part; ++p) flush();
-                run = part == p;
+                for (; p < part[k]; ++p) flush();
+                run = part[k] == p;
                 if (run) {
                     sum.x = __fadd_rn(sum.x, __fmul_rn(w[k], x[k].x)); sum.y = __fadd_rn(sum.y, __fmul_rn(w[k], x[k].y));
                     sum.z = __fadd_rn(sum.z, __fmul_rn(w[k], x[k].z)); sum.w = __fadd_rn(sum.w, __fmul_rn(w[k], x[k].w));
                 }
             }
         for (; p < v.parts; ++p) flush();
+        if (aborted || status) {
+            if (!zero_skipped) continue;
+            y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
         *reinterpret_cast<float4*>(v.y + u64(row) * v.hidden + o) = y;
         if (v.y_bf16)
             *reinterpret_cast<uint2*>(v.y_bf16 + u64(row) * v.hidden + o) =
@@ -212,13 +220,13 @@ int launch_merge_first_error(b200moe_first_error* record, const u32* summary, u3
     merge_first_error_kernel<<<1, 1, 0, stream>>>(record, summary, domain);
     return after_launch("merge_first_error");
 }
-int launch_combine(const b200moe_combine_view& v, cudaStream_t stream, bool zero_skipped) {
+int launch_combine(const b200moe_combine_view& v, cudaStream_t stream, bool zero_skipped, const ChainHints& hints) {
     if (v.rows == 0) return B200MOE_OK;
     // PARTS in one row: a whole call 37.2 us in the general form, 35.5 in the wide one; 32 rows x 8 x 2048 of 8 parts 5.0 and 4.2 us.
     const bool whole = v.y && !v.y_blocks && v.top_k <= kVecTopK;
     if (v.form == B200MOE_COMBINE_PARTS && whole && v.only_part < 0 && v.hidden % 4 == 0 && aligned(v.raw, 16) && aligned(v.y, 16) && aligned(v.shared, 16) && aligned(v.y_bf16, 8)) {
         if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_vec_kernel))) return rc;
-        chain_launch(combine_vec_kernel, dim3((v.hidden + 511) / 512, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v, zero_skipped);
+        chain_launch(combine_vec_kernel, dim3((v.hidden + 511) / 512, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v, zero_skipped, hints.routes_done);
         return after_launch("combine");
     }
     if (v.form == B200MOE_COMBINE_FMA_SLOTS && whole && v.hidden % 2 == 0 && aligned(v.raw, 8) && aligned(v.y, 8) && aligned(v.shared, 8) && aligned(v.y_bf16, 4)) {

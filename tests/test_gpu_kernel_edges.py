@@ -847,3 +847,34 @@ def test_router_logits_tiles(gpu, rows, hidden, experts):
     at = np.unique(np.concatenate([np.arange(min(rows, 33)), np.arange(max(0, rows - 33), rows)]))
     whole = [(0, 0), (0, -hidden % 32)]  # zero products leave a sum that starts at +0 as it is
     assert same(z.cpu().numpy()[at], declared_logits(np.pad(x[at], whole), np.pad(w, whole)) + b)
+
+
+@pytest.mark.parametrize("rows,types,H,I", [(1, 8, 512, 256), (5, 8, 2304, 512), (40, 8, 1024, 1024), (1, 12, 512, 256), (8, 12, 1024, 768), (33, 12, 512, 512), (300, 12, 512, 256), (300, 8, 512, 256)])
+def test_chain_of_launches_under_capture(gpu, rows, types, H, I):
+    """A captured call replayed on other inputs gives the bits of a direct call, and replays back to back do not run into each other."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows)
+    E, top_k = 12, 3
+    gate, up, down = (dv(t, gpu) for t in synth.expert_tensors(rng, E, H, I, types, types))
+    router = dv(synth.router_weight(rng, E, H), gpu)
+    form = {"combine_form": b200moe.COMBINE_PARTS, "parts": 2} if types == 8 else {"combine_form": b200moe.COMBINE_FMA_SLOTS}
+    ffn = ops.MoeFfn(ops.make_shape(H, I, E, top_k, types, types), ops.softmax_policy(E, top_k), gate, up, down, router, capacity=rows, **form)
+    inputs = [dv(synth.activations(rng, rows, H), gpu) for _ in range(3)]
+    want = [ffn(x).clone() for x in inputs]
+    x, outs = inputs[0].clone(), []
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        ffn(x)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = ffn(x)
+    for v in inputs + inputs[::-1]:
+        x.copy_(v)
+        for _ in range(3):
+            graph.replay()
+        outs.append(y.clone())
+    for got, ref in zip(outs, want + want[::-1]):
+        assert same(got.cpu(), ref.cpu())

@@ -1,4 +1,4 @@
-// Q8_0 x A8 experts over windows of 8 rows and more with few entries an expert (grouped_q8.cu takes the others), integer dots on the
+// Q8_0 x A8 experts over windows of 8 rows and more with few entries an expert (grouped_q8.cu takes those with many, gemv_q8_shot.cu sparse ones), integer dots on the
 // tensor cores: the lane-class contract of src/ds41_formats.cpp:188-197 (product_q8_0) with one mma.sync.m16n8k32 (s8 x s8 -> s32) per
 // (16 weight rows, 8 entries, block) instead of 16 x 8 dp4a chains of eight.
 //

@@ -1,11 +1,12 @@
 // Routed experts and dense blocks, Q8_0 in the 32-lane-class contract (src/ds41_formats.cpp:45-50), for windows of fewer rows than the tensor-core forms
-// take: a CTA is ONE item and asks for all of its weights at once.
+// take, and for sparse ones of more: a CTA is ONE item and asks for all of its weights at once.
 //
 // Item = (expert, 64 weight rows): 32 gate and 32 up rows of one output group, or 64 down rows. A stage = a run of 32 blocks (1088 bytes) of the 64 rows, two
 // tiled TMA copies of 32 rows each; as many stages as the rows have runs, up to kStages (the places are used again beyond that). Consumer warps (16) take
 // four rows each, a lane one of the 32 classes, as in gemv_q8.cu, whose bits these are; the entries' codes are read once for a warp's four rows.
 // What bounds it: latencies. One row over 4 of 64 experts of 2048 -> 1024, top 4 (128 + 128 items): the form with a row a warp had one run a warp on its
-// way (35 KB a multiprocessor) and each warp's four runs one behind the other: gate/up 11.5 us behind its routes, down 9.7 behind gate/up.
+// way (35 KB a multiprocessor) and each warp's four runs one behind the other: gate/up 11.5 us behind its routes, down 9.7 behind gate/up, where these
+// take 8 and 5 (a whole call 33.1 -> 24.9). 8 rows over 256 experts of 2048 -> 768, top 8: 131 us a call, 199 in the tensor-core and token-block forms. Where it pays: csrc/api.cu.
 // An early launch of down (ChainHints) fits on the multiprocessors beside gate/up's CTAs and has its weights before it waits.
 #include <algorithm>
 

@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(256) combine_kernel(b200moe_combine_view v, bo
         __syncthreads();  // the previous row's readers are done with the shared arrays
         if (aborted || (v.row_status && v.row_status[row])) {  // fail closed (qwen_moe.cu:291); uniform over the block
             if (zero_skipped && !v.y_blocks && o < v.hidden) {
-                v.y[u64(row) * v.hidden + o] = 0.0f;
+                for (u32 i = 0; i < max(v.only_part_count, 1u); ++i) v.y[i * v.part_stride + u64(row) * v.hidden + o] = 0.0f;  // every destination of the row
                 if (v.y_bf16) v.y_bf16[u64(row) * v.hidden + o] = 0;
             }
             continue;

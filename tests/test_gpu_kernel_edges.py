@@ -878,3 +878,31 @@ def test_chain_of_launches_under_capture(gpu, rows, types, H, I):
         outs.append(y.clone())
     for got, ref in zip(outs, want + want[::-1]):
         assert same(got.cpu(), ref.cpu())
+
+
+@pytest.mark.parametrize("hidden", [256, 320])
+def test_fresh_layer_clears_every_destination(gpu, hidden):
+    """Three partial sums a row, each in a plane of its own: a good call fills all planes with what the single sums give, a row that fails
+    is zero in all of them."""
+    import ctypes as C
+    import b200moe
+    from b200moe import A8Rows, ExpertWeights, LayerView, check, lib, ops, ptr, stream_ptr, synth
+    rng = np.random.default_rng(hidden)
+    E, H, I, K, rows, first, n = 8, 512, hidden, 3, 4, 1, 3
+    gate, up, down = (dv(t, gpu) for t in synth.expert_tensors(rng, E, H, I, 12, 8))
+    ids, w = dv(window(rng, E, K, rows).view(np.int32), gpu), torch.rand((rows, K), device=gpu)
+    layer = ops.MoeLayer(ops.make_shape(H, I, E, K, 12, 8), gate, up, down, capacity=rows, combine_form=b200moe.COMBINE_PARTS, parts=4)
+    codes, deltas, sums = ops.enqueue_quantize_a8(torch.randn((rows, H), device=gpu))
+    bad = deltas.clone()
+    bad[2, 0] = float("inf")
+    for d in (deltas, bad):
+        y = torch.full((n + 1, rows, H), 9.0, device=gpu)
+        v = LayerView(layer.shape, ExpertWeights(ptr(gate), ptr(up), ptr(down)), rows, A8Rows(ptr(codes), ptr(d), ptr(sums), rows, H, H), ptr(ids), ptr(w), None, 0, 0, 0,
+                      b200moe.COMBINE_PARTS, 4, E // 4, first, None, ptr(y), None, None, ptr(layer.ws), layer.ws_bytes, rows, 0, None, None, 0, None, n, rows * H)
+        check(lib().b200moe_layer_fresh(C.byref(v), stream_ptr()))
+        assert bool((y[n] == 9.0).all())
+        if d is deltas:
+            want = torch.stack([layer((codes, d, sums), ids, w, only_part=first + i) for i in range(n)])
+            assert torch.equal(y[:n], want) and bool(want.any())
+        else:
+            assert not y[:n, 2].any()

@@ -446,8 +446,10 @@ typedef struct b200moe_layer_view {
 } b200moe_layer_view;
 uint64_t b200moe_layer_workspace_bytes(const b200moe_shape* shape, uint32_t capacity);
 int b200moe_layer(const b200moe_layer_view* view, void* stream);
+/* A projection that is not finite (B200MOE_ROW_PROJECTION_NONFINITE) or a wait that ran out skips down for the whole job: the summary word is not zero
+ * then and b200moe_layer, b200moe_ffn write no row of y and y_bf16, whatever its own status. */
 /* The same over outputs that were not initialised: rows of y and y_bf16 that b200moe_layer leaves as they were - those of a
- * failed row, all of an aborted job - are set to zero, in each of only_part_count destinations (without y_blocks). */
+ * failed row, all of a job whose summary is not zero - are set to zero, in each of only_part_count destinations (without y_blocks). */
 int b200moe_layer_fresh(const b200moe_layer_view* view, void* stream);
 
 /* Router + A8 + layer from FP32 (or bfloat16) activations: one token block through the whole FFN. */

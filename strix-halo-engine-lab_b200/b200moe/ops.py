@@ -212,7 +212,8 @@ class MoeFfn:
                        self.capacity, self.grouped_min_rows, ev, ptr(summary))
 
     def __call__(self, x, y=None, shared=None, want_routes=False, row_status=None, summary=None):
-        """x: [rows][hidden] float32 or bfloat16 (widened exactly before the router and the A8 quantiser)."""
+        """x: [rows][hidden] float32 or bfloat16 (widened exactly before the router and the A8 quantiser). A job whose summary is not zero
+        leaves y as it was (a y that was not given holds whatever its memory held)."""
         rows = x.shape[0]
         if y is None:
             y = x.new_empty((rows, self.shape.hidden), dtype=torch.float32)

@@ -604,7 +604,9 @@ static int layer_impl(const b200moe_layer_view* v, void* stream, bool routes_rea
     cv.row_status = is_kquant(s.gate_type) ? row_status : nullptr;
     cv.summary = summary;
     tap(6);
-    const int rc = launch_combine(cv, st, fresh, ChainHints{max_union > 0, 0, slots});  // down was admitted after the routes; without an expert there was none
+    // A projection that is not finite skips down for the whole job (any bit of the summary does), so raw holds an earlier call's values for the other rows
+    // too: none is combined. Down was admitted after the routes; without an expert there was none.
+    const int rc = launch_combine(cv, st, 0xffffffffu, fresh, ChainHints{max_union > 0, 0, slots});
     tap(7);
     return rc;
 }

@@ -16,17 +16,18 @@ namespace {
 
 constexpr u32 kMaxTopK = 32;
 
+// skip_bits: with one of them in the job summary raw holds nothing of this job for some slots or for all, and no row is combined.
 // grid (ceil(hidden / 256), min(rows, 65535)); 256 threads; a block walks rows blockIdx.y, blockIdx.y + gridDim.y, ...
-__global__ void __launch_bounds__(256) combine_kernel(b200moe_combine_view v, bool zero_skipped) {
+__global__ void __launch_bounds__(256) combine_kernel(b200moe_combine_view v, u32 skip_bits, bool zero_skipped) {
     chain_begin();
     const u32 o = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool aborted = v.summary && (*v.summary & B200MOE_JOB_WAIT_ABORTED);  // an aborted stage left raw partly unwritten
-    if (aborted && !zero_skipped) return;
+    const bool skipped = v.summary && (*v.summary & skip_bits);
+    if (skipped && !zero_skipped) return;
     __shared__ float s_w[kMaxTopK];
     __shared__ u32 s_slot[kMaxTopK], s_part[kMaxTopK];
     for (u32 row = blockIdx.y; row < v.rows; row += gridDim.y) {
         __syncthreads();  // the previous row's readers are done with the shared arrays
-        if (aborted || (v.row_status && v.row_status[row])) {  // fail closed (qwen_moe.cu:291); uniform over the block
+        if (skipped || (v.row_status && v.row_status[row])) {  // fail closed (qwen_moe.cu:291); uniform over the block
             if (zero_skipped && !v.y_blocks && o < v.hidden) {
                 for (u32 i = 0; i < max(v.only_part_count, 1u); ++i) v.y[i * v.part_stride + u64(row) * v.hidden + o] = 0.0f;  // every destination of the row
                 if (v.y_bf16) v.y_bf16[u64(row) * v.hidden + o] = 0;
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(256) combine_kernel(b200moe_combine_view v, bo
 // early: weights, ids, order and low_counts were complete before the launch in front was admitted (ChainHints), so that what the order leads to is known
 // before the wait.
 constexpr u32 kVecTopK = 8;
-__global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v, bool zero_skipped, bool early) {
+__global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v, u32 skip_bits, bool zero_skipped, bool early) {
     if (!early) chain_begin();
     const u32 o = 4u * (blockIdx.x * 128u + threadIdx.x);
     for (u32 row = blockIdx.y; row < v.rows; row += gridDim.y) {
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
             }
         if (early && row == blockIdx.y) chain_begin();
         if (o >= v.hidden) return;
-        const bool aborted = v.summary && (load(v.summary) & B200MOE_JOB_WAIT_ABORTED);
+        const bool skipped = v.summary && (load(v.summary) & skip_bits);
         const u32 status = v.row_status ? load(v.row_status + row) : 0u;
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
                 }
             }
         for (; p < v.parts; ++p) flush();
-        if (aborted || status) {
+        if (skipped || status) {
             if (!zero_skipped) continue;
             y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
 // row's status, the job's summary, weights, values - is asked for before any of them is looked at: a small window is a chain of
 // memory latencies (three in the general form, with two block barriers between them), a large one wants bytes in flight.
 // 4096 rows x 8 x 2048: 79 us in the general form, 60 here (5.0 TB/s); 8 rows 3.1 and 2.2; 37 rows 4.0 and 2.8.
-__global__ void __launch_bounds__(128) combine_slots_kernel(b200moe_combine_view v, bool zero_skipped) {
+__global__ void __launch_bounds__(128) combine_slots_kernel(b200moe_combine_view v, u32 skip_bits, bool zero_skipped) {
     chain_begin();
     const u32 o = 2u * (blockIdx.x * 128u + threadIdx.x);
     if (o >= v.hidden) return;
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(128) combine_slots_kernel(b200moe_combine_view
         for (u32 k = 0; k < kVecTopK; ++k)
             if (k < v.top_k) y = make_float2(__fmaf_rn(w[k], x[k].x, y.x), __fmaf_rn(w[k], x[k].y, y.y));
         if (v.shared) y = make_float2(__fadd_rn(y.x, sh.x), __fadd_rn(y.y, sh.y));
-        if ((job & B200MOE_JOB_WAIT_ABORTED) || status) {  // an aborted stage left raw partly unwritten; fail closed (qwen_moe.cu:291)
+        if ((job & skip_bits) || status) {  // fail closed (qwen_moe.cu:291)
             if (!zero_skipped) continue;
             y = make_float2(0.0f, 0.0f);
         }
@@ -220,22 +221,22 @@ int launch_merge_first_error(b200moe_first_error* record, const u32* summary, u3
     merge_first_error_kernel<<<1, 1, 0, stream>>>(record, summary, domain);
     return after_launch("merge_first_error");
 }
-int launch_combine(const b200moe_combine_view& v, cudaStream_t stream, bool zero_skipped, const ChainHints& hints) {
+int launch_combine(const b200moe_combine_view& v, cudaStream_t stream, u32 skip_bits, bool zero_skipped, const ChainHints& hints) {
     if (v.rows == 0) return B200MOE_OK;
     // PARTS in one row: a whole call 37.2 us in the general form, 35.5 in the wide one; 32 rows x 8 x 2048 of 8 parts 5.0 and 4.2 us.
     const bool whole = v.y && !v.y_blocks && v.top_k <= kVecTopK;
     if (v.form == B200MOE_COMBINE_PARTS && whole && v.only_part < 0 && v.hidden % 4 == 0 && aligned(v.raw, 16) && aligned(v.y, 16) && aligned(v.shared, 16) && aligned(v.y_bf16, 8)) {
         if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_vec_kernel))) return rc;
-        chain_launch(combine_vec_kernel, dim3((v.hidden + 511) / 512, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v, zero_skipped, hints.routes_done);
+        chain_launch(combine_vec_kernel, dim3((v.hidden + 511) / 512, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v, skip_bits, zero_skipped, hints.routes_done);
         return after_launch("combine");
     }
     if (v.form == B200MOE_COMBINE_FMA_SLOTS && whole && v.hidden % 2 == 0 && aligned(v.raw, 8) && aligned(v.y, 8) && aligned(v.shared, 8) && aligned(v.y_bf16, 4)) {
         if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_slots_kernel))) return rc;
-        chain_launch(combine_slots_kernel, dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v, zero_skipped);
+        chain_launch(combine_slots_kernel, dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v, skip_bits, zero_skipped);
         return after_launch("combine");
     }
     if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_kernel))) return rc;
-    chain_launch(combine_kernel, dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 256, 0, stream, v, zero_skipped);
+    chain_launch(combine_kernel, dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 256, 0, stream, v, skip_bits, zero_skipped);
     return after_launch("combine");
 }
 int launch_canonical_sum(const float* a, const float* b, const float* c, u64 count, float* y, cudaStream_t stream) {

@@ -94,8 +94,8 @@ int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view
 
 // combine.cu
 int launch_merge_first_error(b200moe_first_error* record, const u32* summary, u32 domain, cudaStream_t stream);
-// zero_skipped: rows of y and y_bf16 that a failed row or an aborted job leaves out become zeros
-int launch_combine(const b200moe_combine_view& v, cudaStream_t stream, bool zero_skipped = false, const ChainHints& hints = {});
+// skip_bits: bits of the job summary with which no row is combined. zero_skipped: rows of y and y_bf16 that are left out become zeros
+int launch_combine(const b200moe_combine_view& v, cudaStream_t stream, u32 skip_bits = B200MOE_JOB_WAIT_ABORTED, bool zero_skipped = false, const ChainHints& hints = {});
 int launch_canonical_sum(const float* a, const float* b, const float* c, u64 count, float* y, cudaStream_t stream);
 int launch_fill_u32(u32* p, u32 value, u64 count, cudaStream_t stream);
 // order[row][k] (slots in ascending expert id) for the PARTS combine when no routes were built

@@ -906,3 +906,37 @@ def test_fresh_layer_clears_every_destination(gpu, hidden):
             assert torch.equal(y[:n], want) and bool(want.any())
         else:
             assert not y[:n, 2].any()
+
+
+@pytest.mark.parametrize("rows,top_k,form,parts", [(5, 4, "PARTS", 2), (5, 9, "PARTS", 3), (5, 4, "FMA_SLOTS", 2), (5, 9, "FMA_SLOTS", 2), (40, 2, "PARTS", 2), (40, 2, "FMA_SLOTS", 2)])
+def test_a_job_with_a_failed_projection_combines_no_row(gpu, rows, top_k, form, parts):
+    """Down is skipped for the whole job when one row's projection is not finite: the other rows are zero in the fresh form and as they were in the others,
+    not a combine of what the workspace held. The next good call is whole again."""
+    import ctypes as C
+    import b200moe
+    from b200moe import A8Rows, ExpertWeights, LayerView, check, lib, ops, ptr, stream_ptr, synth
+    rng = np.random.default_rng(rows + top_k)
+    E, H, I = 12, 512, 256
+    gate, up, down = (dv(t, gpu) for t in synth.expert_tensors(rng, E, H, I, 12, 12))
+    sh, how = ops.make_shape(H, I, E, top_k, 12, 12), {"combine_form": getattr(b200moe, "COMBINE_" + form), "parts": parts}
+    layer = ops.MoeLayer(sh, gate, up, down, capacity=rows, **how)
+    ids, w, x = dv(window(rng, E, top_k, rows).view(np.int32), gpu), torch.rand((rows, top_k), device=gpu), torch.randn((rows, H), device=gpu)
+    codes, deltas, sums = ops.enqueue_quantize_a8(x)
+    bad = deltas.clone()
+    bad[2, 0] = float("inf")
+    status, summary = torch.zeros(rows, dtype=torch.int32, device=gpu), torch.zeros(1, dtype=torch.int32, device=gpu)
+    want = layer((codes, deltas, sums), ids, w)
+    for _ in range(2):
+        y, yb = layer((codes, bad, sums), ids, w, bf16=True, row_status=status)
+        assert [r for r in range(rows) if status[r]] == [2] and not y.any() and not yb.any()
+        y = torch.full((rows, H), 9.0, device=gpu)
+        v = LayerView(sh, ExpertWeights(ptr(gate), ptr(up), ptr(down)), rows, A8Rows(ptr(codes), ptr(bad), ptr(sums), rows, H, H), ptr(ids), ptr(w), None, 0, 0, 0,
+                      layer.combine_form, parts, layer.part_experts, -1, None, ptr(y), None, None, ptr(layer.ws), layer.ws_bytes, rows, 0, None, None, 0, ptr(summary))
+        check(lib().b200moe_layer(C.byref(v), stream_ptr()))
+        assert bool((y == 9.0).all()) and int(summary[0]) == b200moe.ROW_PROJECTION_NONFINITE
+        assert torch.equal(layer((codes, deltas, sums), ids, w), want)
+    ffn = ops.MoeFfn(sh, ops.softmax_policy(E, top_k), gate, up, down, dv(synth.router_weight(rng, E, H), gpu), capacity=rows, **how)
+    ffn(x)
+    x[2] = 3e38
+    ffn(x, y=y, summary=summary)
+    assert bool((y == 9.0).all()) and int(summary[0]) == b200moe.ROW_PROJECTION_NONFINITE

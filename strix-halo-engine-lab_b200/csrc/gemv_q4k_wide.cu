@@ -256,7 +256,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     if (tid < kGroups * plan.stages) { mbar_init(&full[tid], 1); mbar_init(&empty[tid], kGroupWarps); }
     if (tid < 2 * kGroups) mbar_init(&met[tid], kGroupWarps);
-    if (tid < 4) ctl[tid] = 0;
+    if (tid < 2) ctl[tid] = 0;  // the list's builder writes the others, and for a dense block there is no barrier between here and there
     if (tid < kGroups * plan.stages + 2 * kGroups) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 
     if (!early) chain_begin();

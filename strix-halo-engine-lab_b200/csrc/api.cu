@@ -355,7 +355,7 @@ int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grou
     if (v.shape.down_type == B200MOE_TYPE_Q4_K) {
         switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.act.sums != nullptr), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, v.max_union, grouped_min_rows, true)) {
             case Q4Form::grouped: return launch_down_q4k_grouped(v, st);
-            case Q4Form::row_stream: return launch_down_q4k_stream(v, rows, hints, st);
+            case Q4Form::row_stream: return launch_down_q4k_stream(v, rows, st);
             case Q4Form::wide: return launch_down_q4k_wide(v, rows, hints, st);
             default: return launch_down_q4k(v, st);
         }

@@ -92,7 +92,6 @@ struct StreamPlan {
     u32 max_entries;   // bound of the entries of one expert (the window's rows)
     u32 x_rows;        // rows of the A8 input copied to shared memory (gate/up)
     u32 stage_entries; // entries of the CTA's run whose activations are copied to shared memory (down)
-    u32 early;         // down: the routes are complete before the launch in front was admitted (ChainHints)
 };
 
 // Ring of stages. An mbarrier's phase test only tells odd from even uses of a slot, and here the successive uses of a
@@ -146,20 +145,14 @@ __device__ __forceinline__ void stage_release(const Ring& ring, u32 slot, u32 q)
 // whatever its size, so one thread - or one warp - issuing 1 KB row copies tops out near half of HBM bandwidth;
 // four warps of eight lanes reach it (measured on B200: 1 warp 3.0 TB/s, 2 warps 5.8, 4 warps 6.5).
 // `row_of(item, octet)` gives the first of the octet's 8 consecutive weight rows.
-// `enter`: called once, by the whole warp, after the ring has been filled for the first time; false: nothing will be consumed.
-template <class RowOf, class Enter>
-__device__ __forceinline__ void produce(const Ring& ring, const StreamPlan& plan, u32 first_item, u32 n_local, u32 pw, RowOf row_of, Enter enter) {
+template <class RowOf>
+__device__ __forceinline__ void produce(const Ring& ring, const StreamPlan& plan, u32 first_item, u32 n_local, u32 pw, RowOf row_of) {
     const u32 lane = threadIdx.x & 31u;
     const bool one_copy = plan.row_stride == plan.row_bytes;  // rows already conflict free: one copy per octet
     const u32 local_octets = n_local * kOctetsPerItem;
     u32 slot = pw % plan.stages, phase = (pw / plan.stages) & 1u, q = pw;
-    bool ok = true, entered = false;
+    bool ok = true;
     for (; q < local_octets; q += kProducers) {
-        if (q >= plan.stages && !entered) {
-            entered = true;
-            ok = enter();
-            if (!ok) break;
-        }
         if (q >= plan.stages) ok = flag_wait(&ring.rel[slot], q - plan.stages + 1u, ring.abort_flag);  // the slot's previous use is done
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -180,7 +173,6 @@ __device__ __forceinline__ void produce(const Ring& ring, const StreamPlan& plan
         slot += kProducers;
         while (slot >= plan.stages) { slot -= plan.stages; phase ^= 1u; }
     }
-    if (!entered) ok = enter();
     if (!ok && lane == 0) {  // wait (bounded) for this producer's copies still in flight before the CTA retires
         const u32 back = (plan.stages + kProducers - 1) / kProducers * kProducers;  // keeps n on this producer's octets
         for (u32 n = q > back ? q - back : pw; n < q; n += kProducers)
@@ -200,14 +192,12 @@ __device__ __forceinline__ u32 warp_inclusive_scan(u32 v, u32 lane) {
     for (int d = 1; d < 32; d <<= 1) { const u32 o = __shfl_up_sync(0xffffffffu, v, d); if (lane >= (u32)d) v += o; }
     return v;
 }
-template <bool L2>  // past the L1 cache: before an early launch's wait
 __device__ __forceinline__ void item_range(const StreamPlan& plan, const b200moe_routes& routes, u32 n_union, u32* first_item, u32* n_local) {
     const u32 lane = threadIdx.x & 31u, G = gridDim.x, b = blockIdx.x, nc = plan.n_chunks;
-    auto begin_of = [&](u32 i) { return L2 ? load_l2(routes.begins + i) : load(routes.begins + i); };
     u32 total = 0;
     for (u32 j0 = 0; j0 < n_union; j0 += 32) {
         const u32 j = j0 + lane;
-        const u32 c = j < n_union ? item_cost(begin_of(j + 1) - begin_of(j)) * nc : 0u;
+        const u32 c = j < n_union ? item_cost(load(routes.begins + j + 1) - load(routes.begins + j)) * nc : 0u;
         total += __shfl_sync(0xffffffffu, warp_inclusive_scan(c, lane), 31);
     }
     const u32 n_items = n_union * nc;
@@ -215,7 +205,7 @@ __device__ __forceinline__ void item_range(const StreamPlan& plan, const b200moe
     u32 lo = n_items, hi = n_items, cum = 0;  // a boundary at `total` means "past the last item"
     for (u32 j0 = 0; j0 < n_union; j0 += 32) {
         const u32 j = j0 + lane;
-        const u32 ci = j < n_union ? item_cost(begin_of(j + 1) - begin_of(j)) : 0u;
+        const u32 ci = j < n_union ? item_cost(load(routes.begins + j + 1) - load(routes.begins + j)) : 0u;
         const u32 c = ci * nc, incl = warp_inclusive_scan(c, lane), excl = cum + incl - c;
         const bool h0 = c && B0 >= excl && B0 < excl + c, h1 = c && B1 >= excl && B1 < excl + c;
         const u32 c0 = h0 ? j * nc + (B0 - excl + ci - 1) / ci : 0u, c1 = h1 ? j * nc + (B1 - excl + ci - 1) / ci : 0u;
@@ -425,19 +415,19 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) gate_up_q4k_
     u32 first_item, n_local;
 
     if (warp >= plan.warps) {  // ------------------------------------------------------------- producer warps
-        item_range<false>(plan, v.routes, n_union, &first_item, &n_local);
+        item_range(plan, v.routes, n_union, &first_item, &n_local);
         produce(ring, plan, first_item, n_local, warp - plan.warps, [&](u32 item, u32 o) {
             u32 j, gx;
             split_item(plan, item, &j, &gx);
             const u64 row = u64(v.routes.experts[j]) * I + 32u * gx + 8u * (o & 3u);
             return (o < 4 ? v.weights.gate : v.weights.up) + row * row_bytes;
-        }, [] { return true; });
+        });
         return;
     }
 
     // ------------------------------------------------------------------------------------------ consumer warps
     copy_x_rows_async(v.x, plan.x_rows, H, x_copy, plan.warps * 32);  // in flight while the item run is worked out
-    item_range<false>(plan, v.routes, n_union, &first_item, &n_local);
+    item_range(plan, v.routes, n_union, &first_item, &n_local);
     const u32 x_row_bytes = H + H / 4;
     const u32 rsub = lane >> 2, p = lane & 3u;
     const u32 swz = p >> 1;  // chunk swap of the staged codes
@@ -538,35 +528,29 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) gate_up_q4k_
 // Item = (expert, 64 hidden outputs) = 8 octets. Activations (the A8 of h) are read from global memory: every lane of a
 // row group reads the same addresses, so the loads are broadcasts served by L1 / L2.
 __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) down_q4k_stream_kernel(b200moe_down_view v, StreamPlan plan) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
     const u32 H = v.shape.hidden, I = v.shape.inter, nblocks = I / 256;
     u64* bars = reinterpret_cast<u64*>(smem + u64(plan.stages) * plan.stage_bytes);
     u32* s_flag = reinterpret_cast<u32*>(bars + 2 * plan.stages);
     const Ring ring{smem, bars, reinterpret_cast<volatile u32*>(bars + plan.stages), reinterpret_cast<volatile u32*>(bars + plan.stages) + plan.stages, s_flag};
     ring_init(ring, plan.stages);
-    // An early launch splits its work and asks for weights before it waits for the launch in front. Every warp waits, on every path.
-    const bool early = plan.early;
-    auto enter = [&]() {  // false: a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
-        chain_begin();
-        return !(v.summary && *v.summary);
-    };
-    if (!early && !enter()) return;
+    if (v.summary && *v.summary) return;  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
 
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const u32 n_union = load_l2(v.routes.counts);
+    const u32 n_union = v.routes.counts[0];
     const u64 row_bytes = plan.row_bytes;
     u32 first_item, n_local;
-    item_range<true>(plan, v.routes, n_union, &first_item, &n_local);
+    item_range(plan, v.routes, n_union, &first_item, &n_local);
     if (warp >= plan.warps) {
         produce(ring, plan, first_item, n_local, warp - plan.warps, [&](u32 item, u32 o) {
             u32 j, cx;
             split_item(plan, item, &j, &cx);
-            const u64 row = u64(load_l2(v.routes.experts + j)) * H + 64u * cx + 8u * o;
+            const u64 row = u64(v.routes.experts[j]) * H + 64u * cx + 8u * o;
             return v.weights.down + row * row_bytes;
-        }, [&]() { return !early || enter(); });
+        });
         return;
     }
-    if (early && !enter()) return;
 
     const u32 act_stride = v.act.stride ? v.act.stride : v.act.width;
     const u32 rsub = lane >> 2, p = lane & 3u;
@@ -725,7 +709,7 @@ int launch_gate_up_q4k_stream(const b200moe_gate_up_view& v, u32 rows, cudaStrea
     return after_launch("gate_up_q4k_stream");
 }
 
-int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream) {
+int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, cudaStream_t stream) {
     (void)rows;
     if (v.max_union == 0) return B200MOE_OK;
     StreamPlan p{};
@@ -733,7 +717,6 @@ int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, const ChainHint
     p.n_chunks = v.shape.hidden / 64;
     p.chunk_magic = static_cast<u32>((u64(1) << 32) / p.n_chunks) + 1;
     p.stage_entries = down_stage_entries(v);
-    p.early = hints.routes_done;
     const u32 smem = plan_smem(p, down_fixed_bytes(v), 0);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(down_q4k_stream_kernel), smem)) return rc;
     chain_launch(down_q4k_stream_kernel, device_sm_count(), (p.warps + kProducers) * 32, smem, stream, v, p);

@@ -57,7 +57,7 @@ int launch_down_q8_chain4(const b200moe_down_view& v, const ChainHints& hints, c
 bool stream_gate_up_fits(const b200moe_gate_up_view& v, u32 rows);
 bool stream_down_fits(const b200moe_down_view& v, u32 rows);
 int launch_gate_up_q4k_stream(const b200moe_gate_up_view& v, u32 rows, cudaStream_t stream);
-int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
+int launch_down_q4k_stream(const b200moe_down_view& v, u32 rows, cudaStream_t stream);
 
 // gemv_q4k_wide.cu: the same contracts with SEGMENTS of the rows (and of the entries' A8 rows) streamed by TMA: any row
 // length, windows of any size whose routes fit shared memory

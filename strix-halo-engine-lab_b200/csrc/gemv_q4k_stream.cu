@@ -535,7 +535,7 @@ __global__ void __launch_bounds__((kMaxWarps + kProducers) * 32, 1) down_q4k_str
     u32* s_flag = reinterpret_cast<u32*>(bars + 2 * plan.stages);
     const Ring ring{smem, bars, reinterpret_cast<volatile u32*>(bars + plan.stages), reinterpret_cast<volatile u32*>(bars + plan.stages) + plan.stages, s_flag};
     ring_init(ring, plan.stages);
-    if (v.summary && *v.summary) return;  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
+    if (block_skips(v.summary)) return;  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
 
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const u32 n_union = v.routes.counts[0];

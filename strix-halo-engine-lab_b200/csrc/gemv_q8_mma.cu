@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
 q8_mma_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, MmaArgs a, MmaPlan plan) {
     chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
-    if (DOWN && a.summary && *a.summary) return;
+    if (DOWN && block_skips(a.summary)) return;
     u32 n_union = a.routes.counts[0];
     if (n_union == 0) return;
     if (n_union > plan.max_union) n_union = plan.max_union;

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q4k_kernel(const __grid_
     u32* s_tile = reinterpret_cast<u32*>(smem + kOffTile);             // [kTilePlaces][kTileWords]
     u32* cum = reinterpret_cast<u32*>(smem + kOffCum);                 // [2][kTileCounts]
 
-    if (kDown && a.summary && *a.summary) return;  // a failed or aborted projection skips the stage (routed_expert.hpp:17-19)
+    if (kDown && block_skips(a.summary)) return;  // a failed or aborted projection skips the stage (routed_expert.hpp:17-19)
 
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const u32 n_union = min(a.routes.counts[0], kMaxUnion);

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kGThreads, 1) grouped_q8_kernel(const __grid_c
     u32* s_tile = reinterpret_cast<u32*>(smem + kOffTile);             // [kTilePlaces][kTileWords]
     u32* cum = reinterpret_cast<u32*>(smem + kOffCum);                 // [2][kTileCounts]
 
-    if (kDown && a.summary && *a.summary) return;  // an aborted projection skips the stage
+    if (kDown && block_skips(a.summary)) return;  // an aborted projection skips the stage
 
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const u32 n_union = min(a.routes.counts[0], kMaxUnion);

@@ -940,3 +940,27 @@ def test_a_job_with_a_failed_projection_combines_no_row(gpu, rows, top_k, form, 
     x[2] = 3e38
     ffn(x, y=y, summary=summary)
     assert bool((y == 9.0).all()) and int(summary[0]) == b200moe.ROW_PROJECTION_NONFINITE
+
+
+@pytest.mark.parametrize("types,form,name", [((12, 12), "FORM_ROW_STREAM", "q4k_stream"), ((12, 12), "FORM_SEGMENT_STREAM", "q4k_wide"), ((12, 12), "FORM_PER_BLOCK", "q4k"),
+                                             ((12, 12), "FORM_GROUPED", "q4k_grouped"), ((8, 8), "FORM_SEGMENT_STREAM", "q8_wide"), ((8, 8), "FORM_PER_BLOCK", "q8"),
+                                             ((8, 8), "FORM_TENSOR", "q8_mma"), ((8, 8), "FORM_GROUPED", "q8_grouped")])
+def test_down_is_left_out_in_every_form(gpu, oracle, types, form, name):
+    """Any bit of the summary leaves the whole stage out, a word of zero lets it run, and the routes serve the next launch either way."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(7)
+    E, H, I, rows = 3, 256, 1024, 20
+    gate, up, down = synth.expert_tensors(rng, E, H, I, *types)
+    ids = window(rng, E, 2, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 2, *types, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
+    sh = ops.make_shape(H, I, E, 2, *types)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), 2 * rows)
+    with forced(getattr(b200moe, form)):
+        for bits in (b200moe.ROW_PROJECTION_NONFINITE, b200moe.JOB_WAIT_ABORTED, 0):
+            raw = torch.full((2 * rows, H), 7.0, device=gpu)
+            ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act, raw=raw, summary=torch.full((1,), bits, dtype=torch.int32, device=gpu))
+            assert b200moe.last_launch() == "down_" + name
+            assert bool((raw == 7.0).all()) if bits else same(raw.cpu(), want)

@@ -82,7 +82,8 @@ const char* b200moe_last_launch(void);
                                       * kernel all producers stop feeding before their n-th stage (no copy of that stage is issued, none is left in flight); 0 = never */
 #define B200MOE_DEBUG_DECODE_FORM 2u /* gate/up and down: 0 = chosen by the plan, 1 = row streaming (Q4_K), 2 = segment streaming (Q4_K;
                                       * Q8_0: the dp4a token-block form), 3 = per-block (Q8_0: one row per warp), 4 = the Q8_0
-                                      * tensor-core form, 5 = the grouped form (each only where it applies; grouped_min_rows is not looked at then) */
+                                      * tensor-core form, 5 = the grouped form, 6 = the Q8_0 one-item form (each only where it applies; grouped_min_rows is not
+                                      * looked at then) */
 int b200moe_debug_set(uint32_t key, uint32_t value);
 
 /* ------------------------------------------------------------------------------------------------ A8 activations

@@ -322,6 +322,7 @@ Q8Form pick_q8_form(const b200moe_shape& s, bool shot_fits, bool wide_fits, bool
     if (grouped_fits && (forced == 5 || (forced == 0 && q8_grouped_pays(s, mma_fits, rows, max_union, down)))) return Q8Form::grouped;
     if (forced == 4 && mma_fits) return Q8Form::mma;
     if (forced == 2 && wide_fits) return Q8Form::wide;
+    if (forced == 6 && shot_fits) return Q8Form::shot;
     if (forced == 0) {
         const u64 slots = u64(rows) * s.top_k;
         const u32 longest = std::max(s.hidden, s.inter);

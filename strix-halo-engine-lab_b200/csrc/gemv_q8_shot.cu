@@ -219,7 +219,7 @@ int launch_shot(const ShotPlan& p, dim3 grid, const CUtensorMap& tm0, const CUte
     const auto kernel = p.cap == 1 ? q8_shot_kernel<DOWN, 1> : p.cap == 2 ? q8_shot_kernel<DOWN, 2> : p.cap <= 4 ? q8_shot_kernel<DOWN, 4> : q8_shot_kernel<DOWN, 8>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), p.smem)) return rc;
     chain_launch(kernel, grid, kThreads, p.smem, stream, tm0, tm1, a);
-    return after_launch(DOWN ? "down_q8" : "gate_up_q8");  // the names of the forms below 8 rows
+    return after_launch(DOWN ? "down_q8_shot" : "gate_up_q8_shot");
 }
 
 }  // namespace

@@ -227,7 +227,7 @@ def test_q8_grouped_units(gpu, oracle, tokens, H, I):
 @pytest.mark.parametrize("rows,top_k,E,H,I,gate_form,down_form", [
     (8, 1, 1, 1024, 7168, "q8_mma", "q8_mma"), (9, 1, 1, 1024, 7168, "q8_grouped", "q8_mma"), (16, 1, 1, 1024, 7168, "q8_grouped", "q8_mma"),
     (17, 4, 10, 1024, 1024, "q8_mma", "q8_mma"), (18, 4, 10, 1024, 1024, "q8_grouped", "q8_mma"), (40, 4, 10, 1024, 1024, "q8_grouped", "q8_grouped"),
-    (20, 2, 2, 1024, 9728, "q8_grouped", "q8_grouped"), (7, 1, 1, 512, 512, "q8", "q8"), (8, 1, 1, 512, 512, "q8_grouped", "q8_grouped"),
+    (20, 2, 2, 1024, 9728, "q8_grouped", "q8_grouped"), (7, 1, 1, 512, 512, "q8_shot", "q8_shot"), (8, 1, 1, 512, 512, "q8_grouped", "q8_grouped"),
     (9, 4, 10, 512, 768, "q8_wide", "q8_wide"), (10, 4, 10, 512, 768, "q8_grouped", "q8_grouped")])
 def test_q8_grouped_form_lines(gpu, oracle, rows, top_k, E, H, I, gate_form, down_form):
     """Both sides of the lines between the streaming and the grouped Q8_0 form, where the tensor-core form applies and where it does not: gate/up and
@@ -639,7 +639,7 @@ def test_grouped_waits_run_out(gpu, oracle, types, H, I, stall):
 
 @pytest.mark.parametrize("types,form,stem", [((12, 12), "FORM_SEGMENT_STREAM", "q4k_wide"), ((12, 12), "FORM_PER_BLOCK", "q4k"), ((12, 12), "FORM_GROUPED", "q4k_grouped"),
                                              ((8, 8), "FORM_SEGMENT_STREAM", "q8_wide"), ((8, 8), "FORM_PER_BLOCK", "q8"), ((8, 8), "FORM_TENSOR", "q8_mma"),
-                                             ((8, 8), "FORM_GROUPED", "q8_grouped")])
+                                             ((8, 8), "FORM_GROUPED", "q8_grouped"), ((8, 8), "FORM_ONE_ITEM", "q8_shot")])
 @pytest.mark.parametrize("rows,top_k", [(9, 1), (70, 2)])
 def test_forced_form_is_the_one_that_runs(gpu, oracle, types, form, stem, rows, top_k):
     """A forced form beats the choice by rows and entries (70 entries an expert, where the plan takes the grouped forms, and about 4)."""
@@ -793,9 +793,9 @@ def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I):
     w = dv(gate, gpu), dv(up, gpu), dv(down, gpu)
     x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
     act, g, u = ops.enqueue_routed_gate_up(sh, *w[:2], r, E, x, rows * top_k, taps=True)
-    assert b200moe.last_launch() == "gate_up_q8"
+    assert b200moe.last_launch() == "gate_up_q8_shot"
     raw = ops.enqueue_routed_down(sh, w[2], r, E, act)
-    assert b200moe.last_launch() == "down_q8"
+    assert b200moe.last_launch() == "down_q8_shot"
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
     layer = ops.MoeLayer(sh, *w, capacity=rows, combine_form=b200moe.COMBINE_PARTS, parts=1)
     for _ in range(2):  # down asks for its weights before its wait
@@ -835,6 +835,10 @@ def test_four_chain_down_by_bulk_copies(gpu, oracle, rows, top_k, E, H, I, down_
     x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
     for _ in range(2):
         assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act = ops.enqueue_routed_gate_up(sh, layer.gate, layer.up, r, E, x, rows * top_k)
+    raw = ops.enqueue_routed_down(sh, layer.down, r, E, act)
+    assert b200moe.last_launch() == ("down_q8_chain4" if I >= 8192 else "down_chain4_stream") and same(raw.cpu(), want["raw"])
 
 
 @pytest.mark.parametrize("rows,hidden,experts", [(1, 132, 1), (5, 100, 33), (9, 516, 15), (600, 260, 40), (1201, 388, 17), (7120, 132, 33), (14207, 4, 1), (3560, 260, 130)])
@@ -944,7 +948,7 @@ def test_a_job_with_a_failed_projection_combines_no_row(gpu, rows, top_k, form, 
 
 @pytest.mark.parametrize("types,form,name", [((12, 12), "FORM_ROW_STREAM", "q4k_stream"), ((12, 12), "FORM_SEGMENT_STREAM", "q4k_wide"), ((12, 12), "FORM_PER_BLOCK", "q4k"),
                                              ((12, 12), "FORM_GROUPED", "q4k_grouped"), ((8, 8), "FORM_SEGMENT_STREAM", "q8_wide"), ((8, 8), "FORM_PER_BLOCK", "q8"),
-                                             ((8, 8), "FORM_TENSOR", "q8_mma"), ((8, 8), "FORM_GROUPED", "q8_grouped")])
+                                             ((8, 8), "FORM_TENSOR", "q8_mma"), ((8, 8), "FORM_GROUPED", "q8_grouped"), ((8, 8), "FORM_ONE_ITEM", "q8_shot")])
 def test_down_is_left_out_in_every_form(gpu, oracle, types, form, name):
     """Any bit of the summary leaves the whole stage out, a word of zero lets it run, and the routes serve the next launch either way."""
     import b200moe
@@ -964,3 +968,26 @@ def test_down_is_left_out_in_every_form(gpu, oracle, types, form, name):
             ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act, raw=raw, summary=torch.full((1,), bits, dtype=torch.int32, device=gpu))
             assert b200moe.last_launch() == "down_" + name
             assert bool((raw == 7.0).all()) if bits else same(raw.cpu(), want)
+
+
+@pytest.mark.parametrize("rows,top_k,E,H,I", [(8, 1, 1, 256, 10240), (9, 1, 1, 256, 10240), (20, 2, 3, 512, 4096), (12, 1, 2, 1024, 2304), (1, 1, 1, 512, 12288)])
+def test_q8_one_item_a_cta_at_its_plan_limits(gpu, oracle, rows, top_k, E, H, I):
+    """Rows so long that a pass holds half of eight entries, that only two stages fit, entries in several passes that bring the rows in again."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 8, 8)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, top_k, 8, 8)
+    w, x = (dv(gate, gpu), dv(up, gpu), dv(down, gpu)), (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu))
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    layer = ops.MoeLayer(sh, *w, capacity=rows, combine_form=b200moe.COMBINE_PARTS, parts=1)
+    with forced(b200moe.FORM_ONE_ITEM):
+        act, g, u = ops.enqueue_routed_gate_up(sh, *w[:2], r, E, x, rows * top_k, taps=True)
+        assert b200moe.last_launch() == "gate_up_q8_shot"
+        raw = ops.enqueue_routed_down(sh, w[2], r, E, act)
+        assert b200moe.last_launch() == "down_q8_shot"
+        assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+        assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])

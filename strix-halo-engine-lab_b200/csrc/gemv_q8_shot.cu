@@ -22,7 +22,7 @@ constexpr u32 kRunBlocks = 32, kRunBytes = kRunBlocks * kQ8Block, kHalf = 32;  /
 constexpr u32 kStageBytes = 2 * kHalf * kRunBytes, kStages = 3;
 constexpr u32 kWarps = 16, kRowsWarp = 64 / kWarps, kThreads = kWarps * 32;
 constexpr u32 kMaxEntries = 8;
-constexpr u32 kWaitPolls = 1u << 18;
+constexpr u32 kWaitPolls = 1u << 18;  // about a second
 
 struct ShotArgs {
     b200moe_routes routes;
@@ -36,6 +36,7 @@ struct ShotArgs {
     u32 rows_per_expert, out_width;
     u32 early;                  // routes and weights are complete before the launch in front was admitted (ChainHints)
     u32 bounded;                // the routes' arrays hold an expert for every CTA
+    u32 wait_limit, stall_stage;  // test hook: run `stall_stage` of a CTA's runs and those behind it are not asked for
 };
 
 template <bool DOWN, int NR>
@@ -109,12 +110,12 @@ __global__ void __launch_bounds__(kThreads) q8_shot_kernel(const __grid_constant
         tma_2d(st + kHalf * kRunBytes, DOWN ? &tm0 : &tm1, x, DOWN ? y + kHalf : y, bar);
     };
     const u32 passes = (ee - eb + a.cap - 1) / a.cap, total = passes * a.runs;  // an expert of more entries than a pass holds has its rows brought in again
-    u32 asked = min(total, a.stages);
+    u32 asked = min(min(total, a.stages), a.stall_stage);
     if (tid == 0) for (u32 n = 0; n < asked; ++n) ask(n);
     if (a.early) chain_begin();
     auto drain = [&](u32 from) {  // one thread: the copies asked for land (the wait is bounded) before the CTA retires
         for (u32 n = from; n < asked; ++n)
-            for (u32 i = 0; i < (kWaitPolls >> 4) + 64u; ++i)
+            for (u32 i = 0; i < (a.wait_limit >> 4) + 64u; ++i)
                 if (mbar_try_wait(&full[n % a.stages], (n / a.stages) & 1u, kWaitHintNs)) break;
     };
     if (DOWN && a.summary && *a.summary) {  // an aborted projection skips the stage
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(kThreads) q8_shot_kernel(const __grid_constant
     }
     const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, groups = a.K / 32;
     bool ok = true;
-    u32 n = 0;
+    u32 n = 0, landed = 0;  // the run in hand; the runs that have been seen to land
     for (u32 p0 = eb; p0 < ee; p0 += a.cap) {
         const u32 nr = min(a.cap, ee - p0);
         const u32 my_slot = lane < nr ? load(a.routes.slots + p0 + lane) : 0u;
@@ -144,17 +145,21 @@ __global__ void __launch_bounds__(kThreads) q8_shot_kernel(const __grid_constant
 #pragma unroll
             for (int r = 0; r < NR; ++r) cls[i][r] = 0.0f;
         for (u32 run = 0; run < a.runs; ++run, ++n) {
-            ok = mbar_wait(&full[n % a.stages], (n / a.stages) & 1u, kWaitPolls, &s_abort);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            shot_run<DOWN, NR>(smem + (n % a.stages) * kStageBytes, min(kRunBlocks, groups - run * kRunBlocks), run * kRunBlocks, warp, lane, s_codes, s_deltas, a.K, nr, cls);
+            // A warp whose wait ran out does no more work, but meets the barriers of the others: the block leaves as one.
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&full[n % a.stages], (n / a.stages) & 1u, a.wait_limit, &s_abort));
+            if (ok) {
+                shot_run<DOWN, NR>(smem + (n % a.stages) * kStageBytes, min(kRunBlocks, groups - run * kRunBlocks), run * kRunBlocks, warp, lane, s_codes, s_deltas, a.K, nr, cls);
+                landed = n + 1u;
+            }
             if (n + a.stages < total) {  // uniform over the block
-                if (__syncthreads_or(*reinterpret_cast<volatile u32*>(&s_abort))) { ok = false; break; }  // the place has been read
-                if (tid == 0) {
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    ask(n + a.stages);
+                if (__syncthreads_or(!ok)) { ok = false; break; }  // the place has been read
+                if (n + a.stages < a.stall_stage) {
+                    if (tid == 0) {
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        ask(n + a.stages);
+                    }
+                    ++asked;
                 }
-                ++asked;
             }
         }
         if (__syncthreads_or(!ok)) { ok = false; break; }
@@ -194,7 +199,7 @@ __global__ void __launch_bounds__(kThreads) q8_shot_kernel(const __grid_constant
     }
     if (!ok) {
         if (tid == 0) {
-            drain(n);
+            drain(landed);
             if (a.summary) atomicOr(a.summary, kAbortBit);
         }
     }
@@ -212,6 +217,12 @@ bool shot_plan(u32 K, u32 rows, ShotPlan* p) {
         }
         if (p->cap == 1) return false;
     }
+}
+
+void set_waits(ShotArgs* a) {
+    const u32 limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT), stall = debug_value(B200MOE_DEBUG_STALL_STAGE);
+    a->wait_limit = limit ? limit : kWaitPolls;
+    a->stall_stage = stall ? stall - 1u : 0xffffffffu;
 }
 
 template <bool DOWN>
@@ -243,6 +254,7 @@ int launch_gate_up_q8_shot(const b200moe_gate_up_view& v, u32 rows, const ChainH
     a.routes = v.routes; a.in = v.x; a.act = v.act; a.gate_out = v.gate_out; a.up_out = v.up_out; a.summary = v.summary; a.limit = v.shape.limit;
     a.K = v.shape.hidden; a.runs = p.runs; a.stages = p.stages; a.cap = p.cap; a.rows_per_expert = v.shape.inter; a.out_width = v.shape.inter;
     a.bounded = hints.slots >= v.max_union;
+    set_waits(&a);
     CUtensorMap tm0, tm1;
     const u64 rb = u64(a.K / 32) * kQ8Block, total = u64(v.shape.experts) * v.shape.inter;
     if (int rc = wide::rows_map(v.weights.gate, rb, total, kRunBytes, kHalf, &tm0)) return rc;
@@ -258,6 +270,7 @@ int launch_down_q8_shot(const b200moe_down_view& v, u32 rows, const ChainHints& 
     a.routes = v.routes; a.in = v.act; a.raw = v.raw; a.summary = const_cast<u32*>(v.summary);
     a.K = v.shape.inter; a.runs = p.runs; a.stages = p.stages; a.cap = p.cap; a.rows_per_expert = v.shape.hidden; a.out_width = v.shape.hidden;
     a.early = hints.routes_done; a.bounded = hints.slots >= v.max_union;
+    set_waits(&a);
     CUtensorMap tm0;
     if (int rc = wide::rows_map(v.weights.down, u64(a.K / 32) * kQ8Block, u64(v.shape.experts) * v.shape.hidden, kRunBytes, kHalf, &tm0)) return rc;
     return launch_shot<true>(p, dim3(v.shape.hidden / 64, v.max_union), tm0, tm0, a, stream);

@@ -991,3 +991,51 @@ def test_q8_one_item_a_cta_at_its_plan_limits(gpu, oracle, rows, top_k, E, H, I)
         assert b200moe.last_launch() == "down_q8_shot"
         assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
         assert same(layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True)[1].cpu(), want["raw"])
+
+
+@contextlib.contextmanager
+def stalled(form, stage, limit=2048):
+    """Producers stop asking for copies before a stage, waits run out after some milliseconds."""
+    import b200moe
+    b200moe.debug_set(b200moe.DEBUG_DECODE_FORM, form)
+    b200moe.debug_set(b200moe.DEBUG_WAIT_LIMIT, limit)
+    b200moe.debug_set(b200moe.DEBUG_STALL_STAGE, stage)
+    try:
+        yield
+    finally:
+        for key in (b200moe.DEBUG_DECODE_FORM, b200moe.DEBUG_WAIT_LIMIT, b200moe.DEBUG_STALL_STAGE):
+            b200moe.debug_set(key, 0)
+
+
+@pytest.mark.parametrize("rows,H,I,stage", [(3, 512, 512, 1), (8, 2304, 3072, 1), (8, 2304, 3072, 2), (8, 2304, 3072, 3), (1, 4096, 5120, 4), (20, 1024, 1024, 2), (20, 2048, 2048, 3),
+                                            (9, 7168, 4096, 6)])
+def test_q8_one_item_waits_run_out(gpu, oracle, rows, H, I, stage):
+    """A run that is never asked for: the first, one of the first places, one that takes a place again, one of a later pass. Both launches return with
+    B200MOE_JOB_WAIT_ABORTED, a layer of them writes nothing, the same calls without the hooks give the oracle's bits."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + H)
+    gate, up, down = synth.expert_tensors(rng, 1, H, I, 8, 8)
+    ids = np.zeros((rows, 1), np.uint32)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, 1, 1, 8, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, 1, 1, 8, 8)
+    w, x = (dv(gate, gpu), dv(up, gpu), dv(down, gpu)), (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu))
+    ids = dv(ids.view(np.int32), gpu)
+    r, one = ops.enqueue_moe_routes(ids, 1, 1), torch.ones((rows, 1), device=gpu)
+    layer = ops.MoeLayer(sh, *w, capacity=rows, combine_form=b200moe.COMBINE_PARTS, parts=1)
+    with forced(b200moe.FORM_ONE_ITEM):
+        good = ops.enqueue_routed_gate_up(sh, *w[:2], r, 1, x, rows)
+    flags = torch.zeros(8, dtype=torch.int32, device=gpu)
+    with stalled(b200moe.FORM_ONE_ITEM, stage):
+        ops.enqueue_routed_gate_up(sh, *w[:2], r, 1, x, rows, summary=flags[:1])
+        assert b200moe.last_launch() == "gate_up_q8_shot"
+        ops.enqueue_routed_down(sh, w[2], r, 1, good, summary=flags[4:5])
+        assert b200moe.last_launch() == "down_q8_shot"
+        assert flags[0].item() & b200moe.JOB_WAIT_ABORTED and flags[4].item() & b200moe.JOB_WAIT_ABORTED
+        assert not layer(x, ids, one).any()
+    with forced(b200moe.FORM_ONE_ITEM):
+        act, g, u = ops.enqueue_routed_gate_up(sh, *w[:2], r, 1, x, rows, taps=True)
+        raw = ops.enqueue_routed_down(sh, w[2], r, 1, act)
+        assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+        assert same(layer(x, ids, one, want_raw=True)[1].cpu(), want["raw"])

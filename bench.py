@@ -438,7 +438,7 @@ GATE_UP_KERNELS = {
     "gate_up_q4k_wide": "q4k_wide_kernel<gate/up> (routed experts, segment-streaming GEMV)",
     "gate_up_q4k_grouped": "grouped_q4k_kernel<gate/up> (routed experts over a token block, tensor-core dots)",
     "gate_up_q4k_stream": "gate_up_q4k_stream_kernel", "gate_up_q4k": "gate_up_q4k_kernel (per-block form)",
-    "gate_up_q8": "gate_up_q8_kernel", "gate_up_q8_wide": "q8_wide_kernel<gate/up>", "gate_up_q8_mma": "q8_mma_kernel<gate/up>",
+    "gate_up_q8": "gate_up_q8_kernel", "gate_up_q8_shot": "q8_shot_kernel<gate/up> (a CTA one item)", "gate_up_q8_wide": "q8_wide_kernel<gate/up>", "gate_up_q8_mma": "q8_mma_kernel<gate/up>",
     "gate_up_q8_grouped": "grouped_q8_kernel<gate/up>"}
 
 

@@ -80,8 +80,8 @@ const char* b200moe_last_launch(void);
                                       * down; 0 = the default (2^22; grouped Q8_0 2^20; one-item and four-chain 2^18). The grouped Q4_K kernel's limit (2^18, about
                                       * a second) and the row-streaming Q4_K kernels' are fixed */
 #define B200MOE_DEBUG_STALL_STAGE 1u /* n > 0: in every CTA of the Q4_K segment-streaming kernel the first producer, in every CTA of a grouped
-                                      * kernel all producers, in every CTA of the one-item Q8_0 kernel its only one stop feeding before their n-th stage (no copy
-                                      * of that stage is issued, none is left in flight); 0 = never */
+                                      * kernel all producers, in every CTA of the one-item Q8_0 kernel and of the four-chain down its only one stop feeding before
+                                      * their n-th stage (no copy of that stage is issued, none is left in flight); 0 = never */
 #define B200MOE_DEBUG_DECODE_FORM 2u /* gate/up and down: 0 = chosen by the plan, 1 = row streaming (Q4_K), 2 = segment streaming (Q4_K;
                                       * Q8_0: the dp4a token-block form), 3 = per-block (Q8_0: one row per warp), 4 = the Q8_0
                                       * tensor-core form, 5 = the grouped form, 6 = the Q8_0 one-item form (each only where it applies; grouped_min_rows is not

@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(256) down_q8_chain4_kernel(b200moe_down_view v
 // 640 -> 2560, top 8, Q5_1) each made that trip twice from registers, eight a multiprocessor and a second wave of 96, took 20 us.
 struct ChainPlan {
     u32 rows_per_item, n_chunks, cap, stage_bytes, a8_bytes;  // a8_bytes: of `cap` entries
-    u32 early, wait_limit;
+    u32 early, wait_limit, stall_stage;  // test hook: item `stall_stage` of a CTA's items and those behind it are not asked for
 };
 template <bool Q51>
 __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_view v, ChainPlan plan) {
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
     };
     u32 asked = 0;
     if (tid == 0)
-        for (; asked < 2 && blockIdx.x + asked * gridDim.x < n_items; ++asked) ask(asked, blockIdx.x + asked * gridDim.x);
+        for (; asked < min(2u, plan.stall_stage) && blockIdx.x + asked * gridDim.x < n_items; ++asked) ask(asked, blockIdx.x + asked * gridDim.x);
     if (plan.early) chain_begin();
     auto drain = [&](u32 from) {  // one thread: the copies asked for land (the wait is bounded) before the CTA retires
         for (u32 n = from; n < asked; ++n)
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
             }
         }
         __syncthreads();  // the stage and the buffer have been read
-        if (tid == 0 && item + 2 * gridDim.x < n_items) {
+        if (tid == 0 && item + 2 * gridDim.x < n_items && n + 2u < plan.stall_stage) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             ask(n + 2, item + 2 * gridDim.x);
             ++asked;
@@ -543,7 +543,9 @@ bool chain_plan(const b200moe_down_view& v, ChainPlan* p, u32* smem, u32* per_sm
     const u64 row_bytes = u64(I / 32) * block;
     p->cap = std::min<u32>(kR, std::max(1u, v.act.rows / v.shape.top_k));
     p->a8_bytes = (p->cap * (I + I / 32 * 8) + 15u) / 16u * 16u;
-    p->wait_limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT) ? debug_value(B200MOE_DEBUG_WAIT_LIMIT) : 1u << 18;
+    const u32 limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT), stall = debug_value(B200MOE_DEBUG_STALL_STAGE);
+    p->wait_limit = limit ? limit : 1u << 18;  // about a second
+    p->stall_stage = stall ? stall - 1u : 0xffffffffu;
     for (u32 R = 64; R >= 16; R /= 2) {
         const u64 stage = (R * row_bytes + 127) / 128 * 128, total = 2 * (stage + p->a8_bytes);
         if (total > 75u * 1024u && !(R == 16 && total <= 226u * 1024u)) continue;

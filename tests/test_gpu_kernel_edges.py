@@ -1039,3 +1039,29 @@ def test_q8_one_item_waits_run_out(gpu, oracle, rows, H, I, stage):
         raw = ops.enqueue_routed_down(sh, w[2], r, 1, act)
         assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
         assert same(layer(x, ids, one, want_raw=True)[1].cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("down_type", [7, 8])
+@pytest.mark.parametrize("rows,top_k,E,H,I,stage", [(1, 1, 1, 256, 544, 1), (9, 2, 3, 512, 640, 1), (8, 8, 32, 2048, 1536, 2), (8, 8, 32, 2048, 1536, 4), (20, 8, 64, 2560, 1088, 3)])
+def test_four_chain_waits_run_out(gpu, oracle, rows, top_k, E, H, I, stage, down_type):
+    """A CTA's first item, its second and one that takes a stage again are never asked for: down returns with B200MOE_JOB_WAIT_ABORTED, a layer writes nothing,
+    the same calls without the hooks give the oracle's bits."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
+    sh = ops.make_shape(H, I, E, top_k, 12, down_type)
+    x, ids, w = (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu)
+    layer = ops.MoeLayer(sh, dv(gate, gpu), dv(up, gpu), dv(down, gpu), capacity=rows, combine_form=b200moe.COMBINE_FMA_SLOTS)
+    r = ops.enqueue_moe_routes(ids, E, E // 2)
+    good = ops.enqueue_routed_gate_up(sh, layer.gate, layer.up, r, E, x, rows * top_k)
+    flag = torch.zeros(1, dtype=torch.int32, device=gpu)
+    with stalled(b200moe.FORM_AUTO, stage):
+        ops.enqueue_routed_down(sh, layer.down, r, E, good, summary=flag)
+        assert b200moe.last_launch() == "down_chain4_stream" and flag.item() & b200moe.JOB_WAIT_ABORTED
+        assert not layer(x, ids, w).any()
+    assert same(ops.enqueue_routed_down(sh, layer.down, r, E, good).cpu(), want)
+    assert same(layer(x, ids, w, want_raw=True)[1].cpu(), want)

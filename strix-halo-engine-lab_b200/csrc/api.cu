@@ -644,9 +644,11 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
     r.weight = v->router_weight; r.logit_bias = v->logit_bias; r.bias = v->select_bias; r.policy = v->policy;
     r.logits = F.logits;  // the scores are not asked for
     r.ids = v->ids ? v->ids : F.ids; r.weights = v->route_weights ? v->route_weights : F.weights;
-    // Up to 8 rows: one launch for A8 and logits. Up to 32: selection and routes share a launch.
+    // Up to 8 rows: one launch for A8 and logits. Up to 32 rows over up to 256 experts: selection and routes share a launch. Over more experts two launches
+    // are the faster ones, since a block that both selects and routes has to hold a row's 32 keys a lane beside the routes (512 experts of 2048 x 256, top-8, two
+    // launches and one, us a call: 29.2 and 32.8 with 1 row, 46.9 and 54.9 with 8, 81 and 101 with 22).
     const LayerScratch L = carve_layer(F.layer, s, v->capacity);
-    const bool fused = select_routes_fusable(r, s.top_k), one_launch = fused && prologue_fusable(r, s.top_k);
+    const bool fused = select_routes_fusable(r, s.top_k), one_launch = prologue_fusable(r, s.top_k);
     // Where the quantiser is a launch of its own it widens on the way (one pass over the activations instead of two).
     b200moe_quantize_a8_view qb = q;
     qb.x = v->x; qb.x_is_bf16 = 1;
@@ -666,9 +668,8 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
         if (widen_in_quantizer)
             if (int rc = launch_quantize_a8(qb, st, F.x_f32, s.hidden)) return rc;
         if (int rc = launch_router_logits(r, st, widen_in_quantizer ? nullptr : &q)) return rc;
-        if (!fused) if (int rc = launch_router_select(r, st)) return rc;
     }
-    if (fused) if (int rc = launch_select_routes(r, rv, clear_of(L, v->row_status, v->summary), st)) return rc;
+    if (int rc = fused ? launch_select_routes(r, rv, clear_of(L, v->row_status, v->summary), st) : launch_router_select(r, st)) return rc;
 
     b200moe_layer_view lv{};
     lv.shape = s; lv.weights = v->weights; lv.rows = v->rows; lv.x = F.x; lv.ids = r.ids; lv.route_weights = r.weights;

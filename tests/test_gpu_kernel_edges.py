@@ -1065,3 +1065,25 @@ def test_four_chain_waits_run_out(gpu, oracle, rows, top_k, E, H, I, stage, down
         assert not layer(x, ids, w).any()
     assert same(ops.enqueue_routed_down(sh, layer.down, r, E, good).cpu(), want)
     assert same(layer(x, ids, w, want_raw=True)[1].cpu(), want)
+
+
+@pytest.mark.parametrize("rows,experts,bf16,launches", [(1, 256, False, 5), (1, 257, False, 6), (8, 300, True, 6), (5, 1000, False, 6), (9, 300, False, 7), (9, 300, True, 7)])
+def test_front_over_many_experts(gpu, oracle, rows, experts, bf16, launches):
+    """Up to eight rows have A8 and logits in one launch over any number of experts; above 256, selection and routes take a launch each."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + experts)
+    H, I, K = 512, 256, 4
+    gate, up, down = synth.expert_tensors(rng, experts, H, I, 12, 12)
+    rw = synth.router_weight(rng, experts, H)
+    x = torch.from_numpy(synth.activations(rng, rows, H)).to(gpu)
+    x = x.bfloat16() if bf16 else x
+    ffn = ops.MoeFfn(ops.make_shape(H, I, experts, K, 12, 12), ops.softmax_policy(experts, K), *(dv(a, gpu) for a in (gate, up, down, rw)), capacity=rows,
+                     combine_form=b200moe.COMBINE_FMA_SLOTS)
+    want = oracle.ffn(O.Shape(H, I, experts, K, 12, 12, float("inf")), O.softmax_policy(experts, K), gate, up, down, rw, x.float().cpu().numpy(), O.COMBINE_FMA_SLOTS)
+    ffn.ws.fill_(0xff)
+    for _ in range(2):
+        before = b200moe.launch_count()
+        y, ids, wts = ffn(x, want_routes=True)
+        assert b200moe.launch_count() - before == launches
+        assert np.array_equal(ids.cpu().numpy().view(np.uint32), want["ids"]) and same(y.cpu(), want["y"])

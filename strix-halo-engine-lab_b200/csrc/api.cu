@@ -648,7 +648,7 @@ int b200moe_ffn(const b200moe_ffn_view* v, void* stream) {
     // are the faster ones, since a block that both selects and routes has to hold a row's 32 keys a lane beside the routes (512 experts of 2048 x 256, top-8, two
     // launches and one, us a call: 29.2 and 32.8 with 1 row, 46.9 and 54.9 with 8, 81 and 101 with 22).
     const LayerScratch L = carve_layer(F.layer, s, v->capacity);
-    const bool fused = select_routes_fusable(r, s.top_k), one_launch = prologue_fusable(r, s.top_k);
+    const bool fused = select_routes_fusable(r, s.top_k), one_launch = prologue_fusable(r);
     // Where the quantiser is a launch of its own it widens on the way (one pass over the activations instead of two).
     b200moe_quantize_a8_view qb = q;
     qb.x = v->x; qb.x_is_bf16 = 1;

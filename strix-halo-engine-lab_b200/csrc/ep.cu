@@ -313,7 +313,7 @@ int b200moe_ep_ffn(void* handle, const b200moe_ep_step_view* v, void* stream) {
     r.x = x32; r.x_stride = s.hidden; r.rows = v->rows; r.hidden = s.hidden;
     r.weight = v->router_weight; r.logit_bias = v->logit_bias; r.bias = v->select_bias; r.policy = ep->policy;
     r.logits = W.logits; r.scores = W.logits; r.ids = W.ids; r.weights = W.wts;
-    if (prologue_fusable(r, s.top_k)) {  // decode windows: A8 and logits in one launch
+    if (prologue_fusable(r)) {  // decode windows: A8 and logits in one launch
         if (int rc = launch_prologue(r, q, st)) return rc;
     } else {
         if (int rc = launch_router_logits(r, st, &q)) return rc;

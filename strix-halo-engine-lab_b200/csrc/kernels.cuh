@@ -89,7 +89,7 @@ int launch_down_q8_grouped(const b200moe_down_view& v, cudaStream_t stream);
 u32 debug_value(u32 key);
 
 // prologue.cu: A8 + router logits of a decode window (rows <= 8) in one launch; q.x / q.x_is_bf16 say where the activations are (r.x is not read)
-bool prologue_fusable(const b200moe_router_view& r, u32 top_k);
+bool prologue_fusable(const b200moe_router_view& r);
 int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view& q, cudaStream_t stream);
 
 // combine.cu

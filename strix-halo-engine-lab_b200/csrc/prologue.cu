@@ -12,8 +12,8 @@
 // 128, hidden 2048), of it 6 to 12 us in that block.
 #include <algorithm>
 
+#include "declared_math.cuh"
 #include "kernels.cuh"
-#include "router_select.cuh"
 
 namespace b200moe {
 namespace {
@@ -151,9 +151,7 @@ __global__ void __launch_bounds__(32 * (int(kBlockExperts) / EW) * (RT / RW)) pr
 
 }  // namespace
 
-bool prologue_fusable(const b200moe_router_view& r, u32 top_k) {
-    return r.rows >= 1 && r.rows <= 8 && u64(r.rows) * top_k <= 256u && r.rows * select_detail::scratch_floats(r.policy.experts) * 4u <= 64u * 1024u;
-}
+bool prologue_fusable(const b200moe_router_view& r) { return r.rows >= 1 && r.rows <= 8; }
 
 int launch_prologue(const b200moe_router_view& r, const b200moe_quantize_a8_view& q, cudaStream_t stream) {
     PrologueArgs a{};

@@ -1067,7 +1067,7 @@ def test_four_chain_waits_run_out(gpu, oracle, rows, top_k, E, H, I, stage, down
     assert same(layer(x, ids, w, want_raw=True)[1].cpu(), want)
 
 
-@pytest.mark.parametrize("rows,experts,bf16,launches", [(1, 256, False, 5), (1, 257, False, 6), (8, 300, True, 6), (5, 1000, False, 6), (9, 300, False, 7), (9, 300, True, 7)])
+@pytest.mark.parametrize("rows,experts,bf16,launches", [(1, 256, False, 5), (1, 257, False, 6), (8, 300, True, 6), (5, 1000, False, 6), (8, 1009, False, 6), (9, 300, False, 7), (9, 300, True, 7)])
 def test_front_over_many_experts(gpu, oracle, rows, experts, bf16, launches):
     """Up to eight rows have A8 and logits in one launch over any number of experts; above 256, selection and routes take a launch each."""
     import b200moe

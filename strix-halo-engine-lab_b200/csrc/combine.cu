@@ -85,37 +85,51 @@ __global__ void __launch_bounds__(256) combine_kernel(b200moe_combine_view v, u3
 
 // The PARTS form over whole rows with up to kVecTopK slots and 16-byte rows: four outputs a thread, every slot's values requested before the
 // first is used and no block-wide step, so that a block's loads overlap. Bound by HBM (raw read once, y written once): the
-// one-output form above, with one load in flight a thread, took 1441 us for 8192 rows x 8 x 7168, this one 613 us. The additions
-// and their order are those of combine_kernel. A small window is a chain of memory latencies: the job's summary, the row's status and its order are asked for
-// together, then all that the order leads to
-// (one row over 64 Q8_0 experts of 2048 -> 1024, top 4, 24.7 -> 23.0 us a call, 512 rows 316 -> 312).
-// early: weights, ids, order and low_counts were complete before the launch in front was admitted (ChainHints), so that what the order leads to is known
-// before the wait.
+// one-output form above, with one load in flight a thread, took 1441 us for 8192 rows x 8 x 7168, this one 444 us. The additions
+// and their order are those of combine_kernel. A small window is a chain of two memory latencies: the row's order, then all that the order leads to and
+// the row's status and the job's summary with it. 64 registers a thread, so that eight CTAs share a multiprocessor and cover the first of them (4096 rows
+// x 8 x 2048 80 us, 100 with five CTAs; 114 while weights and ids were asked for between the two). The order comes through L1: from L2 every warp of a row's CTAs asks
+// one 32-byte sector for it (53 rows x 8 x 7168 6.9 us, 5.0 through L1; the 4096 rows 62).
+// EARLY: order, weights, ids and low_counts were complete before the launch in front was admitted (ChainHints): what the order leads to is known before the
+// wait but for the values. An instance of its own: with a branch between the two, 1 row x 8 x 1024 took 4.4 us, 3.3 without.
 constexpr u32 kVecTopK = 8;
-__global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v, u32 skip_bits, bool zero_skipped, bool early) {
-    if (!early) chain_begin();
+template <bool CHAIN, bool EARLY>
+__global__ void __launch_bounds__(128, EARLY ? 1 : 8) combine_vec_kernel(b200moe_combine_view v, u32 skip_bits, bool zero_skipped) {
+    if (!EARLY) chain_begin_if<CHAIN>();
     const u32 o = 4u * (blockIdx.x * 128u + threadIdx.x);
     for (u32 row = blockIdx.y; row < v.rows; row += gridDim.y) {
-        u32 slot[kVecTopK], part[kVecTopK];
+        u32 slot[kVecTopK], part[kVecTopK], low = 0;  // part: the expert's id until the slot's turn comes, unless EARLY
         float w[kVecTopK];
         float4 x[kVecTopK];
-        const u32 low = v.low_counts ? load_l2(v.low_counts + row) : 0u;
+        auto part_of = [&](u32 k, u32 e) { return v.low_counts ? (k < low ? 0u : 1u) : min(e / v.part_experts, v.parts - 1); };
+        if (EARLY && v.low_counts) low = load_l2(v.low_counts + row);
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
-            if (k < v.top_k) slot[k] = min(load_l2(v.order + row * v.top_k + k), v.rows * v.top_k - 1u);  // the order of a row whose status is not zero may mean nothing
+            if (k < v.top_k) slot[k] = EARLY ? load_l2(v.order + row * v.top_k + k) : load(v.order + row * v.top_k + k);
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
             if (k < v.top_k) {
-                w[k] = __uint_as_float(load_l2(reinterpret_cast<const u32*>(v.weights) + slot[k]));
-                part[k] = v.low_counts ? (k < low ? 0u : 1u) : min(load_l2(v.ids + slot[k]) / v.part_experts, v.parts - 1);
+                slot[k] = min(slot[k], v.rows * v.top_k - 1u);  // the order of a row whose status is not zero may mean nothing
+                if (EARLY) {
+                    w[k] = __uint_as_float(load_l2(reinterpret_cast<const u32*>(v.weights) + slot[k]));
+                    part[k] = part_of(k, v.low_counts ? 0u : load_l2(v.ids + slot[k]));
+                }
             }
-        if (early && row == blockIdx.y) chain_begin();
+        if (EARLY && row == blockIdx.y) chain_begin();
         if (o >= v.hidden) return;
         const bool skipped = v.summary && (load(v.summary) & skip_bits);
         const u32 status = v.row_status ? load(v.row_status + row) : 0u;
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
-            if (k < v.top_k) x[k] = load(reinterpret_cast<const float4*>(v.raw + u64(slot[k]) * v.hidden + o));
+            if (k < v.top_k) {
+                const float4* at = reinterpret_cast<const float4*>(v.raw + u64(slot[k]) * v.hidden + o);
+                x[k] = EARLY ? load(at) : __ldcs(at);
+                if (!EARLY) {
+                    w[k] = load(v.weights + slot[k]);
+                    part[k] = v.low_counts ? 0u : load(v.ids + slot[k]);
+                }
+            }
+        if (!EARLY && v.low_counts) low = load(v.low_counts + row);
         const float4 sh = v.shared ? load(reinterpret_cast<const float4*>(v.shared + u64(row) * v.hidden + o)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         float4 y = sh, sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         u32 p = 0;
@@ -127,8 +141,9 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
 #pragma unroll
         for (u32 k = 0; k < kVecTopK; ++k)
             if (run && k < v.top_k) {
-                for (; p < part[k]; ++p) flush();
-                run = part[k] == p;
+                const u32 to = EARLY ? part[k] : part_of(k, part[k]);
+                for (; p < to; ++p) flush();
+                run = to == p;
                 if (run) {
                     sum.x = __fadd_rn(sum.x, __fmul_rn(w[k], x[k].x)); sum.y = __fadd_rn(sum.y, __fmul_rn(w[k], x[k].y));
                     sum.z = __fadd_rn(sum.z, __fmul_rn(w[k], x[k].z)); sum.w = __fadd_rn(sum.w, __fmul_rn(w[k], x[k].w));
@@ -150,8 +165,9 @@ __global__ void __launch_bounds__(128) combine_vec_kernel(b200moe_combine_view v
 // row's status, the job's summary, weights, values - is asked for before any of them is looked at: a small window is a chain of
 // memory latencies (three in the general form, with two block barriers between them), a large one wants bytes in flight.
 // 4096 rows x 8 x 2048: 79 us in the general form, 60 here (5.0 TB/s); 8 rows 3.1 and 2.2; 37 rows 4.0 and 2.8.
+template <bool CHAIN>
 __global__ void __launch_bounds__(128) combine_slots_kernel(b200moe_combine_view v, u32 skip_bits, bool zero_skipped) {
-    chain_begin();
+    chain_begin_if<CHAIN>();
     const u32 o = 2u * (blockIdx.x * 128u + threadIdx.x);
     if (o >= v.hidden) return;
     const u32 job = v.summary ? load(v.summary) : 0u;
@@ -225,18 +241,23 @@ int launch_combine(const b200moe_combine_view& v, cudaStream_t stream, u32 skip_
     if (v.rows == 0) return B200MOE_OK;
     // PARTS in one row: a whole call 37.2 us in the general form, 35.5 in the wide one; 32 rows x 8 x 2048 of 8 parts 5.0 and 4.2 us.
     const bool whole = v.y && !v.y_blocks && v.top_k <= kVecTopK;
+    const u32 rows = std::min<u32>(v.rows, 65535u);
     if (v.form == B200MOE_COMBINE_PARTS && whole && v.only_part < 0 && v.hidden % 4 == 0 && aligned(v.raw, 16) && aligned(v.y, 16) && aligned(v.shared, 16) && aligned(v.y_bf16, 8)) {
-        if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_vec_kernel))) return rc;
-        chain_launch(combine_vec_kernel, dim3((v.hidden + 511) / 512, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v, skip_bits, zero_skipped, hints.routes_done);
+        const dim3 grid((v.hidden + 511) / 512, rows);
+        if (!chain_pays(u64(grid.x) * rows)) plain_launch(combine_vec_kernel<false, false>, grid, 128, 0, stream, v, skip_bits, zero_skipped);
+        else small_launch(hints.routes_done ? combine_vec_kernel<true, true> : combine_vec_kernel<true, false>, grid, 128, 0, stream, v, skip_bits, zero_skipped);
         return after_launch("combine");
     }
     if (v.form == B200MOE_COMBINE_FMA_SLOTS && whole && v.hidden % 2 == 0 && aligned(v.raw, 8) && aligned(v.y, 8) && aligned(v.shared, 8) && aligned(v.y_bf16, 4)) {
-        if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_slots_kernel))) return rc;
-        chain_launch(combine_slots_kernel, dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 128, 0, stream, v, skip_bits, zero_skipped);
+        const dim3 grid((v.hidden + 255) / 256, rows);
+        if (chain_pays(u64(grid.x) * rows)) small_launch(combine_slots_kernel<true>, grid, 128, 0, stream, v, skip_bits, zero_skipped);
+        else plain_launch(combine_slots_kernel<false>, grid, 128, 0, stream, v, skip_bits, zero_skipped);
         return after_launch("combine");
     }
     if (int rc = prefer_max_shared(reinterpret_cast<const void*>(combine_kernel))) return rc;
-    chain_launch(combine_kernel, dim3((v.hidden + 255) / 256, std::min<u32>(v.rows, 65535u)), 256, 0, stream, v, skip_bits, zero_skipped);
+    const dim3 grid((v.hidden + 255) / 256, rows);
+    if (chain_pays(u64(grid.x) * rows)) chain_launch(combine_kernel, grid, 256, 0, stream, v, skip_bits, zero_skipped);
+    else plain_launch(combine_kernel, grid, 256, 0, stream, v, skip_bits, zero_skipped);
     return after_launch("combine");
 }
 int launch_canonical_sum(const float* a, const float* b, const float* c, u64 count, float* y, cudaStream_t stream) {

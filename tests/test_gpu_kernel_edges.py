@@ -1090,3 +1090,21 @@ def test_front_over_many_experts(gpu, oracle, rows, experts, bf16, launches):
         y, ids, wts = ffn(x, want_routes=True)
         assert b200moe.launch_count() - before == launches
         assert np.array_equal(ids.cpu().numpy().view(np.uint32), want["ids"]) and same(y.cpu(), want["y"])
+
+
+@pytest.mark.parametrize("rows,top_k,hidden", [(1, 4, 2048), (37, 8, 4096), (38, 8, 4096), (150, 3, 516), (296, 1, 512), (297, 1, 512)])
+@pytest.mark.parametrize("form", [0, 1])
+def test_combine_launch_forms(gpu, oracle, rows, top_k, hidden, form):
+    """Both sides of the line between programmatic and plain launches of the combine (two CTAs a multiprocessor), back to back into the same y."""
+    from b200moe import ops
+    rng = np.random.default_rng(rows + hidden)
+    E = 16
+    ids = window(rng, E, top_k, rows)
+    wts = rng.uniform(0.05, 0.6, (rows, top_k)).astype(np.float32)
+    shared = rng.standard_normal((rows, hidden), dtype=np.float32)
+    order = (np.argsort(ids, axis=1) + np.arange(rows)[:, None] * top_k).astype(np.int32)
+    for _ in range(3):
+        raw = rng.standard_normal((rows * top_k, hidden), dtype=np.float32)
+        want = oracle.combine(form, raw, wts, ids, shared=shared, parts=2, part_experts=E // 2) if form == 0 else oracle.combine(form, raw, wts, ids) + shared
+        y = ops.enqueue_moe_combine(form, dv(raw, gpu), dv(wts, gpu), dv(ids.view(np.int32), gpu), order=dv(order, gpu), shared=dv(shared, gpu), parts=2, part_experts=E // 2)
+        assert same(y.cpu(), want)

@@ -13,9 +13,9 @@ namespace {
 
 // WARPS: warps of the CTA, 0 = as launched (8 to 32). A fixed number unrolls the second pass at 48 registers, five CTAs of 8 warps an
 // SM; as launched it takes 29, eight CTAs.
-template <u32 WARPS>
+template <u32 WARPS, bool CHAIN>
 __global__ void __launch_bounds__(WARPS ? WARPS * 32u : 1024u) rmsnorm_a8_kernel(b200moe_rmsnorm_view v) {
-    chain_begin();
+    chain_begin_if<CHAIN>();
     __shared__ float partial[256];
     const u32 r = blockIdx.x, t = threadIdx.x, n = v.n;
     const u32 x_stride = v.x_stride ? v.x_stride : n, out_stride = v.out_stride ? v.out_stride : n;
@@ -76,9 +76,10 @@ int launch_rmsnorm_a8(const b200moe_rmsnorm_view& v, cudaStream_t stream) {
     // as launched; 1024 rows 50.3 as launched against 64.1 with five to six CTAs an SM) and are long enough for it to matter
     // (592 rows of 2048: 11.6 against 11.8; of 1024: 7.5 both).
     const u32 sms = static_cast<u32>(device_sm_count());
-    const u32 warps = v.rows <= 2u * sms ? std::min(32u, (v.n / 32u + 7u) / 8u * 8u) : 8u;
-    if (v.rows > 2u * sms && v.rows <= 5u * sms && v.n >= kWideRow) small_launch(rmsnorm_a8_kernel<8>, v.rows, 256, 0, stream, v);
-    else small_launch(rmsnorm_a8_kernel<0>, v.rows, 32u * warps, 0, stream, v);
+    const u32 warps = std::min(32u, (v.n / 32u + 7u) / 8u * 8u);
+    if (chain_pays(v.rows)) small_launch(rmsnorm_a8_kernel<0, true>, v.rows, 32u * warps, 0, stream, v);
+    else if (v.rows <= 5u * sms && v.n >= kWideRow) plain_launch(rmsnorm_a8_kernel<8, false>, v.rows, 256, 0, stream, v);
+    else plain_launch(rmsnorm_a8_kernel<0, false>, v.rows, 256, 0, stream, v);
     return after_launch("rmsnorm_a8");
 }
 

@@ -35,6 +35,14 @@ __global__ void __launch_bounds__(1024) routes_small_kernel(b200moe_routes_view 
     routes_small_body(v, end, v.ids, counts);
 }
 
+// Windows of a few slots.
+__global__ void __launch_bounds__(32) routes_one_warp_kernel(b200moe_routes_view v, u32 end, Clear clear) {
+    chain_begin();
+    routes_detail::clear_words(clear, v.rows);
+    __syncwarp();  // the rows' status is cleared before it is set
+    routes_detail::routes_one_warp(v, end, v.ids);
+}
+
 // Decode windows: the router's selection (one warp per row) and the routes of the selected ids in ONE block, so the
 // layer prologue costs one launch less. Dynamic shared memory: the rows' selection scratch, then the routes' counts in its place. Up to 256 experts
 // (their keys fit the 64 registers that a block of 1024 threads has) and 8 rows in the form of 256 threads.
@@ -185,6 +193,10 @@ int launch_routes(const b200moe_routes_view& v, const RoutesClear& clear, cudaSt
     const u32 end = v.end ? v.end : v.experts;
     const Clear c{clear.row_status, clear.summary4, clear.summary};
     const u32 smem = counts_bytes(static_cast<u32>(std::min<u64>(n, kChunk)), v.experts);
+    if (n <= routes_detail::kWarpSlots) {
+        small_launch(routes_one_warp_kernel, 1, 32, 0, stream, v, end, c);
+        return after_launch("routes_small");
+    }
     if (n <= kChunk) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(routes_small_kernel), smem)) return rc;
         small_launch(routes_small_kernel, 1, small_threads(static_cast<u32>(n), v.experts), smem, stream, v, end, c);

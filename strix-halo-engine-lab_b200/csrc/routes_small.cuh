@@ -125,6 +125,49 @@ __device__ __forceinline__ u32 rank_of(const u16* counts, u32 run, u32 experts, 
 }
 __host__ __device__ constexpr u32 counts_bytes(u32 slots, u32 experts) { return (((slots + 31u) / 32u * experts * 2u) + 15u) / 16u * 16u; }
 
+// The build of a window of a few slots (kWarpSlots, 32 at most) by one warp: a slot a lane, every count from the other lanes' ids. No scan over the experts and no barrier, which
+// cost the form below more than the walk over the other slots costs here: over 64 and 1024 experts 1 slot 2.5 and 3.2 us a launch, here
+// 1.7 and 1.6, 8 slots 2.8 and 3.3, 2.2 both, 16 slots 2.7 and 3.4, 2.8 both, 32 slots 2.9 and 3.6, 3.8 both.
+constexpr u32 kWarpSlots = 16;
+__device__ __forceinline__ void routes_one_warp(const b200moe_routes_view& v, u32 end, const u32* ids) {
+    const u32 s = threadIdx.x, n = v.rows * v.top_k, K = v.top_k, row = s / K, first = row * K;
+    const u32 id = s < n ? ids[s] : 0xffffffffu;
+    u32 pos = 0, low = 0;
+    bool bad = id >= v.experts, repeats = false;
+    for (u32 i = 0; i < n; ++i) {
+        const u32 o = __shfl_sync(0xffffffffu, id, i);
+        const bool mine = i - first < K, same = mine && o == id && i != s;
+        pos += mine && (o < id || (same && i < s)) ? 1u : 0u;
+        low += mine && o < v.split ? 1u : 0u;
+        bad |= same;
+        repeats |= same && i < s;
+    }
+    const u32 e = s < n && !repeats && owned(id, v.experts, v.first, end) ? id : 0xffffffffu;
+    const u32 peers = __match_any_sync(0xffffffffu, e), rank = __popc(peers & ((1u << s) - 1u));
+    const bool entry = e != 0xffffffffu, head = entry && rank == 0;
+    const u32 heads = __ballot_sync(0xffffffffu, head), entries = __ballot_sync(0xffffffffu, entry), most = __reduce_max_sync(0xffffffffu, entry ? __popc(peers) : 0u);
+    u32 before = 0, uidx = 0;  // entries of the experts below, and how many these are
+    for (u32 i = 0; i < n; ++i) {
+        const bool below = __shfl_sync(0xffffffffu, e, i) < e;  // no entry is above every expert
+        before += below ? 1u : 0u;
+        uidx += below && (heads >> i & 1u) ? 1u : 0u;
+    }
+    if (s < n) {
+        v.out.order[first + pos] = s;
+        if (s == first) v.out.low_counts[row] = low;
+        if (bad && v.row_status) atomicOr(&v.row_status[row], B200MOE_ROW_INVALID_ROUTE);
+    }
+    if (entry) {
+        v.out.rows[before + rank] = row;
+        v.out.slots[before + rank] = s;
+        if (head) { v.out.experts[uidx] = e - v.base; v.out.begins[uidx + 1] = before + __popc(peers); }
+    }
+    if (s == 0) {
+        v.out.begins[0] = 0;
+        v.out.counts[0] = __popc(heads); v.out.counts[1] = most; v.out.counts[2] = __popc(entries); v.out.counts[3] = 0;
+    }
+}
+
 // The whole build of a window of up to kChunk slots by one block. ids: the slots' experts, global or shared memory (written before a barrier);
 // counts: counts_bytes(slots, experts) of shared memory. A slot's place in its row, the row's low count and check come from the row's ids in
 // shared memory, its place among its expert's entries from the ranks above and one scan over the experts: five block barriers.

@@ -692,7 +692,7 @@ def test_selection_by_reductions(gpu, oracle, experts, top_k, groups, kept, scor
                 assert same(gs.cpu(), ws) and np.array_equal(gi.cpu().numpy().view(np.uint32), wi) and same(gw.cpu(), ww)
 
 
-@pytest.mark.parametrize("rows,top_k,experts", [(1, 1, 1), (31, 1, 40), (4, 8, 16), (33, 1, 1024), (8, 32, 1000), (1024, 1, 2), (1024, 1, 1024), (341, 3, 7), (1025, 1, 3), (412, 5, 300), (9000, 2, 5)])
+@pytest.mark.parametrize("rows,top_k,experts", [(1, 1, 1), (16, 1, 1024), (17, 1, 1024), (5, 3, 7), (2, 8, 9), (31, 1, 40), (4, 8, 16), (33, 1, 1024), (8, 32, 1000), (1024, 1, 2), (1024, 1, 1024), (341, 3, 7), (1025, 1, 3), (412, 5, 300), (9000, 2, 5)])
 def test_routes_ranks(gpu, oracle, rows, top_k, experts):
     """Runs of 32 slots with a remainder, more than 255 entries an expert, one block and chunks of 1024 slots that cut rows."""
     from b200moe import ops
@@ -1108,3 +1108,28 @@ def test_combine_launch_forms(gpu, oracle, rows, top_k, hidden, form):
         want = oracle.combine(form, raw, wts, ids, shared=shared, parts=2, part_experts=E // 2) if form == 0 else oracle.combine(form, raw, wts, ids) + shared
         y = ops.enqueue_moe_combine(form, dv(raw, gpu), dv(wts, gpu), dv(ids.view(np.int32), gpu), order=dv(order, gpu), shared=dv(shared, gpu), parts=2, part_experts=E // 2)
         assert same(y.cpu(), want)
+
+
+@pytest.mark.parametrize("rows,top_k,first,end", [(4, 4, 0, 0), (4, 4, 3, 9), (5, 3, 2, 12), (2, 8, 0, 1), (16, 1, 5, 11), (6, 4, 3, 9), (9, 9, 4, 10)])
+def test_routes_with_invalid_rows(gpu, rows, top_k, first, end):
+    """Few slots (one warp) and more (one block): ids out of range, ids that repeat in their row, an owned range of the experts."""
+    import b200moe
+    from b200moe import ops
+    rng = np.random.default_rng(rows + top_k)
+    E = 14
+    ids = window(rng, E, top_k, rows)
+    ids[rows // 2, top_k - 1] = E + 3
+    if top_k > 1:
+        ids[0, 1] = ids[0, 0]
+    status = torch.zeros(rows, dtype=torch.int32, device=gpu)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, 6, first, end, first, row_status=status)
+    entries = [(e, row, row * top_k + k) for e in range(first, end or E) for row in range(rows) for k in range(top_k) if ids[row, k] == e and e not in ids[row, :k]]
+    union = sorted({e for e, _, _ in entries})
+    begins = [0] + [sum(e <= u for e, _, _ in entries) for u in union]
+    counts = [len(union), max([b - a for a, b in zip(begins, begins[1:])], default=0), len(entries), 0]
+    assert r.counts.cpu().tolist() == counts and r.experts.cpu().tolist()[:len(union)] == [e - first for e in union] and r.begins.cpu().tolist()[:len(union) + 1] == begins
+    assert r.rows.cpu().tolist()[:len(entries)] == [x[1] for x in entries] and r.slots.cpu().tolist()[:len(entries)] == [x[2] for x in entries]
+    assert np.array_equal(r.order.cpu().numpy().reshape(rows, top_k), np.argsort(ids, axis=1, kind="stable") + np.arange(rows)[:, None] * top_k)
+    assert np.array_equal(r.low_counts.cpu().numpy(), (ids < 6).sum(axis=1))
+    bad = {rows // 2} | ({0} if top_k > 1 else set())
+    assert [int(x) for x in status.cpu()] == [b200moe.ROW_INVALID_ROUTE if i in bad else 0 for i in range(rows)]

@@ -21,12 +21,13 @@ namespace {
 constexpr int kR = 8;      // entries per pass
 constexpr u32 kWarps = 8;  // weight rows in flight per CTA
 
-// The term of group g of a Q2_K row for one A8 row (codes: the 32 codes of the group, 4-byte aligned).
+// The term of group g of a Q2_K row for one A8 row (codes: the 32 codes of the group, 16-byte aligned: rows are whole groups behind an aligned base).
 __device__ __forceinline__ float term_q2_k(const u8* __restrict__ wrow, u32 g, const i8* __restrict__ codes, float delta) {
     const u8* blk = wrow + u64(g >> 3) * kQ2KBlock;
     const u32 within = g & 7u, half = within >> 2, shift = 2u * (within & 3u);
     const u32* q = reinterpret_cast<const u32*>(blk + 16u + 32u * half);
-    const u32* x = reinterpret_cast<const u32*>(codes);
+    const uint4 xa = load(reinterpret_cast<const uint4*>(codes)), xb = load(reinterpret_cast<const uint4*>(codes) + 1);
+    const u32 x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
     int qx[2] = {0, 0}, sx[2] = {0, 0};
 #pragma unroll
     for (int i = 0; i < 8; ++i) {

@@ -418,8 +418,9 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
         q4k::bulk_g2s(st, v.weights.down + (u64(load_l2(v.routes.experts + j)) * H + R * chunk) * row_bytes, bytes, &full[n & 1u]);
     };
     u32 asked = 0;
+    const u32 n_ask = plan.stall_stage == 0xffffffffu ? n_items : min(n_items, blockIdx.x + plan.stall_stage * gridDim.x);
     if (tid == 0)
-        for (; asked < min(2u, plan.stall_stage) && blockIdx.x + asked * gridDim.x < n_items; ++asked) ask(asked, blockIdx.x + asked * gridDim.x);
+        for (; asked < 2 && blockIdx.x + asked * gridDim.x < n_ask; ++asked) ask(asked, blockIdx.x + asked * gridDim.x);
     if (plan.early) chain_begin();
     auto drain = [&](u32 from) {  // one thread: the copies asked for land (the wait is bounded) before the CTA retires
         for (u32 n = from; n < asked; ++n)
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
             }
         }
         __syncthreads();  // the stage and the buffer have been read
-        if (tid == 0 && item + 2 * gridDim.x < n_items && n + 2u < plan.stall_stage) {
+        if (tid == 0 && item + 2 * gridDim.x < n_ask) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             ask(n + 2, item + 2 * gridDim.x);
             ++asked;

@@ -1045,7 +1045,7 @@ def test_q8_one_item_waits_run_out(gpu, oracle, rows, H, I, stage):
 
 
 @pytest.mark.parametrize("down_type", [7, 8])
-@pytest.mark.parametrize("rows,top_k,E,H,I,stage", [(1, 1, 1, 256, 544, 1), (9, 2, 3, 512, 640, 1), (8, 8, 32, 2048, 1536, 2), (8, 8, 32, 2048, 1536, 4), (20, 8, 64, 2560, 1088, 3)])
+@pytest.mark.parametrize("rows,top_k,E,H,I,stage", [(1, 1, 1, 256, 544, 1), (9, 2, 3, 512, 640, 1), (8, 8, 32, 2048, 768, 2), (8, 8, 32, 2048, 768, 4), (20, 8, 64, 2560, 640, 3)])
 def test_four_chain_waits_run_out(gpu, oracle, rows, top_k, E, H, I, stage, down_type):
     """A CTA's first item, its second and one that takes a stage again are never asked for: down returns with B200MOE_JOB_WAIT_ABORTED, a layer writes nothing,
     the same calls without the hooks give the oracle's bits."""
@@ -1133,3 +1133,21 @@ def test_routes_with_invalid_rows(gpu, rows, top_k, first, end):
     assert np.array_equal(r.low_counts.cpu().numpy(), (ids < 6).sum(axis=1))
     bad = {rows // 2} | ({0} if top_k > 1 else set())
     assert [int(x) for x in status.cpu()] == [b200moe.ROW_INVALID_ROUTE if i in bad else 0 for i in range(rows)]
+
+
+@pytest.mark.parametrize("down_type,rows,top_k,E,H,I,name", [(7, 4, 4, 60, 2560, 1536, "down_q8_chain4"), (7, 1, 4, 60, 2560, 1536, "down_chain4_stream"), (8, 16, 4, 60, 2560, 2048, "down_q8_chain4"),
+                                                             (8, 16, 4, 60, 2560, 768, "down_chain4_stream"), (7, 64, 4, 32, 2048, 1024, "down_q8_chain4"), (7, 64, 4, 32, 2048, 768, "down_chain4_stream")])
+def test_four_chain_form_lines(gpu, oracle, down_type, rows, top_k, E, H, I, name):
+    """Both sides of the line between the two forms of the four-chain down: rows that leave a multiprocessor few threads, over two rounds of items and more."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
+    sh = ops.make_shape(H, I, E, top_k, 12, down_type)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k)
+    raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, min(E, rows * top_k), act)
+    assert b200moe.last_launch() == name and same(raw.cpu(), want)

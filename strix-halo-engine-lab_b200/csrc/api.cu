@@ -292,10 +292,13 @@ Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_f
 // The DS41 family (Q8_0 x A8). Below kFewRows rows: a CTA one item with all its weights asked for at once (gemv_q8_shot.cu, rows of whole units of 256
 // weights), else one weight row per warp. From there on the tensor-core form of gemv_q8_mma.cu (rows of 1024 to 7168 weights), else the dp4a token-block form of
 // gemv_q8_wide.cu. The one-item form pays by the entry and keeps a multiprocessor for one item, so it gives way to the tensor-core form early where an expert has
-// more than four entries of long rows, and late where a window is sparse over short ones. Whole calls, one-item and tensor-core form, us: one expert of
+// more than four entries of long rows. From 8 rows on it is the better one only in windows so sparse that an expert has an entry at most, against the tensor-core
+// form, for down and for few items of gate/up (14 runs of 32 blocks a multiprocessor). Whole calls, one-item and tensor-core form, us: one expert of
 // 7168 x 2048 45 and 53 with 1 row, 55 and 56 with 4, 59 and 57 with 5, 64 and 59 with 7; of 2048 x 1024 31 and 37, 35 and 37 with 4, 37 and 39 with 6,
-// 39 and 38 with 7; 64 of 2048 x 1024, top-4, 80 and 81 with 7 rows, 86 and 90 with 8, 115 and 121 with 12, 125 and 123 with 14; 128 of these 90
-// and 98 with 8 rows, 119 and 123 with 12, 143 and 147 with 16; 16 of 4096 x 1536, top-2, 61 and 64 with 4, 82 and 80 with 6, 86 and 82 with 8.
+// 39 and 38 with 7; 64 of 2048 x 1024, top-4, 80 and 81 with 7 rows; 16 of 4096 x 1536, top-2, 61 and 64 with 4, 82 and 80 with 6, 86 and 82 with 8.
+// Layers, both stages in the tensor-core form, down alone and both in the one-item form: 64 of 2048 x 1024, top-4, 68.4, 63.9 and 67.0 with 8 rows, 93.2, 88.7
+// and 91.3 with 12; 512 of 1024 x 1024, top-4, 79.4, 74.2 and 69.1 with 12, 157.7, 151.6 and 156.1 with 32. Against the token-block form down loses: 256 of 2048 x 768,
+// top-8, 96.7 and 109.9 with 8 rows, 202 and 249 with 24.
 // The grouped form (grouped_q8.cu, tiles of 32 entries) takes over from the tensor-core form where its waves of tiles take less time than the
 // other's waves of items, both by their sizes: a tile 2.3 us + 0.7 a unit of 256 columns with up to 16 entries, 2.6 + 0.77 with more, an item of
 // 32 gate and up rows 3 us + 0.33 a unit, one of 32 down rows half of that. Tensor-core and grouped form, gate/up and down: one expert of
@@ -326,7 +329,9 @@ Q8Form pick_q8_form(const b200moe_shape& s, bool shot_fits, bool wide_fits, bool
     if (forced == 0) {
         const u64 slots = u64(rows) * s.top_k;
         const u32 longest = std::max(s.hidden, s.inter);
-        const bool shot = rows < kFewRows ? longest <= 2048 || slots <= u64(4) * s.experts || !mma_fits : longest <= 2048 && 4 * slots <= u64(3) * s.experts;
+        const bool sparse = mma_fits && longest <= 2048 && 4 * slots <= u64(3) * s.experts;
+        const u64 runs = slots * (s.inter / 32) * ((s.hidden + 1023) / 1024);  // that a sparse window's gate/up brings in, each 32 blocks of 64 rows
+        const bool shot = rows < kFewRows ? longest <= 2048 || slots <= u64(4) * s.experts || !mma_fits : sparse && (down || runs <= u64(14) * static_cast<u32>(device_sm_count()));
         if (shot_fits && shot) return Q8Form::shot;
         if (mma_fits && (rows >= kFewRows || shot_fits)) return Q8Form::mma;
         if (wide_fits && rows >= kFewRows) return Q8Form::wide;

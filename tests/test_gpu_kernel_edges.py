@@ -779,10 +779,11 @@ def test_down_skipped_after_its_weights_were_asked_for(gpu, oracle, rows, H, I, 
             assert same(layer(good, ids, one).cpu(), want["raw"])
 
 
-@pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 256, 256), (1, 4, 8, 2048, 1024), (2, 2, 3, 1280, 2304), (3, 2, 4, 3328, 512), (4, 1, 1, 7168, 4352),
-                                                    (4, 3, 3, 4096, 1024), (7, 1, 1, 2048, 1024), (5, 2, 40, 512, 768), (9, 1, 12, 2048, 512), (30, 3, 120, 1024, 1280)])
-def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I):
-    """Windows below 8 rows and sparse ones above: rows of one run, of whole and broken runs, of more runs than places; 1 to 9 entries an expert, in one pass
+@pytest.mark.parametrize("rows,top_k,E,H,I,forms", [(1, 1, 1, 256, 256, "shot shot"), (1, 4, 8, 2048, 1024, "shot shot"), (2, 2, 3, 1280, 2304, "shot shot"), (3, 2, 4, 3328, 512, "shot shot"),
+                                                    (4, 1, 1, 7168, 4352, "shot shot"), (4, 3, 3, 4096, 1024, "shot shot"), (7, 1, 1, 2048, 1024, "shot shot"), (5, 2, 40, 512, 768, "shot shot"),
+                                                    (9, 1, 12, 2048, 512, "shot wide"), (30, 3, 120, 1024, 1280, "mma shot"), (9, 2, 24, 1024, 1024, "shot shot")])
+def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I, forms):
+    """Windows below 8 rows and sparse ones above (there down where the tensor-core form would be taken, gate/up with few items): rows of one run, of whole and broken runs, of more runs than places; 1 to 9 entries an expert, in one pass
     and in several."""
     import b200moe
     from b200moe import ops, synth
@@ -796,9 +797,9 @@ def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I):
     w = dv(gate, gpu), dv(up, gpu), dv(down, gpu)
     x = dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)
     act, g, u = ops.enqueue_routed_gate_up(sh, *w[:2], r, E, x, rows * top_k, taps=True)
-    assert b200moe.last_launch() == "gate_up_q8_shot"
+    assert b200moe.last_launch() == "gate_up_q8_" + forms.split()[0]
     raw = ops.enqueue_routed_down(sh, w[2], r, E, act)
-    assert b200moe.last_launch() == "down_q8_shot"
+    assert b200moe.last_launch() == "down_q8_" + forms.split()[1]
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
     layer = ops.MoeLayer(sh, *w, capacity=rows, combine_form=b200moe.COMBINE_PARTS, parts=1)
     for _ in range(2):  # down asks for its weights before its wait

@@ -278,14 +278,20 @@ bool grouped_pays(const b200moe_shape& s, u32 rows, u32 max_union, u32 grouped_m
 // experts of 2048 x 768, one row, top 1 to 16, 30.8 and 28.7, 32.9 and 30.8, 36.9 and 34.7 (top 8), 45.1 and 41.2; two rows, top 8, 43.0 and 39.2; 16
 // experts of 512 x 256 28.7 and 26.6; dense 2048 x 2048 23.7 and 17.5, 512 x 512 21.5 and 15.4. B200MOE_DEBUG_DECODE_FORM forces
 // one of the four where it applies, whatever grouped_min_rows says.
+// Stages called by themselves (alone: nothing is known of the launch in front, so none starts early) keep the row-streaming form for one row of up to 2048
+// weights and, where rows are short, for two. A launch, us, row and segment streaming: gate/up of 64 of 2048 x 768, top-4, 6.8 and 7.8 with 1 row, 8.2 and 9.4
+// with 2; down 5.6 and 6.4, 7.3 and 6.7; down of 128 of 1024 x 256, top-8, 4.9 and 6.4, 5.7 and 6.5. Inside a layer gate/up is better off in the segment-streaming
+// form too (the 128 experts above, one row, top 8, whole call 24.0 and 23.5).
+bool row_stream_alone(u32 rows, u32 K, bool down) { return rows <= 1 ? K <= 2048 : rows == 2 && K <= (down ? 512u : 2048u); }
 enum class Q4Form { grouped, row_stream, wide, block };
-Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_fits, bool wide_fits, u32 rows, u32 max_union, u32 grouped_min_rows, bool down) {
+Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_fits, bool wide_fits, u32 rows, u32 max_union, u32 grouped_min_rows, bool alone, bool down) {
     const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
     if (forced == 1 && row_stream_fits) return Q4Form::row_stream;
     if (forced == 2 && wide_fits) return Q4Form::wide;
     if (forced == 3) return Q4Form::block;
     if (forced == 5 && grouped_fits) return Q4Form::grouped;
     if (grouped_fits && grouped_pays(s, rows, max_union, grouped_min_rows, wide_fits, down)) return Q4Form::grouped;
+    if (row_stream_fits && alone && row_stream_alone(rows, down ? s.inter : s.hidden, down)) return Q4Form::row_stream;
     if (wide_fits) return Q4Form::wide;
     return row_stream_fits ? Q4Form::row_stream : Q4Form::block;
 }
@@ -350,7 +356,7 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
         }
     }
     if (v.shape.gate_type == B200MOE_TYPE_Q5_K) return launch_gate_up_q4k(v, st);  // the per-block form reads both K-quant layouts
-    switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.x.sums != nullptr), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, v.max_union, grouped_min_rows, false)) {
+    switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.x.sums != nullptr), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, v.max_union, grouped_min_rows, hints.slots == 0, false)) {
         case Q4Form::grouped: return launch_gate_up_q4k_grouped(v, st);
         case Q4Form::row_stream: return launch_gate_up_q4k_stream(v, rows, st);
         case Q4Form::wide: return launch_gate_up_q4k_wide(v, rows, hints, st);
@@ -359,7 +365,7 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
 }
 int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0, const ChainHints& hints = {}) {
     if (v.shape.down_type == B200MOE_TYPE_Q4_K) {
-        switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.act.sums != nullptr), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, v.max_union, grouped_min_rows, true)) {
+        switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.act.sums != nullptr), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, v.max_union, grouped_min_rows, hints.slots == 0, true)) {
             case Q4Form::grouped: return launch_down_q4k_grouped(v, st);
             case Q4Form::row_stream: return launch_down_q4k_stream(v, rows, st);
             case Q4Form::wide: return launch_down_q4k_wide(v, rows, hints, st);

@@ -1093,6 +1093,45 @@ def test_front_over_many_experts(gpu, oracle, rows, experts, bf16, launches):
         assert np.array_equal(ids.cpu().numpy().view(np.uint32), want["ids"]) and same(y.cpu(), want["y"])
 
 
+@pytest.mark.parametrize("down_type,rows,top_k,E,H,I,name", [(7, 4, 4, 60, 2560, 1536, "down_q8_chain4"), (7, 1, 4, 60, 2560, 1536, "down_chain4_stream"), (8, 16, 4, 60, 2560, 2048, "down_q8_chain4"),
+                                                             (8, 16, 4, 60, 2560, 768, "down_chain4_stream"), (7, 64, 4, 32, 2048, 1024, "down_q8_chain4"), (7, 64, 4, 32, 2048, 768, "down_chain4_stream")])
+def test_four_chain_form_lines(gpu, oracle, down_type, rows, top_k, E, H, I, name):
+    """Both sides of the line between the two forms of the four-chain down: rows that leave a multiprocessor few threads, over two rounds of items and more."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
+    sh = ops.make_shape(H, I, E, top_k, 12, down_type)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k)
+    raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, min(E, rows * top_k), act)
+    assert b200moe.last_launch() == name and same(raw.cpu(), want)
+
+
+@pytest.mark.parametrize("rows,top_k,E,H,I,gate_form,down_form", [(1, 2, 4, 512, 768, "stream", "stream"), (2, 2, 4, 512, 768, "stream", "wide"), (2, 2, 4, 2048, 512, "stream", "stream"),
+                                                                            (3, 2, 4, 512, 256, "wide", "wide"), (1, 2, 4, 2304, 2304, "wide", "wide"), (2, 2, 4, 2304, 256, "wide", "stream")])
+def test_q4_k_forms_of_one_and_two_rows(gpu, oracle, rows, top_k, E, H, I, gate_form, down_form):
+    """Windows of one and two rows without an early start (the stages by themselves) stream whole rows of up to 2048 weights,
+    two rows of down up to 512."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + H)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, 12, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh = ops.make_shape(H, I, E, top_k, 12, 12)
+    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k, taps=True)
+    assert b200moe.last_launch() == "gate_up_q4k_" + gate_form
+    raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+    assert b200moe.last_launch() == "down_q4k_" + down_form
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+
+
 @pytest.mark.parametrize("rows,top_k,hidden", [(1, 4, 2048), (37, 8, 4096), (38, 8, 4096), (150, 3, 516), (296, 1, 512), (297, 1, 512)])
 @pytest.mark.parametrize("form", [0, 1])
 def test_combine_launch_forms(gpu, oracle, rows, top_k, hidden, form):
@@ -1134,21 +1173,3 @@ def test_routes_with_invalid_rows(gpu, rows, top_k, first, end):
     assert np.array_equal(r.low_counts.cpu().numpy(), (ids < 6).sum(axis=1))
     bad = {rows // 2} | ({0} if top_k > 1 else set())
     assert [int(x) for x in status.cpu()] == [b200moe.ROW_INVALID_ROUTE if i in bad else 0 for i in range(rows)]
-
-
-@pytest.mark.parametrize("down_type,rows,top_k,E,H,I,name", [(7, 4, 4, 60, 2560, 1536, "down_q8_chain4"), (7, 1, 4, 60, 2560, 1536, "down_chain4_stream"), (8, 16, 4, 60, 2560, 2048, "down_q8_chain4"),
-                                                             (8, 16, 4, 60, 2560, 768, "down_chain4_stream"), (7, 64, 4, 32, 2048, 1024, "down_q8_chain4"), (7, 64, 4, 32, 2048, 768, "down_chain4_stream")])
-def test_four_chain_form_lines(gpu, oracle, down_type, rows, top_k, E, H, I, name):
-    """Both sides of the line between the two forms of the four-chain down: rows that leave a multiprocessor few threads, over two rounds of items and more."""
-    import b200moe
-    from b200moe import ops, synth
-    rng = np.random.default_rng(rows + I)
-    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
-    ids = window(rng, E, top_k, rows)
-    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
-    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
-    sh = ops.make_shape(H, I, E, top_k, 12, down_type)
-    r = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
-    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top_k)
-    raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, min(E, rows * top_k), act)
-    assert b200moe.last_launch() == name and same(raw.cpu(), want)

@@ -281,7 +281,7 @@ bool grouped_pays(const b200moe_shape& s, u32 rows, u32 max_union, u32 grouped_m
 // Stages called by themselves (alone: nothing is known of the launch in front, so none starts early) keep the row-streaming form for one row of up to 2048
 // weights and, where rows are short, for two. A launch, us, row and segment streaming: gate/up of 64 of 2048 x 768, top-4, 6.8 and 7.8 with 1 row, 8.2 and 9.4
 // with 2; down 5.6 and 6.4, 7.3 and 6.7; down of 128 of 1024 x 256, top-8, 4.9 and 6.4, 5.7 and 6.5. Inside a layer gate/up is better off in the segment-streaming
-// form too (the 128 experts above, one row, top 8, whole call 24.0 and 23.5).
+// form too (a call over 128 experts of 2048 x 768, one row, top 8, 24.0 and 23.5).
 bool row_stream_alone(u32 rows, u32 K, bool down) { return rows <= 1 ? K <= 2048 : rows == 2 && K <= (down ? 512u : 2048u); }
 enum class Q4Form { grouped, row_stream, wide, block };
 Q4Form pick_q4_form(const b200moe_shape& s, bool grouped_fits, bool row_stream_fits, bool wide_fits, u32 rows, u32 max_union, u32 grouped_min_rows, bool alone, bool down) {

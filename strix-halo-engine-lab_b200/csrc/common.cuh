@@ -100,7 +100,7 @@ inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, 
 // Whether a launch of so many CTAs, several of which share a multiprocessor, is better a programmatic one. Such CTAs come onto the multiprocessors as the launch in
 // front leaves them, so that what leaves first gets as many as it can hold and the others none: up to two a multiprocessor that does not matter, and the start
 // that is saved does; above, the most loaded multiprocessor decides, and the chain's instructions cost every CTA (RMSNorm of 409 rows of 7168 22.9 us as a
-// programmatic launch behind another, 17.9 as a plain one; of 741 rows of 4096 20.0 and 17.0).
+// programmatic launch behind another, 18.5 as a plain one; of 741 rows of 4096 20.0 and 17.2).
 inline bool chain_pays(u64 ctas) { return ctas <= 2u * static_cast<u64>(device_sm_count()); }
 template <bool CHAIN>  // a kernel's instance for plain launches: all in front of it is complete, and it admits nothing early
 __device__ __forceinline__ void chain_begin_if() { if (CHAIN) chain_begin(); }

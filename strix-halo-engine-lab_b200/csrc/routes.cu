@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(1024) routes_count_kernel(b200moe_routes_view 
         if (clear.summary && t == 0) *clear.summary = 0u;
     }
     // Rows that are ranked in registers go to neighbouring threads; those that are sorted, in arrays of local memory, to the blocks in turn, so that a
-    // multiprocessor's L1 holds the arrays of its few (129 rows x 32: 63 us with all of them in one block, 258 when the carve-out left that block 28 KB of L1).
+    // multiprocessor's L1 holds the arrays of its few (129 rows x 32: 63 us with all of them in one block, 246 when the carve-out
+    // left that block 28 KB of L1, 51 here).
     for (u32 r = RANKED ? blockIdx.x * blockDim.x + t : t * gridDim.x + blockIdx.x; r < v.rows; r += gridDim.x * blockDim.x) {
         if (clear.row_status) clear.row_status[r] = 0u;  // the row's status is this thread's alone in this launch
         row_order<RANKED>(v.ids, r, v.top_k, v.experts, v.split, v.out.order, v.out.low_counts, v.row_status);

@@ -248,12 +248,12 @@ q8_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
 #pragma unroll
             for (int t = 0; t < (int)kKE; ++t) {
                 if (t < (int)ne) {
+                    float* out = DOWN ? a.raw + u64(__shfl_sync(0xffffffffu, my_slot, t)) * a.out_width + kRows * chunk + 4u * w : nullptr;
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
                         const float val = butterfly32(cls[r][t]);
-                        const u32 slot_id = __shfl_sync(0xffffffffu, my_slot, t);
                         if (lane == 0) {
-                            if (DOWN) a.raw[u64(slot_id) * a.out_width + kRows * chunk + 4u * w + r] = val;
+                            if (DOWN) out[r] = val;
                             else gu[mat * kKE * 32 + t * 32 + 4u * w + r] = val;
                         }
                     }

@@ -442,9 +442,10 @@ GATE_UP_KERNELS = {
     "gate_up_q8_grouped": "grouped_q8_kernel<gate/up>"}
 
 
-def gate_up_kernel_name(shape, gate, up, x, ids, first=0, end=0):
+def gate_up_kernel_name(shape, gate, up, down, x, ids, first=0, end=0):
     """The routed gate/up kernel that the library launches for this window (x: its rows, ids: their experts; [first, end): the experts held here),
-    from one launch of that stage alone, outside the timed regions."""
+    from one launch of that stage alone, outside the timed regions. Windows of one and two rows take another form alone than in a call: there the name is that
+    of the call's down, which runs in the same form."""
     import b200moe
     from b200moe import ops
     rows, top_k = ids.shape
@@ -452,6 +453,11 @@ def gate_up_kernel_name(shape, gate, up, x, ids, first=0, end=0):
     span = (end or shape.experts) - first
     ops.enqueue_routed_gate_up(shape, gate, up, routes, min(rows * top_k, span), ops.enqueue_quantize_a8(x), rows * top_k)
     name = b200moe.last_launch()
+    if rows <= 2:
+        import torch
+        layer = ops.MoeLayer(shape, gate, up, down, capacity=rows, combine_form=b200moe.COMBINE_FMA_SLOTS)
+        layer(ops.enqueue_quantize_a8(x), ids, torch.ones((rows, top_k), device=x.device), first=first, end=end, base=first, combine=False)
+        name = b200moe.last_launch().replace("down_", "gate_up_", 1)
     return GATE_UP_KERNELS.get(name, name)
 
 
@@ -683,7 +689,7 @@ def large_arm(args, cfg, rank, world, dev):
         mine = ids[(ids >= rank * per) & (ids < (rank + 1) * per)]
         uniq.append(len(np.unique(mine)))
         entries.append(mine.size)
-    gate_up_kernel = gate_up_kernel_name(shape, gate, up, torch.from_numpy(batches[-1]).to(dev), torch.from_numpy(ids).to(dev), rank * per if world > 1 else 0,
+    gate_up_kernel = gate_up_kernel_name(shape, gate, up, down, torch.from_numpy(batches[-1]).to(dev), torch.from_numpy(ids).to(dev), rank * per if world > 1 else 0,
                                          (rank + 1) * per if world > 1 else 0)
     uniq, entries = np.array(uniq, np.float64), np.array(entries, np.float64)
 
@@ -1066,7 +1072,7 @@ def decode_arm(args, cfg, rank, world, dev):
         "e2e": {"value": tokens / (host_ms / 1000.0), "unit": UNIT, "h2d_bytes_per_step": B * H * 4, "d2h_bytes_per_step": B * H * 4,
                 "ms_per_step": host_ms / K},
         "gpu_launches": int(round(launches_per_step * K)),
-        "roofline": {"kernel": gate_up_kernel_name(shape, layers[0].gate, layers[0].up, xs[0], ids), "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"kernel": gate_up_kernel_name(shape, layers[0].gate, layers[0].up, layers[0].down, xs[0], ids), "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": f"{peak_kind} HBM copy",
                      # dram read + write per launch from an ncu capture of this kernel on this workload: 1.00 of the algorithmic bytes
                      "traffic": algo_bytes * NCU_TRAFFIC_RATIO if cfg["gate_type"] == 12 else None,

@@ -388,7 +388,7 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
-_current = None  # (stream handle of a device, current device)
+_current = None  # (stream handle of a device, current device), as torch keeps them
 
 
 def stream_ptr(stream=None):

@@ -273,8 +273,8 @@ bool grouped_pays(const b200moe_shape& s, u32 rows, u32 max_union, u32 grouped_m
     return grouped * (rows < kGroupedSureRows ? 107 : 100) < streaming * 100;
 }
 // The other forms of the Q4_K GEMVs: the segment-streaming form (any row length; its items are dealt out dynamically) wherever it applies, else the
-// row-streaming form (a ring of whole rows, its work split fixed per CTA) and the per-block form. The row-streaming form had windows of one and two
-// rows over rows of up to 2048 weights, until the other began its launches with the weights of its first items. Whole calls, row and segment streaming, us: 128
+// row-streaming form (a ring of whole rows, its work split fixed per CTA) and the per-block form. In a call the segment-streaming form has windows of one
+// and two rows too, since it begins its launches with the weights of its first items. Whole calls, row and segment streaming, us: 128
 // experts of 2048 x 768, one row, top 1 to 16, 30.8 and 28.7, 32.9 and 30.8, 36.9 and 34.7 (top 8), 45.1 and 41.2; two rows, top 8, 43.0 and 39.2; 16
 // experts of 512 x 256 28.7 and 26.6; dense 2048 x 2048 23.7 and 17.5, 512 x 512 21.5 and 15.4. B200MOE_DEBUG_DECODE_FORM forces
 // one of the four where it applies, whatever grouped_min_rows says.

@@ -70,10 +70,14 @@ inline bool down_reads_sums(u32 type) { return type == B200MOE_TYPE_Q4_K || type
 // ---- the chain of a call's launches ----------------------------------------------------------------------------------
 // A call is a chain of dependent launches, most of them a few microseconds long. Each is enqueued with programmatic stream
 // serialisation: it is brought onto the SMs while the launch before it still runs and waits there, in chain_begin, until
-// that one has completed and its writes are visible. Every kernel launched so calls chain_begin before it touches global
-// memory, on every path: a launch that has passed it knows that everything enqueued before it is complete, which is also what lets it
-// admit its successor at once. Written data is read by plain loads (load below), never through the read-only path: the kernel
-// runs already while its predecessor writes, and such a load may be moved in front of the wait.
+// that one has completed and its writes are visible. What every kernel launched so keeps to:
+//  * Every CTA waits, on every path, and writes nothing to global memory before. A launch that has passed its wait knows that everything enqueued before it is
+//    complete.
+//  * It admits its successor only behind its own wait (chain_begin does both). So a launch that runs at all knows that what lies in front of the launch in
+//    front is complete; one that admitted first would take that from every early reader behind it.
+//  * Before its wait it reads only what it is told to be older than the launch in front (ChainHints: routes, order, weights, ids, expert tensors), past L1.
+//  * Everything else it reads behind the wait, by plain loads (load below), never through the read-only path: the kernel runs already while its predecessor
+//    writes, and such a load may be moved in front of the wait.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_admit() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin() {

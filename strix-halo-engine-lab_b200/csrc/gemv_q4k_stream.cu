@@ -22,7 +22,8 @@
 // (they still walk their loops, doing no work), the producers drain the copies they have in flight (bounded), bit 30 of the
 // job summary is set and the kernel returns: the host reads a status, the GPU never hangs.
 //
-// Roofline: HBM. Algorithmic bytes per item = 64 rows x K / 256 x 144. Taken where the segment-streaming form (gemv_q4k_wide.cu) does not apply; the figures of both are in api.cu.
+// Roofline: HBM. Algorithmic bytes per item = 64 rows x K / 256 x 144. Taken where the segment-streaming form (gemv_q4k_wide.cu) does not apply, and by stages
+// of one and two rows that are called by themselves; the figures of both are in api.cu.
 
 #include "declared_math.cuh"
 #include "kernels.cuh"

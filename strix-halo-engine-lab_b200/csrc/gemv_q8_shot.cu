@@ -6,8 +6,9 @@
 // four rows each, a lane one of the 32 classes, as in gemv_q8.cu, whose bits these are; the entries' codes are read once for a warp's four rows.
 // What bounds it: latencies. One row over 4 of 64 experts of 2048 -> 1024, top 4 (128 + 128 items): the form with a row a warp had one run a warp on its
 // way (35 KB a multiprocessor) and each warp's four runs one behind the other: gate/up 11.5 us behind its routes, down 9.7 behind gate/up, where these
-// take 8 and 5 (a whole call 33.1 -> 24.9). 8 rows over 256 experts of 2048 -> 768, top 8: 131 us a call, 199 in the tensor-core and token-block forms. Where it pays: csrc/api.cu.
-// An early launch of down (ChainHints) fits on the multiprocessors beside gate/up's CTAs and has its weights before it waits.
+// take 8 and 5 (a whole call 33.1 -> 24.9). Where it pays: csrc/api.cu.
+// An early launch of down (ChainHints) has its first weights before it waits where it fits on the multiprocessors beside gate/up's CTAs: with one entry a pass (62 and
+// 57 registers, 512 threads each) and rows of up to 2048 and 1024 weights (139 and 70 KB); else as those CTAs end.
 #include <algorithm>
 
 #include "declared_math.cuh"

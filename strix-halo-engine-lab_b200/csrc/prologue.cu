@@ -1,5 +1,5 @@
 // Front of a layer call over a decode window (up to 8 rows) in ONE launch: A8 of the activations and the router logits. Selection and routes follow in
-// a launch of one block (routes.cu).
+// a launch of one block (routes.cu), above 256 experts in one each.
 //
 // Contracts are those of the stand-alone kernels (a8.cu, router.cu): logits in the declared lane-strided order without fused multiply-add
 // (src/ds41_moe.cpp:72-82). Bits do not change; bfloat16 activations are widened (exactly) on the way.

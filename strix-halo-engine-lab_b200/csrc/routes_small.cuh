@@ -1,5 +1,5 @@
-// Routes of a decode window (up to 1024 slots, up to 1024 experts) built by ONE block of any size: device code shared by
-// the stand-alone routes kernel (routes.cu) and the fused layer prologue (prologue.cu).
+// Routes of a decode window (up to 1024 slots, up to 1024 experts) built by ONE block of any size, or by one warp: device code shared by
+// the stand-alone routes kernels and the launch that selects too (routes.cu).
 // Contract: strix::ds41::build_window_routes + restrict_routes (src/ds41_moe.cpp:11-61), see routes.cu.
 #pragma once
 #include "common.cuh"

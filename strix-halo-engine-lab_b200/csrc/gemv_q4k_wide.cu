@@ -12,8 +12,8 @@
 //    claim word in device memory (wide_common.cuh).
 //  * A stage = S = 3 super-blocks of the item's 64 rows (one or two tiled TMA copies of 432 bytes x 32 / 64 rows: the rows
 //    lie 432 bytes apart in shared memory, an odd count of 16-byte units, which keeps the 128-bit reads of eight rows
-//    conflict free) PLUS the same K range of the A8 rows of the item's entries (codes, deltas, sums: three bulk copies per
-//    entry, or 16-byte asynchronous copies), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
+//    conflict free) PLUS the same K range of the A8 rows of the item's entries (codes, deltas, sums: gathering copies of four entries' rows each, untiled
+//    copies of an only entry's), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
 //  * Two groups of eight consumer warps share a CTA, each with its own ring of stages and its own producer warp; a group's
 //    producer claims the next item of the grid while its consumers still work on the stages in the ring. The serial chains
 //    acc_p += pair_p never leave their lane.
@@ -59,8 +59,7 @@ struct WidePlan {
     u32 nb;             // super-blocks per row
     u32 nseg;           // stages per item
     u32 stages;         // ring depth per group
-    u32 w_bytes;        // 64 * S * 144
-    u32 x_entry_bytes;  // >= S * 320: codes, deltas, sums of one entry over the stage's K range (+ padding)
+    u32 cap;            // entries that a stage holds: 1, 4 or 8
     u32 stage_bytes;
     u32 n_chunks;       // items per (virtual) expert
     u32 max_union;      // bound of the union
@@ -86,21 +85,29 @@ struct WideArgs {
     u32 raw_vec;           // raw lies on an 8-byte boundary
 };
 
-// Stage geometry for S super-blocks per stage, as compile-time constants: address
-// arithmetic on run-time strides was a measurable part of the instructions. Weight rows lie S * 144 bytes apart, S odd: an odd multiple of 4 (mod 32) words, so a
-// warp's 128-bit reads of 8 rows and its fragments' word reads are conflict free.
-constexpr u32 x_entry_bytes_of(u32 S) {  // codes, deltas, sums of one entry over a stage, padded so that entries lie an odd multiple of
-    u32 b = S * 320u;                     // 4 (mod 32) words apart: the fragments' word reads of eight entries meet every bank once
-    while ((b / 4) % 8 != 4) b += 16;
-    return b;
-}
-template <u32 S_>
+struct WideMaps { CUtensorMap w0, w1, codes, deltas, sums; };  // weight rows (up: w1), the entries' A8 rows
+
+// Stage geometry for S super-blocks per stage and CAP entries (1, 4 or 8), as compile-time constants: address arithmetic on run-time strides was a measurable
+// part of the instructions. Weight rows lie S * 144 bytes apart, S odd: an odd multiple of 4 (mod 32) words, so a warp's 128-bit reads of 8 rows and its
+// fragments' word reads are conflict free. The entries' A8 rows come in fours by gathering copies: the codes in two halves of the stage's columns (boxes that are
+// no wider than the shortest row: wider ones fault), the deltas, the sums. The codes' boxes hold 32 bytes more than the half, and the second four's begin 16 bytes
+// further to the left: eight entries' codes lie 4 (mod 32) words apart, so that a fragment's word reads meet every bank once.
+template <u32 S_, u32 CAP_>
 struct Geo {
-    static constexpr u32 S = S_;
+    static constexpr u32 S = S_, CAP = CAP_, fours = CAP == 8 ? 2u : 1u;
     static constexpr u32 row_bytes = S * kQ4KBlock, half_bytes = kHalfRows * row_bytes;
     static constexpr u32 w_bytes = 2 * half_bytes;
-    static constexpr u32 x_entry_bytes = x_entry_bytes_of(S);
+    static constexpr u32 half_cols = S * 128, box_codes = half_cols + 32, box_group = S * 32;  // bytes of a box's rows
+    static constexpr u32 half_codes = 4 * box_codes, four_codes = 2 * half_codes, four_group = 4 * box_group;
+    static constexpr u32 off_deltas = CAP == 1 ? S * 256u : fours * four_codes, off_sums = off_deltas + (CAP == 1 ? box_group : fours * four_group);
+    static constexpr u32 x_bytes = off_sums + (CAP == 1 ? box_group : fours * four_group);
+    static constexpr u32 stage_bytes = (w_bytes + x_bytes + 127u) / 128u * 128u;
+    static constexpr u32 four_tx = four_codes + 2 * four_group;  // bytes of a four's copies
+    __device__ static constexpr u32 codes_at(u32 e) { return (e & 3u) * box_codes + (e & 4u ? four_codes + 16u : 0u); }
+    __device__ static constexpr u32 column(u32 c) { return c + (c >= half_cols ? half_codes - half_cols : 0u); }  // behind codes_at
 };
+static_assert(Geo<3, 8>::half_codes % 128 == 0 && Geo<1, 8>::half_codes % 128 == 0 && Geo<3, 8>::four_group % 128 == 0 && Geo<1, 8>::four_group % 128 == 0 &&
+              Geo<3, 8>::w_bytes % 128 == 0 && Geo<1, 8>::w_bytes % 128 == 0, "a tiled copy lands on 128 bytes");
 
 // (a0 + a1) + (a2 + a3) over the four pair lanes of a row (lane = 8 * p + row); every lane of the row gets the value.
 __device__ __forceinline__ float tree4(float a) {
@@ -111,16 +118,19 @@ __device__ __forceinline__ float tree4(float a) {
 // Decoded factors of one super-block for pair p as the chains use them: D of the even group, D / 16 of the odd one (the high nibbles stay in
 // place: their dots come as 16 * dot), and -DM of both. A scale's byte goes behind the exponent of 2^23, less 2^23.
 __device__ __forceinline__ float4 pair_factors(const uint4& hdr, u32 p) {
-    const float d = half_bits_to_float(hdr.x & 0xffffu), dm = -half_bits_to_float(hdr.x >> 16);
-    const u32 sc = p < 2u ? hdr.y & 0x3f3f3f3fu : (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
-    const u32 mn = p < 2u ? hdr.z & 0x3f3f3f3fu : ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
+    const float d = half_bits_to_float(hdr.x & 0xffffu), dm = half_bits_to_float(hdr.x >> 16);
     const u32 sel = 0x7440u + 2u * (p & 1u);
-    auto byte = [](u32 w, u32 s) { return __fsub_rn(__uint_as_float(__byte_perm(w, 0x4b000000u, s)), 8388608.0f); };
-    return make_float4(__fmul_rn(d, byte(sc, sel)), __fmul_rn(__fmul_rn(d, 0.0625f), byte(sc, sel + 1u)), __fmul_rn(dm, byte(mn, sel)), __fmul_rn(dm, byte(mn, sel + 1u)));
+    u32 sc, mn;
+    if (p < 2u) { sc = hdr.y & 0x3f3f3f3fu; mn = hdr.z & 0x3f3f3f3fu; }
+    else { sc = (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u); mn = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u); }
+    auto two = [&](u32 w, u32 base) { return make_float2(__uint_as_float(__byte_perm(w, base, sel)), __uint_as_float(__byte_perm(w, base, sel + 1u))); };
+    const float2 D = mul2(make_float2(d, __fmul_rn(d, 0.0625f)), add2(two(sc, 0x4b000000u), both(-8388608.0f)));
+    const float2 M = mul2(both(dm), add2(two(mn, 0xcb000000u), both(8388608.0f)));
+    return make_float4(D.x, D.y, M.x, M.y);
 }
 
 // One stage of one weight row (this lane's pair p of nbk super-blocks, ascending) against one staged A8 row. blk: the row's first
-// super-block of the stage; xs: the entry's area of the stage {codes[S * 256], deltas[S * 8], sums[S * 8]}.
+// super-block of the stage; xs: the stage's A8 rows, of which the first is meant.
 template <class G>
 __device__ __forceinline__ void stage_row(const unsigned char* blk, u32 nbk, u32 p, const unsigned char* xs, float& acc) {
     constexpr u32 S = G::S;
@@ -133,8 +143,8 @@ __device__ __forceinline__ void stage_row(const unsigned char* blk, u32 nbk, u32
         const Nibbles n = split_nibbles(q0, q1);
         const uint4* c = reinterpret_cast<const uint4*>(xs + 256u * b + 64u * p);
         const uint4 c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
-        const float2 e = *reinterpret_cast<const float2*>(xs + 256u * S + 32u * b + 8u * p);
-        const float2 sm = to_float(*reinterpret_cast<const int2*>(xs + 288u * S + 32u * b + 8u * p));
+        const float2 e = *reinterpret_cast<const float2*>(xs + G::off_deltas + 32u * b + 8u * p);
+        const float2 sm = to_float(*reinterpret_cast<const int2*>(xs + G::off_sums + 32u * b + 8u * p));
         int l, h;
         dots(n, c0, c1, c2, c3, &l, &h);
         // x = E * ((D * float(dot)) - (DM * S)) for the pair's two groups; f holds -DM, and (-DM) * S = -(DM * S) exactly
@@ -151,6 +161,8 @@ __device__ __forceinline__ void mma_u8s8(int (&d)[4], const u32 (&a)[4], u32 mas
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
         : "r"(a[0] & mask), "r"(a[1] & mask), "r"(a[2] & mask), "r"(a[3] & mask), "r"(b0), "r"(b1), "r"(0));
 }
+// The entry of MMA column c where the columns hold eight: a lane's two cells are entries t and t + 4, so that four lanes' reads of deltas and sums meet every bank once.
+__device__ __forceinline__ u32 entry_of(u32 c) { return (c >> 1) + 4u * (c & 1u); }
 // One stage of the warp's 32 weight rows and chain (pair p) against up to 8 staged A8 rows with tensor-core dots. blk: the half's first row and super-block
 // of the stage; fac: the warp's scratch, S x kFacFloats. acc[j][e]: the chain of rows 16 j + lane / 4 and the row 8 further with entry 2 (lane % 4) + e; these two rows
 // share every packed instruction. MANY: items of five entries or more. Else the eight columns hold the entries twice, and of a lane's cells the first
@@ -161,7 +173,7 @@ __device__ __forceinline__ void mma_u8s8(int (&d)[4], const u32 (&a)[4], u32 mas
 // where the form before took 88; dp4a takes 32 for one entry and 20 more for every further one.
 template <bool MANY, class G>
 __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk, u32 p, u32 lane, const unsigned char* xs, float* fac, float2 (&acc)[MANY ? 2 : 1][2]) {
-    constexpr u32 x_entry_bytes = G::x_entry_bytes, S = G::S;
+    constexpr u32 S = G::S;
     const u32 g = lane >> 2, t = lane & 3u;
     {   // the factors, lane = row: rows i and i + 8 of a tile meet by a shuffle, so that a row pair lies in natural register pairs
         const bool high = lane & 8u;
@@ -177,24 +189,25 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk
         __syncwarp();
     }
     const unsigned char* rows = blk + g * G::row_bytes + 16u + 32u * p + 4u * t;
-    const unsigned char* codes = xs + (MANY ? g : g & 3u) * x_entry_bytes + 64u * p + 4u * t;
-    const unsigned char* es = xs + 2u * (MANY ? t : t & 1u) * x_entry_bytes + 256u * S + 8u * p;
+    const unsigned char* codes = xs + G::codes_at(MANY ? entry_of(g) : g & 3u) + 4u * t;
+    const unsigned char* es = xs + G::off_deltas + (MANY ? t : 2u * (t & 1u)) * G::box_group + 8u * p;
     const float4* get = reinterpret_cast<const float4*>(fac) + g;
     const bool second = t >= 2u;  // of the few form
 #pragma unroll
     for (u32 b = 0; b < nbk; ++b) {
+        const unsigned char* cb = codes + G::column(256u * b + 64u * p);
         u32 a[2][4], bl[2], bh[2];
 #pragma unroll
         for (u32 j = 0; j < 2; ++j)
 #pragma unroll
             for (u32 i = 0; i < 4; ++i) a[j][i] = *reinterpret_cast<const u32*>(rows + (16u * j + 8u * (i & 1u)) * G::row_bytes + 16u * (i >> 1));
 #pragma unroll
-        for (u32 i = 0; i < 2; ++i) { bl[i] = *reinterpret_cast<const u32*>(codes + 16u * i); bh[i] = *reinterpret_cast<const u32*>(codes + 32u + 16u * i); }
+        for (u32 i = 0; i < 2; ++i) { bl[i] = *reinterpret_cast<const u32*>(cb + 16u * i); bh[i] = *reinterpret_cast<const u32*>(cb + 32u + 16u * i); }
         float2 E[2], Sg[2];
 #pragma unroll
         for (u32 e = 0; e < 2; ++e) {
-            E[e] = *reinterpret_cast<const float2*>(es + e * x_entry_bytes);
-            Sg[e] = to_float(*reinterpret_cast<const int2*>(es + e * x_entry_bytes + 32u * S));
+            E[e] = *reinterpret_cast<const float2*>(es + (MANY ? 4u : 1u) * e * G::box_group);
+            Sg[e] = to_float(*reinterpret_cast<const int2*>(es + (MANY ? 4u : 1u) * e * G::box_group + (G::off_sums - G::off_deltas)));
         }
         int l[2][4], h[2][4];
 #pragma unroll
@@ -218,19 +231,19 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk
                 acc[j][e] = add2(add2(mul2(both(E[e].x), sl), mul2(both(E[e].y), sh)), acc[j][e]);
             }
         }
-        rows += kQ4KBlock; codes += 256; es += 32; get += kFacFloats / 4;
+        rows += kQ4KBlock; es += 32; get += kFacFloats / 4;
     }
 }
 
 // 18 warps: two of the SM's four register partitions (16 K registers each) hold five warps, which caps a thread at
 // 16384 / (5 x 32) = 102 registers, 96 after rounding - what this launch bound gives (112 was tried: the launch is refused).
-// ASYNC: how the entries' A8 rows come in. A bulk copy holds the producer for about 180 clocks, 24 of them a stage for eight entries; asynchronous copies cost
-// instructions that a stage of few entries does not repay. Bulk and asynchronous, us a call: dense 5120 x 17408, 8 rows 77.8 and 74.8, 16 rows 112.5 and
-// 109.7, 5 rows 70.8 and 72.7, 1 row 43.9 and 50. A choice per item inside one kernel costs the items of one entry 1.5 us of these 43.9.
-template <bool DOWN, u32 S_, bool ASYNC>
+// The entries' A8 rows by gathering copies: to ask for a stage's 24 bulk copies (8 entries) took a producer 1,690 clocks on its own and 1,880 beside the consumers,
+// whose work on the stage is 2,030 (64 rows of the large layer); a gathering copy of four rows 83. In a graph, us a call: large layer of 64 rows 720 -> 681, dense 5120 x 17408
+// 42.4 -> 39.6 (1 row) and 65.7 -> 61.8 (8).
+template <bool DOWN, u32 S_, u32 CAP_>
 __global__ void __launch_bounds__(kThreads, 1)
-q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, WideArgs a, WidePlan plan) {
-    using G = Geo<S_>;
+q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan) {
+    using G = Geo<S_, CAP_>;
     extern __shared__ __align__(128) unsigned char smem[];
     // An early launch makes its list and asks for the weights of its groups' first items before it waits for the launch in front. Every path waits.
     const bool early = plan.early;
@@ -278,32 +291,14 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         u64* g_empty = empty + g * plan.stages;
         u32* g_item = slot_item + g * plan.stages;
         unsigned char* g_stage = smem + g * plan.stages * plan.stage_bytes;
-        const u32 e = lane / 3u, part = lane - 3u * e;  // bulk copies: lanes 0 .. 3 * ne - 1 copy one piece of one entry each
         const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, in_gs = in_stride / 32;
         u32 t = 0, slot = 0, use = 0;  // stage count, ring position, lap
         bool ok = true, first = true;
-        // ASYNC: 16-byte asynchronous copies, 20 units a super-block and entry {16 of codes, 2 of deltas, 2 of sums}; a lane takes units `lane` and `lane` + 32 of every entry.
-        auto copy_entries = [&](u32 s, u32 nbk, u32 ne, u32 my_row, unsigned char* xd) {
-#pragma unroll
-            for (u32 half = 0; half < (20u * G::S + 31u) / 32u; ++half) {
-                const u32 u = lane + 32u * half;
-                const bool is_codes = u < 16u * nbk, is_deltas = u < 18u * nbk;
-                const unsigned char* base = is_codes ? reinterpret_cast<const unsigned char*>(a.in.codes) + s * G::S * 256u + 16u * u
-                                          : is_deltas ? reinterpret_cast<const unsigned char*>(a.in.deltas) + s * G::S * 32u + 16u * (u - 16u * nbk)
-                                                      : reinterpret_cast<const unsigned char*>(a.in.sums) + s * G::S * 32u + 16u * (u - 18u * nbk);
-                const u32 pitch = is_codes ? in_stride : in_stride / 8u;  // bytes between rows
-                unsigned char* to = xd + (is_codes ? 16u * u : is_deltas ? 256u * G::S + 16u * (u - 16u * nbk) : 288u * G::S + 16u * (u - 18u * nbk));
-                for (u32 e = 0; e < ne; ++e) {
-                    const u32 row = __shfl_sync(0xffffffffu, my_row, e);
-                    if (u < 20u * nbk) cp_async16(to + e * G::x_entry_bytes, base + u64(row) * pitch);
-                }
-            }
-        };
         auto ask_weights = [&](u32 s, const VExpert& ve, u32 chunk, unsigned char* dst, u64* bar) {  // one lane
             const u32 x = s * G::S * (kQ4KBlock / 8);  // 64-bit elements: a multiple of 18, i.e. of 144 bytes
             const u32 y = ve.expert() * a.rows_per_expert + (DOWN ? kItemRows : kHalfRows) * chunk;
-            tma_2d(dst, &tm0, x, y, bar);
-            tma_2d(dst + G::half_bytes, &tm1, x, DOWN ? y + kHalfRows : y, bar);
+            tma_2d(dst, &maps.w0, x, y, bar);
+            tma_2d(dst + G::half_bytes, &maps.w1, x, DOWN ? y + kHalfRows : y, bar);
         };
         u32 ahead = 0;  // stages of the first item whose weights were asked for before the wait
         if (early) {
@@ -350,9 +345,13 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 ve = table[jv];
             }
             const u32 ve_ne = ve.ne();
-            const u32 mine = ASYNC ? lane : e;  // the entry whose row the lane reads
-            u32 r = 0;
-            if (mine < ve_ne) r = plan.dense_rows ? ve.begin() + mine : load((DOWN ? a.routes.slots : a.routes.rows) + ve.begin() + mine);
+            u32 r[8];  // the entries' A8 rows; in absent places the first one's
+            {
+                u32 mine = 0;
+                if (lane < 8u && !end) { const u32 at = ve.begin() + (lane < ve_ne ? lane : 0u); mine = plan.dense_rows ? at : load((DOWN ? a.routes.slots : a.routes.rows) + at); }
+#pragma unroll
+                for (u32 i = 0; i < 8; ++i) r[i] = i < G::CAP ? __shfl_sync(0xffffffffu, mine, i) : 0u;
+            }
             const u32 nsegs = end ? 1u : plan.nseg;
             for (u32 s = 0; s < nsegs; ++s, ++t, ++slot) {
                 if (slot == plan.stages) { slot = 0; ++use; }
@@ -369,27 +368,32 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 unsigned char* dst = g_stage + slot * plan.stage_bytes;
                 if (lane == 0) {
                     g_item[slot] = item;
-                    const u32 w_bytes = t < ahead ? 0u : G::w_bytes;  // whole boxes: what lies past the row is filled
-                    if (ASYNC) mbar_expect_more(&g_full[slot], w_bytes);
-                    else mbar_expect_tx(&g_full[slot], w_bytes + ve_ne * nbk * 320u);
+                    const bool one = G::CAP == 1 || ve_ne == 1u;  // one entry's rows: untiled copies of what the stage has of them
+                    const bool both_halves = nbk * 256u > G::half_cols;
+                    const u32 four_tx = G::four_tx - (both_halves ? 0u : G::half_codes);
+                    mbar_expect_tx(&g_full[slot], (t < ahead ? 0u : G::w_bytes) + (one ? nbk * 320u : ve_ne > 4u ? 2u * four_tx : four_tx));  // whole boxes: what lies past a row is filled
+                    if (t >= ahead) ask_weights(s, ve, chunk, dst, &g_full[slot]);
+                    unsigned char* xd = dst + G::w_bytes;
+                    if (one) {
+                        bulk_g2s(xd, a.in.codes + u64(r[0]) * in_stride + u64(s) * G::S * 256u, nbk * 256u, &g_full[slot]);
+                        bulk_g2s(xd + G::off_deltas, a.in.deltas + u64(r[0]) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
+                        bulk_g2s(xd + G::off_sums, a.in.sums + u64(r[0]) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
+                    } else {
+                        auto ask_four = [&](unsigned char* codes, unsigned char* group, int left, u32 r0, u32 r1, u32 r2, u32 r3) {  // columns in 64-bit elements
+                            const int xc = static_cast<int>(s * (G::S * 32u)) - left, xg = static_cast<int>(s * (G::S * 4u));
+                            gather_4(codes, &maps.codes, xc, r0, r1, r2, r3, &g_full[slot]);
+                            if (both_halves) gather_4(codes + G::half_codes, &maps.codes, xc + static_cast<int>(G::half_cols / 8u), r0, r1, r2, r3, &g_full[slot]);
+                            gather_4(group, &maps.deltas, xg, r0, r1, r2, r3, &g_full[slot]);
+                            gather_4(group + (G::off_sums - G::off_deltas), &maps.sums, xg, r0, r1, r2, r3, &g_full[slot]);
+                        };
+                        ask_four(xd, xd + G::off_deltas, 0, r[0], r[1], r[2], r[3]);
+                        if (G::CAP == 8 && ve_ne > 4u) ask_four(xd + G::four_codes, xd + G::off_deltas + G::four_group, 2, r[4], r[5], r[6], r[7]);  // see Geo
+                    }
                 }
                 __syncwarp();
-                if (lane == 0 && t >= ahead) ask_weights(s, ve, chunk, dst, &g_full[slot]);
-                if (ASYNC) {  // the arrival that lets the stage complete comes behind the lanes' copies, each of which adds one of its own while it is under way
-                    copy_entries(s, nbk, ve_ne, r, dst + G::w_bytes);
-                    asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(saddr(&g_full[slot])) : "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&g_full[slot]);
-                } else if (e < ve_ne) {
-                    unsigned char* xd = dst + G::w_bytes + e * G::x_entry_bytes;
-                    if (part == 0) bulk_g2s(xd, a.in.codes + u64(r) * in_stride + u64(s) * G::S * 256u, nbk * 256u, &g_full[slot]);
-                    else if (part == 1) bulk_g2s(xd + 256u * G::S, a.in.deltas + u64(r) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
-                    else bulk_g2s(xd + 288u * G::S, a.in.sums + u64(r) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
-                }
             }
             if (!ok || end) break;
         }
-        if (ASYNC) asm volatile("cp.async.wait_all;" ::: "memory");
         if (!ok && lane == 0) {  // wait (bounded) for the copies still in flight before the CTA retires
             for (u32 n = t > plan.stages ? t - plan.stages : 0u; n < t; ++n)
                 for (u32 i = 0; i < (plan.wait_limit >> 4) + 64u; ++i)
@@ -426,7 +430,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         const u32 jv = item / plan.n_chunks, chunk = item - jv * plan.n_chunks;
         const VExpert ve = table[jv];
         const u32 ne = ve.ne(), vbegin = ve.begin();
-        const bool mma = ne > kDpEntries;
+        const bool mma = G::CAP > 1 && ne > kDpEntries;
         const u32 slot_id = w >= ne ? 0u : plan.dense_rows ? vbegin + w : load(a.routes.slots + vbegin + w);  // asked for before the stages, used behind them
         // the item's stages, with the form fixed at compile time inside the loop
         auto stages = [&](auto step) {
@@ -466,7 +470,7 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 for (u32 j = 0; j < (MANY ? 2u : 1u); ++j)
 #pragma unroll
                     for (u32 e = 0; e < 2; ++e) {
-                        const u32 tile = MANY ? j : mt >> 1, entry = 2u * (MANY ? mt : mt & 1u) + e;
+                        const u32 tile = MANY ? j : mt >> 1, entry = MANY ? mt + 4u * e : 2u * (mt & 1u) + e;
                         float* to = meet + ((2u * mp + half) * kKE + entry) * kMeetPitch + 16u * tile + me;
                         to[0] = acc[j][e].x;
                         to[8] = acc[j][e].y;
@@ -484,10 +488,10 @@ q4k_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 continue;
             }
             hand_over([&]() { if (p == 0) meet[half * kKE * kMeetPitch + 8u * mp + rr] = val; });
-        } else if (ne > kFewEntries) {
-            run_mma(std::true_type{});
+        } else if (G::CAP > kFewEntries && ne > kFewEntries) {
+            if constexpr (G::CAP > kFewEntries) run_mma(std::true_type{});
         } else {
-            run_mma(std::false_type{});
+            if constexpr (G::CAP > 1) run_mma(std::false_type{});
         }
         if (!ok) break;
         if (w < ne) {
@@ -549,11 +553,11 @@ bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, WidePlan* p) {
     p->nb = K / 256;
     p->S = p->nb >= 3 ? 3u : 1u;  // odd: see Geo
     p->nseg = (p->nb + p->S - 1) / p->S;
-    p->w_bytes = kItemRows * p->S * kQ4KBlock;
-    p->x_entry_bytes = x_entry_bytes_of(p->S);
     // a stage holds the A8 segments of as many entries as a virtual expert of this window can have: windows of fewer than
     // kKE slots get smaller stages and with them a deeper ring
-    p->stage_bytes = round_up(p->w_bytes + static_cast<u32>(std::min<u64>(kKE, slots)) * p->x_entry_bytes, 128);
+    p->cap = slots == 1 ? 1u : slots <= 4 ? 4u : 8u;
+    p->stage_bytes = p->S == 3 ? (p->cap == 1 ? Geo<3, 1>::stage_bytes : p->cap == 4 ? Geo<3, 4>::stage_bytes : Geo<3, 8>::stage_bytes)
+                               : (p->cap == 1 ? Geo<1, 1>::stage_bytes : p->cap == 4 ? Geo<1, 4>::stage_bytes : Geo<1, 8>::stage_bytes);
     p->n_chunks = n_chunks;
     p->max_union = max_union;
     p->vmax = max_union + static_cast<u32>(slots / kKE) + 1;
@@ -573,8 +577,26 @@ bool a8_bulk_ok(const b200moe_a8_rows& x) {
     return x.sums && aligned(x.codes, 16) && aligned(x.deltas, 16) && aligned(x.sums, 16) && stride % 128 == 0;
 }
 
-// Windows whose experts have kKE entries or more on average: their A8 rows come in by asynchronous copies (the figures are with the kernel).
-bool whole_items(u32 max_union, u64 slots) { return slots >= u64(kKE) * max_union; }
+// The tensor maps of the entries' A8 rows for copies of four rows at a time (unused where a stage holds one entry). Rows beyond the window's are not named by its
+// routes; a window has 8192 slots at most (make_plan), and the maps reach that far whatever its rows, so that a buffer keeps its maps.
+int entry_maps(const b200moe_a8_rows& x, u32 K, const WidePlan& p, WideMaps* m) {
+    m->codes = m->deltas = m->sums = m->w0;
+    if (p.cap == 1) return B200MOE_OK;
+    const u64 pitch = x.stride ? x.stride : x.width;
+    const u32 codes = p.S * 128u + 32u, group = p.S * 32u;  // Geo::box_codes, box_group: no wider than a row of S super-blocks
+    if (int rc = pitched_map(reinterpret_cast<const u8*>(x.codes), K, pitch, 8192, codes, 1, &m->codes)) return rc;
+    if (int rc = pitched_map(reinterpret_cast<const u8*>(x.deltas), K / 8, pitch / 8, 8192, group, 1, &m->deltas)) return rc;
+    return pitched_map(reinterpret_cast<const u8*>(x.sums), K / 8, pitch / 8, 8192, group, 1, &m->sums);
+}
+template <bool DOWN>
+int launch_wide(const WideMaps& m, const WideArgs& a, const WidePlan& p, cudaStream_t stream) {
+    const auto kernel = p.S == 3 ? (p.cap == 1 ? q4k_wide_kernel<DOWN, 3, 1> : p.cap == 4 ? q4k_wide_kernel<DOWN, 3, 4> : q4k_wide_kernel<DOWN, 3, 8>)
+                                 : (p.cap == 1 ? q4k_wide_kernel<DOWN, 1, 1> : p.cap == 4 ? q4k_wide_kernel<DOWN, 1, 4> : q4k_wide_kernel<DOWN, 1, 8>);
+    const u32 smem = plan_smem(p);
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
+    chain_launch(kernel, device_sm_count(), kThreads, smem, stream, m, a, p);
+    return after_launch(DOWN ? "down_q4k_wide" : "gate_up_q4k_wide");
+}
 
 void apply_hooks(WidePlan* p) {
     const u32 limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT), stall = debug_value(B200MOE_DEBUG_STALL_STAGE);
@@ -605,15 +627,12 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const Chain
     WideArgs a{};
     a.routes = v.routes; a.in = v.x; a.act = v.act; a.gate_out = v.gate_out; a.up_out = v.up_out;
     a.row_status = v.row_status; a.summary = v.summary; a.rows_per_expert = v.shape.inter; a.out_width = v.shape.inter;
-    CUtensorMap tm0, tm1;
+    WideMaps m;
     const u64 rb = u64(p.nb) * kQ4KBlock, total_rows = u64(v.shape.experts) * v.shape.inter;
-    if (int rc = rows_map(v.weights.gate, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &tm0)) return rc;
-    if (int rc = rows_map(v.weights.up, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &tm1)) return rc;
-    const u32 smem = plan_smem(p);
-    const auto kernel = p.S != 3 ? q4k_wide_kernel<false, 1, false> : whole_items(v.max_union, u64(rows) * v.shape.top_k) ? q4k_wide_kernel<false, 3, true> : q4k_wide_kernel<false, 3, false>;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-    chain_launch(kernel, device_sm_count(), kThreads, smem, stream, tm0, tm1, a, p);
-    return after_launch("gate_up_q4k_wide");
+    if (int rc = rows_map(v.weights.gate, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &m.w0)) return rc;
+    if (int rc = rows_map(v.weights.up, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &m.w1)) return rc;
+    if (int rc = entry_maps(v.x, v.shape.hidden, p, &m)) return rc;
+    return launch_wide<false>(m, a, p, stream);
 }
 
 int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream) {
@@ -626,13 +645,12 @@ int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints&
     WideArgs a{};
     a.routes = v.routes; a.in = v.act; a.raw = v.raw; a.summary = const_cast<u32*>(v.summary);
     a.rows_per_expert = v.shape.hidden; a.out_width = v.shape.hidden; a.raw_vec = aligned(v.raw, 8);
-    CUtensorMap tm0;
-    if (int rc = rows_map(v.weights.down, u64(p.nb) * kQ4KBlock, u64(v.shape.experts) * v.shape.hidden, p.S * kQ4KBlock, kHalfRows, &tm0)) return rc;
-    const u32 smem = plan_smem(p);
-    const auto kernel = p.S != 3 ? q4k_wide_kernel<true, 1, false> : whole_items(v.max_union, u64(rows) * v.shape.top_k) ? q4k_wide_kernel<true, 3, true> : q4k_wide_kernel<true, 3, false>;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-    chain_launch(kernel, device_sm_count(), kThreads, smem, stream, tm0, tm0, a, p);
-    return after_launch("down_q4k_wide");
+    WideMaps m;
+    const u64 rb = u64(p.nb) * kQ4KBlock;
+    if (int rc = rows_map(v.weights.down, rb, u64(v.shape.experts) * v.shape.hidden, p.S * kQ4KBlock, kHalfRows, &m.w0)) return rc;
+    m.w1 = m.w0;
+    if (int rc = entry_maps(v.act, v.shape.inter, p, &m)) return rc;
+    return launch_wide<true>(m, a, p, stream);
 }
 
 }  // namespace b200moe

@@ -114,11 +114,11 @@ __device__ __forceinline__ void build_dense_list(u32 rows, u32 n_chunks, VExpert
     __syncthreads();
 }
 
-// Tensor map of a [rows][row_bytes] tensor seen as 64-bit elements, boxes of box_bytes (a multiple of 16) x box_rows rows,
+// Tensor map of a tensor of rows of row_bytes, `pitch` bytes apart, seen as 64-bit elements, boxes of box_bytes (a multiple of 16) x box_rows rows,
 // no swizzle. The encoder is the driver's cuTensorMapEncodeTiled, looked up through the runtime (no link against
 // the driver library). Encoded maps are kept per (device, tensor, geometry): encoding is host work of a few microseconds
 // that a decode step would otherwise pay on every call.
-inline int rows_map(const u8* base, u64 row_bytes, u64 rows, u32 box_bytes, u32 box_rows, CUtensorMap* out) {
+inline int pitched_map(const u8* base, u64 row_bytes, u64 pitch, u64 rows, u32 box_bytes, u32 box_rows, CUtensorMap* out) {
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static EncodeFn fn = [] {
@@ -129,15 +129,15 @@ inline int rows_map(const u8* base, u64 row_bytes, u64 rows, u32 box_bytes, u32 
     }();
     if (!fn) return fail(B200MOE_ERR_CUDA, "streaming form: cuTensorMapEncodeTiled is not available from this driver");
     static std::mutex m;
-    static std::map<std::tuple<int, const u8*, u64, u64, u32, u32>, CUtensorMap> cache;
+    static std::map<std::tuple<int, const u8*, u64, u64, u64, u32, u32>, CUtensorMap> cache;
     int dev = 0;
     cudaGetDevice(&dev);
-    const auto key = std::make_tuple(dev, base, row_bytes, rows, box_bytes, box_rows);
+    const auto key = std::make_tuple(dev, base, row_bytes, pitch, rows, box_bytes, box_rows);
     std::lock_guard<std::mutex> lock(m);
     const auto it = cache.find(key);
     if (it != cache.end()) { *out = it->second; return B200MOE_OK; }
     const cuuint64_t dims[2] = {row_bytes / 8, rows};
-    const cuuint64_t strides[1] = {row_bytes};  // bytes between rows: a multiple of 16 (144 per super-block)
+    const cuuint64_t strides[1] = {pitch};  // bytes between rows: a multiple of 16 (144 per super-block)
     const cuuint32_t box[2] = {box_bytes / 8, box_rows};
     const cuuint32_t elem[2] = {1, 1};
     const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<u8*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -146,6 +146,10 @@ inline int rows_map(const u8* base, u64 row_bytes, u64 rows, u32 box_bytes, u32 
     if (cache.size() >= 1024) cache.clear();
     cache.emplace(key, *out);
     return B200MOE_OK;
+}
+// Rows that lie one behind the other: weights.
+inline int rows_map(const u8* base, u64 row_bytes, u64 rows, u32 box_bytes, u32 box_rows, CUtensorMap* out) {
+    return pitched_map(base, row_bytes, row_bytes, rows, box_bytes, box_rows, out);
 }
 
 

@@ -20,8 +20,8 @@
 //  * Two forms of the integer dots, chosen per item by its entry count. One entry: dp4a, lane = (pair p, one of the warp's 8 rows); (a0 + a1) +
 //    (a2 + a3) is two xor-shuffles at the end of the item. From two entries: mma.sync.m16n8k32 (A = nibbles of 16 rows as unsigned bytes, the high ones
 //    left in place as 16 q; B = the codes of up to 8 entries, signed), a warp 32 rows of ONE chain; the four chains meet in shared memory at the end of
-//    the item. With up to 4 entries the eight columns hold them twice, and a lane works for one of the two row tiles only. The row pair of a lane's
-//    cells shares every packed FP32 instruction; both forms produce the contract's bits.
+//    the item. With up to 4 entries the eight columns hold them twice, and a lane works for one of the two row tiles only. The pair's two groups
+//    of a cell share every packed FP32 instruction; both forms produce the contract's bits.
 //  * gate/up: the group meets on an mbarrier once per item and a warp an entry runs SwiGLU + the A8 rule; down: a warp an entry stores the sums.
 // What bounds it: the latency of dependent instructions with four consumer warps a scheduler (64 rows over 64 experts of 7168 -> 2048: 62 % of the issue
 // slots, 67 % of the shared memory's cycles, 49 % of the DRAM's). A warp with 8 rows of four chains, whose factors met 8 rows and which took the tensor cores from
@@ -129,6 +129,18 @@ __device__ __forceinline__ float4 pair_factors(const uint4& hdr, u32 p) {
     return make_float4(D.x, D.y, M.x, M.y);
 }
 
+__device__ __forceinline__ u32 lds32(u32 a) { u32 v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ uint2 lds64(u32 a) { uint2 v; asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a)); return v; }
+__device__ __forceinline__ uint4 lds128(u32 a) { uint4 v; asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a)); return v; }
+__device__ __forceinline__ void sts128(u32 a, const float4& v) { asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory"); }
+// The pair's term of one row and entry: x = E * ((D * float(dot)) - (DM * S)) of its two groups, which share the packed instructions, added. f holds -DM, and
+// (-DM) * S = -(DM * S) exactly. The groups, and not two rows or entries, because all operands then lie in natural register pairs: rows paired, whose entry factors
+// had to be doubled by moves, took 197 instructions a super-block of 32 rows x 8 entries.
+__device__ __forceinline__ float pair_term(const float4& f, int2 dot, float2 E, float2 S) {
+    const float2 x = mul2(E, add2(mul2(make_float2(f.x, f.y), to_float(dot)), mul2(make_float2(f.z, f.w), S)));
+    return __fadd_rn(x.x, x.y);
+}
+
 // One stage of one weight row (this lane's pair p of nbk super-blocks, ascending) against one staged A8 row. blk: the row's first
 // super-block of the stage; xs: the stage's A8 rows, of which the first is meant.
 template <class G>
@@ -147,10 +159,7 @@ __device__ __forceinline__ void stage_row(const unsigned char* blk, u32 nbk, u32
         const float2 sm = to_float(*reinterpret_cast<const int2*>(xs + G::off_sums + 32u * b + 8u * p));
         int l, h;
         dots(n, c0, c1, c2, c3, &l, &h);
-        // x = E * ((D * float(dot)) - (DM * S)) for the pair's two groups; f holds -DM, and (-DM) * S = -(DM * S) exactly
-        const float sl = __fadd_rn(__fmul_rn(f.x, static_cast<float>(l)), __fmul_rn(f.z, sm.x));
-        const float sh = __fadd_rn(__fmul_rn(f.y, static_cast<float>(h)), __fmul_rn(f.w, sm.y));
-        acc = __fadd_rn(acc, __fadd_rn(__fmul_rn(e.x, sl), __fmul_rn(e.y, sh)));
+        acc = __fadd_rn(acc, pair_term(f, make_int2(l, h), e, sm));
     }
 }
 // ---- the mma form of one stage ---------------------------------------------------------------------------------------
@@ -164,50 +173,49 @@ __device__ __forceinline__ void mma_u8s8(int (&d)[4], const u32 (&a)[4], u32 mas
 // The entry of MMA column c where the columns hold eight: a lane's two cells are entries t and t + 4, so that four lanes' reads of deltas and sums meet every bank once.
 __device__ __forceinline__ u32 entry_of(u32 c) { return (c >> 1) + 4u * (c & 1u); }
 // One stage of the warp's 32 weight rows and chain (pair p) against up to 8 staged A8 rows with tensor-core dots. blk: the half's first row and super-block
-// of the stage; fac: the warp's scratch, S x kFacFloats. acc[j][e]: the chain of rows 16 j + lane / 4 and the row 8 further with entry 2 (lane % 4) + e; these two rows
-// share every packed instruction. MANY: items of five entries or more. Else the eight columns hold the entries twice, and of a lane's cells the first
-// tile's count in lanes with lane % 4 < 2, the second tile's in the others: acc[0] alone is used, and half of the work after the dots falls away.
-// Absent entries compute on stale shared memory and are never stored.
+// of the stage; fac: the warp's scratch, S x kFacFloats. Chain 4 j + 2 r + e of a lane: row 16 j + 8 r + lane / 4 with the lane's entry e. MANY: items of five entries or
+// more, a lane's entries are t = lane % 4 and t + 4. Else the eight columns hold the entries twice, and of a lane's cells the first tile's count in lanes with
+// t < 2, the second tile's in the others: four chains, entries 2 (t % 2) and the next, and half of the work after the dots falls away.
+// Absent entries compute on other entries' or stale shared memory and are never stored.
 // Why 32 rows of one chain, and not 8 rows of four chains as before: what bounds the loop is what it reads from shared memory (128 bytes a clock). A token's
-// codes, deltas and sums are read once per 32 rows and a row's factors once per two entries and row pair: 44 (MANY) or 36 wavefronts a warp and super-block
+// codes, deltas and sums are read once per 32 rows and a row's factors once per two entries: 44 (MANY) or 36 wavefronts a warp and super-block
 // where the form before took 88; dp4a takes 32 for one entry and 20 more for every further one.
+// Shared memory is read by explicit 32-bit addresses: out of pointers the compiler made reads with 806,000 bank conflicts a launch (dense 5120 x 17408, 8 rows, gate/up: of
+// 4.11 M wavefronts; 64,000 of 3.37 M now), a call 60.9 us, 59.5 now.
 template <bool MANY, class G>
-__device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk, u32 p, u32 lane, const unsigned char* xs, float* fac, float2 (&acc)[MANY ? 2 : 1][2]) {
+__device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane, u32 xs, u32 fac, float (&acc)[MANY ? 8 : 4]) {
     constexpr u32 S = G::S;
     const u32 g = lane >> 2, t = lane & 3u;
-    {   // the factors, lane = row: rows i and i + 8 of a tile meet by a shuffle, so that a row pair lies in natural register pairs
-        const bool high = lane & 8u;
-        float4* put = reinterpret_cast<float4*>(fac) + 8u * (lane >> 4) + (lane & 7u) + (high ? 16u : 0u);  // [tile][row pair]{D, D, D', D'}, then {-DM, -DM, -DM', -DM'}
-        __syncwarp();   // the previous stage's readers are done with the scratch
+    const u32 head = blk + lane * G::row_bytes, put = fac + 16u * lane;
+    __syncwarp();   // the previous stage's readers are done with the scratch
 #pragma unroll
-        for (u32 b = 0; b < S; ++b) {
-            if (b >= nbk) break;
-            const float4 f = pair_factors(*reinterpret_cast<const uint4*>(blk + b * kQ4KBlock + lane * G::row_bytes), p);
-            const float u = __shfl_xor_sync(0xffffffffu, high ? f.x : f.z, 8), v = __shfl_xor_sync(0xffffffffu, high ? f.y : f.w, 8);
-            put[b * (kFacFloats / 4)] = high ? make_float4(u, f.z, v, f.w) : make_float4(f.x, u, f.y, v);
-        }
-        __syncwarp();
+    for (u32 b = 0; b < S; ++b) {  // the factors, lane = row
+        if (b >= nbk) break;
+        sts128(put + b * (kHalfRows * 16u), pair_factors(lds128(head + b * kQ4KBlock), p));
     }
-    const unsigned char* rows = blk + g * G::row_bytes + 16u + 32u * p + 4u * t;
-    const unsigned char* codes = xs + G::codes_at(MANY ? entry_of(g) : g & 3u) + 4u * t;
-    const unsigned char* es = xs + G::off_deltas + (MANY ? t : 2u * (t & 1u)) * G::box_group + 8u * p;
-    const float4* get = reinterpret_cast<const float4*>(fac) + g;
+    __syncwarp();
+    const u32 rows = blk + g * G::row_bytes + 16u + 32u * p + 4u * t;
+    const u32 codes = xs + G::codes_at(MANY ? entry_of(g) : g & 3u) + 4u * t + 64u * p;
+    const u32 es = xs + G::off_deltas + (MANY ? t : 2u * (t & 1u)) * G::box_group + 8u * p;
     const bool second = t >= 2u;  // of the few form
+    const u32 get = fac + 16u * g + (!MANY && second ? 256u : 0u);
 #pragma unroll
-    for (u32 b = 0; b < nbk; ++b) {
-        const unsigned char* cb = codes + G::column(256u * b + 64u * p);
+    for (u32 b = 0; b < S; ++b) {
+        if (b >= nbk) break;
+        const u32 cb = codes + (G::column(256u * b + 64u * p) - 64u * p);
         u32 a[2][4], bl[2], bh[2];
 #pragma unroll
         for (u32 j = 0; j < 2; ++j)
 #pragma unroll
-            for (u32 i = 0; i < 4; ++i) a[j][i] = *reinterpret_cast<const u32*>(rows + (16u * j + 8u * (i & 1u)) * G::row_bytes + 16u * (i >> 1));
+            for (u32 i = 0; i < 4; ++i) a[j][i] = lds32(rows + b * kQ4KBlock + (16u * j + 8u * (i & 1u)) * G::row_bytes + 16u * (i >> 1));
 #pragma unroll
-        for (u32 i = 0; i < 2; ++i) { bl[i] = *reinterpret_cast<const u32*>(cb + 16u * i); bh[i] = *reinterpret_cast<const u32*>(cb + 32u + 16u * i); }
+        for (u32 i = 0; i < 2; ++i) { bl[i] = lds32(cb + 16u * i); bh[i] = lds32(cb + 32u + 16u * i); }
         float2 E[2], Sg[2];
 #pragma unroll
         for (u32 e = 0; e < 2; ++e) {
-            E[e] = *reinterpret_cast<const float2*>(es + (MANY ? 4u : 1u) * e * G::box_group);
-            Sg[e] = to_float(*reinterpret_cast<const int2*>(es + (MANY ? 4u : 1u) * e * G::box_group + (G::off_sums - G::off_deltas)));
+            const uint2 d = lds64(es + 32u * b + (MANY ? 4u : 1u) * e * G::box_group), m = lds64(es + 32u * b + (MANY ? 4u : 1u) * e * G::box_group + (G::off_sums - G::off_deltas));
+            E[e] = make_float2(__uint_as_float(d.x), __uint_as_float(d.y));
+            Sg[e] = to_float(make_int2(static_cast<int>(m.x), static_cast<int>(m.y)));
         }
         int l[2][4], h[2][4];
 #pragma unroll
@@ -220,18 +228,14 @@ __device__ __forceinline__ void stage_rows_mma(const unsigned char* blk, u32 nbk
             for (u32 i = 0; i < 4; ++i) { l[0][i] = second ? l[1][i] : l[0][i]; h[0][i] = second ? h[1][i] : h[0][i]; }
         }
 #pragma unroll
-        for (u32 j = 0; j < (MANY ? 2u : 1u); ++j) {
-            const u32 tile = MANY ? j : (second ? 1u : 0u);
-            const float4 d4 = get[8u * tile], m4 = get[8u * tile + 16u];
-            const float2 Dl = make_float2(d4.x, d4.y), Dh = make_float2(d4.z, d4.w), Ml = make_float2(m4.x, m4.y), Mh = make_float2(m4.z, m4.w);
+        for (u32 j = 0; j < (MANY ? 2u : 1u); ++j)
 #pragma unroll
-            for (u32 e = 0; e < 2; ++e) {
-                const float2 sl = add2(mul2(Dl, to_float(make_int2(l[j][e], l[j][e + 2]))), mul2(Ml, both(Sg[e].x)));
-                const float2 sh = add2(mul2(Dh, to_float(make_int2(h[j][e], h[j][e + 2]))), mul2(Mh, both(Sg[e].y)));
-                acc[j][e] = add2(add2(mul2(both(E[e].x), sl), mul2(both(E[e].y), sh)), acc[j][e]);
+            for (u32 r = 0; r < 2; ++r) {
+                const uint4 v = lds128(get + b * (kHalfRows * 16u) + 256u * j + 128u * r);
+                const float4 f = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+#pragma unroll
+                for (u32 e = 0; e < 2; ++e) acc[4 * j + 2 * r + e] = __fadd_rn(acc[4 * j + 2 * r + e], pair_term(f, make_int2(l[j][2 * r + e], h[j][2 * r + e]), E[e], Sg[e]));
             }
-        }
-        rows += kQ4KBlock; es += 32; get += kFacFloats / 4;
     }
 }
 
@@ -460,10 +464,10 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         };
         auto run_mma = [&](auto many) {
             constexpr bool MANY = decltype(many)::value;
-            float2 acc[MANY ? 2 : 1][2];
+            float acc[MANY ? 8 : 4];
 #pragma unroll
-            for (u32 j = 0; j < (MANY ? 2u : 1u); ++j) { acc[j][0] = make_float2(0.0f, 0.0f); acc[j][1] = make_float2(0.0f, 0.0f); }
-            stages([&](const unsigned char* st, u32 nbk) { stage_rows_mma<MANY, G>(st + half * G::half_bytes, nbk, mp, lane, st + G::w_bytes, fac, acc); });
+            for (float& c : acc) c = 0.0f;
+            stages([&](const unsigned char* st, u32 nbk) { stage_rows_mma<MANY, G>(saddr(st) + half * G::half_bytes, nbk, mp, lane, saddr(st) + G::w_bytes, saddr(fac), acc); });
             if (!ok) return;
             hand_over([&]() {
 #pragma unroll
@@ -472,8 +476,8 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                     for (u32 e = 0; e < 2; ++e) {
                         const u32 tile = MANY ? j : mt >> 1, entry = MANY ? mt + 4u * e : 2u * (mt & 1u) + e;
                         float* to = meet + ((2u * mp + half) * kKE + entry) * kMeetPitch + 16u * tile + me;
-                        to[0] = acc[j][e].x;
-                        to[8] = acc[j][e].y;
+                        to[0] = acc[4 * j + e];
+                        to[8] = acc[4 * j + 2 + e];
                     }
             });
         };

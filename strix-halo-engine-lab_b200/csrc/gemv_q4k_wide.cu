@@ -22,6 +22,8 @@
 //    left in place as 16 q; B = the codes of up to 8 entries, signed), a warp 32 rows of ONE chain; the four chains meet in shared memory at the end of
 //    the item. With up to 4 entries the eight columns hold them twice, and a lane works for one of the two row tiles only. The pair's two groups
 //    of a cell share every packed FP32 instruction; both forms produce the contract's bits.
+//  * Where there are no more items than CTAs (rows of several stages: a dense block's down) an item is both groups': each takes every other stage, makes what its
+//    super-blocks add to the chains, gets the chains from the other group, adds in order and hands them on (PAIR).
 //  * gate/up: the group meets on an mbarrier once per item and a warp an entry runs SwiGLU + the A8 rule; down: a warp an entry stores the sums.
 // What bounds it: the latency of dependent instructions with four consumer warps a scheduler (64 rows over 64 experts of 7168 -> 2048: 62 % of the issue
 // slots, 67 % of the shared memory's cycles, 49 % of the DRAM's). A warp with 8 rows of four chains, whose factors met 8 rows and which took the tensor cores from
@@ -61,6 +63,7 @@ struct WidePlan {
     u32 stages;         // ring depth per group
     u32 cap;            // entries that a stage holds: 1, 4 or 8
     u32 stage_bytes;
+    u32 pair;           // an item's stages are shared by the CTA's two groups
     u32 n_chunks;       // items per (virtual) expert
     u32 max_union;      // bound of the union
     u32 n_bound;        // ... that the routes' arrays are known to hold too, or 0
@@ -143,8 +146,8 @@ __device__ __forceinline__ float pair_term(const float4& f, int2 dot, float2 E, 
 
 // One stage of one weight row (this lane's pair p of nbk super-blocks, ascending) against one staged A8 row. blk: the row's first
 // super-block of the stage; xs: the stage's A8 rows, of which the first is meant.
-template <class G>
-__device__ __forceinline__ void stage_row(const unsigned char* blk, u32 nbk, u32 p, const unsigned char* xs, float& acc) {
+template <class G, class Put>
+__device__ __forceinline__ void stage_row(const unsigned char* blk, u32 nbk, u32 p, const unsigned char* xs, Put put_term) {
     constexpr u32 S = G::S;
 #pragma unroll
     for (u32 b = 0; b < S; ++b, blk += kQ4KBlock) {
@@ -159,7 +162,7 @@ __device__ __forceinline__ void stage_row(const unsigned char* blk, u32 nbk, u32
         const float2 sm = to_float(*reinterpret_cast<const int2*>(xs + G::off_sums + 32u * b + 8u * p));
         int l, h;
         dots(n, c0, c1, c2, c3, &l, &h);
-        acc = __fadd_rn(acc, pair_term(f, make_int2(l, h), e, sm));
+        put_term(b, 0, pair_term(f, make_int2(l, h), e, sm));
     }
 }
 // ---- the mma form of one stage ---------------------------------------------------------------------------------------
@@ -182,8 +185,8 @@ __device__ __forceinline__ u32 entry_of(u32 c) { return (c >> 1) + 4u * (c & 1u)
 // where the form before took 88; dp4a takes 32 for one entry and 20 more for every further one.
 // Shared memory is read by explicit 32-bit addresses: out of pointers the compiler made reads with 806,000 bank conflicts a launch (dense 5120 x 17408, 8 rows, gate/up: of
 // 4.11 M wavefronts; 64,000 of 3.37 M now), a call 60.9 us, 59.5 now.
-template <bool MANY, class G>
-__device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane, u32 xs, u32 fac, float (&acc)[MANY ? 8 : 4]) {
+template <bool MANY, class G, class Put>
+__device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane, u32 xs, u32 fac, Put put_term) {
     constexpr u32 S = G::S;
     const u32 g = lane >> 2, t = lane & 3u;
     const u32 head = blk + lane * G::row_bytes, put = fac + 16u * lane;
@@ -234,7 +237,7 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
                 const uint4 v = lds128(get + b * (kHalfRows * 16u) + 256u * j + 128u * r);
                 const float4 f = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
 #pragma unroll
-                for (u32 e = 0; e < 2; ++e) acc[4 * j + 2 * r + e] = __fadd_rn(acc[4 * j + 2 * r + e], pair_term(f, make_int2(l[j][2 * r + e], h[j][2 * r + e]), E[e], Sg[e]));
+                for (u32 e = 0; e < 2; ++e) put_term(b, 4 * j + 2 * r + e, pair_term(f, make_int2(l[j][2 * r + e], h[j][2 * r + e]), E[e], Sg[e]));
             }
     }
 }
@@ -244,7 +247,7 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
 // The entries' A8 rows by gathering copies: to ask for a stage's 24 bulk copies (8 entries) took a producer 1,690 clocks on its own and 1,880 beside the consumers,
 // whose work on the stage is 2,030 (64 rows of the large layer); a gathering copy of four rows 83. In a graph, us a call: large layer of 64 rows 720 -> 681, dense 5120 x 17408
 // 42.4 -> 39.6 (1 row) and 65.7 -> 61.8 (8).
-template <bool DOWN, u32 S_, u32 CAP_>
+template <bool DOWN, u32 S_, u32 CAP_, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan) {
     using G = Geo<S_, CAP_>;
@@ -264,17 +267,20 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
     u64* empty = full + kGroups * plan.stages;
     u64* met = empty + kGroups * plan.stages;  // a group's item: its chains are there
     u64* left = met + kGroups;                 // ... and have been read
-    at += (2 * kGroups * plan.stages + 2 * kGroups) * 8;
+    u64* passed = left + kGroups;              // PAIR: [group][warp] the chains are there for the group's next stage
+    at += (2 * kGroups * plan.stages + 2 * kGroups + (PAIR ? kConsumerWarps : 0u)) * 8;
     u32* slot_item = reinterpret_cast<u32*>(at);
     at += kGroups * plan.stages * 4;
+    float* s_pass = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(at) + 64 + 15) & ~uintptr_t(15));  // PAIR: [group][warp][cells][lane]
     u32* ctl = reinterpret_cast<u32*>(at);  // [0] abort flag, [1] producers that have retired, [2] virtual experts, [3] items
     volatile u32* abort_flag = ctl;
 
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     if (tid < kGroups * plan.stages) { mbar_init(&full[tid], 1); mbar_init(&empty[tid], kGroupWarps); }
     if (tid < 2 * kGroups) mbar_init(&met[tid], kGroupWarps);
+    if (PAIR && tid < kConsumerWarps) mbar_init(&passed[tid], 1);
     if (tid < 2) ctl[tid] = 0;  // the list's builder writes the others, and for a dense block there is no barrier between here and there
-    if (tid < kGroups * plan.stages + 2 * kGroups) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (tid < kGroups * plan.stages + (PAIR ? kConsumerWarps : 2 * kGroups)) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 
     if (!early) chain_begin();
     if (DOWN && !early && block_skips(a.summary)) return;  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
@@ -283,6 +289,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
     if (plan.dense_rows) build_dense_list(plan.dense_rows, plan.n_chunks, table, ctl);
     else build_work_list(a.routes, plan.n_bound ? plan.n_bound : min(load_l2(a.routes.counts), plan.max_union), plan.max_union, plan.vmax, plan.n_chunks, reinterpret_cast<u32*>(smem), table, ctl);
     const u32 n_items = ctl[3];
+    const u32 my_segs = PAIR ? (plan.nseg + 1u - (warp < kConsumerWarps ? warp / kGroupWarps : warp - kConsumerWarps)) / 2u : plan.nseg;  // stages of an item that are the group's
     if (n_items == 0) {  // every CTA alike: nobody claims, the claim word stays zero
         if (early) chain_begin();
         return;
@@ -306,16 +313,16 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         };
         u32 ahead = 0;  // stages of the first item whose weights were asked for before the wait
         if (early) {
-            const u32 k = g * gridDim.x + blockIdx.x;
+            const u32 k = PAIR ? blockIdx.x : g * gridDim.x + blockIdx.x;
             if (k < n_items) {
-                ahead = min(plan.nseg, plan.stages);
+                ahead = min(my_segs, plan.stages);
                 if (g == 0) ahead = min(ahead, plan.stall_stage);
                 if (lane == 0) {
                     const u32 jv = k / plan.n_chunks;
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the list was made in the stages' memory
                     for (u32 s = 0; s < ahead; ++s) {
                         mbar_expect_more(&g_full[s], G::w_bytes);
-                        ask_weights(s, table[jv], k - jv * plan.n_chunks, g_stage + s * plan.stage_bytes, &g_full[s]);
+                        ask_weights(PAIR ? 2u * s + g : s, table[jv], k - jv * plan.n_chunks, g_stage + s * plan.stage_bytes, &g_full[s]);
                     }
                 }
             }
@@ -333,10 +340,13 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         for (;;) {
             // A group's first item needs no round trip: group 0 of CTA b takes item b, group 1 item gridDim.x + b - so a
             // launch with fewer items than groups runs one group per SM, which has the SM's issue slots to itself.
-            u32 k = g * gridDim.x + blockIdx.x;
+            u32 k = PAIR ? blockIdx.x : g * gridDim.x + blockIdx.x;
             if (!first) {
-                if (lane == 0) k = gridDim.x * kGroups + claim_item(claim);
-                k = __shfl_sync(0xffffffffu, k, 0);
+                if (PAIR) k = n_items;  // there are no more items than CTAs
+                else {
+                    if (lane == 0) k = gridDim.x * kGroups + claim_item(claim);
+                    k = __shfl_sync(0xffffffffu, k, 0);
+                }
             }
             first = false;
             const bool end = k >= n_items;
@@ -356,8 +366,9 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
 #pragma unroll
                 for (u32 i = 0; i < 8; ++i) r[i] = i < G::CAP ? __shfl_sync(0xffffffffu, mine, i) : 0u;
             }
-            const u32 nsegs = end ? 1u : plan.nseg;
-            for (u32 s = 0; s < nsegs; ++s, ++t, ++slot) {
+            const u32 nsegs = end ? 1u : my_segs;
+            for (u32 i = 0; i < nsegs; ++i, ++t, ++slot) {
+                const u32 s = PAIR ? 2u * i + g : i;
                 if (slot == plan.stages) { slot = 0; ++use; }
                 if (use) ok = mbar_wait(&g_empty[slot], (use - 1u) & 1u, plan.wait_limit, abort_flag);  // the slot's previous use is done
                 ok = __all_sync(0xffffffffu, ok);
@@ -403,7 +414,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                 for (u32 i = 0; i < (plan.wait_limit >> 4) + 64u; ++i)
                     if (mbar_try_wait(&g_full[n % plan.stages], (n / plan.stages) & 1u)) break;
         }
-        if (lane == 0) retire_claims(claim, ctl);
+        if (!PAIR && lane == 0) retire_claims(claim, ctl);
         return;
     }
 
@@ -436,21 +447,51 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         const u32 ne = ve.ne(), vbegin = ve.begin();
         const bool mma = G::CAP > 1 && ne > kDpEntries;
         const u32 slot_id = w >= ne ? 0u : plan.dense_rows ? vbegin + w : load(a.routes.slots + vbegin + w);  // asked for before the stages, used behind them
-        // the item's stages, with the form fixed at compile time inside the loop
-        auto stages = [&](auto step) {
-            for (u32 s = 0; s < plan.nseg; ++s) {
-                if (s) {
+        // The item's stages, with the form fixed at compile time inside the loop: `terms` makes what the stage's super-blocks add to the chains. PAIR: the chains go
+        // to the other group's warp of the same rows after each stage, and the last stage's group ends the item.
+        auto stages = [&](auto& chain, auto terms) {
+            constexpr u32 N = sizeof(chain) / 4u;
+#pragma unroll
+            for (float& c : chain) c = 0.0f;
+            for (u32 i = 0; i < my_segs; ++i) {
+                const u32 s = PAIR ? 2u * i + g : i, nbk = min(G::S, plan.nb - s * G::S);
+                if (i) {
                     ok = mbar_wait(&g_full[slot], phase, plan.wait_limit, abort_flag);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) return;
                 }
-                const unsigned char* st = g_stage + slot * plan.stage_bytes;
-                step(st, min(G::S, plan.nb - s * G::S));
+                float term[G::S][N];
+                terms(g_stage + slot * plan.stage_bytes, nbk, [&](u32 b, u32 c, float v) {
+                    if (PAIR) term[b][c] = v;
+                    else chain[c] = __fadd_rn(chain[c], v);
+                });
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&g_empty[slot]);  // the stage is free for the producer
                 if (++slot == plan.stages) { slot = 0; phase ^= 1u; }
+                float* mine = s_pass + warp * (32u * N);
+                if (PAIR && s) {
+                    ok = mbar_wait(&passed[warp], (i - 1u + g) & 1u, plan.wait_limit, abort_flag);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) return;
+#pragma unroll
+                    for (u32 c = 0; c < N; ++c) chain[c] = mine[32u * c + lane];
+                }
+#pragma unroll
+                for (u32 b = 0; b < G::S; ++b) {
+                    if (!PAIR || b >= nbk) break;
+#pragma unroll
+                    for (u32 c = 0; c < N; ++c) chain[c] = __fadd_rn(chain[c], term[b][c]);
+                }
+                if (PAIR && s + 1u < plan.nseg) {
+                    float* theirs = s_pass + (warp ^ kGroupWarps) * (32u * N);
+#pragma unroll
+                    for (u32 c = 0; c < N; ++c) theirs[32u * c + lane] = chain[c];
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&passed[warp ^ kGroupWarps]);
+                }
             }
         };
+        const bool ends_item = !PAIR || ((plan.nseg - 1u) & 1u) == g;
         // the chains meet in shared memory, once the previous item's have been read
         auto hand_over = [&](auto store) {
             if (kl) ok = mbar_wait(&left[g], (kl - 1u) & 1u, plan.wait_limit, abort_flag);
@@ -465,10 +506,8 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         auto run_mma = [&](auto many) {
             constexpr bool MANY = decltype(many)::value;
             float acc[MANY ? 8 : 4];
-#pragma unroll
-            for (float& c : acc) c = 0.0f;
-            stages([&](const unsigned char* st, u32 nbk) { stage_rows_mma<MANY, G>(saddr(st) + half * G::half_bytes, nbk, mp, lane, saddr(st) + G::w_bytes, saddr(fac), acc); });
-            if (!ok) return;
+            stages(acc, [&](const unsigned char* st, u32 nbk, auto put) { stage_rows_mma<MANY, G>(saddr(st) + half * G::half_bytes, nbk, mp, lane, saddr(st) + G::w_bytes, saddr(fac), put); });
+            if (!ok || !ends_item) return;
             hand_over([&]() {
 #pragma unroll
                 for (u32 j = 0; j < (MANY ? 2u : 1u); ++j)
@@ -483,10 +522,11 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         };
         if (!mma) {
             const u32 only_slot = !DOWN ? 0u : plan.dense_rows ? vbegin : load(a.routes.slots + vbegin);
-            float acc = 0.0f;
-            stages([&](const unsigned char* st, u32 nbk) { stage_row<G>(st + half * G::half_bytes + (8u * mp + rr) * G::row_bytes, nbk, p, st + G::w_bytes, acc); });
+            float acc[1];
+            stages(acc, [&](const unsigned char* st, u32 nbk, auto put) { stage_row<G>(st + half * G::half_bytes + (8u * mp + rr) * G::row_bytes, nbk, p, st + G::w_bytes, put); });
             if (!ok) break;
-            const float val = tree4(acc);
+            if (!ends_item) continue;
+            const float val = tree4(acc[0]);
             if (DOWN) {
                 if (p == 0) a.raw[u64(only_slot) * a.out_width + kItemRows * chunk + 8u * w + rr] = val;
                 continue;
@@ -498,6 +538,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
             if constexpr (G::CAP > 1) run_mma(std::false_type{});
         }
         if (!ok) break;
+        if (!ends_item) continue;
         if (w < ne) {
             const float* mine = meet + w * kMeetPitch;
             constexpr u32 kHalf = kKE * kMeetPitch, kPair = 2 * kHalf;
@@ -547,7 +588,7 @@ u32 round_up(u32 v, u32 a) { return (v + a - 1) / a * a; }
 
 u32 fixed_smem(const WidePlan& p) {
     return kGroups * kMeetFloats * 4 + round_up(p.vmax * static_cast<u32>(sizeof(VExpert)), 16) + kConsumerWarps * p.S * kFacFloats * 4 +
-           (2 * kGroups * p.stages + 2 * kGroups) * 8 + kGroups * p.stages * 4 + 64;
+           (2 * kGroups * p.stages + 2 * kGroups) * 8 + kGroups * p.stages * 4 + 64 + (p.pair ? kConsumerWarps * 8 + 16 + kConsumerWarps * 128 * p.cap : 0u);
 }
 u32 plan_smem(const WidePlan& p) { return kGroups * p.stages * p.stage_bytes + fixed_smem(p); }
 
@@ -566,6 +607,10 @@ bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, WidePlan* p) {
     p->max_union = max_union;
     p->vmax = max_union + static_cast<u32>(slots / kKE) + 1;
     if (u64(p->vmax) * n_chunks + 4096 >= kClaimMask) return false;  // items and the groups' closing claims fit the claim word's count
+    // PAIR where the items, virtual experts at most union + (entries beyond one each) / kKE times the chunks, are no more than CTAs, so that the second group would
+    // have nothing to do. Down of a dense 5120 x 17408 block (80 items of 23 stages): 1 row 29,700 -> 24,400 clocks, 8 rows 53,400 -> 46,800; a call 39.6 -> 38.1 and
+    // 59.5 -> 58.0 us.
+    p->pair = p->S == 3 && p->nseg > 1 && (max_union + (slots - std::min<u64>(slots, max_union)) / kKE) * n_chunks <= static_cast<u32>(device_sm_count());
     for (p->stages = kMaxStages; p->stages >= 2; --p->stages)
         if (plan_smem(*p) <= kSmemBudget) break;
     if (p->stages < 2) return false;
@@ -594,8 +639,9 @@ int entry_maps(const b200moe_a8_rows& x, u32 K, const WidePlan& p, WideMaps* m) 
 }
 template <bool DOWN>
 int launch_wide(const WideMaps& m, const WideArgs& a, const WidePlan& p, cudaStream_t stream) {
-    const auto kernel = p.S == 3 ? (p.cap == 1 ? q4k_wide_kernel<DOWN, 3, 1> : p.cap == 4 ? q4k_wide_kernel<DOWN, 3, 4> : q4k_wide_kernel<DOWN, 3, 8>)
-                                 : (p.cap == 1 ? q4k_wide_kernel<DOWN, 1, 1> : p.cap == 4 ? q4k_wide_kernel<DOWN, 1, 4> : q4k_wide_kernel<DOWN, 1, 8>);
+    const auto kernel = p.pair ? (p.cap == 1 ? q4k_wide_kernel<DOWN, 3, 1, true> : p.cap == 4 ? q4k_wide_kernel<DOWN, 3, 4, true> : q4k_wide_kernel<DOWN, 3, 8, true>)
+                        : p.S == 3 ? (p.cap == 1 ? q4k_wide_kernel<DOWN, 3, 1, false> : p.cap == 4 ? q4k_wide_kernel<DOWN, 3, 4, false> : q4k_wide_kernel<DOWN, 3, 8, false>)
+                                   : (p.cap == 1 ? q4k_wide_kernel<DOWN, 1, 1, false> : p.cap == 4 ? q4k_wide_kernel<DOWN, 1, 4, false> : q4k_wide_kernel<DOWN, 1, 8, false>);
     const u32 smem = plan_smem(p);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
     chain_launch(kernel, device_sm_count(), kThreads, smem, stream, m, a, p);

@@ -808,8 +808,7 @@ def test_q8_one_item_a_cta(gpu, oracle, rows, top_k, E, H, I, forms):
 
 @pytest.mark.parametrize("rows,H,I", [(1, 512, 256), (1, 2560, 1280), (2, 64 * 148, 768), (4, 512, 1024), (5, 1024, 2048), (8, 2048, 1536), (8, 64 * 148 + 256, 512), (9, 512, 768), (7, 512, 768), (17, 1280, 2560)])
 def test_dense_rows_of_few_and_whole_items(gpu, oracle, rows, H, I):
-    """Dense blocks next to the line between bulk and asynchronous copies of the A8 rows (8 rows), with whole and broken last items, more and fewer items than
-    CTAs; rows of 1 to 10 super-blocks."""
+    """Dense blocks with whole and broken last items (8 rows), more and fewer items than CTAs; rows of 1 to 10 super-blocks."""
     import b200moe
     from b200moe import ops, synth
     rng = np.random.default_rng(rows + H)
@@ -1173,3 +1172,34 @@ def test_routes_with_invalid_rows(gpu, rows, top_k, first, end):
     assert np.array_equal(r.low_counts.cpu().numpy(), (ids < 6).sum(axis=1))
     bad = {rows // 2} | ({0} if top_k > 1 else set())
     assert [int(x) for x in status.cpu()] == [b200moe.ROW_INVALID_ROUTE if i in bad else 0 for i in range(rows)]
+
+
+@pytest.mark.parametrize("rows,top_k,E,H,I", [(1, 1, 1, 1024, 1792), (3, 1, 1, 2560, 768), (6, 1, 1, 1536, 3072), (9, 1, 1, 768, 5120), (4, 2, 4, 1024, 1024), (20, 1, 3, 512, 2304)])
+def test_items_by_both_groups_of_a_block(gpu, oracle, rows, top_k, E, H, I):
+    """Fewer items than multiprocessors: their stages are shared by a block's two groups. 1 to 7 stages a row, whole and broken last ones, items of one, a few and many
+    entries; a stage of the one group that is never asked for ends both groups' waits."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, 12, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh, x, w = ops.make_shape(H, I, E, top_k, 12, 12), (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), (dv(gate, gpu), dv(up, gpu), dv(down, gpu))
+    r, union, flags = ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2), min(E, rows * top_k), torch.zeros(8, dtype=torch.int32, device=gpu)
+
+    def run(**k):
+        act, g, u = ops.enqueue_routed_gate_up(sh, w[0], w[1], r, union, x, rows * top_k, taps=True)
+        assert b200moe.last_launch() == "gate_up_q4k_wide"
+        raw = ops.enqueue_routed_down(sh, w[2], r, union, k.get("act", act), summary=k.get("summary"))
+        assert b200moe.last_launch() == "down_q4k_wide"
+        return g, u, raw, act
+
+    with forced(b200moe.FORM_SEGMENT_STREAM):
+        g, u, raw, act = run()
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+    with stalled(b200moe.FORM_SEGMENT_STREAM, 1, 64):
+        run(act=act, summary=flags[:1])
+    assert flags[0].item() & b200moe.JOB_WAIT_ABORTED
+    with forced(b200moe.FORM_SEGMENT_STREAM):
+        assert same(run()[2].cpu(), want["raw"])

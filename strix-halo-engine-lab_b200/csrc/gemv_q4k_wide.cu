@@ -147,22 +147,20 @@ __device__ __forceinline__ float pair_term(const float4& f, int2 dot, float2 E, 
 // One stage of one weight row (this lane's pair p of nbk super-blocks, ascending) against one staged A8 row. blk: the row's first
 // super-block of the stage; xs: the stage's A8 rows, of which the first is meant.
 template <class G, class Put>
-__device__ __forceinline__ void stage_row(const unsigned char* blk, u32 nbk, u32 p, const unsigned char* xs, Put put_term) {
+__device__ __forceinline__ void stage_row(u32 blk, u32 nbk, u32 p, u32 xs, Put put_term) {
     constexpr u32 S = G::S;
+    const u32 q = blk + 16u + 32u * p, cs = xs + 64u * p, es = xs + G::off_deltas + 8u * p;
 #pragma unroll
-    for (u32 b = 0; b < S; ++b, blk += kQ4KBlock) {
+    for (u32 b = 0; b < S; ++b) {
         if (b >= nbk) break;
-        const uint4* w = reinterpret_cast<const uint4*>(blk);
-        const uint4 hdr = w[0], q0 = w[1 + 2 * p], q1 = w[2 + 2 * p];
+        const uint4 hdr = lds128(blk + b * kQ4KBlock), q0 = lds128(q + b * kQ4KBlock), q1 = lds128(q + b * kQ4KBlock + 16u);
         const float4 f = pair_factors(hdr, p);
         const Nibbles n = split_nibbles(q0, q1);
-        const uint4* c = reinterpret_cast<const uint4*>(xs + 256u * b + 64u * p);
-        const uint4 c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
-        const float2 e = *reinterpret_cast<const float2*>(xs + G::off_deltas + 32u * b + 8u * p);
-        const float2 sm = to_float(*reinterpret_cast<const int2*>(xs + G::off_sums + 32u * b + 8u * p));
+        const uint4 c0 = lds128(cs + 256u * b), c1 = lds128(cs + 256u * b + 16u), c2 = lds128(cs + 256u * b + 32u), c3 = lds128(cs + 256u * b + 48u);
+        const uint2 d = lds64(es + 32u * b), m = lds64(es + (G::off_sums - G::off_deltas) + 32u * b);
         int l, h;
         dots(n, c0, c1, c2, c3, &l, &h);
-        put_term(b, 0, pair_term(f, make_int2(l, h), e, sm));
+        put_term(b, 0, pair_term(f, make_int2(l, h), make_float2(__uint_as_float(d.x), __uint_as_float(d.y)), to_float(make_int2(static_cast<int>(m.x), static_cast<int>(m.y)))));
     }
 }
 // ---- the mma form of one stage ---------------------------------------------------------------------------------------
@@ -190,7 +188,7 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
     constexpr u32 S = G::S;
     const u32 g = lane >> 2, t = lane & 3u;
     const u32 head = blk + lane * G::row_bytes, put = fac + 16u * lane;
-    __syncwarp();   // the previous stage's readers are done with the scratch
+    // the previous stage's readers are done with the scratch: they met before they handed the stage back
 #pragma unroll
     for (u32 b = 0; b < S; ++b) {  // the factors, lane = row
         if (b >= nbk) break;
@@ -359,8 +357,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                 const u32 s = PAIR ? 2u * i + g : i;
                 if (slot == plan.stages) { slot = 0; ++use; }
                 if (!PAIR && !end && i + 1u == nsegs && lane == 0) next = claim_item(claim);
-                if (use) ok = mbar_wait(&g_empty[slot], (use - 1u) & 1u, plan.wait_limit, abort_flag);  // the slot's previous use is done
-                ok = __all_sync(0xffffffffu, ok);
+                if (use) ok = warp_wait(&g_empty[slot], (use - 1u) & 1u, plan.wait_limit, abort_flag);  // the slot's previous use is done
                 if (!ok) break;
                 if (g == 0 && t == plan.stall_stage) { ok = false; break; }  // test hook: stop feeding, raise nothing
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the consumers' reads precede the copies below
@@ -426,13 +423,12 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
     u64* g_full = full + g * plan.stages;
     u64* g_empty = empty + g * plan.stages;
     const u32* g_item = slot_item + g * plan.stages;
-    const unsigned char* g_stage = smem + g * plan.stages * plan.stage_bytes;
+    const u32 g_stage = saddr(smem) + g * plan.stages * plan.stage_bytes;
     const u32 act_stride = DOWN ? 0u : (a.act.stride ? a.act.stride : a.act.width);
     u32 slot = 0, phase = 0, kl = 0;  // ring position of the group's next stage, kept incrementally (no divisions in the loop); meetings so far
     bool ok = true;
     for (;;) {
-        ok = mbar_wait(&g_full[slot], phase, plan.wait_limit, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = warp_wait(&g_full[slot], phase, plan.wait_limit, abort_flag);
         if (!ok) break;
         const u32 item = g_item[slot];
         if (item == kEndItem) break;
@@ -450,8 +446,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
             for (u32 i = 0; i < my_segs; ++i) {
                 const u32 s = PAIR ? 2u * i + g : i, nbk = min(G::S, plan.nb - s * G::S);
                 if (i) {
-                    ok = mbar_wait(&g_full[slot], phase, plan.wait_limit, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = warp_wait(&g_full[slot], phase, plan.wait_limit, abort_flag);
                     if (!ok) return;
                 }
                 float term[G::S][N];
@@ -464,8 +459,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                 if (++slot == plan.stages) { slot = 0; phase ^= 1u; }
                 float* mine = s_pass + warp * (32u * N);
                 if (PAIR && s) {
-                    ok = mbar_wait(&passed[warp], (i - 1u + g) & 1u, plan.wait_limit, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = warp_wait(&passed[warp], (i - 1u + g) & 1u, plan.wait_limit, abort_flag);
                     if (!ok) return;
 #pragma unroll
                     for (u32 c = 0; c < N; ++c) chain[c] = mine[32u * c + lane];
@@ -488,19 +482,17 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         const bool ends_item = !PAIR || ((plan.nseg - 1u) & 1u) == g;
         // the chains meet in shared memory, once the previous item's have been read
         auto hand_over = [&](auto store) {
-            if (kl) ok = mbar_wait(&left[g], (kl - 1u) & 1u, plan.wait_limit, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
+            if (kl) ok = warp_wait(&left[g], (kl - 1u) & 1u, plan.wait_limit, abort_flag);
             if (!ok) return;
             store();
             __syncwarp();
             if (lane == 0) mbar_arrive(&met[g]);
-            ok = mbar_wait(&met[g], kl & 1u, plan.wait_limit, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_wait(&met[g], kl & 1u, plan.wait_limit, abort_flag);
         };
         auto run_mma = [&](auto many) {
             constexpr bool MANY = decltype(many)::value;
             float acc[MANY ? 8 : 4];
-            stages(acc, [&](const unsigned char* st, u32 nbk, auto put) { stage_rows_mma<MANY, G>(saddr(st) + half * G::half_bytes, nbk, mp, lane, saddr(st) + G::w_bytes, saddr(fac), put); });
+            stages(acc, [&](u32 st, u32 nbk, auto put) { stage_rows_mma<MANY, G>(st + half * G::half_bytes, nbk, mp, lane, st + G::w_bytes, saddr(fac), put); });
             if (!ok || !ends_item) return;
             hand_over([&]() {
 #pragma unroll
@@ -517,7 +509,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         if (!mma) {
             const u32 only_slot = !DOWN ? 0u : plan.dense_rows ? vbegin : load(a.routes.slots + vbegin);
             float acc[1];
-            stages(acc, [&](const unsigned char* st, u32 nbk, auto put) { stage_row<G>(st + half * G::half_bytes + (8u * mp + rr) * G::row_bytes, nbk, p, st + G::w_bytes, put); });
+            stages(acc, [&](u32 st, u32 nbk, auto put) { stage_row<G>(st + half * G::half_bytes + (8u * mp + rr) * G::row_bytes, nbk, p, st + G::w_bytes, put); });
             if (!ok) break;
             if (!ends_item) continue;
             const float val = tree4(acc[0]);

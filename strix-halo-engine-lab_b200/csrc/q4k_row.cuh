@@ -50,6 +50,11 @@ __device__ __forceinline__ bool mbar_wait(u64* bar, u32 parity, u32 limit, volat
     *abort_flag = 1;
     return false;
 }
+// The same by a whole warp, one answer for all lanes. The common case is one poll and one vote, without a branch that lanes could part at.
+__device__ __forceinline__ bool warp_wait(u64* bar, u32 parity, u32 limit, volatile u32* abort_flag) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit, abort_flag));
+}
 // Untiled bulk copy global -> shared: both addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, u32 bytes, u64* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(saddr(dst)),

@@ -224,15 +224,16 @@ namespace b200moe {
 namespace {
 
 // One warp per row; shared memory per warp: scores[experts] + choice[experts] + 32 group scores.
+template <int EPL>
 __global__ void __launch_bounds__(128) router_select_kernel(const float* logits, float* scores_out, const float* bias,
-                                                            b200moe_route_policy p, u32 rows, u32* ids,
+                                                            const __grid_constant__ b200moe_route_policy p, u32 rows, u32* ids,
                                                             float* weights) {
     chain_begin();
     extern __shared__ __align__(16) float smem[];
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const u32 row = blockIdx.x * 4u + warp;
     if (row >= rows) return;
-    select_detail::select_row<1024>(logits, scores_out, bias, p, row, lane, smem + warp * select_detail::scratch_floats(p.experts), ids, weights);
+    select_detail::select_row<EPL>(logits, scores_out, bias, p, row, lane, smem + warp * select_detail::scratch_floats(p.experts), ids, weights);
 }
 
 }  // namespace
@@ -282,7 +283,8 @@ int launch_router_logits(const b200moe_router_view& v, cudaStream_t stream, cons
 int launch_router_select(const b200moe_router_view& v, cudaStream_t stream) {
     if (v.rows == 0) return B200MOE_OK;
     const u32 smem = 4u * select_detail::scratch_floats(v.policy.experts) * sizeof(float);
-    small_launch(router_select_kernel, (v.rows + 3) / 4, 128, smem, stream, v.logits, v.scores, v.bias, v.policy, v.rows, v.ids, v.weights);
+    const auto kernel = v.policy.experts <= 128u ? router_select_kernel<4> : v.policy.experts <= 256u ? router_select_kernel<8> : router_select_kernel<32>;
+    small_launch(kernel, (v.rows + 3) / 4, 128, smem, stream, v.logits, v.scores, v.bias, v.policy, v.rows, v.ids, v.weights);
     return after_launch("router_select");
 }
 

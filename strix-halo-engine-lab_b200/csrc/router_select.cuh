@@ -73,7 +73,7 @@ __device__ __forceinline__ float key_value(u32 k) { return __uint_as_float((k & 
 // the contract's serial scans are then "largest choice, lowest id on ties" under either key rule, which two warp reductions a pass give (the
 // largest key, then the lowest id that has it; 0 is no candidate's key). Groups are runs of 2^i lanes or whole runs of 32 experts: a group's two
 // best are merged by shuffles or reductions. Returns false - with nothing stored - when the row needs the general path. `s` = this warp's
-// scratch of at least `experts` floats on a 16-byte boundary (shared memory); holds the scores afterwards.
+// scratch of scratch_floats(experts) floats on a 16-byte boundary (shared memory); holds the scores afterwards.
 // The work is a chain of latencies in one warp, mostly run once a call on cold instruction caches, so the long steps (exp, quotient) are
 // rolled loops of four values a lane: 8 rows of 128 took 12,800 clocks with a shuffle tree a pass and everything unrolled.
 template <int EPL>
@@ -191,29 +191,38 @@ __device__ __forceinline__ bool select_row_fast(const float* logits, float* scor
     }
     if (scores_out) for (u32 e = lane; e < E; e += 32) scores_out[u64(row) * E + e] = s[e];
     __syncwarp();
-    u32 my_id = kNone;
+    u32* picks = reinterpret_cast<u32*>(s + E);
 #pragma unroll 1
     for (u32 k = 0; k < p.top_k; ++k) {
         u32 top = 0;
 #pragma unroll
         for (int j = 0; j < EPL; ++j) top = max(top, key[j]);
-        const u32 best = __reduce_max_sync(0xffffffffu, top);
-        u32 id = kNone;
+        const u32 best = __reduce_max_sync(0xffffffffu, top), holders = __ballot_sync(0xffffffffu, top == best);
+        u32 winner = __ffs(holders) - 1u;  // best is some lane's
+        if (holders & (holders - 1u)) {    // several lanes have it: the lowest id (lane + 32 j) does
+            u32 id = kNone;
 #pragma unroll
-        for (int j = EPL - 1; j >= 0; --j) if (key[j] == best) id = lane + 32u * j;
-        id = best ? __reduce_min_sync(0xffffffffu, id) : kNone;
+            for (int j = EPL - 1; j >= 0; --j) if (key[j] == best) id = lane + 32u * j;
+            winner = __reduce_min_sync(0xffffffffu, id) & 31u;
+        }
+        if (lane == winner) {
+            u32 id = kNone;
 #pragma unroll
-        for (int j = 0; j < EPL; ++j) if (lane + 32u * j == id) key[j] = 0u;
-        if (lane == k) my_id = id;
+            for (int j = EPL - 1; j >= 0; --j) if (key[j] == best) id = lane + 32u * j;
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) if (lane + 32u * j == id) key[j] = 0u;
+            picks[k] = best ? id : kNone;
+        }
     }
+    __syncwarp();
+    const u32 my_id = lane < p.top_k ? picks[lane] : kNone;
     *picked = my_id;
     return true;
 }
 
-// Output order, weights and the stores of one row; lane k holds pick k in `my_id`, s[] the scores.
-// ids_copy: the row's ids once more (shared memory), for a block that goes on with them.
-__device__ __forceinline__ void finish_row(const b200moe_route_policy& p, u32 row, u32 lane, const float* s, u32 my_id,
-                                        u32* ids, float* weights, u32* ids_copy) {
+// Output order, weights and the stores of one row; lane k holds pick k in `my_id`, s[] the scores. Returns the lane's id in output order.
+__device__ __forceinline__ u32 finish_row(const b200moe_route_policy& p, u32 row, u32 lane, const float* s, u32 my_id,
+                                        u32* ids, float* weights) {
     if (p.order == B200MOE_ORDER_ASCENDING_ID) {  // rank sort of the (distinct) ids held one per lane
         u32 rank = 0;
         for (u32 k = 0; k < p.top_k; ++k) { const u32 o = __shfl_sync(0xffffffffu, my_id, k); rank += (o < my_id) ? 1u : 0u; }
@@ -226,35 +235,30 @@ __device__ __forceinline__ void finish_row(const b200moe_route_policy& p, u32 ro
     }
     const float my_s = (lane < p.top_k && my_id != kNone) ? s[my_id] : 0.0f;
     float sum = 0.0f;  // ((0 + s0) + s1) + ... in output order (route_policy.hpp:121-123)
-    for (u32 k = 0; k < p.top_k; ++k) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, my_s, k));
+#pragma unroll 1
+    for (u32 k0 = 0; k0 < p.top_k; k0 += 8) {  // eight values asked for at once
+        float v[8];
+#pragma unroll
+        for (u32 i = 0; i < 8; ++i) v[i] = __shfl_sync(0xffffffffu, my_s, k0 + i);
+#pragma unroll
+        for (u32 i = 0; i < 8; ++i) sum = k0 + i < p.top_k ? __fadd_rn(sum, v[i]) : sum;
+    }
     const bool renorm = p.renormalize && (p.top_k > 1 || p.renorm_single);
     const float den = __fadd_rn(sum, p.renorm_eps);
     if (lane < p.top_k) {
         ids[u64(row) * p.top_k + lane] = my_id;
-        if (ids_copy) ids_copy[row * p.top_k + lane] = my_id;
         weights[u64(row) * p.top_k + lane] = __fmul_rn(renorm ? __fdiv_rn(my_s, den) : my_s, p.scale);
     }
+    return my_id;
 }
 
-// One warp selects one row. `s` points to this warp's scratch of 2 * experts + 32 floats on a 16-byte boundary (shared memory).
+// One warp selects one row; select_row returns lane k's id in output order (lanes from top_k on: nothing of meaning). `s` points to this warp's scratch of 2 * experts + 32 floats on
+// a 16-byte boundary (shared memory).
 __host__ __device__ constexpr u32 scratch_floats(u32 experts) { return (2u * experts + 32u + 3u) & ~3u; }
-// MAXE: the most experts that the calling kernel sees.
-template <u32 MAXE>
-__device__ __forceinline__ void select_row(const float* logits, float* scores_out, const float* bias,
-                                           const b200moe_route_policy& p, u32 row, u32 lane, float* s,
-                                           u32* ids, float* weights, u32* ids_copy = nullptr) {
-    const u32 E = p.experts, run = E / p.n_group;
-    if (p.n_group == 1 || run % 32 == 0 || (run < 32 && (run & (run - 1u)) == 0)) {  // the fast path unless a NaN needs the serial rule
-        u32 my_id = kNone;
-        const bool done = E <= 128 ? select_row_fast<4>(logits, scores_out, bias, p, row, lane, s, &my_id)
-                        : MAXE <= 256 || E <= 256 ? select_row_fast<8>(logits, scores_out, bias, p, row, lane, s, &my_id)
-                                   : select_row_fast<MAXE <= 256 ? 8 : 32>(logits, scores_out, bias, p, row, lane, s, &my_id);
-        if (done) {
-            finish_row(p, row, lane, s, my_id, ids, weights, ids_copy);
-            return;
-        }
-        __syncwarp();
-    }
+// The general path of a row: any groups, any values (the serial rules where a NaN is among the choices). Out of line, so that a call's instructions lie in one piece: the kernels
+// run once a call on cold instruction caches, where every jump over code that is not run costs 500 to 1,000 clocks. Returns lane k's pick k.
+static __device__ __noinline__ u32 select_row_general(const float* logits, float* scores_out, const float* bias, const b200moe_route_policy& p, u32 row, u32 lane, float* s) {
+    const u32 E = p.experts;
     float* c = s + E;
     float* gs = c + E;
     const float* z = logits + u64(row) * E;
@@ -303,7 +307,22 @@ __device__ __forceinline__ void select_row(const float* logits, float* scores_ou
         const u32 pick = k_pass(p.key, c, E, lane, taken, allowed, per);
         if (lane == k) my_id = pick;
     }
-    finish_row(p, row, lane, s, my_id, ids, weights, ids_copy);
+    return my_id;
+}
+
+// EPL: a lane's experts on the fast path; 32 EPL is the most that the calling kernel sees.
+template <int EPL>
+__device__ __forceinline__ u32 select_row(const float* logits, float* scores_out, const float* bias,
+                                          const b200moe_route_policy& p, u32 row, u32 lane, float* s,
+                                          u32* ids, float* weights) {
+    const u32 run = p.experts / p.n_group;
+    u32 my_id = kNone;
+    // the fast path unless a NaN needs the serial rule
+    if (!((p.n_group == 1 || run % 32 == 0 || (run < 32 && (run & (run - 1u)) == 0)) && select_row_fast<EPL>(logits, scores_out, bias, p, row, lane, s, &my_id))) {
+        __syncwarp();
+        my_id = select_row_general(logits, scores_out, bias, p, row, lane, s);
+    }
+    return finish_row(p, row, lane, s, my_id, ids, weights);
 }
 
 

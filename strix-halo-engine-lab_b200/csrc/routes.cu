@@ -18,6 +18,7 @@ namespace b200moe {
 namespace {
 
 constexpr u32 kChunk = routes_detail::kChunk;
+constexpr u32 kFusedExperts = 256;  // of the launch that selects too
 
 using routes_detail::block_exclusive_scan;
 using routes_detail::entry_id;
@@ -44,20 +45,79 @@ __global__ void __launch_bounds__(32) routes_one_warp_kernel(b200moe_routes_view
 }
 
 // Decode windows: the router's selection (one warp per row) and the routes of the selected ids in ONE block, so the
-// layer prologue costs one launch less. Dynamic shared memory: the rows' selection scratch, then the routes' counts in its place. Up to 256 experts
-// (their keys fit the 64 registers that a block of 1024 threads has) and 8 rows in the form of 256 threads.
-template <u32 THREADS>
+// layer prologue costs one launch less. Up to 256 experts (their keys fit the 64 registers that a block of 1024 threads has) and 8 rows in the form of 256 threads.
+// What bounds it: a chain of latencies on cold instruction caches. A row's slots are ordered, checked and counted by its own warp, out of registers; the rows
+// of an expert are bits of one word (32 rows at most), so that an entry's place among its expert's is a count of bits and the rest one scan over the experts. With the
+// general build behind the selection (routes_small_body), and the selection's other paths between its steps, the kernel took 19,400 clocks behind its wait with 8 rows x 8 over 128
+// experts and 12,000 with 1 row, 10,100 and 4,450 of them the routes'; 9,800 and 9,500 now, 2,300 both. A call 49.6 -> 45.3 and 22.8 -> 21.4 us.
+template <u32 THREADS, int EPL>
 __global__ void __launch_bounds__(THREADS) select_routes_small_kernel(const float* logits, float* scores_out, const float* bias,
-                                                                      b200moe_route_policy p, u32 rows, u32* ids, float* weights,
+                                                                      const __grid_constant__ b200moe_route_policy p, u32 rows, u32* ids, float* weights,
                                                                       b200moe_routes_view rv, u32 end, Clear clear) {
     extern __shared__ __align__(16) float sel_smem[];
-    __shared__ u32 s_ids[kChunk];
-    const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    __shared__ u32 s_rows[kFusedExperts], s_begin[kFusedExperts], s_total[32], s_most[32];
+    const u32 t = threadIdx.x, lane = t & 31u, warp = t >> 5, E = rv.experts, K = rv.top_k;
+    for (u32 i = t; i < kFusedExperts; i += blockDim.x) s_rows[i] = 0u;
     chain_begin();
     routes_detail::clear_words(clear, rows);
-    if (warp < rows) select_detail::select_row<256>(logits, scores_out, bias, p, warp, lane, sel_smem + warp * select_detail::scratch_floats(p.experts), ids, weights, s_ids);
-    __syncthreads();  // the ids are read by the whole block
-    routes_small_body(rv, end, s_ids, reinterpret_cast<u16*>(sel_smem));
+    __syncthreads();  // the rows' status is cleared before it is set
+    u32 e = 0xffffffffu;  // the expert that the lane's slot is an entry of
+    if (warp < rows) {
+        const u32 id = select_detail::select_row<EPL>(logits, scores_out, bias, p, warp, lane, sel_smem + warp * select_detail::scratch_floats(p.experts), ids, weights);
+        u32 pos = 0;  // the slot's place in ascending expert id
+        bool bad = id >= E, repeats = false;
+#pragma unroll 1
+        for (u32 k0 = 0; k0 < K; k0 += 8) {
+            u32 o[8];
+#pragma unroll
+            for (u32 i = 0; i < 8; ++i) o[i] = __shfl_sync(0xffffffffu, id, k0 + i);
+#pragma unroll
+            for (u32 i = 0; i < 8; ++i) {
+                const u32 k = k0 + i;
+                const bool slot = k < K, same = slot && o[i] == id && k != lane, before = k < lane;
+                pos += (slot && o[i] < id) || (same && before) ? 1u : 0u;
+                bad |= same;
+                repeats |= same && before;
+            }
+        }
+        const u32 low = __popc(__ballot_sync(0xffffffffu, lane < K && id < rv.split));
+        if (lane < K) {
+            rv.out.order[warp * K + pos] = warp * K + lane;
+            if (lane == 0) rv.out.low_counts[warp] = low;
+            if (bad && rv.row_status) atomicOr(&rv.row_status[warp], B200MOE_ROW_INVALID_ROUTE);
+            if (!repeats && routes_detail::owned(id, E, rv.first, end)) {
+                e = id;
+                atomicOr(&s_rows[e], 1u << warp);
+            }
+        }
+    }
+    __syncthreads();
+    const u32 own = t < E ? s_rows[t] : 0u, c = __popc(own), sum = c + (c ? 0x10000u : 0u);  // entries, and experts that have some in the upper half
+    u32 upto = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { const u32 o = __shfl_up_sync(0xffffffffu, upto, d); if (lane >= (u32)d) upto += o; }
+    const u32 most = __reduce_max_sync(0xffffffffu, c);
+    if (lane == 31u) { s_total[warp] = upto; s_most[warp] = most; }
+    __syncthreads();
+    const u32 others = lane < blockDim.x / 32u ? s_total[lane] : 0u, total = __reduce_add_sync(0xffffffffu, others);
+    const u32 at = __reduce_add_sync(0xffffffffu, lane < warp ? others : 0u) + upto - sum, begin = at & 0xffffu, uidx = at >> 16;
+    if (t < E) {
+        s_begin[t] = begin;
+        if (c) { rv.out.experts[uidx] = t - rv.base; rv.out.begins[uidx + 1] = begin + c; }
+    }
+    if (warp == 0) {
+        const u32 maxc = __reduce_max_sync(0xffffffffu, lane < blockDim.x / 32u ? s_most[lane] : 0u);
+        if (lane == 0) {
+            rv.out.begins[0] = 0;
+            rv.out.counts[0] = total >> 16; rv.out.counts[1] = maxc; rv.out.counts[2] = total & 0xffffu; rv.out.counts[3] = 0;
+        }
+    }
+    __syncthreads();
+    if (e != 0xffffffffu) {
+        const u32 to = s_begin[e] + __popc(s_rows[e] & ((1u << warp) - 1u));
+        rv.out.rows[to] = warp;
+        rv.out.slots[to] = warp * K + lane;
+    }
 }
 
 // ---- chunked form --------------------------------------------------------------------------------------------------
@@ -169,13 +229,13 @@ u64 routes_scratch_words(u32 rows, u32 top_k, u32 experts) {
 u32 small_threads(u32 slots, u32 experts) { return std::min(1024u, std::max(256u, (std::max(slots, experts) + 31u) / 32u * 32u)); }
 
 bool select_routes_fusable(const b200moe_router_view& r, u32 top_k) {
-    return r.rows <= 32 && u64(r.rows) * top_k <= kChunk && r.policy.experts <= 256 && u64(r.rows) * select_detail::scratch_floats(r.policy.experts) * 4u <= 96u * 1024u;
+    return r.rows <= 32 && u64(r.rows) * top_k <= kChunk && r.policy.experts <= kFusedExperts && u64(r.rows) * select_detail::scratch_floats(r.policy.experts) * 4u <= 96u * 1024u;
 }
 int launch_select_routes(const b200moe_router_view& r, const b200moe_routes_view& v, const RoutesClear& clear, cudaStream_t stream) {
     if (r.rows == 0) return B200MOE_OK;
-    const u32 n = v.rows * v.top_k, smem = std::max(r.rows * select_detail::scratch_floats(r.policy.experts) * 4u, counts_bytes(n, v.experts));
-    const u32 threads = std::max(32u * r.rows, small_threads(n, v.experts));
-    const auto kernel = threads <= 256u ? select_routes_small_kernel<256> : select_routes_small_kernel<1024>;
+    const u32 smem = r.rows * select_detail::scratch_floats(r.policy.experts) * 4u, threads = std::max(32u * r.rows, 256u);  // a thread an expert
+    const bool few = r.policy.experts <= 128u;
+    const auto kernel = threads <= 256u ? (few ? select_routes_small_kernel<256, 4> : select_routes_small_kernel<256, 8>) : few ? select_routes_small_kernel<1024, 4> : select_routes_small_kernel<1024, 8>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
     small_launch(kernel, 1, threads, smem, stream, r.logits, r.scores, r.bias, r.policy, r.rows, r.ids, r.weights, v, v.end ? v.end : v.experts,
                  Clear{clear.row_status, clear.summary4, clear.summary});

@@ -1203,3 +1203,27 @@ def test_items_by_both_groups_of_a_block(gpu, oracle, rows, top_k, E, H, I):
     assert flags[0].item() & b200moe.JOB_WAIT_ABORTED
     with forced(b200moe.FORM_SEGMENT_STREAM):
         assert same(run()[2].cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("rows,top_k,experts,nan", [(1, 1, 1, False), (1, 8, 128, False), (8, 8, 129, False), (9, 9, 64, False), (5, 5, 5, False), (31, 3, 40, False), (32, 32, 256, False), (32, 8, 100, True)])
+def test_selection_and_routes_in_one_launch(gpu, oracle, rows, top_k, experts, nan):
+    """Windows of 1 to 32 rows over up to 256 experts: rows as bits of a word (the first and the last), every expert chosen by every row, fewer experts than a warp, slots beyond eight a row, and
+    rows whose NaN takes the serial rule. Both combine forms: one reads the routes' order."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + experts)
+    H, I = 256, 256
+    gate, up, down = synth.expert_tensors(rng, experts, H, I, 12, 12)
+    rw, bias = synth.router_weight(rng, experts, H), rng.standard_normal(experts).astype(np.float32)
+    if nan:
+        bias[3] = np.nan
+    x = rng.standard_normal((rows, H), dtype=np.float32)
+    for form in (O.COMBINE_PARTS, O.COMBINE_FMA_SLOTS):
+        parts = 2 if experts > 1 else 1
+        ffn = ops.MoeFfn(ops.make_shape(H, I, experts, top_k, 12, 12), ops.softmax_policy(experts, top_k), *(dv(a, gpu) for a in (gate, up, down, rw)), capacity=rows, combine_form=form,
+                         parts=parts, logit_bias=dv(bias, gpu))
+        y, ids, wts = ffn(dv(x, gpu), want_routes=True)
+        _, _, wi, ww = oracle.router(O.softmax_policy(experts, top_k), x=x, w=rw, logit_bias=bias)
+        assert np.array_equal(ids.cpu().numpy().view(np.uint32), wi) and same(wts.cpu(), ww)
+        layer = ops.MoeLayer(ops.make_shape(H, I, experts, top_k, 12, 12), *(dv(a, gpu) for a in (gate, up, down)), capacity=rows, combine_form=form, parts=parts)
+        assert same(y.cpu(), layer(ops.enqueue_quantize_a8(dv(x, gpu)), ids, wts).cpu())  # routes of a launch of their own

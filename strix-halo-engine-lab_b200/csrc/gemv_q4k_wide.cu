@@ -12,8 +12,8 @@
 //    claim word in device memory (wide_common.cuh).
 //  * A stage = S = 3 super-blocks of the item's 64 rows (one or two tiled TMA copies of 432 bytes x 32 / 64 rows: the rows
 //    lie 432 bytes apart in shared memory, an odd count of 16-byte units, which keeps the 128-bit reads of eight rows
-//    conflict free) PLUS the same K range of the A8 rows of the item's entries (codes, deltas, sums: gathering copies of four entries' rows each, untiled
-//    copies of an only entry's), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
+//    conflict free) PLUS the same K range of the A8 rows of the item's entries (codes, deltas, sums: tiled copies of a dense block's neighbouring
+//    rows, untiled copies of each entry's row otherwise), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
 //  * Two groups of eight consumer warps share a CTA, each with its own ring of stages and its own producer warp; a group's
 //    producer claims the next item of the grid while its consumers still work on the stages in the ring. The serial chains
 //    acc_p += pair_p never leave their lane.
@@ -63,6 +63,7 @@ struct WidePlan {
     u32 stages;         // ring depth per group
     u32 cap;            // entries that a stage holds: 1, 4 or 8
     u32 stage_bytes;
+    u32 boxes;          // the entries' A8 rows are neighbours and come by tiled copies (dense blocks)
     u32 pair;           // an item's stages are shared by the CTA's two groups
     u32 n_chunks;       // items per (virtual) expert
     u32 max_union;      // bound of the union
@@ -88,29 +89,27 @@ struct WideArgs {
     u32 raw_vec;           // raw lies on an 8-byte boundary
 };
 
-struct WideMaps { CUtensorMap w0, w1, codes, deltas, sums; };  // weight rows (up: w1), the entries' A8 rows
+struct WideMaps { CUtensorMap w0, w1, codes, deltas, sums; };  // weight rows (up: w1), a dense block's A8 rows
 
 // Stage geometry for S super-blocks per stage and CAP entries (1, 4 or 8), as compile-time constants: address arithmetic on run-time strides was a measurable
 // part of the instructions. Weight rows lie S * 144 bytes apart, S odd: an odd multiple of 4 (mod 32) words, so a warp's 128-bit reads of 8 rows and its
-// fragments' word reads are conflict free. The entries' A8 rows come in fours by gathering copies: the codes in two halves of the stage's columns (boxes that are
-// no wider than the shortest row: wider ones fault), the deltas, the sums. The codes' boxes hold 32 bytes more than the half, and the second four's begin 16 bytes
-// further to the left: eight entries' codes lie 4 (mod 32) words apart, so that a fragment's word reads meet every bank once.
+// fragments' word reads are conflict free. The entries' codes lie S * 256 + 16 bytes apart, 4 (mod 32) words: eight entries' word reads meet every bank once.
 template <u32 S_, u32 CAP_>
 struct Geo {
     static constexpr u32 S = S_, CAP = CAP_, fours = CAP == 8 ? 2u : 1u;
     static constexpr u32 row_bytes = S * kQ4KBlock, half_bytes = kHalfRows * row_bytes;
     static constexpr u32 w_bytes = 2 * half_bytes;
-    static constexpr u32 half_cols = S * 128, box_codes = half_cols + 32, box_group = S * 32;  // bytes of a box's rows
-    static constexpr u32 half_codes = 4 * box_codes, four_codes = 2 * half_codes, four_group = 4 * box_group;
-    static constexpr u32 off_deltas = CAP == 1 ? S * 256u : fours * four_codes, off_sums = off_deltas + (CAP == 1 ? box_group : fours * four_group);
-    static constexpr u32 x_bytes = off_sums + (CAP == 1 ? box_group : fours * four_group);
+    static constexpr u32 box_codes = CAP == 1 ? S * 256u : S * 256u + 16u, box_group = S * 32u;  // bytes of an entry's codes (with their gap), deltas, sums
+    static constexpr u32 off_deltas = (CAP * box_codes + 127u) / 128u * 128u, off_sums = off_deltas + CAP * box_group;
+    static constexpr u32 x_bytes = off_sums + CAP * box_group;
     static constexpr u32 stage_bytes = (w_bytes + x_bytes + 127u) / 128u * 128u;
-    static constexpr u32 four_tx = four_codes + 2 * four_group;  // bytes of a four's copies
-    __device__ static constexpr u32 codes_at(u32 e) { return (e & 3u) * box_codes + (e & 4u ? four_codes + 16u : 0u); }
-    __device__ static constexpr u32 column(u32 c) { return c + (c >= half_cols ? half_codes - half_cols : 0u); }  // behind codes_at
+    static constexpr u32 boxes_tx = CAP * (box_codes + 2u * box_group);  // what the tiled copies bring: whole boxes, what lies past the tensor is filled
 };
-static_assert(Geo<3, 8>::half_codes % 128 == 0 && Geo<1, 8>::half_codes % 128 == 0 && Geo<3, 8>::four_group % 128 == 0 && Geo<1, 8>::four_group % 128 == 0 &&
-              Geo<3, 8>::w_bytes % 128 == 0 && Geo<1, 8>::w_bytes % 128 == 0, "a tiled copy lands on 128 bytes");
+template <u32 S, u32 CAP> constexpr bool lands() {  // a tiled copy lands on 128 bytes
+    using G = Geo<S, CAP>;
+    return G::w_bytes % 128 == 0 && G::half_bytes % 128 == 0 && G::off_deltas % 128 == 0 && G::off_sums % 128 == 0 && G::stage_bytes % 128 == 0;
+}
+static_assert(lands<3, 8>() && lands<3, 4>() && lands<1, 8>() && lands<1, 4>());
 
 // (a0 + a1) + (a2 + a3) over the four pair lanes of a row (lane = 8 * p + row); every lane of the row gets the value.
 __device__ __forceinline__ float tree4(float a) {
@@ -196,14 +195,14 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
     }
     __syncwarp();
     const u32 rows = blk + g * G::row_bytes + 16u + 32u * p + 4u * t;
-    const u32 codes = xs + G::codes_at(MANY ? entry_of(g) : g & 3u) + 4u * t + 64u * p;
+    const u32 codes = xs + (MANY ? entry_of(g) : g & 3u) * G::box_codes + 4u * t + 64u * p;
     const u32 es = xs + G::off_deltas + (MANY ? t : 2u * (t & 1u)) * G::box_group + 8u * p;
     const bool second = t >= 2u;  // of the few form
     const u32 get = fac + 16u * g + (!MANY && second ? 256u : 0u);
 #pragma unroll
     for (u32 b = 0; b < S; ++b) {
         if (b >= nbk) break;
-        const u32 cb = codes + (G::column(256u * b + 64u * p) - 64u * p);
+        const u32 cb = codes + 256u * b;
         u32 a[2][4], bl[2], bh[2];
 #pragma unroll
         for (u32 j = 0; j < 2; ++j)
@@ -242,9 +241,6 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
 
 // 18 warps: two of the SM's four register partitions (16 K registers each) hold five warps, which caps a thread at
 // 16384 / (5 x 32) = 102 registers, 96 after rounding - what this launch bound gives (112 was tried: the launch is refused).
-// The entries' A8 rows by gathering copies: to ask for a stage's 24 bulk copies (8 entries) took a producer 1,690 clocks on its own and 1,880 beside the consumers,
-// whose work on the stage is 2,030 (64 rows of the large layer); a gathering copy of four rows 83. In a graph, us a call: large layer of 64 rows 720 -> 681, dense 5120 x 17408
-// 42.4 -> 39.6 (1 row) and 65.7 -> 61.8 (8).
 template <bool DOWN, u32 S_, u32 CAP_, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan) {
@@ -350,8 +346,10 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                 ve = table[jv];
             }
             const u32 ve_ne = ve.ne();
-            u32 mine = 0, r[8];  // the entries' A8 rows; in absent places the first one's
-            if (lane < 8u && !end) { const u32 at = ve.begin() + (lane < ve_ne ? lane : 0u); mine = plan.dense_rows ? at : load((DOWN ? a.routes.slots : a.routes.rows) + at); }
+            // Untiled copies: lane 3 e + part brings one part of entry e's row.
+            const u32 e = lane / 3u, part = lane - 3u * e;
+            u32 row = 0;
+            if (e < ve_ne && !end) { const u32 at = ve.begin() + e; row = plan.dense_rows ? at : load((DOWN ? a.routes.slots : a.routes.rows) + at); }
             const u32 nsegs = end ? 1u : my_segs;
             for (u32 i = 0; i < nsegs; ++i, ++t, ++slot) {
                 const u32 s = PAIR ? 2u * i + g : i;
@@ -367,33 +365,23 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                 }
                 const u32 nbk = min(G::S, plan.nb - s * G::S);
                 unsigned char* dst = g_stage + slot * plan.stage_bytes;
-                if (i == 0) {
-#pragma unroll
-                    for (u32 k = 0; k < 8; ++k) r[k] = k < G::CAP ? __shfl_sync(0xffffffffu, mine, k) : 0u;
-                }
                 if (lane == 0) {
                     g_item[slot] = item;
-                    const bool one = G::CAP == 1 || ve_ne == 1u;  // one entry's rows: untiled copies of what the stage has of them
-                    const bool both_halves = nbk * 256u > G::half_cols;
-                    const u32 four_tx = G::four_tx - (both_halves ? 0u : G::half_codes);
-                    mbar_expect_tx(&g_full[slot], (t < ahead ? 0u : G::w_bytes) + (one ? nbk * 320u : ve_ne > 4u ? 2u * four_tx : four_tx));  // whole boxes: what lies past a row is filled
+                    mbar_expect_tx(&g_full[slot], (t < ahead ? 0u : G::w_bytes) + (plan.boxes ? G::boxes_tx : ve_ne * nbk * 320u));
                     if (t >= ahead) ask_weights(s, ve, chunk, dst, &g_full[slot]);
-                    unsigned char* xd = dst + G::w_bytes;
-                    if (one) {
-                        bulk_g2s(xd, a.in.codes + u64(r[0]) * in_stride + u64(s) * G::S * 256u, nbk * 256u, &g_full[slot]);
-                        bulk_g2s(xd + G::off_deltas, a.in.deltas + u64(r[0]) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
-                        bulk_g2s(xd + G::off_sums, a.in.sums + u64(r[0]) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
-                    } else {
-                        auto ask_four = [&](unsigned char* codes, unsigned char* group, int left, u32 r0, u32 r1, u32 r2, u32 r3) {  // columns in 64-bit elements
-                            const int xc = static_cast<int>(s * (G::S * 32u)) - left, xg = static_cast<int>(s * (G::S * 4u));
-                            gather_4(codes, &maps.codes, xc, r0, r1, r2, r3, &g_full[slot]);
-                            if (both_halves) gather_4(codes + G::half_codes, &maps.codes, xc + static_cast<int>(G::half_cols / 8u), r0, r1, r2, r3, &g_full[slot]);
-                            gather_4(group, &maps.deltas, xg, r0, r1, r2, r3, &g_full[slot]);
-                            gather_4(group + (G::off_sums - G::off_deltas), &maps.sums, xg, r0, r1, r2, r3, &g_full[slot]);
-                        };
-                        ask_four(xd, xd + G::off_deltas, 0, r[0], r[1], r[2], r[3]);
-                        if (G::CAP == 8 && ve_ne > 4u) ask_four(xd + G::four_codes, xd + G::off_deltas + G::four_group, 2, r[4], r[5], r[6], r[7]);  // see Geo
+                }
+                __syncwarp();  // the bytes are expected
+                unsigned char* xd = dst + G::w_bytes;
+                if (plan.boxes) {
+                    if (lane == 0) {
+                        tma_2d(xd, &maps.codes, s * (G::S * 32u), ve.begin(), &g_full[slot]);  // 64-bit elements
+                        tma_2d(xd + G::off_deltas, &maps.deltas, s * (G::S * 4u), ve.begin(), &g_full[slot]);
+                        tma_2d(xd + G::off_sums, &maps.sums, s * (G::S * 4u), ve.begin(), &g_full[slot]);
                     }
+                } else if (e < ve_ne) {
+                    if (part == 0) bulk_g2s(xd + e * G::box_codes, a.in.codes + u64(row) * in_stride + u64(s) * G::S * 256u, nbk * 256u, &g_full[slot]);
+                    else if (part == 1) bulk_g2s(xd + G::off_deltas + e * G::box_group, a.in.deltas + u64(row) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
+                    else bulk_g2s(xd + G::off_sums + e * G::box_group, a.in.sums + u64(row) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
                 }
                 __syncwarp();
             }
@@ -612,16 +600,19 @@ bool a8_bulk_ok(const b200moe_a8_rows& x) {
     return x.sums && aligned(x.codes, 16) && aligned(x.deltas, 16) && aligned(x.sums, 16) && stride % 128 == 0;
 }
 
-// The tensor maps of the entries' A8 rows for copies of four rows at a time (unused where a stage holds one entry). Rows beyond the window's are not named by its
-// routes; a window has 8192 slots at most (make_plan), and the maps reach that far whatever its rows, so that a buffer keeps its maps.
-int entry_maps(const b200moe_a8_rows& x, u32 K, const WidePlan& p, WideMaps* m) {
+// The tensor maps of a dense block's A8 rows: exactly the window's rows. Rows shorter than a box come by untiled copies. Why boxes: to ask for one untiled copy takes a
+// producer 70 clocks, for 24 (8 entries) 1,690 of the 2,030 that its consumers work on the stage; three boxes are asked for by one lane. Dense 5120 x 17408, us a call, all
+// changes of the kernel together: 8 rows 66.1 -> 55.6, 1 row (three untiled copies a stage) 42.7 -> 37.5. Routed entries lie anywhere and keep the untiled copies: 64 rows of the
+// large layer 725 -> 719. Gathering copies of four rows were faster there (681) but raised an illegal memory access where the rows began a mapping: not understood, not used.
+int entry_maps(const b200moe_a8_rows& x, u32 K, WidePlan* p, WideMaps* m) {
     m->codes = m->deltas = m->sums = m->w0;
-    if (p.cap == 1) return B200MOE_OK;
+    const u32 codes = p->S * 256u + 16u, group = p->S * 32u;  // Geo::box_codes, box_group
+    p->boxes = p->dense_rows && p->cap > 1 && K >= codes;
+    if (!p->boxes) return B200MOE_OK;
     const u64 pitch = x.stride ? x.stride : x.width;
-    const u32 codes = p.S * 128u + 32u, group = p.S * 32u;  // Geo::box_codes, box_group: no wider than a row of S super-blocks
-    if (int rc = pitched_map(reinterpret_cast<const u8*>(x.codes), K, pitch, 8192, codes, 1, &m->codes)) return rc;
-    if (int rc = pitched_map(reinterpret_cast<const u8*>(x.deltas), K / 8, pitch / 8, 8192, group, 1, &m->deltas)) return rc;
-    return pitched_map(reinterpret_cast<const u8*>(x.sums), K / 8, pitch / 8, 8192, group, 1, &m->sums);
+    if (int rc = pitched_map(reinterpret_cast<const u8*>(x.codes), K, pitch, p->dense_rows, codes, p->cap, &m->codes)) return rc;
+    if (int rc = pitched_map(reinterpret_cast<const u8*>(x.deltas), K / 8, pitch / 8, p->dense_rows, group, p->cap, &m->deltas)) return rc;
+    return pitched_map(reinterpret_cast<const u8*>(x.sums), K / 8, pitch / 8, p->dense_rows, group, p->cap, &m->sums);
 }
 template <bool DOWN>
 int launch_wide(const WideMaps& m, const WideArgs& a, const WidePlan& p, cudaStream_t stream) {
@@ -667,7 +658,7 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const Chain
     const u64 rb = u64(p.nb) * kQ4KBlock, total_rows = u64(v.shape.experts) * v.shape.inter;
     if (int rc = rows_map(v.weights.gate, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &m.w0)) return rc;
     if (int rc = rows_map(v.weights.up, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &m.w1)) return rc;
-    if (int rc = entry_maps(v.x, v.shape.hidden, p, &m)) return rc;
+    if (int rc = entry_maps(v.x, v.shape.hidden, &p, &m)) return rc;
     return launch_wide<false>(m, a, p, stream);
 }
 
@@ -685,7 +676,7 @@ int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints&
     const u64 rb = u64(p.nb) * kQ4KBlock;
     if (int rc = rows_map(v.weights.down, rb, u64(v.shape.experts) * v.shape.hidden, p.S * kQ4KBlock, kHalfRows, &m.w0)) return rc;
     m.w1 = m.w0;
-    if (int rc = entry_maps(v.act, v.shape.inter, p, &m)) return rc;
+    if (int rc = entry_maps(v.act, v.shape.inter, &p, &m)) return rc;
     return launch_wide<true>(m, a, p, stream);
 }
 

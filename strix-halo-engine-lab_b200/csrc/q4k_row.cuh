@@ -68,12 +68,6 @@ __device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, u32 x,
                  "l"(reinterpret_cast<u64>(map)), "r"(x), "r"(y), "r"(saddr(bar))
                  : "memory");
 }
-// The boxes (one row high) of four rows of a 2-D tensor map at column x, one behind the other in shared memory. x may lie outside the row: zeros.
-__device__ __forceinline__ void gather_4(void* dst, const CUtensorMap* map, int x, u32 y0, u32 y1, u32 y2, u32 y3, u64* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(saddr(dst)),
-                 "l"(reinterpret_cast<u64>(map)), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3), "r"(saddr(bar))
-                 : "memory");
-}
 __device__ __forceinline__ int dp4a_us(u32 a, u32 b, int c) {  // unsigned bytes of a times signed bytes of b
     int d;
     asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));

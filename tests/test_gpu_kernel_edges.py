@@ -1227,3 +1227,40 @@ def test_selection_and_routes_in_one_launch(gpu, oracle, rows, top_k, experts, n
         assert np.array_equal(ids.cpu().numpy().view(np.uint32), wi) and same(wts.cpu(), ww)
         layer = ops.MoeLayer(ops.make_shape(H, I, experts, top_k, 12, 12), *(dv(a, gpu) for a in (gate, up, down)), capacity=rows, combine_form=form, parts=parts)
         assert same(y.cpu(), layer(ops.enqueue_quantize_a8(dv(x, gpu)), ids, wts).cpu())  # routes of a launch of their own
+
+
+@pytest.mark.parametrize("H,I", [(512, 256), (768, 512), (1024, 768), (2560, 1280)])
+@pytest.mark.parametrize("at_end", [False, True])
+def test_segment_streaming_rows_at_the_ends_of_their_memory(gpu, oracle, H, I, at_end):
+    """Activations that begin where an allocation begins, or end where it ends: experts of 2 to 9 entries that hold the first and the last row, rows of whole and broken stages. Nothing beside
+    them is touched."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(H)
+    E, rows, size = 8, 40, 32 << 20
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, 12)
+    ids = np.zeros((rows, 2), np.uint32)
+    ids[:, 0] = rng.integers(4, 8, rows)
+    ids[:, 1] = rng.integers(0, 4, rows)
+    ids[0], ids[rows - 1] = (5, 1), (6, 1)
+    for e, n in ((0, 5), (1, 7), (2, 6)):  # the first and the last row in items of 5 to 7
+        ids[:, 1] = np.where(ids[:, 1] == e, 3, ids[:, 1])
+        ids[np.linspace(0, rows - 1, n).astype(int) if e == 1 else 1 + e + 4 * np.arange(n), 1] = e
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 2, 12, 12, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+
+    def place(a, dtype):
+        flat = torch.empty(size, dtype=torch.uint8, device=gpu)
+        n = a.size * a.itemsize
+        t = (flat[size - n:] if at_end else flat[:n]).view(dtype).view(a.shape)
+        t.copy_(torch.from_numpy(np.ascontiguousarray(a)))
+        return t
+
+    sh, r = ops.make_shape(H, I, E, 2, 12, 12), ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E // 2)
+    with forced(b200moe.FORM_SEGMENT_STREAM):
+        act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (place(codes, torch.int8), place(deltas, torch.float32), place(sums, torch.int32)), rows * 2, taps=True)
+        assert b200moe.last_launch() == "gate_up_q4k_wide"
+        act = tuple(place(t.cpu().numpy(), t.dtype) for t in act)
+        raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+        assert b200moe.last_launch() == "down_q4k_wide"
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])

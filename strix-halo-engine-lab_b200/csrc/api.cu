@@ -355,7 +355,12 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
             default: return launch_gate_up_q8(v, st);
         }
     }
-    if (v.shape.gate_type == B200MOE_TYPE_Q5_K) return launch_gate_up_q4k(v, st);  // the per-block form reads both K-quant layouts
+    // Q5_K: the segment-streaming and the per-block form read both K-quant layouts. The first wherever it fits; us a layer call, per-block form and this: 1 row of 2560 -> 768
+    // 36.2 and 27.2 (1024 -> 512: 22.8 and 21.8), 24 rows of 2560 -> 1024 228 and 120, 100 rows of 2560 -> 768 457 and 166, 400 rows of 2048 -> 544 1697 and 589.
+    if (v.shape.gate_type == B200MOE_TYPE_Q5_K) {
+        const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
+        return (forced == 0 || forced == 2) && wide_gate_up_fits(v, rows) ? launch_gate_up_q4k_wide(v, rows, hints, st) : launch_gate_up_q4k(v, st);
+    }
     switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.x.sums != nullptr), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, v.max_union, grouped_min_rows, hints.slots == 0, false)) {
         case Q4Form::grouped: return launch_gate_up_q4k_grouped(v, st);
         case Q4Form::row_stream: return launch_gate_up_q4k_stream(v, rows, st);

@@ -92,12 +92,13 @@ struct WideArgs {
 struct WideMaps { CUtensorMap w0, w1, codes, deltas, sums; };  // weight rows (up: w1), a dense block's A8 rows
 
 // Stage geometry for S super-blocks per stage and CAP entries (1, 4 or 8), as compile-time constants: address arithmetic on run-time strides was a measurable
-// part of the instructions. Weight rows lie S * 144 bytes apart, S odd: an odd multiple of 4 (mod 32) words, so a warp's 128-bit reads of 8 rows and its
+// part of the instructions. Weight rows lie S * 144 (Q5_K: 176) bytes apart, S odd: an odd multiple of 4 (mod 32) words, so a warp's 128-bit reads of 8 rows and its
 // fragments' word reads are conflict free. The entries' codes lie S * 256 + 16 bytes apart, 4 (mod 32) words: eight entries' word reads meet every bank once.
-template <u32 S_, u32 CAP_>
+template <u32 S_, u32 CAP_, bool Q5K_ = false>
 struct Geo {
-    static constexpr u32 S = S_, CAP = CAP_, fours = CAP == 8 ? 2u : 1u;
-    static constexpr u32 row_bytes = S * kQ4KBlock, half_bytes = kHalfRows * row_bytes;
+    static constexpr bool Q5K = Q5K_;  // 32 bytes of fifth bits lie between a super-block's header and its nibbles
+    static constexpr u32 S = S_, CAP = CAP_, block = Q5K ? kQ5KBlock : kQ4KBlock, nibbles = Q5K ? 48u : 16u;
+    static constexpr u32 row_bytes = S * block, half_bytes = kHalfRows * row_bytes;
     static constexpr u32 w_bytes = 2 * half_bytes;
     static constexpr u32 box_codes = CAP == 1 ? S * 256u : S * 256u + 16u, box_group = S * 32u;  // bytes of an entry's codes (with their gap), deltas, sums
     static constexpr u32 off_deltas = (CAP * box_codes + 127u) / 128u * 128u, off_sums = off_deltas + CAP * box_group;
@@ -105,11 +106,12 @@ struct Geo {
     static constexpr u32 stage_bytes = (w_bytes + x_bytes + 127u) / 128u * 128u;
     static constexpr u32 boxes_tx = CAP * (box_codes + 2u * box_group);  // what the tiled copies bring: whole boxes, what lies past the tensor is filled
 };
-template <u32 S, u32 CAP> constexpr bool lands() {  // a tiled copy lands on 128 bytes
-    using G = Geo<S, CAP>;
+template <u32 S, u32 CAP, bool Q5K> constexpr bool lands() {  // a tiled copy lands on 128 bytes
+    using G = Geo<S, CAP, Q5K>;
     return G::w_bytes % 128 == 0 && G::half_bytes % 128 == 0 && G::off_deltas % 128 == 0 && G::off_sums % 128 == 0 && G::stage_bytes % 128 == 0;
 }
-static_assert(lands<3, 8>() && lands<3, 4>() && lands<1, 8>() && lands<1, 4>());
+static_assert(lands<3, 8, false>() && lands<3, 4, false>() && lands<1, 8, false>() && lands<1, 4, false>());
+static_assert(lands<3, 8, true>() && lands<3, 4, true>() && lands<1, 8, true>() && lands<1, 4, true>());
 
 // (a0 + a1) + (a2 + a3) over the four pair lanes of a row (lane = 8 * p + row); every lane of the row gets the value.
 __device__ __forceinline__ float tree4(float a) {
@@ -117,8 +119,9 @@ __device__ __forceinline__ float tree4(float a) {
     return __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 16));
 }
 
-// Decoded factors of one super-block for pair p as the chains use them: D of the even group, D / 16 of the odd one (the high nibbles stay in
-// place: their dots come as 16 * dot), and -DM of both. A scale's byte goes behind the exponent of 2^23, less 2^23.
+// Decoded factors of one super-block for pair p as the chains use them: D of the even group, D of the odd one - of Q4_K D / 16, whose high nibbles stay in
+// place: their dots come as 16 * dot -, and -DM of both. A scale's byte goes behind the exponent of 2^23, less 2^23.
+template <bool Q5K>
 __device__ __forceinline__ float4 pair_factors(const uint4& hdr, u32 p) {
     const float d = half_bits_to_float(hdr.x & 0xffffu), dm = half_bits_to_float(hdr.x >> 16);
     const u32 sel = 0x7440u + 2u * (p & 1u);
@@ -126,7 +129,7 @@ __device__ __forceinline__ float4 pair_factors(const uint4& hdr, u32 p) {
     if (p < 2u) { sc = hdr.y & 0x3f3f3f3fu; mn = hdr.z & 0x3f3f3f3fu; }
     else { sc = (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u); mn = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u); }
     auto two = [&](u32 w, u32 base) { return make_float2(__uint_as_float(__byte_perm(w, base, sel)), __uint_as_float(__byte_perm(w, base, sel + 1u))); };
-    const float2 D = mul2(make_float2(d, __fmul_rn(d, 0.0625f)), add2(two(sc, 0x4b000000u), both(-8388608.0f)));
+    const float2 D = mul2(make_float2(d, Q5K ? d : __fmul_rn(d, 0.0625f)), add2(two(sc, 0x4b000000u), both(-8388608.0f)));
     const float2 M = mul2(both(dm), add2(two(mn, 0xcb000000u), both(8388608.0f)));
     return make_float4(D.x, D.y, M.x, M.y);
 }
@@ -143,18 +146,27 @@ __device__ __forceinline__ float pair_term(const float4& f, int2 dot, float2 E, 
     return __fadd_rn(x.x, x.y);
 }
 
+// Bit j of the four bytes of a word of high bits as bit 4 of four quants.
+__device__ __forceinline__ u32 fifth_bits(u32 h, u32 j) { return ((h >> j) << 4) & 0x10101010u; }
+
 // One stage of one weight row (this lane's pair p of nbk super-blocks, ascending) against one staged A8 row. blk: the row's first
 // super-block of the stage; xs: the stage's A8 rows, of which the first is meant.
 template <class G, class Put>
 __device__ __forceinline__ void stage_row(u32 blk, u32 nbk, u32 p, u32 xs, Put put_term) {
     constexpr u32 S = G::S;
-    const u32 q = blk + 16u + 32u * p, cs = xs + 64u * p, es = xs + G::off_deltas + 8u * p;
+    const u32 q = blk + G::nibbles + 32u * p, cs = xs + 64u * p, es = xs + G::off_deltas + 8u * p;
 #pragma unroll
     for (u32 b = 0; b < S; ++b) {
         if (b >= nbk) break;
-        const uint4 hdr = lds128(blk + b * kQ4KBlock), q0 = lds128(q + b * kQ4KBlock), q1 = lds128(q + b * kQ4KBlock + 16u);
-        const float4 f = pair_factors(hdr, p);
-        const Nibbles n = split_nibbles(q0, q1);
+        const uint4 hdr = lds128(blk + b * G::block), q0 = lds128(q + b * G::block), q1 = lds128(q + b * G::block + 16u);
+        const float4 f = pair_factors<G::Q5K>(hdr, p);
+        Nibbles n = split_nibbles(q0, q1);
+        if (G::Q5K) {
+            const uint4 h0 = lds128(blk + b * G::block + 16u), h1 = lds128(blk + b * G::block + 32u);
+            const u32 h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { n.lo[i] |= fifth_bits(h[i], 2u * p); n.hi[i] = (n.hi[i] >> 4) | fifth_bits(h[i], 2u * p + 1u); }
+        }
         const uint4 c0 = lds128(cs + 256u * b), c1 = lds128(cs + 256u * b + 16u), c2 = lds128(cs + 256u * b + 32u), c3 = lds128(cs + 256u * b + 48u);
         const uint2 d = lds64(es + 32u * b), m = lds64(es + (G::off_sums - G::off_deltas) + 32u * b);
         int l, h;
@@ -165,10 +177,9 @@ __device__ __forceinline__ void stage_row(u32 blk, u32 nbk, u32 p, u32 xs, Put p
 // ---- the mma form of one stage ---------------------------------------------------------------------------------------
 // 16 weight rows x 8 entries x one group: unsigned nibble bytes times signed codes. d[0], d[1]: row lane / 4, entries 2 (lane % 4) and the next; d[2],
 // d[3]: row lane / 4 + 8.
-__device__ __forceinline__ void mma_u8s8(int (&d)[4], const u32 (&a)[4], u32 mask, u32 b0, u32 b1) {
+__device__ __forceinline__ void mma_u8s8(int (&d)[4], const u32 (&a)[4], u32 b0, u32 b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-        : "r"(a[0] & mask), "r"(a[1] & mask), "r"(a[2] & mask), "r"(a[3] & mask), "r"(b0), "r"(b1), "r"(0));
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
 }
 // The entry of MMA column c where the columns hold eight: a lane's two cells are entries t and t + 4, so that four lanes' reads of deltas and sums meet every bank once.
 __device__ __forceinline__ u32 entry_of(u32 c) { return (c >> 1) + 4u * (c & 1u); }
@@ -191,10 +202,10 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
 #pragma unroll
     for (u32 b = 0; b < S; ++b) {  // the factors, lane = row
         if (b >= nbk) break;
-        sts128(put + b * (kHalfRows * 16u), pair_factors(lds128(head + b * kQ4KBlock), p));
+        sts128(put + b * (kHalfRows * 16u), pair_factors<G::Q5K>(lds128(head + b * G::block), p));
     }
     __syncwarp();
-    const u32 rows = blk + g * G::row_bytes + 16u + 32u * p + 4u * t;
+    const u32 rows = blk + g * G::row_bytes + G::nibbles + 32u * p + 4u * t, high = blk + g * G::row_bytes + 16u + 4u * t;
     const u32 codes = xs + (MANY ? entry_of(g) : g & 3u) * G::box_codes + 4u * t + 64u * p;
     const u32 es = xs + G::off_deltas + (MANY ? t : 2u * (t & 1u)) * G::box_group + 8u * p;
     const bool second = t >= 2u;  // of the few form
@@ -203,11 +214,20 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
     for (u32 b = 0; b < S; ++b) {
         if (b >= nbk) break;
         const u32 cb = codes + 256u * b;
-        u32 a[2][4], bl[2], bh[2];
+        u32 lo[2][4], hi[2][4], bl[2], bh[2];
 #pragma unroll
         for (u32 j = 0; j < 2; ++j)
 #pragma unroll
-            for (u32 i = 0; i < 4; ++i) a[j][i] = lds32(rows + b * kQ4KBlock + (16u * j + 8u * (i & 1u)) * G::row_bytes + 16u * (i >> 1));
+            for (u32 i = 0; i < 4; ++i) {
+                const u32 at = b * G::block + (16u * j + 8u * (i & 1u)) * G::row_bytes + 16u * (i >> 1), q = lds32(rows + at);
+                lo[j][i] = q & 0x0f0f0f0fu;
+                hi[j][i] = q & 0xf0f0f0f0u;
+                if (G::Q5K) {
+                    const u32 h = lds32(high + at);
+                    lo[j][i] |= fifth_bits(h, 2u * p);
+                    hi[j][i] = (hi[j][i] >> 4) | fifth_bits(h, 2u * p + 1u);
+                }
+            }
 #pragma unroll
         for (u32 i = 0; i < 2; ++i) { bl[i] = lds32(cb + 16u * i); bh[i] = lds32(cb + 32u + 16u * i); }
         float2 E[2], Sg[2];
@@ -220,8 +240,8 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
         int l[2][4], h[2][4];
 #pragma unroll
         for (u32 j = 0; j < 2; ++j) {
-            mma_u8s8(l[j], a[j], 0x0f0f0f0fu, bl[0], bl[1]);
-            mma_u8s8(h[j], a[j], 0xf0f0f0f0u, bh[0], bh[1]);
+            mma_u8s8(l[j], lo[j], bl[0], bl[1]);
+            mma_u8s8(h[j], hi[j], bh[0], bh[1]);
         }
         if (!MANY) {
 #pragma unroll
@@ -241,10 +261,10 @@ __device__ __forceinline__ void stage_rows_mma(u32 blk, u32 nbk, u32 p, u32 lane
 
 // 18 warps: two of the SM's four register partitions (16 K registers each) hold five warps, which caps a thread at
 // 16384 / (5 x 32) = 102 registers, 96 after rounding - what this launch bound gives (112 was tried: the launch is refused).
-template <bool DOWN, u32 S_, u32 CAP_, bool PAIR>
+template <bool DOWN, u32 S_, u32 CAP_, bool PAIR, bool Q5K>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan) {
-    using G = Geo<S_, CAP_>;
+    using G = Geo<S_, CAP_, Q5K>;
     extern __shared__ __align__(128) unsigned char smem[];
     // An early launch makes its list and asks for the weights of its groups' first items before it waits for the launch in front. Every path waits.
     const bool early = plan.early;
@@ -300,7 +320,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         u32 t = 0, slot = 0, use = 0;  // stage count, ring position, lap
         bool ok = true;
         auto ask_weights = [&](u32 s, const VExpert& ve, u32 chunk, unsigned char* dst, u64* bar) {  // one lane
-            const u32 x = s * G::S * (kQ4KBlock / 8);  // 64-bit elements: a multiple of 18, i.e. of 144 bytes
+            const u32 x = s * G::S * (G::block / 8);  // 64-bit elements: a multiple of 18 or 22, i.e. of 144 or 176 bytes
             const u32 y = ve.expert() * a.rows_per_expert + (DOWN ? kItemRows : kHalfRows) * chunk;
             tma_2d(dst, &maps.w0, x, y, bar);
             tma_2d(dst + G::half_bytes, &maps.w1, x, DOWN ? y + kHalfRows : y, bar);
@@ -567,7 +587,7 @@ u32 fixed_smem(const WidePlan& p) {
 u32 plan_smem(const WidePlan& p) { return kGroups * p.stages * p.stage_bytes + fixed_smem(p); }
 
 // K: the row length; n_chunks: items per expert; slots: rows * top_k of the window. False when the form does not apply.
-bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, WidePlan* p) {
+bool make_plan(bool q5k, u32 K, u32 n_chunks, u32 max_union, u64 slots, WidePlan* p) {
     if (K == 0 || K % 256 || max_union == 0 || slots == 0 || slots > 8192) return false;
     p->nb = K / 256;
     p->S = p->nb >= 3 ? 3u : 1u;  // odd: see Geo
@@ -575,8 +595,9 @@ bool make_plan(u32 K, u32 n_chunks, u32 max_union, u64 slots, WidePlan* p) {
     // a stage holds the A8 segments of as many entries as a virtual expert of this window can have: windows of fewer than
     // kKE slots get smaller stages and with them a deeper ring
     p->cap = slots == 1 ? 1u : slots <= 4 ? 4u : 8u;
-    p->stage_bytes = p->S == 3 ? (p->cap == 1 ? Geo<3, 1>::stage_bytes : p->cap == 4 ? Geo<3, 4>::stage_bytes : Geo<3, 8>::stage_bytes)
-                               : (p->cap == 1 ? Geo<1, 1>::stage_bytes : p->cap == 4 ? Geo<1, 4>::stage_bytes : Geo<1, 8>::stage_bytes);
+    auto bytes = [&](auto s3, auto s1) { return p->S == 3 ? decltype(s3)::stage_bytes : decltype(s1)::stage_bytes; };
+    if (q5k) p->stage_bytes = p->cap == 1 ? bytes(Geo<3, 1, true>{}, Geo<1, 1, true>{}) : p->cap == 4 ? bytes(Geo<3, 4, true>{}, Geo<1, 4, true>{}) : bytes(Geo<3, 8, true>{}, Geo<1, 8, true>{});
+    else p->stage_bytes = p->cap == 1 ? bytes(Geo<3, 1>{}, Geo<1, 1>{}) : p->cap == 4 ? bytes(Geo<3, 4>{}, Geo<1, 4>{}) : bytes(Geo<3, 8>{}, Geo<1, 8>{});
     p->n_chunks = n_chunks;
     p->max_union = max_union;
     p->vmax = max_union + static_cast<u32>(slots / kKE) + 1;
@@ -614,11 +635,11 @@ int entry_maps(const b200moe_a8_rows& x, u32 K, WidePlan* p, WideMaps* m) {
     if (int rc = pitched_map(reinterpret_cast<const u8*>(x.deltas), K / 8, pitch / 8, p->dense_rows, group, p->cap, &m->deltas)) return rc;
     return pitched_map(reinterpret_cast<const u8*>(x.sums), K / 8, pitch / 8, p->dense_rows, group, p->cap, &m->sums);
 }
-template <bool DOWN>
+template <bool DOWN, bool Q5K>
 int launch_wide(const WideMaps& m, const WideArgs& a, const WidePlan& p, cudaStream_t stream) {
-    const auto kernel = p.pair ? (p.cap == 1 ? q4k_wide_kernel<DOWN, 3, 1, true> : p.cap == 4 ? q4k_wide_kernel<DOWN, 3, 4, true> : q4k_wide_kernel<DOWN, 3, 8, true>)
-                        : p.S == 3 ? (p.cap == 1 ? q4k_wide_kernel<DOWN, 3, 1, false> : p.cap == 4 ? q4k_wide_kernel<DOWN, 3, 4, false> : q4k_wide_kernel<DOWN, 3, 8, false>)
-                                   : (p.cap == 1 ? q4k_wide_kernel<DOWN, 1, 1, false> : p.cap == 4 ? q4k_wide_kernel<DOWN, 1, 4, false> : q4k_wide_kernel<DOWN, 1, 8, false>);
+    const auto kernel = p.pair ? (p.cap == 1 ? q4k_wide_kernel<DOWN, 3, 1, true, Q5K> : p.cap == 4 ? q4k_wide_kernel<DOWN, 3, 4, true, Q5K> : q4k_wide_kernel<DOWN, 3, 8, true, Q5K>)
+                        : p.S == 3 ? (p.cap == 1 ? q4k_wide_kernel<DOWN, 3, 1, false, Q5K> : p.cap == 4 ? q4k_wide_kernel<DOWN, 3, 4, false, Q5K> : q4k_wide_kernel<DOWN, 3, 8, false, Q5K>)
+                                   : (p.cap == 1 ? q4k_wide_kernel<DOWN, 1, 1, false, Q5K> : p.cap == 4 ? q4k_wide_kernel<DOWN, 1, 4, false, Q5K> : q4k_wide_kernel<DOWN, 1, 8, false, Q5K>);
     const u32 smem = plan_smem(p);
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
     chain_launch(kernel, device_sm_count(), kThreads, smem, stream, m, a, p);
@@ -635,19 +656,20 @@ void apply_hooks(WidePlan* p) {
 
 bool wide_gate_up_fits(const b200moe_gate_up_view& v, u32 rows) {
     WidePlan p{};
-    return v.shape.gate_type == B200MOE_TYPE_Q4_K && rows && a8_bulk_ok(v.x) && v.shape.inter % 32 == 0 &&
-           make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, &p);
+    return is_kquant(v.shape.gate_type) && rows && a8_bulk_ok(v.x) && v.shape.inter % 32 == 0 &&
+           make_plan(v.shape.gate_type == B200MOE_TYPE_Q5_K, v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, &p);
 }
 bool wide_down_fits(const b200moe_down_view& v, u32 rows) {
     WidePlan p{};
     return v.shape.down_type == B200MOE_TYPE_Q4_K && rows && a8_bulk_ok(v.act) && v.shape.hidden % 64 == 0 &&
-           make_plan(v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, &p);
+           make_plan(false, v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, &p);
 }
 
 int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     WidePlan p{};
-    if (!make_plan(v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, &p))
+    const bool q5k = v.shape.gate_type == B200MOE_TYPE_Q5_K;
+    if (!make_plan(q5k, v.shape.hidden, v.shape.inter / 32, v.max_union, u64(rows) * v.shape.top_k, &p))
         return fail(B200MOE_ERR_UNSUPPORTED, "gate_up: the segment-streaming form does not apply to this shape");
     apply_hooks(&p);
     p.early = hints.routes_done || hints.dense_rows; p.dense_rows = hints.dense_rows; p.n_bound = static_cast<u32>(std::min<u64>(v.max_union, hints.slots));
@@ -655,17 +677,18 @@ int launch_gate_up_q4k_wide(const b200moe_gate_up_view& v, u32 rows, const Chain
     a.routes = v.routes; a.in = v.x; a.act = v.act; a.gate_out = v.gate_out; a.up_out = v.up_out;
     a.row_status = v.row_status; a.summary = v.summary; a.rows_per_expert = v.shape.inter; a.out_width = v.shape.inter;
     WideMaps m;
-    const u64 rb = u64(p.nb) * kQ4KBlock, total_rows = u64(v.shape.experts) * v.shape.inter;
-    if (int rc = rows_map(v.weights.gate, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &m.w0)) return rc;
-    if (int rc = rows_map(v.weights.up, rb, total_rows, p.S * kQ4KBlock, kHalfRows, &m.w1)) return rc;
+    const u32 block = q5k ? kQ5KBlock : kQ4KBlock;
+    const u64 rb = u64(p.nb) * block, total_rows = u64(v.shape.experts) * v.shape.inter;
+    if (int rc = rows_map(v.weights.gate, rb, total_rows, p.S * block, kHalfRows, &m.w0)) return rc;
+    if (int rc = rows_map(v.weights.up, rb, total_rows, p.S * block, kHalfRows, &m.w1)) return rc;
     if (int rc = entry_maps(v.x, v.shape.hidden, &p, &m)) return rc;
-    return launch_wide<false>(m, a, p, stream);
+    return q5k ? launch_wide<false, true>(m, a, p, stream) : launch_wide<false, false>(m, a, p, stream);
 }
 
 int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream) {
     if (v.max_union == 0) return B200MOE_OK;
     WidePlan p{};
-    if (!make_plan(v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, &p))
+    if (!make_plan(false, v.shape.inter, v.shape.hidden / 64, v.max_union, u64(rows) * v.shape.top_k, &p))
         return fail(B200MOE_ERR_UNSUPPORTED, "down: the segment-streaming form does not apply to this shape");
     apply_hooks(&p);
     p.early = hints.routes_done || hints.dense_rows; p.dense_rows = hints.dense_rows; p.n_bound = static_cast<u32>(std::min<u64>(v.max_union, hints.slots));
@@ -677,7 +700,7 @@ int launch_down_q4k_wide(const b200moe_down_view& v, u32 rows, const ChainHints&
     if (int rc = rows_map(v.weights.down, rb, u64(v.shape.experts) * v.shape.hidden, p.S * kQ4KBlock, kHalfRows, &m.w0)) return rc;
     m.w1 = m.w0;
     if (int rc = entry_maps(v.act, v.shape.inter, &p, &m)) return rc;
-    return launch_wide<true>(m, a, p, stream);
+    return launch_wide<true, false>(m, a, p, stream);
 }
 
 }  // namespace b200moe

@@ -1264,3 +1264,19 @@ def test_segment_streaming_rows_at_the_ends_of_their_memory(gpu, oracle, H, I, a
         raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
         assert b200moe.last_launch() == "down_q4k_wide"
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("H,I,E,rows,top", [(256, 96, 3, 1, 1), (512, 64, 4, 3, 1), (768, 96, 3, 1, 1), (1024, 64, 4, 4, 1), (1280, 160, 2, 9, 2), (2560, 768, 6, 2, 2), (2560, 544, 5, 41, 3)])
+def test_segment_streaming_q5_k(gpu, oracle, H, I, E, rows, top):
+    """Q5_K gate / up: stages of one and three super-blocks (whole and broken), experts of one, of few and of many entries, items of one group and of both."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(H + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 13, 8)
+    ids = np.stack([rng.permutation(E)[:top] for _ in range(rows)]).astype(np.uint32)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top, 13, 8, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh, r = ops.make_shape(H, I, E, top, 13, 8), ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, min(E, rows * top))
+    _, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, min(E, rows * top), tuple(dv(t, gpu) for t in (codes, deltas, sums)), rows * top, taps=True)
+    assert b200moe.last_launch() == "gate_up_q4k_wide"
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])

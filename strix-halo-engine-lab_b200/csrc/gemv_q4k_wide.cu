@@ -13,7 +13,7 @@
 //  * A stage = S = 3 super-blocks of the item's 64 rows (one or two tiled TMA copies of 432 bytes x 32 / 64 rows: the rows
 //    lie 432 bytes apart in shared memory, an odd count of 16-byte units, which keeps the 128-bit reads of eight rows
 //    conflict free) PLUS the same K range of the A8 rows of the item's entries (codes, deltas, sums: tiled copies of a dense block's neighbouring
-//    rows, untiled copies of each entry's row otherwise), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
+//    rows; otherwise an untiled copy of each entry's codes and 16-byte asynchronous copies of the deltas and sums), all counted on one mbarrier. The consumers therefore find everything a stage needs in shared memory.
 //  * Two groups of eight consumer warps share a CTA, each with its own ring of stages and its own producer warp; a group's
 //    producer claims the next item of the grid while its consumers still work on the stages in the ring. The serial chains
 //    acc_p += pair_p never leave their lane.
@@ -317,6 +317,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
         u32* g_item = slot_item + g * plan.stages;
         unsigned char* g_stage = smem + g * plan.stages * plan.stage_bytes;
         const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, in_gs = in_stride / 32;
+        const u32 e = lane >> 2, part = lane & 3u;  // entries that lie anywhere: four lanes an entry, the first for the codes, two each for the deltas and the sums
         u32 t = 0, slot = 0, use = 0;  // stage count, ring position, lap
         bool ok = true;
         auto ask_weights = [&](u32 s, const VExpert& ve, u32 chunk, unsigned char* dst, u64* bar) {  // one lane
@@ -366,8 +367,6 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                 ve = table[jv];
             }
             const u32 ve_ne = ve.ne();
-            // Untiled copies: lane 3 e + part brings one part of entry e's row.
-            const u32 e = lane / 3u, part = lane - 3u * e;
             u32 row = 0;
             if (e < ve_ne && !end) { const u32 at = ve.begin() + e; row = plan.dense_rows ? at : load((DOWN ? a.routes.slots : a.routes.rows) + at); }
             const u32 nsegs = end ? 1u : my_segs;
@@ -387,7 +386,7 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                 unsigned char* dst = g_stage + slot * plan.stage_bytes;
                 if (lane == 0) {
                     g_item[slot] = item;
-                    mbar_expect_tx(&g_full[slot], (t < ahead ? 0u : G::w_bytes) + (plan.boxes ? G::boxes_tx : ve_ne * nbk * 320u));
+                    mbar_expect_more(&g_full[slot], (t < ahead ? 0u : G::w_bytes) + (plan.boxes ? G::boxes_tx : ve_ne * nbk * 256u));
                     if (t >= ahead) ask_weights(s, ve, chunk, dst, &g_full[slot]);
                 }
                 __syncwarp();  // the bytes are expected
@@ -398,16 +397,25 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
                         tma_2d(xd + G::off_deltas, &maps.deltas, s * (G::S * 4u), ve.begin(), &g_full[slot]);
                         tma_2d(xd + G::off_sums, &maps.sums, s * (G::S * 4u), ve.begin(), &g_full[slot]);
                     }
-                } else if (e < ve_ne) {
-                    if (part == 0) bulk_g2s(xd + e * G::box_codes, a.in.codes + u64(row) * in_stride + u64(s) * G::S * 256u, nbk * 256u, &g_full[slot]);
-                    else if (part == 1) bulk_g2s(xd + G::off_deltas + e * G::box_group, a.in.deltas + u64(row) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
-                    else bulk_g2s(xd + G::off_sums + e * G::box_group, a.in.sums + u64(row) * in_gs + u64(s) * G::S * 8u, nbk * 32u, &g_full[slot]);
+                } else {  // the arrival that lets the stage complete comes behind the lanes' copies, each of which adds one of its own while it is under way
+                    if (e < ve_ne) {
+                        if (part == 0) bulk_g2s(xd + e * G::box_codes, a.in.codes + u64(row) * in_stride + u64(s) * G::S * 256u, nbk * 256u, &g_full[slot]);
+                        const unsigned char* from = (part & 2u ? reinterpret_cast<const unsigned char*>(a.in.sums) : reinterpret_cast<const unsigned char*>(a.in.deltas)) + (u64(row) * in_gs + u64(s) * G::S * 8u) * 4u + 16u * (part & 1u);
+                        unsigned char* to = xd + (part & 2u ? G::off_sums : G::off_deltas) + e * G::box_group + 16u * (part & 1u);
+#pragma unroll
+                        for (u32 b = 0; b < G::S; ++b)
+                            if (b < nbk) cp_async16(to + 32u * b, from + 32u * b);
+                    }
+                    asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(saddr(&g_full[slot])) : "memory");
+                    __syncwarp();
                 }
+                if (lane == 0) mbar_arrive(&g_full[slot]);
                 __syncwarp();
             }
             if (!ok || end) break;
             item = PAIR ? n_items : gridDim.x * kGroups + __shfl_sync(0xffffffffu, next, 0);  // PAIR: there are no more items than CTAs
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         if (!ok && lane == 0) {  // wait (bounded) for the copies still in flight before the CTA retires
             for (u32 n = t > plan.stages ? t - plan.stages : 0u; n < t; ++n)
                 for (u32 i = 0; i < (plan.wait_limit >> 4) + 64u; ++i)
@@ -623,8 +631,10 @@ bool a8_bulk_ok(const b200moe_a8_rows& x) {
 
 // The tensor maps of a dense block's A8 rows: exactly the window's rows. Rows shorter than a box come by untiled copies. Why boxes: to ask for one untiled copy takes a
 // producer 70 clocks, for 24 (8 entries) 1,690 of the 2,030 that its consumers work on the stage; three boxes are asked for by one lane. Dense 5120 x 17408, us a call, all
-// changes of the kernel together: 8 rows 66.1 -> 55.6, 1 row (three untiled copies a stage) 42.7 -> 37.5. Routed entries lie anywhere and keep the untiled copies: 64 rows of the
-// large layer 725 -> 719. Gathering copies of four rows were faster there (681) but raised an illegal memory access where the rows began a mapping: not understood, not used.
+// changes of the kernel together: 8 rows 66.1 -> 55.6, 1 row (three untiled copies a stage) 42.7 -> 37.5. Routed entries lie anywhere: one untiled copy of each entry's codes,
+// and the deltas and sums, two thirds of the copies and a fifth of the bytes, as three asynchronous copies a lane. All untiled and so, us a call: 64 rows of the large layer
+// 719 and 680, 37 rows over 128 experts of 2048 -> 768 93.9 and 91.9, one row 22.5 and 21.7. Gathering copies of four rows took 681 there, but raised an illegal memory access
+// where the rows began a mapping: not understood, not used.
 int entry_maps(const b200moe_a8_rows& x, u32 K, WidePlan* p, WideMaps* m) {
     m->codes = m->deltas = m->sums = m->w0;
     const u32 codes = p->S * 256u + 16u, group = p->S * 32u;  // Geo::box_codes, box_group

@@ -268,7 +268,7 @@ bool grouped_pays(const b200moe_shape& s, u32 rows, u32 max_union, u32 grouped_m
     const Window w = window_of(s, rows, max_union);
     const u64 blocks = (down ? s.inter : s.hidden) / 256, sms = static_cast<u64>(device_sm_count());
     const u64 items = w.items8 * (down ? s.hidden / 64 : s.inter / 32), start = blocks < 3 ? 1700 : 1000;  // ns
-    const u64 streaming = items <= sms ? start + 500 * blocks : waves(items, 2 * sms) * (start + 560 * blocks);
+    const u64 streaming = items <= sms ? start + 400 * blocks : waves(items, 2 * sms) * (start + 480 * blocks);
     const u64 grouped = waves(w.tiles32 * grouped_row_tiles(down ? s.hidden : s.inter, down), sms) * (2000 + 1750 * blocks);
     return grouped * (rows < kGroupedSureRows ? 107 : 100) < streaming * 100;
 }
@@ -361,7 +361,7 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
         const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
         return (forced == 0 || forced == 2) && wide_gate_up_fits(v, rows) ? launch_gate_up_q4k_wide(v, rows, hints, st) : launch_gate_up_q4k(v, st);
     }
-    switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.x.sums != nullptr), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, v.max_union, grouped_min_rows, hints.slots == 0, false)) {
+    switch (pick_q4_form(v.shape, grouped_gate_up_fits(v), stream_gate_up_fits(v, rows), wide_gate_up_fits(v, rows), rows, v.max_union, grouped_min_rows, hints.slots == 0, false)) {
         case Q4Form::grouped: return launch_gate_up_q4k_grouped(v, st);
         case Q4Form::row_stream: return launch_gate_up_q4k_stream(v, rows, st);
         case Q4Form::wide: return launch_gate_up_q4k_wide(v, rows, hints, st);
@@ -370,7 +370,7 @@ int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u3
 }
 int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0, const ChainHints& hints = {}) {
     if (v.shape.down_type == B200MOE_TYPE_Q4_K) {
-        switch (pick_q4_form(v.shape, grouped_fits(v.shape, v.act.sums != nullptr), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, v.max_union, grouped_min_rows, hints.slots == 0, true)) {
+        switch (pick_q4_form(v.shape, grouped_down_fits(v), stream_down_fits(v, rows), wide_down_fits(v, rows), rows, v.max_union, grouped_min_rows, hints.slots == 0, true)) {
             case Q4Form::grouped: return launch_down_q4k_grouped(v, st);
             case Q4Form::row_stream: return launch_down_q4k_stream(v, rows, st);
             case Q4Form::wide: return launch_down_q4k_wide(v, rows, hints, st);

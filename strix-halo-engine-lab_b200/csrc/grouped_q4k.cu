@@ -470,14 +470,17 @@ bool es_units(const b200moe_a8_rows& x) {
     return stride % 128 == 0 && aligned(x.deltas, 16) && aligned(x.sums, 16);
 }
 
-bool grouped_shape_ok(const b200moe_shape& s) {
-    return s.gate_type == B200MOE_TYPE_Q4_K && s.down_type == B200MOE_TYPE_Q4_K && s.hidden % 256 == 0 && s.inter % 256 == 0 &&
-           s.experts <= kMaxUnion;
-}
-
 }  // namespace
 
-bool grouped_fits(const b200moe_shape& s, bool have_sums) { return have_sums && grouped_shape_ok(s); }
+// Each stage by itself: gate/up is the same kernel whatever the down's blocks are. An expert has at least a tile of rows, whole groups of outputs.
+bool grouped_gate_up_fits(const b200moe_gate_up_view& v) {
+    const b200moe_shape& s = v.shape;
+    return v.x.sums && s.gate_type == B200MOE_TYPE_Q4_K && s.hidden % 256 == 0 && s.inter % 32 == 0 && s.inter >= kOutRows && s.experts <= kMaxUnion;
+}
+bool grouped_down_fits(const b200moe_down_view& v) {
+    const b200moe_shape& s = v.shape;
+    return v.act.sums && s.gate_type == B200MOE_TYPE_Q4_K && s.down_type == B200MOE_TYPE_Q4_K && s.hidden % 256 == 0 && s.inter % 256 == 0 && s.experts <= kMaxUnion;
+}
 u32 grouped_row_tiles(u32 outputs, bool down) { return (outputs + (down ? kGM : kOutRows) - 1) / (down ? kGM : kOutRows); }
 
 int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t stream) {

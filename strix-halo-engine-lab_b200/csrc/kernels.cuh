@@ -32,7 +32,8 @@ int launch_routes(const b200moe_routes_view& v, const RoutesClear& clear, cudaSt
 // zero (optional): count floats cleared on the way
 int launch_dense_routes(const b200moe_routes& out, u32 rows, u32* row_status, u32* summary4, float* zero, u64 count, cudaStream_t stream);
 // grouped (token-block) form of the Q4_K experts on the tensor cores (grouped_q4k.cu)
-bool grouped_fits(const b200moe_shape& s, bool have_sums);
+bool grouped_gate_up_fits(const b200moe_gate_up_view& v);
+bool grouped_down_fits(const b200moe_down_view& v);
 u32 grouped_row_tiles(u32 outputs, bool down);  // of an expert
 int launch_gate_up_q4k_grouped(const b200moe_gate_up_view& v, cudaStream_t stream);
 int launch_down_q4k_grouped(const b200moe_down_view& v, cudaStream_t stream);

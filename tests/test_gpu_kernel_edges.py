@@ -1280,3 +1280,22 @@ def test_segment_streaming_q5_k(gpu, oracle, H, I, E, rows, top):
     _, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, min(E, rows * top), tuple(dv(t, gpu) for t in (codes, deltas, sums)), rows * top, taps=True)
     assert b200moe.last_launch() == "gate_up_q4k_wide"
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"])
+
+
+@pytest.mark.parametrize("I,down_type", [(96, 8), (128, 7), (544, 7), (640, 8), (992, 8)])
+def test_grouped_gate_up_of_mixed_layers(gpu, oracle, I, down_type):
+    """Q4_K gate / up in the grouped form before a down of other blocks: tiles of 96 outputs with each remainder of an expert's, experts of 1 to 40 entries and of none."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(I)
+    H, E, rows, top = 512, 5, 70, 2
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = np.stack([np.where(np.arange(rows) < 40, 0, 1), np.where(np.arange(rows) == 7, 4, 2)], 1).astype(np.uint32)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)
+    sh, r = ops.make_shape(H, I, E, top, 12, down_type), ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E)
+    with forced(b200moe.FORM_GROUPED):
+        act, g, u = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, tuple(dv(t, gpu) for t in (codes, deltas, sums)), rows * top, taps=True)
+        assert b200moe.last_launch() == "gate_up_q4k_grouped"
+    raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+    assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])

@@ -252,12 +252,13 @@ u64 waves(u64 items, u64 at_once) { return (items + at_once - 1) / at_once; }
 // windows of Q4_K experts take the persistent bulk-copy forms, prompts the grouped form.
 // grouped_min_rows: windows of at least that many rows take the grouped form; 0 = chosen here, for gate/up and down each.
 // Where the segment-streaming form applies, the grouped one (tiles of 32 entries) takes over from it (items of 8) where its waves take less time,
-// both by their sizes: a tile 2 us + 1.75 a super-block of its rows; an item 1 us + 0.56 a super-block (1.7 + 0.56 where rows have less than three and a
-// stage holds one), two an SM, or 0.5 a super-block where there are no more items than SMs. Whole calls with both launches in the streaming and in the
-// grouped form, us: 128 experts of 2048 x 768, top-8, 167 and 216 with 128 rows, 200 and 220 with 160, 223 and 226 with 192; 64 of 7168 x 2048, top-8,
-// 548 and 778 with 64 rows, 639 and 778 with 80, 741 and 793 with 96, 896 and 813 with 128; one expert of 5120 x 17408 134 and 224 with 24 rows, 185
-// to 195 and 226 with 32, 241 and 259 with 48, 322 and 268 with 64; of 2048 x 8192 78 and 114 with 64. The estimates lie within 5 % of these. Below 32 rows
-// they have not been followed, below 48 only where they see more than a few percent gained.
+// both by their sizes: a tile 2 us + 1.75 a super-block of its rows; an item 1.38 us + 0.46 a super-block (1.7 + 0.56 where rows have less than three and a
+// stage holds one), two an SM, or 0.4 a super-block where there are no more items than SMs. Whole calls with both launches in the streaming and in the
+// grouped form, us: 128 experts of 2048 x 768, top-8, 143 and 200 with 128 rows, 190 and 212 with 192, 213 and 219 with 224, 234 and 225 with 256; 64 of 7168 x 2048,
+// top-8, 470 and 775 with 64 rows, 638 and 765 with 96, 718 and 785 with 112, 802 and 818 with 128 (781 with gate/up grouped); 16 of 4096 x 1536, top-2, 123 and 140 with 128,
+// 165 and 142 with 200; one expert of 5120 x 17408 108 and 215 with 24 rows, 158 and 216 with 32, 180 and 252 with 40 (197 with gate/up grouped), 213 and 255 with 56 (197),
+// 265 and 257 with 64 (229). The estimates of the waves lie within 10 % of these. Below 32 rows they have not been followed, below 48 only where they see more than a few
+// percent gained. Layers with a down of other blocks, gate/up in either form: 64 of 2560 x 768, top-4, 262 and 274 with 204 rows, 449 and 424 with 400.
 // Where the segment-streaming form does not apply (more than 8192 slots, rows that bulk copies cannot take) the alternative is the
 // per-block form, and 128 rows are the line.
 constexpr u32 kGroupedLeastRows = 32, kGroupedSureRows = 48, kGroupedRowsElse = 128;
@@ -267,8 +268,8 @@ bool grouped_pays(const b200moe_shape& s, u32 rows, u32 max_union, u32 grouped_m
     if (rows < kGroupedLeastRows) return false;
     const Window w = window_of(s, rows, max_union);
     const u64 blocks = (down ? s.inter : s.hidden) / 256, sms = static_cast<u64>(device_sm_count());
-    const u64 items = w.items8 * (down ? s.hidden / 64 : s.inter / 32), start = blocks < 3 ? 1700 : 1000;  // ns
-    const u64 streaming = items <= sms ? start + 400 * blocks : waves(items, 2 * sms) * (start + 480 * blocks);
+    const u64 items = w.items8 * (down ? s.hidden / 64 : s.inter / 32), item = blocks < 3 ? 1700 + 560 * blocks : 1375 + 460 * blocks;  // ns
+    const u64 streaming = items <= sms ? std::min<u64>(item, 1375 + 400 * blocks) : waves(items, 2 * sms) * item;
     const u64 grouped = waves(w.tiles32 * grouped_row_tiles(down ? s.hidden : s.inter, down), sms) * (2000 + 1750 * blocks);
     return grouped * (rows < kGroupedSureRows ? 107 : 100) < streaming * 100;
 }

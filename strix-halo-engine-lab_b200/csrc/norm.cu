@@ -1,5 +1,5 @@
 // RMSNorm in front of the FFN, fused with the A8 quantiser of its output (the rows the router and the experts read).
-// One CTA per row; 256 of its threads are the 256 lanes of the host rule (src/cpu/core/reference.cpp:86-103): lane l runs
+// One CTA per row, several in short windows; 256 of a CTA's threads are the 256 lanes of the host rule (src/cpu/core/reference.cpp:86-103): lane l runs
 // a = fma(x[i], x[i], a) over i = l, l + L, ... (L = 128 below n = 512), the lanes fold by the halving tree, and
 // s = 1 / sqrt(sum / n + eps) - IEEE division and square root. The second pass is warp-per-group: y = (x * s) * w for
 // 32 consecutive values, written out and / or quantised by the A8 rule on the spot. HBM traffic: x once (the second
@@ -11,42 +11,47 @@
 namespace b200moe {
 namespace {
 
-// WARPS: warps of the CTA, 0 = as launched (8 to 32). A fixed number unrolls the second pass at 48 registers, five CTAs of 8 warps an
-// SM; as launched it takes 29, eight CTAs.
-template <u32 WARPS, bool CHAIN>
-__global__ void __launch_bounds__(WARPS ? WARPS * 32u : 1024u) rmsnorm_a8_kernel(b200moe_rmsnorm_view v) {
+// A row takes gridDim.y CTAs: each makes the whole sum (the row comes out of L2) and takes every gridDim.y-th set of a group a warp of the second pass, whose
+// first values and weights are asked for with the row's. What bounds a short window is the chain of trips and of dependent instructions: asks for BATCH
+// values a lane at once, adds zeros behind the row's end (fma(0, 0, a) is a), and every warp folds the lanes itself, in the tree's order, behind one barrier. One CTA a
+// row that asked for eight values at once, folded by a barrier a level and asked for the weights behind the sum: 1 row of 2560 4.9 us, 2.1 now; of 7168 10.1 and 2.4.
+template <u32 THREADS, u32 BATCH, bool CHAIN>
+__global__ void __launch_bounds__(THREADS) rmsnorm_a8_kernel(b200moe_rmsnorm_view v) {
     chain_begin_if<CHAIN>();
+    constexpr u32 kWarps = THREADS / 32u;
     __shared__ float partial[256];
-    const u32 r = blockIdx.x, t = threadIdx.x, n = v.n;
-    const u32 x_stride = v.x_stride ? v.x_stride : n, out_stride = v.out_stride ? v.out_stride : n;
+    const u32 r = blockIdx.x, t = threadIdx.x, lane = t & 31u, n = v.n, groups = n / 32u;
+    const u32 x_stride = v.x_stride ? v.x_stride : n, out_stride = v.out_stride ? v.out_stride : n, a8_stride = v.a8.stride ? v.a8.stride : v.a8.width;
     const float* x = v.x + u64(r) * x_stride;
     const u32 lanes = n >= 512u ? 256u : 128u;
+    u32 g = kWarps * blockIdx.y + (t >> 5);
+    float mine = 0.0f, weight = 1.0f;
+    if (g < groups) { mine = x[32u * g + lane]; if (v.weight) weight = v.weight[32u * g + lane]; }
     float a = 0.0f;
     if (t < lanes) {
-#pragma unroll 8
-        for (u32 i = t; i < n; i += lanes) { const float xi = x[i]; a = __fmaf_rn(xi, xi, a); }
+        for (u32 i0 = t; i0 < n; i0 += BATCH * lanes) {
+            float xi[BATCH];
+#pragma unroll
+            for (u32 k = 0; k < BATCH; ++k) xi[k] = i0 + k * lanes < n ? x[i0 + k * lanes] : 0.0f;
+#pragma unroll
+            for (u32 k = 0; k < BATCH; ++k) a = __fmaf_rn(xi[k], xi[k], a);
+        }
         partial[t] = a;
     }
     __syncthreads();
-    for (u32 h = lanes / 2; h >= 32; h >>= 1) {
-        if (t < h) partial[t] = __fadd_rn(partial[t], partial[t + h]);
-        __syncthreads();
-    }
-    if (t < 32) {  // the last five levels inside one warp: lane t < h adds lane t + h, as above
-        float p = partial[t];
+    auto four = [&](u32 o, u32 d) { return __fadd_rn(__fadd_rn(partial[lane + o], partial[lane + o + 2u * d]), __fadd_rn(partial[lane + o + d], partial[lane + o + 3u * d])); };
+    float p = lanes == 256u ? __fadd_rn(four(0, 64), four(32, 64)) : four(0, 32);
 #pragma unroll
-        for (u32 h = 16; h > 0; h >>= 1) p = __fadd_rn(p, __shfl_down_sync(0xffffffffu, p, h));
-        if (t == 0) partial[0] = p;
-    }
-    __syncthreads();
-    const float s = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(partial[0], static_cast<float>(n)), v.eps)));
-    const u32 lane = t & 31u, warp = t >> 5, groups = n / 32;
-    const u32 a8_stride = v.a8.stride ? v.a8.stride : v.a8.width;
+    for (u32 h = 16; h > 0; h >>= 1) p = __fadd_rn(p, __shfl_down_sync(0xffffffffu, p, h));
+    p = __shfl_sync(0xffffffffu, p, 0);
+    const float s = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(p, static_cast<float>(n)), v.eps)));
     bool bad = false;
-    for (u32 g = warp; g < groups; g += WARPS ? WARPS : blockDim.x >> 5) {
-        const u32 i = 32u * g + lane;
-        float y = __fmul_rn(x[i], s);
-        if (v.weight) y = __fmul_rn(y, v.weight[i]);
+    for (;;) {
+        if (g >= groups) break;
+        const u32 i = 32u * g + lane, next = g + kWarps * gridDim.y;
+        float y = __fmul_rn(mine, s);
+        if (v.weight) y = __fmul_rn(y, weight);
+        if (next < groups) { mine = x[32u * next + lane]; if (v.weight) weight = v.weight[32u * next + lane]; }
         if (v.out) v.out[u64(r) * out_stride + i] = y;
         if (v.a8.codes) {
             float delta;
@@ -59,27 +64,41 @@ __global__ void __launch_bounds__(WARPS ? WARPS * 32u : 1024u) rmsnorm_a8_kernel
             }
         }
         bad |= !finite_f(y);
+        g = next;
     }
     if (v.status && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&v.status[r], B200MOE_ROW_NONFINITE_ACTIVATION);
 }
+// A CTA reads all of its row while others write theirs: not where the results lie on the rows.
+bool apart(const void* a, u64 an, const void* b, u64 bn) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return !b || x + an <= y || y + bn <= x;
+}
+bool results_apart(const b200moe_rmsnorm_view& v) {
+    const u64 xb = (u64(v.rows - 1) * (v.x_stride ? v.x_stride : v.n) + v.n) * 4, ob = (u64(v.rows - 1) * (v.out_stride ? v.out_stride : v.n) + v.n) * 4;
+    const u64 as = v.a8.stride ? v.a8.stride : v.a8.width, ab = u64(v.rows) * as;
+    return apart(v.x, xb, v.out, ob) && apart(v.x, xb, v.a8.codes, ab) && apart(v.x, xb, v.a8.deltas, ab / 8) && apart(v.x, xb, v.a8.sums, ab / 8);
+}
 
-constexpr u32 kWideRow = 2048;
+// A chained launch asks for as much of a row at once as may be: it waits for trips. A long window has other rows to work on and asks for eight values, or for the ten
+// of rows up to 2560 (2048 of these 22.6 us with ten, 23.8 with eight; 1024 rows of 4096 18.3 with eight, 18.9 with 16; 8192 of 7168 217, and 222 with 16).
+template <u32 THREADS>
+void launch_parts(const b200moe_rmsnorm_view& v, u32 parts, cudaStream_t stream) {
+    const auto kernel = v.n <= 8 * 256 ? rmsnorm_a8_kernel<THREADS, 8, true> : v.n <= 16 * 256 ? rmsnorm_a8_kernel<THREADS, 16, true> : rmsnorm_a8_kernel<THREADS, 32, true>;
+    small_launch(kernel, dim3(v.rows, parts), THREADS, 0, stream, v);
+}
 
 }  // namespace
 
 int launch_rmsnorm_a8(const b200moe_rmsnorm_view& v, cudaStream_t stream) {
     if (v.rows == 0 || v.n == 0) return B200MOE_OK;
-    // Up to two rows an SM a row takes a warp per group in the second pass, up to 32 (the first pass has 256 lanes by contract): 5.8 us
-    // with 32 warps against 8.6 with eight for 1 row of 2560, 24.8 against 31.1 for 296 of 7168. Warps without a group only
-    // cost: 1 row of 256 takes 2.97 us with 32 warps, 2.73 with eight, 296 rows 3.48 and 3.02. Above two rows an SM eight warps keep
-    // more rows in flight, in the unrolled form while all rows fit on the SMs at once (740 rows of 7168: 38.6 us against 40.4
-    // as launched; 1024 rows 50.3 as launched against 64.1 with five to six CTAs an SM) and are long enough for it to matter
-    // (592 rows of 2048: 11.6 against 11.8; of 1024: 7.5 both).
     const u32 sms = static_cast<u32>(device_sm_count());
-    const u32 warps = std::min(32u, (v.n / 32u + 7u) / 8u * 8u);
-    if (chain_pays(v.rows)) small_launch(rmsnorm_a8_kernel<0, true>, v.rows, 32u * warps, 0, stream, v);
-    else if (v.rows <= 5u * sms && v.n >= kWideRow) plain_launch(rmsnorm_a8_kernel<8, false>, v.rows, 256, 0, stream, v);
-    else plain_launch(rmsnorm_a8_kernel<0, false>, v.rows, 256, 0, stream, v);
+    // Up to two rows an SM a row takes as many CTAs of 256 threads as have a group for every warp and as two an SM allow, two beyond one row an SM: 64 rows of 7168 10.4 us
+    // with one CTA of 32 warps, 4.8 so, 5.7 with four CTAs an SM; 296 rows 13.8 and 11.1. Results that lie on the rows keep one CTA a row, of 32 warps where these have groups.
+    const u32 parts = std::min((v.n / 32u + 7u) / 8u, v.rows <= sms ? 2u * sms / v.rows : 2u);
+    if (!chain_pays(v.rows)) plain_launch(v.n > 8 * 256 && v.n <= 10 * 256 ? rmsnorm_a8_kernel<256, 10, false> : rmsnorm_a8_kernel<256, 8, false>, v.rows, 256, 0, stream, v);
+    else if (results_apart(v)) launch_parts<256>(v, parts, stream);
+    else if (v.n > 256u) launch_parts<1024>(v, 1, stream);
+    else launch_parts<256>(v, 1, stream);
     return after_launch("rmsnorm_a8");
 }
 

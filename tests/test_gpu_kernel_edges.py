@@ -1299,3 +1299,25 @@ def test_grouped_gate_up_of_mixed_layers(gpu, oracle, I, down_type):
         assert b200moe.last_launch() == "gate_up_q4k_grouped"
     raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
     assert same(g.cpu(), want["gate"]) and same(u.cpu(), want["up"]) and same(raw.cpu(), want["raw"])
+
+
+@pytest.mark.parametrize("n", [32, 480, 512, 2048, 2080, 2560, 2592, 4096, 4128, 8448])
+@pytest.mark.parametrize("rows", [1, 9, 160, 300])
+def test_rmsnorm_rows_over_several_blocks(gpu, oracle, n, rows):
+    """A row's values in whole and broken batches, over one to many blocks, with results apart from the rows and on them; a row of infinities beside."""
+    import b200moe
+    from b200moe import ops
+    rng = np.random.default_rng(n + rows)
+    x, w = rng.standard_normal((rows, n), dtype=np.float32), rng.standard_normal(n, dtype=np.float32)
+    want = oracle.rmsnorm(x, w, 1e-6)
+    wc, wd, ws = oracle.quantize_a8(want)
+    y, (codes, deltas, sums) = ops.enqueue_rmsnorm_a8(dv(x, gpu), dv(w, gpu), 1e-6)
+    assert same(y.cpu(), want) and np.array_equal(codes.cpu(), wc) and same(deltas.cpu(), wd) and np.array_equal(sums.cpu(), ws)
+    on, wg = dv(x, gpu), dv(w, gpu)
+    v = b200moe.RmsnormView(on.data_ptr(), rows, n, n, wg.data_ptr(), 1e-6, on.data_ptr(), 0, b200moe.A8Rows(), None)
+    b200moe.check(b200moe.lib().b200moe_rmsnorm_a8(v, b200moe.stream_ptr()))
+    assert same(on.cpu(), want)
+    x[rows // 2, n - 1] = np.inf
+    status = torch.zeros(rows, dtype=torch.int32, device=gpu)
+    ops.enqueue_rmsnorm_a8(dv(x, gpu), wg, 1e-6, status=status)
+    assert np.array_equal(status.cpu().numpy() != 0, np.arange(rows) == rows // 2)

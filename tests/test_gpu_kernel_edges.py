@@ -1321,3 +1321,47 @@ def test_rmsnorm_rows_over_several_blocks(gpu, oracle, n, rows):
     status = torch.zeros(rows, dtype=torch.int32, device=gpu)
     ops.enqueue_rmsnorm_a8(dv(x, gpu), wg, 1e-6, status=status)
     assert np.array_equal(status.cpu().numpy() != 0, np.arange(rows) == rows // 2)
+
+
+@pytest.mark.parametrize("I,down_type", [(32, 8), (32, 7), (96, 8), (160, 7), (544, 8), (544, 7), (768, 8), (1056, 8), (1536, 8), (1536, 7), (2048, 7)])
+def test_four_chain_down_on_tensor_cores(gpu, oracle, I, down_type):
+    """Experts of 1, 8, 9, 17, 33 and 70 entries against steps of 16 and 32; items of 64 and 32 rows; fewer groups than chains, odd group counts (Q8_0 rows that start between words);
+    more items than CTAs and fewer."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(I + down_type)
+    H, E = 512 if I < 1000 else 256, 24
+    counts = [1, 8, 9, 17, 33, 70] + [2] * (E - 6)
+    flat = np.repeat(np.arange(E, dtype=np.uint32), counts)
+    rows = flat.size
+    ids = flat[rng.permutation(rows)][:, None].copy()
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, 1, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums, taps=True)["raw"]
+    sh, r = ops.make_shape(H, I, E, 1, 12, down_type), ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E)
+    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows)
+    with forced(b200moe.FORM_GROUPED):
+        raw = ops.enqueue_routed_down(sh, dv(down, gpu), r, E, act)
+    assert b200moe.last_launch() == "down_chain4_mma" and same(raw.cpu(), want)
+
+
+@pytest.mark.parametrize("down_type", [7, 8])
+@pytest.mark.parametrize("stage", [1, 2, 4])
+def test_four_chain_tensor_core_waits_run_out(gpu, oracle, down_type, stage):
+    """A CTA's first item, its second and one that takes a place again are never asked for: JOB_WAIT_ABORTED, and the oracle's bits without the hook."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(stage)
+    rows, top, E, H, I = 40, 4, 16, 2048, 544
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
+    sh, r = ops.make_shape(H, I, E, top, 12, down_type), ops.enqueue_moe_routes(dv(ids.view(np.int32), gpu), E, E)
+    act = ops.enqueue_routed_gate_up(sh, dv(gate, gpu), dv(up, gpu), r, E, (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), rows * top)
+    flag, d = torch.zeros(1, dtype=torch.int32, device=gpu), dv(down, gpu)
+    with stalled(b200moe.FORM_GROUPED, stage):
+        ops.enqueue_routed_down(sh, d, r, E, act, summary=flag)
+        assert b200moe.last_launch() == "down_chain4_mma" and flag.item() & b200moe.JOB_WAIT_ABORTED
+    with forced(b200moe.FORM_GROUPED):
+        assert same(ops.enqueue_routed_down(sh, d, r, E, act).cpu(), want)

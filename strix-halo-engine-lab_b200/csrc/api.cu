@@ -345,14 +345,14 @@ Q8Form pick_q8_form(const b200moe_shape& s, bool shot_fits, bool wide_fits, bool
     }
     return Q8Form::row_per_warp;
 }
-// The four-chain down on the tensor cores (down_chain4_mma.cu), else in the dp4a forms of gemv_q4k.cu: from three entries an expert, for rows of 896 weights and more from one. A
-// launch, us, the better dp4a form and this: 64 experts of 768 -> 2560, top 4, Q5_1 16 rows 28.3 and 29.2, 32 42.2 and 36.2, 48 53 and 44, 128 113 and 53, 1024 693 and 206, Q8_0
-// 31 and 27, 48 and 38, 60 and 42, 111 and 48, 686 and 164; 128 of 640 -> 2560, top 8, Q8_0 16 rows 48 and 58, 32 69 and 76, 48 83 and 81, 64 98 and 84; 60 of 1536 -> 2560, top 4,
-// Q5_1 15 rows 49 and 48, 60 107 and 81, Q8_0 83 and 44, 157 and 71; 32 of 896 -> 2048, top 4, 8 rows 18 and 16, 22 and 16; 32 of 512 -> 1024, top 2, Q5_1 48 rows 12.2 and 12.3,
-// 128 21 and 14. A stage called by itself (alone) keeps the dp4a forms up to 256 entries, where the two lie closest.
+// The four-chain down on the tensor cores (down_chain4_mma.cu), else in the dp4a forms of gemv_q4k.cu: from three entries an expert, four for Q5_1, and for rows of 896 weights
+// and more from one. A launch, us, the better dp4a form and this: 60 experts of 768 -> 2560, top 4, Q5_1 15 rows 21 and 27, 30 34.5 and 37.5, 45 44 and 40, Q8_0 26 and 27, 47 and 37,
+// 55 and 40; 64 of these with 128 rows 113 and 53, 111 and 48, with 1024 693 and 206, 686 and 164; 128 of 640 -> 2560, top 8, Q5_1 48 rows 68 and 73, 64 92 and 78, Q8_0 32 rows 65 and 73,
+// 48 79 and 78; 64 of 512 -> 1024, top 4, 48 rows 17.4 and 18.5, 18.4 and 16.5; 60 of 1536 -> 2560, top 4, Q5_1 15 rows 49 and 48, 60 107 and 81, Q8_0 83 and 44, 157 and 71; 32 of
+// 896 -> 2048, top 4, 8 rows 18 and 16, 22 and 16. A stage called by itself (alone) keeps the dp4a forms up to 256 entries, where the two lie closest.
 bool chain4_mma_pays(const b200moe_shape& s, u64 slots, u32 max_union, bool alone) {
     if (alone && slots <= 256) return false;
-    return slots >= u64(3) * max_union || (s.inter >= 896 && slots >= s.experts);
+    return slots >= u64(s.down_type == B200MOE_TYPE_Q5_1 ? 4 : 3) * max_union || (s.inter >= 896 && slots >= s.experts);
 }
 int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0, const ChainHints& hints = {}) {
     if (v.shape.gate_type == B200MOE_TYPE_Q2_K) return launch_gate_up_ds41_any(v, st);  // the generic form of the family reads every block type

@@ -17,6 +17,8 @@
 //
 // Roofline: HBM. Algorithmic bytes per (expert, call) = 2 * inter * hidden / 256 * 144 (gate, up) and
 // hidden * inter / 256 * 144 (down), read once however many of the <= 8 staged rows use the expert.
+#include <type_traits>
+
 #include "declared_math.cuh"
 #include "grouped_common.cuh"
 #include "kernels.cuh"
@@ -296,7 +298,7 @@ __device__ __forceinline__ void spread_chain_block(ChainBlock<Q51>& o) {
     const u32 qs[4] = {o.q[0], o.q[1], o.q[2], o.q[3]}, hd = o.q[4], hb = o.q[5];
     o.d = half_bits_to_float(hd & 0xffffu);
     o.mn = half_bits_to_float(hd >> 16);
-    auto spread = [](u32 x) { return ((x & 1u) | ((x & 2u) << 7) | ((x & 4u) << 14) | ((x & 8u) << 21)) << 4; };
+    auto spread = [](u32 x) { return ((x & 15u) * 0x02040810u) & 0x10101010u; };  // bit k of four to bit 4 of byte k
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         o.q[i] = (qs[i] & 0x0f0f0f0fu) | spread(hb >> (4 * i));
@@ -410,17 +412,25 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
     __syncthreads();
     if (!plan.early) chain_begin();
     const u32 n_items = load_l2(v.routes.counts) * plan.n_chunks;
-    auto ask = [&](u32 n, u32 item) {  // one thread
-        const u32 j = item / plan.n_chunks, chunk = item - j * plan.n_chunks;
+    struct Item { u32 id, j, chunk; };  // j: place of its expert in the union. The CTA's items are gridDim.x apart
+    const u32 dj = gridDim.x / plan.n_chunks, dc = gridDim.x - dj * plan.n_chunks;
+    auto onward = [&](Item x) {
+        x.id += gridDim.x; x.j += dj; x.chunk += dc;
+        if (x.chunk >= plan.n_chunks) { x.chunk -= plan.n_chunks; ++x.j; }
+        return x;
+    };
+    const Item first_item{blockIdx.x, blockIdx.x / plan.n_chunks, blockIdx.x % plan.n_chunks};
+    auto ask = [&](u32 n, const Item& x) {  // one thread
         unsigned char* st = smem_raw + (n & 1u) * plan.stage_bytes;
         const u32 bytes = R * static_cast<u32>(row_bytes);
         q4k::mbar_expect_tx(&full[n & 1u], bytes);
-        q4k::bulk_g2s(st, v.weights.down + (u64(load_l2(v.routes.experts + j)) * H + R * chunk) * row_bytes, bytes, &full[n & 1u]);
+        q4k::bulk_g2s(st, v.weights.down + (u64(load_l2(v.routes.experts + x.j)) * H + R * x.chunk) * row_bytes, bytes, &full[n & 1u]);
     };
     u32 asked = 0;
+    Item to_ask = first_item;
     const u32 n_ask = plan.stall_stage == 0xffffffffu ? n_items : min(n_items, blockIdx.x + plan.stall_stage * gridDim.x);
     if (tid == 0)
-        for (; asked < 2 && blockIdx.x + asked * gridDim.x < n_ask; ++asked) ask(asked, blockIdx.x + asked * gridDim.x);
+        for (; asked < 2 && to_ask.id < n_ask; ++asked, to_ask = onward(to_ask)) ask(asked, to_ask);
     if (plan.early) chain_begin();
     auto drain = [&](u32 from) {  // one thread: the copies asked for land (the wait is bounded) before the CTA retires
         for (u32 n = from; n < asked; ++n)
@@ -453,25 +463,25 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
             }
         }
     };
-    auto entries = [&](u32 item, u32& first, u32& count) {
-        const u32 j = item / plan.n_chunks;
-        first = load(v.routes.begins + j);
-        count = load(v.routes.begins + j + 1) - first;
+    auto entries = [&](const Item& x, u32& first, u32& count) {
+        first = load(v.routes.begins + x.j);
+        count = load(v.routes.begins + x.j + 1) - first;
     };
     u32 first = 0, count = 0;
     if (blockIdx.x < n_items) {
-        entries(blockIdx.x, first, count);
+        entries(first_item, first, count);
         stage(0, first, min(plan.cap, count));
     }
     bool ok = true;
     u32 n = 0;
-    for (u32 item = blockIdx.x; item < n_items; item += gridDim.x, ++n) {
-        const u32 b = n & 1u, o = R * (item % plan.n_chunks) + my_row;
+    for (Item item = first_item; item.id < n_items; item = onward(item), ++n) {
+        const u32 b = n & 1u, o = R * item.chunk + my_row;
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         u32 next_first = 0, next_count = 0;
-        if (item + gridDim.x < n_items) {
-            entries(item + gridDim.x, next_first, next_count);
+        const Item next = onward(item);
+        if (next.id < n_items) {
+            entries(next, next_first, next_count);
             stage(b ^ 1u, next_first, min(plan.cap, next_count));
         }
         ok = q4k::mbar_wait(&full[b], (n >> 1) & 1u, plan.wait_limit, &s_abort);
@@ -488,43 +498,53 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 __syncthreads();
             }
-            float acc[kR];
+            // Up to so many entries; one and two, the common counts of a window that keeps this form, have code of their own: a launch fetches its instructions cold, and the checks
+            // of eight entries were a third of them. 4 rows over 128 experts of 640 -> 2560, top 8, Q5_1: 18.8 -> 12.1 us a launch, with the items' divisions gone, the fifth bits spread by a product
+            // and four blocks of an only entry at once (two, and of more entries too, 14.5: more registers, fewer CTAs).
+            auto run = [&](auto most) {
+                constexpr int kMost = decltype(most)::value;
+                float acc[kMost];
 #pragma unroll
-            for (int r = 0; r < kR; ++r) acc[r] = 0.0f;
-#pragma unroll 2
-            for (u32 g = chain; g < groups; g += 4) {
-                ChainBlock<Q51> w;
-                load_chain_block<Q51>(wrow + g * block, w);
-                spread_chain_block<Q51>(w);
+                for (int r = 0; r < kMost; ++r) acc[r] = 0.0f;
+#pragma unroll (kMost == 1 ? 4 : 1)
+                for (u32 g = chain; g < groups; g += 4) {
+                    ChainBlock<Q51> w;
+                    load_chain_block<Q51>(wrow + g * block, w);
+                    spread_chain_block<Q51>(w);
 #pragma unroll
-                for (int r = 0; r < kR; ++r) {
-                    if (r < (int)nr) {
-                        const uint4* c = reinterpret_cast<const uint4*>(from + r * I + 32u * g);
-                        const uint4 c0 = c[0], c1 = c[1];
-                        int da = __dp4a((int)w.q[0], (int)c0.x, 0), db = __dp4a((int)w.q[4], (int)c1.x, 0);
-                        da = __dp4a((int)w.q[1], (int)c0.y, da); db = __dp4a((int)w.q[5], (int)c1.y, db);
-                        da = __dp4a((int)w.q[2], (int)c0.z, da); db = __dp4a((int)w.q[6], (int)c1.z, db);
-                        da = __dp4a((int)w.q[3], (int)c0.w, da); db = __dp4a((int)w.q[7], (int)c1.w, db);
-                        float combined = __fmul_rn(w.d, static_cast<float>(da + db));
-                        if (Q51) combined = __fadd_rn(combined, __fmul_rn(w.mn, static_cast<float>(sums[r * groups + g])));
-                        acc[r] = __fadd_rn(acc[r], __fmul_rn(deltas[r * groups + g], combined));
+                    for (int r = 0; r < kMost; ++r) {
+                        if (kMost <= 2 || r < (int)nr) {
+                            const uint4* c = reinterpret_cast<const uint4*>(from + r * I + 32u * g);
+                            const uint4 c0 = c[0], c1 = c[1];
+                            int da = __dp4a((int)w.q[0], (int)c0.x, 0), db = __dp4a((int)w.q[4], (int)c1.x, 0);
+                            da = __dp4a((int)w.q[1], (int)c0.y, da); db = __dp4a((int)w.q[5], (int)c1.y, db);
+                            da = __dp4a((int)w.q[2], (int)c0.z, da); db = __dp4a((int)w.q[6], (int)c1.z, db);
+                            da = __dp4a((int)w.q[3], (int)c0.w, da); db = __dp4a((int)w.q[7], (int)c1.w, db);
+                            float combined = __fmul_rn(w.d, static_cast<float>(da + db));
+                            if (Q51) combined = __fadd_rn(combined, __fmul_rn(w.mn, static_cast<float>(sums[r * groups + g])));
+                            acc[r] = __fadd_rn(acc[r], __fmul_rn(deltas[r * groups + g], combined));
+                        }
                     }
                 }
-            }
 #pragma unroll
-            for (int r = 0; r < kR; ++r) {
-                if (r < (int)nr) {  // uniform over the block
-                    const float pair = __fadd_rn(acc[r], __shfl_xor_sync(0xffffffffu, acc[r], 1));
-                    const float y = __fadd_rn(pair, __shfl_xor_sync(0xffffffffu, pair, 2));
-                    if (chain == 0) v.raw[u64(s_slots[b][r]) * H + o] = y;
+                for (int r = 0; r < kMost; ++r) {
+                    if (kMost <= 2 || r < (int)nr) {  // uniform over the block
+                        const float pair = __fadd_rn(acc[r], __shfl_xor_sync(0xffffffffu, acc[r], 1));
+                        const float y = __fadd_rn(pair, __shfl_xor_sync(0xffffffffu, pair, 2));
+                        if (chain == 0) v.raw[u64(s_slots[b][r]) * H + o] = y;
+                    }
                 }
-            }
+            };
+            if (nr == 1u) run(std::integral_constant<int, 1>{});
+            else if (nr == 2u) run(std::integral_constant<int, 2>{});
+            else run(std::integral_constant<int, kR>{});
         }
         __syncthreads();  // the stage and the buffer have been read
-        if (tid == 0 && item + 2 * gridDim.x < n_ask) {
+        if (tid == 0 && to_ask.id < n_ask) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            ask(n + 2, item + 2 * gridDim.x);
+            ask(n + 2, to_ask);
             ++asked;
+            to_ask = onward(to_ask);
         }
         first = next_first; count = next_count;
     }

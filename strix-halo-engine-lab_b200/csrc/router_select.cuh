@@ -191,31 +191,21 @@ __device__ __forceinline__ bool select_row_fast(const float* logits, float* scor
     }
     if (scores_out) for (u32 e = lane; e < E; e += 32) scores_out[u64(row) * E + e] = s[e];
     __syncwarp();
-    u32* picks = reinterpret_cast<u32*>(s + E);
+    u32 my_id = kNone;
 #pragma unroll 1
     for (u32 k = 0; k < p.top_k; ++k) {
         u32 top = 0;
 #pragma unroll
         for (int j = 0; j < EPL; ++j) top = max(top, key[j]);
-        const u32 best = __reduce_max_sync(0xffffffffu, top), holders = __ballot_sync(0xffffffffu, top == best);
-        u32 winner = __ffs(holders) - 1u;  // best is some lane's
-        if (holders & (holders - 1u)) {    // several lanes have it: the lowest id (lane + 32 j) does
-            u32 id = kNone;
+        const u32 best = __reduce_max_sync(0xffffffffu, top);
+        u32 id = kNone;
 #pragma unroll
-            for (int j = EPL - 1; j >= 0; --j) if (key[j] == best) id = lane + 32u * j;
-            winner = __reduce_min_sync(0xffffffffu, id) & 31u;
-        }
-        if (lane == winner) {
-            u32 id = kNone;
+        for (int j = EPL - 1; j >= 0; --j) if (key[j] == best) id = lane + 32u * j;
+        id = best ? __reduce_min_sync(0xffffffffu, id) : kNone;
 #pragma unroll
-            for (int j = EPL - 1; j >= 0; --j) if (key[j] == best) id = lane + 32u * j;
-#pragma unroll
-            for (int j = 0; j < EPL; ++j) if (lane + 32u * j == id) key[j] = 0u;
-            picks[k] = best ? id : kNone;
-        }
+        for (int j = 0; j < EPL; ++j) if (lane + 32u * j == id) key[j] = 0u;
+        if (lane == k) my_id = id;
     }
-    __syncwarp();
-    const u32 my_id = lane < p.top_k ? picks[lane] : kNone;
     *picked = my_id;
     return true;
 }

@@ -559,7 +559,8 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
 
 // Rows of an item and entries of a pass: as many rows (64, 32 or 16) as let three CTAs share a multiprocessor, fewer CTAs for rows so long that not even 16
 // do. False where the form above is the better one: rows too long for two stages, and windows of more than two rounds of items whose long rows leave a
-// multiprocessor few threads (four a row and CTA), fewer than 256, for Q5_1 with its longer decoding 512. Layers of Q4_K gate/up, this form and the one above, us:
+// multiprocessor few threads (four a row and CTA), fewer than 256, for Q5_1 with its longer decoding 512. Layers of Q4_K gate/up, this form and the one above, us (before one and two
+// entries had loops of their own here and before windows of several entries an expert left for down_chain4_mma.cu):
 // 60 experts of 2560, top 4, Q5_1: 768 wide 1 row 19.4 and 20.4, 8 rows 41.9 and 41.6, 512 rows 543 and 601; 1536 wide (192 threads) 1 row 20.9 and 26.2, 4 rows
 // 47.0 and 44.6, 8 rows 84 and 65, 512 rows 1515 and 956; 2816 wide (64 threads) 1 row 34.3 and 38.4, 512 rows 5660 and 1550. Over 1200 such layers (1 to 128 experts, 1 to 512 rows, 256 to 2816 wide) the rule
 // is 18 % faster than the form above everywhere, and slower than it by 3 to 7 % in 33.

@@ -25,11 +25,11 @@
 //  * Where there are no more items than CTAs (rows of several stages: a dense block's down) an item is both groups': each takes every other stage, makes what its
 //    super-blocks add to the chains, gets the chains from the other group, adds in order and hands them on (PAIR).
 //  * gate/up: the group meets on an mbarrier once per item and a warp an entry runs SwiGLU + the A8 rule; down: a warp an entry stores the sums.
-// What bounds it: the latency of dependent instructions with four consumer warps a scheduler (64 rows over 64 experts of 7168 -> 2048: 62 % of the issue
-// slots, 67 % of the shared memory's cycles, 49 % of the DRAM's). A warp with 8 rows of four chains, whose factors met 8 rows and which took the tensor cores from
-// 5 entries and dp4a of up to 4 entries below, read shared memory twice as much: 64 rows of the large layer (256 experts) 880 to 917 us a call, 804 to 855
-// now; dense 5120 x 17408, 8 rows, 84.5 and 77.9; 37 rows over 128 experts of 2048 -> 768 112.0 and 109.3. Copies of 144-byte rows (a super-block
-// each) into a ring of 4 stages of two super-blocks instead of 2 of three: dense 1 row 49.8 -> 57.5, 8 rows 84.4 -> 98.3.
+// What bounds it: the latency of dependent instructions with four consumer warps a scheduler (64 experts of 7168 -> 2048, 64 rows: 64 % of the issue
+// slots, 58 % of the shared memory's cycles, 57 % of the DRAM's). Measured forms before: a warp with 8 rows of four chains, whose factors met 8 rows and which took the tensor cores from
+// 5 entries and dp4a of up to 4 entries below, read shared memory twice as much (64 rows of the large layer, 256 experts, 880 to 917 us a call, 804 to 855 with 32 rows of one chain; rows, not
+// groups, as the lanes of the packed instructions then 725 to 745 in a graph, 680 to 696 now). Copies of 144-byte rows (a super-block each) into a ring of 4 stages of two super-blocks instead
+// of 2 of three: dense 5120 x 17408 1 row 49.8 -> 57.5, 8 rows 84.4 -> 98.3.
 //
 // Every wait is bounded (plan.wait_limit polls): a waiter that runs out raises the CTA's abort flag, every role leaves
 // its loops, the producers wait (bounded) for the copies they still have in flight, B200MOE_JOB_WAIT_ABORTED is set in the

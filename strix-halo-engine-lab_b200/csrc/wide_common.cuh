@@ -152,6 +152,5 @@ inline int rows_map(const u8* base, u64 row_bytes, u64 rows, u32 box_bytes, u32 
     return pitched_map(base, row_bytes, row_bytes, rows, box_bytes, box_rows, out);
 }
 
-
 }  // namespace wide
 }  // namespace b200moe

@@ -10,7 +10,7 @@ import math
 import torch
 
 from . import (A8Rows, CombineView, DenseView, DownView, ExpertWeights, FfnView, GateUpView, LayerView, Q8A8View,
-               QuantizeA8View, RoutePolicy, RouterView, Routes, RoutesView, Shape, a8_rows, check, lib, ptr, stream_ptr,
+               QuantizeA8View, RmsnormView, RoutePolicy, RouterView, Routes, RoutesView, Shape, a8_rows, check, lib, ptr, stream_ptr,
                COMBINE_FMA_SLOTS, COMBINE_PARTS, TYPE_Q4_K, TYPE_Q8_0)
 
 
@@ -18,11 +18,16 @@ def _dev(t):
     return t.device if t is not None else torch.device("cuda")
 
 
+def _like(x, dtype):
+    """New row-major memory of x's shape (0.5 us cheaper than new_empty)."""
+    return torch.empty_like(x, dtype=dtype, memory_format=torch.contiguous_format)
+
+
 def enqueue_quantize_a8(x, status=None, stride=0):
     """x [rows][width] float32 or bfloat16 -> (codes int8, deltas float32, sums int32)."""
     rows, width = x.shape
     st = stride or width
-    codes = x.new_empty((rows, st), dtype=torch.int8)
+    codes = _like(x, torch.int8) if st == width else x.new_empty((rows, st), dtype=torch.int8)
     deltas = x.new_empty((rows, st // 32 if st % 32 == 0 else 1), dtype=torch.float32)
     sums = torch.empty_like(deltas, dtype=torch.int32)
     v = QuantizeA8View(ptr(x), rows, width, x.stride(0), int(x.dtype == torch.bfloat16),
@@ -33,12 +38,11 @@ def enqueue_quantize_a8(x, status=None, stride=0):
 
 def enqueue_rmsnorm_a8(x, weight=None, eps=1e-6, want_out=True, want_a8=True, status=None):
     """x [rows][n] float32 -> (y float32 or None, (codes, deltas, sums) or None): RMSNorm and the A8 of its output in one launch."""
-    from . import RmsnormView
     rows, n = x.shape
-    y = x.new_empty((rows, n), dtype=torch.float32) if want_out else None
+    y = _like(x, torch.float32) if want_out else None
     a8, rows_view = None, A8Rows()
     if want_a8:
-        codes = x.new_empty((rows, n), dtype=torch.int8)
+        codes = _like(x, torch.int8)
         deltas = x.new_empty((rows, max(n // 32, 1)), dtype=torch.float32)
         sums = torch.empty_like(deltas, dtype=torch.int32)
         a8, rows_view = (codes, deltas, sums), A8Rows(ptr(codes), ptr(deltas), ptr(sums), rows, n, n)
@@ -166,7 +170,7 @@ class MoeLayer:
         dev = self.gate.device
         fresh = combine and y_blocks is None  # the call itself leaves zeros where it writes nothing
         y = self.gate.new_empty((rows, self.shape.hidden), dtype=torch.float32) if fresh else None
-        yb = (self.gate.new_empty if fresh else self.gate.new_zeros)((rows, self.shape.hidden), dtype=torch.bfloat16) if bf16 else None
+        yb = None if not bf16 else _like(y, torch.bfloat16) if fresh else self.gate.new_zeros((rows, self.shape.hidden), dtype=torch.bfloat16)
         raw = torch.zeros((rows * self.shape.top_k, self.shape.hidden), dtype=torch.float32, device=dev) if want_raw else None
         v = LayerView(self.shape, ExpertWeights(ptr(self.gate), ptr(self.up), ptr(self.down)), rows, a8_rows(*x_a8), ptr(ids),
                       ptr(route_weights), ptr(shared), first, end, base, self.combine_form, self.parts, self.part_experts, only_part,

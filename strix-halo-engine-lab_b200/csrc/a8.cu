@@ -36,18 +36,19 @@ __global__ void __launch_bounds__(256) quantize_a8_kernel(const void* x, u32 row
 }
 
 // The same rule with four values a lane and eight lanes a group: wide loads, three shuffles a reduction instead of five, a
-// quarter of the warps. Bound by issue slots (72 % busy at 8192 x 7168 FP32) and the pipe that the divisions' reciprocals take (62 %):
-// 108 us there, 0.44 of the measured copy bandwidth; 1024 rows 15.6 us, 38.9 in the one-value form. With `wide` the bfloat16 values
+// quarter of the warps. Bound by issue slots; with a division a value (72 % of them busy, and 62 % of the pipe that takes the reciprocals) and one for the item's row 8192 x 7168
+// FP32 took 104 us, with one reciprocal a group, exact quotients near halves alone and a product for the row 86, 0.54 of the measured copy bandwidth; 1024 rows 13.1 -> 10.9 us, 4096 x 2048
+// bfloat16 14.9 -> 13.5. With `wide` the bfloat16 values
 // are also written out as FP32 for the router, instead of by a pass of their own before this one (8192 x 7168: 119 + 305 -> 218 us).
 template <bool BF16>
-__global__ void __launch_bounds__(256) quantize_a8_vec_kernel(const void* x, u32 items, u32 groups, u32 x_stride, i8* codes,
+__global__ void __launch_bounds__(256) quantize_a8_vec_kernel(const void* x, u32 items, u32 groups, u32 per_group, u32 shift, u32 x_stride, i8* codes,
                                                               float* deltas, i32* sums, u32 stride, u32* status,
                                                               float* wide, u32 wide_stride) {
     chain_begin();
     const u32 t = blockIdx.x * 256u + threadIdx.x, sub = t & 7u;
     const bool valid = (t >> 3) < items;
     const u32 item = valid ? t >> 3 : items - 1u;  // spare lanes of the last warp repeat its last group and store nothing
-    const u32 r = item / groups, g = item - r * groups;
+    const u32 r = static_cast<u32>(u64(item) * per_group >> shift), g = item - r * groups;  // item / groups: see the launch
     const u64 at = u64(r) * x_stride + 32u * g + 4u * sub;
     float v[4];
     if (BF16) {
@@ -63,11 +64,18 @@ __global__ void __launch_bounds__(256) quantize_a8_vec_kernel(const void* x, u32
     for (int d = 4; d; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
     const bool tiny = amax > 0.0f && amax < 0x1p-119f;
     const float delta = (amax == 0.0f || tiny) ? 1.0f : __fdiv_rn(amax, 127.0f);
+    const float inverse = __frcp_rn(delta);
+    float quotient[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) quotient[i] = __fmul_rn(v[i], inverse);
     int sum = 0;
     u32 word = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const float q = tiny ? 0.0f : rintf(__fdiv_rn(v[i], delta));
+        float q = rintf(quotient[i]);
+        // The product lies within 2^-15 of the quotient and the quotient's rounding within 2^-17 of it, so the integers can differ near a half alone (or where there is no number).
+        if (!(fabsf(__fsub_rn(quotient[i], q)) < 0.5f - 0x1p-13f)) q = rintf(__fdiv_rn(v[i], delta));
+        if (tiny) q = 0.0f;
         const float lo = (-127.0f < q) ? q : -127.0f;
         const int code = static_cast<int>((lo < 127.0f) ? lo : 127.0f);
         sum += code;
@@ -115,10 +123,14 @@ int launch_quantize_a8(const b200moe_quantize_a8_view& v, cudaStream_t stream, f
     const u32 x_stride = v.x_stride ? v.x_stride : v.width, stride = v.out.stride ? v.out.stride : v.width;
     if (quantize_a8_vec_ok(v) && (wide || items > 8u * static_cast<u32>(device_sm_count()))) {
         const u32 vec_blocks = static_cast<u32>((items + 31) / 32);
+        // n / groups = n * per_group >> shift for every n below 2^28: per_group * groups lies between 2^shift and 2^shift + groups, and groups is no more than 2^(shift - 28).
+        u32 shift = 28;
+        while ((1ull << (shift - 28)) < groups) ++shift;
+        const u32 per_group = static_cast<u32>((1ull << shift) / groups + 1);
         if (v.x_is_bf16)
-            small_launch(quantize_a8_vec_kernel<true>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, wide, wide_stride);
+            small_launch(quantize_a8_vec_kernel<true>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, per_group, shift, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, wide, wide_stride);
         else
-            small_launch(quantize_a8_vec_kernel<false>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, nullptr, 0);
+            small_launch(quantize_a8_vec_kernel<false>, vec_blocks, 256, 0, stream, v.x, static_cast<u32>(items), groups, per_group, shift, x_stride, v.out.codes, v.out.deltas, v.out.sums, stride, v.status, nullptr, 0);
         return after_launch("quantize_a8");
     }
     const u32 blocks = static_cast<u32>((items + 7) / 8);

@@ -1365,3 +1365,20 @@ def test_four_chain_tensor_core_waits_run_out(gpu, oracle, down_type, stage):
         assert b200moe.last_launch() == "down_chain4_mma" and flag.item() & b200moe.JOB_WAIT_ABORTED
     with forced(b200moe.FORM_GROUPED):
         assert same(ops.enqueue_routed_down(sh, d, r, E, act).cpu(), want)
+
+
+@pytest.mark.parametrize("width", [32, 96, 2048, 7168])
+def test_quantize_a8_at_halves(gpu, oracle, width):
+    """Values whose quotient by the group's delta lies at a half between two codes, and next to it, at both ends of the exponents; zeros, values below the smallest delta, infinities."""
+    from b200moe import ops
+    rng = np.random.default_rng(width)
+    rows = 1500 * 64 // width + 1100 * 32 // width + 3
+    a = (rng.uniform(0.5, 1, (rows, width // 32, 1)) * np.exp2(rng.integers(-118, 126, (rows, width // 32, 1)))).astype(np.float32)
+    x = ((rng.integers(-127, 127, (rows, width // 32, 32)) + 0.5) * (a / np.float32(127)).astype(np.float64)).astype(np.float32)
+    x = np.where(rng.random(x.shape) < 0.5, x, np.nextafter(x, (rng.choice([-1, 1], x.shape) * np.inf).astype(np.float32)))
+    x[:, :, :1] = a
+    x = np.clip(x, -a, a).reshape(rows, width).astype(np.float32)
+    x[0, :32], x[1, :32], x[2, :31], x[2, 31] = 0, 2.0 ** -140, 1, np.inf
+    wc, wd, ws = oracle.quantize_a8(x)
+    codes, deltas, sums = ops.enqueue_quantize_a8(dv(x, gpu))
+    assert np.array_equal(codes.cpu(), wc) and same(deltas.cpu(), wd) and np.array_equal(sums.cpu(), ws)

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) down_chain4_mma_kernel(b200m
             for (u32 i = 0; i < (plan.wait_limit >> 4) + 64u; ++i)
                 if (mbar_try_wait(&full[n & 1u], (n >> 1) & 1u, kWaitHintNs)) break;
     };
-    if (v.summary && *v.summary) {  // a failed projection skips the whole down stage (routed_expert.hpp:17-19)
+    if (block_skips(v.summary)) {  // a failed projection skips the whole down stage (routed_expert.hpp:17-19)
         if (tid == 0) drain_asked(0);
         return;
     }

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kWarps * 32) down_ds41_any_kernel(b200moe_down
     __shared__ u32 s_slots[kR];
     __shared__ const i8* s_codes[kR];
     __shared__ const float* s_deltas[kR];
-    if (v.summary && *v.summary) return;
+    if (block_skips(v.summary)) return;
     const u32 j = blockIdx.y;
     if (j >= v.routes.counts[0]) return;
     const u32 H = v.shape.hidden, I = v.shape.inter, groups = I / 32;

@@ -227,7 +227,7 @@ template <int LPR>
 __global__ void __launch_bounds__(256) down_q4k_kernel(b200moe_down_view v, u32 rows_per_cta) {
     chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (v.summary && *v.summary) return;  // a failed projection skips the whole down stage (routed_expert.hpp:17-19)
+    if (block_skips(v.summary)) return;  // a failed projection skips the whole down stage (routed_expert.hpp:17-19)
     const u32 j = blockIdx.y;
     if (j >= v.routes.counts[0]) return;
     const u32 H = v.shape.hidden, I = v.shape.inter, groups = I / 32, nblocks = I / 256;
@@ -318,7 +318,7 @@ template <bool Q51>
 __global__ void __launch_bounds__(256) down_q8_chain4_kernel(b200moe_down_view v) {
     chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (v.summary && *v.summary) return;
+    if (block_skips(v.summary)) return;
     const u32 j = blockIdx.y;
     if (j >= v.routes.counts[0]) return;
     const u32 H = v.shape.hidden, I = v.shape.inter, groups = I / 32;
@@ -396,7 +396,7 @@ struct ChainPlan {
     u32 early, wait_limit, stall_stage;  // test hook: item `stall_stage` of a CTA's items and those behind it are not asked for
 };
 template <bool Q51>
-__global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_view v, ChainPlan plan) {
+__global__ void __launch_bounds__(256, 4) down_chain4_stream_kernel(b200moe_down_view v, ChainPlan plan) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const u32 H = v.shape.hidden, I = v.shape.inter, groups = I / 32, R = plan.rows_per_item;
     constexpr u32 block = Q51 ? kQ51Block : kQ8Block;
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(256) down_chain4_stream_kernel(b200moe_down_vi
             for (u32 i = 0; i < (plan.wait_limit >> 4) + 64u; ++i)
                 if (q4k::mbar_try_wait(&full[n & 1u], (n >> 1) & 1u, q4k::kWaitHintNs)) break;
     };
-    if (v.summary && *v.summary) {  // a failed projection skips the whole down stage (routed_expert.hpp:17-19)
+    if (block_skips(v.summary)) {  // a failed projection skips the whole down stage (routed_expert.hpp:17-19)
         if (tid == 0) drain(0);
         return;
     }

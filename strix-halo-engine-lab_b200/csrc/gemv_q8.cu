@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(1024) down_q8_kernel(b200moe_down_view v, u32 
         have_pre = true;
     }
     if (early) chain_begin();
-    if (v.summary && *v.summary) return;
+    if (block_skips(v.summary)) return;
     for (u32 p0 = eb + kR * blockIdx.z; p0 < ee; p0 += kR * gridDim.z) {  // grid.z shares an expert's passes of kR entries
         const int nr = static_cast<int>(min(u32(kR), ee - p0));
         __syncthreads();

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kThreads) q8_shot_kernel(const __grid_constant
             for (u32 i = 0; i < (a.wait_limit >> 4) + 64u; ++i)
                 if (mbar_try_wait(&full[n % a.stages], (n / a.stages) & 1u, kWaitHintNs)) break;
     };
-    if (DOWN && a.summary && *a.summary) {  // an aborted projection skips the stage
+    if (DOWN && block_skips(a.summary)) {  // an aborted projection skips the stage
         if (tid == 0) drain(0);
         return;
     }

@@ -951,7 +951,9 @@ def test_a_job_with_a_failed_projection_combines_no_row(gpu, rows, top_k, form, 
 
 @pytest.mark.parametrize("types,form,name", [((12, 12), "FORM_ROW_STREAM", "q4k_stream"), ((12, 12), "FORM_SEGMENT_STREAM", "q4k_wide"), ((12, 12), "FORM_PER_BLOCK", "q4k"),
                                              ((12, 12), "FORM_GROUPED", "q4k_grouped"), ((8, 8), "FORM_SEGMENT_STREAM", "q8_wide"), ((8, 8), "FORM_PER_BLOCK", "q8"),
-                                             ((8, 8), "FORM_TENSOR", "q8_mma"), ((8, 8), "FORM_GROUPED", "q8_grouped"), ((8, 8), "FORM_ONE_ITEM", "q8_shot")])
+                                             ((8, 8), "FORM_TENSOR", "q8_mma"), ((8, 8), "FORM_GROUPED", "q8_grouped"), ((8, 8), "FORM_ONE_ITEM", "q8_shot"),
+                                             ((12, 8), "FORM_GROUPED", "chain4_mma"), ((12, 7), "FORM_GROUPED", "chain4_mma"), ((12, 8), "FORM_SEGMENT_STREAM", "chain4_stream"),
+                                             ((12, 7), "FORM_SEGMENT_STREAM", "chain4_stream"), ((12, 8), "FORM_PER_BLOCK", "q8_chain4"), ((12, 7), "FORM_PER_BLOCK", "q8_chain4")])
 def test_down_is_left_out_in_every_form(gpu, oracle, types, form, name):
     """Any bit of the summary leaves the whole stage out, a word of zero lets it run, and the routes serve the next launch either way."""
     import b200moe
@@ -1382,3 +1384,29 @@ def test_quantize_a8_at_halves(gpu, oracle, width):
     wc, wd, ws = oracle.quantize_a8(x)
     codes, deltas, sums = ops.enqueue_quantize_a8(dv(x, gpu))
     assert np.array_equal(codes.cpu(), wc) and same(deltas.cpu(), wd) and np.array_equal(sums.cpu(), ws)
+
+
+@pytest.mark.parametrize("down_type", [7, 8])
+@pytest.mark.parametrize("rows,top_k,E,H,I,name", [(3, 1, 4, 512, 640, "stream"), (2, 2, 3, 2560, 96, "stream"), (40, 4, 16, 512, 544, "mma"), (40, 2, 4, 2560, 1024, "mma")])
+def test_four_chain_down_skipped_after_its_weights_were_asked_for(gpu, oracle, rows, top_k, E, H, I, name, down_type):
+    """A layer's four-chain down asks for weights before gate/up has finished: a projection that is not finite skips it with the copies in flight (no row is combined), the next
+    call gives the oracle's bits."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    bad = deltas.copy()
+    bad[rows - 1, 0] = np.inf
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
+    sh = ops.make_shape(H, I, E, top_k, 12, down_type)
+    layer = ops.MoeLayer(sh, dv(gate, gpu), dv(up, gpu), dv(down, gpu), capacity=rows, combine_form=b200moe.COMBINE_FMA_SLOTS)
+    ids, w = dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu)
+    for _ in range(3):
+        fail, good = ((dv(codes, gpu), dv(d, gpu), dv(sums, gpu)) for d in (bad, deltas))
+        status = torch.zeros(rows, dtype=torch.int32, device=gpu)
+        assert not layer(fail, ids, w, row_status=status).any() and int(status[rows - 1]) == b200moe.ROW_PROJECTION_NONFINITE
+        assert same(layer(good, ids, w, want_raw=True)[1].cpu(), want)
+    layer(good, ids, w, combine=False)
+    assert b200moe.last_launch() == "down_chain4_" + name

@@ -247,6 +247,11 @@ Window window_of(const b200moe_shape& s, u32 rows, u32 max_union) {
     const u64 e16 = 16 * u64(rows) * s.top_k / s.experts;  // entries an expert, in sixteenths
     return Window{(max_union * std::max<u64>(16, e16 / 8 + 7) + 15) / 16, (max_union * std::max<u64>(16, (e16 + 192) / 32) + 15) / 16, e16 <= 12 * 16};
 }
+// Experts that have an entry, of the max_union that may, where the choice is spread evenly.
+u32 experts_met(const b200moe_shape& s, u64 slots, u32 max_union) {
+    const double of = slots > max_union ? max_union : s.experts;
+    return std::min(max_union, static_cast<u32>(std::ceil(of * -std::expm1(-static_cast<double>(slots) / s.experts))));
+}
 u64 waves(u64 items, u64 at_once) { return (items + at_once - 1) / at_once; }
 // Plan by window size, chosen on the host from the sizes (no environment reads inside numerical code): decode
 // windows of Q4_K experts take the persistent bulk-copy forms, prompts the grouped form.
@@ -345,14 +350,25 @@ Q8Form pick_q8_form(const b200moe_shape& s, bool shot_fits, bool wide_fits, bool
     }
     return Q8Form::row_per_warp;
 }
-// The four-chain down on the tensor cores (down_chain4_mma.cu), else in the dp4a forms of gemv_q4k.cu: from three entries an expert, four for Q5_1, and for rows of 896 weights
-// and more from one. A launch, us, the better dp4a form and this: 60 experts of 768 -> 2560, top 4, Q5_1 15 rows 21 and 27, 30 34.5 and 37.5, 45 44 and 40, Q8_0 26 and 27, 47 and 37,
-// 55 and 40; 64 of these with 128 rows 113 and 53, 111 and 48, with 1024 693 and 206, 686 and 164; 128 of 640 -> 2560, top 8, Q5_1 48 rows 68 and 73, 64 92 and 78, Q8_0 32 rows 65 and 73,
-// 48 79 and 78; 64 of 512 -> 1024, top 4, 48 rows 17.4 and 18.5, 18.4 and 16.5; 60 of 1536 -> 2560, top 4, Q5_1 15 rows 49 and 48, 60 107 and 81, Q8_0 83 and 44, 157 and 71; 32 of
-// 896 -> 2048, top 4, 8 rows 18 and 16, 22 and 16. A stage called by itself (alone) keeps the dp4a forms up to 256 entries, where the two lie closest.
-bool chain4_mma_pays(const b200moe_shape& s, u64 slots, u32 max_union, bool alone) {
-    if (alone && slots <= 256) return false;
-    return slots >= u64(s.down_type == B200MOE_TYPE_Q5_1 ? 4 : 3) * max_union || (s.inter >= 896 && slots >= s.experts);
+// The four-chain down on the tensor cores (down_chain4_mma.cu), else in the dp4a forms of gemv_q4k.cu. By the entries of an expert: slots over ALL experts, since of a rank's share
+// of the experts the window's slots are a share too. The dp4a forms pay by the entry, and the more the longer the rows, so the line falls with their length: from 3.5 (Q8_0) and 4.5
+// entries (Q5_1) at 128 weights to none and one at 1024. A window whose items are no more than SMs is one item's time and has the tensor cores at any number. Layers, us, the better
+// dp4a form and this: 128 experts of 640 -> 2560, top 8, Q5_1 16 rows 74.0 and 85.9, 40 115.5 and 121.4, 48 127.0 and 129.4, 64 151.8 and 139.9, a quarter of them owned 31.3 and
+// 35.3, 43.6 and 41.5, 44.2 and 41.8, 56.2 and 48.7; Q8_0 24 rows 104 and 114, 32 119 and 121, 48 146 and 138, a quarter owned 40.4 and 39.5, 48.4 and 46.8, 53.3 and 48.2; 60 of
+// 768 -> 2560, top 4, Q5_1 15 rows 48.3 and 53.2, 30 74.7 and 73.2, 45 86.6 and 78.4, Q8_0 8 rows 40.0 and 42.3, 15 52.3 and 51.5, 30 78.9 and 67.0; of 1536 -> 2560 Q5_1 8 rows
+// 64.0 and 68.9, 15 91.3 and 95.8, 60 176 and 147, Q8_0 1 row 20.0 and 19.5, 15 115 and 81; 128 of 128 -> 1024, top 8, 40 rows 30.9 and 37.8, 30.3 and 38.0, 80 38.6 and 41.1, 37.8 and
+// 41.2; one wave: 16 of 640 -> 512, top 2, 3 rows 13.1 and 12.6, 13.3 and 12.9, 8 of 64 of 512 -> 1024, top 4, 24 rows 15.8 and 14.3, 16.5 and 14.3. Over 1500 random layers (1 to
+// 256 experts, all or a half to an eighth of them owned, 128 to 2048 wide, 0.1 to 12 entries an expert) the choice lies 0.6 % above the best form's time.
+// A stage called by itself cannot ask for weights ahead, which the tensor-core form lives on more: the line lies 256 weights further, and 24 entries or fewer keep the dp4a forms
+// (16 of 640 -> 512, top 2, 3 rows, a launch, 3.7 and 4.3). So do Q5_1 rows of up to 1024 weights with 256 entries or fewer, where they are the slower ones (32 of 1024 -> 2048, top 4,
+// 64 rows 57 and 26): the line between the two dp4a forms is held by calls of that size.
+bool chain4_mma_pays(const b200moe_down_view& v, u64 slots, bool alone, u32 chunks) {
+    const b200moe_shape& s = v.shape;
+    const bool q51 = s.down_type == B200MOE_TYPE_Q5_1;
+    if (alone && slots <= (q51 && s.inter <= 1024 ? 256u : 24u)) return false;
+    if (!alone && u64(experts_met(s, slots, v.max_union)) * chunks <= static_cast<u32>(device_sm_count())) return true;
+    const u32 none = (q51 ? 1280u : 1024u) + (alone ? 256u : 0u), least = std::max(q51 ? 256u : 0u, none - std::min(none, s.inter));  // in 256ths of an entry
+    return slots * 256 > u64(s.experts) * least;
 }
 int enqueue_gate_up(const b200moe_gate_up_view& v, u32 rows, cudaStream_t st, u32 grouped_min_rows = 0, const ChainHints& hints = {}) {
     if (v.shape.gate_type == B200MOE_TYPE_Q2_K) return launch_gate_up_ds41_any(v, st);  // the generic form of the family reads every block type
@@ -389,7 +405,8 @@ int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grou
     }
     if (is_kquant(v.shape.gate_type)) {  // chain4: Q8_0 and Q5_1 blocks
         const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
-        if ((forced == 5 || (forced == 0 && chain4_mma_pays(v.shape, u64(rows) * v.shape.top_k, v.max_union, hints.slots == 0))) && chain4_mma_fits(v)) return launch_down_chain4_mma(v, hints, st);
+        const u32 chunks = forced == 0 || forced == 5 ? chain4_mma_chunks(v) : 0u;
+        if (chunks && (forced == 5 || chain4_mma_pays(v, u64(rows) * v.shape.top_k, hints.slots == 0, chunks))) return launch_down_chain4_mma(v, hints, st);
         return launch_down_q8_chain4(v, hints, st);
     }
     if (v.shape.down_type == B200MOE_TYPE_Q2_K) return launch_down_ds41_any(v, st);

@@ -293,11 +293,12 @@ bool chain_mma_plan(const b200moe_down_view& v, ChainMmaPlan* p, u32* smem) {
 
 }  // namespace
 
-bool chain4_mma_fits(const b200moe_down_view& v) {
+u32 chain4_mma_chunks(const b200moe_down_view& v) {
     ChainMmaPlan p{};
     u32 smem;
     const bool q51 = v.shape.down_type == B200MOE_TYPE_Q5_1;
-    return (q51 || v.shape.down_type == B200MOE_TYPE_Q8_0) && (!q51 || v.act.sums) && aligned(v.weights.down, 16) && chain_mma_plan(v, &p, &smem);
+    const bool fits = (q51 || v.shape.down_type == B200MOE_TYPE_Q8_0) && (!q51 || v.act.sums) && aligned(v.weights.down, 16) && chain_mma_plan(v, &p, &smem);
+    return fits ? p.n_chunks : 0u;
 }
 
 int launch_down_chain4_mma(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream) {

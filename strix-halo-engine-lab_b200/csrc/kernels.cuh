@@ -53,7 +53,7 @@ int launch_down_q4k(const b200moe_down_view& v, cudaStream_t stream);
 int launch_gate_up_ds41_any(const b200moe_gate_up_view& v, cudaStream_t stream);
 int launch_down_ds41_any(const b200moe_down_view& v, cudaStream_t stream);
 int launch_down_q8_chain4(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream);
-bool chain4_mma_fits(const b200moe_down_view& v);
+u32 chain4_mma_chunks(const b200moe_down_view& v);  // items an expert makes in the form, 0 where it does not apply
 int launch_down_chain4_mma(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream);
 
 // gemv_q4k_stream.cu: the same Q4_K contracts as persistent kernels fed by bulk copies (decode windows up to 64 rows)

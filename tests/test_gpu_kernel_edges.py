@@ -1387,7 +1387,7 @@ def test_quantize_a8_at_halves(gpu, oracle, width):
 
 
 @pytest.mark.parametrize("down_type", [7, 8])
-@pytest.mark.parametrize("rows,top_k,E,H,I,name", [(3, 1, 4, 512, 640, "stream"), (2, 2, 3, 2560, 96, "stream"), (40, 4, 16, 512, 544, "mma"), (40, 2, 4, 2560, 1024, "mma")])
+@pytest.mark.parametrize("rows,top_k,E,H,I,name", [(3, 2, 16, 2560, 640, "stream"), (2, 4, 8, 2560, 96, "stream"), (40, 4, 16, 512, 544, "mma"), (40, 2, 4, 2560, 1024, "mma")])
 def test_four_chain_down_skipped_after_its_weights_were_asked_for(gpu, oracle, rows, top_k, E, H, I, name, down_type):
     """A layer's four-chain down asks for weights before gate/up has finished: a projection that is not finite skips it with the copies in flight (no row is combined), the next
     call gives the oracle's bits."""
@@ -1410,3 +1410,25 @@ def test_four_chain_down_skipped_after_its_weights_were_asked_for(gpu, oracle, r
         assert same(layer(good, ids, w, want_raw=True)[1].cpu(), want)
     layer(good, ids, w, combine=False)
     assert b200moe.last_launch() == "down_chain4_" + name
+
+
+@pytest.mark.parametrize("down_type,rows,top_k,E,own,H,I,name", [(8, 40, 8, 128, 64, 2048, 128, "stream"), (8, 54, 8, 128, 64, 1024, 256, "mma"), (7, 40, 4, 64, 16, 2048, 512, "stream"),
+                                                                 (7, 80, 4, 64, 16, 2048, 512, "mma"), (7, 24, 8, 64, 32, 1024, 256, "stream"), (8, 8, 8, 128, 32, 1024, 640, "stream"),
+                                                                 (7, 3, 2, 16, 16, 512, 640, "mma"), (8, 5, 4, 64, 8, 1024, 96, "mma"), (7, 1, 1, 1, 1, 2048, 512, "mma")])
+def test_four_chain_tensor_core_line(gpu, oracle, down_type, rows, top_k, E, own, H, I, name):
+    """A layer's down on both sides of the line to the tensor cores, by the entries of an expert whatever part of the experts is owned, and where its items are no more than SMs."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top_k, rows)
+    first = E - own
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
+    cut = lambda t: dv(t.reshape(E, -1)[first:].reshape(-1), gpu)
+    layer = ops.MoeLayer(ops.make_shape(H, I, E, top_k, 12, down_type), cut(gate), cut(up), cut(down), capacity=rows, combine_form=b200moe.COMBINE_FMA_SLOTS)
+    raw = layer((dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu)), dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), first=first, end=E, base=first,
+                want_raw=True, combine=False)[1]
+    assert b200moe.last_launch() == "down_chain4_" + name
+    mine = ids.reshape(-1) >= first
+    assert same(raw.cpu().numpy()[mine], want[mine]) and not raw.cpu().numpy()[~mine].any()

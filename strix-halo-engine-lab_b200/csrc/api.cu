@@ -113,6 +113,11 @@ std::atomic<u32> g_debug[3] = {{0}, {0}, {0}};
 }
 u32 debug_value(u32 key) { return key < 3 ? g_debug[key].load(std::memory_order_relaxed) : 0u; }
 
+u32 experts_met(const b200moe_shape& s, u64 slots, u32 max_union) {
+    const double of = slots > max_union ? max_union : s.experts;
+    return std::min(max_union, static_cast<u32>(std::ceil(of * -std::expm1(-static_cast<double>(slots) / s.experts))));
+}
+
 namespace {
 
 constexpr u32 kMaxExperts = 1024, kMaxTopK = 32;
@@ -246,11 +251,6 @@ Window window_of(const b200moe_shape& s, u32 rows, u32 max_union) {
     if (s.experts == 1) return Window{(u64(rows) + 7) / 8, (u64(rows) + 31) / 32, rows <= 16};
     const u64 e16 = 16 * u64(rows) * s.top_k / s.experts;  // entries an expert, in sixteenths
     return Window{(max_union * std::max<u64>(16, e16 / 8 + 7) + 15) / 16, (max_union * std::max<u64>(16, (e16 + 192) / 32) + 15) / 16, e16 <= 12 * 16};
-}
-// Experts that have an entry, of the max_union that may, where the choice is spread evenly.
-u32 experts_met(const b200moe_shape& s, u64 slots, u32 max_union) {
-    const double of = slots > max_union ? max_union : s.experts;
-    return std::min(max_union, static_cast<u32>(std::ceil(of * -std::expm1(-static_cast<double>(slots) / s.experts))));
 }
 u64 waves(u64 items, u64 at_once) { return (items + at_once - 1) / at_once; }
 // Plan by window size, chosen on the host from the sizes (no environment reads inside numerical code): decode
@@ -407,7 +407,7 @@ int enqueue_down(const b200moe_down_view& v, u32 rows, cudaStream_t st, u32 grou
         const u32 forced = debug_value(B200MOE_DEBUG_DECODE_FORM);
         const u32 chunks = forced == 0 || forced == 5 ? chain4_mma_chunks(v) : 0u;
         if (chunks && (forced == 5 || chain4_mma_pays(v, u64(rows) * v.shape.top_k, hints.slots == 0, chunks))) return launch_down_chain4_mma(v, hints, st);
-        return launch_down_q8_chain4(v, hints, st);
+        return launch_down_q8_chain4(v, rows, hints, st);
     }
     if (v.shape.down_type == B200MOE_TYPE_Q2_K) return launch_down_ds41_any(v, st);
     switch (pick_q8_form(v.shape, q8_shot_down_fits(v, rows), q8_wide_down_fits(v, rows), q8_mma_down_fits(v, rows), grouped_q8_down_fits(v), rows, v.max_union, true)) {

@@ -558,16 +558,15 @@ __global__ void __launch_bounds__(256, 4) down_chain4_stream_kernel(b200moe_down
 }
 
 // Rows of an item and entries of a pass: as many rows (64, 32 or 16) as let three CTAs share a multiprocessor, fewer CTAs for rows so long that not even 16
-// do. False where the form above is the better one: rows too long for two stages, and windows of more than two rounds of items whose long rows leave a
-// multiprocessor few threads (four a row and CTA), fewer than 256, for Q5_1 with its longer decoding 512. Layers of Q4_K gate/up, this form and the one above, us (before one and two
-// entries had loops of their own here and before windows of several entries an expert left for down_chain4_mma.cu):
-// 60 experts of 2560, top 4, Q5_1: 768 wide 1 row 19.4 and 20.4, 8 rows 41.9 and 41.6, 512 rows 543 and 601; 1536 wide (192 threads) 1 row 20.9 and 26.2, 4 rows
-// 47.0 and 44.6, 8 rows 84 and 65, 512 rows 1515 and 956; 2816 wide (64 threads) 1 row 34.3 and 38.4, 512 rows 5660 and 1550. Over 1200 such layers (1 to 128 experts, 1 to 512 rows, 256 to 2816 wide) the rule
-// is 18 % faster than the form above everywhere, and slower than it by 3 to 7 % in 33.
-bool chain_plan(const b200moe_down_view& v, ChainPlan* p, u32* smem, u32* per_sm) {
+// do. False where the form above is the better one: rows too long for two stages, and windows of more than four rounds of items (over the experts that are met) whose long rows leave
+// a multiprocessor no more than 128 threads (four a row and CTA), for Q5_1 with its longer decoding fewer than 512. Layers of Q4_K gate/up, this form and the one above, us:
+// 60 experts of 2560, top 4, Q5_1: 768 wide 1 row 15.1 and 17.7, 30 rows 74.7 and 79.2; 1536 wide 1 row 17.2 and 22.6, 4 rows 40.9 and 44.7, 8 rows 64.0 and 65.8, 15 rows 96 and 91,
+// 60 rows 236 and 176; 2816 wide 1 row 23.5 and 32.2, 2 rows 36.7 and 42.0, 4 rows 60 and 66, 8 rows 137 and 95; Q8_0: 1536 wide 8 rows 74 and 82, 15 rows 115 and 121; 2816 wide
+// 1 row 29.3 and 48.6, 2 rows 45.0 and 66.6, 4 rows 108 and 94, 8 rows 174 and 142. Over 527 random layers that keep the dp4a forms the choice takes 0.7 % more than the better of the two.
+bool chain_plan(const b200moe_down_view& v, u32 rows, ChainPlan* p, u32* smem, u32* per_sm) {
     const u32 I = v.shape.inter, H = v.shape.hidden, block = v.shape.down_type == B200MOE_TYPE_Q5_1 ? kQ51Block : kQ8Block;
     const u64 row_bytes = u64(I / 32) * block;
-    p->cap = std::min<u32>(kR, std::max(1u, v.act.rows / v.shape.top_k));
+    p->cap = std::min<u32>(kR, std::max(1u, rows));
     p->a8_bytes = (p->cap * (I + I / 32 * 8) + 15u) / 16u * 16u;
     const u32 limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT), stall = debug_value(B200MOE_DEBUG_STALL_STAGE);
     p->wait_limit = limit ? limit : 1u << 18;  // about a second
@@ -578,9 +577,9 @@ bool chain_plan(const b200moe_down_view& v, ChainPlan* p, u32* smem, u32* per_sm
         p->rows_per_item = R; p->n_chunks = H / R; p->stage_bytes = static_cast<u32>(stage);
         *smem = static_cast<u32>(total);
         *per_sm = std::max(1u, std::min(2048u / (4u * R), 227u * 1024u / (*smem + 1024u)));
-        const u64 items = u64(p->n_chunks) * v.max_union, at_once = u64(*per_sm) * static_cast<u32>(device_sm_count());
-        if (4u * R * *per_sm < (block == kQ51Block ? 512u : 256u) && items > 2 * at_once) return false;
-        return items < (1u << 30);
+        const u64 at_once = u64(*per_sm) * static_cast<u32>(device_sm_count());
+        if (4u * R * *per_sm < (block == kQ51Block ? 512u : 129u) && u64(p->n_chunks) * experts_met(v.shape, u64(rows) * v.shape.top_k, v.max_union) > 4 * at_once) return false;
+        return u64(p->n_chunks) * v.max_union < (1u << 30);
     }
     return false;
 }
@@ -638,13 +637,13 @@ int launch_down_q4k(const b200moe_down_view& v, cudaStream_t stream) {
     return after_launch("down_q4k");
 }
 
-int launch_down_q8_chain4(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream) {
+int launch_down_q8_chain4(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream) {
     const u32 H = v.shape.hidden, I = v.shape.inter;
     if (v.max_union == 0) return B200MOE_OK;
     const bool q51 = v.shape.down_type == B200MOE_TYPE_Q5_1;
     ChainPlan p{};
     u32 smem = 0, per_sm = 0;
-    if (debug_value(B200MOE_DEBUG_DECODE_FORM) != 3 && aligned(v.weights.down, 16) && chain_plan(v, &p, &smem, &per_sm)) {
+    if (debug_value(B200MOE_DEBUG_DECODE_FORM) != 3 && aligned(v.weights.down, 16) && chain_plan(v, rows, &p, &smem, &per_sm)) {
         p.early = hints.routes_done;
         const u32 grid = static_cast<u32>(std::min<u64>(u64(per_sm) * static_cast<u32>(device_sm_count()), u64(p.n_chunks) * v.max_union));
         const auto kernel = q51 ? down_chain4_stream_kernel<true> : down_chain4_stream_kernel<false>;

@@ -52,7 +52,7 @@ int launch_down_q4k(const b200moe_down_view& v, cudaStream_t stream);
 // gemv_ds41_any.cu: the DS41 family over any of its block types (Q8_0, Q2_K), one weight row per warp, weights read in place.
 int launch_gate_up_ds41_any(const b200moe_gate_up_view& v, cudaStream_t stream);
 int launch_down_ds41_any(const b200moe_down_view& v, cudaStream_t stream);
-int launch_down_q8_chain4(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream);
+int launch_down_q8_chain4(const b200moe_down_view& v, u32 rows, const ChainHints& hints, cudaStream_t stream);
 u32 chain4_mma_chunks(const b200moe_down_view& v);  // items an expert makes in the form, 0 where it does not apply
 int launch_down_chain4_mma(const b200moe_down_view& v, const ChainHints& hints, cudaStream_t stream);
 
@@ -90,6 +90,7 @@ int launch_gate_up_q8_grouped(const b200moe_gate_up_view& v, cudaStream_t stream
 int launch_down_q8_grouped(const b200moe_down_view& v, cudaStream_t stream);
 // value of a B200MOE_DEBUG_* hook (api.cu)
 u32 debug_value(u32 key);
+u32 experts_met(const b200moe_shape& s, u64 slots, u32 max_union);  // that have an entry, of the max_union that may, where the choice is spread evenly (api.cu)
 
 // prologue.cu: A8 + router logits of a decode window (rows <= 8) in one launch; q.x / q.x_is_bf16 say where the activations are (r.x is not read)
 bool prologue_fusable(const b200moe_router_view& r);

@@ -1432,3 +1432,21 @@ def test_four_chain_tensor_core_line(gpu, oracle, down_type, rows, top_k, E, own
     assert b200moe.last_launch() == "down_chain4_" + name
     mine = ids.reshape(-1) >= first
     assert same(raw.cpu().numpy()[mine], want[mine]) and not raw.cpu().numpy()[~mine].any()
+
+
+@pytest.mark.parametrize("down_type,rows,top_k,E,H,I,name", [(8, 1, 8, 32, 2048, 2048, "down_chain4_stream"), (7, 2, 4, 60, 2560, 1536, "down_chain4_stream"), (8, 3, 4, 40, 2048, 2816, "down_q8_chain4"),
+                                                             (7, 5, 4, 40, 2048, 2816, "down_q8_chain4")])
+def test_four_chain_dp4a_forms_by_rounds(gpu, oracle, down_type, rows, top_k, E, H, I, name):
+    """Both sides of four rounds of items, in a workspace of the window's size and in a larger one."""
+    import b200moe
+    from b200moe import ops, synth
+    rng = np.random.default_rng(rows + I)
+    gate, up, down = synth.expert_tensors(rng, E, H, I, 12, down_type)
+    ids = window(rng, E, top_k, rows)
+    codes, deltas, sums = oracle.quantize_a8(rng.standard_normal((rows, H), dtype=np.float32))
+    want = oracle.experts(O.Shape(H, I, E, top_k, 12, down_type, float("inf")), gate, up, down, ids, codes, deltas, sums)["raw"]
+    w, x = (dv(gate, gpu), dv(up, gpu), dv(down, gpu)), (dv(codes, gpu), dv(deltas, gpu), dv(sums, gpu))
+    for capacity in (rows, 64):
+        layer = ops.MoeLayer(ops.make_shape(H, I, E, top_k, 12, down_type), *w, capacity=capacity, combine_form=b200moe.COMBINE_FMA_SLOTS)
+        raw = layer(x, dv(ids.view(np.int32), gpu), torch.ones((rows, top_k), device=gpu), want_raw=True, combine=False)[1]
+        assert b200moe.last_launch() == name and same(raw.cpu(), want)

@@ -1,5 +1,6 @@
 """A down stage is left out by whole blocks: a block of the same launch whose wait ran out may raise the job summary while others read it, and threads that read the word one by
-one could part in front of a barrier or of copies that each of them has a share of. So the kernels of the stage read the word to leave through one helper alone."""
+one could part in front of a barrier or of copies that each of them has a share of. So the kernels of the stage read the word to leave through one helper alone. An early launch of
+the segment-streaming kernel has a producer warp read it for its group, whose consumers leave by an end mark."""
 import glob
 import os
 import re
@@ -14,4 +15,5 @@ def test_the_summary_is_read_by_the_block():
     assert len(kernels) >= 11
     for name, s in kernels.items():
         assert "block_skips(" in s, name
-        assert not re.search(r"\*\s*[av]\.summary", s), name
+        reads = re.findall(r"[^\n]*\*\s*[av]\.summary[^\n]*", s)
+        assert [r.strip() for r in reads] == (["u32 skips = DOWN && a.summary ? *a.summary : 0u;"] if name == "gemv_q4k_wide.cu" else []), name

@@ -297,7 +297,10 @@ q4k_wide_kernel(const __grid_constant__ WideMaps maps, WideArgs a, WidePlan plan
     if (tid < kGroups * plan.stages + (PAIR ? kConsumerWarps : 2 * kGroups)) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 
     if (!early) chain_begin();
-    if (DOWN && !early && block_skips(a.summary)) return;  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
+    if (DOWN && !early && block_skips(a.summary)) {  // a failed or aborted projection skips the whole stage (routed_expert.hpp:17-19)
+        if (!PAIR && tid == 0) retire_block(claim);
+        return;
+    }
 
     // ---- the virtual expert list (the stage area is free until the first copy is issued: it holds the copied routes)
     if (plan.dense_rows) build_dense_list(plan.dense_rows, plan.n_chunks, table, ctl);

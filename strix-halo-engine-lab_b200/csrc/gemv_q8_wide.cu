@@ -105,11 +105,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 q8_wide_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, Q8Args a, Q8Plan plan) {
     chain_begin();
     extern __shared__ __align__(128) unsigned char smem[];
-    if (DOWN && block_skips(a.summary)) return;
+    u32* claim = a.routes.counts + 3;  // the grid's claim word (wide_common.cuh)
+    if (DOWN && block_skips(a.summary)) {
+        if (threadIdx.x == 0) retire_block(claim);
+        return;
+    }
     u32 n_union = a.routes.counts[0];
     if (n_union == 0) return;
     if (n_union > plan.max_union) n_union = plan.max_union;
-    u32* claim = a.routes.counts + 3;  // the grid's claim word (wide_common.cuh)
 
     unsigned char* at = smem + kGroups * plan.stages * plan.stage_bytes;
     float* s_gu = reinterpret_cast<float*>(at);  // [group][buffer][gate | up][entry][32]

@@ -43,11 +43,14 @@ __device__ __forceinline__ u32 warp_inclusive_scan(u32 v, u32 lane) {
 constexpr u32 kClaimBits = 22, kClaimMask = (1u << kClaimBits) - 1u;
 __host__ __device__ constexpr u32 work_list_scratch_words(u32 max_union, u32 vmax) { return 2 * max_union + 2 + vmax + kKE; }
 __device__ __forceinline__ u32 claim_item(u32* claim) { return atomicAdd(claim, 1u) & kClaimMask; }
-// Called once per producer warp (lane 0) when it will claim no more; ctl[1] counts the CTA's producers that have finished.
-__device__ __forceinline__ void retire_claims(u32* claim, u32* ctl) {
-    if (atomicAdd(&ctl[1], 1u) != kGroups - 1u) return;
+// Once a CTA, by one thread: it will claim no more. A CTA that is left out retires too, since one that is not may have made claims.
+__device__ __forceinline__ void retire_block(u32* claim) {
     const u32 before = atomicAdd(claim, 1u << kClaimBits);
     if ((before >> kClaimBits) == gridDim.x - 1u) atomicExch(claim, 0u);
+}
+// Called once per producer warp (lane 0) when it will claim no more; ctl[1] counts the CTA's producers that have finished.
+__device__ __forceinline__ void retire_claims(u32* claim, u32* ctl) {
+    if (atomicAdd(&ctl[1], 1u) == kGroups - 1u) retire_block(claim);
 }
 
 // Builds the work list: `table` gets the virtual experts (an expert of the union with at most kKE of its entries; an expert

@@ -108,9 +108,9 @@ int launch_widen_bf16(const u16* in, float* out, u64 count, cudaStream_t stream)
     return after_launch("widen_bf16");
 }
 
-// Four values a lane need whole 16- (FP32) or 8-byte (bfloat16) units in x and 4-byte units in the codes; the one-value form
-// takes every other layout, and what its blocks of eight groups cover with one an SM: there one division a lane is shorter than four
-// in a row (1 row of 256: 1.43 against 1.47 us, 8 rows of 2048: 1.84 against 1.91; 8 rows of 7168, above the line: 1.95 against 1.88).
+// Four values a lane need whole 16- (FP32) or 8-byte (bfloat16) units in x and 4-byte units in the codes. The one-value form takes every other layout, and what its blocks of eight
+// groups cover with three an SM: up to there a launch is one block's chain, whose reductions are one instruction each (FP32, us, one value and four: 1 row of 256 1.09 and 1.26, 8 of
+// 2048 1.16 and 1.41, 8 of 7168 1.24 and 1.43, 16 of 7168, above the line, 1.43 and 1.45, 20 of 7168 2.02 and 1.41; bfloat16 alike).
 bool quantize_a8_vec_ok(const b200moe_quantize_a8_view& v) {
     const u32 x_stride = v.x_stride ? v.x_stride : v.width;
     return aligned(v.x, v.x_is_bf16 ? 8 : 16) && x_stride % 4 == 0 && aligned(v.out.codes, 4) && u64(v.rows) * (v.width / 32) < (1ull << 28);
@@ -121,7 +121,7 @@ int launch_quantize_a8(const b200moe_quantize_a8_view& v, cudaStream_t stream, f
     const u64 items = u64(v.rows) * groups;
     if (items == 0) return B200MOE_OK;
     const u32 x_stride = v.x_stride ? v.x_stride : v.width, stride = v.out.stride ? v.out.stride : v.width;
-    if (quantize_a8_vec_ok(v) && (wide || items > 8u * static_cast<u32>(device_sm_count()))) {
+    if (quantize_a8_vec_ok(v) && (wide || items > 3u * 8u * static_cast<u32>(device_sm_count()))) {
         const u32 vec_blocks = static_cast<u32>((items + 31) / 32);
         // n / groups = n * per_group >> shift for every n below 2^28: per_group * groups lies between 2^shift and 2^shift + groups, and groups is no more than 2^(shift - 28).
         u32 shift = 28;

@@ -363,10 +363,11 @@ def test_rmsnorm_forms_at_their_lines(gpu, oracle, n, per_sm):
         assert same(y.cpu(), want) and np.array_equal(codes.cpu().numpy(), wc) and same(deltas.cpu(), wd) and np.array_equal(sums.cpu().numpy(), ws)
 
 
-@pytest.mark.parametrize("rows,width,offset", [(37, 1024, 0), (38, 1024, 0), (38, 1024, 4), (38, 1024, 1), (38, 1024, 2), (401, 96, 0)])
+@pytest.mark.parametrize("rows,width,offset", [(37, 1024, 0), (38, 1024, 0), (38, 1024, 4), (38, 1024, 1), (38, 1024, 2), (401, 96, 0),
+                                                (111, 1024, 0), (112, 1024, 0), (112, 1024, 4), (112, 1024, 1), (112, 1024, 2), (1190, 96, 0)])
 @pytest.mark.parametrize("bf16", [False, True])
 def test_quantizer_sizes(gpu, oracle, rows, width, offset, bf16):
-    """More groups than one block of the one-value form an SM holds (8 x 148 = 1184): four values a lane where x allows whole loads,
+    """Groups about one and about three blocks of the one-value form an SM (8 x 148 = 1184, 3552): four values a lane from there where x allows whole loads,
     the last warp partly spare; a NaN and an infinity are flagged."""
     from b200moe import ops
     rng = np.random.default_rng(rows + offset)

@@ -1326,7 +1326,8 @@ def test_rmsnorm_rows_over_several_blocks(gpu, oracle, n, rows):
     assert np.array_equal(status.cpu().numpy() != 0, np.arange(rows) == rows // 2)
 
 
-@pytest.mark.parametrize("I,down_type", [(32, 8), (32, 7), (96, 8), (160, 7), (544, 8), (544, 7), (768, 8), (1056, 8), (1536, 8), (1536, 7), (2048, 7)])
+@pytest.mark.parametrize("I,down_type", [(32, 8), (32, 7), (96, 8), (160, 7), (544, 8), (544, 7), (768, 8), (1056, 8), (1536, 8), (1536, 7), (2048, 7),
+                                         (1184, 8), (1280, 8), (1024, 7), (1152, 7), (1472, 7)])
 def test_four_chain_down_on_tensor_cores(gpu, oracle, I, down_type):
     """Experts of 1, 8, 9, 17, 33 and 70 entries against steps of 16 and 32; items of 64 and 32 rows; fewer groups than chains, odd group counts (Q8_0 rows that start between words);
     more items than CTAs and fewer."""

@@ -40,9 +40,7 @@ __device__ __forceinline__ void mma_s8(int (&d)[4], const u32 (&a)[4], u32 b0, u
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
 }
 
-__device__ __forceinline__ u32 lds32(u32 a) { u32 v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
 __device__ __forceinline__ u32 lds16(u32 a) { u16 v; asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a)); return v; }
-__device__ __forceinline__ uint2 lds64(u32 a) { uint2 v; asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a)); return v; }
 
 // A row's blocks of one chain, for one lane: its quants 4 t .. 4 t + 3 and 16 + 4 t .., the factor and the minimum. Four Q8_0 blocks are whole words, so all of a chain's blocks
 // of a row begin alike, on a word or between two. A word past the block's end may be read, of which nothing is used.
@@ -127,7 +125,6 @@ __global__ void __launch_bounds__(kChainThreads, 1) down_chain4_mma_kernel(b200m
         return;
     }
     const u32 stride = v.act.stride ? v.act.stride : v.act.width;
-    const bool vec = reinterpret_cast<uintptr_t>(v.act.codes) % 16 == 0 && stride % 16 == 0;
     struct Step { Item item; u32 first, nr, last; };  // entries first .. first + nr; whether they are the item's last
     auto step_at = [&](const Item& x, u32 first) {
         const u32 end = s_begins[x.j + 1], nr = min(kCap, end - first);
@@ -154,8 +151,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) down_chain4_mma_kernel(b200m
             if (lane == 0) s_slots[b][r] = mine[k];
             unsigned char* to = a8 + b * a8_bytes + r * kCell;
             const i8* c = v.act.codes + u64(mine[k]) * stride;
-            if (vec) for (u32 i = lane; i < 2u * groups; i += 32) cp_async16(to + (i >> 1) * (kCap * kCell) + 16u * (i & 1u), c + 16u * i);
-            else for (u32 i = lane; i < 8u * groups; i += 32) *reinterpret_cast<u32*>(to + (i >> 3) * (kCap * kCell) + 4u * (i & 7u)) = *reinterpret_cast<const u32*>(c + 4u * i);
+            for (u32 i = lane; i < 2u * groups; i += 32) cp_async16(to + (i >> 1) * (kCap * kCell) + 16u * (i & 1u), c + 16u * i);
             const float* deltas = v.act.deltas + u64(mine[k]) * (stride / 32);
             const i32* sums = v.act.sums + u64(mine[k]) * (stride / 32);
             for (u32 i = lane; i < groups; i += 32) {
@@ -264,7 +260,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) down_chain4_mma_kernel(b200m
     }
 }
 
-// Rows of an item and entries of a step: 64 x 32, 64 x 16 (a step's rows come out of L2 once an item), 32 x 32 or 32 x 16, as shared memory allows; false where rows are too long for that.
+// Rows of an item and entries of a step: 64 x 32, 64 x 16 (a step's rows come out of L2 once an item), 32 x 32 (Q8_0; a group of Q5_1 takes in it what it takes in 64 x 16) or
+// 32 x 16, as shared memory allows; false where rows are too long for that. H is whole blocks of a K-quant gate/up, a multiple of 256.
 bool chain_mma_plan(const b200moe_down_view& v, ChainMmaPlan* p, u32* smem) {
     const u32 H = v.shape.hidden, groups = v.shape.inter / 32, row_bytes = groups * (v.shape.down_type == B200MOE_TYPE_Q5_1 ? kQ51Block : kQ8Block);
     const u32 limit = debug_value(B200MOE_DEBUG_WAIT_LIMIT), stall = debug_value(B200MOE_DEBUG_STALL_STAGE);
@@ -279,12 +276,11 @@ bool chain_mma_plan(const b200moe_down_view& v, ChainMmaPlan* p, u32* smem) {
     constexpr u32 forms[4][2] = {{64, 32}, {64, 16}, {32, 32}, {32, 16}};
     for (u32 i = 0; i < 4; ++i) {
         const u32 R = forms[i][0], cap = forms[i][1];
-        if (H % R) continue;
         p->form = i;
         p->n_chunks = H / R;
         p->stage_bytes = (R * row_bytes + R / p->copy_rows * p->row_gap + 127u) / 128u * 128u;
         const u64 total = 2 * u64(p->stage_bytes) + 2 * u64(groups) * cap * kCell + 4 * u64(cap) * (R + 4) * 4 + (2 * u64(v.max_union) + 1) * 4;
-        if (total > 226u * 1024u) continue;
+        if (total > 226u * 1024u || (i == 2 && v.shape.down_type == B200MOE_TYPE_Q5_1)) continue;
         *smem = static_cast<u32>(total);
         return u64(p->n_chunks) * v.max_union < (1u << 30);
     }
@@ -310,7 +306,7 @@ int launch_down_chain4_mma(const b200moe_down_view& v, const ChainHints& hints, 
     const bool q51 = v.shape.down_type == B200MOE_TYPE_Q5_1;
     const auto kernel = p.form == 0 ? (q51 ? down_chain4_mma_kernel<true, 4, 1, 4> : down_chain4_mma_kernel<false, 4, 1, 4>)
                       : p.form == 1 ? (q51 ? down_chain4_mma_kernel<true, 4, 1, 2> : down_chain4_mma_kernel<false, 4, 1, 2>)
-                      : p.form == 2 ? (q51 ? down_chain4_mma_kernel<true, 2, 2, 2> : down_chain4_mma_kernel<false, 2, 2, 2>)
+                      : p.form == 2 ? down_chain4_mma_kernel<false, 2, 2, 2>
                                     : (q51 ? down_chain4_mma_kernel<true, 2, 2, 1> : down_chain4_mma_kernel<false, 2, 2, 1>);
     const u32 grid = static_cast<u32>(std::min<u64>(static_cast<u32>(device_sm_count()), u64(p.n_chunks) * v.max_union));
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;

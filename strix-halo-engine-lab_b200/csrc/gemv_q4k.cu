@@ -443,7 +443,6 @@ __global__ void __launch_bounds__(256, 4) down_chain4_stream_kernel(b200moe_down
     }
     unsigned char* a8 = smem_raw + 2 * plan.stage_bytes;
     const u32 stride = v.act.stride ? v.act.stride : v.act.width;
-    const bool vec = reinterpret_cast<uintptr_t>(v.act.codes) % 16 == 0 && stride % 16 == 0;
     // entries [first, first + nr) into buffer b: codes[nr][I], deltas[cap][groups], sums[cap][groups]
     auto stage = [&](u32 b, u32 first, u32 nr) {
         unsigned char* to = a8 + b * plan.a8_bytes;
@@ -453,8 +452,7 @@ __global__ void __launch_bounds__(256, 4) down_chain4_stream_kernel(b200moe_down
             const u32 slot = load(v.routes.slots + first + r);
             if (tid == 0) s_slots[b][r] = slot;
             const i8* c = v.act.codes + u64(slot) * stride;
-            if (vec) for (u32 i = tid; i < I / 16; i += blockDim.x) grouped::cp_async16(to + r * I + 16u * i, c + 16u * i);
-            else for (u32 i = tid; i < I / 4; i += blockDim.x) *reinterpret_cast<u32*>(to + r * I + 4u * i) = *reinterpret_cast<const u32*>(c + 4u * i);
+            for (u32 i = tid; i < I / 16; i += blockDim.x) grouped::cp_async16(to + r * I + 16u * i, c + 16u * i);
             const float* d = v.act.deltas + u64(slot) * (stride / 32);
             const i32* sm = v.act.sums ? v.act.sums + u64(slot) * (stride / 32) : nullptr;
             for (u32 i = tid; i < groups; i += blockDim.x) {

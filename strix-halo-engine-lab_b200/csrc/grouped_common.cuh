@@ -26,6 +26,10 @@ __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 to_float(int2 v) { return make_float2(static_cast<float>(v.x), static_cast<float>(v.y)); }
 __device__ __forceinline__ float2 pick(bool c, float2 x, float2 y) { return make_float2(c ? x.x : y.x, c ? x.y : y.y); }
 
+// Shared memory by explicit 32-bit addresses.
+__device__ __forceinline__ u32 lds32(u32 a) { u32 v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ uint2 lds64(u32 a) { uint2 v; asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a)); return v; }
+
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(q4k::saddr(dst)), "l"(src) : "memory");
 }

@@ -76,16 +76,18 @@ const char* b200moe_last_launch(void);
  * bounded wait run out WITHOUT a device fault and so that the forms of the decode GEMVs can be compared on one input; a
  * production caller never sets them. The reference has the same kind of seam (TierDev::timeout_ns,
  * src/cuda/tiered_experts.cu:107-127). Returns B200MOE_ERR_INVALID_ARGUMENT for an unknown key. */
-#define B200MOE_DEBUG_WAIT_LIMIT 0u  /* polls of every bounded wait in the segment-streaming, the one-item Q8_0 and the grouped Q8_0 kernels and the four-chain
-                                      * down; 0 = the default (2^22; grouped Q8_0 2^20; one-item and four-chain 2^18). The grouped Q4_K kernel's limit (2^18, about
-                                      * a second) and the row-streaming Q4_K kernels' are fixed */
-#define B200MOE_DEBUG_STALL_STAGE 1u /* n > 0: in every CTA of the Q4_K segment-streaming kernel the first producer, in every CTA of a grouped
-                                      * kernel all producers, in every CTA of the one-item Q8_0 kernel and of the four-chain down its only one stop feeding before
-                                      * their n-th stage (no copy of that stage is issued, none is left in flight); 0 = never */
-#define B200MOE_DEBUG_DECODE_FORM 2u /* gate/up and down: 0 = chosen by the plan, 1 = row streaming (Q4_K), 2 = segment streaming (Q4_K;
-                                      * Q8_0: the dp4a token-block form), 3 = per-block (Q8_0: one row per warp), 4 = the Q8_0
-                                      * tensor-core form, 5 = the grouped form, 6 = the Q8_0 one-item form (each only where it applies; grouped_min_rows is not
-                                      * looked at then) */
+#define B200MOE_DEBUG_WAIT_LIMIT 0u  /* polls of every bounded wait in the segment-streaming, the one-item Q8_0 and the grouped Q8_0 kernels and in the four-chain
+                                      * downs by bulk copies and on the tensor cores; 0 = the default (2^22; grouped Q8_0 2^20; one-item and four-chain 2^18). The
+                                      * grouped Q4_K kernel's limit (2^18, about a second) and the row-streaming Q4_K kernels' are fixed */
+#define B200MOE_DEBUG_STALL_STAGE 1u /* n > 0: in every CTA of the Q4_K / Q5_K segment-streaming kernel the first producer, in every CTA of a grouped
+                                      * kernel, of the one-item Q8_0 kernel and of the four-chain downs by bulk copies (one thread) and on the tensor cores (a lane
+                                      * of each warp) all that ask for weights stop before their n-th stage or item (no copy of it is issued, none is left in
+                                      * flight); 0 = never */
+#define B200MOE_DEBUG_DECODE_FORM 2u /* gate/up and down: 0 = chosen by the plan, 1 = row streaming (Q4_K), 2 = segment streaming (Q4_K; Q5_K
+                                      * gate/up; Q8_0: the dp4a token-block form), 3 = per-block (Q8_0: one row per warp; four-chain down: the
+                                      * register form), 4 = the Q8_0 tensor-core form, 5 = the grouped form (four-chain down: on the tensor cores), 6 = the Q8_0
+                                      * one-item form (each only where it applies; grouped_min_rows is not looked at then). 1, 2, 4 and 6 leave the four-chain
+                                      * down to its dp4a forms */
 int b200moe_debug_set(uint32_t key, uint32_t value);
 
 /* ------------------------------------------------------------------------------------------------ A8 activations

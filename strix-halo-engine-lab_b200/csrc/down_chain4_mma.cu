@@ -5,9 +5,9 @@
 // entries, whose A8 rows come by asynchronous copies a step ahead; the weights stay for the item's further steps. A warp has one chain of 16 weight rows (the MMA's rows)
 // against the step's entries, eight an MMA (mma.sync m16n8k32, s8 x s8, one block); the chains meet in shared memory at the step's end, and a warp an entry stores the sums.
 // One CTA of 16 warps an SM: two items and two steps of long rows fill its shared memory.
-// What bounds it: issue slots (55 to 64 % busy with four warps a scheduler) - 33 instructions a block and warp with eight entries, 15 more for every further eight, where the dp4a
-// forms take 18 for 32 cells - and, with few entries, a step's ends: two barriers, the entries' copies, the meeting. More items in flight and two CTAs of 8 warps an SM gave
-// nothing; a k order that reads 8 Q8_0 quants as three words cost bank conflicts (1024 rows below 182 -> 186 us).
+// What bounds it: latency with four warps a scheduler (issue slots 47 to 59 % busy; a warp's wait between dependent instructions and, with few entries, a step's ends - two barriers,
+// the entries' copies, the meeting - are the top stalls) and the instructions beside the MMAs: 67 of all warps an MMA at 8 entries an expert (95 of Q5_1), 41 at 64. More items in flight
+// and two CTAs of 8 warps an SM gave nothing; a k order that reads 8 Q8_0 quants as three words cost bank conflicts (1024 rows below 182 -> 186 us).
 // 64 experts of 768 -> 2560, top 4, Q8_0, us a launch, the dp4a form and this: 64 rows 69 and 43, 128 111 and 48, 1024 686 and 164.
 // Q8_0 blocks are 34 bytes: a lane reads two words and a byte permute puts its quants together where they do not lie on one.
 // Every wait is bounded; where one runs out B200MOE_JOB_WAIT_ABORTED is set in the job summary once the copies in flight have landed.

@@ -1,5 +1,5 @@
-// Routes of a decode window (up to 1024 slots, up to 1024 experts) built by ONE block of any size, or by one warp: device code shared by
-// the stand-alone routes kernels and the launch that selects too (routes.cu).
+// Routes of a decode window (up to 1024 slots, up to 1024 experts) built by ONE block of any size, or by one warp: device code of
+// the stand-alone routes kernels (routes.cu); the launch that selects too has a build of its own.
 // Contract: strix::ds41::build_window_routes + restrict_routes (src/ds41_moe.cpp:11-61), see routes.cu.
 #pragma once
 #include "common.cuh"
@@ -168,8 +168,7 @@ __device__ __forceinline__ void routes_one_warp(const b200moe_routes_view& v, u3
     }
 }
 
-// The whole build of a window of up to kChunk slots by one block. ids: the slots' experts, global or shared memory (written before a barrier);
-// counts: counts_bytes(slots, experts) of shared memory. A slot's place in its row, the row's low count and check come from the row's ids in
+// The whole build of a window of up to kChunk slots by one block. ids: the slots' experts; counts: counts_bytes(slots, experts) of shared memory. A slot's place in its row, the row's low count and check come from the row's ids in
 // shared memory, its place among its expert's entries from the ranks above and one scan over the experts: five block barriers.
 __device__ inline void routes_small_body(const b200moe_routes_view& v, u32 end, const u32* ids, u16* counts) {
     __shared__ u32 sid[kChunk], ent[kChunk], ebegin[1024], warp_tot[32], total_s, maxc;

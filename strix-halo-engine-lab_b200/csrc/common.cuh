@@ -93,13 +93,25 @@ __device__ __forceinline__ u32 load_l2(const u32* p) { return __ldcg(p); }
 __device__ __forceinline__ bool block_skips(const u32* summary) { return __syncthreads_or(summary && *summary) != 0; }
 // Enqueues a kernel of the chain; its status is read by after_launch.
 template <class... P, class... A>
-inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, cudaStream_t stream, A&&... args) {
-    cudaLaunchAttribute attr[1];
+inline void chain_launch_attrs(u32 extra, void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxL1;
     cudaLaunchConfig_t c{};
-    c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = attr; c.numAttrs = 1;
+    c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = attr; c.numAttrs = 1 + extra;
     (void)cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, cudaStream_t stream, A&&... args) {
+    chain_launch_attrs(0, kernel, grid, block, smem, stream, std::forward<A>(args)...);
+}
+// The same for a kernel that reads its weights several times out of L1, of no more CTAs than multiprocessors: behind a launch that takes all shared memory it would run with the
+// L1 that is left beside that. With several CTAs a multiprocessor the preference would cost their places.
+template <class... P, class... A>
+inline void chain_launch_l1(void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, cudaStream_t stream, A&&... args) {
+    chain_launch_attrs(u64(grid.x) * grid.y * grid.z <= static_cast<u64>(device_sm_count()) ? 1u : 0u, kernel, grid, block, smem, stream, std::forward<A>(args)...);
 }
 // Whether a launch of so many CTAs, several of which share a multiprocessor, is better a programmatic one. Such CTAs come onto the multiprocessors as the launch in
 // front leaves them, so that what leaves first gets as many as it can hold and the others none: up to two a multiprocessor that does not matter, and the start

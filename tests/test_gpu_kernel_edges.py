@@ -1305,7 +1305,7 @@ def test_grouped_gate_up_of_mixed_layers(gpu, oracle, I, down_type):
 
 
 @pytest.mark.parametrize("n", [32, 480, 512, 2048, 2080, 2560, 2592, 4096, 4128, 8448])
-@pytest.mark.parametrize("rows", [1, 9, 160, 300])
+@pytest.mark.parametrize("rows", [1, 9, 160, 186, 300, 1600])
 def test_rmsnorm_rows_over_several_blocks(gpu, oracle, n, rows):
     """A row's values in whole and broken batches, over one to many blocks, with results apart from the rows and on them; a row of infinities beside."""
     import b200moe

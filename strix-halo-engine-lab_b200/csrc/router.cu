@@ -225,9 +225,10 @@ __global__ void __launch_bounds__(128 * WR) router_logits_tile_kernel(const floa
 namespace b200moe {
 namespace {
 
-// One warp per row; shared memory per warp: scores[experts] + choice[experts] + 32 group scores.
+// One warp per row; shared memory per warp: scores[experts] + choice[experts] + 32 group scores. 32 experts a lane took 96 registers, five CTAs a multiprocessor: 3000 rows of 1024 a
+// second wave, 32 us, 26 with six.
 template <int EPL>
-__global__ void __launch_bounds__(128) router_select_kernel(const float* logits, float* scores_out, const float* bias,
+__global__ void __launch_bounds__(128, EPL == 32 ? 6 : 1) router_select_kernel(const float* logits, float* scores_out, const float* bias,
                                                             const __grid_constant__ b200moe_route_policy p, u32 rows, u32* ids,
                                                             float* weights) {
     chain_begin();
@@ -237,6 +238,8 @@ __global__ void __launch_bounds__(128) router_select_kernel(const float* logits,
     if (row >= rows) return;
     select_detail::select_row<EPL>(logits, scores_out, bias, p, row, lane, smem + warp * select_detail::scratch_floats(p.experts), ids, weights);
 }
+
+// One warp per row; shared memory per warp: scores[experts] + choice[experts] + 32 group scores.
 
 }  // namespace
 
@@ -285,10 +288,15 @@ int launch_router_logits(const b200moe_router_view& v, cudaStream_t stream, cons
 int launch_router_select(const b200moe_router_view& v, cudaStream_t stream) {
     if (v.rows == 0) return B200MOE_OK;
     // A launch admitted early is placed wherever the one in front leaves room, by the dozen on the first multiprocessors that come free. So a CTA asks for its share of a
-    // multiprocessor's shared memory. Selection alone, us, without and with: 4096 rows of 128 8.4 and 6.3, of 256 13.1 and 9.6; a call of 1609 rows over 160 experts 444.7 and 440.6.
-    const u32 ctas = (v.rows + 3) / 4, sms = static_cast<u32>(device_sm_count()), share = ctas > sms ? 227u * 1024u / ((ctas + sms - 1) / sms) : 0u;
-    const u32 scratch = 4u * select_detail::scratch_floats(v.policy.experts) * sizeof(float), smem = std::max(scratch, share > 2048u ? std::min(share - 1024u, 100u * 1024u) & ~15u : 0u);
-    const auto kernel = v.policy.experts <= 128u ? router_select_kernel<4> : v.policy.experts <= 256u ? router_select_kernel<8> : router_select_kernel<32>;
+    // multiprocessor's shared memory, from seven CTAs for eight multiprocessors on (48 to 128 experts: from more than one each). Below 48 experts the logits in front leave
+    // multiprocessors free that hold all of the CTAs, and it pays only from five a multiprocessor on. us, without and with: selection alone, 4096 rows of 128 8.4 and 6.3, of 256 13.1 and
+    // 9.6; with logits over 512, 1400 rows of 160 22.6 and 18.1, 592 of 256 19.2 and 13.9, 1400 of 16 6.5 and 7.6.
+    const u32 experts = v.policy.experts, ctas = (v.rows + 3) / 4, sms = static_cast<u32>(device_sm_count()), eighths = experts < 48u ? 40u : experts <= 128u ? 8u : 7u;
+    const u32 share = u64(ctas) * 8u > u64(eighths) * sms ? 227u * 1024u / ((ctas + sms - 1) / sms) : 0u;
+    const u32 scratch = 4u * select_detail::scratch_floats(experts) * sizeof(float), smem = std::max(scratch, share > 2048u ? std::min(share - 1024u, 100u * 1024u) & ~15u : 0u);
+    // Groups that no row of takes the fast path (12, 20 or 48 experts, say) have a kernel of the general path alone: 64 rows, 96 experts in 8 groups 13.6 us, 15.9 with
+    // that path called out of line, 384 experts 25.4 and 34.
+    const auto kernel = !select_detail::fast_groups(v.policy) ? router_select_kernel<0> : experts <= 128u ? router_select_kernel<4> : experts <= 256u ? router_select_kernel<8> : router_select_kernel<32>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
     small_launch(kernel, ctas, 128, smem, stream, v.logits, v.scores, v.bias, v.policy, v.rows, v.ids, v.weights);
     return after_launch("router_select");

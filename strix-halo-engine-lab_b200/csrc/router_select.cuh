@@ -245,9 +245,8 @@ __device__ __forceinline__ u32 finish_row(const b200moe_route_policy& p, u32 row
 // One warp selects one row; select_row returns lane k's id in output order (lanes from top_k on: nothing of meaning). `s` points to this warp's scratch of 2 * experts + 32 floats on
 // a 16-byte boundary (shared memory).
 __host__ __device__ constexpr u32 scratch_floats(u32 experts) { return (2u * experts + 32u + 3u) & ~3u; }
-// The general path of a row: any groups, any values (the serial rules where a NaN is among the choices). Out of line, so that a call's instructions lie in one piece: the kernels
-// run once a call on cold instruction caches, where every jump over code that is not run costs 500 to 1,000 clocks. Returns lane k's pick k.
-static __device__ __noinline__ u32 select_row_general(const float* logits, float* scores_out, const float* bias, const b200moe_route_policy& p, u32 row, u32 lane, float* s) {
+// The general path of a row: any groups, any values (the serial rules where a NaN is among the choices). Returns lane k's pick k.
+__device__ __forceinline__ u32 select_row_general(const float* logits, float* scores_out, const float* bias, const b200moe_route_policy& p, u32 row, u32 lane, float* s) {
     const u32 E = p.experts;
     float* c = s + E;
     float* gs = c + E;
@@ -300,17 +299,28 @@ static __device__ __noinline__ u32 select_row_general(const float* logits, float
     return my_id;
 }
 
-// EPL: a lane's experts on the fast path; 32 EPL is the most that the calling kernel sees.
+// The same out of line, for a kernel that runs once a call on cold instruction caches, where every jump over code that is not run costs 500 to 1,000 clocks.
+static __device__ __noinline__ u32 select_row_apart(const float* logits, float* scores_out, const float* bias, const b200moe_route_policy& p, u32 row, u32 lane, float* s) {
+    return select_row_general(logits, scores_out, bias, p, row, lane, s);
+}
+
+// Whether a policy's groups let rows take the fast path: all experts one group, runs of 2^i lanes or whole runs of 32.
+__host__ __device__ __forceinline__ bool fast_groups(const b200moe_route_policy& p) {
+    const u32 run = p.experts / p.n_group;
+    return p.n_group == 1 || run % 32 == 0 || (run < 32 && (run & (run - 1u)) == 0);
+}
+
+// EPL: a lane's experts on the fast path; 32 EPL is the most that the calling kernel sees. 0: the general path alone, in line.
 template <int EPL>
 __device__ __forceinline__ u32 select_row(const float* logits, float* scores_out, const float* bias,
                                           const b200moe_route_policy& p, u32 row, u32 lane, float* s,
                                           u32* ids, float* weights) {
-    const u32 run = p.experts / p.n_group;
     u32 my_id = kNone;
-    // the fast path unless a NaN needs the serial rule
-    if (!((p.n_group == 1 || run % 32 == 0 || (run < 32 && (run & (run - 1u)) == 0)) && select_row_fast<EPL>(logits, scores_out, bias, p, row, lane, s, &my_id))) {
-        __syncwarp();
+    if constexpr (EPL == 0) {
         my_id = select_row_general(logits, scores_out, bias, p, row, lane, s);
+    } else if (!(fast_groups(p) && select_row_fast<EPL>(logits, scores_out, bias, p, row, lane, s, &my_id))) {  // the fast path unless a NaN needs the serial rule
+        __syncwarp();
+        my_id = select_row_apart(logits, scores_out, bias, p, row, lane, s);
     }
     return finish_row(p, row, lane, s, my_id, ids, weights);
 }

@@ -667,7 +667,8 @@ def test_forced_form_is_the_one_that_runs(gpu, oracle, types, form, stem, rows, 
 
 # choices in registers: up to 128, 256 and 1024 experts; groups of whole runs of 32 (one, two, three a group), of 2 to 16 lanes, and of 12 (general path)
 @pytest.mark.parametrize("experts,top_k,groups,kept", [(1, 1, 1, 1), (60, 6, 1, 1), (127, 32, 1, 1), (129, 8, 1, 1), (256, 8, 1, 1), (1000, 8, 1, 1), (1024, 32, 1, 1), (256, 8, 8, 4),
-                                                       (256, 8, 4, 2), (192, 6, 2, 1), (512, 8, 8, 3), (64, 8, 32, 5), (64, 8, 8, 4), (128, 8, 8, 4), (96, 8, 8, 4)])
+                                                       (256, 8, 4, 2), (192, 6, 2, 1), (512, 8, 8, 3), (64, 8, 32, 5), (64, 8, 8, 4), (128, 8, 8, 4), (96, 8, 8, 4),
+                                                       (160, 8, 8, 4), (384, 8, 8, 4), (1000, 8, 8, 3)])
 @pytest.mark.parametrize("score", [O.SOFTMAX, O.SIGMOID])
 def test_selection_by_reductions(gpu, oracle, experts, top_k, groups, kept, score):
     """Random rows, rows full of ties (four values, zeros of both signs), rows with infinities and a row with a NaN, under both key rules."""

@@ -352,7 +352,8 @@ Q8Form pick_q8_form(const b200moe_shape& s, bool shot_fits, bool wide_fits, bool
 }
 // The four-chain down on the tensor cores (down_chain4_mma.cu), else in the dp4a forms of gemv_q4k.cu. By the entries of an expert: slots over ALL experts, since of a rank's share
 // of the experts the window's slots are a share too. The dp4a forms pay by the entry, and the more the longer the rows, so the line falls with their length: from 3.5 (Q8_0) and 4.5
-// entries (Q5_1) at 128 weights to none and one at 1024. A window whose items are no more than SMs is one item's time and has the tensor cores at any number. Layers, us, the better
+// entries (Q5_1) at 128 weights to none and one at 1024. A window whose items are no more than SMs is one item's time and has the tensor cores from a
+// quarter of an entry on (below, a share of the experts often has none, and a launch without items takes 1.2 us longer there). Layers, us, the better
 // dp4a form and this: 128 experts of 640 -> 2560, top 8, Q5_1 16 rows 74.0 and 85.9, 40 115.5 and 121.4, 48 127.0 and 129.4, 64 151.8 and 139.9, a quarter of them owned 31.3 and
 // 35.3, 43.6 and 41.5, 44.2 and 41.8, 56.2 and 48.7; Q8_0 24 rows 104 and 114, 32 119 and 121, 48 146 and 138, a quarter owned 40.4 and 39.5, 48.4 and 46.8, 53.3 and 48.2; 60 of
 // 768 -> 2560, top 4, Q5_1 15 rows 48.3 and 53.2, 30 74.7 and 73.2, 45 86.6 and 78.4, Q8_0 8 rows 40.0 and 42.3, 15 52.3 and 51.5, 30 78.9 and 67.0; of 1536 -> 2560 Q5_1 8 rows
@@ -366,7 +367,7 @@ bool chain4_mma_pays(const b200moe_down_view& v, u64 slots, bool alone, u32 chun
     const b200moe_shape& s = v.shape;
     const bool q51 = s.down_type == B200MOE_TYPE_Q5_1;
     if (alone && slots <= (q51 && s.inter <= 1024 ? 256u : 24u)) return false;
-    if (!alone && u64(experts_met(s, slots, v.max_union)) * chunks <= static_cast<u32>(device_sm_count())) return true;
+    if (!alone && slots * 4 >= s.experts && u64(experts_met(s, slots, v.max_union)) * chunks <= static_cast<u32>(device_sm_count())) return true;
     const u32 none = (q51 ? 1280u : 1024u) + (alone ? 256u : 0u), least = std::max(q51 ? 256u : 0u, none - std::min(none, s.inter));  // in 256ths of an entry
     return slots * 256 > u64(s.experts) * least;
 }

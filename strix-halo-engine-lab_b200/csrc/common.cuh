@@ -88,9 +88,9 @@ template <class T>
 __device__ __forceinline__ T load(const T* p) { return *p; }
 // The same past the L1 cache, for what is known to be complete before the wait (ChainHints): the multiprocessor's L1 may hold lines of an earlier call.
 __device__ __forceinline__ u32 load_l2(const u32* p) { return __ldcg(p); }
-// Whether the block leaves a stage out because the job's summary says so: one answer for all of its threads (every one calls it). Another block of the same
+// Whether the block leaves a stage out because the job's summary says so: one answer for all of its threads (every one calls it; no barrier where there is no summary). Another block of the same
 // launch may raise the word meanwhile, and threads that read it one by one could part: those that stay would wait at a barrier of counted warps for good.
-__device__ __forceinline__ bool block_skips(const u32* summary) { return __syncthreads_or(summary && *summary) != 0; }
+__device__ __forceinline__ bool block_skips(const u32* summary) { return summary && __syncthreads_or(*summary != 0u) != 0; }
 // Enqueues a kernel of the chain; its status is read by after_launch.
 template <class... P, class... A>
 inline void chain_launch_attrs(u32 extra, void (*kernel)(P...), dim3 grid, dim3 block, u32 smem, cudaStream_t stream, A&&... args) {

@@ -115,7 +115,8 @@ u32 debug_value(u32 key) { return key < 3 ? g_debug[key].load(std::memory_order_
 
 u32 experts_met(const b200moe_shape& s, u64 slots, u32 max_union) {
     const double of = slots > max_union ? max_union : s.experts;
-    return std::min(max_union, static_cast<u32>(std::ceil(of * -std::expm1(-static_cast<double>(slots) / s.experts))));
+    const double none = std::pow(1.0 - static_cast<double>(s.top_k) / s.experts, static_cast<double>(slots) / s.top_k);  // of its rows, whose experts are distinct, choose one
+    return std::min(max_union, static_cast<u32>(std::ceil(of * (1.0 - none) - 1e-6)));
 }
 
 namespace {

@@ -1417,7 +1417,8 @@ def test_four_chain_down_skipped_after_its_weights_were_asked_for(gpu, oracle, r
 
 @pytest.mark.parametrize("down_type,rows,top_k,E,own,H,I,name", [(8, 40, 8, 128, 64, 2048, 128, "stream"), (8, 54, 8, 128, 64, 1024, 256, "mma"), (7, 40, 4, 64, 16, 2048, 512, "stream"),
                                                                  (7, 80, 4, 64, 16, 2048, 512, "mma"), (7, 24, 8, 64, 32, 1024, 256, "stream"), (8, 8, 8, 128, 32, 1024, 640, "stream"),
-                                                                 (7, 3, 2, 16, 16, 512, 640, "mma"), (8, 5, 4, 64, 8, 1024, 96, "mma"), (7, 1, 1, 1, 1, 2048, 512, "mma")])
+                                                                 (7, 3, 2, 16, 16, 512, 640, "mma"), (8, 5, 4, 64, 8, 1024, 96, "mma"), (7, 1, 1, 1, 1, 2048, 512, "mma"),
+                                                                 (7, 1, 8, 8, 8, 1280, 768, "stream"), (7, 1, 8, 8, 8, 1024, 768, "mma"), (8, 2, 1, 16, 8, 512, 640, "stream")])
 def test_four_chain_tensor_core_line(gpu, oracle, down_type, rows, top_k, E, own, H, I, name):
     """A layer's down on both sides of the line to the tensor cores, by the entries of an expert whatever part of the experts is owned, and where its items are no more than SMs."""
     import b200moe

@@ -119,17 +119,14 @@ __global__ void __launch_bounds__(kThreads) q8_shot_kernel(const __grid_constant
             for (u32 i = 0; i < (a.wait_limit >> 4) + 64u; ++i)
                 if (mbar_try_wait(&full[n % a.stages], (n / a.stages) & 1u, kWaitHintNs)) break;
     };
-    u32 my_slot = lane < min(a.cap, ee - eb) ? load(a.routes.slots + eb + lane) : 0u;  // under way while the summary is
-    if (DOWN && block_skips(a.summary)) {  // an aborted projection skips the stage
-        if (tid == 0) drain(0);
-        return;
-    }
+    // An aborted projection skips the stage: one answer for the block, at the barrier that its first entries' rows are waited for at. A barrier for it alone took 0.2 us of a one-row call.
+    const u32 skips = DOWN && a.summary ? *a.summary : 0u;
     const u32 in_stride = a.in.stride ? a.in.stride : a.in.width, groups = a.K / 32;
     bool ok = true;
     u32 n = 0, landed = 0;  // the run in hand; the runs that have been seen to land
     for (u32 p0 = eb; p0 < ee; p0 += a.cap) {
         const u32 nr = min(a.cap, ee - p0);
-        if (p0 != eb) my_slot = lane < nr ? load(a.routes.slots + p0 + lane) : 0u;
+        const u32 my_slot = lane < nr ? load(a.routes.slots + p0 + lane) : 0u;
         const u32 my_row = DOWN || lane >= nr ? my_slot : load(a.routes.rows + p0 + lane);
         if (p0 != eb) __syncthreads();  // the previous pass has read the entries' rows and the outputs
         for (u32 r = 0; r < nr; ++r) {
@@ -140,7 +137,10 @@ __global__ void __launch_bounds__(kThreads) q8_shot_kernel(const __grid_constant
             for (u32 i = tid; i < groups; i += kThreads) grouped::cp_async4(s_deltas + r * groups + i, d + i);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
+        if (__syncthreads_or(p0 == eb && skips != 0u)) {
+            if (tid == 0) drain(0);
+            return;
+        }
         float cls[kRowsWarp][NR];
 #pragma unroll
         for (u32 i = 0; i < kRowsWarp; ++i)
